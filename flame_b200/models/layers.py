@@ -465,17 +465,14 @@ class Mamba(nn.Module):
             self.dt_proj.bias.copy_((dt + torch.log(-torch.expm1(-dt))).to(dev))
 
     def forward(self, x: torch.Tensor, meta: VarlenMeta) -> torch.Tensor:
-        from ..ops.scan import selective_scan
+        from ..ops.gates import split_columns
+        from ..ops.scan import mamba_scan_gate
         Di, N, R = self.intermediate_size, self.ssm_state_size, self.time_step_rank
-        xz = self.in_proj(x)
-        h, z = xz[:, :Di], xz[:, Di:]
+        h, z = split_columns(self.in_proj(x), (Di, Di))
         h = self.conv1d(h.contiguous(), meta)
-        ssm = self.x_proj(h)
-        dt, B, C = ssm[:, :R], ssm[:, R:R + N], ssm[:, R + N:]
-        delta = F.softplus(self.dt_proj(dt.contiguous()).float())
+        dt, B, C = split_columns(self.x_proj(h), (R, N, N))
         A = -torch.exp(self.A_log.float())
-        y = selective_scan(h, delta, A, B, C, self.D, meta)
-        y = y * F.silu(z)
+        y = mamba_scan_gate(h, self.dt_proj(dt.contiguous()), A, B, C, self.D, z, meta)
         return self.out_proj(y.to(x.dtype))
 
 

@@ -224,56 +224,84 @@ class ScalarPrep(torch.autograd.Function):
         return dq, dk_, (dg if ctx.has_g else None), None
 
 
-_lib.register("fb_sscan_fwd", [c_void_p] * 8 + [c_int] + [c_void_p] * 4 + [c_int, c_int, c_int, c_void_p])
-_lib.register("fb_sscan_bwd", [c_void_p] * 9 + [c_int] + [c_void_p] * 10 + [c_int, c_int, c_int, c_void_p])
+_vp, _i, _ll = c_void_p, c_int, c_longlong
+_SSCAN_IN = [_vp, _ll, _vp, _ll, _i, _vp, _ll, _vp, _ll, _vp, _ll, _i, _vp, _vp, _vp, _vp, _vp, _i]
+_lib.register("fb_sscan_fwd", _SSCAN_IN + [_vp] * 4 + [_i] * 4 + [_vp])
+_lib.register("fb_sscan_bwd", _SSCAN_IN + [_vp] * 13 + [_ll] + [_i] * 3 + [_vp])
 _lib.register("fb_sscan_channel_blocks", [c_int])
+_lib.register("fb_sscan_padded", [c_int])
+
+
+def _rows(x: torch.Tensor) -> torch.Tensor:
+    """``x`` with unit stride along its rows (the kernels take any row stride)."""
+    return x if x.stride(1) == 1 or x.shape[1] == 1 else x.contiguous()
 
 
 class SelectiveScan(torch.autograd.Function):
-    """Mamba-1 selective scan on the chunk-parallel kernels of ``csrc/sscan.cu``.  Inputs in the 64-token chunk layout:
-    u ``[NC, 64, Di]`` bf16, delta ``[NC, 64, Di]`` fp32, A ``[Di, 16]`` fp32, B, C ``[NC, 64, 16]`` fp32, D ``[Di]`` fp32;
-    ``first`` / ``last``: int64 chunk range of every document.  Returns y ``[NC, 64, Di]`` bf16."""
+    """Mamba-1 selective scan on the chunk-parallel kernels of ``csrc/sscan.cu``, on packed tokens: u ``[T, Di]`` bf16, delta
+    ``[T, Di]`` (fp32, or with ``raw`` the bf16 argument of a softplus), A ``[Di, 16]`` fp32, B, C ``[T, 16]`` (both bf16 or both
+    fp32), D ``[Di]`` fp32; z ``[T, Di]`` bf16 or None.  Rows may have any stride.  Returns bf16 ``[T, Di]``: y, or ``y silu(z)``.
+    ``lay``: the 64-token ``ChunkLayout`` of the documents."""
 
     @staticmethod
-    def forward(ctx, u, delta, A, B, C, D, first, last):
-        u, delta, A, B, C, D = (t.contiguous() for t in (u, delta, A, B, C, D))
-        NC, L, Di = u.shape
-        N = A.shape[1]
-        assert L == 64 and N == 16 and u.dtype == torch.bfloat16
+    def forward(ctx, u, delta, A, B, C, D, z, lay, raw):
+        u, delta, B, C = _rows(u), _rows(delta), _rows(B), _rows(C)
+        z = None if z is None else _rows(z)
+        A, D = A.contiguous(), D.contiguous()
+        A = A if A.data_ptr() % 16 == 0 else A.clone()
+        T, Di = lay.T, u.shape[1]
+        for t in (u, delta, B, C) + (() if z is None else (z,)):
+            if t.shape[0] < T:
+                raise ValueError(f"selective scan: {t.shape[0]} rows for documents of {T} tokens")
         dev = u.device
-        hloc = torch.empty(NC, Di, N, dtype=torch.float32, device=dev)
-        P, hin = torch.empty_like(hloc), torch.empty_like(hloc)
-        y = torch.empty_like(u)
-        rc = _lib.lib().fb_sscan_fwd(u.data_ptr(), delta.data_ptr(), A.data_ptr(), B.data_ptr(), C.data_ptr(), D.data_ptr(),
-                                     first.data_ptr(), last.data_ptr(), first.numel(), hloc.data_ptr(), P.data_ptr(),
-                                     hin.data_ptr(), y.data_ptr(), NC, Di, N, _lib.stream_ptr())
+        L = _lib.lib()
+        DiP = int(L.fb_sscan_padded(Di))
+        keep = any(ctx.needs_input_grad)
+        st = torch.empty(lay.NC, 4, 16, DiP, dtype=torch.float32, device=dev)
+        sdl = torch.empty(lay.NC, DiP, dtype=torch.float32, device=dev)
+        y = torch.empty(T, Di, dtype=torch.bfloat16, device=dev) if keep or z is None else None
+        out = torch.empty(T, Di, dtype=torch.bfloat16, device=dev) if z is not None else None
+        ctx.geometry = (lay, raw, DiP)
+        rc = L.fb_sscan_fwd(*SelectiveScan._operands(u, delta, A, B, C, D, z, lay, raw), st.data_ptr(), sdl.data_ptr(), _lib.ptr(y),
+                            _lib.ptr(out), int(keep), lay.NC, Di, A.shape[1], _lib.stream_ptr())
         _lib.check(rc, "fb_sscan_fwd")
         _lib.count_launch(3)
-        ctx.save_for_backward(u, delta, A, B, C, D, first, last, P, hin)
-        return y
+        ctx.save_for_backward(u, delta, A, B, C, D, z, st, sdl, y if z is not None else None)
+        return y if z is None else out
 
     @staticmethod
-    def backward(ctx, dy):
-        u, delta, A, B, C, D, first, last, P, hin = ctx.saved_tensors
-        NC, L, Di = u.shape
-        N = A.shape[1]
+    def _operands(u, delta, A, B, C, D, z, lay, raw):
+        return (u.data_ptr(), u.stride(0), delta.data_ptr(), delta.stride(0), int(raw), _lib.ptr(z), 0 if z is None else z.stride(0),
+                B.data_ptr(), B.stride(0), C.data_ptr(), C.stride(0), int(B.dtype == torch.bfloat16), A.data_ptr(), D.data_ptr(),
+                lay.inv_i32.data_ptr(), lay.first.data_ptr(), lay.last.data_ptr(), lay.first.numel())
+
+    @staticmethod
+    def backward(ctx, dout):
+        u, delta, A, B, C, D, z, st, sdl, y = ctx.saved_tensors
+        lay, raw, DiP = ctx.geometry
+        T, Di = lay.T, u.shape[1]
         dev = u.device
-        dy = dy.to(torch.bfloat16).contiguous()
-        gloc, gout = torch.empty_like(P), torch.empty_like(P)
-        du = torch.empty(NC, L, Di, dtype=torch.float32, device=dev)
-        ddl = torch.empty_like(du)
-        nblk = int(_lib.lib().fb_sscan_channel_blocks(Di))
-        dA = torch.empty(NC, Di, N, dtype=torch.float32, device=dev)      # per-chunk partials, summed below
-        dB = torch.empty(nblk, NC, L, N, dtype=torch.float32, device=dev)  # per-channel-block partials
-        dC = torch.empty_like(dB)
-        dD = torch.empty(NC, Di, dtype=torch.float32, device=dev)
-        rc = _lib.lib().fb_sscan_bwd(u.data_ptr(), delta.data_ptr(), A.data_ptr(), B.data_ptr(), C.data_ptr(), D.data_ptr(),
-                                     dy.data_ptr(), first.data_ptr(), last.data_ptr(), first.numel(), P.data_ptr(),
-                                     hin.data_ptr(), gloc.data_ptr(), gout.data_ptr(), du.data_ptr(), ddl.data_ptr(),
-                                     dA.data_ptr(), dB.data_ptr(), dC.data_ptr(), dD.data_ptr(), NC, Di, N, _lib.stream_ptr())
+        L = _lib.lib()
+        dout = dout.to(torch.bfloat16).contiguous()
+
+        def grad(like):  # rows past the documents have no part in the result
+            t = torch.empty(like.shape, dtype=like.dtype, device=dev)
+            if like.shape[0] > T:
+                t[T:].zero_()
+            return t
+        du, ddl, dB, dC = grad(u), grad(delta), grad(B), grad(C)
+        dz = None if z is None else grad(z)
+        nblk = int(L.fb_sscan_channel_blocks(Di))
+        adj = torch.empty(lay.NC, 16, DiP, dtype=torch.float32, device=dev)
+        dA = torch.empty(lay.NC, 16, DiP, dtype=torch.float32, device=dev)     # per-chunk partials, summed below
+        dD = torch.empty(lay.NC, DiP, dtype=torch.float32, device=dev)
+        part = torch.empty(nblk, T, 32, dtype=torch.float32, device=dev)       # per-channel-block partials of dB | dC
+        rc = L.fb_sscan_bwd(*SelectiveScan._operands(u, delta, A, B, C, D, z, lay, raw), st.data_ptr(), sdl.data_ptr(), _lib.ptr(y),
+                            dout.data_ptr(), adj.data_ptr(), du.data_ptr(), ddl.data_ptr(), _lib.ptr(dz), dA.data_ptr(),
+                            part.data_ptr(), dD.data_ptr(), dB.data_ptr(), dC.data_ptr(), T, lay.NC, Di, A.shape[1], _lib.stream_ptr())
         _lib.check(rc, "fb_sscan_bwd")
-        _lib.count_launch(3)
-        return du.to(u.dtype), ddl, dA.sum(0), dB.sum(0), dC.sum(0), dD.sum(0), None, None
+        _lib.count_launch(4)
+        return du, ddl, dA.sum(0)[:, :Di].t(), dB, dC, dD.sum(0)[:Di], dz, None, None
 
 
 _lib.register("fb_vdecay_diag_fwd", [c_void_p] * 4 + [c_int, c_int, c_int, c_void_p])

@@ -230,6 +230,46 @@ def test_selective_scan_kernels_match_recurrence():
         assert rel_err(a, b) < 2e-2
 
 
+@pytest.mark.parametrize("Di,lens", [(2, [1]), (70, [15, 16, 17]), (129, [31, 33, 1, 48]), (130, [63, 64, 65, 2]), (192, [200, 127, 49])])
+@pytest.mark.parametrize("gate", [False, True])
+def test_selective_scan_edges(Di, lens, gate):
+    """Channel counts and documents around the blocks' edges, operands as strided columns of a projection, with and without
+    the layer's softplus and gate, against the token-by-token recurrence in fp64.  Operands and results are bf16 (2^-9 of
+    rounding each, sums over 16 states and up to 300 steps of same-sized terms): 1e-2."""
+    from flame_b200.ops.scan import mamba_scan_gate, selective_scan
+    torch.manual_seed(6)
+    meta = _meta(lens)
+    T, N, R = sum(lens), 16, 3
+    wide = lambda n: torch.randn(T, n, device=DEV, dtype=torch.bfloat16).requires_grad_(True)  # noqa: E731
+    uz, ssm, raw = wide(2 * Di), wide(R + 2 * N), wide(Di)
+    Alog = torch.log(torch.rand(Di, N, device=DEV) * 8 + 0.1).requires_grad_(True)
+    D = torch.randn(Di, device=DEV).requires_grad_(True)
+    ins = [uz, ssm, raw, Alog, D]
+    dy = torch.randn(T, Di, device=DEV, dtype=torch.bfloat16)
+
+    def grads(y):
+        return [y.detach()] + list(torch.autograd.grad(y, ins, dy.to(y.dtype), retain_graph=True))
+    A = -torch.exp(Alog)
+    cols = lambda c: (c(uz)[:, :Di], c(ssm)[:, R:R + N], c(ssm)[:, R + N:], c(uz)[:, Di:])  # noqa: E731
+    u, B, C, z = cols(lambda t: t)
+    if gate:
+        out = grads(mamba_scan_gate(u, raw, A, B, C, D, z, meta))
+    else:
+        out = grads(selective_scan(u, F.softplus(raw.float()), A, B, C, D, meta) + 0 * z)
+    u, B, C, z = cols(lambda t: t.double())
+    h, rows = None, []
+    dl = F.softplus(raw.double())
+    starts = set(meta.cu_cpu().tolist())
+    for t in range(T):
+        h = torch.zeros(Di, N, device=DEV, dtype=torch.float64) if t in starts else h
+        h = h * (dl[t][:, None] * A.double()).exp() + (dl[t] * u[t])[:, None] * B[t][None]
+        rows.append((h * C[t][None]).sum(-1) + D.double() * u[t])
+    y = torch.stack(rows)
+    ref = grads(y * F.silu(z) if gate else y + 0 * z)
+    for a, b in zip(out, ref):
+        assert rel_err(a, b) < 1e-2
+
+
 def test_gsa_kernels_match_fp32_chunk_reference():
     from flame_b200.ops import linear_attn as la
     from flame_b200.ops.gla import gsa
