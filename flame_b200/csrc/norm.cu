@@ -1,6 +1,5 @@
 // Fused RMSNorm (+ residual add) forward and backward, and the gated variant used by the linear-attention
-// layers.  Bandwidth-bound: one warp owns a row, 16-byte loads, fp32 math, a single pass over HBM
-// (the second sweep over the row hits L1).
+// layers.  Bandwidth-bound: 16-byte loads, fp32 math, a single pass over HBM.
 //
 //   forward :  r = x (+ residual_in);  y = r * rsqrt(mean(r^2) + eps) * w;   optionally writes r and rstd
 //   backward:  dx = rstd * (dy*w - xhat * mean(dy*w*xhat)) (+ d_residual);   dw = sum_rows dy * xhat
@@ -103,208 +102,219 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
-__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// Forward for short rows (D <= 256): LPR = D / 8 lanes (rounded up to a power of two) share a row, so that a warp of the
+// per-head norms is full, and a thread takes FR rows at once to keep FR (gated: 2 FR) 16-byte loads in flight.  D = 128,
+// 524,288 rows: the one-warp-per-row form above took 0.107 ms (2.5 TB/s), half of its lanes without work.
+constexpr int FR = 4;
+template <bool HAS_RES, bool WRITE_RES, int GATE, int LPR>
+__global__ void __launch_bounds__(WARPS * 32)
+rmsnorm_fwd_short_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in, const __nv_bfloat16* __restrict__ w,
+                         const __nv_bfloat16* __restrict__ gate, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out,
+                         float* __restrict__ rstd, long long rows, int D, float eps) {
+  constexpr int SLOTS = WARPS * 32 / LPR;
+  const int l = threadIdx.x % LPR, col = l * 8;
+  const bool live = col < D;
+  const long long r0 = (long long)blockIdx.x * (SLOTS * FR) + threadIdx.x / LPR;
+  float ww[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) ww[j] = 1.f;
+  if (w != nullptr && live) unpack8(*reinterpret_cast<const uint4*>(w + col), ww);
+  uint4 xa[FR], ra[HAS_RES ? FR : 1], ta[GATE ? FR : 1];
+#pragma unroll
+  for (int k = 0; k < FR; ++k) {
+    const long long row = r0 + k * SLOTS;
+    const bool ok = live && row < rows;
+    xa[k] = ok ? *reinterpret_cast<const uint4*>(x + row * D + col) : make_uint4(0, 0, 0, 0);
+    if (HAS_RES) ra[k] = ok ? *reinterpret_cast<const uint4*>(res_in + row * D + col) : make_uint4(0, 0, 0, 0);
+    if (GATE) ta[k] = ok ? *reinterpret_cast<const uint4*>(gate + row * D + col) : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int k = 0; k < FR; ++k) {
+    const long long row = r0 + k * SLOTS;
+    const bool ok = live && row < rows;
+    float a[8];
+    unpack8(xa[k], a);
+    if (HAS_RES) {
+      float b[8];
+      unpack8(ra[k], b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] += b[j];
+    }
+    if (WRITE_RES) {
+      const uint4 q = pack8(a);
+      if (ok) *reinterpret_cast<uint4*>(res_out + row * D + col) = q;
+      unpack8(q, a);  // normalise what was stored, so backward sees identical values
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += a[j] * a[j];
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    const float rs = rsqrtf(ss / (float)D + eps);
+    if (l == 0 && row < rows && rstd != nullptr) rstd[row] = rs;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) a[j] = a[j] * rs * ww[j];
+    if (GATE) {
+      float g[8];
+      unpack8(ta[k], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) a[j] *= (GATE == 1) ? g[j] * sigmoidf_(g[j]) : sigmoidf_(g[j]);
+    }
+    if (ok) *reinterpret_cast<uint4*>(y + row * D + col) = pack8(a);
+  }
+}
 
-// Backward.  `xin` is the tensor that was normalised (the stored residual sum when a residual was fused).
-// dw partials: each CTA reduces its rows into dw_part[blockIdx.x, :]; a second kernel sums the CTAs in order.
-template <bool HAS_DRES, int GATE, int NITER>
-__global__ void __launch_bounds__(WARPS * 32, 2)
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ xin,
-                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                   const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ dres,
-                   __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dgate, float* __restrict__ dw_part,
-                   long long rows, int D, int rows_per_cta) {
-  extern __shared__ float s_dw_all[];  // [WARPS][D]: every warp owns a private row, so no atomics and a fixed order
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nvec = D >> 3;
-  float* s_dw = s_dw_all + (size_t)warp * D;
-  for (int i = threadIdx.x; i < WARPS * D; i += blockDim.x) s_dw_all[i] = 0.f;
-  __syncthreads();
-  const long long row0 = (long long)blockIdx.x * rows_per_cta;
-  const long long row1 = min(rows, row0 + rows_per_cta);
-  const uint4* wv = reinterpret_cast<const uint4*>(w);
-  // NITER > 0: D == 256 * NITER and each lane keeps its dw columns in registers across all of its rows
-  float dw_reg[NITER > 0 ? NITER : 1][8];
+// Backward.  `xin` is the tensor that was normalised (the stored residual sum when a residual was fused).  A thread owns
+// eight columns and keeps their dw in registers over all rows of its CTA; a row belongs to LPR lanes of a warp (D <= 256,
+// LPR = D / 8 rounded up to a power of two, several rows side by side) or to the whole CTA (LPR = 0, D / 8 threads rounded
+// up to warps, sums through shared memory).  BR rows per trip: their 2 BR to 3 BR 16-byte loads are issued together and
+// stay packed in registers, so every operand is read once and enough bytes are in flight to be bound by DRAM; one warp
+// per row, as before, kept one row's loads in flight and re-read D > 1024 and D < 256 through L1 (D = 128, 524,288 rows: 0.28 ms;
+// D = 2048, 32,768 rows: 0.24 ms; both 1.6 TB/s).  dw partials: one row per CTA, which a second kernel sums in order.
+template <bool HAS_DRES, int GATE, int LPR, int BR, int TPB>
+__global__ void __launch_bounds__(TPB, TPB == 256 ? 2 : 1)
+rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ xin, const __nv_bfloat16* __restrict__ w,
+                   const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ dres,
+                   __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dgate, float* __restrict__ dw_part, long long rows, int D,
+                   int rows_per_cta) {
+  constexpr int SLOTS = LPR ? WARPS * 32 / (LPR ? LPR : 1) : 1;
+  __shared__ float s_c[LPR ? 1 : 2][LPR ? 1 : BR][LPR ? 1 : 32];
+  __shared__ float s_dw[LPR ? SLOTS : 1][LPR ? LPR * 8 + 1 : 1];
+  const int l = LPR ? threadIdx.x % (LPR ? LPR : 1) : threadIdx.x, slot = LPR ? threadIdx.x / (LPR ? LPR : 1) : 0;
+  const int col = l * 8;
+  const bool live = col < D;
+  const long long row0 = (long long)blockIdx.x * rows_per_cta, row1 = min(rows, row0 + rows_per_cta);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  float ww[8], dw[8];
 #pragma unroll
-  for (int a = 0; a < (NITER > 0 ? NITER : 1); ++a)
+  for (int j = 0; j < 8; ++j) ww[j] = 1.f, dw[j] = 0.f;
+  if (w != nullptr && live) unpack8(*reinterpret_cast<const uint4*>(w + col), ww);
+  const float inv_d = 1.f / (float)D;
+  int flip = 0;
+  for (long long rb = row0; rb < row1; rb += SLOTS * BR, flip ^= 1) {
+    uint4 xa[BR], ga[BR], ra[HAS_DRES ? BR : 1], ta[GATE ? BR : 1];
+    float rs[BR], c[BR];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dw_reg[a][j] = 0.f;
-  if constexpr (NITER > 0) {
-    // D == 256 * NITER: a lane owns NITER vectors of 8 columns.  x, dy (and the residual gradient, the gate) of a row are
-    // read ONCE and stay in registers as packed bf16 for both passes, so a row costs one round trip and half the L1
-    // traffic of re-reading; only the 2 KB weight vector is re-read (L1 resident).
-    for (long long row = row0 + warp; row < row1; row += WARPS) {
-      const uint4* dyr = reinterpret_cast<const uint4*>(dy + row * D);
-      const uint4* xr = reinterpret_cast<const uint4*>(xin + row * D);
-      uint4 xa[NITER], ga[NITER], ra[HAS_DRES ? NITER : 1], ta[GATE ? NITER : 1];
+    for (int k = 0; k < BR; ++k) {
+      const long long row = rb + slot + k * SLOTS;
+      const bool ok = live && row < row1;
+      // streaming loads: every operand row is read exactly once
+      const uint4 none = make_uint4(0, 0, 0, 0);
+      xa[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(xin + row * D + col)) : none;
+      ga[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(dy + row * D + col)) : none;
+      if (HAS_DRES) ra[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(dres + row * D + col)) : none;
+      if (GATE) ta[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(gate + row * D + col)) : none;
+      rs[k] = row < row1 ? rstd[row] : 0.f;
+    }
 #pragma unroll
-      for (int it = 0; it < NITER; ++it) {
-        // streaming loads: every operand row is read exactly once, so it should not displace the weight vector in L1
-        xa[it] = __ldcs(&xr[lane + it * 32]);
-        ga[it] = __ldcs(&dyr[lane + it * 32]);
-        if (HAS_DRES) ra[it] = __ldcs(&reinterpret_cast<const uint4*>(dres + row * D)[lane + it * 32]);
-        if (GATE) ta[it] = __ldcs(&reinterpret_cast<const uint4*>(gate + row * D)[lane + it * 32]);
-      }
-      const float rs = rstd[row];
-      float c = 0.f;
-#pragma unroll
-      for (int it = 0; it < NITER; ++it) {
-        float a[8], g[8], ww[8];
-        unpack8(xa[it], a);
-        unpack8(ga[it], g);
-        if (w != nullptr) unpack8(wv[lane + it * 32], ww);
-        if (GATE) {
-          float gt[8];
-          unpack8(ta[it], gt);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float sg = sigmoidf_(gt[j]);
-            g[j] *= (GATE == 1) ? gt[j] * sg : sg;
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) c += g[j] * (w != nullptr ? ww[j] : 1.f) * a[j] * rs;
-      }
-      c = warp_sum(c) / (float)D;
-      // keep the compiler from carrying the unpacked fp32 values of the first pass (twice the registers) into the second
-#pragma unroll
-      for (int it = 0; it < NITER; ++it) {
-        asm volatile("" : "+r"(xa[it].x), "+r"(xa[it].y), "+r"(xa[it].z), "+r"(xa[it].w));
-        asm volatile("" : "+r"(ga[it].x), "+r"(ga[it].y), "+r"(ga[it].z), "+r"(ga[it].w));
-      }
-      uint4* dxr = reinterpret_cast<uint4*>(dx + row * D);
-      uint4* dgr = GATE ? reinterpret_cast<uint4*>(dgate + row * D) : nullptr;
-#pragma unroll
-      for (int it = 0; it < NITER; ++it) {
-        float a[8], g[8], ww[8], o[8], gt[8], dgo[8];
-        unpack8(xa[it], a);
-        unpack8(ga[it], g);
-        if (w != nullptr) unpack8(wv[lane + it * 32], ww);
-        if (GATE) unpack8(ta[it], gt);
+    for (int k = 0; k < BR; ++k) {
+      float a[8], g[8];
+      unpack8(xa[k], a);
+      unpack8(ga[k], g);
+      if (GATE) {
+        float gt[8];
+        unpack8(ta[k], gt);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float xhat = a[j] * rs;
-          const float wj = (w != nullptr ? ww[j] : 1.f);
-          float gy = g[j];
-          if (GATE) {
-            const float sg = sigmoidf_(gt[j]);
-            const float act = (GATE == 1) ? gt[j] * sg : sg;
-            const float dact = (GATE == 1) ? sg * (1.f + gt[j] * (1.f - sg)) : sg * (1.f - sg);
-            dgo[j] = g[j] * xhat * wj * dact;
-            gy = g[j] * act;
-          }
-          o[j] = rs * (gy * wj - xhat * c);
-          if (w != nullptr) dw_reg[it][j] += gy * xhat;
+          const float sg = sigmoidf_(gt[j]);
+          g[j] *= (GATE == 1) ? gt[j] * sg : sg;
         }
-        if (HAS_DRES) {
-          float b[8];
-          unpack8(ra[it], b);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += b[j];
-        }
-        __stcs(&dxr[lane + it * 32], pack8(o));
-        if (GATE) __stcs(&dgr[lane + it * 32], pack8(dgo));
       }
+      float s = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += g[j] * ww[j] * a[j] * rs[k];
+#pragma unroll
+      for (int o = (LPR ? LPR : 32) / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      c[k] = s * inv_d;
+    }
+    if constexpr (LPR == 0) {
+      if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < BR; ++k) s_c[flip][k][warp] = c[k];
+      }
+      __syncthreads();  // the two buffers alternate: one barrier per trip separates the writes of a buffer from its last reads
+#pragma unroll
+      for (int k = 0; k < BR; ++k) {
+        float s = 0.f;
+        for (int i = 0; i < nwarps; ++i) s += s_c[flip][k][i];
+        c[k] = s;
+      }
+    }
+    // keep the compiler from carrying the unpacked fp32 values of the first pass (twice the registers) into the second
+#pragma unroll
+    for (int k = 0; k < BR; ++k) {
+      asm volatile("" : "+r"(xa[k].x), "+r"(xa[k].y), "+r"(xa[k].z), "+r"(xa[k].w));
+      asm volatile("" : "+r"(ga[k].x), "+r"(ga[k].y), "+r"(ga[k].z), "+r"(ga[k].w));
+      if (GATE) asm volatile("" : "+r"(ta[k].x), "+r"(ta[k].y), "+r"(ta[k].z), "+r"(ta[k].w));
+    }
+#pragma unroll
+    for (int k = 0; k < BR; ++k) {
+      const long long row = rb + slot + k * SLOTS;
+      float a[8], g[8], o[8], gt[8], dgo[8];
+      unpack8(xa[k], a);
+      unpack8(ga[k], g);
+      if (GATE) unpack8(ta[k], gt);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float xhat = a[j] * rs[k];
+        float gy = g[j];
+        if (GATE) {
+          const float sg = sigmoidf_(gt[j]);
+          const float act = (GATE == 1) ? gt[j] * sg : sg;
+          const float dact = (GATE == 1) ? sg * (1.f + gt[j] * (1.f - sg)) : sg * (1.f - sg);
+          dgo[j] = g[j] * xhat * ww[j] * dact;
+          gy = g[j] * act;
+        }
+        o[j] = rs[k] * (gy * ww[j] - xhat * c[k]);
+        dw[j] += gy * xhat;
+      }
+      if (HAS_DRES) {
+        float b[8];
+        unpack8(ra[k], b);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] += b[j];
+      }
+      if (live && row < row1) {
+        __stcs(reinterpret_cast<uint4*>(dx + row * D + col), pack8(o));
+        if (GATE) __stcs(reinterpret_cast<uint4*>(dgate + row * D + col), pack8(dgo));
+      }
+    }
+  }
+  if (w == nullptr) return;
+  if constexpr (LPR == 0) {
+    if (live) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dw_part[(long long)blockIdx.x * D + col + j] = dw[j];
     }
   } else {
-    for (long long row = row0 + warp; row < row1; row += WARPS) {
-      const uint4* dyr = reinterpret_cast<const uint4*>(dy + row * D);
-      const uint4* xr = reinterpret_cast<const uint4*>(xin + row * D);
-      const uint4* gr = GATE ? reinterpret_cast<const uint4*>(gate + row * D) : nullptr;
-      if (row + WARPS < row1) {
-        // pull this warp's NEXT row into L2 while the current one is processed: the row's two passes then see cache latency
-        const long long nrow = row + WARPS;
-        for (int i = lane; i < nvec; i += 32) {
-          prefetch_l2(dy + nrow * D + i * 8);
-          prefetch_l2(xin + nrow * D + i * 8);
-          if (HAS_DRES) prefetch_l2(dres + nrow * D + i * 8);
-          if (GATE) prefetch_l2(gate + nrow * D + i * 8);
-        }
-      }
-      const float rs = rstd[row];
-      float c = 0.f;
-      for (int i = lane; i < nvec; i += 32) {
-        float a[8], g[8], ww[8];
-        unpack8(xr[i], a);
-        unpack8(dyr[i], g);
-        if (w != nullptr) unpack8(wv[i], ww);
-        if (GATE) {
-          float gt[8];
-          unpack8(gr[i], gt);
-  #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float s = sigmoidf_(gt[j]);
-            g[j] *= (GATE == 1) ? gt[j] * s : s;
-          }
-        }
-  #pragma unroll
-        for (int j = 0; j < 8; ++j) c += g[j] * (w != nullptr ? ww[j] : 1.f) * a[j] * rs;
-      }
-      c = warp_sum(c) / (float)D;
-      uint4* dxr = reinterpret_cast<uint4*>(dx + row * D);
-      const uint4* drr = HAS_DRES ? reinterpret_cast<const uint4*>(dres + row * D) : nullptr;
-      uint4* dgr = GATE ? reinterpret_cast<uint4*>(dgate + row * D) : nullptr;
-  #pragma unroll
-      for (int it = 0; it < (NITER > 0 ? NITER : 64); ++it) {
-        const int i = lane + it * 32;
-        if (NITER == 0 && i >= nvec) break;
-        float a[8], g[8], ww[8], o[8];
-        unpack8(xr[i], a);
-        unpack8(dyr[i], g);
-        if (w != nullptr) unpack8(wv[i], ww);
-        float gt[8], dgo[8];
-        if (GATE) unpack8(gr[i], gt);
-  #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float xhat = a[j] * rs;
-          const float wj = (w != nullptr ? ww[j] : 1.f);
-          float gy = g[j];
-          if (GATE) {
-            const float s = sigmoidf_(gt[j]);
-            const float act = (GATE == 1) ? gt[j] * s : s;
-            const float dact = (GATE == 1) ? s * (1.f + gt[j] * (1.f - s)) : s * (1.f - s);
-            dgo[j] = g[j] * xhat * wj * dact;
-            gy = g[j] * act;
-          }
-          o[j] = rs * (gy * wj - xhat * c);
-          if (w != nullptr) {
-            if (NITER > 0) dw_reg[NITER > 0 ? it : 0][j] += gy * xhat;
-            else s_dw[i * 8 + j] += gy * xhat;
-          }
-        }
-        if (HAS_DRES) {
-          float b[8];
-          unpack8(drr[i], b);
-  #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += b[j];
-        }
-        dxr[i] = pack8(o);
-        if (GATE) dgr[i] = pack8(dgo);
-      }
-    }
-}
-  if (NITER > 0 && w != nullptr) {
 #pragma unroll
-    for (int it = 0; it < (NITER > 0 ? NITER : 1); ++it)
-#pragma unroll
-      for (int j = 0; j < 8; ++j) s_dw[(lane + it * 32) * 8 + j] = dw_reg[it][j];
-  }
-  __syncthreads();
-  if (w != nullptr)
+    for (int j = 0; j < 8; ++j) s_dw[slot][col + j] = dw[j];
+    __syncthreads();
     for (int i = threadIdx.x; i < D; i += blockDim.x) {
       float t = 0.f;
-#pragma unroll
-      for (int k = 0; k < WARPS; ++k) t += s_dw_all[(size_t)k * D + i];
+#pragma unroll 8
+      for (int k = 0; k < SLOTS; ++k) t += s_dw[k][i];
       dw_part[(long long)blockIdx.x * D + i] = t;
     }
+  }
 }
 
-__global__ void colsum_partials_kernel(const float* __restrict__ part, int nparts, int D, float* __restrict__ out,
-                                       int accumulate) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= D) return;
+// Column sums of the CTAs' partial rows in a fixed order: 32 columns x 16 groups of rows per block.
+constexpr int CS_GROUPS = 16;
+__global__ void __launch_bounds__(32 * CS_GROUPS) colsum_partials_kernel(const float* __restrict__ part, int nparts, int D,
+                                                                         float* __restrict__ out, int accumulate) {
+  __shared__ float red[CS_GROUPS][33];
+  const int i = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
-  for (int p = 0; p < nparts; ++p) s += part[(long long)p * D + i];
+  if (i < D) {
+#pragma unroll 8
+    for (int p = threadIdx.y; p < nparts; p += CS_GROUPS) s += part[(long long)p * D + i];
+  }
+  red[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y != 0 || i >= D) return;
+#pragma unroll
+  for (int k = 1; k < CS_GROUPS; ++k) s += red[k][threadIdx.x];
   out[i] = accumulate ? out[i] + s : s;
 }
 
@@ -322,15 +332,24 @@ int fb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, const void*
                    float* rstd, long long rows, int D, float eps, int gate_mode, cudaStream_t stream) {
   if (rows == 0) return 0;
   if (D % 8) return -2;
-  const unsigned grid = (unsigned)((rows + WARPS - 1) / WARPS);
+  const int lpr = D <= 64 ? 8 : D <= 128 ? 16 : 32;  // lanes of a row, D <= 256
+  const int per_block = D <= 256 ? WARPS * 32 / lpr * FR : WARPS;
+  const unsigned grid = (unsigned)((rows + per_block - 1) / per_block);
   const auto X = (const __nv_bfloat16*)x;
   const auto R = (const __nv_bfloat16*)res_in;
   const auto W = (const __nv_bfloat16*)w;
   const auto G = (const __nv_bfloat16*)gate;
   auto Y = (__nv_bfloat16*)y;
   auto RO = (__nv_bfloat16*)res_out;
-#define FWD(HR, WR, GM) \
-  rmsnorm_fwd_kernel<HR, WR, GM><<<grid, WARPS * 32, 0, stream>>>(X, R, W, G, Y, RO, rstd, rows, D, eps)
+#define FWD_S(HR, WR, GM, LP) \
+  rmsnorm_fwd_short_kernel<HR, WR, GM, LP><<<grid, WARPS * 32, 0, stream>>>(X, R, W, G, Y, RO, rstd, rows, D, eps)
+#define FWD(HR, WR, GM)                                                                                            \
+  do {                                                                                                             \
+    if (D <= 64) FWD_S(HR, WR, GM, 8);                                                                             \
+    else if (D <= 128) FWD_S(HR, WR, GM, 16);                                                                      \
+    else if (D <= 256) FWD_S(HR, WR, GM, 32);                                                                      \
+    else rmsnorm_fwd_kernel<HR, WR, GM><<<grid, WARPS * 32, 0, stream>>>(X, R, W, G, Y, RO, rstd, rows, D, eps);   \
+  } while (0)
   if (gate_mode == 0) {
     if (res_in && res_out) FWD(true, true, 0);
     else if (res_in) FWD(true, false, 0);
@@ -341,6 +360,7 @@ int fb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, const void*
     FWD(false, false, 2);
   }
 #undef FWD
+#undef FWD_S
   return fb::launch_ok("rmsnorm_fwd_kernel");
 }
 
@@ -352,25 +372,20 @@ int fb_rmsnorm_bwd(const void* dy, const void* xin, const void* w, const float* 
   if (D % 8) return -2;
   const int parts = fb_rmsnorm_bwd_parts(rows);
   const int rows_per_cta = (int)((rows + parts - 1) / parts);
-  const size_t smem = (size_t)WARPS * D * sizeof(float);
-  if (smem > 220 * 1024) return -3;
-#define BWD_N(HD, GM, NI)                                                                                         \
-  do {                                                                                                            \
-    if (smem > 48 * 1024)                                                                                         \
-      cudaFuncSetAttribute(rmsnorm_bwd_kernel<HD, GM, NI>, cudaFuncAttributeMaxDynamicSharedMemorySize,           \
-                           (int)smem);                                                                            \
-    rmsnorm_bwd_kernel<HD, GM, NI><<<parts, WARPS * 32, smem, stream>>>(                                          \
-        (const __nv_bfloat16*)dy, (const __nv_bfloat16*)xin, (const __nv_bfloat16*)w, rstd,                       \
-        (const __nv_bfloat16*)gate, (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dgate,        \
-        dw_part, rows, D, rows_per_cta);                                                                          \
-  } while (0)
+  if (D > 7040) return -3;
+  const int threads = D <= 256 ? WARPS * 32 : (D / 8 + 31) / 32 * 32;
+#define BWD_N(HD, GM, LP, NR, TPB)                                                                                  \
+  rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB><<<parts, threads, 0, stream>>>(                                           \
+      (const __nv_bfloat16*)dy, (const __nv_bfloat16*)xin, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)gate, \
+      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dgate, dw_part, rows, D, rows_per_cta)
+  // rows per trip by what 128 registers hold packed; one row where a CTA has more than eight warps to overlap (64 registers)
 #define BWD(HD, GM)                                                                                               \
   do {                                                                                                            \
-    if (D == 256) BWD_N(HD, GM, 1);                                                                               \
-    else if (D == 512) BWD_N(HD, GM, 2);                                                                          \
-    else if (D == 1024) BWD_N(HD, GM, 4);                                                                         \
-    else if (D == 2048) BWD_N(HD, GM, 0); /* eight vectors per lane would spill */                                \
-    else BWD_N(HD, GM, 0);                                                                                        \
+    if (D <= 64) BWD_N(HD, GM, 8, (GM ? 2 : 4), 256);                                                             \
+    else if (D <= 128) BWD_N(HD, GM, 16, (GM ? 2 : 4), 256);                                                      \
+    else if (D <= 256) BWD_N(HD, GM, 32, (GM ? 2 : 4), 256);                                                      \
+    else if (D <= 2048) BWD_N(HD, GM, 0, (GM ? 2 : 4), 256);                                                      \
+    else BWD_N(HD, GM, 0, 1, 1024);                                                                               \
   } while (0)
   if (gate_mode == 0) {
     if (dres) { BWD(true, 0); } else { BWD(false, 0); }
@@ -384,7 +399,7 @@ int fb_rmsnorm_bwd(const void* dy, const void* xin, const void* w, const float* 
   int rc = fb::launch_ok("rmsnorm_bwd_kernel");
   if (rc) return rc;
   if (w != nullptr) {
-    colsum_partials_kernel<<<(D + 255) / 256, 256, 0, stream>>>(dw_part, parts, D, dw, accumulate_dw);
+    colsum_partials_kernel<<<(D + 31) / 32, dim3(32, CS_GROUPS), 0, stream>>>(dw_part, parts, D, dw, accumulate_dw);
     rc = fb::launch_ok("colsum_partials_kernel");
   }
   return rc;

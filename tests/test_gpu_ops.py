@@ -192,6 +192,34 @@ def test_short_conv_forward_backward():
             assert rel_err(g, r) < 2e-2
 
 
+@pytest.mark.parametrize("D", [8, 40, 64, 96, 128, 192, 256, 264, 512, 1000, 2048, 2304, 4096, 7040])
+@pytest.mark.parametrize("rows,form", [(1, "plain"), (37, "residual"), (37, "gate"), (700, "plain"), (5000, "residual")])
+def test_rms_norm_every_row_length(D, rows, form):
+    """Row lengths around the forms of the kernels (lanes of a warp, warps of a block), row counts that leave the last block ragged;
+    bf16 results (2^-9) of fp32 arithmetic, weight gradients summed over the rows in fp32 and rounded once: 5e-3."""
+    from flame_b200.ops.norm import rms_norm, rms_norm_gated
+    torch.manual_seed(14)
+    leaf = lambda *s: torch.randn(*s, device=DEV, dtype=torch.bfloat16).requires_grad_(True)  # noqa: E731
+    x, o, w = leaf(rows, D), leaf(rows, D), leaf(D)
+    dy, dr = torch.randn_like(x), torch.randn_like(x)
+    xd, od, wd = (t.detach().double().requires_grad_(True) for t in (x, o, w))
+    if form == "residual":
+        out = list(rms_norm(x, w, 1e-6, o, True))
+        r = (x.detach() + o.detach()).double().requires_grad_(True)   # the sum is stored in bf16 before it is normalised
+        ref = [r * torch.rsqrt(r.pow(2).mean(-1, keepdim=True) + 1e-6) * wd, r]
+        got = torch.autograd.grad(out, [x, w], [dy, dr])
+        want = torch.autograd.grad(ref, [r, wd], [dy.double(), dr.double()])
+    else:
+        gate = o if form == "gate" else None
+        out = [rms_norm_gated(x, o, w, 1e-6) if form == "gate" else rms_norm(x, w, 1e-6)]
+        y = xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * wd
+        ref = [y * torch.nn.functional.silu(od) if gate is not None else y]
+        got = torch.autograd.grad(out, [x, w] + ([o] if gate is not None else []), dy)
+        want = torch.autograd.grad(ref, [xd, wd] + ([od] if gate is not None else []), dy.double())
+    for a, b in zip(out + list(got), ref + list(want)):
+        assert rel_err(a, b) < 5e-3
+
+
 def test_fused_linear_cross_entropy_and_cross_entropy():
     from flame_b200.ops.cross_entropy import cross_entropy, fused_linear_cross_entropy
     torch.manual_seed(5)
