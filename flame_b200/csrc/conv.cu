@@ -1,8 +1,9 @@
 // Depthwise causal short convolution (kernel width <= 8) over packed sequences, with optional bias and SiLU.
 //   pre[t, d] = b[d] + sum_{j < W, j <= pos[t]} w[d, W-1-j] * x[t-j, d];   y = act(pre)
 // `pos[t]` is the token's offset inside its document, so taps never reach into the previous document.
-// Backward runs as: (1) dpre = dy * act'(pre) with pre recomputed, (2) dx[t] = sum_j w[., W-1-j] dpre[t+j] (same
-// document only) together with per-CTA partial sums of dw / db, (3) a fixed-order reduction of the partials.
+// Backward: dpre = dy * act'(pre) with pre recomputed, dx[t] = sum_j w[., W-1-j] dpre[t+j] (same document only) and partial
+// sums of dw / db per strip of rows, then a fixed-order reduction of the partials.  Width 4 (every configuration's) does
+// the first three in one kernel and never stores dpre; the other widths take a dpre pass and a strip pass.
 // Semantics of fla/modules/conv/triton/kernels.py:37-345; the row-strip partial reduction replaces its atomics.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -150,11 +151,10 @@ int launch_conv_point(const void* x, const void* w, const void* b, const int* po
   const __nv_bfloat16 *xx = (const __nv_bfloat16*)x, *ww = (const __nv_bfloat16*)w, *bb = (const __nv_bfloat16*)b,
                       *gg = (const __nv_bfloat16*)dy;
   __nv_bfloat16* oo = (__nv_bfloat16*)out;
-  if (W == 4 || W == 2 || W == 3) {
+  if (W == 2 || W == 3) {
     const int rows = 32;
     dim3 grid((D / 8 + 63) / 64, (unsigned)((T + rows - 1) / rows));
-    if (W == 4) conv_strip_kernel<SILU, WRITE_DPRE, 4><<<grid, 64, 0, stream>>>(xx, ww, bb, pos, gg, oo, T, D, ldx, ldo, rows);
-    else if (W == 3) conv_strip_kernel<SILU, WRITE_DPRE, 3><<<grid, 64, 0, stream>>>(xx, ww, bb, pos, gg, oo, T, D, ldx, ldo, rows);
+    if (W == 3) conv_strip_kernel<SILU, WRITE_DPRE, 3><<<grid, 64, 0, stream>>>(xx, ww, bb, pos, gg, oo, T, D, ldx, ldo, rows);
     else conv_strip_kernel<SILU, WRITE_DPRE, 2><<<grid, 64, 0, stream>>>(xx, ww, bb, pos, gg, oo, T, D, ldx, ldo, rows);
     return fb::launch_ok("conv_strip_kernel");
   }
@@ -221,111 +221,188 @@ __global__ void conv_bwd_kernel(const __nv_bfloat16* __restrict__ dpre, const __
   }
 }
 
-// Width-specialised backward: one pass over the strip with register windows of the last W inputs (for dw) and the last W
-// dpre rows (for dx, written W-1 rows behind the read position), so dpre and x are each read once.
-template <int W>
-__global__ void __launch_bounds__(64) conv_bwd_strip_kernel(const __nv_bfloat16* __restrict__ dpre, const __nv_bfloat16* __restrict__ x,
-                                                            const __nv_bfloat16* __restrict__ w, const int* __restrict__ pos,
-                                                            __nv_bfloat16* __restrict__ dx, float* __restrict__ part, long long T,
-                                                            int D, long long ldx, long long ldd, int rows_per_strip) {
-  const int v = blockIdx.x * 64 + threadIdx.x;
-  if (v >= (D >> 3)) return;
-  const int d0 = v * 8;
-  const long long r0 = (long long)blockIdx.y * rows_per_strip;
-  const long long r1 = min(T, r0 + rows_per_strip);
-  float wv[W][8], dw[W][8], db[8], xwin[W][8], gwin[W][8];
-  int pwin[W];
+// Width 4.  Both directions move each row once and compute little, so what bounds them is bytes in flight: a thread owns
+// four channels (8-byte accesses, a warp covers 128 channels of a row) and a few consecutive rows, and issues all of its
+// loads before it uses any of them; the rows around its own come from L1, where the neighbouring warps of the block bring
+// them.  At 65,536 x 1,024 the walking form of one thread per eight channels took 0.086 ms forward (3.1 TB/s) and
+// 0.33 ms backward in three kernels.
+constexpr int CW = 4;          // taps
+constexpr int CLANES = 32;     // threads along the channels
+constexpr int CGROUPS = 8;     // row groups of a block
+constexpr int FROWS = 8;       // rows of a thread, forward
+constexpr int BROWS = 8;       // rows of a thread, backward
+constexpr int BTILE = BROWS * CGROUPS;
+
+__device__ __forceinline__ void unpack4(const uint2& q, float (&f)[4]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+  const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
+  f[0] = a.x, f[1] = a.y, f[2] = b.x, f[3] = b.y;
+}
+__device__ __forceinline__ uint2 pack4(const float (&f)[4]) {
+  uint2 q;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&q);
+  h[0] = __floats2bfloat162_rn(f[0], f[1]);
+  h[1] = __floats2bfloat162_rn(f[2], f[3]);
+  return q;
+}
+__device__ __forceinline__ void load_taps(const __nv_bfloat16* w, const __nv_bfloat16* b, int d0, float (&wv)[CW][4], float (&bias)[4]) {
+  // four channels' taps are 32 contiguous bytes; as sixteen 2-byte loads they cost the L1 more than the rows themselves
+  const uint4* w4 = reinterpret_cast<const uint4*>(w + (long long)d0 * CW);
 #pragma unroll
-  for (int j = 0; j < W; ++j) {
+  for (int h = 0; h < 2; ++h) {
+    float f[8];
+    unpack8(w4[h], f);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      wv[j][c] = __bfloat162float(w[(d0 + c) * W + (W - 1 - j)]);  // tap at distance j
-      dw[j][c] = 0.f;
-      gwin[j][c] = 0.f;
-    }
-    pwin[j] = -1;
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+      for (int j = 0; j < CW; ++j) wv[j][2 * h + c] = f[c * CW + (CW - 1 - j)];  // tap at distance j
   }
 #pragma unroll
-  for (int c = 0; c < 8; ++c) db[c] = 0.f;
-  // xwin[j] = x[u - j] at the top of iteration u (xwin[0] is loaded inside)
+  for (int c = 0; c < 4; ++c) bias[c] = 0.f;
+  if (b != nullptr) unpack4(*reinterpret_cast<const uint2*>(b + d0), bias);
+}
+
+template <bool SILU>
+__global__ void __launch_bounds__(CLANES * CGROUPS) conv4_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
+                                                                     const __nv_bfloat16* __restrict__ b, const int* __restrict__ pos,
+                                                                     __nv_bfloat16* __restrict__ y, long long T, int D, long long ldx,
+                                                                     long long ldy) {
+  const int d0 = (blockIdx.x * CLANES + threadIdx.x) * 4;
+  const long long r0 = ((long long)blockIdx.y * CGROUPS + threadIdx.y) * FROWS;
+  if (d0 >= D || r0 >= T) return;
+  uint2 xq[FROWS + CW - 1];
+  int p[FROWS];
 #pragma unroll
-  for (int j = 1; j < W; ++j) {
-    if (r0 - j >= 0) {
-      unpack8(*reinterpret_cast<const uint4*>(x + (r0 - j) * ldx + d0), xwin[j]);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) xwin[j][c] = 0.f;
-    }
+  for (int i = 0; i < FROWS + CW - 1; ++i) {
+    const long long r = r0 + i - (CW - 1);
+    xq[i] = r >= 0 && r < T ? *reinterpret_cast<const uint2*>(x + r * ldx + d0) : make_uint2(0u, 0u);
   }
-  const long long u_end = r1 + (W - 1);
-  // Four rows per trip: their dpre / x / position loads are issued together before any of them is used, so a thread
-  // keeps eight 16-byte loads in flight instead of two (the walk is serial per thread and latency-bound otherwise).
-  for (long long ub = r0; ub < u_end; ub += 4) {
-    uint4 gq[4], xq[4];
-    int pq[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long long u = ub + i;
-      const bool in_t = u < T && u < u_end;
-      gq[i] = in_t ? *reinterpret_cast<const uint4*>(dpre + u * ldd + d0) : make_uint4(0, 0, 0, 0);
-      pq[i] = in_t ? pos[u] : -1;
-      xq[i] = u < r1 ? *reinterpret_cast<const uint4*>(x + u * ldx + d0) : make_uint4(0, 0, 0, 0);
-    }
+  for (int i = 0; i < FROWS; ++i) p[i] = r0 + i < T ? pos[r0 + i] : 0;
+  float wv[CW][4], bias[4];
+  load_taps(w, b, d0, wv, bias);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long long u = ub + i;
-      if (u >= u_end) break;
-      // shift the dpre / position windows and take row u (zero / invalid past the end of the tensor)
+  for (int i = 0; i < FROWS; ++i) {
+    if (r0 + i >= T) break;
+    float acc[4] = {bias[0], bias[1], bias[2], bias[3]};
 #pragma unroll
-      for (int j = W - 1; j >= 1; --j) {
+    for (int j = 0; j < CW; ++j) {
+      if (j <= p[i]) {
+        float xv[4];
+        unpack4(xq[i + CW - 1 - j], xv);
 #pragma unroll
-        for (int c = 0; c < 8; ++c) gwin[j][c] = gwin[j - 1][c];
-        pwin[j] = pwin[j - 1];
+        for (int c = 0; c < 4; ++c) acc[c] = fmaf(wv[j][c], xv[c], acc[c]);
       }
-      unpack8(gq[i], gwin[0]);
-      pwin[0] = pq[i];
-      if (u < r1) {
-        // weight / bias gradients of row u: dw[tap j] += dpre[u] * x[u - j]
-        unpack8(xq[i], xwin[0]);
+    }
 #pragma unroll
-        for (int c = 0; c < 8; ++c) db[c] += gwin[0][c];
+    for (int c = 0; c < 4; ++c)
+      if (SILU) acc[c] *= sigmoidf_(acc[c]);
+    *reinterpret_cast<uint2*>(y + (r0 + i) * ldy + d0) = pack4(acc);
+  }
+}
+
+// A block walks the tiles of 64 rows of its strip; dpre of the three rows behind a thread's own is recomputed (11 rows for 8).
+template <bool SILU>
+__global__ void __launch_bounds__(CLANES * CGROUPS, 2) conv4_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                                                                        const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
+                                                                        const int* __restrict__ pos, __nv_bfloat16* __restrict__ dx,
+                                                                        float* __restrict__ part, long long T, int D, long long ldx, long long ldy,
+                                                                        long long ldd, int tiles_per_strip) {
+  __shared__ float red[CGROUPS][CLANES * 4 * (CW + 1)];
+  const int d0 = (blockIdx.x * CLANES + threadIdx.x) * 4;
+  const bool live = d0 < D;
+  float wv[CW][4], bias[4], dw[CW][4], db[4];
+  if (live) load_taps(w, b, d0, wv, bias);
 #pragma unroll
-        for (int j = 0; j < W; ++j) {
-          if (j <= pwin[0]) {
+  for (int c = 0; c < 4; ++c) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) dw[j][c] = fmaf(gwin[0][c], xwin[j][c], dw[j][c]);
+    for (int j = 0; j < CW; ++j) dw[j][c] = 0.f;
+    db[c] = 0.f;
+  }
+  constexpr int H = CW - 1;
+  for (int tile = 0; tile < tiles_per_strip; ++tile) {
+    const long long r0 = (((long long)blockIdx.y * tiles_per_strip + tile) * CGROUPS + threadIdx.y) * BROWS;
+    if (!live || r0 >= T) break;
+    uint2 xq[BROWS + 2 * H], gq[BROWS + H];
+    int p[BROWS + H];
+#pragma unroll
+    for (int i = 0; i < BROWS + 2 * H; ++i) {
+      const long long r = r0 + i - H;
+      xq[i] = r >= 0 && r < T ? *reinterpret_cast<const uint2*>(x + r * ldx + d0) : make_uint2(0u, 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < BROWS + H; ++i) {
+      const bool in = r0 + i < T;
+      gq[i] = in ? *reinterpret_cast<const uint2*>(dy + (r0 + i) * ldy + d0) : make_uint2(0u, 0u);
+      p[i] = in ? pos[r0 + i] : -1;
+    }
+    float g[CW][4];  // dpre of the last four rows, g[0] the newest
+#pragma unroll
+    for (int i = 0; i < BROWS + H; ++i) {
+#pragma unroll
+      for (int j = CW - 1; j >= 1; --j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) g[j][c] = g[j - 1][c];
+      unpack4(gq[i], g[0]);
+      float xv[CW][4];
+#pragma unroll
+      for (int j = 0; j < CW; ++j) unpack4(xq[i + H - j], xv[j]);
+      if (SILU) {
+        float pre[4] = {bias[0], bias[1], bias[2], bias[3]};
+#pragma unroll
+        for (int j = 0; j < CW; ++j)
+          if (j <= p[i]) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) pre[c] = fmaf(wv[j][c], xv[j][c], pre[c]);
           }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float sg = sigmoidf_(pre[c]);
+          g[0][c] *= sg * (1.f + pre[c] * (1.f - sg));
         }
-#pragma unroll
-        for (int j = W - 1; j >= 1; --j)
-#pragma unroll
-          for (int c = 0; c < 8; ++c) xwin[j][c] = xwin[j - 1][c];
       }
-      // input gradient of row s = u - (W-1): dx[s] = sum_j w[tap j] dpre[s + j] while s + j stays in the same document
-      const long long srow = u - (W - 1);
-      if (srow >= r0) {
-        float acc[8];
+      if (i < BROWS) {  // the rows behind belong to other threads' sums
 #pragma unroll
-        for (int c = 0; c < 8; ++c) acc[c] = wv[0][c] * gwin[W - 1][c];
+        for (int c = 0; c < 4; ++c) db[c] += g[0][c];
+#pragma unroll
+        for (int j = 0; j < CW; ++j)
+          if (j <= p[i]) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) dw[j][c] = fmaf(g[0][c], xv[j][c], dw[j][c]);
+          }
+      }
+      if (i >= H && r0 + i - H < T) {  // dx[s] = sum_j w[tap j] dpre[s + j] while row s + j is at least j tokens into its document
+        float acc[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] = wv[0][c] * g[H][c];
         bool alive = true;
 #pragma unroll
-        for (int j = 1; j < W; ++j) {
-          alive = alive && (pwin[W - 1 - j] >= j);  // row s + j exists and is at least j tokens into the same document
+        for (int j = 1; j < CW; ++j) {
+          alive = alive && p[i - H + j] >= j;
           if (alive) {
 #pragma unroll
-            for (int c = 0; c < 8; ++c) acc[c] = fmaf(wv[j][c], gwin[W - 1 - j][c], acc[c]);
+            for (int c = 0; c < 4; ++c) acc[c] = fmaf(wv[j][c], g[H - j][c], acc[c]);
           }
         }
-        *reinterpret_cast<uint4*>(dx + srow * ldx + d0) = pack8(acc);
+        *reinterpret_cast<uint2*>(dx + (r0 + i - H) * ldd + d0) = pack4(acc);
       }
     }
   }
-  float* dst = part + ((long long)blockIdx.y * D + d0) * (W + 1);
+  float* mine = red[threadIdx.y] + threadIdx.x * 4 * (CW + 1);
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
+  for (int c = 0; c < 4; ++c) {
 #pragma unroll
-    for (int j = 0; j < W; ++j) dst[c * (W + 1) + (W - 1 - j)] = dw[j][c];
-    dst[c * (W + 1) + W] = db[c];
+    for (int j = 0; j < CW; ++j) mine[c * (CW + 1) + (CW - 1 - j)] = dw[j][c];
+    mine[c * (CW + 1) + CW] = db[c];
+  }
+  __syncthreads();
+  const int n = min(CLANES * 4, D - (int)blockIdx.x * CLANES * 4) * (CW + 1);
+  float* dst = part + ((long long)blockIdx.y * D + (long long)blockIdx.x * CLANES * 4) * (CW + 1);
+  for (int i = threadIdx.y * CLANES + threadIdx.x; i < n; i += CLANES * CGROUPS) {
+    float v = 0.f;
+#pragma unroll
+    for (int k = 0; k < CGROUPS; ++k) v += red[k][i];
+    dst[i] = v;
   }
 }
 
@@ -358,10 +435,9 @@ __global__ void conv_reduce_kernel(const float* __restrict__ part, int strips, i
 
 extern "C" {
 
-// 64-row strips: the backward walks a strip serially per thread, so the strip count is what gives it parallelism
-// (65,536 tokens x 1024 channels -> 1024 strips x 128 threads)
+// Strips of at least 64 rows, whose weight-gradient partials the reduction adds up: 65,536 tokens give 1024 strips.
 int fb_short_conv_strips(long long T) {
-  long long s = (T + 63) / 64;
+  long long s = (T + BTILE - 1) / BTILE;
   return (int)(s < 1 ? 1 : (s > 2048 ? 2048 : s));
 }
 
@@ -369,29 +445,46 @@ int fb_short_conv_fwd(const void* x, const void* w, const void* b, const int* po
                       long long ldx, long long ldy, int silu, cudaStream_t stream) {
   if (T == 0) return 0;
   if ((D % 8) || W > MAXW || (ldx % 8) || (ldy % 8)) return -2;
+  if (W == CW) {
+    if (((uintptr_t)w & 15) || ((uintptr_t)b & 7) || ((uintptr_t)x & 7)) return -2;
+    const dim3 grid((D / 4 + CLANES - 1) / CLANES, (unsigned)((T + FROWS * CGROUPS - 1) / (FROWS * CGROUPS))), block(CLANES, CGROUPS);
+    const __nv_bfloat16 *xx = (const __nv_bfloat16*)x, *ww = (const __nv_bfloat16*)w, *bb = (const __nv_bfloat16*)b;
+    if (grid.y > 65535) return -2;
+    if (silu) conv4_fwd_kernel<true><<<grid, block, 0, stream>>>(xx, ww, bb, pos, (__nv_bfloat16*)y, T, D, ldx, ldy);
+    else conv4_fwd_kernel<false><<<grid, block, 0, stream>>>(xx, ww, bb, pos, (__nv_bfloat16*)y, T, D, ldx, ldy);
+    return fb::launch_ok("conv4_fwd_kernel");
+  }
   return silu ? launch_conv_point<true, false>(x, w, b, pos, nullptr, y, T, D, W, ldx, ldy, stream)
               : launch_conv_point<false, false>(x, w, b, pos, nullptr, y, T, D, W, ldx, ldy, stream);
 }
 
-// dpre: bf16 [T, D] scratch; part: fp32 [fb_short_conv_strips(T), D, W + 1] scratch; dw: fp32 [D, W]; db: fp32 [D] or null
+// dx: bf16 [T, D], row stride ldd (= ldx unless W is 4); dpre: bf16 [T, D] scratch with dy's row stride, not used when W is 4;
+// part: fp32 [fb_short_conv_strips(T), D, W + 1] scratch; dw: fp32 [D, W]; db: fp32 [D] or null
 int fb_short_conv_bwd(const void* dy, const void* x, const void* w, const void* b, const int* pos, void* dx, void* dpre,
-                      float* part, float* dw, float* db, long long T, int D, int W, long long ldx, long long ldy, int silu,
+                      float* part, float* dw, float* db, long long T, int D, int W, long long ldx, long long ldy, long long ldd, int silu,
                       int accumulate, cudaStream_t stream) {
   if (T == 0) return 0;
-  if ((D % 8) || W > MAXW || (ldx % 8) || (ldy % 8)) return -2;
-  int rc = silu ? launch_conv_point<true, true>(x, w, b, pos, dy, dpre, T, D, W, ldx, ldy, stream)
-                : launch_conv_point<false, true>(x, w, b, pos, dy, dpre, T, D, W, ldx, ldy, stream);
-  if (rc) return rc;
-  const int strips = fb_short_conv_strips(T);
-  const int rows_per_strip = (int)((T + strips - 1) / strips);
-  dim3 grid((D / 8 + 63) / 64, strips);
-  if (W == 4)
-    conv_bwd_strip_kernel<4><<<grid, 64, 0, stream>>>((const __nv_bfloat16*)dpre, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-                                                      pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, rows_per_strip);
-  else
-    conv_bwd_kernel<<<grid, 64, 0, stream>>>((const __nv_bfloat16*)dpre, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w,
-                                             pos, (__nv_bfloat16*)dx, part, T, D, W, ldx, ldy, rows_per_strip);
-  rc = fb::launch_ok("conv_bwd_kernel");
+  if ((D % 8) || W > MAXW || (ldx % 8) || (ldy % 8) || (ldd % 8)) return -2;
+  int strips = fb_short_conv_strips(T), rc;
+  const __nv_bfloat16 *gg = (const __nv_bfloat16*)dy, *xx = (const __nv_bfloat16*)x, *ww = (const __nv_bfloat16*)w, *bb = (const __nv_bfloat16*)b;
+  if (W == CW) {
+    if (((uintptr_t)w & 15) || ((uintptr_t)b & 7) || ((uintptr_t)x & 7) || ((uintptr_t)dy & 7)) return -2;
+    const int tiles = (int)((T + BTILE - 1) / BTILE), per = (tiles + strips - 1) / strips;
+    strips = (tiles + per - 1) / per;
+    const dim3 grid((D / 4 + CLANES - 1) / CLANES, strips), block(CLANES, CGROUPS);
+    if (silu) conv4_bwd_kernel<true><<<grid, block, 0, stream>>>(gg, xx, ww, bb, pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, ldd, per);
+    else conv4_bwd_kernel<false><<<grid, block, 0, stream>>>(gg, xx, ww, bb, pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, ldd, per);
+    rc = fb::launch_ok("conv4_bwd_kernel");
+  } else {
+    if (ldd != ldx) return -2;
+    rc = silu ? launch_conv_point<true, true>(x, w, b, pos, dy, dpre, T, D, W, ldx, ldy, stream)
+              : launch_conv_point<false, true>(x, w, b, pos, dy, dpre, T, D, W, ldx, ldy, stream);
+    if (rc) return rc;
+    const int rows_per_strip = (int)((T + strips - 1) / strips);
+    conv_bwd_kernel<<<dim3((D / 8 + 63) / 64, strips), 64, 0, stream>>>((const __nv_bfloat16*)dpre, xx, ww, pos, (__nv_bfloat16*)dx, part, T, D,
+                                                                        W, ldx, ldy, rows_per_strip);
+    rc = fb::launch_ok("conv_bwd_kernel");
+  }
   if (rc) return rc;
   conv_reduce_kernel<<<(D * (W + 1) + 31) / 32, 256, 0, stream>>>(part, strips, D, W, dw, db, accumulate);
   return fb::launch_ok("conv_reduce_kernel");

@@ -469,7 +469,7 @@ class Mamba(nn.Module):
         from ..ops.scan import mamba_scan_gate
         Di, N, R = self.intermediate_size, self.ssm_state_size, self.time_step_rank
         h, z = split_columns(self.in_proj(x), (Di, Di))
-        h = self.conv1d(h.contiguous(), meta)
+        h = self.conv1d(h, meta)
         dt, B, C = split_columns(self.x_proj(h), (R, N, N))
         A = -torch.exp(self.A_log.float())
         y = mamba_scan_gate(h, self.dt_proj(dt.contiguous()), A, B, C, self.D, z, meta)
@@ -519,7 +519,7 @@ class Mamba2(nn.Module):
         zxbcdt = self.in_proj(x)
         # column blocks as views whose gradients are written side by side in one pass
         z, xBC, dt = gates.split_columns(zxbcdt, (Di, self.conv_dim, zxbcdt.shape[1] - Di - self.conv_dim))
-        xBC = self.conv1d(xBC.contiguous(), meta)
+        xBC = self.conv1d(xBC, meta)
         xs, B, C = gates.split_columns(xBC, (Di, G * N, G * N))
         if not (self.rmsnorm and self.norm_before_gate):
             # everything elementwise around the SSD core in two kernels: dt = softplus(dt + bias), the log decay and

@@ -17,7 +17,14 @@ from .varlen import VarlenMeta
 vp, i32, i64 = c_void_p, c_int, c_longlong
 _lib.register("fb_short_conv_strips", [i64])
 _lib.register("fb_short_conv_fwd", [vp, vp, vp, vp, vp, i64, i32, i32, i64, i64, i32, vp])
-_lib.register("fb_short_conv_bwd", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i64, i64, i32, i32, vp])
+_lib.register("fb_short_conv_bwd", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i64, i64, i64, i32, i32, vp])
+
+
+def _aligned(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """``t``, contiguous and on a 16-byte boundary (the kernels load it in vectors)."""
+    if t is None or (t.is_contiguous() and t.data_ptr() % 16 == 0):
+        return t
+    return t.clone(memory_format=torch.contiguous_format)
 
 
 class _ShortConvFn(torch.autograd.Function):
@@ -25,11 +32,12 @@ class _ShortConvFn(torch.autograd.Function):
     def forward(ctx, x, weight, bias, meta: VarlenMeta, silu: bool):
         T, D = x.shape
         W = weight.shape[-1]
-        x = x if (x.stride(1) == 1 and x.stride(0) % 8 == 0) else x.contiguous()
-        w2 = weight.reshape(D, W)
+        x = x if (x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0) else x.contiguous()
+        w2 = _aligned(weight.detach().reshape(D, W))
+        b2 = _aligned(bias.detach()) if bias is not None else None
         y = torch.empty(T, D, dtype=x.dtype, device=x.device)
         pos = meta.position_ids
-        rc = _lib.lib().fb_short_conv_fwd(x.data_ptr(), w2.data_ptr(), _lib.ptr(bias), pos.data_ptr(), y.data_ptr(), T, D,
+        rc = _lib.lib().fb_short_conv_fwd(x.data_ptr(), w2.data_ptr(), _lib.ptr(b2), pos.data_ptr(), y.data_ptr(), T, D,
                                           W, x.stride(0), y.stride(0), 1 if silu else 0, _lib.stream_ptr())
         _lib.check(rc, "fb_short_conv_fwd")
         _lib.count_launch()
@@ -43,10 +51,11 @@ class _ShortConvFn(torch.autograd.Function):
         T, D = x.shape
         W = weight.shape[-1]
         L = _lib.lib()
-        dy = dy if dy.is_contiguous() else dy.contiguous()
-        w2 = weight.reshape(D, W)
+        dy = _aligned(dy)
+        w2 = _aligned(weight.detach().reshape(D, W))
+        b2 = _aligned(bias.detach()) if bias is not None else None
         dx = torch.empty(T, D, dtype=x.dtype, device=x.device)
-        dpre = torch.empty(T, D, dtype=x.dtype, device=x.device)
+        dpre = torch.empty(T, D, dtype=x.dtype, device=x.device) if W != 4 else None
         strips = int(L.fb_short_conv_strips(T))
         part = torch.empty(strips, D, W + 1, dtype=torch.float32, device=x.device)
         mg_w = getattr(weight, "main_grad", None)
@@ -56,13 +65,14 @@ class _ShortConvFn(torch.autograd.Function):
         db = None
         if bias is not None:
             db = mg_b if use_main else torch.empty(D, dtype=torch.float32, device=x.device)
-        # dx is written with the row stride of x only when x is contiguous; keep both contiguous
-        xs = x if x.is_contiguous() else x.contiguous()
-        rc = L.fb_short_conv_bwd(dy.data_ptr(), xs.data_ptr(), w2.data_ptr(), _lib.ptr(bias), ctx.meta.position_ids.data_ptr(),
-                                 dx.data_ptr(), dpre.data_ptr(), part.data_ptr(), dw.data_ptr(), _lib.ptr(db), T, D, W,
-                                 xs.stride(0), dy.stride(0), 1 if ctx.silu else 0, 1 if use_main else 0, _lib.stream_ptr())
+        # the two-pass form of the other widths writes dx with the row stride of x
+        xs = x if W == 4 or x.is_contiguous() else x.contiguous()
+        rc = L.fb_short_conv_bwd(dy.data_ptr(), xs.data_ptr(), w2.data_ptr(), _lib.ptr(b2), ctx.meta.position_ids.data_ptr(),
+                                 dx.data_ptr(), _lib.ptr(dpre), part.data_ptr(), dw.data_ptr(), _lib.ptr(db), T, D, W,
+                                 xs.stride(0), dy.stride(0), dx.stride(0), 1 if ctx.silu else 0, 1 if use_main else 0,
+                                 _lib.stream_ptr())
         _lib.check(rc, "fb_short_conv_bwd")
-        _lib.count_launch(3)
+        _lib.count_launch(2 if W == 4 else 3)
         gw = None if use_main else dw.view_as(weight).to(weight.dtype)
         gb = None if (bias is None or use_main) else db.to(bias.dtype)
         return dx, gw, gb, None, None

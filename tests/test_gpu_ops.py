@@ -220,6 +220,34 @@ def test_rms_norm_every_row_length(D, rows, form):
         assert rel_err(a, b) < 5e-3
 
 
+@pytest.mark.parametrize("D,lens", [(8, [1]), (136, [2, 3, 1, 4]), (120, [7, 57, 1]), (264, [64, 63, 65, 130]), (128, [4500, 3])])
+@pytest.mark.parametrize("silu", [True, False])
+def test_short_conv_width_four_edges(D, lens, silu):
+    """Rows and channels around the block's tiles, documents shorter than the taps, a strided input, against fp64; bf16
+    results of up to four taps (2^-9 each way), weight gradients summed in fp32 and rounded to bf16: 5e-3."""
+    from flame_b200.ops.conv import short_conv
+    torch.manual_seed(9)
+    meta = _meta(lens)
+    T = sum(lens)
+    wide = torch.randn(T, 2 * D, device=DEV, dtype=torch.bfloat16).requires_grad_(True)
+    w = (torch.randn(D, 1, 4, device=DEV) * 0.5).to(torch.bfloat16).requires_grad_(True)
+    b = torch.randn(D, device=DEV).to(torch.bfloat16).requires_grad_(True)
+    dy = torch.randn(T, D, device=DEV, dtype=torch.bfloat16)
+    act = "silu" if silu else None
+    y = short_conv(wide[:, D:], w, b, meta, act)
+    out = [y] + list(torch.autograd.grad(y, [wide, w, b], dy))
+    f = [t.detach().double().requires_grad_(True) for t in (wide, w, b)]
+    x, pos = f[0][:, D:], meta.position_ids.long()
+    yr = f[2].expand(T, D)
+    for j in range(min(4, T)):
+        shifted = torch.cat([x.new_zeros(j, D), x[:T - j]])
+        yr = yr + torch.where((pos >= j)[:, None], shifted, torch.zeros_like(x)) * f[1][:, 0, 3 - j]
+    yr = torch.nn.functional.silu(yr) if silu else yr
+    ref = [yr] + list(torch.autograd.grad(yr, f, dy.double()))
+    for a, r in zip(out, ref):
+        assert rel_err(a, r) < 5e-3
+
+
 def test_fused_linear_cross_entropy_and_cross_entropy():
     from flame_b200.ops.cross_entropy import cross_entropy, fused_linear_cross_entropy
     torch.manual_seed(5)
