@@ -294,6 +294,91 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
   }
 }
 
+// The plain loss (no smoothing, scaling, capping or z-loss) of rows that fit the registers of their CTA: NV 16-byte vectors per
+// thread are loaded at once and stay packed, so a row is read from memory once, with the whole row in flight, and the maximum
+// needs no exponentials.  The walking form above reads the row again for the gradient and keeps one vector per thread in
+// flight: 0.384 ms for 12,289 rows of 32,000 (4.1 TB/s of one read and one write).
+template <int NV>
+__global__ void __launch_bounds__(CE_THREADS, 2)
+cross_entropy_row_kernel(__nv_bfloat16* __restrict__ logits, const long long* __restrict__ targets, float* __restrict__ loss_rows,
+                         float* __restrict__ lse_rows, const int* __restrict__ n_valid, float scale_num, int V, long long ld, int ignore_index,
+                         int write_grad) {
+  constexpr int W = CE_THREADS / 32;
+  __shared__ float s_max[W], s_sum[W];
+  const long long row = blockIdx.x;
+  uint4* lr = reinterpret_cast<uint4*>(logits + row * ld);
+  const long long tgt = targets[row];
+  const bool ignored = tgt == (long long)ignore_index;
+  const int nvec = V >> 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr uint32_t NEG = 0xff80ff80u;  // two bf16 -inf
+  uint4 x[NV];
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = threadIdx.x + k * CE_THREADS;
+    x[k] = i < nvec ? __ldcs(lr + i) : make_uint4(NEG, NEG, NEG, NEG);
+  }
+  float m = -INFINITY;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    float f[8];
+    unpack8(x[k], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = fmaxf(m, f[j]);
+  }
+  // keep the compiler from carrying unpacked values from one sweep to the next
+  auto repack = [&]() {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) asm volatile("" : "+r"(x[k].x), "+r"(x[k].y), "+r"(x[k].z), "+r"(x[k].w));
+  };
+  repack();
+  m = warp_max(m);
+  if (lane == 0) s_max[warp] = m;
+  // the target logit, read before anyone overwrites it (the barriers below)
+  float zt = 0.f;
+  if (threadIdx.x == 0 && !ignored) zt = __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(lr)[tgt]);
+  __syncthreads();
+  m = s_max[0];
+#pragma unroll
+  for (int w = 1; w < W; ++w) m = fmaxf(m, s_max[w]);
+  float s = 0.f;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    float f[8];
+    unpack8(x[k], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
+  }
+  repack();
+  s = warp_sum(s);
+  if (lane == 0) s_sum[warp] = s;
+  __syncthreads();
+  s = 0.f;
+#pragma unroll
+  for (int w = 0; w < W; ++w) s += s_sum[w];
+  if (threadIdx.x == 0) {
+    const float lse = m + __logf(s);
+    loss_rows[row] = ignored ? 0.f : lse - zt;
+    if (lse_rows) lse_rows[row] = lse;
+  }
+  if (!write_grad) return;
+  const float gs = ignored ? 0.f : scale_num / (float)max(*n_valid, 1);
+  const float inv = 1.f / s;
+#pragma unroll
+  for (int k = 0; k < NV; ++k) {
+    const int i = threadIdx.x + k * CE_THREADS;
+    if (i >= nvec) break;
+    float f[8];
+    unpack8(x[k], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float pr = __expf(f[j] - m) * inv;
+      if ((long long)(i * 8 + j) == tgt) pr -= 1.f;
+      f[j] = pr * gs;
+    }
+    lr[i] = pack8(f);
+  }
+}
+
 // ------------------------------------------------------------------------------------------------
 // Vocabulary-parallel cross-entropy (tensor parallelism): every rank holds a column slice of the logits.
 //   stats kernel : per row the slice's max, its sum of exp(x - max) and the target logit if the target falls in the slice
@@ -689,6 +774,18 @@ int fb_cross_entropy_opt(void* logits, const long long* targets, float* loss_row
   if (rows == 0) return 0;
   if ((ld % 8) || ((uintptr_t)logits & 15)) return -2;
   CeOptions opt = {label_smoothing, logit_scale, lse_square_scale, softcap};
+  // rows of whole vectors that two CTAs per SM can hold in registers; others (and the loss with options) walk the row
+  const bool plain = label_smoothing == 0.f && logit_scale == 1.f && lse_square_scale == 0.f && softcap <= 0.f;
+  if (plain && (V & 7) == 0 && V <= 8 * 8 * CE_THREADS) {
+#define CE_ROW(NV)                                                                                                            \
+  cross_entropy_row_kernel<NV><<<(unsigned)rows, CE_THREADS, 0, stream>>>((__nv_bfloat16*)logits, targets, loss_rows, lse_rows, \
+                                                                          n_valid, scale_num, V, ld, ignore_index, write_grad)
+    if (V <= 2 * 8 * CE_THREADS) CE_ROW(2);
+    else if (V <= 4 * 8 * CE_THREADS) CE_ROW(4);
+    else CE_ROW(8);
+#undef CE_ROW
+    return fb::launch_ok("cross_entropy_row_kernel");
+  }
   cross_entropy_kernel<<<(unsigned)rows, CE_THREADS, 0, stream>>>((__nv_bfloat16*)logits, targets, loss_rows, lse_rows,
                                                                   n_valid, scale_num, V, ld, ignore_index, write_grad, opt);
   return fb::launch_ok("cross_entropy_kernel");

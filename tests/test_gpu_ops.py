@@ -248,6 +248,29 @@ def test_short_conv_width_four_edges(D, lens, silu):
         assert rel_err(a, r) < 5e-3
 
 
+@pytest.mark.parametrize("V", [8, 1000, 8192, 8200, 16384, 16392, 32000, 32768, 32776])
+def test_cross_entropy_row_lengths(V):
+    """Vocabularies around what a CTA holds in registers (and beyond, where it walks the row); ignored rows, a row with -inf
+    entries, a large common offset; loss in fp32 (1e-5), gradients rounded to bf16 (2^-8)."""
+    from flame_b200.ops.cross_entropy import cross_entropy
+    torch.manual_seed(15)
+    rows = 9
+    base = (torch.randn(rows, V, device=DEV) * 3).to(torch.bfloat16)
+    base[3] += 200.0
+    base[4, ::2] = float("-inf")
+    lab = torch.randint(0, V, (rows,), device=DEV)
+    lab[1] = -100
+    lab[4] = lab[4] // 2 * 2 + 1
+    ref_in = base.double().requires_grad_(True)
+    ref = torch.nn.functional.cross_entropy(ref_in, lab)
+    (want,) = torch.autograd.grad(ref, ref_in)
+    leaf = base.clone().requires_grad_(True)
+    loss = cross_entropy(leaf * 1.0, lab)
+    (got,) = torch.autograd.grad(loss, leaf)
+    assert abs(loss.item() - ref.item()) < 1e-5 * abs(ref.item()) + 1e-6
+    assert rel_err(got, want) < 4e-3
+
+
 def test_fused_linear_cross_entropy_and_cross_entropy():
     from flame_b200.ops.cross_entropy import cross_entropy, fused_linear_cross_entropy
     torch.manual_seed(5)
