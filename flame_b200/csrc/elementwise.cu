@@ -525,19 +525,27 @@ __global__ void embedding_fwd_kernel(const long long* __restrict__ ids, const __
   if (id >= 0 && id < V) q = reinterpret_cast<const uint4*>(table + id * D)[v];
   reinterpret_cast<uint4*>(out + t * D)[v] = q;
 }
-// Deterministic scatter-add: tokens are pre-sorted by id (perm), seg_start marks runs of equal ids.
-// One warp per unique id sums its rows in sorted order and adds them to the fp32 gradient row.
-__global__ void embedding_bwd_sorted_kernel(const long long* __restrict__ sorted_ids,
-                                            const long long* __restrict__ perm, const int* __restrict__ seg_start,
-                                            int nseg, long long T, const __nv_bfloat16* __restrict__ dout,
-                                            float* __restrict__ dtable, int D, long long V) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// Deterministic scatter-add: tokens are pre-sorted by id (perm); an id's rows are summed in that order and added to the fp32
+// gradient row.
+// One warp per sorted position; the one that stands on the first occurrence of an id adds up that id's rows, in sorted order.
+// (Finding the first occurrences on the host's side of the stream cost a synchronisation in the middle of every backward.)
+__global__ void embedding_bwd_sorted_kernel(const long long* __restrict__ sorted_ids, const long long* __restrict__ perm, long long T,
+                                            const __nv_bfloat16* __restrict__ dout, float* __restrict__ dtable, int D, long long V) {
+  const long long b = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  if (warp >= nseg) return;
-  const long long b = seg_start[warp];
-  const long long e = (warp + 1 < nseg) ? (long long)seg_start[warp + 1] : T;
+  if (b >= T) return;
   const long long id = sorted_ids[b];
-  if (id < 0 || id >= V) return;
+  if (id < 0 || id >= V || (b > 0 && sorted_ids[b - 1] == id)) return;
+  long long e = b + 1;
+  while (true) {  // 32 positions at a time
+    const bool same = e + lane < T && sorted_ids[e + lane] == id;
+    const unsigned m = __ballot_sync(0xffffffffu, same);
+    if (m != 0xffffffffu) {
+      e += __ffs(~m) - 1;
+      break;
+    }
+    e += 32;
+  }
   const int vec = D >> 3;
   for (int v = lane; v < vec; v += 32) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -827,12 +835,11 @@ int fb_embedding_fwd(const long long* ids, const void* table, void* out, long lo
                                                                         (__nv_bfloat16*)out, T, D, V);
   return fb::launch_ok("embedding_fwd_kernel");
 }
-int fb_embedding_bwd_sorted(const long long* sorted_ids, const long long* perm, const int* seg_start, int nseg,
-                            long long T, const void* dout, float* dtable, int D, long long V, cudaStream_t stream) {
-  if (nseg == 0) return 0;
+int fb_embedding_bwd_sorted(const long long* sorted_ids, const long long* perm, long long T, const void* dout, float* dtable, int D,
+                            long long V, cudaStream_t stream) {
+  if (T == 0) return 0;
   if (D % 8) return -2;
-  embedding_bwd_sorted_kernel<<<blocks_for((long long)nseg * 32, 256), 256, 0, stream>>>(
-      sorted_ids, perm, seg_start, nseg, T, (const __nv_bfloat16*)dout, dtable, D, V);
+  embedding_bwd_sorted_kernel<<<(unsigned)((T * 32 + 255) / 256), 256, 0, stream>>>(sorted_ids, perm, T, (const __nv_bfloat16*)dout, dtable, D, V);
   return fb::launch_ok("embedding_bwd_sorted_kernel");
 }
 

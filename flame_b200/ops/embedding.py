@@ -15,7 +15,7 @@ from . import _lib
 
 vp, i32, i64 = c_void_p, c_int, c_longlong
 _lib.register("fb_embedding_fwd", [vp, vp, vp, i64, i32, i64, vp])
-_lib.register("fb_embedding_bwd_sorted", [vp, vp, vp, i32, i64, vp, vp, i32, i64, vp])
+_lib.register("fb_embedding_bwd_sorted", [vp, vp, i64, vp, vp, i32, i64, vp])
 
 
 class _EmbeddingFn(torch.autograd.Function):
@@ -40,14 +40,10 @@ class _EmbeddingFn(torch.autograd.Function):
         d2 = dout.reshape(T, D)
         d2 = d2 if d2.is_contiguous() else d2.contiguous()
         sorted_ids, perm = torch.sort(flat, stable=True)
-        is_start = torch.ones(T, dtype=torch.bool, device=flat.device)
-        is_start[1:] = sorted_ids[1:] != sorted_ids[:-1]
-        seg_start = torch.nonzero(is_start).flatten().to(torch.int32)
-        nseg = seg_start.numel()
         mg = getattr(weight, "main_grad", None)
         dtable = mg if mg is not None else torch.zeros(V, D, dtype=torch.float32, device=weight.device)
-        rc = _lib.lib().fb_embedding_bwd_sorted(sorted_ids.data_ptr(), perm.data_ptr(), seg_start.data_ptr(), nseg, T,
-                                                d2.data_ptr(), dtable.data_ptr(), D, V, _lib.stream_ptr())
+        rc = _lib.lib().fb_embedding_bwd_sorted(sorted_ids.data_ptr(), perm.data_ptr(), T, d2.data_ptr(), dtable.data_ptr(),
+                                                D, V, _lib.stream_ptr())
         _lib.check(rc, "fb_embedding_bwd_sorted")
         _lib.count_launch()
         return None, (None if mg is not None else dtable.to(weight.dtype))

@@ -271,6 +271,23 @@ def test_cross_entropy_row_lengths(V):
     assert rel_err(got, want) < 4e-3
 
 
+def test_embedding_backward_runs_of_ids():
+    """Runs of one id longer than a warp, ids outside the table (another rank's vocabulary slice), against index_add in fp64."""
+    from flame_b200.ops.embedding import embedding
+    torch.manual_seed(16)
+    V, D = 50, 136
+    ids = torch.cat([torch.full((100,), 7), torch.randint(0, V, (333,)), torch.full((64,), 49), torch.tensor([-3, V, V + 9, 0])]).to(DEV)
+    ids = ids[torch.randperm(ids.numel(), device=DEV)]
+    w = torch.randn(V, D, device=DEV, dtype=torch.bfloat16).requires_grad_(True)
+    y = embedding(ids, w)
+    dy = torch.randn_like(y)
+    (dw,) = torch.autograd.grad(y, w, dy)
+    keep = (ids >= 0) & (ids < V)
+    ref = torch.zeros(V, D, device=DEV, dtype=torch.float64).index_add_(0, ids[keep], dy[keep].double())
+    assert rel_err(dw, ref) < 4e-3
+    assert torch.equal(y[~keep], torch.zeros_like(y[~keep]))
+
+
 def test_fused_linear_cross_entropy_and_cross_entropy():
     from flame_b200.ops.cross_entropy import cross_entropy, fused_linear_cross_entropy
     torch.manual_seed(5)
