@@ -25,8 +25,16 @@ class KernelError(RuntimeError):
     pass
 
 
+_CUDA_SEEN = False
+
+
 def cuda_present() -> bool:
-    return torch.cuda.is_available()
+    """Whether there is a CUDA device; a device once seen does not go away, so the driver is not asked again (every op asks
+    this several times)."""
+    global _CUDA_SEEN
+    if not _CUDA_SEEN:
+        _CUDA_SEEN = torch.cuda.is_available()
+    return _CUDA_SEEN
 
 
 def available() -> bool:
@@ -60,7 +68,8 @@ def reset_launches() -> None:
 
 
 def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    # the raw handle: a Stream object per launch costs more than the launch's own arguments
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def ptr(t: Optional[torch.Tensor]) -> int:
