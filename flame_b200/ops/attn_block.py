@@ -12,8 +12,7 @@ from typing import Optional, Tuple
 
 import torch
 
-from . import _lib
-from .attention import _AttnFn, _kernel_ok, attention_reference
+from . import _lib, attention as _attention, sac  # noqa: F401 - attention declares the kernels' signatures
 from .rope import rope_from_fp32_, rope_inplace_, rope_reference
 from .varlen import VarlenMeta
 
@@ -107,7 +106,9 @@ def qkv_attention(qkv: torch.Tensor, meta: VarlenMeta, H: int, Hkv: int, Dh: int
             else:
                 q, k = rope_reference(q, pos, cos, sin), rope_reference(k, pos, cos, sin)
         return sequence_parallel_attention(q, k, v, sl, scale, window or 0).reshape(T, H * Dh)
-    if _lib.available() and qkv.is_cuda and qkv.dtype == torch.bfloat16 and Dh == 64:
+    # head dim 128 under operator-level selective checkpointing goes through ``attention``, which keeps its output on the tape
+    if (_lib.available() and qkv.is_cuda and qkv.dtype == torch.bfloat16
+            and (Dh == 64 or (Dh == 128 and (sac.current() is None or not torch.is_grad_enabled())))):
         return _QkvAttnFn.apply(qkv, meta, H, Hkv, Dh, cos, sin, scale, window or 0)
     q = qkv[:, : H * Dh].reshape(T, H, Dh)
     k = qkv[:, H * Dh: (H + Hkv) * Dh].reshape(T, Hkv, Dh)

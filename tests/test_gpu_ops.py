@@ -288,6 +288,29 @@ def test_embedding_backward_runs_of_ids():
     assert torch.equal(y[~keep], torch.zeros_like(y[~keep]))
 
 
+@pytest.mark.parametrize("H,Hkv,window", [(3, 3, 0), (4, 2, 100)])
+def test_fused_qkv_attention_head_dim_128(H, Hkv, window):
+    """Rotary attention of head dim 128 on the fused projection buffer against the definition on its slices, in fp32; ragged
+    documents (bf16 operands: 2e-2)."""
+    from flame_b200.ops.attention import attention_reference
+    from flame_b200.ops.attn_block import qkv_attention
+    from flame_b200.ops.rope import rope_reference, rope_tables
+    torch.manual_seed(17)
+    meta = _meta([300, 1, 77])
+    T, Dh = 378, 128
+    qkv = torch.randn(T, (H + 2 * Hkv) * Dh, device=DEV, dtype=torch.bfloat16).requires_grad_(True)
+    rope = rope_tables(Dh, 512, 10000.0, torch.device(DEV))
+    do = torch.randn(T, H * Dh, device=DEV, dtype=torch.bfloat16)
+    o = qkv_attention(qkv * 1.0, meta, H, Hkv, Dh, rope=rope, window=window)   # the node rotates its input in place
+    (got,) = torch.autograd.grad(o, qkv, do)
+    f = qkv.detach().float().requires_grad_(True)
+    q, k, v = f[:, :H * Dh].view(T, H, Dh), f[:, H * Dh:(H + Hkv) * Dh].view(T, Hkv, Dh), f[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
+    q, k = rope_reference(q, meta.position_ids, *rope), rope_reference(k, meta.position_ids, *rope)
+    ref = attention_reference(q, k, v, meta, Dh ** -0.5, window).reshape(T, H * Dh)
+    (want,) = torch.autograd.grad(ref, f, do.float())
+    assert rel_err(o, ref) < 2e-2 and rel_err(got, want) < 2e-2
+
+
 def test_fused_linear_cross_entropy_and_cross_entropy():
     from flame_b200.ops.cross_entropy import cross_entropy, fused_linear_cross_entropy
     torch.manual_seed(5)
