@@ -16,6 +16,7 @@
 // works on the transposed score tile (see attn_bwd128_kernel).
 //
 // Takes the place of flash_attn_varlen_func as called by fla/layers/attn.py:146-174.
+#include "sb_math.cuh"
 #include "tc05.cuh"
 #include "host_utils.cuh"
 #include <math.h>
@@ -271,17 +272,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tmem_ld_wait();
 #pragma unroll
           for (int c = 24; c >= 0; c -= 8) {
-            float e[8];
-#pragma unroll
-            for (int i = 7; i >= 0; --i) {
-              const bool dead = diag && (kv0 + c0 + c + i >= q_idx);
-              float x = __uint_as_float(xr[c + i]) * p.scale_log2;
-              x = fminf(fmaxf(x, -100.f), 100.f);
-              const float t = fast_exp2(x);
-              const float inv = __frcp_rn(1.f + t);
-              e[i] = dead ? 0.f : t * inv * E;
-              E = dead ? E : E * inv;
-            }
+            float e[8], sig[8];
+            if (diag) sb_group<true>(xr + c, p.scale_log2, sb_dead_bits(false, true, kv0 + c0 + c, q_idx), E, sig, e);
+            else sb_group<false>(xr + c, p.scale_log2, 0u, E, sig, e);
             uint4 q;
             q.x = pack_bf16(e[0], e[1]);
             q.y = pack_bf16(e[2], e[3]);

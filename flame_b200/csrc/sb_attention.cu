@@ -10,8 +10,11 @@
 // Tot_i - R with Tot_i = do_i . o_i - drem_i (1 - rem_i), known up front.  Per key tile the tensor core forms S and dP,
 // one thread per query row turns them into P = att and dS = dl (bf16, swizzled smem), and three more MMAs produce the
 // tile's dV, dK (fresh each tile, added to fp32 accumulators in global memory by TMA reduce) and dQ (accumulated in
-// TMEM across the whole walk, no atomics).  The reference reaches the same sums with spin-locked adds
+// TMEM across the whole walk, no atomics).  Warps: TMA, MMA, four that form P and dS, four that move dV and dK out, so that
+// the move of one tile (two trips through a staging tile, about as long as the weights' own arithmetic) overlaps the next
+// tile's weights; one group of four did both in turn (12.4 us per tile, 5.7 ms for 8 x 4,096 tokens and 16 heads).  The reference reaches the same sums with spin-locked adds
 // (custom_models/sba/stickbreaking_attention/sb_varlen/sb_varlen_bwd.py:13-52); here nothing spins unbounded.
+#include "sb_math.cuh"
 #include "tc05.cuh"
 #include "host_utils.cuh"
 #include <math.h>
@@ -63,7 +66,9 @@ struct Smem {
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-__global__ void __launch_bounds__(192, 1)
+constexpr int SB_THREADS = 320;
+
+__global__ void __launch_bounds__(SB_THREADS, 1)
 sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                    const __grid_constant__ CUtensorMap tmdK, const __grid_constant__ CUtensorMap tmdV, SbBwdParams p) {
@@ -89,7 +94,8 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* dkv_full = pds_ready + 1;
   uint64_t* dkv_free = dkv_full + 1;
   uint64_t* grp_bar = dkv_free + 1;
-  uint32_t* tmem_slot = (uint32_t*)(grp_bar + 1);
+  uint64_t* dq_full = grp_bar + 1;
+  uint32_t* tmem_slot = (uint32_t*)(dq_full + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -104,6 +110,7 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(dkv_full, 1);
     mbar_init(dkv_free, 128);
     mbar_init(grp_bar, 128);
+    mbar_init(dq_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmQ);
@@ -193,26 +200,108 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         }
         mma_commit(&empty_bar[stage]);
         mma_commit(dkv_full);
+        if (it + 1 == n_iter) mma_commit(dq_full);
         if (it + 1 < n_iter) {
           if (!issue_sdp(it + 1)) { ok = false; break; }
         }
       }
     }
-  } else {
+  } else if (warp < 6) {
+    // ------------------------------------------------------------------ weights: one thread per query row
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
     const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
     uint8_t* sP = smem + L::P_OFF;
     uint8_t* sDS = smem + L::DS_OFF;
-    uint8_t* sSTG = smem + L::STG_OFF;
-    const bool issuer = (warp == 2 && lane == 0);
     const int q_idx = q0 + r;
     const bool valid = q_idx < doc_len;
+    const bool ragged = q0 + BQ > doc_len;
     const long long tok = (long long)doc_start + q_idx;
     const float tot = valid ? p.tot[(long long)head * p.total_tokens + tok] : 0.f;
     const float drem = (valid && p.drem != nullptr) ? p.drem[(long long)head * p.total_tokens + tok] : 0.f;
     float E = 1.f;  // product of (1 - sigma) over the keys already seen
     float R = 0.f;  // sum of dA over the keys already seen
+    bool ok = true;
+    for (int it = 0; it < n_iter && ok; ++it) {
+      const int j = ti - it;
+      const int kv0 = j * BKV;
+      const bool diag = (it == 0);
+      // the commit behind this barrier also covers the previous tile's products: P and dS may be overwritten
+      if (!mbar_wait_warp(sdp_full, it & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+      tc_fence_after();
+#pragma unroll 1
+      for (int c0 = BKV - 32; c0 >= 0; c0 -= 32) {
+        uint32_t xr[32], dr[32];
+        tmem_ld_32x32(tmem_S + lane_sel + c0, xr);
+        tmem_ld_32x32(tmem_dP + lane_sel + c0, dr);
+        tmem_ld_wait();
+#pragma unroll
+        for (int c = 24; c >= 0; c -= 8) {
+          float sig[8], a[8], d[8];
+          uint32_t dead = 0u;
+          if (diag || ragged) {
+            dead = sb_dead_bits(!valid, diag, kv0 + c0 + c, q_idx);
+            sb_group<true>(xr + c, p.scale_log2, dead, E, sig, a);
+#pragma unroll
+            for (int i = 0; i < 8; ++i)  // what stands in another document's rows does not count, whatever it is
+              if ((dead >> i) & 1u) dr[c + i] = 0u;
+          }
+          else sb_group<false>(xr + c, p.scale_log2, 0u, E, sig, a);
+          uint4 q;
+          q.x = pack_bf16(a[0], a[1]); q.y = pack_bf16(a[2], a[3]); q.z = pack_bf16(a[4], a[5]); q.w = pack_bf16(a[6], a[7]);
+          // The forward formed o from the bf16 rounding of att, and tot = do . o is the total the running sum R has to
+          // meet exactly at the end of the walk: the same rounded weight enters dA here (the remainder term keeps the
+          // fp32 weight, as rem was formed from it).  With fp32 att in this place the mismatch of the two roundings,
+          // multiplied by sigma for every key of the row, was a 20 % error in dq at 4096-token rows.
+          const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int i = 7; i >= 0; --i) {
+            const float att16 = __uint_as_float((i & 1) ? (qw[i >> 1] & 0xffff0000u) : (qw[i >> 1] << 16));
+            const float dA = att16 * __uint_as_float(dr[c + i]) - a[i] * drem;  // zero for keys that do not count
+            d[i] = dA - sig[i] * (tot - R);
+            R += dA;
+          }
+          const int cc = c0 + c;
+          const uint32_t off = (cc >> 6) * (BQ * 128) + sw128_offset(r, cc & 63);
+          *reinterpret_cast<uint4*>(sP + off) = q;
+          q.x = pack_bf16(d[0], d[1]); q.y = pack_bf16(d[2], d[3]); q.z = pack_bf16(d[4], d[5]); q.w = pack_bf16(d[6], d[7]);
+          *reinterpret_cast<uint4*>(sDS + off) = q;
+        }
+      }
+      tc_fence_before();
+      fence_async_smem();
+      mbar_arrive(pds_ready);
+    }
+    if (ok) ok = mbar_wait_warp(dq_full, 0, p.status, abort_flag, ERR_WAIT_TMEM_FULL);
+    if (ok) {
+      // dQ of this query tile
+      tc_fence_after();
+      __nv_bfloat16* dqrow = p.dQ + tok * p.dq_stride_t + (long long)head * DH;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t v[32];
+        tmem_ld_32x32(tmem_dQ + lane_sel + half * 32, v);
+        tmem_ld_wait();
+        if (valid) {
+#pragma unroll
+          for (int g = 0; g < 4; ++g) {
+            uint4 q;
+            q.x = pack_bf16(__uint_as_float(v[g * 8 + 0]) * p.scale, __uint_as_float(v[g * 8 + 1]) * p.scale);
+            q.y = pack_bf16(__uint_as_float(v[g * 8 + 2]) * p.scale, __uint_as_float(v[g * 8 + 3]) * p.scale);
+            q.z = pack_bf16(__uint_as_float(v[g * 8 + 4]) * p.scale, __uint_as_float(v[g * 8 + 5]) * p.scale);
+            q.w = pack_bf16(__uint_as_float(v[g * 8 + 6]) * p.scale, __uint_as_float(v[g * 8 + 7]) * p.scale);
+            *reinterpret_cast<uint4*>(dqrow + half * 32 + g * 8) = q;
+          }
+        }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ dV and dK of every tile
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;
+    const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
+    uint8_t* sSTG = smem + L::STG_OFF;
+    const bool issuer = (warp == 6 && lane == 0);
     bool ok = true;
     uint32_t grp_phase = 0;
     auto group_sync = [&]() -> bool {
@@ -247,53 +336,7 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       return true;
     };
     for (int it = 0; it < n_iter && ok; ++it) {
-      const int j = ti - it;
-      const int kv0 = j * BKV;
-      const bool diag = (it == 0);
-      if (!mbar_wait_warp(sdp_full, it & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
-      tc_fence_after();
-#pragma unroll 1
-      for (int c0 = BKV - 32; c0 >= 0; c0 -= 32) {
-        uint32_t xr[32], dr[32];
-        tmem_ld_32x32(tmem_S + lane_sel + c0, xr);
-        tmem_ld_32x32(tmem_dP + lane_sel + c0, dr);
-        tmem_ld_wait();
-#pragma unroll
-        for (int c = 24; c >= 0; c -= 8) {
-          float a[8], d[8];
-#pragma unroll
-          for (int i = 7; i >= 0; --i) {
-            const bool dead = !valid || (diag && (kv0 + c0 + c + i >= q_idx));
-            float x = __uint_as_float(xr[c + i]) * p.scale_log2;
-            x = fminf(fmaxf(x, -100.f), 100.f);
-            const float t = exp2f(x);
-            const float inv = __frcp_rn(1.f + t);
-            const float sig = t * inv;
-            const float att = dead ? 0.f : sig * E;
-            // The forward formed o from the bf16 rounding of att, and tot = do . o is the total the running sum R has to
-            // meet exactly at the end of the walk: the same rounded weight enters dA here (the remainder term keeps the
-            // fp32 weight, as rem was formed from it).  With fp32 att in this place the mismatch of the two roundings,
-            // multiplied by sigma for every key of the row, was a 20 % error in dq at 4096-token rows.
-            const float att16 = __bfloat162float(__float2bfloat16(att));
-            const float dA = att16 * __uint_as_float(dr[c + i]) - att * drem;
-            a[i] = att;
-            d[i] = dead ? 0.f : dA - sig * (tot - R);
-            R += dA;
-            E = dead ? E : E * inv;
-          }
-          const int cc = c0 + c;
-          const uint32_t off = (cc >> 6) * (BQ * 128) + sw128_offset(r, cc & 63);
-          uint4 q;
-          q.x = pack_bf16(a[0], a[1]); q.y = pack_bf16(a[2], a[3]); q.z = pack_bf16(a[4], a[5]); q.w = pack_bf16(a[6], a[7]);
-          *reinterpret_cast<uint4*>(sP + off) = q;
-          q.x = pack_bf16(d[0], d[1]); q.y = pack_bf16(d[2], d[3]); q.z = pack_bf16(d[4], d[5]); q.w = pack_bf16(d[6], d[7]);
-          *reinterpret_cast<uint4*>(sDS + off) = q;
-        }
-      }
-      tc_fence_before();
-      fence_async_smem();
-      mbar_arrive(pds_ready);
-      // this tile's dV and dK: wait for the MMAs, move them out through the staging tile, release TMEM
+      const int kv0 = (ti - it) * BKV;
       if (!mbar_wait_warp(dkv_full, it & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       if (!flush_tile(tmem_dV, &tmdV, 1.f, doc_start + kv0)) { ok = false; break; }
@@ -301,29 +344,7 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       tc_fence_before();
       mbar_arrive(dkv_free);
     }
-    if (ok) {
-      // dQ of this query tile: all MMAs are complete (dkv_full of the last tile covered them)
-      tc_fence_after();
-      __nv_bfloat16* dqrow = p.dQ + tok * p.dq_stride_t + (long long)head * DH;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t v[32];
-        tmem_ld_32x32(tmem_dQ + lane_sel + half * 32, v);
-        tmem_ld_wait();
-        if (valid) {
-#pragma unroll
-          for (int g = 0; g < 4; ++g) {
-            uint4 q;
-            q.x = pack_bf16(__uint_as_float(v[g * 8 + 0]) * p.scale, __uint_as_float(v[g * 8 + 1]) * p.scale);
-            q.y = pack_bf16(__uint_as_float(v[g * 8 + 2]) * p.scale, __uint_as_float(v[g * 8 + 3]) * p.scale);
-            q.z = pack_bf16(__uint_as_float(v[g * 8 + 4]) * p.scale, __uint_as_float(v[g * 8 + 5]) * p.scale);
-            q.w = pack_bf16(__uint_as_float(v[g * 8 + 6]) * p.scale, __uint_as_float(v[g * 8 + 7]) * p.scale);
-            *reinterpret_cast<uint4*>(dqrow + half * 32 + g * 8) = q;
-          }
-        }
-      }
-      if (issuer) tma_store_wait_all<0>();
-    }
+    if (issuer) tma_store_wait_all<0>();
   }
   tc_fence_before();
   __syncthreads();
@@ -431,7 +452,7 @@ int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
     done = true;
   }
   dim3 grid(max_tiles, H);
-  sb_attn_bwd_kernel<<<grid, 192, Smem::TOTAL, stream>>>(tmQ, tmK, tmV, tmdO, tmdK, tmdV, p);
+  sb_attn_bwd_kernel<<<grid, SB_THREADS, Smem::TOTAL, stream>>>(tmQ, tmK, tmV, tmdO, tmdK, tmdV, p);
   return fb::launch_ok("sb_attn_bwd_kernel");
 }
 

@@ -92,19 +92,20 @@ class StickBreakingAttention(nn.Module):
         self.o_proj = Linear(hidden_size, hidden_size)
 
     def forward(self, x: torch.Tensor, meta: VarlenMeta) -> torch.Tensor:
-        from ..ops.stickbreaking import sb_attention
+        from ..ops.stickbreaking import sb_attention, sb_qkv_attention
         T = x.shape[0]
         H, Hkv, Dh = self.num_heads, self.num_kv_heads, self.head_dim
         if self.q_proj.bias is None:
             qkv = fused_projection(x, (self.q_proj, self.k_proj, self.v_proj))
         else:
             qkv = torch.cat([self.q_proj(x), self.k_proj(x), self.v_proj(x)], -1)
+        if Hkv == H:
+            return self.o_proj(sb_qkv_attention(qkv, meta, H, Dh).reshape(T, H * Dh))
         q = qkv[:, : H * Dh].view(T, H, Dh)  # strided views of the fused projection output
         k = qkv[:, H * Dh: (H + Hkv) * Dh].view(T, Hkv, Dh)
         v = qkv[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
-        if Hkv != H:
-            k = k.repeat_interleave(H // Hkv, 1)
-            v = v.repeat_interleave(H // Hkv, 1)
+        k = k.repeat_interleave(H // Hkv, 1)
+        v = v.repeat_interleave(H // Hkv, 1)
         o, _ = sb_attention(q, k, v, meta)
         return self.o_proj(o.reshape(T, H * Dh))
 
