@@ -1,22 +1,22 @@
 // Batched bf16 GEMM for the chunk-parallel token mixers (linear attention, delta rule, SSD):
 //
-//   C[b] = epilogue( alpha * A[b] * B[b]^T )      b = (hi, lo) = (chunk, head)
+//   C[b] = epilogue( alpha * sum_i (+-) A_i[b] * B_i[b]^T )      b = (hi, lo) = (chunk, head), up to six products i
 //
 // Thousands of small problems (64 x 64 x dk score blocks, dk x dv chunk states, 64 x dv outputs) run as ONE persistent
 // launch: every operand is a 4-D tensor map (inner, row, lo, hi), so a tile of any batch is a TMA box and the batch
 // coordinates come from the work-unit index (optionally through an index table, which is how the chunk-by-chunk state
 // recurrence of documents with different lengths addresses "chunk s of every document that has one").  The main loop is
-// the single-CTA tcgen05 pipeline of gemm.cu (TMA warp, MMA warp, four epilogue warps, two TMEM accumulators); the
+// the single-CTA tcgen05 pipeline of gemm.cu (TMA warp, MMA warp, epilogue warps, two or four TMEM accumulators); the
+// several products of one result (the state's and the scores' share of an output, the terms of a gradient) accumulate in
+// tensor memory one after the other, so that no partial result is written and read back.  The
 // epilogue adds what the chunk algorithms need so no elementwise pass follows the GEMM:
 //   * causal masks (keep col <= row, or col < row),
-//   * a decay factor exp(d[row] - d[col]) from a per-batch fp32 vector (scalar-gated attention scores),
+//   * a decay factor exp(d[row] - d[col]) from a per-batch fp32 vector (scalar-gated attention scores), a factor per row,
 //   * the state step   C = alpha * acc + gamma[b] * Cin[b'] + add16[b''] (+ C)   with a bf16 copy of the result written
 //     to a batch of its own (C may be its own Cin: an fp32 state updated in place, small enough to stay in L2).
 //
 // Stands in for the tl.dot bodies of the reference's Triton chunk kernels (fla/ops/common/chunk_h.py,
 // fla/ops/common/chunk_o.py, fla/ops/gated_delta_rule/wy_fast.py, fla/ops/common/chunk_scaled_dot_kkt.py).
-#include <stdlib.h>
-
 #include "tc05.cuh"
 #include "host_utils.cuh"
 
@@ -26,12 +26,17 @@ namespace {
 
 constexpr int BM = 128;
 constexpr int BK = 64;
-constexpr int STAGES = 4;
-constexpr int MAX_BN = 256;
+constexpr int MAX_STAGES = 8;
 // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue: two warps per TMEM lane quarter, each taking half of the tile's columns.
 // The chunk algorithms' problems mostly have 64 rows, which live in two lane quarters only; with one warp per quarter
 // two warps would drain every accumulator and the epilogue, not memory, would set the pace.
 constexpr int BGEMM_THREADS = 320;
+// A work unit of the chunk algorithms is one to four K blocks, so a CTA spends its time in hand-offs and in the epilogue's
+// round trips to memory (one unit took about 1,500 clocks, whatever its size): tiles of at most 128 columns leave room for
+// two CTAs per SM (half of tensor memory and of shared memory each), whose epilogues overlap.
+constexpr int MAX_BN = 128;
+constexpr int TMEM_COLS = 256;
+constexpr int RING_BYTES = 96 * 1024;
 
 struct BOperandIdx {
   const int* hi_index;  // optional: hi coordinate = hi_index[hi_raw]
@@ -39,11 +44,25 @@ struct BOperandIdx {
   int lo_div;           // lo coordinate = lo / lo_div (grouped value heads)
 };
 
+constexpr int MAX_PAIRS = 6;
+
+struct BPair {
+  BOperandIdx a, b;
+  int num_kb, a_mn, b_mn, neg;
+};
+
+struct BMaps {
+  CUtensorMap a[MAX_PAIRS], b[MAX_PAIRS];
+};
+
 struct BGemmParams {
-  int M, N, K;
-  int tiles_m, tiles_n, num_kb, bn;
+  int M, N;
+  int tiles_m, tiles_n, n_pairs, bn;
+  int sum_lo;          // every product is summed over this many lo coordinates (the heads of a group): lo * sum_lo + 0, 1, ..
+  BPair pair[MAX_PAIRS];
+  int a_rows, stages;  // rows of the A box (64 when M <= 64: the tile's other rows are never looked at), depth of the ring
   int n_lo, n_batch;
-  BOperandIdx a, b, c, cin, c16i, add16i;
+  BOperandIdx c, cin, c16i, add16i;
   void* C;
   long long ldc, c_stride_lo, c_stride_hi;
   const float* Cin;    // optional fp32 addend, same layout as C (may BE C: in-place state), scaled by gamma[hi(A) * n_lo + lo]
@@ -55,6 +74,8 @@ struct BGemmParams {
   long long ld16, stride_lo16, stride_hi16;
   const float* decay;  // optional: value *= exp(decay[row] - decay[col]); element (hi, lo, r) at hi*d_hi + lo*d_lo + r*d_r
   long long d_hi, d_lo, d_r;
+  const float* rowscale;  // optional: value *= rowscale[row], element (hi, lo, r) at hi*r_hi + lo*r_lo + r*r_r
+  long long r_hi, r_lo, r_r;
   float alpha;
   int out_mode;        // 0 bf16 store, 1 fp32 store, 2 fp32 accumulate
   int mask_mode;       // 0 none, 1 keep col <= row, 2 keep col < row
@@ -62,10 +83,7 @@ struct BGemmParams {
 };
 
 struct Smem {
-  static constexpr int A_BYTES = BM * BK * 2;
-  static constexpr int B_BYTES = MAX_BN * BK * 2;
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BAR_OFFSET = STAGES * STAGE_BYTES;
+  static constexpr int BAR_OFFSET = RING_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;
 };
 
@@ -88,40 +106,43 @@ __device__ __forceinline__ int hi_of(const BOperandIdx& o, int hi_raw) {
   return (o.hi_index != nullptr ? o.hi_index[hi_raw] : hi_raw) + o.hi_offset;
 }
 
-template <bool A_MN, bool B_MN>
-__global__ void __launch_bounds__(BGEMM_THREADS, 1)
-bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, BGemmParams p) {
+__global__ void __launch_bounds__(BGEMM_THREADS, 2)
+bgemm_bf16_kernel(const __grid_constant__ BMaps maps, const __grid_constant__ BGemmParams p) {
   using L = Smem;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full_bar = (uint64_t*)(smem + L::BAR_OFFSET);
-  uint64_t* empty_bar = full_bar + STAGES;
-  uint64_t* tfull_bar = empty_bar + STAGES;
-  uint64_t* tempty_bar = tfull_bar + 2;
-  uint32_t* tmem_slot = (uint32_t*)(tempty_bar + 2);
+  uint64_t* empty_bar = full_bar + MAX_STAGES;
+  uint64_t* tfull_bar = empty_bar + MAX_STAGES;
+  uint64_t* tempty_bar = tfull_bar + 4;
+  uint32_t* tmem_slot = (uint32_t*)(tempty_bar + 4);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int total_units = p.n_batch * p.tiles_m * p.tiles_n;
-  const int BN = p.bn;
-  const uint32_t stage_tx = (uint32_t)(L::A_BYTES + BN * BK * 2);
+  const int BN = p.bn, STAGES = p.stages;
+  const int a_bytes = p.a_rows * BK * 2;
+  const int stage_bytes = a_bytes + BN * BK * 2;
+  const int n_acc = TMEM_COLS / BN;  // accumulators in flight: 2 (BN = 128) or 4
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 1);
       mbar_init(&empty_bar[s], 1);
     }
-    for (int a = 0; a < 2; ++a) {
+    for (int a = 0; a < n_acc; ++a) {
       mbar_init(&tfull_bar[a], 1);
       mbar_init(&tempty_bar[a], (blockDim.x >> 5) - 2);
     }
     *abort_flag = 0;
     mbar_fence_init();
-    tma_prefetch_desc(&tmA);
-    tma_prefetch_desc(&tmB);
+    for (int i = 0; i < p.n_pairs; ++i) {
+      tma_prefetch_desc(&maps.a[i]);
+      tma_prefetch_desc(&maps.b[i]);
+    }
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 2 * MAX_BN);
+    tmem_alloc(tmem_slot, TMEM_COLS);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -136,81 +157,84 @@ bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       bool ok = true;
       for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
         const Unit u = decode(p, unit);
-        const int a_hi = hi_of(p.a, u.hi_raw), a_lo = u.lo / p.a.lo_div;
-        const int b_hi = hi_of(p.b, u.hi_raw), b_lo = u.lo / p.b.lo_div;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, abort_flag, ERR_WAIT_EMPTY)) { ok = false; break; }
-          uint8_t* sA = smem + stage * L::STAGE_BYTES;
-          uint8_t* sB = sA + L::A_BYTES;
-          mbar_expect_tx(&full_bar[stage], stage_tx);
-          if (!A_MN) {
-            tma_load_4d(sA, &tmA, &full_bar[stage], kb * BK, u.tm * BM, a_lo, a_hi);
-          } else {
-#pragma unroll
-            for (int g = 0; g < BM / 64; ++g)
-              tma_load_4d(sA + g * (64 * BK * 2), &tmA, &full_bar[stage], u.tm * BM + g * 64, kb * BK, a_lo, a_hi);
+        for (int i = 0; i < p.n_pairs && ok; ++i) {
+          const BPair& pr = p.pair[i];
+          const int a_hi = hi_of(pr.a, u.hi_raw), b_hi = hi_of(pr.b, u.hi_raw);
+          for (int sk = 0, kb = 0, lo = u.lo * p.sum_lo; sk < p.sum_lo * pr.num_kb; ++sk) {
+            const int a_lo = lo / pr.a.lo_div, b_lo = lo / pr.b.lo_div;
+            if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, abort_flag, ERR_WAIT_EMPTY)) { ok = false; break; }
+            uint8_t* sA = smem + stage * stage_bytes;
+            uint8_t* sB = sA + a_bytes;
+            mbar_expect_tx(&full_bar[stage], (uint32_t)stage_bytes);
+            if (!pr.a_mn) {
+              tma_load_4d(sA, &maps.a[i], &full_bar[stage], kb * BK, u.tm * BM, a_lo, a_hi);
+            } else {
+              for (int g = 0; g < p.a_rows / 64; ++g)
+                tma_load_4d(sA + g * (64 * BK * 2), &maps.a[i], &full_bar[stage], u.tm * BM + g * 64, kb * BK, a_lo, a_hi);
+            }
+            if (!pr.b_mn) {
+              tma_load_4d(sB, &maps.b[i], &full_bar[stage], kb * BK, u.tn * BN, b_lo, b_hi);
+            } else {
+              for (int g = 0; g < BN / 64; ++g)
+                tma_load_4d(sB + g * (64 * BK * 2), &maps.b[i], &full_bar[stage], u.tn * BN + g * 64, kb * BK, b_lo, b_hi);
+            }
+            if (++kb == pr.num_kb) { kb = 0; ++lo; }
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
           }
-          if (!B_MN) {
-            tma_load_4d(sB, &tmB, &full_bar[stage], kb * BK, u.tn * BN, b_lo, b_hi);
-          } else {
-            for (int g = 0; g < BN / 64; ++g)
-              tma_load_4d(sB + g * (64 * BK * 2), &tmB, &full_bar[stage], u.tn * BN + g * 64, kb * BK, b_lo, b_hi);
-          }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t idesc = make_idesc_bf16(BM, BN, A_MN ? 1 : 0, B_MN ? 1 : 0);
-      constexpr uint32_t A_LBO = A_MN ? 64 * BK * 2 : 16;
-      constexpr uint32_t B_LBO = B_MN ? 64 * BK * 2 : 16;
-      constexpr uint32_t A_KSTEP = A_MN ? 16 * 128 : 32;
-      constexpr uint32_t B_KSTEP = B_MN ? 16 * 128 : 32;
       int stage = 0;
       uint32_t phase = 0;
-      int it = 0;
       bool ok = true;
-      for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x, ++it) {
-        const int acc = it & 1;
-        if (!mbar_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, p.status, abort_flag, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+      int acc = 0;
+      uint32_t acc_phase = 0;
+      for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
+        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, p.status, abort_flag, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t d_tmem = tmem_base + acc * MAX_BN;
-        for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, p.status, abort_flag, ERR_WAIT_FULL)) { ok = false; break; }
-          tc_fence_after();
-          const uint32_t sA = smem_u32(smem + stage * L::STAGE_BYTES);
-          const uint32_t sB = sA + L::A_BYTES;
-          const uint64_t adesc = make_smem_desc(sA, A_LBO, 1024);
-          const uint64_t bdesc = make_smem_desc(sB, B_LBO, 1024);
+        const uint32_t d_tmem = tmem_base + acc * BN;
+        bool first = true;
+        for (int i = 0; i < p.n_pairs && ok; ++i) {
+          const BPair& pr = p.pair[i];
+          const uint32_t idesc = make_idesc_bf16(BM, BN, pr.a_mn, pr.b_mn) | (pr.neg ? 1u << 13 : 0u);  // bit 13: negate A
+          const uint32_t a_lbo = pr.a_mn ? 64 * BK * 2 : 16, b_lbo = pr.b_mn ? 64 * BK * 2 : 16;
+          const uint32_t a_kstep = pr.a_mn ? 16 * 128 : 32, b_kstep = pr.b_mn ? 16 * 128 : 32;
+          for (int kb = 0; kb < p.sum_lo * pr.num_kb; ++kb) {
+            if (!mbar_wait(&full_bar[stage], phase, p.status, abort_flag, ERR_WAIT_FULL)) { ok = false; break; }
+            tc_fence_after();
+            const uint32_t sA = smem_u32(smem + stage * stage_bytes);
+            const uint32_t sB = sA + a_bytes;
+            const uint64_t adesc = make_smem_desc(sA, a_lbo, 1024);
+            const uint64_t bdesc = make_smem_desc(sB, b_lbo, 1024);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            mma_ss(d_tmem, desc_advance(adesc, k * A_KSTEP), desc_advance(bdesc, k * B_KSTEP), idesc,
-                   (kb > 0 || k > 0) ? 1u : 0u);
-          mma_commit(&empty_bar[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+            for (int k = 0; k < BK / 16; ++k)
+              mma_ss(d_tmem, desc_advance(adesc, k * a_kstep), desc_advance(bdesc, k * b_kstep), idesc, (!first || k > 0) ? 1u : 0u);
+            first = false;
+            mma_commit(&empty_bar[stage]);
+            if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          }
         }
         if (ok) mma_commit(&tfull_bar[acc]);
+        if (++acc == n_acc) { acc = 0; acc_phase ^= 1; }
       }
     }
   } else {
     const int quarter = warp & 3;
-    // eight epilogue warps: two per lane quarter, each takes half of the tile's columns (tiles are 64..256 wide);
-    // four: one per quarter takes them all
-    const bool split = blockDim.x == BGEMM_THREADS;
+    // two warps per lane quarter, each takes half of the tile's columns (tiles are 64 or 128 wide)
     const int half = (warp - 2) >> 2;
-    const int c_begin = split ? half * (BN / 2) : 0;
-    const int c_end = split ? c_begin + BN / 2 : BN;
-    int it = 0;
+    const int c_begin = half * (BN / 2), c_end = c_begin + BN / 2;
+    int acc = 0;
+    uint32_t acc_phase = 0;
     bool ok = true;
-    for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x, ++it) {
+    for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
       const Unit u = decode(p, unit);
-      const int acc = it & 1;
-      if (!mbar_wait_warp(&tfull_bar[acc], (it >> 1) & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+      if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const int row = u.tm * BM + quarter * 32 + lane;
       const bool row_ok = row < p.M;
-      const uint32_t t_row = tmem_base + acc * MAX_BN + ((uint32_t)(quarter * 32) << 16);
+      const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
       const long long c_base = (long long)hi_of(p.c, u.hi_raw) * p.c_stride_hi + (long long)(u.lo / p.c.lo_div) * p.c_stride_lo +
                                (long long)row * p.ldc;
       const float* cin_row = nullptr;
@@ -218,7 +242,7 @@ bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (p.Cin != nullptr) {
         cin_row = p.Cin + (long long)hi_of(p.cin, u.hi_raw) * p.c_stride_hi + (long long)(u.lo / p.cin.lo_div) * p.c_stride_lo +
                   (long long)row * p.ldc;
-        gamma = p.gamma != nullptr ? p.gamma[(long long)hi_of(p.a, u.hi_raw) * p.n_lo + u.lo] : 1.f;
+        gamma = p.gamma != nullptr ? p.gamma[(long long)hi_of(p.pair[0].a, u.hi_raw) * p.n_lo + u.lo] : 1.f;
       }
       const long long lo16 = (long long)(u.lo / p.c.lo_div) * p.stride_lo16 + (long long)row * p.ld16;
       __nv_bfloat16* c16_row = p.C16 != nullptr ? p.C16 + (long long)hi_of(p.c16i, u.hi_raw) * p.stride_hi16 + lo16 : nullptr;
@@ -229,6 +253,9 @@ bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         dec = p.decay + (long long)u.hi_raw * p.d_hi + (long long)u.lo * p.d_lo;
         if (row_ok) dec_row = dec[(long long)row * p.d_r];
       }
+      float scale = p.alpha;
+      if (p.rowscale != nullptr && row_ok)
+        scale *= p.rowscale[(long long)u.hi_raw * p.r_hi + (long long)u.lo * p.r_lo + (long long)row * p.r_r];
 #pragma unroll 1
       for (int c = c_begin; c < c_end; c += 32) {
         const int col0 = u.tn * BN + c;
@@ -236,37 +263,31 @@ bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         uint32_t r[32];
         tmem_ld_32x32(t_row + c, r);
         const bool full = (col0 + 32 <= p.N);
-        const bool vec = full && row_ok && p.out_mode != 0;
-        // every global read of this piece is issued before any store, so the loads overlap (one round trip per piece)
-        float4 o_acc[8], o_cin[8];
-        uint4 o_add[4];
-        if (vec) {
-          const float* dst = (const float*)p.C + c_base + col0;
-          if (p.out_mode == 2) {
+        const bool vec = full && row_ok;
+        // the addend (or, in the accumulating mode, the old result: never both in registers) is fetched while the
+        // accumulator comes in
+        uint4 side[8];
+        float dec_col = 0.f;
+        if (vec && p.out_mode == 2) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o_acc[j] = *reinterpret_cast<const float4*>(dst + 4 * j);
-          }
-          if (cin_row != nullptr) {
+          for (int j = 0; j < 8; ++j) side[j] = *reinterpret_cast<const uint4*>((const float*)p.C + c_base + col0 + 4 * j);
+        } else if (vec && add_row != nullptr) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) o_cin[j] = *reinterpret_cast<const float4*>(cin_row + col0 + 4 * j);
-          }
-          if (add_row != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) o_add[j] = *reinterpret_cast<const uint4*>(add_row + col0 + 8 * j);
-          }
+          for (int j = 0; j < 4; ++j) side[j] = *reinterpret_cast<const uint4*>(add_row + col0 + 8 * j);
         }
+        if (dec != nullptr && col0 + lane < p.N) dec_col = dec[(long long)(col0 + lane) * p.d_r];
         tmem_ld_wait();
-        if (!row_ok) continue;
         float v[32];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
+        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * scale;
         if (dec != nullptr) {
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             const int col = col0 + j;
+            const float dj = __shfl_sync(0xffffffffu, dec_col, j);  // before any lane leaves
             // masked entries may have a positive exponent: they are dropped, never multiplied
             const bool keep = col < p.N && (p.mask_mode == 0 || (p.mask_mode == 1 ? col <= row : col < row));
-            v[j] = keep ? v[j] * __expf(dec_row - dec[(long long)col * p.d_r]) : 0.f;
+            v[j] = keep ? v[j] * __expf(dec_row - dj) : 0.f;
           }
         } else if (p.mask_mode != 0) {
 #pragma unroll
@@ -275,14 +296,14 @@ bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             if (!(p.mask_mode == 1 ? col <= row : col < row)) v[j] = 0.f;
           }
         }
+        if (!row_ok) continue;
         if (p.out_mode == 0) {
           __nv_bfloat16* dst = (__nv_bfloat16*)p.C + c_base + col0;
           if (add_row != nullptr) {  // bf16 result with a bf16 addend (v_new = u - w S, o = q S + A v)
             if (full) {
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
-                const uint4 a4 = *reinterpret_cast<const uint4*>(add_row + col0 + 8 * j);
-                const uint32_t w4[4] = {a4.x, a4.y, a4.z, a4.w};
+                const uint32_t w4[4] = {side[j].x, side[j].y, side[j].z, side[j].w};
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
                   v[8 * j + 2 * t] += __uint_as_float(w4[t] << 16);
@@ -312,19 +333,24 @@ bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
           float* dst = (float*)p.C + c_base + col0;
           if (p.out_mode == 2) {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) { v[4 * j] += o_acc[j].x; v[4 * j + 1] += o_acc[j].y; v[4 * j + 2] += o_acc[j].z; v[4 * j + 3] += o_acc[j].w; }
+            for (int j = 0; j < 8; ++j) {
+              v[4 * j] += __uint_as_float(side[j].x); v[4 * j + 1] += __uint_as_float(side[j].y);
+              v[4 * j + 2] += __uint_as_float(side[j].z); v[4 * j + 3] += __uint_as_float(side[j].w);
+            }
           }
           if (cin_row != nullptr) {
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
-              v[4 * j] = fmaf(gamma, o_cin[j].x, v[4 * j]); v[4 * j + 1] = fmaf(gamma, o_cin[j].y, v[4 * j + 1]);
-              v[4 * j + 2] = fmaf(gamma, o_cin[j].z, v[4 * j + 2]); v[4 * j + 3] = fmaf(gamma, o_cin[j].w, v[4 * j + 3]);
+              const float4 o = *reinterpret_cast<const float4*>(cin_row + col0 + 4 * j);
+              v[4 * j] = fmaf(gamma, o.x, v[4 * j]); v[4 * j + 1] = fmaf(gamma, o.y, v[4 * j + 1]);
+              v[4 * j + 2] = fmaf(gamma, o.z, v[4 * j + 2]); v[4 * j + 3] = fmaf(gamma, o.w, v[4 * j + 3]);
             }
           }
           if (add_row != nullptr) {
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-              const uint32_t w4[4] = {o_add[j].x, o_add[j].y, o_add[j].z, o_add[j].w};
+              const uint4 a4 = p.out_mode == 2 ? *reinterpret_cast<const uint4*>(add_row + col0 + 8 * j) : side[j];
+              const uint32_t w4[4] = {a4.x, a4.y, a4.z, a4.w};
 #pragma unroll
               for (int t = 0; t < 4; ++t) {
                 v[8 * j + 2 * t] += __uint_as_float(w4[t] << 16);
@@ -362,6 +388,7 @@ bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+      if (++acc == n_acc) { acc = 0; acc_phase ^= 1; }
     }
   }
 
@@ -369,16 +396,14 @@ bgemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 2 * MAX_BN);
+    tmem_dealloc(tmem_base, TMEM_COLS);
   }
 }
 
-template <bool A_MN, bool B_MN>
-int launch_b(const CUtensorMap& tmA, const CUtensorMap& tmB, const BGemmParams& p, cudaStream_t stream) {
-  auto kern = bgemm_bf16_kernel<A_MN, B_MN>;
+int launch_b(const BMaps& maps, const BGemmParams& p, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(bgemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
@@ -390,12 +415,8 @@ int launch_b(const CUtensorMap& tmA, const CUtensorMap& tmB, const BGemmParams& 
     if (sms <= 0) sms = 148;
   }
   const long long units = (long long)p.n_batch * p.tiles_m * p.tiles_n;
-  const int grid = (int)(units < sms ? units : sms);
-  static const int threads = []() {
-    const char* e = getenv("FLAME_B200_BGEMM_EPI_WARPS");  // 4: one epilogue warp per TMEM lane quarter
-    return (e && e[0] == '4') ? 192 : BGEMM_THREADS;
-  }();
-  kern<<<grid, threads, Smem::TOTAL, stream>>>(tmA, tmB, p);
+  const int grid = (int)(units < 2 * sms ? units : 2 * sms);
+  bgemm_bf16_kernel<<<grid, BGEMM_THREADS, Smem::TOTAL, stream>>>(maps, p);
   return fb::launch_ok("bgemm_bf16_kernel");
 }
 
@@ -414,6 +435,8 @@ struct FbBOperand {
   int lo_div;
   int hi_offset;
   const int* hi_index;
+  int k;               // K of the product this operand belongs to
+  int neg;             // A operands: subtract this product
 };
 
 struct FbBEpilogue {
@@ -434,33 +457,39 @@ struct FbBEpilogue {
   long long ld16, stride_lo16, stride_hi16;
   const float* decay;  // optional fp32 vector per batch, see bgemm.cu header
   long long d_hi, d_lo, d_r;
+  const float* rowscale;  // optional fp32 factor per row
+  long long r_hi, r_lo, r_r;
   float alpha;
   int out_mode, mask_mode;
 };
 
-// n_hi_batch x n_lo_batch problems of size M x N x K.  Returns 0 on success.
-int fb_bgemm_bf16(const FbBOperand* a, const FbBOperand* b, const FbBEpilogue* e, int n_hi_batch, int n_lo_batch, int M,
-                  int N, int K, cudaStream_t stream) {
-  if (n_hi_batch <= 0 || n_lo_batch <= 0 || M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((a->ld & 7) || (b->ld & 7) || (a->stride_lo & 7) || (b->stride_lo & 7) || (a->stride_hi & 7) || (b->stride_hi & 7) ||
-      ((uintptr_t)a->ptr & 15) || ((uintptr_t)b->ptr & 15)) {
-    fprintf(stderr, "[flame_b200] bgemm: operand bases and strides must be multiples of 16 bytes\n");
-    return -2;
+// n_hi_batch x n_lo_batch problems of size M x N; ops: n_pairs times (A, B), each product summed over sum_lo consecutive lo
+// coordinates.  Returns 0 on success.
+int fb_bgemm_bf16(const FbBOperand* ops, int n_pairs, const FbBEpilogue* e, int n_hi_batch, int n_lo_batch, int sum_lo, int M, int N,
+                  cudaStream_t stream) {
+  if (n_hi_batch <= 0 || n_lo_batch <= 0 || M <= 0 || N <= 0) return 0;
+  if (n_pairs < 1 || n_pairs > MAX_PAIRS || sum_lo < 1) return -2;
+  for (int i = 0; i < 2 * n_pairs; ++i) {
+    const FbBOperand& o = ops[i];
+    if ((o.ld & 7) || (o.stride_lo & 7) || (o.stride_hi & 7) || ((uintptr_t)o.ptr & 15) || o.k <= 0) {
+      fprintf(stderr, "[flame_b200] bgemm: operand bases and strides must be multiples of 16 bytes\n");
+      return -2;
+    }
   }
   if ((e->ldc & 7) || (e->stride_lo & 7) || (e->stride_hi & 7) || ((uintptr_t)e->C & 15)) {
     fprintf(stderr, "[flame_b200] bgemm: output base and strides must be multiples of 8 elements\n");
     return -2;
   }
   BGemmParams p;
-  p.M = M; p.N = N; p.K = K;
-  p.bn = N <= 64 ? 64 : (N <= 128 ? 128 : 256);
+  p.M = M; p.N = N; p.n_pairs = n_pairs; p.sum_lo = sum_lo;
+  p.bn = N <= 64 ? 64 : MAX_BN;
+  p.a_rows = M <= 64 ? 64 : BM;
+  p.stages = RING_BYTES / ((p.a_rows + p.bn) * BK * 2);
+  if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
   p.tiles_m = (M + BM - 1) / BM;
   p.tiles_n = (N + p.bn - 1) / p.bn;
-  p.num_kb = (K + BK - 1) / BK;
   p.n_lo = n_lo_batch;
   p.n_batch = n_hi_batch * n_lo_batch;
-  p.a = {a->hi_index, a->hi_offset, a->lo_div > 0 ? a->lo_div : 1};
-  p.b = {b->hi_index, b->hi_offset, b->lo_div > 0 ? b->lo_div : 1};
   p.c = {e->c_hi_index, e->c_hi_offset, e->c_lo_div > 0 ? e->c_lo_div : 1};
   p.cin = {e->cin_hi_index, e->cin_hi_offset, p.c.lo_div};
   p.C = e->C; p.ldc = e->ldc; p.c_stride_lo = e->stride_lo; p.c_stride_hi = e->stride_hi;
@@ -471,23 +500,28 @@ int fb_bgemm_bf16(const FbBOperand* a, const FbBOperand* b, const FbBEpilogue* e
   p.ld16 = e->ld16; p.stride_lo16 = e->stride_lo16; p.stride_hi16 = e->stride_hi16;
   p.Cin = e->Cin; p.gamma = e->gamma;
   p.decay = e->decay; p.d_hi = e->d_hi; p.d_lo = e->d_lo; p.d_r = e->d_r;
+  p.rowscale = e->rowscale; p.r_hi = e->r_hi; p.r_lo = e->r_lo; p.r_r = e->r_r;
   p.alpha = e->alpha; p.out_mode = e->out_mode; p.mask_mode = e->mask_mode;
   p.status = fb::status_ptr();
   if ((p.C16 != nullptr || p.Cin != nullptr) && p.out_mode == 0) return -3;
   if ((p.C16 != nullptr || p.add16 != nullptr) && ((p.ld16 & 7) || (p.stride_lo16 & 7) || (p.stride_hi16 & 7))) return -2;
-  CUtensorMap tmA, tmB;
-  int rc;
-  // dims: (inner, rows, lo, hi)
-  if (!a->mn) rc = fb::make_tmap_4d(&tmA, a->ptr, 2, a->n_hi, a->n_lo, M, K, a->stride_hi, a->stride_lo, a->ld, BM, BK, true);
-  else        rc = fb::make_tmap_4d(&tmA, a->ptr, 2, a->n_hi, a->n_lo, K, M, a->stride_hi, a->stride_lo, a->ld, BK, 64, true);
-  if (rc) return rc;
-  if (!b->mn) rc = fb::make_tmap_4d(&tmB, b->ptr, 2, b->n_hi, b->n_lo, N, K, b->stride_hi, b->stride_lo, b->ld, p.bn, BK, true);
-  else        rc = fb::make_tmap_4d(&tmB, b->ptr, 2, b->n_hi, b->n_lo, K, N, b->stride_hi, b->stride_lo, b->ld, BK, 64, true);
-  if (rc) return rc;
-  if (!a->mn && !b->mn) return launch_b<false, false>(tmA, tmB, p, stream);
-  if (!a->mn && b->mn)  return launch_b<false, true>(tmA, tmB, p, stream);
-  if (a->mn && !b->mn)  return launch_b<true, false>(tmA, tmB, p, stream);
-  return launch_b<true, true>(tmA, tmB, p, stream);
+  BMaps maps;
+  for (int i = 0; i < n_pairs; ++i) {
+    const FbBOperand &a = ops[2 * i], &b = ops[2 * i + 1];
+    BPair& pr = p.pair[i];
+    pr.a = {a.hi_index, a.hi_offset, a.lo_div > 0 ? a.lo_div : 1};
+    pr.b = {b.hi_index, b.hi_offset, b.lo_div > 0 ? b.lo_div : 1};
+    pr.num_kb = (a.k + BK - 1) / BK;
+    pr.a_mn = a.mn; pr.b_mn = b.mn; pr.neg = a.neg;
+    // dims: (inner, rows, lo, hi)
+    int rc = a.mn ? fb::make_tmap_4d(&maps.a[i], a.ptr, 2, a.n_hi, a.n_lo, a.k, M, a.stride_hi, a.stride_lo, a.ld, BK, 64, true)
+                  : fb::make_tmap_4d(&maps.a[i], a.ptr, 2, a.n_hi, a.n_lo, M, a.k, a.stride_hi, a.stride_lo, a.ld, p.a_rows, BK, true);
+    if (rc) return rc;
+    rc = b.mn ? fb::make_tmap_4d(&maps.b[i], b.ptr, 2, b.n_hi, b.n_lo, b.k, N, b.stride_hi, b.stride_lo, b.ld, BK, 64, true)
+              : fb::make_tmap_4d(&maps.b[i], b.ptr, 2, b.n_hi, b.n_lo, N, b.k, b.stride_hi, b.stride_lo, b.ld, p.bn, BK, true);
+    if (rc) return rc;
+  }
+  return launch_b(maps, p, stream);
 }
 
 }  // extern "C"

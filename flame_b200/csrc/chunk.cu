@@ -7,17 +7,32 @@
 
 namespace {
 
-// T = (I + A)^-1 for a strictly lower-triangular 64 x 64 A (the WY "solve" of the delta rule; the reference does it by
-// blockwise forward substitution in fla/ops/utils/solve_tril.py).  One 64-thread block per matrix: thread c solves
-// (I + A) x = e_c by forward substitution with x in registers; every A element is a shared-memory broadcast.
-__global__ void __launch_bounds__(64) tri_inverse_kernel(const float* __restrict__ A, __nv_bfloat16* __restrict__ out16,
-                                                         float* __restrict__ out32, long long n) {
+// T = (I + diag(beta) P)^-1 of the strictly lower-triangular score blocks P (the WY "solve" of the delta rule; the reference
+// does it by blockwise forward substitution in fla/ops/utils/solve_tril.py).  One 64-thread block per 64 x 64 diagonal block:
+// thread c solves (I + A) x = e_c by forward substitution with x in registers; every A element is a shared-memory
+// broadcast.  P: [n, C, C] fp32, C = 64 or 128; T: [n, C, C] bf16.
+//   C = 64:  also Tu = T diag(beta) and (b given) Tw = T diag(beta e^b), the matrices the values and keys are multiplied with,
+//            which used to be passes of their own over T
+//   C = 128: the two diagonal blocks of T, zeros above them, and A21 = the scaled lower-left block in bf16, from which two
+//            products make T's lower-left block
+// beta, b: element (chunk, head, i) at ((chunk * C + i) * H + head); a null beta means 1.
+__global__ void __launch_bounds__(64) delta_inverse_kernel(const float* __restrict__ P, const float* __restrict__ beta, const float* __restrict__ b,
+                                                           int C, int H, __nv_bfloat16* __restrict__ T, __nv_bfloat16* __restrict__ Tu,
+                                                           __nv_bfloat16* __restrict__ Tw, __nv_bfloat16* __restrict__ A21,
+                                                           float* __restrict__ T32) {
   __shared__ float sA[64 * 64];
-  const long long m = blockIdx.x;
-  if (m >= n) return;
-  const float* a = A + m * 4096;
-  for (int i = threadIdx.x; i < 4096 / 4; i += 64)
-    reinterpret_cast<float4*>(sA)[i] = reinterpret_cast<const float4*>(a)[i];
+  const int halves = C >> 6;
+  const long long m = blockIdx.x / halves;
+  const int half = (int)(blockIdx.x - m * halves), ch = (int)(m / H), h = (int)(m - (long long)ch * H);
+  const float* a = P + m * C * C + (long long)half * 64 * (C + 1);
+  auto beta_of = [&](int i) { return beta != nullptr ? beta[((long long)ch * C + i) * H + h] : 1.f; };
+  for (int i = threadIdx.x; i < 4096 / 4; i += 64) {
+    const int r = i >> 4;
+    float4 v = *reinterpret_cast<const float4*>(a + (long long)r * C + (i & 15) * 4);
+    const float f = beta_of(half * 64 + r);
+    v.x *= f, v.y *= f, v.z *= f, v.w *= f;
+    reinterpret_cast<float4*>(sA)[i] = v;
+  }
   __syncthreads();
   const int c = threadIdx.x;
   float x[64];
@@ -28,46 +43,218 @@ __global__ void __launch_bounds__(64) tri_inverse_kernel(const float* __restrict
     for (int j = 0; j < i; ++j) s = fmaf(-sA[i * 64 + j], x[j], s);
     x[i] = s;
   }
-  if (out16 != nullptr) {
-    __nv_bfloat16* o = out16 + m * 4096;
+  if (T32 != nullptr) {  // C = 64, full precision, nothing else
 #pragma unroll
-    for (int i = 0; i < 64; ++i) o[i * 64 + c] = __float2bfloat16(x[i]);
+    for (int i = 0; i < 64; ++i) T32[m * 4096 + i * 64 + c] = x[i];
+    return;
   }
-  if (out32 != nullptr) {
-    float* o = out32 + m * 4096;
+  __nv_bfloat16* o = T + m * C * C + (long long)half * 64 * (C + 1) + c;
 #pragma unroll
-    for (int i = 0; i < 64; ++i) o[i * 64 + c] = x[i];
+  for (int i = 0; i < 64; ++i) o[(long long)i * C] = __float2bfloat16(x[i]);
+  if (Tu != nullptr) {
+    const float f = beta_of(c);
+    __nv_bfloat16* u = Tu + m * 4096 + c;
+#pragma unroll
+    for (int i = 0; i < 64; ++i) u[i * 64] = __float2bfloat16(x[i] * f);
+    if (Tw != nullptr) {
+      const float fw = f * __expf(b[((long long)ch * C + c) * H + h]);
+      __nv_bfloat16* w = Tw + m * 4096 + c;
+#pragma unroll
+      for (int i = 0; i < 64; ++i) w[i * 64] = __float2bfloat16(x[i] * fw);
+    }
+  }
+  if (C == 128) {
+    if (half == 0) {
+      __nv_bfloat16* z = T + m * C * C + 64 + c;
+      for (int i = 0; i < 64; ++i) z[(long long)i * C] = __float2bfloat16(0.f);
+    } else {
+      const float* a21 = P + m * C * C + 64ll * C + c;
+      for (int i = 0; i < 64; ++i) A21[m * 4096 + i * 64 + c] = __float2bfloat16(a21[(long long)i * C] * beta_of(64 + i));
+    }
   }
 }
 
-// Elementwise chunk-state recurrence without a transition matrix:
-//   forward  X[c+1] = alpha[c] * X[c] + X[c+1]      reverse  X[c] = alpha[c] * X[c+1] + X[c]
-// over the chunks listed for one chunk position; alpha is [NC, H] (per_row = 0) or [NC, H, rows] (per_row = 1).
-// X is [NC + 1, H, rows, cols] fp32 with a bf16 mirror.
-__global__ void state_step_kernel(const int* __restrict__ idx, int n_idx, const float* __restrict__ alpha, int per_row,
-                                  float* __restrict__ X, __nv_bfloat16* __restrict__ X16, int H, int rows, int cols,
-                                  int reverse) {
-  const long long per_chunk = (long long)H * rows * cols;
-  const long long total = (long long)n_idx * per_chunk / 4;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long e = i * 4;
-    const int b = (int)(e / per_chunk);
-    const long long r = e - (long long)b * per_chunk;
-    const int c = idx[b];
-    const int h = (int)(r / ((long long)rows * cols));
-    const int row = (int)((r / cols) % rows);
-    const float al = per_row ? alpha[((long long)c * H + h) * rows + row] : alpha[(long long)c * H + h];
-    const long long src = (long long)(reverse ? c + 1 : c) * per_chunk + r;
-    const long long dst = (long long)(reverse ? c : c + 1) * per_chunk + r;
-    const float4 s = *reinterpret_cast<const float4*>(X + src);
-    float4 d = *reinterpret_cast<float4*>(X + dst);
-    d.x = fmaf(al, s.x, d.x); d.y = fmaf(al, s.y, d.y); d.z = fmaf(al, s.z, d.z); d.w = fmaf(al, s.w, d.w);
-    *reinterpret_cast<float4*>(X + dst) = d;
-    __nv_bfloat162 lo = __floats2bfloat162_rn(d.x, d.y), hi = __floats2bfloat162_rn(d.z, d.w);
-    uint2 q;
-    q.x = *reinterpret_cast<uint32_t*>(&lo);
-    q.y = *reinterpret_cast<uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(X16 + dst) = q;
+// Tu = T diag(beta), Tw = T diag(beta e^b) (C = 128, where T's corner comes from a product).  One block per matrix.
+__global__ void __launch_bounds__(256) delta_scale_kernel(const __nv_bfloat16* __restrict__ T, const float* __restrict__ beta, const float* __restrict__ b,
+                                                          int C, int H, __nv_bfloat16* __restrict__ Tu, __nv_bfloat16* __restrict__ Tw) {
+  __shared__ float fu[128], fw[128];
+  const long long m = blockIdx.x;
+  const int ch = (int)(m / H), h = (int)(m - (long long)ch * H);
+  for (int i = threadIdx.x; i < C; i += 256) {
+    const long long o = ((long long)ch * C + i) * H + h;
+    fu[i] = beta[o];
+    fw[i] = b != nullptr ? beta[o] * __expf(b[o]) : 0.f;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < C * C / 8; i += 256) {
+    const int j0 = (i * 8) & (C - 1);
+    const uint4 q = reinterpret_cast<const uint4*>(T + m * C * C)[i];
+    const __nv_bfloat162* t2 = reinterpret_cast<const __nv_bfloat162*>(&q);
+    uint4 qu, qw;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 t = __bfloat1622float2(t2[e]);
+      reinterpret_cast<__nv_bfloat162*>(&qu)[e] = __floats2bfloat162_rn(t.x * fu[j0 + 2 * e], t.y * fu[j0 + 2 * e + 1]);
+      reinterpret_cast<__nv_bfloat162*>(&qw)[e] = __floats2bfloat162_rn(t.x * fw[j0 + 2 * e], t.y * fw[j0 + 2 * e + 1]);
+    }
+    reinterpret_cast<uint4*>(Tu + m * C * C)[i] = qu;
+    if (Tw != nullptr) reinterpret_cast<uint4*>(Tw + m * C * C)[i] = qw;
+  }
+}
+
+__device__ __forceinline__ void unpack8f(const uint4& q, float (&f)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(h[i]);
+    f[2 * i] = t.x, f[2 * i + 1] = t.y;
+  }
+}
+__device__ __forceinline__ uint4 pack8f(const float (&f)[8]) {
+  uint4 q;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) reinterpret_cast<__nv_bfloat162*>(&q)[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+  return q;
+}
+
+// Backward of Tu and Tw: dT = dTu diag(beta) + dTw diag(beta e^b) (bf16), and over the rows
+//   dbeta_j = scale sum_i T_ij (dTu_ij + e^{b_j} dTw_ij),   db_j = scale sum_i beta_j e^{b_j} T_ij dTw_ij      (written, not added).
+// dTw and b null: one matrix served both products.  One block of 256 threads per (chunk, head); a thread keeps eight
+// columns' sums over its rows in registers, so a row costs no atomics.
+__global__ void __launch_bounds__(256) delta_bwd_t_kernel(const __nv_bfloat16* __restrict__ T, const __nv_bfloat16* __restrict__ dTu,
+                                                          const __nv_bfloat16* __restrict__ dTw, const float* __restrict__ beta,
+                                                          const float* __restrict__ b, int C, int H, float scale, __nv_bfloat16* __restrict__ dT,
+                                                          float* __restrict__ dbeta, float* __restrict__ db) {
+  __shared__ float su[16][132], sw[16][132];
+  const long long m = blockIdx.x;
+  const int ch = (int)(m / H), h = (int)(m - (long long)ch * H);
+  const int nv = C >> 3, v = threadIdx.x % nv, r0 = threadIdx.x / nv, groups = 256 / nv;  // 32 or 16 groups of rows
+  float fu[8], fe[8], au[8], aw[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const long long o = ((long long)ch * C + v * 8 + e) * H + h;
+    fu[e] = beta[o];
+    fe[e] = b != nullptr ? __expf(b[o]) : 0.f;
+    au[e] = aw[e] = 0.f;
+  }
+  for (int i = r0; i < C; i += groups) {
+    const long long o = (m * C * C + (long long)i * C) / 8 + v;
+    float t[8], gu[8], gw[8];
+    unpack8f(reinterpret_cast<const uint4*>(T)[o], t);
+    unpack8f(reinterpret_cast<const uint4*>(dTu)[o], gu);
+    if (dTw != nullptr) unpack8f(reinterpret_cast<const uint4*>(dTw)[o], gw);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float w = dTw != nullptr ? gw[e] * fe[e] : 0.f;
+      au[e] = fmaf(t[e], gu[e] + w, au[e]);
+      aw[e] = fmaf(t[e], w, aw[e]);
+      gu[e] = fu[e] * (gu[e] + w);
+    }
+    reinterpret_cast<uint4*>(dT)[o] = pack8f(gu);
+  }
+  // lanes of a warp hold the same columns for 32 / nv groups: add those by shuffle, the warps through shared memory
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    for (int o = nv; o < 32; o <<= 1) {
+      au[e] += __shfl_xor_sync(0xffffffffu, au[e], o);
+      aw[e] += __shfl_xor_sync(0xffffffffu, aw[e], o);
+    }
+  const int warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) < nv) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) su[warp][v * 8 + e] = au[e], sw[warp][v * 8 + e] = aw[e];
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < C; j += 256) {
+    float x = 0.f, y = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) x += su[w][j], y += sw[w][j];
+    const long long o = ((long long)ch * C + j) * H + h;
+    dbeta[o] = scale * x;
+    if (db != nullptr) db[o] = scale * beta[o] * y;
+  }
+}
+
+// Backward of the score blocks A = diag(beta) P (strict, P = k k^T decayed) and Q = tril(q k^T decayed):
+//   g_ij  = beta_i dA_ij e^{b_i - b_j} [j < i],   gq_ij = dQ_ij e^{b_i - b_j} [j <= i]     (bf16 operands of the dq, dk products)
+//   dbeta_i += scale sum_j dA_ij P_ij,   db_i += scale (row sum_i - column sum_i) of beta dA P + dQ Q
+// dA, P fp32 (null: only the second block, for the scalar-gated attention without a delta rule); dQ, Q bf16 and b only with a
+// decay (without one the products' epilogues already give gq).
+__global__ void __launch_bounds__(256) delta_bwd_scores_kernel(const float* __restrict__ dA, const float* __restrict__ P,
+                                                               const __nv_bfloat16* __restrict__ dQ, const __nv_bfloat16* __restrict__ Q,
+                                                               const float* __restrict__ beta, const float* __restrict__ b, int C, int H, float scale,
+                                                               __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ gq,
+                                                               float* __restrict__ dbeta, float* __restrict__ db) {
+  __shared__ float sb[128], srow[128], scol[8][132];
+  const long long m = blockIdx.x;
+  const int ch = (int)(m / H), h = (int)(m - (long long)ch * H);
+  for (int i = threadIdx.x; i < C; i += 256) sb[i] = b != nullptr ? b[((long long)ch * C + i) * H + h] : 0.f;
+  __syncthreads();
+  const int nv = C >> 3, v = threadIdx.x % nv, r0 = threadIdx.x / nv, groups = 256 / nv;
+  float col[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) col[e] = 0.f;
+  for (int i = r0; i < C; i += groups) {
+    const long long row = m * C * C + (long long)i * C + v * 8;
+    const long long ob = ((long long)ch * C + i) * H + h;
+    const float bi = sb[i], be = beta != nullptr ? beta[ob] : 0.f;
+    float gg[8], rs = 0.f, rd = 0.f;
+    if (dA != nullptr) {
+      float da[8], pp[8];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        *reinterpret_cast<float4*>(da + 4 * k) = *reinterpret_cast<const float4*>(dA + row + 4 * k);
+        *reinterpret_cast<float4*>(pp + 4 * k) = *reinterpret_cast<const float4*>(P + row + 4 * k);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int j = v * 8 + e;
+        const float x = j < i ? da[e] : 0.f, y = j < i ? x * pp[e] : 0.f;  // both operands are zero or unread above the diagonal
+        gg[e] = j < i ? x * be * (b != nullptr ? __expf(bi - sb[j]) : 1.f) : 0.f;
+        rs += y;
+        rd += be * y;
+        col[e] += be * y;
+      }
+      *reinterpret_cast<uint4*>(g + row) = pack8f(gg);
+    }
+    if (dQ != nullptr) {
+      float dq[8], qq[8];
+      unpack8f(*reinterpret_cast<const uint4*>(dQ + row), dq);
+      unpack8f(*reinterpret_cast<const uint4*>(Q + row), qq);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int j = v * 8 + e;
+        const float y = j <= i ? dq[e] * qq[e] : 0.f;
+        gg[e] = j <= i ? dq[e] * __expf(bi - sb[j]) : 0.f;
+        rd += y;
+        col[e] += y;
+      }
+      *reinterpret_cast<uint4*>(gq + row) = pack8f(gg);
+    }
+    for (int o = nv >> 1; o > 0; o >>= 1) {
+      rs += __shfl_xor_sync(0xffffffffu, rs, o);
+      rd += __shfl_xor_sync(0xffffffffu, rd, o);
+    }
+    if (v == 0) {
+      if (dbeta != nullptr) dbeta[ob] += scale * rs;
+      srow[i] = rd;
+    }
+  }
+  if (db == nullptr) return;
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    for (int o = nv; o < 32; o <<= 1) col[e] += __shfl_xor_sync(0xffffffffu, col[e], o);
+  const int warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) < nv) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) scol[warp][v * 8 + e] = col[e];
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < C; j += 256) {
+    float x = srow[j];
+#pragma unroll
+    for (int w = 0; w < 8; ++w) x -= scol[w][j];
+    db[((long long)ch * C + j) * H + h] += scale * x;
   }
 }
 
@@ -75,96 +262,353 @@ __global__ void state_step_kernel(const int* __restrict__ idx, int n_idx, const 
 
 extern "C" {
 
-int fb_tri_inverse(const float* A, void* out16, float* out32, long long n, cudaStream_t stream) {
-  if (n <= 0) return 0;
-  tri_inverse_kernel<<<(unsigned)n, 64, 0, stream>>>(A, (__nv_bfloat16*)out16, out32, n);
-  return fb::launch_ok("tri_inverse_kernel");
+int fb_delta_inverse(const float* P, const float* beta, const float* b, int NC, int H, int C, void* T, void* Tu, void* Tw, void* A21,
+                     float* T32, cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  if ((C != 64 && C != 128) || (T32 != nullptr && C != 64)) return -2;
+  delta_inverse_kernel<<<(unsigned)(NC * H * (C / 64)), 64, 0, stream>>>(P, beta, b, C, H, (__nv_bfloat16*)T, (__nv_bfloat16*)(C == 64 ? Tu : nullptr),
+                                                                         (__nv_bfloat16*)Tw, (__nv_bfloat16*)A21, T32);
+  return fb::launch_ok("delta_inverse_kernel");
 }
 
-int fb_state_step(const int* idx, int n_idx, const float* alpha, int per_row, float* X, void* X16, int H, int rows, int cols,
-                  int reverse, cudaStream_t stream) {
-  if (n_idx <= 0) return 0;
-  if (cols & 3) return -2;
-  const long long total = (long long)n_idx * H * rows * cols / 4;
-  long long blocks = (total + 255) / 256;
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  state_step_kernel<<<(unsigned)blocks, 256, 0, stream>>>(idx, n_idx, alpha, per_row, X, (__nv_bfloat16*)X16, H, rows, cols,
-                                                          reverse);
-  return fb::launch_ok("state_step_kernel");
+int fb_delta_scale(const void* T, const float* beta, const float* b, int NC, int H, int C, void* Tu, void* Tw, cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  if (C != 64 && C != 128) return -2;
+  delta_scale_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)T, beta, b, C, H, (__nv_bfloat16*)Tu, (__nv_bfloat16*)Tw);
+  return fb::launch_ok("delta_scale_kernel");
+}
+
+int fb_delta_bwd_t(const void* T, const void* dTu, const void* dTw, const float* beta, const float* b, int NC, int H, int C, float scale, void* dT,
+                   float* dbeta, float* db, cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  if (C != 64 && C != 128) return -2;
+  delta_bwd_t_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)T, (const __nv_bfloat16*)dTu, (const __nv_bfloat16*)dTw, beta, b,
+                                                             C, H, scale, (__nv_bfloat16*)dT, dbeta, db);
+  return fb::launch_ok("delta_bwd_t_kernel");
+}
+
+int fb_delta_bwd_scores(const float* dA, const float* P, const void* dQ, const void* Q, const float* beta, const float* b, int NC, int H, int C,
+                        float scale, void* g, void* gq, float* dbeta, float* db, cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  if (C != 64 && C != 128) return -2;
+  delta_bwd_scores_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>(dA, P, (const __nv_bfloat16*)dQ, (const __nv_bfloat16*)Q, beta, b, C, H, scale,
+                                                                  (__nv_bfloat16*)g, (__nv_bfloat16*)gq, dbeta, db);
+  return fb::launch_ok("delta_bwd_scores_kernel");
 }
 
 }  // extern "C"
 
 // ---------------------------------------------------------------------------------------------------------------
-// GLA intra-chunk scores, diagonal 16 x 16 sub-blocks:  A_ij = scale * sum_d q_id k_jd exp(b_id - b_jd),  j <= i,
-// evaluated pairwise so that no exponent is positive whatever the gates are (the "secondary chunking" of
-// fla/ops/gla/chunk.py:88-170; the off-diagonal sub-blocks are re-based products on the batched GEMM).
-// q, k: [NC, 64, H, dk] bf16; b: [NC, 64, H, dk] fp32 (within-chunk cumulative log decay); A: [NC, H, 64, 64].
-// Grid (NC * H, 4); 256 threads = one (i, j) pair each.
+// Scalar-gated attention with queries and keys shared by groups of heads (Mamba2's SSD): what is elementwise around its
+// products, on the value side.  v, do, ..: [NC, C, H, dv] bf16; g, b: [NC, C, H] fp32; one block per (chunk, head), a row of
+// dv in dv / 8 lanes (a power of two up to 32), so that the row sums are shuffles.
 namespace {
 
-__global__ void __launch_bounds__(256) gla_diag_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                                                           const float* __restrict__ b, float* __restrict__ A, int H, int dk,
-                                                           float scale) {
-  extern __shared__ float sm[];
-  const int ld = dk + 1;
-  float* sq = sm;
-  float* sk = sq + 16 * ld;
-  float* sb = sk + 16 * ld;
-  const int ch = blockIdx.x, c = ch / H, h = ch - c * H, blk = blockIdx.y;
-  const long long row0 = ((long long)c * 64 + blk * 16);
-  for (int idx = threadIdx.x; idx < 16 * dk; idx += 256) {
-    const int r = idx / dk, d = idx - r * dk;
-    const long long g = ((row0 + r) * H + h) * dk + d;
-    sq[r * ld + d] = __bfloat162float(q[g]);
-    sk[r * ld + d] = __bfloat162float(k[g]);
-    sb[r * ld + d] = b[g];
-  }
-  __syncthreads();
-  const int i = threadIdx.x >> 4, j = threadIdx.x & 15;
-  float acc = 0.f;
-  if (j <= i) {
-    for (int d = 0; d < dk; ++d) acc = fmaf(sq[i * ld + d] * sk[j * ld + d], __expf(sb[i * ld + d] - sb[j * ld + d]), acc);
-  }
-  A[((long long)ch * 64 + blk * 16 + i) * 64 + blk * 16 + j] = acc * scale;
+__device__ __forceinline__ void group_rows(int C, int H, int dv, int& ch, int& h, int& v, int& r0, int& groups) {
+  ch = blockIdx.x / H, h = blockIdx.x - ch * H;
+  const int nv = dv >> 3;
+  v = threadIdx.x % nv, r0 = threadIdx.x / nv, groups = blockDim.x / nv;
 }
 
-// Backward of the diagonal sub-blocks: dq_id = scale sum_{j<=i} dA_ij k_jd e^{b_id-b_jd}, dk_jd = scale sum_{i>=j} dA_ij q_id e^{b_id-b_jd},
-// db = q dq - k dk (all ADDED into fp32 [NC, 64, H, dk] buffers).
-__global__ void __launch_bounds__(256) gla_diag_bwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                                                           const float* __restrict__ b, const float* __restrict__ dA,
-                                                           float* __restrict__ dq, float* __restrict__ dk_, float* __restrict__ db,
-                                                           int H, int dk, float scale) {
-  extern __shared__ float sm[];
-  const int ld = dk + 1;
-  float* sq = sm;
-  float* sk = sq + 16 * ld;
-  float* sb = sk + 16 * ld;
-  float* sdA = sb + 16 * ld;  // 16 x 16
-  const int ch = blockIdx.x, c = ch / H, h = ch - c * H, blk = blockIdx.y;
-  const long long row0 = ((long long)c * 64 + blk * 16);
-  for (int idx = threadIdx.x; idx < 16 * dk; idx += 256) {
-    const int r = idx / dk, d = idx - r * dk;
-    const long long g = ((row0 + r) * H + h) * dk + d;
-    sq[r * ld + d] = __bfloat162float(q[g]);
-    sk[r * ld + d] = __bfloat162float(k[g]);
-    sb[r * ld + d] = b[g];
-  }
-  {
-    const int i = threadIdx.x >> 4, j = threadIdx.x & 15;
-    sdA[threadIdx.x] = (j <= i) ? dA[((long long)ch * 64 + blk * 16 + i) * 64 + blk * 16 + j] * scale : 0.f;
+// b = cumsum(g), eb = scale e^b (fp32, the factor of an output row), alpha = e^{b_last}, vhat = v e^{b_last - b}
+__global__ void __launch_bounds__(256) group_prep_fwd_kernel(const __nv_bfloat16* __restrict__ v, const float* __restrict__ g, int C, int H, int dv,
+                                                             float scale, float* __restrict__ b, float* __restrict__ eb, float* __restrict__ alpha,
+                                                             __nv_bfloat16* __restrict__ vhat) {
+  __shared__ float sb[128];
+  int ch, h, vv, r0, groups;
+  group_rows(C, H, dv, ch, h, vv, r0, groups);
+  if (threadIdx.x < 32) {  // warp 0: inclusive sum of up to 128 steps, four per lane
+    const int lane = threadIdx.x, per = C >> 5;
+    float loc[4], s = 0.f;
+    for (int k = 0; k < per; ++k) {
+      s += g[((long long)ch * C + lane * per + k) * H + h];
+      loc[k] = s;
+    }
+    float pre = s;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_up_sync(0xffffffffu, pre, o);
+      if (lane >= o) pre += t;
+    }
+    pre -= s;
+    for (int k = 0; k < per; ++k) sb[lane * per + k] = pre + loc[k];
   }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < 16 * dk; idx += 256) {
-    const int r = idx / dk, d = idx - r * dk;
-    const float br = sb[r * ld + d];
-    float gq = 0.f, gk = 0.f;
-    for (int j = 0; j <= r; ++j) gq = fmaf(sdA[r * 16 + j] * sk[j * ld + d], __expf(br - sb[j * ld + d]), gq);
-    for (int i = r; i < 16; ++i) gk = fmaf(sdA[i * 16 + r] * sq[i * ld + d], __expf(sb[i * ld + d] - br), gk);
-    const long long g = ((row0 + r) * H + h) * dk + d;
-    dq[g] += gq;
-    dk_[g] += gk;
-    db[g] += sq[r * ld + d] * gq - sk[r * ld + d] * gk;
+  const float last = sb[C - 1];
+  for (int i = threadIdx.x; i < C; i += blockDim.x) {
+    const long long o = ((long long)ch * C + i) * H + h;
+    b[o] = sb[i];
+    eb[o] = scale * __expf(sb[i]);
+  }
+  if (threadIdx.x == 0) alpha[(long long)ch * H + h] = __expf(last);
+  for (int i = r0; i < C; i += groups) {
+    const long long o = (((long long)ch * C + i) * H + h) * dv + vv * 8;
+    float x[8];
+    unpack8f(*reinterpret_cast<const uint4*>(v + o), x);
+    const float f = __expf(last - sb[i]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] *= f;
+    *reinterpret_cast<uint4*>(vhat + o) = pack8f(x);
+  }
+}
+
+// dos = do eb (the gradient of q S), db_i = sum do_i o1_i with o1 = eb (q S) (written, not added)
+__global__ void __launch_bounds__(256) group_bwd1_kernel(const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ o1,
+                                                         const float* __restrict__ eb, int C, int H, int dv, __nv_bfloat16* __restrict__ dos,
+                                                         float* __restrict__ db) {
+  int ch, h, vv, r0, groups;
+  group_rows(C, H, dv, ch, h, vv, r0, groups);
+  const int nv = dv >> 3;
+  for (int i = r0; i < C; i += groups) {
+    const long long ob = ((long long)ch * C + i) * H + h, o = ob * dv + vv * 8;
+    float x[8], y[8], s = 0.f;
+    unpack8f(*reinterpret_cast<const uint4*>(dout + o), x);
+    unpack8f(*reinterpret_cast<const uint4*>(o1 + o), y);
+    const float f = eb[ob];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      s = fmaf(x[e], y[e], s);
+      x[e] *= f;
+    }
+    *reinterpret_cast<uint4*>(dos + o) = pack8f(x);
+    for (int k = nv >> 1; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    if (vv == 0) db[ob] = s;
+  }
+}
+
+// dv = dv1 + dvhat e^{b_last - b}; db_i -= sum dvhat vhat, the chunk's last step gets that sum over all steps and
+// alpha dalpha; dg = reverse cumulative sum of db
+__global__ void __launch_bounds__(256) group_bwd2_kernel(const __nv_bfloat16* __restrict__ dvhat, const __nv_bfloat16* __restrict__ vhat,
+                                                         const __nv_bfloat16* __restrict__ dv1, const float* __restrict__ b,
+                                                         const float* __restrict__ db, const float* __restrict__ alpha, const float* __restrict__ dalpha,
+                                                         int C, int H, int dv, __nv_bfloat16* __restrict__ dvo, float* __restrict__ dg) {
+  __shared__ float sdb[128], sv[128];
+  int ch, h, vv, r0, groups;
+  group_rows(C, H, dv, ch, h, vv, r0, groups);
+  const int nv = dv >> 3;
+  const float last = b[((long long)ch * C + C - 1) * H + h];
+  for (int i = r0; i < C; i += groups) {
+    const long long ob = ((long long)ch * C + i) * H + h, o = ob * dv + vv * 8;
+    float x[8], y[8], z[8], s = 0.f;
+    unpack8f(*reinterpret_cast<const uint4*>(dvhat + o), x);
+    unpack8f(*reinterpret_cast<const uint4*>(vhat + o), y);
+    unpack8f(*reinterpret_cast<const uint4*>(dv1 + o), z);
+    const float f = __expf(last - b[ob]);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      s = fmaf(x[e], y[e], s);
+      z[e] = fmaf(x[e], f, z[e]);
+    }
+    *reinterpret_cast<uint4*>(dvo + o) = pack8f(z);
+    for (int k = nv >> 1; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    if (vv == 0) {
+      sdb[i] = db[ob] - s;
+      sv[i] = s;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < 32) {  // warp 0: suffix sums, up to four steps per lane
+    const int lane = threadIdx.x, per = C >> 5;
+    float tot = 0.f, mine = 0.f, loc[4];
+    for (int k = 0; k < per; ++k) tot += sv[lane * per + k];
+    for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+    tot += alpha[(long long)ch * H + h] * dalpha[(long long)ch * H + h];  // everything that enters through the last step
+    for (int k = per - 1; k >= 0; --k) {
+      mine += sdb[lane * per + k];
+      loc[k] = mine;
+    }
+    float suf = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float t = __shfl_down_sync(0xffffffffu, suf, o);
+      if (lane + o < 32) suf += t;
+    }
+    suf -= mine;
+    for (int k = 0; k < per; ++k) dg[((long long)ch * C + lane * per + k) * H + h] = loc[k] + suf + tot;
+  }
+}
+
+inline bool group_shape_ok(int C, int dv) {
+  const int nv = dv >> 3;
+  return (C == 64 || C == 128) && (dv & 7) == 0 && nv >= 1 && nv <= 32 && (nv & (nv - 1)) == 0;
+}
+
+}  // namespace
+
+extern "C" {
+
+int fb_group_prep_fwd(const void* v, const float* g, int NC, int C, int H, int dv, float scale, float* b, float* eb, float* alpha, void* vhat,
+                      cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  if (!group_shape_ok(C, dv)) return -2;
+  group_prep_fwd_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)v, g, C, H, dv, scale, b, eb, alpha, (__nv_bfloat16*)vhat);
+  return fb::launch_ok("group_prep_fwd_kernel");
+}
+
+int fb_group_bwd1(const void* dout, const void* o1, const float* eb, int NC, int C, int H, int dv, void* dos, float* db, cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  if (!group_shape_ok(C, dv)) return -2;
+  group_bwd1_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)o1, eb, C, H, dv, (__nv_bfloat16*)dos, db);
+  return fb::launch_ok("group_bwd1_kernel");
+}
+
+int fb_group_bwd2(const void* dvhat, const void* vhat, const void* dv1, const float* b, const float* db, const float* alpha, const float* dalpha, int NC,
+                  int C, int H, int dv, void* dvo, float* dg, cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  if (!group_shape_ok(C, dv)) return -2;
+  group_bwd2_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)dvhat, (const __nv_bfloat16*)vhat, (const __nv_bfloat16*)dv1, b, db,
+                                                            alpha, dalpha, C, H, dv, (__nv_bfloat16*)dvo, dg);
+  return fb::launch_ok("group_bwd2_kernel");
+}
+
+}  // extern "C"
+
+// ---------------------------------------------------------------------------------------------------------------
+// GLA intra-chunk scores  A_ij = scale * sum_d q_id k_jd exp(b_id - b_jd),  j <= i, of 64-token chunks.  The diagonal 16 x 16
+// sub-blocks are evaluated pairwise so that no exponent is positive whatever the gates are (the "secondary chunking" of
+// fla/ops/gla/chunk.py:88-170); the sub-blocks left of them come in from a batched GEMM on re-based operands.
+// q, k: [NC, 64, H, dk] bf16; b: [NC, 64, H, dk] fp32 (within-chunk cumulative log decay); blk: [3 NC, H, 16, 48] bf16, entry
+// (3 c + I - 1) holding the 16 rows of sub-block I; A: [NC, H, 64, 64] bf16, written in full.
+// One block per (chunk, head).  The pairs with j <= i of the four sub-blocks are 4 x 136 = 544 = 17 full warps, a thread each;
+// operands of 64 channels at a time in shared memory, rows 4 words apart modulo the banks, read as float4: four loads
+// and an exponential per four channels and pair bound it.  With a thread per (i, j) of a sub-block half of the threads had
+// nothing to do and every operand was a 4-byte load: 0.29 ms at 65,536 tokens, 4 heads of 128.
+namespace {
+
+constexpr int GD_T = 64;        // channels per trip
+constexpr int GD_LD = GD_T + 4;
+constexpr int GD_THREADS = 544;
+
+template <typename TQ>
+__global__ void __launch_bounds__(GD_THREADS, 2) gla_scores_kernel(const TQ* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+                                                                const float* __restrict__ b, const __nv_bfloat16* __restrict__ blk,
+                                                                __nv_bfloat16* __restrict__ A, int H, int dk, float scale) {
+  extern __shared__ __align__(16) float sm[];
+  float *sq = sm, *sk = sq + 64 * GD_LD, *sb = sk + 64 * GD_LD;
+  const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
+  const int sub = threadIdx.x / 136, pr = threadIdx.x - sub * 136;
+  int i = (int)((sqrtf(8.f * pr + 1.f) - 1.f) * 0.5f);
+  while ((i + 1) * (i + 2) / 2 <= pr) ++i;
+  while (i * (i + 1) / 2 > pr) --i;
+  const int j = pr - i * (i + 1) / 2;
+  const float4* qi = reinterpret_cast<const float4*>(sq + (sub * 16 + i) * GD_LD);
+  const float4* bi = reinterpret_cast<const float4*>(sb + (sub * 16 + i) * GD_LD);
+  const float4* kj = reinterpret_cast<const float4*>(sk + (sub * 16 + j) * GD_LD);
+  const float4* bj = reinterpret_cast<const float4*>(sb + (sub * 16 + j) * GD_LD);
+  float acc = 0.f;
+  for (int d0 = 0; d0 < dk; d0 += GD_T) {
+    const int n = min(GD_T, dk - d0);
+    __syncthreads();
+    for (int idx = threadIdx.x; idx < 64 * GD_T; idx += GD_THREADS) {
+      const int r = idx / GD_T, d = idx % GD_T;
+      const bool in = d < n;
+      const long long g = (((long long)c * 64 + r) * H + h) * dk + d0 + d;
+      sq[r * GD_LD + d] = in ? (float)q[g] : 0.f;
+      sk[r * GD_LD + d] = in ? __bfloat162float(k[g]) : 0.f;
+      sb[r * GD_LD + d] = in ? b[g] * 1.4426950408889634f : 0.f;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int d = 0; d < GD_T / 4; ++d) {
+      const float4 a4 = qi[d], k4 = kj[d], x = bi[d], y = bj[d];
+      acc = fmaf(a4.x * k4.x, exp2f(x.x - y.x), acc);
+      acc = fmaf(a4.y * k4.y, exp2f(x.y - y.y), acc);
+      acc = fmaf(a4.z * k4.z, exp2f(x.z - y.z), acc);
+      acc = fmaf(a4.w * k4.w, exp2f(x.w - y.w), acc);
+    }
+  }
+  __nv_bfloat16* o = A + (long long)ch * 4096;
+  o[(sub * 16 + i) * 64 + sub * 16 + j] = __float2bfloat16(acc * scale);
+  // the rest of the matrix: sub-blocks to the left from the GEMM, zeros to the right (16-byte pieces), zeros above the diagonal
+  for (int idx = threadIdx.x; idx < 64 * 8; idx += GD_THREADS) {
+    const int r = idx >> 3, c8 = (idx & 7) * 8, I = r >> 4;
+    if ((c8 >> 4) == I) continue;
+    uint4 v = make_uint4(0u, 0u, 0u, 0u);
+    if (c8 < 16 * I) v = *reinterpret_cast<const uint4*>(blk + ((((long long)c * 3 + I - 1) * H + h) * 16 + (r & 15)) * 48 + c8);
+    *reinterpret_cast<uint4*>(o + r * 64 + c8) = v;
+  }
+  for (int idx = threadIdx.x; idx < 4 * 256; idx += GD_THREADS) {
+    const int I = idx >> 8, r = (idx >> 4) & 15, cc = idx & 15;
+    if (cc > r) o[(I * 16 + r) * 64 + I * 16 + cc] = __float2bfloat16(0.f);
+  }
+}
+
+// The whole channel-wise backward of a chunk: diagonal sub-blocks and preparation.  A thread owns one channel of one (chunk,
+// head); per sub-block its 16 rows of q, k and b sit in registers and each of the 136 pairs costs one exponential that serves
+// dq and dk (the pairwise kernel took one for each, read its operands from shared memory, and added into fp32 arrays that
+// others had to clear, convert and add up: 0.66 ms + 0.44 ms + about 0.6 ms of passes at 65,536 tokens, 4 heads of 128).
+//   dq_id = scale sum_{j<=i} dA_ij k_jd e^{b_id-b_jd} + dqbar_id scale e^{b_id} + dqt_id e^{b_id-r_I}
+//   dk_jd = scale sum_{i>=j} dA_ij q_id e^{b_id-b_jd} + dkhat_jd e^{b_last-b_jd} + sum_I dk3[I]_jd e^{r_I-b_jd}
+//   db    = q dq - k dk (+ what enters through b_last: khat and alpha), dg = reverse cumulative sum of db
+// dA: bf16 [NC, H, 64, 64] (only the diagonal sub-blocks are read).
+__global__ void __launch_bounds__(128, 3) gla_bwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+                                                      const float* __restrict__ b, const __nv_bfloat16* __restrict__ dA,
+                                                      const __nv_bfloat16* __restrict__ dkhat, const __nv_bfloat16* __restrict__ dqbar,
+                                                      const __nv_bfloat16* __restrict__ dqt, const __nv_bfloat16* __restrict__ dk3,
+                                                      const float* __restrict__ dalpha, __nv_bfloat16* __restrict__ dq,
+                                                      __nv_bfloat16* __restrict__ dk_, float* __restrict__ dg, int H, int dk, float scale) {
+  __shared__ float sA[4][16][16];
+  __shared__ float sgb[64][128];
+  const int d = blockIdx.y * 128 + threadIdx.x;
+  const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
+  for (int idx = threadIdx.x; idx < 1024; idx += 128) {
+    const int I = idx >> 8, r = (idx >> 4) & 15, cc = idx & 15;
+    sA[I][r][cc] = cc <= r ? __bfloat162float(dA[((long long)ch * 64 + I * 16 + r) * 64 + I * 16 + cc]) * scale : 0.f;
+  }
+  __syncthreads();
+  if (d >= dk) return;
+  constexpr float LOG2E = 1.4426950408889634f;
+  const long long rs = (long long)H * dk;
+  const long long base = ((long long)c * 64 * H + h) * dk + d;
+  const long long k3base = (((long long)c * 3) * 48 * H + h) * dk + d;
+  float r[4];
+#pragma unroll
+  for (int I = 0; I < 4; ++I) r[I] = b[base + (long long)(16 * I) * rs] * LOG2E;
+  const float b_last = b[base + 63 * rs] * LOG2E;
+  float acc_last = 0.f;
+#pragma unroll 1
+  for (int I = 0; I < 4; ++I) {
+    float qv[16], kv[16], bv[16], gq[16], gk[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const long long off = base + (long long)(I * 16 + i) * rs;
+      qv[i] = __bfloat162float(q[off]);
+      kv[i] = __bfloat162float(k[off]);
+      bv[i] = b[off] * LOG2E;
+      gq[i] = gk[i] = 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) {
+        const float t = i == j ? sA[I][i][j] : sA[I][i][j] * exp2f(bv[i] - bv[j]);
+        gq[i] = fmaf(t, kv[j], gq[i]);
+        gk[j] = fmaf(t, qv[i], gk[j]);
+      }
+    const float rI = r[0] * (I == 0) + r[1] * (I == 1) + r[2] * (I == 2) + r[3] * (I == 3);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const long long off = base + (long long)(I * 16 + i) * rs;
+      const float g_khat = __bfloat162float(dkhat[off]) * exp2f(b_last - bv[i]);
+      gq[i] = fmaf(__bfloat162float(dqbar[off]), exp2f(bv[i]) * scale, gq[i]);
+      if (I > 0) gq[i] = fmaf(__bfloat162float(dqt[off]), exp2f(bv[i] - rI), gq[i]);
+      gk[i] += g_khat;
+      acc_last = fmaf(g_khat, kv[i], acc_last);
+      if (I < 3) {
+#pragma unroll
+        for (int J = 1; J <= 3; ++J)
+          if (J > I) gk[i] = fmaf(__bfloat162float(dk3[k3base + ((long long)(J - 1) * 48 + I * 16 + i) * rs]), exp2f(r[J] - bv[i]), gk[i]);
+      }
+      dq[off] = __float2bfloat16(gq[i]);
+      dk_[off] = __float2bfloat16(gk[i]);
+      sgb[I * 16 + i][threadIdx.x] = qv[i] * gq[i] - kv[i] * gk[i];
+    }
+  }
+  float tail = acc_last + dalpha[(long long)ch * dk + d] * exp2f(b_last);  // gradient of b_last
+#pragma unroll 8
+  for (int i = 63; i >= 0; --i) {
+    tail += sgb[i][threadIdx.x];
+    dg[base + i * rs] = tail;
   }
 }
 
@@ -172,31 +616,33 @@ __global__ void __launch_bounds__(256) gla_diag_bwd_kernel(const __nv_bfloat16* 
 
 extern "C" {
 
-int fb_gla_diag_fwd(const void* q, const void* k, const float* b, float* A, int NC, int H, int dk, float scale,
-                    cudaStream_t stream) {
+int fb_gla_scores(const void* q, int q32, const void* k, const float* b, const void* blk, void* A, int NC, int H, int dk, float scale,
+                  cudaStream_t stream) {
   if (NC <= 0) return 0;
-  const int smem = 3 * 16 * (dk + 1) * 4;
-  static int configured = 0;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(gla_diag_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
-    configured = smem;
+  constexpr int smem = 3 * 64 * GD_LD * 4;
+  static bool configured = false;
+  if (!configured) {
+    if (cudaFuncSetAttribute(gla_scores_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
+        cudaFuncSetAttribute(gla_scores_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+      return -2;
+    configured = true;
   }
-  gla_diag_fwd_kernel<<<dim3(NC * H, 4), 256, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, b, A, H, dk, scale);
-  return fb::launch_ok("gla_diag_fwd_kernel");
+  if (q32)
+    gla_scores_kernel<<<NC * H, GD_THREADS, smem, stream>>>((const float*)q, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)blk,
+                                                           (__nv_bfloat16*)A, H, dk, scale);
+  else
+    gla_scores_kernel<<<NC * H, GD_THREADS, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)blk,
+                                                           (__nv_bfloat16*)A, H, dk, scale);
+  return fb::launch_ok("gla_scores_kernel");
 }
 
-int fb_gla_diag_bwd(const void* q, const void* k, const float* b, const float* dA, float* dq, float* dk_, float* db, int NC,
-                    int H, int dk, float scale, cudaStream_t stream) {
+int fb_gla_bwd(const void* q, const void* k, const float* b, const void* dA, const void* dkhat, const void* dqbar, const void* dqt,
+               const void* dk3, const float* dalpha, void* dq, void* dk_, float* dg, int NC, int H, int dk, float scale, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  const int smem = 3 * 16 * (dk + 1) * 4 + 256 * 4;
-  static int configured = 0;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(gla_diag_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
-    configured = smem;
-  }
-  gla_diag_bwd_kernel<<<dim3(NC * H, 4), 256, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, b, dA, dq, dk_, db,
-                                                             H, dk, scale);
-  return fb::launch_ok("gla_diag_bwd_kernel");
+  gla_bwd_kernel<<<dim3(NC * H, (dk + 127) / 128), 128, 0, stream>>>(
+      (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)dA, (const __nv_bfloat16*)dkhat, (const __nv_bfloat16*)dqbar,
+      (const __nv_bfloat16*)dqt, (const __nv_bfloat16*)dk3, dalpha, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk_, dg, H, dk, scale);
+  return fb::launch_ok("gla_bwd_kernel");
 }
 
 }  // extern "C"
@@ -447,62 +893,71 @@ extern "C" int fb_pair_dot(const void* x, const void* y, float* out, long long B
   return fb::launch_ok("pair_dot_kernel");
 }
 
-// Whole elementwise chunk-state recurrence of one document in ONE launch (no transition matrix):
-//   forward  X[c+1] = alpha[c] * X[c] + X[c+1]   for c = first .. last-1        (X[first] is the zero initial state)
-//   reverse  X[c]   = alpha[c] * X[c+1] + X[c]   for c = last-1 .. first
-// Each thread owns four state elements of one (document, head) and carries them in registers across the chunks, so the
-// fp32 array is read once and written once.  X: [NC + 1, H, rows, cols] fp32, X16 its bf16 mirror;
-// alpha: [NC, H] (per_row = 0) or [NC, H, rows] (per_row = 1).  Grid: (ceil(H*rows*cols/4 / 256), documents).
+// ---------------------------------------------------------------------------------------------------------------
+// Chunk-state recurrence without a transition matrix (GLA, GSA, SSD), all chunks of every document in one launch:
+//   forward   out[c] = state entering chunk c:            s = 0;  out[c] = s;  s = alpha[c] s + x[c],   c ascending
+//   reverse   out[c] = adjoint of the state leaving c:    s = 0;  out[c] = s;  s = alpha[c] s + x[c],   c descending
+// x: increments (fp32) or gradients of the states (bf16) [NC, H, rows, cols]; out bf16; alpha: [NC, H] (per_row = 0) or
+// [NC, H, rows] (per_row = 1).  Each thread owns four state elements of one document and carries them in registers, with
+// four chunks' loads in flight.  Nothing but the bf16 states is written: writing the running fp32 state beside them, which
+// nobody reads, and copying bf16 gradients to fp32 first took twice the traffic.
+// Grid: (ceil(H*rows*cols/4 / 256), documents).
 namespace {
+template <typename TIn>
 __global__ void __launch_bounds__(256) state_scan_kernel(const long long* __restrict__ first, const long long* __restrict__ last,
-                                                         const float* __restrict__ alpha, int per_row, float* __restrict__ X,
-                                                         __nv_bfloat16* __restrict__ X16, int H, int rows, int cols, int reverse) {
+                                                         const float* __restrict__ alpha, int per_row, const TIn* __restrict__ X,
+                                                         __nv_bfloat16* __restrict__ out, int H, int rows, int cols, int reverse) {
   const long long per_chunk = (long long)H * rows * cols;
   const long long e = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
   if (e >= per_chunk) return;
   const int doc = blockIdx.y;
-  const long long c0 = first[doc], c1 = last[doc];
+  const long long c0 = first[doc];
+  const int cnt = (int)(last[doc] - c0) + 1;
   const int h = (int)(e / ((long long)rows * cols));
   const int row = (int)((e / cols) % rows);
-  auto a_of = [&](long long c) { return per_row ? alpha[(c * H + h) * rows + row] : alpha[c * H + h]; };
-  auto store16 = [&](long long off, const float4& v) {
-    __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-    uint2 q;
-    q.x = *reinterpret_cast<uint32_t*>(&lo);
-    q.y = *reinterpret_cast<uint32_t*>(&hi);
-    *reinterpret_cast<uint2*>(X16 + off) = q;
-  };
-  if (!reverse) {
-    float4 s = *reinterpret_cast<const float4*>(X + c0 * per_chunk + e);
-    for (long long c = c0; c < c1; ++c) {
-      const float al = a_of(c);
-      const long long off = (c + 1) * per_chunk + e;
-      float4 d = *reinterpret_cast<const float4*>(X + off);
-      s.x = fmaf(al, s.x, d.x); s.y = fmaf(al, s.y, d.y); s.z = fmaf(al, s.z, d.z); s.w = fmaf(al, s.w, d.w);
-      *reinterpret_cast<float4*>(X + off) = s;
-      store16(off, s);
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i0 = 0; i0 < cnt; i0 += 4) {
+    float4 x[4];
+    float al[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i0 + k >= cnt) break;
+      const long long c = c0 + (reverse ? cnt - 1 - i0 - k : i0 + k);
+      al[k] = per_row ? alpha[(c * H + h) * rows + row] : alpha[c * H + h];
+      if constexpr (sizeof(TIn) == 4) {
+        x[k] = *reinterpret_cast<const float4*>(X + c * per_chunk + e);
+      } else {
+        const uint2 q = *reinterpret_cast<const uint2*>(X + c * per_chunk + e);
+        const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.x));
+        const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&q.y));
+        x[k] = make_float4(lo.x, lo.y, hi.x, hi.y);
+      }
     }
-  } else {
-    float4 s = *reinterpret_cast<const float4*>(X + c1 * per_chunk + e);
-    for (long long c = c1 - 1; c >= c0; --c) {
-      const float al = a_of(c);
-      const long long off = c * per_chunk + e;
-      float4 d = *reinterpret_cast<const float4*>(X + off);
-      s.x = fmaf(al, s.x, d.x); s.y = fmaf(al, s.y, d.y); s.z = fmaf(al, s.z, d.z); s.w = fmaf(al, s.w, d.w);
-      *reinterpret_cast<float4*>(X + off) = s;
-      store16(off, s);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (i0 + k >= cnt) break;
+      const long long c = c0 + (reverse ? cnt - 1 - i0 - k : i0 + k);
+      const __nv_bfloat162 lo = __floats2bfloat162_rn(s.x, s.y), hi = __floats2bfloat162_rn(s.z, s.w);
+      uint2 q;
+      q.x = *reinterpret_cast<const uint32_t*>(&lo);
+      q.y = *reinterpret_cast<const uint32_t*>(&hi);
+      *reinterpret_cast<uint2*>(out + c * per_chunk + e) = q;
+      s.x = fmaf(al[k], s.x, x[k].x); s.y = fmaf(al[k], s.y, x[k].y); s.z = fmaf(al[k], s.z, x[k].z); s.w = fmaf(al[k], s.w, x[k].w);
     }
   }
 }
 }  // namespace
 
-extern "C" int fb_state_scan(const long long* first, const long long* last, int n_docs, const float* alpha, int per_row, float* X,
-                             void* X16, int H, int rows, int cols, int reverse, cudaStream_t stream) {
+extern "C" int fb_state_scan(const long long* first, const long long* last, int n_docs, const float* alpha, int per_row, const void* X,
+                             int x16, void* out, int H, int rows, int cols, int reverse, cudaStream_t stream) {
   if (n_docs <= 0) return 0;
   if (cols & 3) return -2;
   const long long per_chunk = (long long)H * rows * cols;
   dim3 grid((unsigned)((per_chunk / 4 + 255) / 256), (unsigned)n_docs);
-  state_scan_kernel<<<grid, 256, 0, stream>>>(first, last, alpha, per_row, X, (__nv_bfloat16*)X16, H, rows, cols, reverse);
+  if (x16)
+    state_scan_kernel<<<grid, 256, 0, stream>>>(first, last, alpha, per_row, (const __nv_bfloat16*)X, (__nv_bfloat16*)out, H, rows, cols, reverse);
+  else
+    state_scan_kernel<<<grid, 256, 0, stream>>>(first, last, alpha, per_row, (const float*)X, (__nv_bfloat16*)out, H, rows, cols, reverse);
   return fb::launch_ok("state_scan_kernel");
 }
 
@@ -556,63 +1011,6 @@ __global__ void __launch_bounds__(128) gla_prep_fwd_kernel(const __nv_bfloat16* 
   }
 }
 
-// Backward of the preparation.  Null gradient pointers count as zero.  dg receives the gradient of the log decay:
-// db_i collects every use of b_i, and g_j feeds b_i for all i >= j (and b_last), hence the reverse cumulative sum.
-__global__ void __launch_bounds__(128) gla_prep_bwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                                                           const float* __restrict__ b, const __nv_bfloat16* __restrict__ dkhat,
-                                                           const __nv_bfloat16* __restrict__ dqbar, const __nv_bfloat16* __restrict__ dqt,
-                                                           const __nv_bfloat16* __restrict__ dk3, const float* __restrict__ dalpha,
-                                                           const float* __restrict__ db_in, __nv_bfloat16* __restrict__ dq,
-                                                           __nv_bfloat16* __restrict__ dk_, float* __restrict__ dg, int H, int dk,
-                                                           float scale) {
-  const int d = blockIdx.y * 128 + threadIdx.x;
-  if (d >= dk) return;
-  const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
-  const long long rs = (long long)H * dk;
-  const long long base = ((long long)c * 64 * H + h) * dk + d;
-  const long long k3base = (((long long)c * 3) * 48 * H + h) * dk + d;
-  float r[4];
-#pragma unroll
-  for (int I = 0; I < 4; ++I) r[I] = b[base + (long long)(16 * I) * rs];
-  const float b_last = b[base + 63 * rs];
-  float acc_last = 0.f;
-#pragma unroll 4
-  for (int i = 0; i < 64; ++i) {
-    const long long off = base + i * rs;
-    const float bi = b[off];
-    const float qi = __bfloat162float(q[off]), ki = __bfloat162float(k[off]);
-    const float e = __expf(bi) * scale, ek = __expf(b_last - bi), et = __expf(bi - r[i >> 4]);
-    const float g_qbar = dqbar ? __bfloat162float(dqbar[off]) : 0.f;
-    const float g_qt = dqt ? __bfloat162float(dqt[off]) : 0.f;
-    const float g_khat = dkhat ? __bfloat162float(dkhat[off]) : 0.f;
-    float gq = g_qbar * e + g_qt * et;
-    float gk = g_khat * ek;
-    float gb = qi * gq - g_khat * ek * ki;
-    acc_last += g_khat * ek * ki;
-    if (dk3 != nullptr && i < 48) {
-#pragma unroll
-      for (int I = 1; I <= 3; ++I) {
-        if (i < 16 * I) {
-          const float t = __bfloat162float(dk3[k3base + ((long long)(I - 1) * 48 + i) * rs]) * __expf(r[I] - bi);
-          gk += t;
-          gb -= t * ki;
-        }
-      }
-    }
-    if (db_in != nullptr) gb += db_in[off];
-    dq[off] = __float2bfloat16(gq);
-    dk_[off] = __float2bfloat16(gk);
-    dg[off] = gb;
-  }
-  float tail = acc_last + (dalpha ? dalpha[(long long)ch * dk + d] * __expf(b_last) : 0.f);  // gradient of b_last
-#pragma unroll 8
-  for (int i = 63; i >= 0; --i) {
-    const long long off = base + i * rs;
-    tail += dg[off];
-    dg[off] = tail;
-  }
-}
-
 }  // namespace
 
 extern "C" {
@@ -624,17 +1022,6 @@ int fb_gla_prep_fwd(const void* q, const void* k, const float* g, float* b, void
   gla_prep_fwd_kernel<<<grid, 128, 0, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, g, b, (__nv_bfloat16*)khat,
                                                 (__nv_bfloat16*)qbar, (__nv_bfloat16*)qt, (__nv_bfloat16*)k3, alpha, H, dk, scale);
   return fb::launch_ok("gla_prep_fwd_kernel");
-}
-
-int fb_gla_prep_bwd(const void* q, const void* k, const float* b, const void* dkhat, const void* dqbar, const void* dqt,
-                    const void* dk3, const float* dalpha, const float* db_in, void* dq, void* dk_, float* dg, int NC, int H,
-                    int dk, float scale, cudaStream_t stream) {
-  if (NC <= 0) return 0;
-  dim3 grid(NC * H, (dk + 127) / 128);
-  gla_prep_bwd_kernel<<<grid, 128, 0, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)dkhat,
-                                                (const __nv_bfloat16*)dqbar, (const __nv_bfloat16*)dqt, (const __nv_bfloat16*)dk3,
-                                                dalpha, db_in, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk_, dg, H, dk, scale);
-  return fb::launch_ok("gla_prep_bwd_kernel");
 }
 
 }  // extern "C"
@@ -781,75 +1168,198 @@ int fb_scalar_prep_bwd(const void* q, const void* k, const float* b, const void*
 }  // extern "C"
 
 // ---------------------------------------------------------------------------------------------------------------
-// Value-side decay (first pass of gated slot attention), diagonal 16 x 16 sub-blocks evaluated pairwise:
-//   o[i, c] = sum_{j <= i, same sub-block} P[i, j] v[j, c] exp(b[i, c] - b[j, c])
-// P: [NC, H, 64, 64] fp32 (causal scores), v: [NC, 64, H, M] bf16, b: [NC, 64, H, M] fp32, o: [NC, 64, H, M] fp32.
-// Grid (NC * H, 4), 256 threads.  (fla/ops/gsa/chunk.py evaluates the same sub-blocks inside its intra-chunk kernel.)
+// First pass of gated slot attention: o_ic = scale sum_{j<=i} (q_i . k_j) v_jc exp(b_ic - b_jc), a decay along the VALUE
+// dimension c (the slots, M of them), then a softmax over the slots (fla/ops/gsa/chunk.py:826-871).  64-token chunks, layouts
+// as for GLA: v [NC, 64, H, M] bf16; g, b, o: [NC, 64, H, M] fp32; P = tril(q k^T) [NC, H, 64, 64].  A thread owns a channel of
+// a (chunk, head) and keeps 16 rows in registers; the products of rows across sub-blocks and chunks come from batched
+// GEMMs.  These kernels are everything between the GEMMs: as a chain of elementwise passes over fp32 [.., H, M] arrays and
+// pairwise kernels over padded matrices this pass took 236 launches with the rest of the layer and 2.5 ms at 32,767 tokens.
 namespace {
 
-__global__ void __launch_bounds__(256) vdecay_diag_fwd_kernel(const float* __restrict__ P, const __nv_bfloat16* __restrict__ v,
-                                                              const float* __restrict__ b, float* __restrict__ o, int H, int M) {
-  extern __shared__ float sm[];
-  float* sP = sm;            // 16 x 16
-  float* sv = sP + 256;      // 16 x M
-  float* sb = sv + 16 * M;   // 16 x M
-  const int ch = blockIdx.x, c = ch / H, h = ch - c * H, blk = blockIdx.y;
-  const long long row0 = (long long)c * 64 + blk * 16;
-  sP[threadIdx.x] = P[((long long)ch * 64 + blk * 16 + (threadIdx.x >> 4)) * 64 + blk * 16 + (threadIdx.x & 15)];
-  for (int idx = threadIdx.x; idx < 16 * M; idx += 256) {
-    const int r = idx / M, cc = idx - r * M;
-    const long long g = ((row0 + r) * H + h) * M + cc;
-    sv[idx] = __bfloat162float(v[g]);
-    sb[idx] = b[g];
+constexpr float VD_LOG2E = 1.4426950408889634f;
+
+// b = cumsum(g); vhat = v e^{b_last - b}; v3[I-1]_j = v_j e^{r_I - b_j} for j < 16 I (zero beyond); alpha = e^{b_last}
+__global__ void __launch_bounds__(128) vdecay_prep_kernel(const __nv_bfloat16* __restrict__ v, const float* __restrict__ g, float* __restrict__ b,
+                                                          __nv_bfloat16* __restrict__ vhat, __nv_bfloat16* __restrict__ v3, float* __restrict__ alpha,
+                                                          int H, int M, int n) {
+  const int e = blockIdx.x * 128 + threadIdx.x;  // (chunk, head, channel)
+  if (e >= n) return;
+  const int c = e / (H * M), hm = e - c * H * M;
+  const long long rs = (long long)H * M, base = (long long)c * 64 * rs + hm, base3 = (long long)c * 144 * rs + hm;
+  float run = 0.f, r[4];
+#pragma unroll 8
+  for (int i = 0; i < 64; ++i) {
+    run += g[base + i * rs];
+    b[base + i * rs] = run;
+    if ((i & 15) == 0) r[i >> 4] = run;
   }
-  __syncthreads();
-  for (int idx = threadIdx.x; idx < 16 * M; idx += 256) {
-    const int r = idx / M, cc = idx - r * M;
-    const float br = sb[idx];
-    float acc = 0.f;
-    for (int j = 0; j <= r; ++j) acc = fmaf(sP[r * 16 + j] * sv[j * M + cc], __expf(br - sb[j * M + cc]), acc);
-    o[((row0 + r) * H + h) * M + cc] = acc;
+  alpha[e] = __expf(run);
+#pragma unroll 4
+  for (int i = 0; i < 64; ++i) {
+    const float bi = b[base + i * rs], x = __bfloat162float(v[base + i * rs]);
+    vhat[base + i * rs] = __float2bfloat16(x * __expf(run - bi));
+    if (i < 48) {
+#pragma unroll
+      for (int I = 1; I <= 3; ++I) v3[base3 + ((I - 1) * 48 + i) * rs] = __float2bfloat16(i < 16 * I ? x * __expf(r[I] - bi) : 0.f);
+    }
   }
 }
 
-// dP (diagonal sub-blocks, lower triangle), dv and db of the forward above; dout: [NC, 64, H, M] fp32.
-__global__ void __launch_bounds__(256) vdecay_diag_bwd_kernel(const float* __restrict__ P, const __nv_bfloat16* __restrict__ v,
-                                                              const float* __restrict__ b, const float* __restrict__ dout,
-                                                              float* __restrict__ dP, float* __restrict__ dv, float* __restrict__ db,
-                                                              int H, int M) {
+// o = scale (o1 e^b + acc e^{b - r_I} + diagonal sub-blocks), qv = softmax over the slots (null: not wanted).  One block per (chunk, head), 4 threads
+// per slot: thread (I, c) forms the 16 rows of sub-block I.  o1 [NC, 64, H, M] fp32, acc [NC, 48, H, M] fp32 (rows 16..63).
+__global__ void vdecay_out_kernel(const float* __restrict__ o1, const float* __restrict__ acc, const float* __restrict__ P,
+                                  const __nv_bfloat16* __restrict__ v, const float* __restrict__ b, int H, int M, float scale,
+                                  float* __restrict__ o, __nv_bfloat16* __restrict__ qv) {
   extern __shared__ float sm[];
-  float* sP = sm;
-  float* sv = sP + 256;
-  float* sb = sv + 16 * M;
-  float* sd = sb + 16 * M;   // 16 x M
-  const int ch = blockIdx.x, c = ch / H, h = ch - c * H, blk = blockIdx.y;
-  const long long row0 = (long long)c * 64 + blk * 16;
-  const int pi = threadIdx.x >> 4, pj = threadIdx.x & 15;
-  const long long pidx = ((long long)ch * 64 + blk * 16 + pi) * 64 + blk * 16 + pj;
-  sP[threadIdx.x] = P[pidx];
-  for (int idx = threadIdx.x; idx < 16 * M; idx += 256) {
-    const int r = idx / M, cc = idx - r * M;
-    const long long g = ((row0 + r) * H + h) * M + cc;
-    sv[idx] = __bfloat162float(v[g]);
-    sb[idx] = b[g];
-    sd[idx] = dout[g];
+  float* sP = sm;          // [4][16][16]
+  float* so = sm + 1024;   // [64][M + 1]
+  const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
+  for (int idx = threadIdx.x; idx < 1024; idx += blockDim.x) {
+    const int I = idx >> 8, r = (idx >> 4) & 15, cc = idx & 15;
+    sP[idx] = P[((long long)ch * 64 + I * 16 + r) * 64 + I * 16 + cc];
   }
   __syncthreads();
-  float gp = 0.f;
-  if (pj <= pi) {
-    for (int cc = 0; cc < M; ++cc)
-      gp = fmaf(sd[pi * M + cc] * sv[pj * M + cc], __expf(sb[pi * M + cc] - sb[pj * M + cc]), gp);
+  const long long rs = (long long)H * M;
+  for (int t = threadIdx.x; t < 4 * M; t += blockDim.x) {
+    const int I = t / M, m = t - I * M;
+    const long long base = ((long long)c * 64 + I * 16) * rs + (long long)h * M + m;
+    const long long basea = ((long long)c * 48 + (I - 1) * 16) * rs + (long long)h * M + m;
+    float vv[16], bv[16], out[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      vv[i] = __bfloat162float(v[base + i * rs]);
+      bv[i] = b[base + i * rs] * VD_LOG2E;
+      out[i] = o1[base + i * rs] * exp2f(bv[i]);
+    }
+    if (I > 0) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) out[i] = fmaf(acc[basea + i * rs], exp2f(bv[i] - bv[0]), out[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) out[i] = fmaf(sP[I * 256 + i * 16 + j] * vv[j], i == j ? 1.f : exp2f(bv[i] - bv[j]), out[i]);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      if (qv != nullptr) so[(I * 16 + i) * (M + 1) + m] = out[i] * scale;
+      else o[base + i * rs] = out[i] * scale;
+    }
   }
-  dP[pidx] = gp;
-  for (int idx = threadIdx.x; idx < 16 * M; idx += 256) {
-    const int r = idx / M, cc = idx - r * M;
-    const float br = sb[idx];
-    float orc = 0.f, gv = 0.f;
-    for (int j = 0; j <= r; ++j) orc = fmaf(sP[r * 16 + j] * sv[j * M + cc], __expf(br - sb[j * M + cc]), orc);
-    for (int i = r; i < 16; ++i) gv = fmaf(sP[i * 16 + r] * sd[i * M + cc], __expf(sb[i * M + cc] - br), gv);
-    const long long g = ((row0 + r) * H + h) * M + cc;
-    dv[g] = gv;
-    db[g] = sd[idx] * orc - sv[idx] * gv;
+  if (qv == nullptr) return;
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+  for (int i = warp; i < 64; i += warps) {
+    const float* row = so + i * (M + 1);
+    float mx = -INFINITY, s = 0.f;
+    for (int m = lane; m < M; m += 32) mx = fmaxf(mx, row[m]);
+    for (int k = 16; k > 0; k >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, k));
+    for (int m = lane; m < M; m += 32) s += __expf(row[m] - mx);
+    for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    const float inv = 1.f / s;
+    const long long g = ((long long)c * 64 + i) * rs + (long long)h * M;
+    for (int m = lane; m < M; m += 32) {
+      o[g + m] = row[m];
+      qv[g + m] = __float2bfloat16(__expf(row[m] - mx) * inv);
+    }
+  }
+}
+
+// Softmax backward and the two scaled operands: d = p (dqv - sum p dqv) (the gradient of o; or given as d32), do = scale d (fp32),
+// do1 = do e^b, dacc = do e^{b - r_I} (rows 16..63), both bf16.  One warp per (token, head).
+__global__ void __launch_bounds__(256) vdecay_bwd1_kernel(const float* __restrict__ o, const __nv_bfloat16* __restrict__ dqv,
+                                                          const float* __restrict__ d32, const float* __restrict__ b,
+                                                          int H, int M, float scale, long long rows, float* __restrict__ dout,
+                                                          __nv_bfloat16* __restrict__ do1, __nv_bfloat16* __restrict__ dacc) {
+  const long long row = ((long long)blockIdx.x * 256 + threadIdx.x) >> 5;  // (chunk, i, head)
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  const int h = (int)(row % H);
+  const long long tok = row / H;
+  const int i = (int)(tok & 63);
+  const long long c = tok >> 6, g = row * M;
+  const float* r0 = b + ((c * 64 + (i & 48)) * H + h) * M;  // first row of the sub-block
+  float mx = -INFINITY, s = 0.f, dot = 0.f;
+  if (d32 == nullptr)
+    for (int m = lane; m < M; m += 32) mx = fmaxf(mx, o[g + m]);
+  for (int k = 16; k > 0; k >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, k));
+  for (int m = lane; d32 == nullptr && m < M; m += 32) {
+    const float e = __expf(o[g + m] - mx);
+    s += e;
+    dot = fmaf(e, __bfloat162float(dqv[g + m]), dot);
+  }
+  for (int k = 16; k > 0; k >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, k);
+    dot += __shfl_xor_sync(0xffffffffu, dot, k);
+  }
+  const float inv = 1.f / s;
+  dot *= inv;
+  for (int m = lane; m < M; m += 32) {
+    const float bi = b[g + m];
+    const float d = scale * (d32 != nullptr ? d32[g + m] : __expf(o[g + m] - mx) * inv * (__bfloat162float(dqv[g + m]) - dot));
+    dout[g + m] = d;
+    do1[g + m] = __float2bfloat16(d * __expf(bi));
+    if (i >= 16) dacc[((c * 48 + i - 16) * H + h) * M + m] = __float2bfloat16(d * __expf(bi - r0[m]));
+  }
+}
+
+// dv = dvhat e^{b_last - b} + sum_I dv3[I] e^{r_I - b} + diagonal sub-blocks;  db = do o / scale - v dv (+ what enters through
+// b_last: vhat and alpha), dg = reverse cumulative sum.  `o` carries the factor scale and so does `do`, hence the division.
+__global__ void __launch_bounds__(128) vdecay_bwd2_kernel(const float* __restrict__ P, const __nv_bfloat16* __restrict__ v, const float* __restrict__ b,
+                                                          const float* __restrict__ dout, const float* __restrict__ o,
+                                                          const __nv_bfloat16* __restrict__ dvhat, const __nv_bfloat16* __restrict__ dv3,
+                                                          const float* __restrict__ dalpha, int H, int M, float inv_scale, __nv_bfloat16* __restrict__ dv,
+                                                          float* __restrict__ dg) {
+  __shared__ float sP[4][16][16];
+  __shared__ float sgb[64][128];
+  const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
+  for (int idx = threadIdx.x; idx < 1024; idx += 128) {
+    const int I = idx >> 8, r = (idx >> 4) & 15, cc = idx & 15;
+    sP[I][r][cc] = P[((long long)ch * 64 + I * 16 + r) * 64 + I * 16 + cc];
+  }
+  __syncthreads();
+  const int m = blockIdx.y * 128 + threadIdx.x;
+  if (m >= M) return;
+  const long long rs = (long long)H * M, base = (long long)c * 64 * rs + (long long)h * M + m, base3 = (long long)c * 144 * rs + (long long)h * M + m;
+  float r[4];
+#pragma unroll
+  for (int I = 0; I < 4; ++I) r[I] = b[base + 16 * I * rs] * VD_LOG2E;
+  const float b_last = b[base + 63 * rs] * VD_LOG2E;
+  float acc_last = 0.f;
+#pragma unroll 1
+  for (int I = 0; I < 4; ++I) {
+    float bv[16], dd[16], gv[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const long long off = base + (I * 16 + i) * rs;
+      bv[i] = b[off] * VD_LOG2E;
+      dd[i] = dout[off];
+      gv[i] = 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+#pragma unroll
+      for (int j = 0; j <= i; ++j) gv[j] = fmaf(sP[I][i][j] * dd[i], i == j ? 1.f : exp2f(bv[i] - bv[j]), gv[j]);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const long long off = base + (I * 16 + i) * rs;
+      const float x = __bfloat162float(v[off]);
+      const float gl = __bfloat162float(dvhat[off]) * exp2f(b_last - bv[i]);
+      gv[i] += gl;
+      acc_last = fmaf(gl, x, acc_last);
+      if (I < 3) {
+#pragma unroll
+        for (int J = 1; J <= 3; ++J)
+          if (J > I) gv[i] = fmaf(__bfloat162float(dv3[base3 + ((J - 1) * 48 + I * 16 + i) * rs]), exp2f(r[J] - bv[i]), gv[i]);
+      }
+      dv[off] = __float2bfloat16(gv[i]);
+      sgb[I * 16 + i][threadIdx.x] = dd[i] * o[off] * inv_scale - x * gv[i];
+    }
+  }
+  float tail = acc_last + dalpha[(long long)ch * M + m] * exp2f(b_last);
+#pragma unroll 8
+  for (int i = 63; i >= 0; --i) {
+    tail += sgb[i][threadIdx.x];
+    dg[base + i * rs] = tail;
   }
 }
 
@@ -857,29 +1367,38 @@ __global__ void __launch_bounds__(256) vdecay_diag_bwd_kernel(const float* __res
 
 extern "C" {
 
-int fb_vdecay_diag_fwd(const float* P, const void* v, const float* b, float* o, int NC, int H, int M, cudaStream_t stream) {
+int fb_vdecay_prep(const void* v, const float* g, float* b, void* vhat, void* v3, float* alpha, int NC, int H, int M, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  const int smem = (256 + 2 * 16 * M) * 4;
-  static int configured = 0;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(vdecay_diag_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
-    configured = smem;
-  }
-  vdecay_diag_fwd_kernel<<<dim3(NC * H, 4), 256, smem, stream>>>(P, (const __nv_bfloat16*)v, b, o, H, M);
-  return fb::launch_ok("vdecay_diag_fwd_kernel");
+  const int n = NC * H * M;
+  vdecay_prep_kernel<<<(n + 127) / 128, 128, 0, stream>>>((const __nv_bfloat16*)v, g, b, (__nv_bfloat16*)vhat, (__nv_bfloat16*)v3, alpha, H, M, n);
+  return fb::launch_ok("vdecay_prep_kernel");
 }
 
-int fb_vdecay_diag_bwd(const float* P, const void* v, const float* b, const float* dout, float* dP, float* dv, float* db, int NC,
-                       int H, int M, cudaStream_t stream) {
+int fb_vdecay_out(const float* o1, const float* acc, const float* P, const void* v, const float* b, int NC, int H, int M, float scale, float* o,
+                  void* qv, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  const int smem = (256 + 3 * 16 * M) * 4;
-  static int configured = 0;
-  if (smem > configured) {
-    if (cudaFuncSetAttribute(vdecay_diag_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -2;
-    configured = smem;
-  }
-  vdecay_diag_bwd_kernel<<<dim3(NC * H, 4), 256, smem, stream>>>(P, (const __nv_bfloat16*)v, b, dout, dP, dv, db, H, M);
-  return fb::launch_ok("vdecay_diag_bwd_kernel");
+  if (qv != nullptr && M > 512) return -2;
+  const int smem = (1024 + (qv != nullptr ? 64 * (M + 1) : 0)) * 4;
+  if (cudaFuncSetAttribute(vdecay_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -3;
+  vdecay_out_kernel<<<NC * H, 256, smem, stream>>>(o1, acc, P, (const __nv_bfloat16*)v, b, H, M, scale, o, (__nv_bfloat16*)qv);
+  return fb::launch_ok("vdecay_out_kernel");
+}
+
+int fb_vdecay_bwd1(const float* o, const void* dqv, const float* d32, const float* b, int NC, int H, int M, float scale, float* dout, void* do1, void* dacc,
+                   cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  const long long rows = (long long)NC * 64 * H;
+  vdecay_bwd1_kernel<<<(unsigned)((rows * 32 + 255) / 256), 256, 0, stream>>>(o, (const __nv_bfloat16*)dqv, d32, b, H, M, scale, rows, dout,
+                                                                              (__nv_bfloat16*)do1, (__nv_bfloat16*)dacc);
+  return fb::launch_ok("vdecay_bwd1_kernel");
+}
+
+int fb_vdecay_bwd2(const float* P, const void* v, const float* b, const float* dout, const float* o, const void* dvhat, const void* dv3,
+                   const float* dalpha, int NC, int H, int M, float inv_scale, void* dv, float* dg, cudaStream_t stream) {
+  if (NC <= 0) return 0;
+  vdecay_bwd2_kernel<<<dim3(NC * H, (M + 127) / 128), 128, 0, stream>>>(P, (const __nv_bfloat16*)v, b, dout, o, (const __nv_bfloat16*)dvhat,
+                                                                        (const __nv_bfloat16*)dv3, dalpha, H, M, inv_scale, (__nv_bfloat16*)dv, dg);
+  return fb::launch_ok("vdecay_bwd2_kernel");
 }
 
 }  // extern "C"

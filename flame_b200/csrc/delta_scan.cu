@@ -8,7 +8,7 @@
 // (document, head, 128-wide slice of dv), so each CTA owns one such triple and walks its chunks with the state resident:
 // fp32 in tensor memory, a bf16 copy in shared memory as the B operand of the next step's MMA.  One step is
 //   T = op(M_c) S16          one tcgen05 product, A tiles streamed by TMA through a two-stage ring
-//   S = alpha_c S - T + add  by the four epilogue warps (a thread owns state rows r and r + 128), written back to tensor
+//   S = alpha_c S - T + add  by the eight epilogue warps (a thread owns half of state rows r and r + 128), written back to tensor
 //                            memory, to shared memory (bf16, the MN-major B layout) and to global memory (bf16: the state
 //                            that the output stage and the backward pass read).
 // It replaces one batched-GEMM launch per chunk position (about 20 us each, 2 x 63 of them per layer at 4096-token
@@ -23,12 +23,18 @@ namespace {
 
 constexpr int BN = 128;     // dv columns per CTA
 constexpr int STAGES = 2;
+// warp 0 TMA, warp 1 MMA, warps 2..9 the state update: two warps per tensor-memory lane quarter, half of the columns each.  A
+// step is a chain (product -> update -> operand of the next product), so the update's own length counts in full: with one
+// warp per quarter a step took 5.8 us (0.37 ms per direction for 28 documents, 65,536 tokens, 8 heads of 128).
+constexpr int THREADS = 320;
+constexpr int CW = BN / 2;  // columns of a thread
 
 struct ScanParams {
   const int* first;        // [n_docs] first chunk of every document
   const int* last;         // [n_docs] last chunk
   int n_docs, H, NC, dk, dv;
-  int reverse;
+  int reverse, shift;      // shift (reverse only): chunk c of `out` receives the adjoint of the state LEAVING it, L_{c+1} (0 at
+                           // a document's last chunk), every chunk is written and L of the first chunk is not computed
   const float* alpha;      // [NC, H]
   const __nv_bfloat16* add;  // forward: B [NC, H, dk, dv]; reverse: G [NC (+1), H, dk, dv]
   __nv_bfloat16* out;      // forward: S16 [NC + 1, H, dk, dv] (chunk c + 1 receives the state after chunk c);
@@ -51,7 +57,7 @@ __device__ __forceinline__ uint32_t sw128(int row, int col) {  // byte offset in
 }
 
 template <int DK>
-__global__ void __launch_bounds__(192, DK == 128 ? 2 : 1)
+__global__ void __launch_bounds__(THREADS, DK == 128 ? 2 : 1)
 delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
   using L = Smem<DK>;
   constexpr int HALVES = DK / 128;
@@ -59,7 +65,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
   constexpr uint32_t TCOLS = HALVES * 2 * BN;  // T and the fp32 state, per half
   const int vt = blockIdx.x, head = blockIdx.y, doc = blockIdx.z;
   const int c_first = p.first[doc], c_last = p.last[doc];
-  const int n_steps = c_last - c_first;   // chunks that have a successor
+  const int n_succ = c_last - c_first;    // chunks that have a successor
+  const int n_steps = p.shift ? max(n_succ - 1, 0) : n_succ;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   extern __shared__ uint8_t smem_raw[];
@@ -84,7 +91,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(t_full, 1);
-    mbar_init(s_ready, 128);
+    mbar_init(s_ready, THREADS - 64);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmM);
@@ -158,6 +165,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
   } else {
     const int quarter = warp & 3;
     const int r = quarter * 32 + lane;
+    const int c_lo = ((warp - 2) >> 2) * CW, c_hi = c_lo + CW;
     const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
     bool ok = true;
     // initial state: forward 0; reverse G[last] (which is also what L16[last] holds)
@@ -168,7 +176,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
         const int row = h * 128 + r;
         const __nv_bfloat16* src = p.reverse ? state_ptr(p.add, c_init, row) : nullptr;
 #pragma unroll 1
-        for (int c0 = 0; c0 < BN; c0 += 32) {
+        for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
           uint32_t st[32];
           uint4 packed[4];
 #pragma unroll
@@ -188,11 +196,19 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
         }
       }
       tmem_st_wait();
-      if (!p.reverse) {  // the state entering the first chunk is zero
-        __nv_bfloat16* dst0 = const_cast<__nv_bfloat16*>(state_ptr(p.out, c_first, 0));
+      if (p.shift && n_succ > 0) {
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h) {
+          const __nv_bfloat16* src = state_ptr(p.add, c_last, h * 128 + r);
+          __nv_bfloat16* dst = const_cast<__nv_bfloat16*>(state_ptr(p.out, c_last - 1, h * 128 + r));
+          for (int c0 = c_lo; c0 < c_hi; c0 += 8) *reinterpret_cast<uint4*>(dst + c0) = *reinterpret_cast<const uint4*>(src + c0);
+        }
+      }
+      if (!p.reverse || p.shift) {  // the state entering the first chunk is zero, and so is the adjoint of the one leaving the last
+        __nv_bfloat16* dst0 = const_cast<__nv_bfloat16*>(state_ptr(p.out, p.reverse ? c_last : c_first, 0));
 #pragma unroll
         for (int h = 0; h < HALVES; ++h)
-          for (int c0 = 0; c0 < BN; c0 += 8)
+          for (int c0 = c_lo; c0 < c_hi; c0 += 8)
             *reinterpret_cast<uint4*>(dst0 + (long long)(h * 128 + r) * p.dv + c0) = make_uint4(0u, 0u, 0u, 0u);
       }
       tc_fence_before();
@@ -201,16 +217,16 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
     }
     for (int s = 0; s < n_steps && ok; ++s) {
       const int c = p.reverse ? c_last - 1 - s : c_first + s;
-      const int c_out = p.reverse ? c : c + 1;
+      const int c_out = p.reverse ? c - p.shift : c + 1;
       const float a = __ldg(p.alpha + (long long)c * p.H + head);
       // the addend rows of this step are fetched BEFORE waiting for the product: their global-memory latency (they are
       // read once, from L2 or HBM) then overlaps the tensor-core work instead of adding to every 32-column piece
       // (the second half of a 256-row state fetches its row when its turn comes: 64 more registers would spill)
-      uint4 ad[BN / 8];
+      uint4 ad[CW / 8];
       {
-        const __nv_bfloat16* addrow = state_ptr(p.add, c, r);
+        const __nv_bfloat16* addrow = state_ptr(p.add, c, r) + c_lo;
 #pragma unroll
-        for (int g = 0; g < BN / 8; ++g) ad[g] = __ldg(reinterpret_cast<const uint4*>(addrow + g * 8));
+        for (int g = 0; g < CW / 8; ++g) ad[g] = __ldg(reinterpret_cast<const uint4*>(addrow + g * 8));
       }
       if (!mbar_wait_warp(t_full, s & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
@@ -218,20 +234,21 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
       for (int h = 0; h < HALVES; ++h) {
         const int row = h * 128 + r;
         if (h > 0) {
-          const __nv_bfloat16* addrow = state_ptr(p.add, c, row);
+          const __nv_bfloat16* addrow = state_ptr(p.add, c, row) + c_lo;
 #pragma unroll
-          for (int g = 0; g < BN / 8; ++g) ad[g] = __ldg(reinterpret_cast<const uint4*>(addrow + g * 8));
+          for (int g = 0; g < CW / 8; ++g) ad[g] = __ldg(reinterpret_cast<const uint4*>(addrow + g * 8));
         }
         __nv_bfloat16* outrow = const_cast<__nv_bfloat16*>(state_ptr(p.out, c_out, row));
 #pragma unroll
-        for (int c0 = 0; c0 < BN; c0 += 32) {
+        for (int cc = 0; cc < CW; cc += 32) {
+          const int c0 = c_lo + cc;
           uint32_t t[32], st[32];
           tmem_ld_32x32(tmem_base + h * 2 * BN + lane_sel + c0, t);
           tmem_ld_32x32(tmem_base + h * 2 * BN + BN + lane_sel + c0, st);
           tmem_ld_wait();
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
-            const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&ad[(c0 >> 3) + g]);
+            const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&ad[(cc >> 3) + g]);
             uint4 q;
             uint32_t* qw = reinterpret_cast<uint32_t*>(&q);
 #pragma unroll
@@ -275,7 +292,7 @@ int launch_scan(const CUtensorMap& tm, const ScanParams& p, cudaStream_t stream)
     configured = true;
   }
   dim3 grid(p.dv / BN, p.H, p.n_docs);
-  kern<<<grid, 192, Smem<DK>::TOTAL, stream>>>(tm, p);
+  kern<<<grid, THREADS, Smem<DK>::TOTAL, stream>>>(tm, p);
   return fb::launch_ok("delta_scan_kernel");
 }
 
@@ -284,7 +301,8 @@ int launch_scan(const CUtensorMap& tm, const ScanParams& p, cudaStream_t stream)
 extern "C" {
 
 // M [NC, H, dk, dk], add [>= NC, H, dk, dv], out [NC + 1, H, dk, dv] bf16 contiguous; alpha [NC, H] fp32; first / last
-// [n_docs] chunk indices.  dk in {128, 256}, dv a multiple of 128.  reverse = 0 / 1 as described at the top of the file.
+// [n_docs] chunk indices.  dk in {128, 256}, dv a multiple of 128.  reverse = 0 / 1 as described at the top of the file; 2:
+// reverse with shifted output (out [NC, ...]).
 int fb_delta_scan(const void* M, const void* add, const float* alpha, void* out, const int* first, const int* last,
                   int n_docs, int H, int NC, int dk, int dv, int reverse, cudaStream_t stream) {
   if (n_docs <= 0 || NC <= 0) return 0;
@@ -293,7 +311,7 @@ int fb_delta_scan(const void* M, const void* add, const float* alpha, void* out,
   int rc = fb::make_tmap_2d(&tm, M, 2, (uint64_t)NC * H * dk, (uint64_t)dk, (uint64_t)dk, 64, 64, true);
   if (rc) return rc;
   ScanParams p;
-  p.first = first; p.last = last; p.n_docs = n_docs; p.H = H; p.NC = NC; p.dk = dk; p.dv = dv; p.reverse = reverse;
+  p.first = first; p.last = last; p.n_docs = n_docs; p.H = H; p.NC = NC; p.dk = dk; p.dv = dv; p.reverse = reverse != 0; p.shift = reverse == 2;
   p.alpha = alpha; p.add = (const __nv_bfloat16*)add; p.out = (__nv_bfloat16*)out;
   p.status = fb::status_ptr();
   return dk == 128 ? launch_scan<128>(tm, p, stream) : launch_scan<256>(tm, p, stream);

@@ -18,7 +18,7 @@ from __future__ import annotations
 
 import ctypes
 from ctypes import POINTER, c_float, c_int, c_longlong, c_void_p
-from typing import Optional
+from typing import Optional, Sequence
 
 import torch
 
@@ -28,7 +28,7 @@ from . import _lib
 class _Operand(ctypes.Structure):
     _fields_ = [("ptr", c_void_p), ("ld", c_longlong), ("stride_lo", c_longlong), ("stride_hi", c_longlong),
                 ("n_lo", c_int), ("n_hi", c_int), ("mn", c_int), ("lo_div", c_int), ("hi_offset", c_int),
-                ("hi_index", c_void_p)]
+                ("hi_index", c_void_p), ("k", c_int), ("neg", c_int)]
 
 
 class _Epilogue(ctypes.Structure):
@@ -39,11 +39,12 @@ class _Epilogue(ctypes.Structure):
                 ("add16", c_void_p), ("add16_hi_offset", c_int), ("add16_hi_index", c_void_p),
                 ("ld16", c_longlong), ("stride_lo16", c_longlong), ("stride_hi16", c_longlong),
                 ("decay", c_void_p), ("d_hi", c_longlong), ("d_lo", c_longlong), ("d_r", c_longlong),
+                ("rowscale", c_void_p), ("r_hi", c_longlong), ("r_lo", c_longlong), ("r_r", c_longlong),
                 ("alpha", c_float), ("out_mode", c_int), ("mask_mode", c_int)]
 
 
-_lib.register("fb_bgemm_bf16", [POINTER(_Operand), POINTER(_Operand), POINTER(_Epilogue), c_int, c_int, c_int, c_int,
-                                c_int, c_void_p])
+_lib.register("fb_bgemm_bf16", [POINTER(_Operand), c_int, POINTER(_Epilogue), c_int, c_int, c_int, c_int, c_int,
+                                c_void_p])
 
 MASK_NONE, MASK_TRIL, MASK_STRICT = 0, 1, 2
 
@@ -58,9 +59,9 @@ def _inner_contig(t: torch.Tensor) -> torch.Tensor:
     return t if ok else t.contiguous()
 
 
-def _operand(t: torch.Tensor, mn: bool, lo_div: int, index: Optional[torch.Tensor], offset: int) -> _Operand:
+def _operand(t: torch.Tensor, mn: bool, lo_div: int, index: Optional[torch.Tensor], offset: int, neg: bool = False) -> _Operand:
     return _Operand(t.data_ptr(), t.stride(2), t.stride(1), t.stride(0), t.shape[1], t.shape[0], int(mn), lo_div, offset,
-                    _lib.ptr(index))
+                    _lib.ptr(index), t.shape[2] if mn else t.shape[3], int(neg))
 
 
 def _mkn(a, b, a_mn, b_mn):
@@ -85,8 +86,13 @@ def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = 
           cin_offset: int = 0, a_offset: int = 0, b_offset: int = 0, n_hi: Optional[int] = None,
           n_lo: Optional[int] = None, out16_index: Optional[torch.Tensor] = None, out16_offset: int = 0,
           add16: Optional[torch.Tensor] = None, add16_index: Optional[torch.Tensor] = None,
-          add16_offset: int = 0) -> torch.Tensor:
+          add16_offset: int = 0, rowscale: Optional[torch.Tensor] = None,
+          more: Sequence[tuple] = (), sum_lo: int = 1) -> torch.Tensor:
     """``out[hi, lo] = alpha * a[hi, lo] @ b[hi, lo]^T`` (no autograd).
+
+    ``more``: up to three further products ``(a, b, a_mn, b_mn, sign)`` of the same result, added (or subtracted) in the
+    accumulator.  ``rowscale``: fp32 ``[hi, lo, M]`` (any strides), a factor per row.  ``sum_lo``: every product is summed over
+    that many consecutive lo coordinates of its operands (the heads of a group, in the accumulator too).
 
     ``a``/``b``: ``[hi, lo, rows, inner]`` bf16 views.  ``n_lo`` defaults to the larger head count; an operand with
     fewer heads is shared by ``n_lo / heads`` consecutive batches.  ``*_index`` (int32 ``[n_hi]``) select the hi
@@ -97,7 +103,9 @@ def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = 
     ``[*, lo, M, N]`` tensors with hi coordinates of their own (index / offset; default: the batch number).
     """
     M, N, K = _mkn(a, b, a_mn, b_mn)
-    n_lo = n_lo or max(a.shape[1], b.shape[1])
+    n_lo = n_lo or max(a.shape[1], b.shape[1]) // sum_lo
+    n_op = n_lo * sum_lo
+    assert not (more and (a_index is not None or b_index is not None or a_offset or b_offset))
     if n_hi is None:
         n_hi = len(a_index) if a_index is not None else (len(b_index) if b_index is not None else min(a.shape[0], b.shape[0]))
     if out is None:
@@ -112,8 +120,20 @@ def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = 
         a = _inner_contig(a)
         b = _inner_contig(b)
         assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-        ea = _operand(a, a_mn, n_lo // a.shape[1], a_index, a_offset)
-        eb = _operand(b, b_mn, n_lo // b.shape[1], b_index, b_offset)
+        ops = (_Operand * (2 + 2 * len(more)))()
+        ops[0] = _operand(a, a_mn, n_op // a.shape[1], a_index, a_offset)
+        ops[1] = _operand(b, b_mn, n_op // b.shape[1], b_index, b_offset)
+        hold = []
+        for i, (ai, bi, ai_mn, bi_mn, sign) in enumerate(more):
+            assert _mkn(ai, bi, ai_mn, bi_mn)[:2] == (M, N) and ai.dtype == bi.dtype == torch.bfloat16
+            ai, bi = _inner_contig(ai), _inner_contig(bi)
+            hold.append((ai, bi))
+            ops[2 + 2 * i] = _operand(ai, ai_mn, n_op // ai.shape[1], None, 0, sign < 0)
+            ops[3 + 2 * i] = _operand(bi, bi_mn, n_op // bi.shape[1], None, 0)
+        r_hi = r_lo = r_r = 0
+        if rowscale is not None:
+            assert rowscale.dtype == torch.float32 and rowscale.shape[-1] == M
+            r_hi, r_lo, r_r = rowscale.stride()
         if cin is not None:
             assert cin.dtype == torch.float32 and cin.stride() == out.stride()
         side = out16 if out16 is not None else add16
@@ -135,9 +155,8 @@ def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = 
                        _lib.ptr(c_index), _lib.ptr(cin), cin_offset, _lib.ptr(cin_index), _lib.ptr(gamma),
                        _lib.ptr(out16), out16_offset, _lib.ptr(out16_index), _lib.ptr(add16), add16_offset,
                        _lib.ptr(add16_index), ld16, slo16, shi16,
-                       _lib.ptr(decay), d_hi, d_lo, d_r, float(alpha), mode, int(mask))
-        rc = _lib.lib().fb_bgemm_bf16(ctypes.byref(ea), ctypes.byref(eb), ctypes.byref(ep), n_hi, n_lo, M, N, K,
-                                      _lib.stream_ptr())
+                       _lib.ptr(decay), d_hi, d_lo, d_r, _lib.ptr(rowscale), r_hi, r_lo, r_r, float(alpha), mode, int(mask))
+        rc = _lib.lib().fb_bgemm_bf16(ops, 1 + len(more), ctypes.byref(ep), n_hi, n_lo, sum_lo, M, N, _lib.stream_ptr())
         _lib.check(rc, "fb_bgemm_bf16")
         _lib.count_launch()
         return out
@@ -148,11 +167,20 @@ def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = 
         t = t[off:off + n_hi] if index is None else t[index.long() + off]
         return t.repeat_interleave(div, dim=1) if div > 1 else t
 
-    af = pick(a, a_index, n_lo // a.shape[1], a_offset).float()
-    bf = pick(b, b_index, n_lo // b.shape[1], b_offset).float()
+    af = pick(a, a_index, n_op // a.shape[1], a_offset).float()
+    bf = pick(b, b_index, n_op // b.shape[1], b_offset).float()
     af = af.transpose(-1, -2) if a_mn else af
     bf = bf if b_mn else bf.transpose(-1, -2)
-    r = torch.matmul(af, bf) * alpha
+    r = torch.matmul(af, bf)
+    for ai, bi, ai_mn, bi_mn, sign in more:
+        x = pick(ai, None, n_op // ai.shape[1], 0).float()
+        y = pick(bi, None, n_op // bi.shape[1], 0).float()
+        r = r + sign * torch.matmul(x.transpose(-1, -2) if ai_mn else x, y if bi_mn else y.transpose(-1, -2))
+    if sum_lo > 1:
+        r = r.reshape(n_hi, n_lo, sum_lo, M, N).sum(2)
+    r = r * alpha
+    if rowscale is not None:
+        r = r * rowscale[:n_hi].float()[..., None]
     if decay is not None:
         d = decay[:n_hi].float()
         r = r * (d[..., :, None] - d[..., None, :]).clamp_max(0.0 if mask else 80.0).exp()

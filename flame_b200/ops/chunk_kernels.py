@@ -7,8 +7,10 @@ import torch
 
 from . import _lib
 
-_lib.register("fb_tri_inverse", [c_void_p, c_void_p, c_void_p, c_longlong, c_void_p])
-_lib.register("fb_state_step", [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_void_p])
+_lib.register("fb_delta_inverse", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 6)
+_lib.register("fb_delta_scale", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 3)
+_lib.register("fb_delta_bwd_t", [c_void_p] * 5 + [c_int] * 3 + [c_float] + [c_void_p] * 4)
+_lib.register("fb_delta_bwd_scores", [c_void_p] * 6 + [c_int] * 3 + [c_float] + [c_void_p] * 5)
 
 
 def tri_inverse(A: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
@@ -18,43 +20,136 @@ def tri_inverse(A: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16) -> tor
     out = torch.empty(A.shape, dtype=out_dtype, device=A.device)
     n = A.numel() // 4096
     o16, o32 = (out.data_ptr(), 0) if out_dtype == torch.bfloat16 else (0, out.data_ptr())
-    _lib.check(_lib.lib().fb_tri_inverse(A.data_ptr(), o16, o32, n, _lib.stream_ptr()), "fb_tri_inverse")
+    _lib.check(_lib.lib().fb_delta_inverse(A.data_ptr(), 0, 0, n, 1, 64, o16, 0, 0, 0, o32, _lib.stream_ptr()), "fb_delta_inverse")
     _lib.count_launch()
     return out
 
 
-def state_step(idx: torch.Tensor, alpha: torch.Tensor, X: torch.Tensor, X16: torch.Tensor, reverse: bool) -> None:
-    """One chunk position of ``X[c+1] = alpha_c X[c] + X[c+1]`` (or its reverse) for the chunks in ``idx``."""
-    _, H, rows, cols = X.shape
-    per_row = 1 if alpha.dim() == 3 else 0
-    rc = _lib.lib().fb_state_step(idx.data_ptr(), idx.numel(), alpha.data_ptr(), per_row, X.data_ptr(), X16.data_ptr(), H,
-                                  rows, cols, int(reverse), _lib.stream_ptr())
-    _lib.check(rc, "fb_state_step")
+def delta_inverse(P: torch.Tensor, beta: torch.Tensor, b, bgemm):
+    """``T = (I + diag(beta) P)^-1``, ``Tu = T diag(beta)`` and, with a decay ``b``, ``Tw = T diag(beta e^b)`` (bf16) for the
+    strictly lower-triangular fp32 ``P [NC, H, C, C]``, C = 64 or 128; beta, b ``[NC, C, H]`` fp32 contiguous.  At C = 128 the
+    diagonal blocks are inverted and ``T21 = -T22 A21 T11`` comes from two batched GEMMs."""
+    NC, H, C, _ = P.shape
+    new = lambda: torch.empty(P.shape, dtype=torch.bfloat16, device=P.device)  # noqa: E731
+    T, Tu, Tw = new(), new(), None if b is None else new()
+    A21 = torch.empty(NC, H, 64, 64, dtype=torch.bfloat16, device=P.device) if C == 128 else None
+    L = _lib.lib()
+    _lib.check(L.fb_delta_inverse(P.data_ptr(), beta.data_ptr(), _lib.ptr(b), NC, H, C, T.data_ptr(), Tu.data_ptr(), _lib.ptr(Tw),
+                                  _lib.ptr(A21), 0, _lib.stream_ptr()), "fb_delta_inverse")
     _lib.count_launch()
+    if C == 128:
+        X = bgemm(T[..., 64:, 64:], A21, b_mn=True)
+        bgemm(X, T[..., :64, :64], b_mn=True, alpha=-1.0, out=T[..., 64:, :64])
+        _lib.check(L.fb_delta_scale(T.data_ptr(), beta.data_ptr(), _lib.ptr(b), NC, H, C, Tu.data_ptr(), _lib.ptr(Tw), _lib.stream_ptr()),
+                   "fb_delta_scale")
+        _lib.count_launch()
+    return T, Tu, Tw
 
 
-_lib.register("fb_gla_diag_fwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_void_p])
-_lib.register("fb_gla_diag_bwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int,
-                                  c_float, c_void_p])
+def delta_bwd_t(T, dTu, dTw, beta, b, scale: float):
+    """``dT`` (bf16) from the gradients of ``Tu`` and ``Tw``, and the parts of ``dbeta``, ``db`` (``[NC, C, H]`` fp32, times
+    ``scale``) that come from the column factors.  ``dTw`` and ``b`` are None without a decay."""
+    NC, H, C, _ = T.shape
+    dT = torch.empty_like(T)
+    dbeta = torch.empty_like(beta)
+    db = None if b is None else torch.empty_like(b)
+    _lib.check(_lib.lib().fb_delta_bwd_t(T.data_ptr(), dTu.data_ptr(), _lib.ptr(dTw), beta.data_ptr(), _lib.ptr(b), NC, H, C, float(scale),
+                                         dT.data_ptr(), dbeta.data_ptr(), _lib.ptr(db), _lib.stream_ptr()), "fb_delta_bwd_t")
+    _lib.count_launch()
+    return dT, dbeta, db
 
 
-def gla_diag_fwd(q: torch.Tensor, k: torch.Tensor, b: torch.Tensor, scale: float, A: torch.Tensor) -> None:
-    """Writes the four diagonal 16 x 16 sub-blocks of ``A [NC, H, 64, 64]`` (fp32); q, k ``[NC, 64, H, dk]`` bf16,
-    b ``[NC, 64, H, dk]`` fp32, all contiguous."""
+def delta_bwd_scores(dA, P, dQ, Q, beta, b, scale: float, dbeta, db):
+    """The bf16 operands ``g`` (of k k^T) and, with a decay, ``gq`` (of q k^T) of the dq / dk products; adds to ``dbeta`` and
+    ``db``."""
+    NC, H, C, _ = P.shape
+    g = torch.empty(P.shape, dtype=torch.bfloat16, device=P.device)
+    gq = None if b is None else torch.empty_like(g)
+    _lib.check(_lib.lib().fb_delta_bwd_scores(dA.data_ptr(), P.data_ptr(), 0 if b is None else dQ.data_ptr(), 0 if b is None else Q.data_ptr(),
+                                              beta.data_ptr(), _lib.ptr(b), NC, H, C, float(scale), g.data_ptr(), _lib.ptr(gq),
+                                              dbeta.data_ptr(), _lib.ptr(db), _lib.stream_ptr()), "fb_delta_bwd_scores")
+    _lib.count_launch()
+    return g, gq
+
+
+_lib.register("fb_group_prep_fwd", [c_void_p] * 2 + [c_int] * 4 + [c_float] + [c_void_p] * 5)
+_lib.register("fb_group_bwd1", [c_void_p] * 3 + [c_int] * 4 + [c_void_p] * 3)
+_lib.register("fb_group_bwd2", [c_void_p] * 7 + [c_int] * 4 + [c_void_p] * 3)
+
+
+def group_supported(C: int, dv: int) -> bool:
+    n = dv // 8
+    return C in (64, 128) and dv % 8 == 0 and 1 <= n <= 32 and (n & (n - 1)) == 0
+
+
+def group_prep(v, g, scale: float):
+    """``b = cumsum(g)``, ``eb = scale e^b``, ``alpha = e^{b_last}``, ``vhat = v e^{b_last - b}`` for v ``[NC, C, H, dv]`` bf16 and g
+    ``[NC, C, H]`` fp32, both contiguous."""
+    NC, C, H, dv = v.shape
+    b, eb = torch.empty_like(g), torch.empty_like(g)
+    alpha = torch.empty(NC, H, dtype=torch.float32, device=v.device)
+    vhat = torch.empty_like(v)
+    _lib.check(_lib.lib().fb_group_prep_fwd(v.data_ptr(), g.data_ptr(), NC, C, H, dv, float(scale), b.data_ptr(), eb.data_ptr(),
+                                            alpha.data_ptr(), vhat.data_ptr(), _lib.stream_ptr()), "fb_group_prep_fwd")
+    _lib.count_launch()
+    return b, eb, alpha, vhat
+
+
+def group_bwd1(do, o1, eb):
+    """``do eb`` and the row sums of ``do o1``."""
+    NC, C, H, dv = do.shape
+    dos, db = torch.empty_like(do), torch.empty_like(eb)
+    _lib.check(_lib.lib().fb_group_bwd1(do.data_ptr(), o1.data_ptr(), eb.data_ptr(), NC, C, H, dv, dos.data_ptr(), db.data_ptr(),
+                                        _lib.stream_ptr()), "fb_group_bwd1")
+    _lib.count_launch()
+    return dos, db
+
+
+def group_bwd2(dvhat, vhat, dv1, b, db, alpha, dalpha):
+    """``dv`` and ``dg`` (see ``csrc/chunk.cu: group_bwd2_kernel``)."""
+    NC, C, H, dv = vhat.shape
+    dvo, dg = torch.empty_like(vhat), torch.empty_like(b)
+    _lib.check(_lib.lib().fb_group_bwd2(dvhat.data_ptr(), vhat.data_ptr(), dv1.data_ptr(), b.data_ptr(), db.data_ptr(), alpha.data_ptr(),
+                                        dalpha.data_ptr(), NC, C, H, dv, dvo.data_ptr(), dg.data_ptr(), _lib.stream_ptr()), "fb_group_bwd2")
+    _lib.count_launch()
+    return dvo, dg
+
+
+def scores_bwd(dQ, Q, b, db):
+    """bf16 ``dQ_ij e^{b_i - b_j}`` (j <= i) and, added to ``db [NC, C, H]``, the gradient of ``b`` through ``Q``: the part of
+    ``delta_bwd_scores`` that attention without a delta rule has."""
+    NC, H, C, _ = Q.shape
+    gq = torch.empty_like(Q)
+    _lib.check(_lib.lib().fb_delta_bwd_scores(0, 0, dQ.data_ptr(), Q.data_ptr(), 0, b.data_ptr(), NC, H, C, 1.0, 0, gq.data_ptr(), 0,
+                                              db.data_ptr(), _lib.stream_ptr()), "fb_delta_bwd_scores")
+    _lib.count_launch()
+    return gq
+
+
+_lib.register("fb_gla_scores", [c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 3 + [c_float, c_void_p])
+_lib.register("fb_gla_bwd", [c_void_p] * 12 + [c_int] * 3 + [c_float, c_void_p])
+
+
+def gla_scores(q, k, b, blk, scale: float) -> torch.Tensor:
+    """bf16 ``A [NC, H, 64, 64]``: diagonal 16 x 16 sub-blocks computed here, the ones left of them from ``blk [3 NC, H, 16, 48]``
+    bf16; q (or fp32), k ``[NC, 64, H, dk]`` bf16, b fp32, all contiguous."""
     NC, _, H, dk = q.shape
-    rc = _lib.lib().fb_gla_diag_fwd(q.data_ptr(), k.data_ptr(), b.data_ptr(), A.data_ptr(), NC, H, dk, float(scale),
-                                    _lib.stream_ptr())
-    _lib.check(rc, "fb_gla_diag_fwd")
+    A = torch.empty(NC, H, 64, 64, dtype=torch.bfloat16, device=q.device)
+    _lib.check(_lib.lib().fb_gla_scores(q.data_ptr(), int(q.dtype == torch.float32), k.data_ptr(), b.data_ptr(), blk.data_ptr(), A.data_ptr(), NC, H, dk, float(scale),
+                                        _lib.stream_ptr()), "fb_gla_scores")
     _lib.count_launch()
+    return A
 
 
-def gla_diag_bwd(q, k, b, dA, dq, dk_, db, scale: float) -> None:
-    """Adds the diagonal sub-blocks' gradient contributions into fp32 ``dq, dk, db [NC, 64, H, dk]``."""
+def gla_bwd(q, k, b, dA, dkhat, dqbar, dqt, dk3, dalpha, scale: float):
+    """``dq, dk`` (bf16) and ``dg`` (fp32) of a chunk (see ``csrc/chunk.cu: gla_bwd_kernel``); every operand contiguous."""
     NC, _, H, dk = q.shape
-    rc = _lib.lib().fb_gla_diag_bwd(q.data_ptr(), k.data_ptr(), b.data_ptr(), dA.data_ptr(), dq.data_ptr(), dk_.data_ptr(),
-                                    db.data_ptr(), NC, H, dk, float(scale), _lib.stream_ptr())
-    _lib.check(rc, "fb_gla_diag_bwd")
+    dq, dk_, dg = torch.empty_like(q), torch.empty_like(k), torch.empty_like(b)
+    _lib.check(_lib.lib().fb_gla_bwd(q.data_ptr(), k.data_ptr(), b.data_ptr(), dA.data_ptr(), dkhat.data_ptr(), dqbar.data_ptr(),
+                                     dqt.data_ptr(), dk3.data_ptr(), dalpha.data_ptr(), dq.data_ptr(), dk_.data_ptr(), dg.data_ptr(), NC,
+                                     H, dk, float(scale), _lib.stream_ptr()), "fb_gla_bwd")
     _lib.count_launch()
+    return dq, dk_, dg
 
 
 _lib.register("fb_l2norm_fwd", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_float, c_void_p])
@@ -107,70 +202,44 @@ def pair_dot(x: torch.Tensor, y: torch.Tensor, per_row: bool) -> torch.Tensor:
     return out
 
 
-_lib.register("fb_state_scan", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_int,
+_lib.register("fb_state_scan", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int,
                                 c_void_p])
 
 
-def state_scan(first: torch.Tensor, last: torch.Tensor, alpha: torch.Tensor, X: torch.Tensor, X16: torch.Tensor,
-               reverse: bool) -> None:
-    """The whole recurrence ``X[c+1] = alpha_c X[c] + X[c+1]`` (or its reverse) of every document in one launch;
-    ``first`` / ``last`` are the int64 chunk ranges of the documents."""
-    _, H, rows, cols = X.shape
+def state_scan(first: torch.Tensor, last: torch.Tensor, alpha: torch.Tensor, x: torch.Tensor, reverse: bool) -> torch.Tensor:
+    """bf16 ``[NC, H, rows, cols]``: the state entering every chunk (reverse: the adjoint of the state leaving it) of the
+    recurrence ``s = alpha_c s + x_c`` over the chunks ``first .. last`` (int64) of every document, from zero; ``x`` fp32 or bf16."""
+    x = x.contiguous()
+    _, H, rows, cols = x.shape
+    out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
     per_row = 1 if alpha.dim() == 3 else 0
-    rc = _lib.lib().fb_state_scan(first.data_ptr(), last.data_ptr(), first.numel(), alpha.data_ptr(), per_row, X.data_ptr(),
-                                  X16.data_ptr(), H, rows, cols, int(reverse), _lib.stream_ptr())
+    rc = _lib.lib().fb_state_scan(first.data_ptr(), last.data_ptr(), first.numel(), alpha.data_ptr(), per_row, x.data_ptr(),
+                                  int(x.dtype == torch.bfloat16), out.data_ptr(), H, rows, cols, int(reverse), _lib.stream_ptr())
     _lib.check(rc, "fb_state_scan")
     _lib.count_launch()
+    return out
 
 
 _lib.register("fb_gla_prep_fwd", [c_void_p] * 9 + [c_int, c_int, c_int, c_float, c_void_p])
-_lib.register("fb_gla_prep_bwd", [c_void_p] * 12 + [c_int, c_int, c_int, c_float, c_void_p])
 
 
-class GlaPrep(torch.autograd.Function):
-    """One pass over a chunk's q, k, g producing the cumulative decay and every scaled operand of the GLA chunk
-    algorithm (see ``csrc/chunk.cu: gla_prep_fwd_kernel``).  q, k ``[NC, 64, H, dk]`` bf16, g ``[NC, 64, H, dk]`` fp32.
-    Returns ``(b, khat, qbar, qt, k3, alpha)``."""
-
-    @staticmethod
-    def forward(ctx, qp, kp, gp, scale):
-        qp, kp, gp = qp.contiguous(), kp.contiguous(), gp.contiguous()
-        NC, C, H, dk = qp.shape
-        assert C == 64 and qp.dtype == torch.bfloat16 and gp.dtype == torch.float32
-        dev = qp.device
-        b = torch.empty_like(gp)
-        khat, qbar, qt = torch.empty_like(kp), torch.empty_like(qp), torch.empty_like(qp)
-        k3 = torch.empty(NC, 3, 48, H, dk, dtype=torch.bfloat16, device=dev)
-        alpha = torch.empty(NC, H, dk, dtype=torch.float32, device=dev)
-        rc = _lib.lib().fb_gla_prep_fwd(qp.data_ptr(), kp.data_ptr(), gp.data_ptr(), b.data_ptr(), khat.data_ptr(),
-                                        qbar.data_ptr(), qt.data_ptr(), k3.data_ptr(), alpha.data_ptr(), NC, H, dk,
-                                        float(scale), _lib.stream_ptr())
-        _lib.check(rc, "fb_gla_prep_fwd")
-        _lib.count_launch()
-        ctx.save_for_backward(qp, kp, b)
-        ctx.scale = scale
-        return b, khat, qbar, qt, k3, alpha
-
-    @staticmethod
-    def backward(ctx, db, dkhat, dqbar, dqt, dk3, dalpha):
-        qp, kp, b = ctx.saved_tensors
-        NC, C, H, dk = qp.shape
-
-        def c16(t):
-            return None if t is None else t.to(torch.bfloat16).contiguous()
-
-        def c32(t):
-            return None if t is None else t.float().contiguous()
-        dkhat, dqbar, dqt, dk3 = c16(dkhat), c16(dqbar), c16(dqt), c16(dk3)
-        db, dalpha = c32(db), c32(dalpha)
-        dq, dk_ = torch.empty_like(qp), torch.empty_like(kp)
-        dg = torch.empty_like(b)
-        rc = _lib.lib().fb_gla_prep_bwd(qp.data_ptr(), kp.data_ptr(), b.data_ptr(), _lib.ptr(dkhat), _lib.ptr(dqbar),
-                                        _lib.ptr(dqt), _lib.ptr(dk3), _lib.ptr(dalpha), _lib.ptr(db), dq.data_ptr(),
-                                        dk_.data_ptr(), dg.data_ptr(), NC, H, dk, float(ctx.scale), _lib.stream_ptr())
-        _lib.check(rc, "fb_gla_prep_bwd")
-        _lib.count_launch()
-        return dq, dk_, dg, None
+def gla_prep(qp, kp, gp, scale: float):
+    """One pass over a chunk's q, k, g producing the cumulative decay and every scaled operand of the GLA chunk algorithm (see
+    ``csrc/chunk.cu: gla_prep_fwd_kernel``).  q, k ``[NC, 64, H, dk]`` bf16, g ``[NC, 64, H, dk]`` fp32, all contiguous.  Returns
+    ``(b, khat, qbar, qt, k3, alpha)``."""
+    NC, C, H, dk = qp.shape
+    assert C == 64 and qp.dtype == torch.bfloat16 and gp.dtype == torch.float32
+    dev = qp.device
+    b = torch.empty_like(gp)
+    khat, qbar, qt = torch.empty_like(kp), torch.empty_like(qp), torch.empty_like(qp)
+    k3 = torch.empty(NC, 3, 48, H, dk, dtype=torch.bfloat16, device=dev)
+    alpha = torch.empty(NC, H, dk, dtype=torch.float32, device=dev)
+    rc = _lib.lib().fb_gla_prep_fwd(qp.data_ptr(), kp.data_ptr(), gp.data_ptr(), b.data_ptr(), khat.data_ptr(),
+                                    qbar.data_ptr(), qt.data_ptr(), k3.data_ptr(), alpha.data_ptr(), NC, H, dk,
+                                    float(scale), _lib.stream_ptr())
+    _lib.check(rc, "fb_gla_prep_fwd")
+    _lib.count_launch()
+    return b, khat, qbar, qt, k3, alpha
 
 
 _lib.register("fb_scalar_prep_fwd", [c_void_p] * 7 + [c_int, c_int, c_int, c_int, c_float, c_void_p])
@@ -182,25 +251,40 @@ def scalar_prep_supported(C: int, dk: int) -> bool:
     return C in (64, 128) and dk % 8 == 0 and n > 0 and (n & (n - 1)) == 0
 
 
+def scalar_prep(qp, kp, gp, scale: float):
+    """``b = cumsum(g)``, ``khat = k e^{b_last - b}``, ``qbar = scale q e^{b}``, ``alpha = e^{b_last}`` in one kernel; q, k
+    ``[NC, C, H, dk]`` bf16, g ``[NC, C, H]`` fp32, all contiguous."""
+    NC, C, H, dk = qp.shape
+    dev = qp.device
+    b = torch.empty(NC, C, H, dtype=torch.float32, device=dev)
+    khat, qbar = torch.empty_like(kp), torch.empty_like(qp)
+    alpha = torch.empty(NC, H, dtype=torch.float32, device=dev)
+    rc = _lib.lib().fb_scalar_prep_fwd(qp.data_ptr(), kp.data_ptr(), _lib.ptr(gp), b.data_ptr(), khat.data_ptr(),
+                                       qbar.data_ptr(), alpha.data_ptr(), NC, C, H, dk, float(scale), _lib.stream_ptr())
+    _lib.check(rc, "fb_scalar_prep_fwd")
+    _lib.count_launch()
+    return b, khat, qbar, alpha
+
+
+def scalar_prep_bwd(qp, kp, b, dkhat, dqbar, dalpha, db, scale: float):
+    """``dq, dk`` (bf16) and ``dg`` (fp32) of ``scalar_prep``; the incoming gradients are contiguous (or None)."""
+    NC, C, H, dk = qp.shape
+    dq, dk_, dg = torch.empty_like(qp), torch.empty_like(kp), torch.empty_like(b)
+    rc = _lib.lib().fb_scalar_prep_bwd(qp.data_ptr(), kp.data_ptr(), b.data_ptr(), _lib.ptr(dkhat), _lib.ptr(dqbar),
+                                       _lib.ptr(dalpha), _lib.ptr(db), dq.data_ptr(), dk_.data_ptr(), dg.data_ptr(), NC,
+                                       C, H, dk, float(scale), _lib.stream_ptr())
+    _lib.check(rc, "fb_scalar_prep_bwd")
+    _lib.count_launch()
+    return dq, dk_, dg
+
+
 class ScalarPrep(torch.autograd.Function):
-    """Cumulative decay and the two token-sized scalings of the scalar-gated chunk algorithms in one kernel:
-    ``b = cumsum(g)``, ``khat = k e^{b_last - b}``, ``qbar = scale q e^{b}``, ``alpha = e^{b_last}``.
-    q, k ``[NC, C, H, dk]`` bf16, g ``[NC, C, H]`` fp32 or None.  Returns ``(b, khat, qbar, alpha)``."""
+    """``scalar_prep`` with its gradients: the token-sized operands of the scalar-gated chunk algorithms."""
 
     @staticmethod
     def forward(ctx, qp, kp, gp, scale):
         qp, kp = qp.contiguous(), kp.contiguous()
-        NC, C, H, dk = qp.shape
-        dev = qp.device
-        if gp is not None:
-            gp = gp.float().contiguous()
-        b = torch.empty(NC, C, H, dtype=torch.float32, device=dev)
-        khat, qbar = torch.empty_like(kp), torch.empty_like(qp)
-        alpha = torch.empty(NC, H, dtype=torch.float32, device=dev)
-        rc = _lib.lib().fb_scalar_prep_fwd(qp.data_ptr(), kp.data_ptr(), _lib.ptr(gp), b.data_ptr(), khat.data_ptr(),
-                                           qbar.data_ptr(), alpha.data_ptr(), NC, C, H, dk, float(scale), _lib.stream_ptr())
-        _lib.check(rc, "fb_scalar_prep_fwd")
-        _lib.count_launch()
+        b, khat, qbar, alpha = scalar_prep(qp, kp, None if gp is None else gp.float().contiguous(), scale)
         ctx.save_for_backward(qp, kp, b)
         ctx.scale = scale
         ctx.has_g = gp is not None
@@ -209,18 +293,11 @@ class ScalarPrep(torch.autograd.Function):
     @staticmethod
     def backward(ctx, db, dkhat, dqbar, dalpha):
         qp, kp, b = ctx.saved_tensors
-        NC, C, H, dk = qp.shape
         dkhat = None if dkhat is None else dkhat.to(torch.bfloat16).contiguous()
         dqbar = None if dqbar is None else dqbar.to(torch.bfloat16).contiguous()
         db = None if db is None else db.float().contiguous()
         dalpha = None if dalpha is None else dalpha.float().contiguous()
-        dq, dk_ = torch.empty_like(qp), torch.empty_like(kp)
-        dg = torch.empty_like(b)
-        rc = _lib.lib().fb_scalar_prep_bwd(qp.data_ptr(), kp.data_ptr(), b.data_ptr(), _lib.ptr(dkhat), _lib.ptr(dqbar),
-                                           _lib.ptr(dalpha), _lib.ptr(db), dq.data_ptr(), dk_.data_ptr(), dg.data_ptr(), NC,
-                                           C, H, dk, float(ctx.scale), _lib.stream_ptr())
-        _lib.check(rc, "fb_scalar_prep_bwd")
-        _lib.count_launch()
+        dq, dk_, dg = scalar_prep_bwd(qp, kp, b, dkhat, dqbar, dalpha, db, ctx.scale)
         return dq, dk_, (dg if ctx.has_g else None), None
 
 
@@ -304,38 +381,59 @@ class SelectiveScan(torch.autograd.Function):
         return du, ddl, dA.sum(0)[:, :Di].t(), dB, dC, dD.sum(0)[:Di], dz, None, None
 
 
-_lib.register("fb_vdecay_diag_fwd", [c_void_p] * 4 + [c_int, c_int, c_int, c_void_p])
-_lib.register("fb_vdecay_diag_bwd", [c_void_p] * 7 + [c_int, c_int, c_int, c_void_p])
+_lib.register("fb_vdecay_prep", [c_void_p] * 6 + [c_int] * 3 + [c_void_p])
+_lib.register("fb_vdecay_out", [c_void_p] * 5 + [c_int] * 3 + [c_float] + [c_void_p] * 3)
+_lib.register("fb_vdecay_bwd1", [c_void_p] * 4 + [c_int] * 3 + [c_float] + [c_void_p] * 4)
+_lib.register("fb_vdecay_bwd2", [c_void_p] * 8 + [c_int] * 3 + [c_float] + [c_void_p] * 3)
+VDECAY_SOFTMAX_MAX = 512   # slots whose softmax rides on ``vdecay_out``
 
 
-class VdecayDiag(torch.autograd.Function):
-    """Diagonal 16 x 16 sub-blocks of the value-decayed intra-chunk product (``csrc/chunk.cu: vdecay_diag_*``):
-    P ``[NC, H, 64, 64]`` fp32, v ``[NC, 64, H, M]`` bf16, b ``[NC, 64, H, M]`` fp32 -> ``[NC, 64, H, M]`` fp32."""
+def vdecay_prep(v, g):
+    """``b = cumsum(g)``, ``vhat = v e^{b_last - b}``, ``v3`` (values re-based for the sub-blocks behind them, ``[NC, 3, 48, H, M]``)
+    and ``alpha = e^{b_last}``; v ``[NC, 64, H, M]`` bf16, g fp32, contiguous."""
+    NC, C, H, M = v.shape
+    assert C == 64 and v.dtype == torch.bfloat16 and g.dtype == torch.float32
+    b, vhat = torch.empty_like(g), torch.empty_like(v)
+    v3 = torch.empty(NC, 3, 48, H, M, dtype=v.dtype, device=v.device)
+    alpha = torch.empty(NC, H, M, dtype=torch.float32, device=v.device)
+    _lib.check(_lib.lib().fb_vdecay_prep(v.data_ptr(), g.data_ptr(), b.data_ptr(), vhat.data_ptr(), v3.data_ptr(), alpha.data_ptr(), NC, H,
+                                         M, _lib.stream_ptr()), "fb_vdecay_prep")
+    _lib.count_launch()
+    return b, vhat, v3, alpha
 
-    @staticmethod
-    def forward(ctx, P, v, b):
-        P, v, b = P.float().contiguous(), v.contiguous(), b.contiguous()
-        NC, C, H, M = v.shape
-        assert C == 64 and v.dtype == torch.bfloat16
-        o = torch.empty(NC, C, H, M, dtype=torch.float32, device=v.device)
-        _lib.check(_lib.lib().fb_vdecay_diag_fwd(P.data_ptr(), v.data_ptr(), b.data_ptr(), o.data_ptr(), NC, H, M,
-                                                 _lib.stream_ptr()), "fb_vdecay_diag_fwd")
-        _lib.count_launch()
-        ctx.save_for_backward(P, v, b)
-        return o
 
-    @staticmethod
-    def backward(ctx, do):
-        P, v, b = ctx.saved_tensors
-        NC, C, H, M = v.shape
-        do = do.float().contiguous()
-        dP = torch.zeros_like(P)
-        dv = torch.empty(NC, C, H, M, dtype=torch.float32, device=v.device)
-        db = torch.empty_like(dv)
-        _lib.check(_lib.lib().fb_vdecay_diag_bwd(P.data_ptr(), v.data_ptr(), b.data_ptr(), do.data_ptr(), dP.data_ptr(),
-                                                 dv.data_ptr(), db.data_ptr(), NC, H, M, _lib.stream_ptr()), "fb_vdecay_diag_bwd")
-        _lib.count_launch()
-        return dP, dv.to(v.dtype), db
+def vdecay_out(o1, acc, P, v, b, scale: float, softmax: bool):
+    """``o`` fp32 and, with ``softmax``, its softmax over the last dimension in bf16 (see ``csrc/chunk.cu: vdecay_out_kernel``)."""
+    NC, C, H, M = v.shape
+    o = torch.empty_like(b)
+    qv = torch.empty_like(v) if softmax else None
+    _lib.check(_lib.lib().fb_vdecay_out(o1.data_ptr(), acc.data_ptr(), P.data_ptr(), v.data_ptr(), b.data_ptr(), NC, H, M, float(scale),
+                                        o.data_ptr(), _lib.ptr(qv), _lib.stream_ptr()), "fb_vdecay_out")
+    _lib.count_launch()
+    return o, qv
+
+
+def vdecay_bwd1(o, dqv, d32, b, scale: float):
+    """``do`` (fp32, from the gradient ``dqv`` of the softmax, or ``d32`` of ``o``), ``do e^b`` and ``do e^{b - r_I}`` (rows 16..63)."""
+    NC, C, H, M = b.shape
+    do = torch.empty_like(b)
+    do1 = torch.empty(b.shape, dtype=torch.bfloat16, device=b.device)
+    dacc = torch.empty(NC, 48, H, M, dtype=torch.bfloat16, device=b.device)
+    _lib.check(_lib.lib().fb_vdecay_bwd1(o.data_ptr(), _lib.ptr(dqv), _lib.ptr(d32), b.data_ptr(), NC, H, M, float(scale), do.data_ptr(),
+                                         do1.data_ptr(), dacc.data_ptr(), _lib.stream_ptr()), "fb_vdecay_bwd1")
+    _lib.count_launch()
+    return do, do1, dacc
+
+
+def vdecay_bwd2(P, v, b, do, o, dvhat, dv3, dalpha, scale: float):
+    """``dv`` (bf16) and ``dg`` (fp32)."""
+    NC, C, H, M = v.shape
+    dv, dg = torch.empty_like(v), torch.empty_like(b)
+    _lib.check(_lib.lib().fb_vdecay_bwd2(P.data_ptr(), v.data_ptr(), b.data_ptr(), do.data_ptr(), o.data_ptr(), dvhat.data_ptr(),
+                                         dv3.data_ptr(), dalpha.data_ptr(), NC, H, M, 1.0 / scale, dv.data_ptr(), dg.data_ptr(),
+                                         _lib.stream_ptr()), "fb_vdecay_bwd2")
+    _lib.count_launch()
+    return dv, dg
 
 
 _lib.register("fb_scores_bwd_prep", [c_void_p] * 5 + [c_longlong] * 3 + [c_int] * 4 + [c_void_p, c_void_p, c_void_p])

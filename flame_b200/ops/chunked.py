@@ -245,137 +245,331 @@ def _like(t: torch.Tensor) -> torch.Tensor:
     return _empty_like_layout(t)
 
 
-def tri_inverse(A: torch.Tensor) -> torch.Tensor:
-    """``(I + A)^-1`` for strictly lower-triangular ``A [NC, H, n, n]`` (fp32), n = 64 or 128, no autograd.
-    n = 128 is inverted blockwise: with A = [[A11, 0], [A21, A22]] the inverse is [[T11, 0], [-T22 A21 T11, T22]]
-    where T11, T22 come from the 64 x 64 kernel and the corner from two batched GEMMs."""
-    n = A.shape[-1]
-    if _lib.available() and A.is_cuda:
-        from . import chunk_kernels
-        if n == 64:
-            return chunk_kernels.tri_inverse(A, torch.bfloat16)
-        assert n == 128, "chunk sizes 64 and 128 are supported"
-        h = 64
-        diag = torch.stack((A[..., :h, :h], A[..., h:, h:]), 0).contiguous()
-        Td = chunk_kernels.tri_inverse(diag, torch.bfloat16)            # [2, NC, H, 64, 64]
-        T11, T22 = Td[0], Td[1]
-        X = bgemm(T22, A[..., h:, :h].to(torch.bfloat16), b_mn=True)     # T22 A21
-        out = torch.zeros(A.shape, dtype=torch.bfloat16, device=A.device)
-        out[..., :h, :h] = T11
-        out[..., h:, h:] = T22
-        bgemm(X, T11, b_mn=True, alpha=-1.0, out=out[..., h:, :h])
-        return out
-    eye = torch.eye(n, dtype=torch.float32, device=A.device)
-    return torch.linalg.solve_triangular(eye + A.float(), eye.expand_as(A).contiguous(), upper=False, unitriangular=True)
-
-
-class _TriInv(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, A):
-        T = tri_inverse(A).to(torch.bfloat16 if A.is_cuda else A.dtype).contiguous()
-        ctx.save_for_backward(T)
-        return T
+class _DecayStates(torch.autograd.Function):
+    """States at the start of every chunk for ``S_{c+1} = alpha_c S_c + khat_c^T u_c`` (S = 0 at the first chunk of a
+    document); ``alpha`` is ``[NC, H]`` or ``[NC, H, dk]`` (one decay per key channel).  The increments and the running state
+    are fp32, the states handed out bf16."""
 
     @staticmethod
-    def backward(ctx, dT):
-        (T,) = ctx.saved_tensors
-        dT = dT.to(T.dtype)
-        # dA = -T^T dT T^T, kept on the strict lower triangle
-        x = bgemm(T, dT, a_mn=True, b_mn=True)
-        dA = bgemm(x, T, alpha=-1.0, mask=MASK_STRICT, out_dtype=torch.float32)
-        return dA
-
-
-class _DeltaScan(torch.autograd.Function):
-    """States at the start of every chunk for ``S_{c+1} = alpha_c S_c - (khat_c^T w_c) S_c + khat_c^T u_c`` (S = 0 at
-    the first chunk of a document).  ``w = None`` drops the middle term (plain gated linear attention); then ``alpha``
-    may also be ``[NC, H, dk]`` (one decay per key channel).
-
-    With ``w`` the running state lives in ONE fp32 buffer per document (``[docs, H, dk, dv]``, updated in place by the
-    GEMM epilogue and small enough to stay in L2); only its bf16 copy is written per chunk."""
-
-    @staticmethod
-    def forward(ctx, alpha, khat, w, u, lay: ChunkLayout):
-        # alpha [NC, H] fp32; khat, w [NC, H, C, dk]; u [NC, H, C, dv] (operand views); without w, khat may have fewer
-        # heads than u (keys shared by groups of heads)
-        NC, _, _, dk = khat.shape
-        H = u.shape[1]
-        dv = u.shape[-1]
-        dev = khat.device
+    def forward(ctx, alpha, khat, u, lay: ChunkLayout):
+        # alpha fp32; khat [NC, G, C, dk]; u [NC, H, C, dv] (operand views); keys may be shared by groups of heads
         alpha = alpha.contiguous()
-        S16 = torch.empty(NC + 1, H, dk, dv, dtype=khat.dtype, device=dev)
-        S16.index_fill_(0, lay.first, 0.0)
-        if w is not None:
-            M = bgemm(khat, w, a_mn=True, b_mn=True)                 # [NC, H, dk, dk] chunk transition
-            B16 = bgemm(khat, u, a_mn=True, b_mn=True)               # [NC, H, dk, dv] chunk increment
-            if _scan_kernel_ok(M, B16, alpha, dk, dv):
-                _delta_scan(M, B16, alpha, S16, lay, reverse=False)   # one persistent launch walks every document
-            else:  # shapes the scan kernel does not cover: one batched GEMM per chunk position
-                state = torch.zeros(lay.n_docs, H, dk, dv, dtype=torch.float32, device=dev)
-                for idx, docs in zip(lay.steps, lay.step_docs):
-                    bgemm(M, S16, b_mn=True, a_index=idx, b_index=idx, out=state, c_index=docs, cin=state,
-                          cin_index=docs, gamma=alpha, alpha=-1.0, add16=B16, add16_index=idx, out16=S16,
-                          out16_index=idx, out16_offset=1, n_hi=len(idx))
-        else:
-            M = None
-            Sf = torch.empty(NC + 1, H, dk, dv, dtype=torch.float32, device=dev)
-            bgemm(khat, u, a_mn=True, b_mn=True, out=Sf, c_offset=1)
-            Sf.index_fill_(0, lay.first, 0.0)
-            _elementwise_steps(lay, alpha, Sf, S16, reverse=False)
-        ctx.save_for_backward(alpha, khat, w, u, M, S16)
+        S = _state_scan(lay, alpha, bgemm(khat, u, a_mn=True, b_mn=True, out_dtype=torch.float32), khat.dtype, reverse=False)
+        ctx.save_for_backward(alpha, khat, u, S)
         ctx.lay = lay
-        return S16[:NC]
+        return S
 
     @staticmethod
     def backward(ctx, dS):
-        alpha, khat, w, u, M, S16 = ctx.saved_tensors
+        alpha, khat, u, S = ctx.saved_tensors
         lay = ctx.lay
-        NC, _, _, dk = khat.shape
+        NC, G, _, dk = khat.shape
         H = u.shape[1]
-        dv = u.shape[-1]
-        dev = khat.device
-        dS = dS.to(khat.dtype).contiguous()
-        L16 = torch.empty(NC + 1, H, dk, dv, dtype=khat.dtype, device=dev)
-        L16[:NC] = dS
-        L16[NC] = 0
-        if M is not None and _scan_kernel_ok(M, dS, alpha, dk, dv):
-            _delta_scan(M, dS, alpha, L16, lay, reverse=True)
-        elif M is not None:
-            # adjoint state per document, started from the gradient of the document's last chunk state
-            lam = dS.index_select(0, lay.last).float()
-            for idx, docs in zip(lay.steps[::-1], lay.step_docs[::-1]):
-                bgemm(M, L16, a_mn=True, b_mn=True, a_index=idx, b_index=idx, b_offset=1, out=lam, c_index=docs, cin=lam,
-                      cin_index=docs, gamma=alpha, alpha=-1.0, add16=dS, add16_index=idx, out16=L16, out16_index=idx,
-                      n_hi=len(idx))
-        else:
-            Lf = torch.empty(NC + 1, H, dk, dv, dtype=torch.float32, device=dev)
-            Lf[:NC] = dS
-            Lf[NC] = 0
-            _elementwise_steps(lay, alpha, Lf, L16, reverse=True)
         # adjoint of the state entering the NEXT chunk; zero where the next chunk belongs to another document
-        L16.index_fill_(0, lay.first, 0.0)
-        Ln = L16[1:]
-        S = S16[:NC]
-        dalpha = dkhat = dw = du = None
+        Ln = _state_scan(lay, alpha, dS.to(khat.dtype).contiguous(), khat.dtype, reverse=True)
+        dalpha = dkhat = du = None
         if ctx.needs_input_grad[0]:
             dalpha = _pair_dot(Ln, S, per_row=alpha.dim() == 3)
-        # B_c = khat^T u
-        dkh = bgemm(u, Ln, out_dtype=torch.float32, out=_token_major(NC, H, lay.chunk, dk, torch.float32, dev))
-        if ctx.needs_input_grad[3]:
+        if ctx.needs_input_grad[2]:
             du = _like(u)
             bgemm(khat, Ln, b_mn=True, out=du)
-        if w is not None:
-            dM = bgemm(Ln, S, alpha=-1.0)  # [NC, H, dk, dk]
-            bgemm(w, dM, out=dkh, accumulate=True)
-            if ctx.needs_input_grad[2]:
-                dw = _like(w)
-                bgemm(khat, dM, b_mn=True, out=dw)
         if ctx.needs_input_grad[1]:
-            G = khat.shape[1]
             if G < H:  # keys shared by the heads of a group
-                dkh = dkh.reshape(NC, G, H // G, *dkh.shape[2:]).sum(2)
-            dkhat = dkh.to(khat.dtype)
-        return dalpha, dkhat, dw, du, None
+                dkh = bgemm(u, Ln, out_dtype=torch.float32, out=_token_major(NC, H, lay.chunk, dk, torch.float32, khat.device))
+                dkhat = dkh.reshape(NC, G, H // G, *dkh.shape[2:]).sum(2).to(khat.dtype)
+            else:
+                dkhat = bgemm(u, Ln, out=_token_major(NC, H, lay.chunk, dk, khat.dtype, khat.device))
+        return dalpha, dkhat, du, None
+
+
+def _state_scan(lay: ChunkLayout, alpha, x, dtype, reverse: bool) -> torch.Tensor:
+    """``s = 0; for every chunk of a document (backwards when ``reverse``): out_c = s; s = alpha_c s + x_c``."""
+    if _lib.available() and x.is_cuda:
+        from . import chunk_kernels
+        return chunk_kernels.state_scan(lay.first, lay.last, alpha, x, reverse)
+    al = alpha[..., None] if alpha.dim() == 3 else alpha[..., None, None]
+    out = torch.zeros(x.shape, dtype=torch.float32, device=x.device)
+    for idx in (lay.steps[::-1] if reverse else lay.steps):
+        i = idx.long()
+        src, dst = (i + 1, i) if reverse else (i, i + 1)
+        out[dst] = al[src] * out[src] + x[src].float()
+    return out.to(dtype)
+
+
+def _delta_states(M, B, alpha, lay: ChunkLayout) -> torch.Tensor:
+    """``[NC, H, dk, dv]``: the state entering every chunk of ``S_{c+1} = alpha_c S_c - M_c S_c + B_c``."""
+    NC, H, dk, dv = B.shape
+    S = torch.empty(NC + 1, H, dk, dv, dtype=B.dtype, device=B.device)
+    if _scan_kernel_ok(M, B, alpha, dk, dv):
+        _delta_scan(M, B, alpha, S, lay, reverse=False)   # one persistent launch walks every document
+    else:
+        # shapes the scan kernel does not cover: one batched GEMM per chunk position; the running state lives in ONE fp32
+        # buffer per document, updated in place by the epilogue
+        S.index_fill_(0, lay.first, 0.0)
+        state = torch.zeros(lay.n_docs, H, dk, dv, dtype=torch.float32, device=B.device)
+        for idx, docs in zip(lay.steps, lay.step_docs):
+            bgemm(M, S, b_mn=True, a_index=idx, b_index=idx, out=state, c_index=docs, cin=state, cin_index=docs, gamma=alpha,
+                  alpha=-1.0, add16=B, add16_index=idx, out16=S, out16_index=idx, out16_offset=1, n_hi=len(idx))
+    return S[:NC]
+
+
+def _delta_adjoint(M, dS, alpha, lay: ChunkLayout) -> torch.Tensor:
+    """``[NC, H, dk, dv]``: the adjoint of the state LEAVING every chunk (zero at a document's last) for the state gradients
+    ``dS`` of the recurrence above."""
+    NC, H, dk, dv = dS.shape
+    if _scan_kernel_ok(M, dS, alpha, dk, dv):
+        Ln = torch.empty_like(dS)
+        _delta_scan(M, dS, alpha, Ln, lay, reverse=2)
+        return Ln
+    L = torch.empty(NC + 1, H, dk, dv, dtype=dS.dtype, device=dS.device)
+    L[:NC] = dS
+    L[NC] = 0
+    lam = dS.index_select(0, lay.last).float()
+    for idx, docs in zip(lay.steps[::-1], lay.step_docs[::-1]):
+        bgemm(M, L, a_mn=True, b_mn=True, a_index=idx, b_index=idx, b_offset=1, out=lam, c_index=docs, cin=lam, cin_index=docs,
+              gamma=alpha, alpha=-1.0, add16=dS, add16_index=idx, out16=L, out16_index=idx, n_hi=len(idx))
+    L.index_fill_(0, lay.first, 0.0)
+    return L[1:]
+
+
+# the C x C stages of the delta rule: kernels of csrc/chunk.cu, or their definitions
+def _delta_inverse(P, beta, b):
+    if _lib.available() and P.is_cuda:
+        from . import chunk_kernels
+        return chunk_kernels.delta_inverse(P, beta, b, bgemm)
+    C = P.shape[-1]
+    br = beta.permute(0, 2, 1)
+    eye = torch.eye(C, dtype=torch.float32, device=P.device)
+    T = torch.linalg.solve_triangular(eye + br[..., None] * P.float(), eye.expand_as(P).contiguous(), upper=False, unitriangular=True)
+    return T, T * br[..., None, :], None if b is None else T * (br * b.permute(0, 2, 1).exp())[..., None, :]
+
+
+def _delta_bwd_t(T, dTu, dTw, beta, b, scale):
+    if _lib.available() and T.is_cuda:
+        from . import chunk_kernels
+        return chunk_kernels.delta_bwd_t(T, dTu, dTw, beta, b, scale)
+    br = beta.permute(0, 2, 1)[..., None, :]
+    w = 0 if b is None else dTw * b.permute(0, 2, 1).exp()[..., None, :]
+    dbeta = scale * (T * (dTu + w)).sum(-2).permute(0, 2, 1)
+    db = None if b is None else scale * (br * T * w).sum(-2).permute(0, 2, 1)
+    return br * (dTu + w), dbeta, db
+
+
+def _delta_bwd_scores(dA, P, dQ, Q, beta, b, scale, dbeta, db):
+    if _lib.available() and P.is_cuda:
+        from . import chunk_kernels
+        return chunk_kernels.delta_bwd_scores(dA, P, dQ, Q, beta, b, scale, dbeta, db)
+    C = P.shape[-1]
+    br = beta.permute(0, 2, 1)[..., None]
+    dA = dA.masked_fill(~_mask(C, C, MASK_STRICT, P.device), 0.0)
+    dbeta += scale * (dA * P).sum(-1).permute(0, 2, 1)
+    if b is None:
+        return dA * br, None
+    d = b.permute(0, 2, 1)
+    w = (d[..., :, None] - d[..., None, :]).masked_fill(~_mask(C, C, MASK_TRIL, P.device), float("-inf")).exp()
+    e = br * dA * P + dQ * Q
+    db += scale * (e.sum(-1) - e.sum(-2)).permute(0, 2, 1)
+    return br * dA * w, dQ * w
+
+
+class _GatedDelta(torch.autograd.Function):
+    """The whole chunk pipeline of the (gated) delta rule on packed chunks: q, k ``[NC, C, H, dk]``, v ``[NC, C, H, dv]``, beta
+    and the log decay g ``[NC, C, H]`` fp32 (g may be None).  One node instead of one per product: the terms of an output or of
+    a gradient accumulate in one GEMM, nothing is added up by passes of its own, and without a decay the operands that a
+    decay would rescale are the inputs themselves.  ``scale`` is a factor of the output; the backward runs without it and
+    puts it into the last products."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, beta, g, scale, lay):
+        q, k, v, beta = q.contiguous(), k.contiguous(), v.contiguous(), beta.contiguous()
+        NC, C, H, dk = q.shape
+        dv = v.shape[-1]
+        if g is not None:
+            b, khat, qbar, alpha = _scalar_prep_raw(q, k, g.contiguous())
+            d = b.permute(0, 2, 1)
+        else:
+            b = d = None
+            khat, qbar = k, q
+            alpha = torch.ones(NC, H, dtype=torch.float32, device=q.device)
+        qh, kh, vh, khh, qbh = (_hm(t) for t in (q, k, v, khat, qbar))
+        P = bgemm(kh, kh, mask=MASK_STRICT, decay=d, out_dtype=torch.float32)             # [NC, H, C, C]
+        Q = bgemm(qh, kh, mask=MASK_TRIL, decay=d)
+        T, Tu, Tw = _delta_inverse(P, beta, b)
+        T, Tu = T.to(q.dtype), Tu.to(q.dtype)
+        Tw = Tu if Tw is None else Tw.to(q.dtype)
+        u = bgemm(Tu, vh, b_mn=True, out=_token_major(NC, H, C, dv, q.dtype, q.device))
+        w = bgemm(Tw, kh, b_mn=True, out=_token_major(NC, H, C, dk, q.dtype, q.device))
+        M = bgemm(khh, w, a_mn=True, b_mn=True)                                           # [NC, H, dk, dk] chunk transition
+        S = _delta_states(M, bgemm(khh, u, a_mn=True, b_mn=True), alpha, lay)             # [NC, H, dk, dv]
+        vn = bgemm(w, S, b_mn=True, alpha=-1.0, add16=u, out=_token_major(NC, H, C, dv, q.dtype, q.device))      # u - w S
+        o = bgemm(qbh, S, b_mn=True, alpha=scale, more=[(Q, vn, False, True, 1)],
+                  out=_token_major(NC, H, C, dv, q.dtype, q.device))
+        ctx.save_for_backward(q, k, v, beta, b, khat if b is not None else None, qbar if b is not None else None, alpha, P, Q, T, Tu,
+                              Tw if b is not None else None, u, w, M, S, vn)
+        ctx.cfg = (scale, lay)
+        return o.permute(0, 2, 1, 3)
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, beta, b, khat, qbar, alpha, P, Q, T, Tu, Tw, u, w, M, S, vn = ctx.saved_tensors
+        scale, lay = ctx.cfg
+        NC, C, H, dk = q.shape
+        dt, dev = q.dtype, q.device
+        dv = v.shape[-1]
+        gated = b is not None
+        doh = _hm(do.to(dt).contiguous())
+        qh, kh, vh = _hm(q), _hm(k), _hm(v)
+        khh, qbh = (_hm(khat), _hm(qbar)) if gated else (kh, qh)
+        Tw = Tw if gated else Tu
+        tok = lambda n: _token_major(NC, H, C, n, dt, dev)                                # noqa: E731
+        dvn = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(dv))
+        gq = bgemm(doh, vn, mask=MASK_TRIL)                                               # dQ (without a decay also its operand)
+        Ln = _delta_adjoint(M, bgemm(qbh, doh, a_mn=True, b_mn=True, more=[(w, dvn, True, True, -1)]), alpha, lay)
+        dM = bgemm(Ln, S, alpha=-1.0)                                                     # [NC, H, dk, dk]
+        du = bgemm(khh, Ln, b_mn=True, add16=dvn, out=tok(dv))
+        dw = bgemm(khh, dM, b_mn=True, more=[(dvn, S, False, False, -1)], out=tok(dk))
+        if gated:
+            dTu, dTw = bgemm(du, vh), bgemm(dw, kh)
+        else:
+            dTu, dTw = bgemm(du, vh, more=[(dw, kh, False, False, 1)]), None
+        dvv = bgemm(Tu, du, a_mn=True, b_mn=True, alpha=scale, out=tok(dv))
+        dT, dbeta, db = _delta_bwd_t(T, dTu, dTw, beta, b, scale)
+        # T = (I + A)^-1: dA = -T^T dT T^T on the strict lower triangle
+        dA = bgemm(bgemm(T, dT, a_mn=True, b_mn=True), T, alpha=-1.0, mask=MASK_STRICT, out_dtype=torch.float32)
+        gk, gq2 = _delta_bwd_scores(dA, P, gq, Q, beta, b, scale, dbeta, db)
+        gk = gk.to(dt)
+        keys = [(gk, kh, False, True, 1), (gk, kh, True, True, 1)]
+        dg = None
+        if gated:
+            gq = gq2.to(dt)
+            dqbar, dkhat = bgemm(doh, S, out=tok(dk)), bgemm(u, Ln, alpha=scale, more=[(w, dM, False, False, 1)], out=tok(dk))
+            dalpha = _pair_dot(Ln, S, per_row=False) * scale
+            dq0, dk0, dg = _scalar_prep_raw_bwd(q, k, b, dkhat.permute(0, 2, 1, 3), dqbar.permute(0, 2, 1, 3), dalpha, db, scale)
+            dq = bgemm(gq, kh, b_mn=True, alpha=scale, add16=_hm(dq0), out=tok(dk))
+            dkk = bgemm(Tw, dw, a_mn=True, b_mn=True, alpha=scale, more=keys + [(gq, qh, True, True, 1)], add16=_hm(dk0), out=tok(dk))
+        else:
+            dq = bgemm(doh, S, alpha=scale, more=[(gq, kh, False, True, 1)], out=tok(dk))
+            dkk = bgemm(Tu, dw, a_mn=True, b_mn=True, alpha=scale, out=tok(dk),
+                        more=keys + [(gq, qh, True, True, 1), (u, Ln, False, False, 1), (w, dM, False, False, 1)])
+        back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
+        return back(dq), back(dkk), back(dvv), dbeta, dg, None, None
+
+
+class _GroupedScalarGla(torch.autograd.Function):
+    """The chunk pipeline of scalar-gated attention whose queries and keys ``[NC, C, G, dk]`` serve groups of H / G heads
+    (Mamba2's C and B), v ``[NC, C, H, dv]``, g ``[NC, C, H]`` fp32.  They are never expanded: the decay moves to the value side
+    of the state update (``S += k^T (v e^{b_last - b})``) and to the rows of the output, and the gradients of q and k add the
+    heads of a group up in the accumulator of one product."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, scale, lay):
+        q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+        NC, C, H, dv = v.shape
+        b, eb, alpha, vhat = _group_prep(v, g, scale)
+        d = b.permute(0, 2, 1)
+        qh, kh = _hm(q), _hm(k)
+        Q = bgemm(qh, kh, alpha=scale, mask=MASK_TRIL, decay=d, n_lo=H)                   # [NC, H, C, C] from the shared q / k
+        S = _state_scan(lay, alpha, bgemm(kh, _hm(vhat), a_mn=True, b_mn=True, out_dtype=torch.float32), q.dtype, reverse=False)
+        o1 = bgemm(qh, S, b_mn=True, rowscale=eb.permute(0, 2, 1), out=_token_major(NC, H, C, dv, q.dtype, q.device))
+        o = bgemm(Q, _hm(v), b_mn=True, add16=o1, out=_token_major(NC, H, C, dv, q.dtype, q.device))
+        ctx.save_for_backward(q, k, v, b, eb, alpha, vhat, Q, S, o1.permute(0, 2, 1, 3))
+        ctx.lay, ctx.scale = lay, scale
+        return o.permute(0, 2, 1, 3)
+
+    @staticmethod
+    def backward(ctx, do):
+        q, k, v, b, eb, alpha, vhat, Q, S, o1 = ctx.saved_tensors
+        lay = ctx.lay
+        NC, C, H, dv = v.shape
+        G, dk = q.shape[2:]
+        dt, dev = q.dtype, q.device
+        tok = lambda h, n: _token_major(NC, h, C, n, dt, dev)                             # noqa: E731
+        do = do.to(dt).contiguous()
+        dos, db = _group_bwd1(do, o1, eb)
+        doh, dosh, qh, kh, vhh = _hm(do), _hm(dos), _hm(q), _hm(k), _hm(vhat)
+        gq = _scores_bwd(bgemm(doh, _hm(v), mask=MASK_TRIL), Q, b, db).to(dt)
+        if ctx.scale != 1.0:   # Q has the factor (so the gradient of b has it), its operand's gradient not yet
+            gq = gq * ctx.scale
+        dv1 = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(H, dv))
+        Ln = _state_scan(lay, alpha, bgemm(qh, dosh, a_mn=True, b_mn=True), dt, reverse=True)
+        dvhat = bgemm(kh, Ln, b_mn=True, out=tok(H, dv))
+        back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
+        dvv, dg = _group_bwd2(back(dvhat), vhat, back(dv1), b, db, alpha, _pair_dot(Ln, S, per_row=False))
+        r = H // G
+        dq = bgemm(dosh, S, more=[(gq, kh, False, True, 1)], sum_lo=r, out=tok(G, dk))
+        dkk = bgemm(vhh, Ln, more=[(gq, qh, True, True, 1)], sum_lo=r, out=tok(G, dk))
+        return back(dq), back(dkk), dvv, dg, None, None
+
+
+def _group_kernels(v) -> bool:
+    if not (_lib.available() and v.is_cuda):
+        return False
+    from . import chunk_kernels
+    return chunk_kernels.group_supported(v.shape[1], v.shape[-1])
+
+
+def _group_prep(v, g, scale):
+    if _group_kernels(v):
+        from . import chunk_kernels
+        return chunk_kernels.group_prep(v, g, scale)
+    b = g.cumsum(1)
+    last = b[:, -1:]
+    return b, scale * b.exp(), last[:, 0].exp().contiguous(), (v.float() * (last - b).exp()[..., None]).to(v.dtype)
+
+
+def _group_bwd1(do, o1, eb):
+    if _group_kernels(do):
+        from . import chunk_kernels
+        return chunk_kernels.group_bwd1(do, o1, eb)
+    return (do.float() * eb[..., None]).to(do.dtype), (do.float() * o1.float()).sum(-1)
+
+
+def _group_bwd2(dvhat, vhat, dv1, b, db, alpha, dalpha):
+    if _group_kernels(vhat):
+        from . import chunk_kernels
+        return chunk_kernels.group_bwd2(dvhat, vhat, dv1, b, db, alpha, dalpha)
+    s = (dvhat.float() * vhat.float()).sum(-1)
+    db = db - s
+    db[:, -1] += s.sum(1) + alpha * dalpha
+    dv = dv1.float() + dvhat.float() * (b[:, -1:] - b).exp()[..., None]
+    return dv.to(dv1.dtype), db.flip(1).cumsum(1).flip(1)
+
+
+def _scores_bwd(dQ, Q, b, db):
+    if _lib.available() and Q.is_cuda:
+        from . import chunk_kernels
+        return chunk_kernels.scores_bwd(dQ, Q, b, db)
+    C = Q.shape[-1]
+    d = b.permute(0, 2, 1)
+    w = (d[..., :, None] - d[..., None, :]).masked_fill(~_mask(C, C, MASK_TRIL, Q.device), float("-inf")).exp()
+    e = dQ.float() * Q.float()
+    db += (e.sum(-1) - e.sum(-2)).permute(0, 2, 1)
+    return dQ * w
+
+
+def _scalar_prep_raw(q, k, g):
+    """``b = cumsum(g)``, ``khat = k e^{b_last - b}``, ``qbar = q e^b``, ``alpha = e^{b_last}`` without autograd."""
+    if _lib.available() and q.is_cuda:
+        from . import chunk_kernels
+        if chunk_kernels.scalar_prep_supported(q.shape[1], q.shape[-1]):
+            return chunk_kernels.scalar_prep(q, k, g, 1.0)
+    b = g.cumsum(1)
+    return (b, k * (b[:, -1:] - b).exp().to(k.dtype)[..., None], q * b.exp().to(q.dtype)[..., None], b[:, -1].exp().contiguous())
+
+
+def _scalar_prep_raw_bwd(q, k, b, dkhat, dqbar, dalpha, db, scale):
+    """Gradients of ``_scalar_prep_raw``; ``scale`` multiplies ``dqbar`` (the other incoming gradients have it already)."""
+    if _lib.available() and q.is_cuda:
+        from . import chunk_kernels
+        if chunk_kernels.scalar_prep_supported(q.shape[1], q.shape[-1]):
+            return chunk_kernels.scalar_prep_bwd(q, k, b, dkhat, dqbar, dalpha, db, scale)
+    last = b[:, -1:]
+    dq = dqbar.float() * (b.exp() * scale)[..., None]
+    dk = dkhat.float() * (last - b).exp()[..., None]
+    kd = (k.float() * dk).sum(-1)
+    db = db + (q.float() * dq).sum(-1) - kd
+    db[:, -1] += kd.sum(1) + dalpha * b[:, -1].exp()
+    return dq.to(q.dtype), dk.to(k.dtype), db.flip(1).cumsum(1).flip(1)
 
 
 def _scan_kernel_ok(M: torch.Tensor, add: torch.Tensor, alpha: torch.Tensor, dk: int, dv: int) -> bool:
@@ -386,13 +580,14 @@ def _scan_kernel_ok(M: torch.Tensor, add: torch.Tensor, alpha: torch.Tensor, dk:
 
 
 def _delta_scan(M: torch.Tensor, add: torch.Tensor, alpha: torch.Tensor, out16: torch.Tensor, lay: "ChunkLayout",
-                reverse: bool) -> None:
-    """The chunk-state recurrence of every (document, head) in one persistent kernel (``csrc/delta_scan.cu``)."""
+                reverse: int) -> None:
+    """The chunk-state recurrence of every (document, head) in one persistent kernel (``csrc/delta_scan.cu``); reverse 2:
+    with the output shifted to the chunk that the state leaves."""
     NC, H, dk, _ = M.shape
     dv = add.shape[-1]
     first, last = lay.first_i32, lay.last_i32
     rc = _lib.lib().fb_delta_scan(M.data_ptr(), add.data_ptr(), alpha.data_ptr(), out16.data_ptr(), first.data_ptr(),
-                                  last.data_ptr(), lay.n_docs, H, NC, dk, dv, 1 if reverse else 0, _lib.stream_ptr())
+                                  last.data_ptr(), lay.n_docs, H, NC, dk, dv, int(reverse), _lib.stream_ptr())
     _lib.check(rc, "fb_delta_scan")
     _lib.count_launch()
 
@@ -407,22 +602,6 @@ def _pair_dot(x: torch.Tensor, y: torch.Tensor, per_row: bool) -> torch.Tensor:
 
 def _token_major(NC, H, R, D, dtype, dev):
     return torch.empty(NC, R, H, D, dtype=dtype, device=dev).permute(0, 2, 1, 3)
-
-
-def _elementwise_steps(lay: ChunkLayout, alpha, Xf, X16, reverse: bool) -> None:
-    """Forward: X[c+1] = alpha_c X[c] + X[c+1].  Reverse: X[c] = alpha_c X[c+1] + X[c] (fp32, bf16 mirror)."""
-    if _lib.available() and Xf.is_cuda:
-        from . import chunk_kernels
-        chunk_kernels.state_scan(lay.first, lay.last, alpha, Xf, X16, reverse)
-        return
-    steps = lay.steps[::-1] if reverse else lay.steps
-    for idx in steps:
-        i = idx.long()
-        src, dst = (i + 1, i) if reverse else (i, i + 1)
-        al = alpha[i][..., None] if alpha.dim() == 3 else alpha[i][..., None, None]
-        r = Xf[dst] + al * Xf[src]
-        Xf[dst] = r
-        X16[dst] = r.to(X16.dtype)
 
 
 # --------------------------------------------------------------------------------------------------------
@@ -460,24 +639,8 @@ def gated_delta_rule_tc(q, k, v, beta, g, meta: VarlenMeta, scale: Optional[floa
     lay = ChunkLayout.of(meta, chunk or scalar_chunk(dk, dv))
     dt = torch.bfloat16 if q.is_cuda else q.dtype
     qp, kp, vp = lay.pack(q).to(dt), lay.pack(k).to(dt), lay.pack(v).to(dt)   # [NC, C, H, d]
-    bp = lay.pack(beta.float())                                      # [NC, C, H]
-    # the only token-sized derived operands: khat = k e^{b_last - b} and qbar = scale q e^{b}; every other scaling
-    # (beta, beta e^{b}) is folded into the C x C matrices
-    b, khat, qbar, alpha = _scalar_prep(qp, kp, None if g is None else lay.pack(g.float()), scale, dt)
-    d = b.permute(0, 2, 1)                                           # [NC, H, 64] view
-    beta_r = bp.permute(0, 2, 1)                                     # [NC, H, 64]
-    Akk = _Scores.apply(_hm(kp), _hm(kp), d, 1.0, MASK_STRICT, torch.float32) * beta_r[..., None]
-    Aqk = _Scores.apply(_hm(qp), _hm(kp), d, scale, MASK_TRIL, dt)
-    Tm = _TriInv.apply(Akk)                                          # [NC, H, 64, 64]
-    Tu = Tm * beta_r.to(dt)[..., None, :]
-    Tw = Tm * (beta_r * d.exp()).to(dt)[..., None, :]
-    u = bmm(Tu, _hm(vp), b_mn=True, token_major=True, out_dtype=dt)  # [NC, H, 64, dv] view of [NC, 64, H, dv]
-    w = bmm(Tw, _hm(kp), b_mn=True, token_major=True, out_dtype=dt)
-    S = _DeltaScan.apply(alpha, _hm(khat), w, u, lay)                # [NC, H, dk, dv]
-    v_new = bmm(w, S, b_mn=True, token_major=True, out_dtype=dt, alpha=-1.0, addend=u)      # u - w S
-    o = bmm(_hm(qbar), S, b_mn=True, token_major=True, out_dtype=dt)
-    o = bmm(Aqk, v_new, b_mn=True, token_major=True, out_dtype=dt, addend=o)
-    return lay.unpack(o.permute(0, 2, 1, 3)).to(v.dtype)
+    o = _GatedDelta.apply(qp, kp, vp, lay.pack(beta.float()), None if g is None else lay.pack(g.float()), scale, lay)
+    return lay.unpack(o).to(v.dtype)
 
 
 @_recomputable
@@ -490,55 +653,67 @@ def scalar_gla_tc(q, k, v, g, meta: VarlenMeta, scale: float = 1.0, chunk: Optio
     dt = torch.bfloat16 if q.is_cuda else q.dtype
     qp, kp, vp = lay.pack(q).to(dt), lay.pack(k).to(dt), lay.pack(v).to(dt)
     if G < H:
-        # q and k are shared by groups of H / G heads (Mamba2's B and C): they are never expanded.  The decay moves to the
-        # value side of the state update (S += k^T (v e^{b_last - b})) and to the rows of the inter-chunk output.
-        b = lay.pack(g.float()).cumsum(1)                              # [NC, C, H]
-        b_last = b[:, -1]
-        vhat = vp * (b_last[:, None] - b).exp().to(dt)[..., None]
-        d = b.permute(0, 2, 1)
-        Aqk = _Scores.apply(_hm(qp), _hm(kp), d, scale, MASK_TRIL, dt)  # [NC, H, C, C] from the G shared q / k
-        S = _DeltaScan.apply(b_last.exp(), _hm(kp), None, _hm(vhat), lay)
-        o = bmm(_hm(qp), S, b_mn=True, token_major=True, out_dtype=dt) * (b.exp() * scale).to(dt).permute(0, 2, 1)[..., None]
-        o = bmm(Aqk, _hm(vp), b_mn=True, token_major=True, out_dtype=dt, addend=o)
-        return lay.unpack(o.permute(0, 2, 1, 3)).to(v.dtype)
+        o = _GroupedScalarGla.apply(qp, kp, vp, lay.pack(g.float()), scale, lay)
+        return lay.unpack(o).to(v.dtype)
     b, khat, qbar, alpha = _scalar_prep(qp, kp, lay.pack(g.float()), scale, dt)
     d = b.permute(0, 2, 1)
     Aqk = _Scores.apply(_hm(qp), _hm(kp), d, scale, MASK_TRIL, dt)
-    S = _DeltaScan.apply(alpha, _hm(khat), None, _hm(vp), lay)
+    S = _DecayStates.apply(alpha, _hm(khat), _hm(vp), lay)
     o = bmm(_hm(qbar), S, b_mn=True, token_major=True, out_dtype=dt)
     o = bmm(Aqk, _hm(vp), b_mn=True, token_major=True, out_dtype=dt, addend=o)
     return lay.unpack(o.permute(0, 2, 1, 3)).to(v.dtype)
 
 
-class _GlaDiag(torch.autograd.Function):
-    """Diagonal 16 x 16 sub-blocks of the GLA intra-chunk scores (exact pairwise exponents) on the CUDA kernel."""
+class _Gla(torch.autograd.Function):
+    """The whole chunk pipeline of gated linear attention on packed 64-token chunks, on the kernels: q, k ``[NC, 64, H, dk]``, v
+    ``[NC, 64, H, dv]`` bf16, g ``[NC, 64, H, dk]`` fp32.  One node, so that the two halves of the output and of dv accumulate in
+    one GEMM each, and the channel-wise backward of preparation and diagonal sub-blocks is one kernel."""
 
     @staticmethod
-    def forward(ctx, qp, kp, b, scale):
+    def forward(ctx, q, k, v, g, scale, lay):
         from . import chunk_kernels
-        NC, C, H, dk = qp.shape
-        A = torch.zeros(NC, H, C, C, dtype=torch.float32, device=qp.device)
-        qp, kp, b = qp.contiguous(), kp.contiguous(), b.contiguous()
-        chunk_kernels.gla_diag_fwd(qp, kp, b, scale, A)
-        ctx.save_for_backward(qp, kp, b)
-        ctx.scale = scale
-        return A
+        q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+        NC, C, H, dk = q.shape
+        dv = v.shape[-1]
+        b, khat, qbar, qt, k3, alpha = chunk_kernels.gla_prep(q, k, g, scale)
+        vh = _hm(v)
+        S = _state_scan(lay, alpha, bgemm(_hm(khat), vh, a_mn=True, b_mn=True, out_dtype=torch.float32), q.dtype, reverse=False)
+        # off-diagonal sub-blocks: batch (chunk, I) multiplies the 16 query rows of sub-block I, re-based on the sub-block's
+        # first row, with the keys before it re-based on the same row; later keys are zero in k3
+        qt3 = qt[:, 16:].reshape(NC * 3, 16, H, dk)
+        k3 = k3.view(NC * 3, 48, H, dk)
+        A = chunk_kernels.gla_scores(q, k, b, bgemm(_hm(qt3), _hm(k3), alpha=scale), scale)
+        o = bgemm(_hm(qbar), S, b_mn=True, more=[(A, vh, False, True, 1)], out=_token_major(NC, H, C, dv, q.dtype, q.device))
+        ctx.save_for_backward(q, k, v, b, khat, qbar, qt3, k3, alpha, S, A)
+        ctx.cfg = (scale, lay)
+        return o.permute(0, 2, 1, 3)
 
     @staticmethod
-    def backward(ctx, dA):
+    def backward(ctx, do):
         from . import chunk_kernels
-        qp, kp, b = ctx.saved_tensors
-        dq = torch.zeros(qp.shape, dtype=torch.float32, device=qp.device)
-        dk = torch.zeros_like(dq)
-        db = torch.zeros_like(dq)
-        chunk_kernels.gla_diag_bwd(qp, kp, b, dA.float().contiguous(), dq, dk, db, ctx.scale)
-        return dq.to(qp.dtype), dk.to(kp.dtype), db, None
+        q, k, v, b, khat, qbar, qt3, k3, alpha, S, A = ctx.saved_tensors
+        scale, lay = ctx.cfg
+        NC, C, H, dk = q.shape
+        dv = v.shape[-1]
+        dt, dev = q.dtype, q.device
+        doh, vh = _hm(do.to(dt).contiguous()), _hm(v)
+        tok = lambda n: _token_major(NC, H, C, n, dt, dev)                                # noqa: E731
+        back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
+        Ln = _state_scan(lay, alpha, bgemm(_hm(qbar), doh, a_mn=True, b_mn=True), dt, reverse=True)
+        dvv = bgemm(_hm(khat), Ln, b_mn=True, more=[(A, doh, True, True, 1)], out=tok(dv))
+        dA = bgemm(doh, vh, mask=MASK_TRIL)
+        dqbar, dkhat = bgemm(doh, S, out=tok(dk)), bgemm(vh, Ln, out=tok(dk))
+        dblk = dA.view(NC, H, 4, 16, 64)[:, :, 1:, :, :48].permute(0, 2, 1, 3, 4).reshape(NC * 3, H, 16, 48)
+        dqt = torch.empty(NC, 64, H, dk, dtype=dt, device=dev)                            # rows of sub-block 0 are not read
+        dqt3 = bgemm(dblk, _hm(k3), b_mn=True, alpha=scale, out=_token_major(NC * 3, H, 16, dk, dt, dev))
+        dqt[:, 16:].copy_(back(dqt3).reshape(NC, 48, H, dk))
+        dk3 = bgemm(dblk, _hm(qt3), a_mn=True, b_mn=True, alpha=scale, out=_token_major(NC * 3, H, 48, dk, dt, dev))
+        dq, dkk, dg = chunk_kernels.gla_bwd(q, k, b, dA, back(dkhat), back(dqbar), dqt, back(dk3), _pair_dot(Ln, S, per_row=True), scale)
+        return dq, dkk, back(dvv), dg, None, None
 
 
 def _gla_diag(qp, kp, b, scale, sub: int = 16):
     """[NC, H, 64, 64] fp32 holding only the diagonal sub-blocks of A_ij = scale sum_d q_id k_jd exp(b_id - b_jd), j <= i."""
-    if _lib.available() and qp.is_cuda:
-        return _GlaDiag.apply(qp, kp, b, scale)
     NC, C, H, dk = qp.shape
     A = torch.zeros(NC, H, C, C, dtype=torch.float32, device=qp.device)
     tri = torch.tril(torch.ones(sub, sub, dtype=torch.bool, device=qp.device))
@@ -566,24 +741,22 @@ def gla_tc(q, k, v, g, meta: VarlenMeta, scale: Optional[float] = None, sub: int
     NC = qp.shape[0]
     ncol = C - sub
     if _lib.available() and q.is_cuda and C == 64 and sub == 16:
-        # cumulative decay and every scaled operand in one kernel (and one for the whole backward of this stage)
-        from .chunk_kernels import GlaPrep
-        b, khat, qbar, qt, k3, alpha = GlaPrep.apply(qp, kp, lay.pack(g.float()), scale)
-    else:
-        b = lay.pack(g.float()).cumsum(1)                                      # [NC, 64, H, dk]
-        b_last = b[:, -1]                                                      # [NC, H, dk]
-        alpha = b_last.exp()
-        khat = kp * (b_last[:, None] - b).exp().to(dt)
-        qbar = qp * (b.exp() * scale).to(dt)
-        # off-diagonal sub-blocks: batch (chunk, I) multiplies the 16 query rows of sub-block I, re-based on the
-        # sub-block's first row, with the keys before it re-based on the same row; later keys are zeroed
-        r = b[:, ::sub].detach()                                               # [NC, nb, H, dk]
-        qt = qp * (b - r.repeat_interleave(sub, 1)).exp().to(dt)
-        expo = r[:, 1:, None] - b[:, None, :ncol]                              # [NC, nb-1, ncol, H, dk]
-        keep = (torch.arange(ncol, device=q.device)[None, :] < (torch.arange(1, nb, device=q.device) * sub)[:, None])
-        keep = keep[None, :, :, None, None]
-        k3 = (kp[:, None, :ncol] * torch.where(keep, expo, expo.new_full((), float("-inf"))).exp().to(dt))
-    S = _DeltaScan.apply(alpha, _hm(khat), None, _hm(vp), lay)                 # [NC, H, dk, dv]
+        o = _Gla.apply(qp, kp, vp, lay.pack(g.float()), scale, lay)
+        return lay.unpack(o).to(v.dtype)
+    b = lay.pack(g.float()).cumsum(1)                                          # [NC, 64, H, dk]
+    b_last = b[:, -1]                                                          # [NC, H, dk]
+    alpha = b_last.exp()
+    khat = kp * (b_last[:, None] - b).exp().to(dt)
+    qbar = qp * (b.exp() * scale).to(dt)
+    # off-diagonal sub-blocks: batch (chunk, I) multiplies the 16 query rows of sub-block I, re-based on the
+    # sub-block's first row, with the keys before it re-based on the same row; later keys are zeroed
+    r = b[:, ::sub].detach()                                                   # [NC, nb, H, dk]
+    qt = qp * (b - r.repeat_interleave(sub, 1)).exp().to(dt)
+    expo = r[:, 1:, None] - b[:, None, :ncol]                                  # [NC, nb-1, ncol, H, dk]
+    keep = (torch.arange(ncol, device=q.device)[None, :] < (torch.arange(1, nb, device=q.device) * sub)[:, None])
+    keep = keep[None, :, :, None, None]
+    k3 = (kp[:, None, :ncol] * torch.where(keep, expo, expo.new_full((), float("-inf"))).exp().to(dt))
+    S = _DecayStates.apply(alpha, _hm(khat), _hm(vp), lay)                 # [NC, H, dk, dv]
     o = bmm(_hm(qbar), S, b_mn=True, token_major=True, out_dtype=dt)
     A = _gla_diag(qp, kp, b, scale, sub)
     # all off-diagonal sub-blocks in ONE batched GEMM
@@ -596,6 +769,75 @@ def gla_tc(q, k, v, g, meta: VarlenMeta, scale: Optional[float] = None, sub: int
     return lay.unpack(o.permute(0, 2, 1, 3)).to(v.dtype)
 
 
+class _VDecay(torch.autograd.Function):
+    """The chunk pipeline with a decay along the VALUE dimension (first pass of gated slot attention) on packed 64-token chunks,
+    on the kernels: q, k ``[NC, 64, H, dk]``, v ``[NC, 64, H, M]`` bf16, g ``[NC, 64, H, M]`` fp32.  Returns ``o`` in fp32, or with
+    ``softmax`` its softmax over the slots in bf16.  The state is carried transposed (``[M, dk]``)."""
+
+    @staticmethod
+    def forward(ctx, q, k, v, g, scale, softmax, lay):
+        from . import chunk_kernels
+        q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+        NC, C, H, dk = q.shape
+        M = v.shape[-1]
+        qh, kh = _hm(q), _hm(k)
+        b, vhat, v3, alpha = chunk_kernels.vdecay_prep(v, g)
+        v3 = v3.view(NC * 3, 48, H, M)
+        S = _state_scan(lay, alpha, bgemm(_hm(vhat), kh, a_mn=True, b_mn=True, out_dtype=torch.float32), q.dtype, reverse=False)
+        o1 = bgemm(qh, S, out=_token_major(NC, H, C, M, torch.float32, q.device))
+        P16 = torch.empty(NC, H, C, C, dtype=q.dtype, device=q.device)
+        P = bgemm(qh, kh, mask=MASK_TRIL, out_dtype=torch.float32, out16=P16)
+        P3 = P16.view(NC, H, 4, 16, C)[:, :, 1:, :, :48].permute(0, 2, 1, 3, 4).reshape(NC * 3, H, 16, 48)
+        acc = bgemm(P3, _hm(v3), b_mn=True, out=_token_major(NC * 3, H, 16, M, torch.float32, q.device))
+        o, qv = chunk_kernels.vdecay_out(o1.permute(0, 2, 1, 3), acc.permute(0, 2, 1, 3), P, v, b, scale, softmax)
+        ctx.save_for_backward(q, k, v, b, vhat, v3, alpha, S, P, P3, o)
+        ctx.cfg = (scale, softmax, lay)
+        return qv if softmax else o
+
+    @staticmethod
+    def backward(ctx, dout):
+        from . import chunk_kernels
+        q, k, v, b, vhat, v3, alpha, S, P, P3, o = ctx.saved_tensors
+        scale, softmax, lay = ctx.cfg
+        NC, C, H, dk = q.shape
+        M = v.shape[-1]
+        dt, dev = q.dtype, q.device
+        qh, kh = _hm(q), _hm(k)
+        back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
+        dqv, d32 = (dout.to(dt).contiguous(), None) if softmax else (None, dout.float().contiguous())
+        do, do1, dacc = chunk_kernels.vdecay_bwd1(o, dqv, d32, b, scale)
+        do1h, dacch = _hm(do1), _hm(dacc.view(NC * 3, 16, H, M))
+        Ln = _state_scan(lay, alpha, bgemm(do1h, qh, a_mn=True, b_mn=True), dt, reverse=True)
+        dvhat = bgemm(kh, Ln, out=_token_major(NC, H, C, M, dt, dev))
+        dv3 = bgemm(P3, dacch, a_mn=True, b_mn=True, out=_token_major(NC * 3, H, 48, M, dt, dev))
+        # gradient of the scores: off-diagonal sub-blocks by GEMM, the diagonal ones are pairwise sums like GLA's own scores
+        dP = chunk_kernels.gla_scores(do, v, b, bgemm(dacch, _hm(v3)), 1.0)
+        dq = bgemm(do1h, S, b_mn=True, more=[(dP, kh, False, True, 1)], out=_token_major(NC, H, C, dk, dt, dev))
+        dkk = bgemm(_hm(vhat), Ln, b_mn=True, more=[(dP, qh, True, True, 1)], out=_token_major(NC, H, C, dk, dt, dev))
+        dv, dg = chunk_kernels.vdecay_bwd2(P, v, b, do, o, back(dvhat), back(dv3), _pair_dot(Ln, S, per_row=True), scale)
+        return back(dq), back(dkk), dv, dg, None, None, None
+
+
+def gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> Optional[torch.Tensor]:
+    """Both passes of gated slot attention without leaving the chunk layout between them (the slots' softmax rides on the first
+    pass); None where the kernels do not apply."""
+    from . import chunk_kernels
+    M = s.shape[-1]
+    if not (_lib.available() and q.is_cuda and M <= chunk_kernels.VDECAY_SOFTMAX_MAX and M % 8 == 0 and v.dtype == torch.bfloat16):
+        return None
+    return _gsa_chunks(q, k, v, s, g, meta, scale)
+
+
+@_recomputable
+def _gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> torch.Tensor:
+    lay = ChunkLayout.of(meta)
+    dt = torch.bfloat16
+    qp, kp, vp, sp = (lay.pack(t).to(dt) for t in (q, k, v, s))
+    gp = lay.pack(g.float())
+    qv = _VDecay.apply(qp, kp, sp, gp, scale, True, lay)
+    return lay.unpack(_Gla.apply(qv, sp, vp, gp, 1.0, lay)).to(v.dtype)
+
+
 @_recomputable
 def gla_vdecay_tc(q, k, v, gv, meta: VarlenMeta, scale: float, sub: int = 16) -> torch.Tensor:
     """``S_t = S_{t-1} diag(exp gv_t) + k_t v_t^T,  o_t = scale q_t^T S_t``: the state decays along its VALUE dimension
@@ -606,13 +848,14 @@ def gla_vdecay_tc(q, k, v, gv, meta: VarlenMeta, scale: float, sub: int = 16) ->
     dt = torch.bfloat16 if q.is_cuda else q.dtype
     C = lay.chunk
     qp, kp, vp = lay.pack(q).to(dt), lay.pack(k).to(dt), lay.pack(v).to(dt)
+    if _lib.available() and q.is_cuda and C == 64 and sub == 16 and vp.shape[-1] % 8 == 0:
+        return lay.unpack(_VDecay.apply(qp, kp, vp, lay.pack(gv.float()), scale, False, lay))
     b = lay.pack(gv.float()).cumsum(1)                                         # [NC, 64, H, dv]
     b_last = b[:, -1]
     vhat = vp * (b_last[:, None] - b).exp().to(dt)
-    St = _DeltaScan.apply(b_last.exp(), _hm(vhat), None, _hm(kp), lay)         # [NC, H, dv, dk]
+    St = _DecayStates.apply(b_last.exp(), _hm(vhat), _hm(kp), lay)         # [NC, H, dv, dk]
     o = bmm(_hm(qp), St, token_major=True, out_dtype=torch.float32).permute(0, 2, 1, 3) * b.exp()   # [NC, 64, H, dv]
     P = bgemm_scores_plain(qp, kp)                                             # [NC, H, 64, 64] tril(q k^T)
-    use_kernel = _lib.available() and q.is_cuda and C == 64 and sub == 16
     nb, ncol, NC = C // sub, C - sub, qp.shape[0]
     dv = vp.shape[-1]
     # off-diagonal sub-blocks, all in ONE batched GEMM: batch (chunk, I) multiplies the 16 score rows of sub-block I with
@@ -628,17 +871,13 @@ def gla_vdecay_tc(q, k, v, gv, meta: VarlenMeta, scale: float, sub: int = 16) ->
               out_dtype=torch.float32)                                         # [NC*(nb-1), H, sub, dv] over [.., sub, H, dv]
     acc = acc.permute(0, 2, 1, 3).reshape(NC, ncol, H, dv) * (b[:, sub:] - r[:, 1:].repeat_interleave(sub, 1)).exp()
     o = o + torch.nn.functional.pad(acc, (0, 0, 0, 0, sub, 0))
-    if use_kernel:
-        from .chunk_kernels import VdecayDiag
-        o = o + VdecayDiag.apply(P, vp, b)                                     # all diagonal sub-blocks, exact
-    else:
-        tri = torch.tril(torch.ones(sub, sub, dtype=torch.bool, device=q.device))
-        parts = []
-        for i in range(nb):
-            rows = slice(i * sub, (i + 1) * sub)
-            dd = (b[:, rows, None] - b[:, None, rows]).masked_fill(~tri[None, :, :, None, None], float("-inf")).exp()
-            parts.append(torch.einsum("nhij,njhc,nijhc->nihc", P[:, :, rows, rows].float(), vp[:, rows].float(), dd))
-        o = o + torch.cat(parts, 1)
+    tri = torch.tril(torch.ones(sub, sub, dtype=torch.bool, device=q.device))
+    parts = []
+    for i in range(nb):
+        rows = slice(i * sub, (i + 1) * sub)
+        dd = (b[:, rows, None] - b[:, None, rows]).masked_fill(~tri[None, :, :, None, None], float("-inf")).exp()
+        parts.append(torch.einsum("nhij,njhc,nijhc->nihc", P[:, :, rows, rows].float(), vp[:, rows].float(), dd))
+    o = o + torch.cat(parts, 1)
     o = o * scale
     return lay.unpack(o)
 

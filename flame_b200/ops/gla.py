@@ -101,7 +101,7 @@ def gla_state_passing(q, k, v, g, meta: VarlenMeta, scale: Optional[float], sl) 
 def gsa(q, k, v, s, g, meta: VarlenMeta, scale: Optional[float] = None) -> torch.Tensor:
     """Two chained passes (fla/ops/gsa/chunk.py:826-871): slots written with key k and value s under a value-side
     decay g; softmax over the slot read-out; values read through the slot memory with a key-side decay g."""
-    from .chunked import gla_tc, gla_vdecay_tc
+    from .chunked import gla_tc, gla_vdecay_tc, gsa_chunks
     sl = getattr(meta, "sequence_slice", None)
     if sl is not None:
         # context parallelism cut the row inside documents: both passes are diagonal-decay recurrences, each hands its
@@ -113,6 +113,9 @@ def gsa(q, k, v, s, g, meta: VarlenMeta, scale: Optional[float] = None) -> torch
         return gla_state_passing(qv, s, v, g, meta, 1.0, sl).to(v.dtype)
     K = q.shape[-1]
     scale = K ** -0.5 if scale is None else scale
+    o = gsa_chunks(q, k, v, s, g, meta, scale)
+    if o is not None:
+        return o
     ok = gla_vdecay_tc(q, k, s, g, meta, scale)
     qv = torch.softmax(ok.float(), -1).to(v.dtype)
     return gla_tc(qv, s, v, g, meta, scale=1.0).to(v.dtype)

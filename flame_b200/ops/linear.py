@@ -133,7 +133,7 @@ class _LinearFn(torch.autograd.Function):
                 c += w.shape[0]
         gb = None
         if ctx.has_bias and ctx.needs_input_grad[1]:
-            gb = dy2.float().sum(0).to(dy.dtype)
+            gb = dy2.sum(0, dtype=torch.float32).to(dy.dtype)
         return (dx, gb, None, *grads)
 
 

@@ -86,6 +86,21 @@ def test_gated_delta_rule_tc_matches_recurrence(gated, chunk):
         assert rel_err(a, b) < 1e-4
 
 
+@pytest.mark.parametrize("G,H,scale,chunk", [(1, 4, 1.0, 64), (2, 6, 0.3, 64), (2, 4, 0.5, 128), (3, 3, 1.0, 64)])
+def test_scalar_gla_grouped_heads_match_expanded_heads(G, H, scale, chunk):
+    """Queries and keys shared by groups of heads against the same ones repeated per head: output and every gradient (fp32
+    sums in another order: 1e-5)."""
+    torch.manual_seed(3)
+    meta = _meta(LENS)
+    T, dk, dv = sum(LENS), 16, 8
+    q, k, v, graw = _leaf(T, G, dk), _leaf(T, G, dk), _leaf(T, H, dv), _leaf(T, H)
+    ins = [q, k, v, graw]
+    ref = _run(lambda: scalar_gla_tc(q.repeat_interleave(H // G, 1), k.repeat_interleave(H // G, 1), v, -F.softplus(graw), meta, scale, chunk), ins)
+    out = _run(lambda: scalar_gla_tc(q, k, v, -F.softplus(graw), meta, scale, chunk), ins)
+    for a, b in zip(out, ref):
+        assert rel_err(a, b) < 1e-5
+
+
 def test_scalar_gla_tc_matches_chunk_reference():
     torch.manual_seed(3)
     meta = _meta(LENS)

@@ -87,6 +87,74 @@ def test_bgemm_mask_decay_and_state_step():
     assert rel_err(X16, want16) < 1e-2
 
 
+@pytest.mark.parametrize("M,N,K,K2", [(16, 48, 128, 64), (64, 64, 64, 72), (64, 128, 128, 64), (128, 136, 256, 16), (130, 264, 64, 200)])
+def test_bgemm_sums_of_products(M, N, K, K2):
+    """Several products in one accumulator (added and subtracted, every storage sense), a factor per row, a sum over the heads
+    of a group; fp32 accumulation of bf16 operands: 1e-5 in fp32, 2^-8 after rounding to bf16."""
+    from flame_b200.ops.bgemm import bgemm
+    torch.manual_seed(11)
+    hi, G, r = 3, 2, 3
+    t = lambda *s: torch.randn(*s, device=DEV).to(torch.bfloat16)  # noqa: E731
+    pad = lambda n: (n + 7) // 8 * 8  # noqa: E731
+    a, b = t(hi, G * r, M, K), t(hi, G, N, K)                       # b is shared by the heads of a group
+    a2, b2 = t(hi, G * r, K2, pad(M))[..., :M], t(hi, G * r, K2, pad(N))[..., :N]
+    scale = torch.randn(hi, M, G * r, device=DEV).permute(0, 2, 1)
+    bx = b.repeat_interleave(r, 1)
+    one, two = a.float() @ bx.float().transpose(-1, -2), a2.float().transpose(-1, -2) @ b2.float()
+    Np = pad(N)
+    out = torch.empty(hi, G * r, M, Np, device=DEV)[..., :N]
+    bgemm(a, b, alpha=0.5, out=out, more=[(a2, b2, True, True, -1)], rowscale=scale)
+    assert rel_err(out, 0.5 * (one - two) * scale[..., None]) < 1e-5
+    out16 = torch.empty(hi, M, G, Np, device=DEV, dtype=torch.bfloat16)[..., :N].permute(0, 2, 1, 3)
+    bgemm(a, b, out=out16, sum_lo=r, more=[(a2, b2, True, True, 1)])
+    assert rel_err(out16, (one + two).reshape(hi, G, r, M, N).sum(2)) < 4e-3
+
+
+@pytest.mark.parametrize("gates", ["mild", "hard"])
+@pytest.mark.parametrize("dk,dv,lens", [(64, 64, [1, 64, 65]), (72, 40, [15, 17, 48, 200]), (256, 128, [130, 63])])
+def test_gla_edges(dk, dv, lens, gates):
+    """Head sizes that are no multiple of the kernels' channel tiles, documents around sub-block and chunk edges, gates so hard
+    that a re-based exponent would overflow if any were positive; against the fp32 recurrence (bf16 operands: 2e-2)."""
+    from flame_b200.ops import linear_attn as la
+    from flame_b200.ops.chunked import gla_tc
+    torch.manual_seed(12)
+    meta = _meta(lens)
+    T, H = sum(lens), 3
+    leaf = lambda *s: torch.randn(*s, device=DEV, dtype=torch.bfloat16).requires_grad_(True)  # noqa: E731
+    q, k, v, graw = leaf(T, H, dk), leaf(T, H, dk), leaf(T, H, dv), leaf(T, H, dk)
+    ins = [q, k, v, graw]
+    gate = lambda: F.logsigmoid(graw.float() * 2) / 4 if gates == "mild" else -F.softplus(graw.float()) * 20  # noqa: E731
+    ref = _run(lambda c: la.gla_recurrent(c(q), c(k), c(v), gate(), meta), ins, True)
+    out = _run(lambda c: gla_tc(c(q), c(k), c(v), gate(), meta), ins, False)
+    for a, b in zip(out, ref):
+        assert rel_err(a, b) < 2e-2
+
+
+@pytest.mark.parametrize("M,dk,lens", [(8, 64, [1, 16, 17]), (64, 72, [63, 65, 130]), (200, 64, [100, 48])])
+def test_gsa_edges(M, dk, lens):
+    """Slots around the kernels' thread counts, documents around sub-block and chunk edges; the fused pair of passes and the first
+    pass alone (the form context parallelism uses) against the fp32 recurrences."""
+    from flame_b200.ops import linear_attn as la
+    from flame_b200.ops.chunked import gla_vdecay_tc
+    from flame_b200.ops.gla import gsa
+    torch.manual_seed(13)
+    meta = _meta(lens)
+    T, H, dv = sum(lens), 2, 64
+    leaf = lambda *s: torch.randn(*s, device=DEV, dtype=torch.bfloat16).requires_grad_(True)  # noqa: E731
+    q, k, v, sl, graw = leaf(T, H, dk), leaf(T, H, dk), leaf(T, H, dv), leaf(T, H, M), leaf(T, H, M)
+    gate = lambda: F.logsigmoid(graw.float()) / 4  # noqa: E731
+    ins = [q, k, v, sl, graw]
+    ref = _run(lambda c: la.gsa_recurrent(c(q), c(k), c(v), c(sl), gate(), meta, 0.3), ins, True)
+    out = _run(lambda c: gsa(c(q), c(k), c(v), c(sl), gate(), meta, 0.3), ins, False)
+    for a, b in zip(out, ref):
+        assert rel_err(a, b) < 4e-2
+    ins = [q, k, sl, graw]
+    ref = _run(lambda c: la.gla_recurrent_vdecay(c(q), c(k), c(sl), gate(), meta, 0.3), ins, True)
+    out = _run(lambda c: gla_vdecay_tc(c(q), c(k), c(sl), gate(), meta, 0.3), ins, False)
+    for a, b in zip(out, ref):
+        assert rel_err(a, b) < 2e-2
+
+
 def test_tri_inverse_and_l2norm():
     from flame_b200.ops.chunk_kernels import l2norm, tri_inverse
     torch.manual_seed(2)
