@@ -17,7 +17,10 @@
 // tokens x 2,048 channels; the forward needs two sweeps, the backward three.  Everything else has to stay below that in
 // issue slots: sweeps (1), (3), (4) give a thread a whole channel (16 states, B / C read as float4 broadcasts, no
 // shuffles), sweep (6) gives it 2 channels x 4 states, so that the sums over states and over channels are mostly
-// additions in registers, finished through shared memory; pairs of states use the packed fp32x2 instructions.
+// additions in registers, finished through shared memory; pairs of states use the packed fp32x2 instructions.  Every
+// sweep fetches its operands a group of four steps ahead: waiting for memory at each group, not the MUFU, set the pace before.
+// At that size with gate and softplus, before and after: (1) 0.44 -> 0.31 ms, (3) 0.84 -> 0.47, (4) 0.59 -> 0.36,
+// (6) 2.17 -> 1.63.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -122,20 +125,40 @@ __device__ __forceinline__ void load_A(const ScanArgs& a, int d, bool live, f2* 
   }
 }
 
-// a channel's column of a row-major operand, starting at the chunk's first token; rows by 32-bit offsets
-template <bool RAW>
-struct DeltaCol {
-  const __nv_bfloat16* r;
-  const float* f;
+// A channel's column of a row-major operand, starting at the chunk's first token; rows by 32-bit offsets.  Loads and
+// conversions are apart: the loads go out together, a group of steps ahead of their use (ncu on the form that loaded a group
+// right before its use: 10 of 16 stall cycles per issue on these loads, the exponential pipe at 0.33 to 0.60 of its peak), and
+// as read-only loads they may pass the kernels' stores.
+typedef unsigned short u16;
+__device__ __forceinline__ float bf(u16 v) { return __uint_as_float((uint32_t)v << 16); }
+struct Col16 {
+  const u16* p;
   int stride;
-  __device__ __forceinline__ DeltaCol(const ScanArgs& a, long long row0, int d) : stride(a.ds) {
-    if (RAW) r = (const __nv_bfloat16*)a.dl + row0 * a.ds + d;
-    else f = (const float*)a.dl + row0 * a.ds + d;
-  }
-  __device__ __forceinline__ float operator()(int t) const { return RAW ? softplus(__bfloat162float(r[t * stride])) : f[t * stride]; }
+  __device__ __forceinline__ Col16(const __nv_bfloat16* base, long long row0, int stride_, int d)
+      : p(reinterpret_cast<const u16*>(base) + row0 * stride_ + d), stride(stride_) {}
+  __device__ __forceinline__ u16 operator()(int t, bool ok) const { return ok ? __ldg(p + t * stride) : (u16)0; }
+};
+template <bool RAW>
+struct DeltaCol;
+template <>
+struct DeltaCol<true> {
+  typedef u16 T;
+  Col16 c;
+  __device__ __forceinline__ DeltaCol(const ScanArgs& a, long long row0, int d) : c((const __nv_bfloat16*)a.dl, row0, a.ds, d) {}
+  __device__ __forceinline__ T operator()(int t, bool ok) const { return c(t, ok); }
+  static __device__ __forceinline__ float value(T v, bool ok) { return ok ? softplus(bf(v)) : 0.f; }
+};
+template <>
+struct DeltaCol<false> {
+  typedef float T;
+  const float* p;
+  int stride;
+  __device__ __forceinline__ DeltaCol(const ScanArgs& a, long long row0, int d) : p((const float*)a.dl + row0 * a.ds + d), stride(a.ds) {}
+  __device__ __forceinline__ T operator()(int t, bool ok) const { return ok ? __ldg(p + t * stride) : 0.f; }
+  static __device__ __forceinline__ float value(T v, bool) { return v; }
 };
 
-constexpr int PF = 8;  // steps whose operands are fetched together
+constexpr int PF = 4;  // steps whose operands are fetched together, one group ahead
 
 // (1)
 template <bool RAW>
@@ -153,16 +176,27 @@ __global__ void __launch_bounds__(CT) sscan_local_kernel(ScanArgs a, float* __re
   for (int p = 0; p < N / 2; ++p) h[p] = 0ull;
   float s = 0.f;
   const DeltaCol<RAW> delta(a, row0, d);
-  const __nv_bfloat16* pu = a.u + row0 * a.us + d;
+  const Col16 ucol(a.u, row0, a.us, d);
+  typename DeltaCol<RAW>::T nd[PF];
+  u16 nu[PF];
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int i = 0; i < PF; ++i) {
+      const bool ok = live && t0 + i < len;
+      nd[i] = delta(t0 + i, ok);
+      nu[i] = ucol(t0 + i, ok);
+    }
+  };
+  fetch(0);
   __syncthreads();
   for (int t0 = 0; t0 < len; t0 += PF) {
     float dl[PF], u[PF];
 #pragma unroll
     for (int i = 0; i < PF; ++i) {
-      const bool ok = live && t0 + i < len;
-      dl[i] = ok ? delta(t0 + i) : 0.f;
-      u[i] = ok ? __bfloat162float(pu[(t0 + i) * a.us]) : 0.f;
+      dl[i] = DeltaCol<RAW>::value(nd[i], live && t0 + i < len);
+      u[i] = bf(nu[i]);
     }
+    if (t0 + PF < len) fetch(t0 + PF);
 #pragma unroll
     for (int i = 0; i < PF; ++i) {
       const F4* b4 = reinterpret_cast<const F4*>(sB + (t0 + i) * N);
@@ -236,7 +270,19 @@ __global__ void __launch_bounds__(CT, 4) sscan_out_kernel(ScanArgs a, float* __r
   for (int p = 0; p < N / 2; ++p) h[p] = pk(s0[(2 * p) * a.DiP], s0[(2 * p + 1) * a.DiP]);
   const float Dd = live ? a.Dv[d] : 0.f;
   const DeltaCol<RAW> delta(a, row0, d);
-  const __nv_bfloat16 *pu = a.u + row0 * a.us + d, *pz = GATE ? a.z + row0 * a.zs + d : nullptr;
+  const Col16 ucol(a.u, row0, a.us, d), zcol(GATE ? a.z : a.u, row0, GATE ? a.zs : a.us, d);
+  typename DeltaCol<RAW>::T nd[PF];
+  u16 nu[PF], nz[PF];
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int i = 0; i < PF; ++i) {
+      const bool ok = live && t0 + i < len;
+      nd[i] = delta(t0 + i, ok);
+      nu[i] = ucol(t0 + i, ok);
+      if (GATE) nz[i] = zcol(t0 + i, ok);
+    }
+  };
+  fetch(0);
   y += row0 * a.Di + d;
   out += row0 * a.Di + d;
   __syncthreads();
@@ -254,11 +300,11 @@ __global__ void __launch_bounds__(CT, 4) sscan_out_kernel(ScanArgs a, float* __r
     float dl[PF], u[PF], zz[PF];
 #pragma unroll
     for (int i = 0; i < PF; ++i) {
-      const bool ok = live && t0 + i < len;
-      dl[i] = ok ? delta(t0 + i) : 0.f;
-      u[i] = ok ? __bfloat162float(pu[(t0 + i) * a.us]) : 0.f;
-      if (GATE) zz[i] = ok ? __bfloat162float(pz[(t0 + i) * a.zs]) : 0.f;
+      dl[i] = DeltaCol<RAW>::value(nd[i], live && t0 + i < len);
+      u[i] = bf(nu[i]);
+      if (GATE) zz[i] = bf(nz[i]);
     }
+    if (t0 + PF < len) fetch(t0 + PF);
 #pragma unroll
     for (int i = 0; i < PF; ++i) {
       const F4* b4 = reinterpret_cast<const F4*>(sB + (t0 + i) * N);
@@ -298,20 +344,33 @@ __global__ void __launch_bounds__(CT) sscan_local_bwd_kernel(ScanArgs a, const _
 #pragma unroll
   for (int p = 0; p < N / 2; ++p) g[p] = 0ull;
   const DeltaCol<RAW> delta(a, row0, d);
-  const __nv_bfloat16 *po = dout + row0 * a.Di + d, *pz = GATE ? a.z + row0 * a.zs + d : nullptr;
-  __syncthreads();
-  for (int t0 = (len - 1) / PF * PF; t0 >= 0; t0 -= PF) {
-    float dl[PF], dy[PF];
+  const Col16 ocol(dout, row0, a.Di, d), zcol(GATE ? a.z : dout, row0, GATE ? a.zs : a.Di, d);
+  typename DeltaCol<RAW>::T nd[PF];
+  u16 no[PF], nz[PF];
+  auto fetch = [&](int t0) {
 #pragma unroll
     for (int i = 0; i < PF; ++i) {
       const bool ok = live && t0 + i < len;
-      dl[i] = ok ? delta(t0 + i) : 0.f;
-      dy[i] = ok ? __bfloat162float(po[(t0 + i) * a.Di]) : 0.f;
-      if (GATE && ok) {
-        const float z = __bfloat162float(pz[(t0 + i) * a.zs]);
+      nd[i] = delta(t0 + i, ok);
+      no[i] = ocol(t0 + i, ok);
+      if (GATE) nz[i] = zcol(t0 + i, ok);
+    }
+  };
+  const int t_first = (len - 1) / PF * PF;
+  fetch(t_first);
+  __syncthreads();
+  for (int t0 = t_first; t0 >= 0; t0 -= PF) {
+    float dl[PF], dy[PF];
+#pragma unroll
+    for (int i = 0; i < PF; ++i) {
+      dl[i] = DeltaCol<RAW>::value(nd[i], live && t0 + i < len);
+      dy[i] = bf(no[i]);
+      if (GATE) {
+        const float z = bf(nz[i]);
         dy[i] *= z * sigm(z);
       }
     }
+    if (t0 > 0) fetch(t0 - PF);
 #pragma unroll
     for (int i = PF - 1; i >= 0; --i) {
       const F4* c4 = reinterpret_cast<const F4*>(sC + (t0 + i) * N);
@@ -356,8 +415,8 @@ template <bool RAW, bool GATE>
 __global__ void __launch_bounds__(BT, 3) sscan_bwd_kernel(ScanArgs a, const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y,
                                                           const float* __restrict__ st, const float* __restrict__ adj,
                                                           __nv_bfloat16* __restrict__ du, void* __restrict__ ddl,
-                                                          __nv_bfloat16* __restrict__ dz, float* __restrict__ dA, float* __restrict__ part,
-                                                          float* __restrict__ dD, long long T) {
+                                                          __nv_bfloat16* __restrict__ dz, int dzs, float* __restrict__ dA,
+                                                          float* __restrict__ part, float* __restrict__ dD, long long T) {
   extern __shared__ __align__(16) unsigned char raw_smem[];
   BwdSmem& s = *reinterpret_cast<BwdSmem*>(raw_smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = lane & 3, cg = lane >> 2;
@@ -389,35 +448,50 @@ __global__ void __launch_bounds__(BT, 3) sscan_bwd_kernel(ScanArgs a, const __nv
   float dD0 = 0.f, dD1 = 0.f;
   const int st_ch = tid % BC, st_t = tid / BC, st_d = d0 + st_ch;
   const bool st_live = st_d < a.Di;
-  const DeltaCol<RAW> delta(a, row0, st_d);
-  const long long col = row0 * a.Di + st_d;
-  const __nv_bfloat16 *pu = a.u + row0 * a.us + st_d, *po = dout + col, *pz = GATE ? a.z + row0 * a.zs + st_d : nullptr;
-  const __nv_bfloat16* py = GATE ? y + col : nullptr;
-  __nv_bfloat16* pdz = GATE ? dz + col : nullptr;
+  const DeltaCol<RAW> delta(a, row0, st_d), fdelta(a, row0, fd);
+  const Col16 ucol(a.u, row0, a.us, st_d), ocol(dout, row0, a.Di, st_d), zcol(GATE ? a.z : dout, row0, GATE ? a.zs : a.Di, st_d),
+      ycol(GATE ? y : dout, row0, a.Di, st_d), fu(a.u, row0, a.us, fd);
+  __nv_bfloat16* pdz = GATE ? dz + row0 * dzs + st_d : nullptr;
 
   for (int seg = (len - 1) / SEG; seg >= 0; --seg) {
     const int tb = seg * SEG;
     __syncthreads();
-    // a thread stages one channel of eight steps
-#pragma unroll 4
-    for (int i = 0; i < SEG * BC / BT; ++i) {
-      const int t = i * (BT / BC) + st_t;
-      const bool ok = tb + t < len && st_live;
-      float dlv = 0.f, uv = 0.f, dyv = 0.f;
-      if (ok) {
-        const int r = tb + t;
-        dlv = delta(r);
-        uv = __bfloat162float(pu[r * a.us]);
-        dyv = __bfloat162float(po[r * a.Di]);
+    // a thread stages one channel of eight steps; all of its loads go out first, the kept states' with them
+    const float* hs = st + ((long long)c * NSEG + seg) * N * a.DiP + dc;
+    float2 hv[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) hv[p] = __ldg(reinterpret_cast<const float2*>(hs + (q * 4 + p) * a.DiP));
+    {
+      constexpr int NT = SEG * BC / BT;
+      typename DeltaCol<RAW>::T rd[NT];
+      u16 ru[NT], ro[NT], rz[NT], ry[NT];
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        const int r = tb + i * (BT / BC) + st_t;
+        const bool ok = r < len && st_live;
+        rd[i] = delta(r, ok);
+        ru[i] = ucol(r, ok);
+        ro[i] = ocol(r, ok);
         if (GATE) {
-          const float z = __bfloat162float(pz[r * a.zs]), sg = sigm(z), sl = z * sg;
-          pdz[r * a.Di] = __float2bfloat16(dyv * __bfloat162float(py[r * a.Di]) * (sg + sl * (1.f - sg)));
-          dyv *= sl;
+          rz[i] = zcol(r, ok);
+          ry[i] = ycol(r, ok);
         }
       }
-      reinterpret_cast<float2*>(&s.dl[t][0])[st_ch] = make_float2(dlv, dlv);
-      reinterpret_cast<float2*>(&s.x[t][0])[st_ch] = make_float2(dlv * uv, dlv * uv);
-      reinterpret_cast<float2*>(&s.dy[t][0])[st_ch] = make_float2(dyv, dyv);
+#pragma unroll
+      for (int i = 0; i < NT; ++i) {
+        const int t = i * (BT / BC) + st_t, r = tb + t;
+        const bool ok = r < len && st_live;
+        const float dlv = DeltaCol<RAW>::value(rd[i], ok), uv = bf(ru[i]);
+        float dyv = bf(ro[i]);
+        if (GATE) {
+          const float z = bf(rz[i]), sg = sigm(z), sl = z * sg;
+          if (ok) pdz[r * dzs] = __float2bfloat16(dyv * bf(ry[i]) * (sg + sl * (1.f - sg)));
+          dyv *= sl;
+        }
+        reinterpret_cast<float2*>(&s.dl[t][0])[st_ch] = make_float2(dlv, dlv);
+        reinterpret_cast<float2*>(&s.x[t][0])[st_ch] = make_float2(dlv * uv, dlv * uv);
+        reinterpret_cast<float2*>(&s.dy[t][0])[st_ch] = make_float2(dyv, dyv);
+      }
     }
     for (int i = tid; i < SEG * N; i += BT) {
       const int t = i / N, n = i % N;
@@ -425,13 +499,10 @@ __global__ void __launch_bounds__(BT, 3) sscan_bwd_kernel(ScanArgs a, const __nv
       s.B[t][n] = ok ? load_bc(a, a.B, a.bs, row0 + tb + t, n) : 0.f;
       s.C[t][n] = ok ? load_bc(a, a.C, a.cs, row0 + tb + t, n) : 0.f;
     }
-    const float* hs = st + ((long long)c * NSEG + seg) * N * a.DiP + dc;
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
-      const int n = q * 4 + 2 * p;
-      const float2 lo = *reinterpret_cast<const float2*>(hs + n * a.DiP), hi = *reinterpret_cast<const float2*>(hs + (n + 1) * a.DiP);
-      h[0][p] = pk(lo.x, hi.x);
-      h[1][p] = pk(lo.y, hi.y);
+      h[0][p] = pk(hv[2 * p].x, hv[2 * p + 1].x);
+      h[1][p] = pk(hv[2 * p].y, hv[2 * p + 1].y);
     }
     __syncthreads();
     // states entering steps 4, 8, 12
@@ -455,6 +526,15 @@ __global__ void __launch_bounds__(BT, 3) sscan_bwd_kernel(ScanArgs a, const __nv
       if (sb < 3) {
         const F4 k0 = *reinterpret_cast<const F4*>(&s.ck[sb][0][tid]), k1 = *reinterpret_cast<const F4*>(&s.ck[sb][1][tid]);
         h[0][0] = k0.a, h[0][1] = k0.b, h[1][0] = k1.a, h[1][1] = k1.b;
+      }
+      // what the finishing lanes need of u and raw, on its way while the states are recomputed
+      const int ft = tb + sb * 4 + (lane >> 3);
+      const bool f0 = ft < len && fd < a.Di, f1 = ft < len && fd + 1 < a.Di;
+      const u16 fu0 = fu(ft, f0), fu1 = f1 ? __ldg(fu.p + ft * fu.stride + 1) : (u16)0;
+      u16 fr0 = 0, fr1 = 0;
+      if constexpr (RAW) {
+        fr0 = fdelta(ft, f0);
+        fr1 = f1 ? __ldg(fdelta.c.p + ft * fdelta.c.stride + 1) : (u16)0;
       }
       f2 dec[4][2][2], w[4][2][2];
 #pragma unroll
@@ -522,11 +602,11 @@ __global__ void __launch_bounds__(BT, 3) sscan_bwd_kernel(ScanArgs a, const __nv
           for (int k = 0; k < 2; ++k) {
             const int d = fd + k;
             if (d < a.Di) {
-              const float uv = __bfloat162float(a.u[row * a.us + d]);
+              const float uv = bf(k ? fu1 : fu0);
               float dd = fmaf(uv, m2[k], m1[k] * LN2);
               du[row * a.Di + d] = __float2bfloat16(fmaf(k ? D1 : D0, dyv[k], dlv[k] * m2[k]));
               if (RAW) {
-                dd *= sigm(__bfloat162float(((const __nv_bfloat16*)a.dl)[row * a.ds + d]));
+                dd *= sigm(bf(k ? fr1 : fr0));
                 ((__nv_bfloat16*)ddl)[row * a.Di + d] = __float2bfloat16(dd);
               } else {
                 ((float*)ddl)[row * a.Di + d] = dd;
@@ -649,12 +729,12 @@ int fb_sscan_fwd(const void* u, long long us, const void* dl, long long ds, int 
 }
 
 // Backward.  dout: gradient of the (gated) output, bf16 [T, Di]; y: ungated output (with z).  adj: fp32 [NC, 16, DiP] scratch;
-// du: bf16 [T, Di]; ddl: bf16 (raw) or fp32 [T, Di]; dz: bf16 [T, Di] (with z); dB, dC: [T, 16] in B's type.  Partial results
+// du: bf16 [T, Di]; ddl: bf16 (raw) or fp32 [T, Di]; dz: bf16 [T, Di], row stride dzs (with z); dB, dC: [T, 16] in B's type.  Partial results
 // for the caller to add over the chunks: dA [NC, 16, DiP], dD [NC, DiP].  part: fp32 [channel blocks, T, 32] scratch.
 int fb_sscan_bwd(const void* u, long long us, const void* dl, long long ds, int raw, const void* z, long long zs, const void* B, long long bs,
                  const void* C, long long cs, int bc16, const float* A, const float* Dv, const int* inv, const long long* first,
                  const long long* last, int n_docs, const float* st, const float* sdl, const void* y, const void* dout, float* adj, void* du,
-                 void* ddl, void* dz, float* dA, float* part, float* dD, void* dB, void* dC, long long T, int NC, int Di, int n_state,
+                 void* ddl, void* dz, long long dzs, float* dA, float* part, float* dD, void* dB, void* dC, long long T, int NC, int Di, int n_state,
                  cudaStream_t stream) {
   if (NC <= 0) return 0;
   if (n_state != N) return -2;
@@ -678,7 +758,7 @@ int fb_sscan_bwd(const void* u, long long us, const void* dl, long long ds, int 
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BwdSmem));
     if (e != cudaSuccess) return -3;
     kernel<<<dim3(NC, nblk), BT, sizeof(BwdSmem), stream>>>(a, go, (const __nv_bfloat16*)y, st, adj, (__nv_bfloat16*)du, ddl,
-                                                                 (__nv_bfloat16*)dz, dA, part, dD, T);
+                                                                 (__nv_bfloat16*)dz, (int)dzs, dA, part, dD, T);
     return fb::launch_ok("sscan_bwd_kernel");
   };
   if (z) rc = raw ? go_bwd(sscan_bwd_kernel<true, true>) : go_bwd(sscan_bwd_kernel<false, true>);
