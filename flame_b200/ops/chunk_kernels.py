@@ -304,7 +304,7 @@ class ScalarPrep(torch.autograd.Function):
 _vp, _i, _ll = c_void_p, c_int, c_longlong
 _SSCAN_IN = [_vp, _ll, _vp, _ll, _i, _vp, _ll, _vp, _ll, _vp, _ll, _i, _vp, _vp, _vp, _vp, _vp, _i]
 _lib.register("fb_sscan_fwd", _SSCAN_IN + [_vp] * 4 + [_i] * 4 + [_vp])
-_lib.register("fb_sscan_bwd", _SSCAN_IN + [_vp] * 13 + [_ll] + [_i] * 3 + [_vp])
+_lib.register("fb_sscan_bwd", _SSCAN_IN + [_vp] * 8 + [_ll] + [_vp] * 5 + [_ll] + [_i] * 3 + [_vp])
 _lib.register("fb_sscan_channel_blocks", [c_int])
 _lib.register("fb_sscan_padded", [c_int])
 
@@ -374,7 +374,8 @@ class SelectiveScan(torch.autograd.Function):
         dD = torch.empty(lay.NC, DiP, dtype=torch.float32, device=dev)
         part = torch.empty(nblk, T, 32, dtype=torch.float32, device=dev)       # per-channel-block partials of dB | dC
         rc = L.fb_sscan_bwd(*SelectiveScan._operands(u, delta, A, B, C, D, z, lay, raw), st.data_ptr(), sdl.data_ptr(), _lib.ptr(y),
-                            dout.data_ptr(), adj.data_ptr(), du.data_ptr(), ddl.data_ptr(), _lib.ptr(dz), dA.data_ptr(),
+                            dout.data_ptr(), adj.data_ptr(), du.data_ptr(), ddl.data_ptr(), _lib.ptr(dz),
+                            0 if dz is None else dz.stride(0), dA.data_ptr(),
                             part.data_ptr(), dD.data_ptr(), dB.data_ptr(), dC.data_ptr(), T, lay.NC, Di, A.shape[1], _lib.stream_ptr())
         _lib.check(rc, "fb_sscan_bwd")
         _lib.count_launch(4)
