@@ -31,12 +31,13 @@ constexpr int MAX_STAGES = 8;
 // The chunk algorithms' problems mostly have 64 rows, which live in two lane quarters only; with one warp per quarter
 // two warps would drain every accumulator and the epilogue, not memory, would set the pace.
 constexpr int BGEMM_THREADS = 320;
-// A work unit of the chunk algorithms is one to four K blocks, so a CTA spends its time in hand-offs and in the epilogue's
-// round trips to memory (one unit took about 1,500 clocks, whatever its size): tiles of at most 128 columns leave room for
-// two CTAs per SM (half of tensor memory and of shared memory each), whose epilogues overlap.
+// A work unit of the chunk algorithms is one to four K blocks, so a CTA spends its time in hand-offs between its warps: tiles of
+// at most 128 columns leave room for two CTAs per SM (half of tensor memory and of shared memory each), whose chains overlap.
 constexpr int MAX_BN = 128;
 constexpr int TMEM_COLS = 256;
-constexpr int RING_BYTES = 96 * 1024;
+// Shared memory of a CTA: the ring, and where results leave by TMA 4 KB for every epilogue warp that has rows.
+constexpr int MAIN_BYTES = 104 * 1024;
+constexpr int STG_BYTES = 4096;
 
 struct BOperandIdx {
   const int* hi_index;  // optional: hi coordinate = hi_index[hi_raw]
@@ -53,6 +54,7 @@ struct BPair {
 
 struct BMaps {
   CUtensorMap a[MAX_PAIRS], b[MAX_PAIRS];
+  CUtensorMap c, add;  // TMA_OUT: boxes of 32 rows x 128 bytes of the result and of the bf16 addend
 };
 
 struct BGemmParams {
@@ -79,12 +81,14 @@ struct BGemmParams {
   float alpha;
   int out_mode;        // 0 bf16 store, 1 fp32 store, 2 fp32 accumulate
   int mask_mode;       // 0 none, 1 keep col <= row, 2 keep col < row
+  int stg_offset;      // TMA_OUT: the epilogue warps' boxes begin here
+  int arrivals;        // epilogue warps that drain an accumulator
   int* status;
 };
 
 struct Smem {
-  static constexpr int BAR_OFFSET = RING_BYTES;
-  static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;
+  static constexpr int BAR_OFFSET = MAIN_BYTES;
+  static constexpr int TOTAL = BAR_OFFSET + 512 + 1024;
 };
 
 struct Unit {
@@ -102,10 +106,29 @@ __device__ __forceinline__ Unit decode(const BGemmParams& p, int unit) {
   u.lo = batch - u.hi_raw * p.n_lo;
   return u;
 }
+// The unit `step` (a decoded distance) further on, without divisions.
+__device__ __forceinline__ void advance(const BGemmParams& p, Unit& u, const Unit& step) {
+  u.tm += step.tm;
+  u.tn += step.tn;
+  u.lo += step.lo;
+  u.hi_raw += step.hi_raw;
+  if (u.tm >= p.tiles_m) u.tm -= p.tiles_m, ++u.tn;
+  if (u.tn >= p.tiles_n) u.tn -= p.tiles_n, ++u.lo;
+  if (u.lo >= p.n_lo) u.lo -= p.n_lo, ++u.hi_raw;
+}
+__device__ __forceinline__ int lo_of(const BOperandIdx& o, int lo) { return o.lo_div == 1 ? lo : lo / o.lo_div; }
 __device__ __forceinline__ int hi_of(const BOperandIdx& o, int hi_raw) {
   return (o.hi_index != nullptr ? o.hi_index[hi_raw] : hi_raw) + o.hi_offset;
 }
 
+// TMA_OUT: each epilogue warp puts 32 rows x 128 bytes of the result into shared memory and one thread hands them to the TMA
+// unit (the accumulating mode adds in L2, a bf16 addend comes in the same way while the products are formed).  Results with a
+// state step, a hi index or a layout that has no tensor map are stored row by row: a warp's 16-byte stores to 32 different
+// rows then take the load/store unit 64 cycles each, and that unit, not memory, set the pace (a unit of 128 x 128 took 13,000
+// clocks in two CTAs, 8,200 of them in these stores).  The ten to twenty-five launches of a layer's forward and backward,
+// row by row and by TMA: DeltaNet 3.77 -> 1.90 ms (65,536 tokens, 8 heads of 128), GLA 1.79 -> 0.84, GSA 1.49 -> 0.66, Mamba2
+// 2.38 -> 1.06, Gated DeltaNet 2.14 -> 1.28.
+template <bool TMA_OUT>
 __global__ void __launch_bounds__(BGEMM_THREADS, 2)
 bgemm_bf16_kernel(const __grid_constant__ BMaps maps, const __grid_constant__ BGemmParams p) {
   using L = Smem;
@@ -115,7 +138,8 @@ bgemm_bf16_kernel(const __grid_constant__ BMaps maps, const __grid_constant__ BG
   uint64_t* empty_bar = full_bar + MAX_STAGES;
   uint64_t* tfull_bar = empty_bar + MAX_STAGES;
   uint64_t* tempty_bar = tfull_bar + 4;
-  uint32_t* tmem_slot = (uint32_t*)(tempty_bar + 4);
+  uint64_t* stg_bar = tempty_bar + 4;
+  uint32_t* tmem_slot = (uint32_t*)(stg_bar + 8);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -132,14 +156,16 @@ bgemm_bf16_kernel(const __grid_constant__ BMaps maps, const __grid_constant__ BG
     }
     for (int a = 0; a < n_acc; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], (blockDim.x >> 5) - 2);
+      mbar_init(&tempty_bar[a], p.arrivals);
     }
+    for (int w = 0; w < 8; ++w) mbar_init(&stg_bar[w], 1);
     *abort_flag = 0;
     mbar_fence_init();
     for (int i = 0; i < p.n_pairs; ++i) {
       tma_prefetch_desc(&maps.a[i]);
       tma_prefetch_desc(&maps.b[i]);
     }
+    if (TMA_OUT) tma_prefetch_desc(&maps.c);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, TMEM_COLS);
@@ -155,13 +181,14 @@ bgemm_bf16_kernel(const __grid_constant__ BMaps maps, const __grid_constant__ BG
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
-        const Unit u = decode(p, unit);
+      Unit u = decode(p, blockIdx.x);
+      const Unit step = decode(p, gridDim.x);
+      for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x, advance(p, u, step)) {
         for (int i = 0; i < p.n_pairs && ok; ++i) {
           const BPair& pr = p.pair[i];
           const int a_hi = hi_of(pr.a, u.hi_raw), b_hi = hi_of(pr.b, u.hi_raw);
           for (int sk = 0, kb = 0, lo = u.lo * p.sum_lo; sk < p.sum_lo * pr.num_kb; ++sk) {
-            const int a_lo = lo / pr.a.lo_div, b_lo = lo / pr.b.lo_div;
+            const int a_lo = lo_of(pr.a, lo), b_lo = lo_of(pr.b, lo);
             if (!mbar_wait(&empty_bar[stage], phase ^ 1, p.status, abort_flag, ERR_WAIT_EMPTY)) { ok = false; break; }
             uint8_t* sA = smem + stage * stage_bytes;
             uint8_t* sB = sA + a_bytes;
@@ -220,6 +247,124 @@ bgemm_bf16_kernel(const __grid_constant__ BMaps maps, const __grid_constant__ BG
         if (++acc == n_acc) { acc = 0; acc_phase ^= 1; }
       }
     }
+  } else if constexpr (TMA_OUT) {
+    const int quarter = warp & 3;
+    const int half = (warp - 2) >> 2;
+    // Tiles of 128 columns: the two warps of a lane quarter take half of the columns each.  Tiles of 64: every second unit, so
+    // that a box of the result is 128 bytes wide there too.  Either way a warp drains two groups of 32 columns.
+    const bool alt = BN == 64;
+    const int c_begin = alt ? 0 : half * 64;
+    const bool b16 = p.out_mode == 0, add = p.add16 != nullptr;
+    int acc = 0, n = 0;
+    uint32_t acc_phase = 0, stg_phase = 0;
+    bool ok = quarter * 32 < p.a_rows;  // warps of rows that the tile does not have
+    const int slot = half * (p.a_rows >> 5) + quarter;
+    uint8_t* stg = smem + p.stg_offset + (ok ? slot : 0) * STG_BYTES;
+    uint64_t* my_bar = &stg_bar[warp - 2];
+    auto at = [&](int chunk) { return stg + lane * 128 + ((chunk ^ (lane & 7)) << 4); };  // the 128-byte swizzle of the maps
+    Unit u = decode(p, blockIdx.x);
+    const Unit step = decode(p, gridDim.x);
+    for (int unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x, advance(p, u, step), ++n) {
+      if (!alt || (n & 1) == half) {
+        const int row0 = u.tm * BM + quarter * 32, row = row0 + lane, colw = u.tn * BN + c_begin;
+        const bool any = row0 < p.M && colw < p.N;
+        if (add && any && lane == 0) {
+          tma_store_wait_read<0>();
+          mbar_expect_tx(my_bar, STG_BYTES);
+          tma_load_4d(stg, &maps.add, my_bar, colw, row0, u.lo, u.hi_raw + p.add16i.hi_offset);
+        }
+        float scale = p.alpha, dec_row = 0.f;
+        const float* dec = nullptr;
+        if (p.rowscale != nullptr && row < p.M)
+          scale *= p.rowscale[(long long)u.hi_raw * p.r_hi + (long long)u.lo * p.r_lo + (long long)row * p.r_r];
+        if (p.decay != nullptr) {
+          dec = p.decay + (long long)u.hi_raw * p.d_hi + (long long)u.lo * p.d_lo;
+          if (row < p.M) dec_row = dec[(long long)row * p.d_r];
+        }
+        if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16) + c_begin;
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+          const int col = colw + 32 * k;
+          const bool live = any && col < p.N;  // warp-uniform
+          uint32_t r[32];
+          float dec_col = 0.f;
+          if (live) {
+            tmem_ld_32x32(t_row + 32 * k, r);
+            if (dec != nullptr && col + lane < p.N) dec_col = dec[(long long)(col + lane) * p.d_r];
+            if (!b16 || k == 0) {  // the box is free: its last store has been read, or the addend has come
+              if (add) {
+                if (!mbar_wait_warp(my_bar, stg_phase, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) ok = false;
+                stg_phase ^= 1;
+              } else {
+                if (lane == 0) tma_store_wait_read<0>();
+                __syncwarp();
+              }
+            }
+            tmem_ld_wait();
+          }
+          if (k == 1) {  // everything is in registers
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&tempty_bar[acc]);
+          }
+          if (!live) continue;
+#pragma unroll
+          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * scale);
+          if (dec != nullptr) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) {
+              const float dj = __shfl_sync(0xffffffffu, dec_col, j);
+              // masked entries may have a positive exponent: they are dropped, never multiplied
+              const bool keep = p.mask_mode == 0 || (p.mask_mode == 1 ? col + j <= row : col + j < row);
+              r[j] = keep ? __float_as_uint(__uint_as_float(r[j]) * __expf(dec_row - dj)) : 0u;
+            }
+          } else if (p.mask_mode != 0) {
+            const int first_out = row - col + (p.mask_mode == 1 ? 1 : 0);  // the first column that is dropped
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (j >= first_out) r[j] = 0u;
+          }
+          if (b16) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              uint4* dst = reinterpret_cast<uint4*>(at(4 * k + j));
+              if (add) {  // v_new = u - w S, o = q S + A v
+                const uint4 a4 = *dst;
+                const uint32_t w4[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                  r[8 * j + 2 * t] = __float_as_uint(__uint_as_float(r[8 * j + 2 * t]) + __uint_as_float(w4[t] << 16));
+                  r[8 * j + 2 * t + 1] = __float_as_uint(__uint_as_float(r[8 * j + 2 * t + 1]) + __uint_as_float(w4[t] & 0xffff0000u));
+                }
+              }
+              uint4 q;
+              q.x = pack_bf16(__uint_as_float(r[8 * j]), __uint_as_float(r[8 * j + 1]));
+              q.y = pack_bf16(__uint_as_float(r[8 * j + 2]), __uint_as_float(r[8 * j + 3]));
+              q.z = pack_bf16(__uint_as_float(r[8 * j + 4]), __uint_as_float(r[8 * j + 5]));
+              q.w = pack_bf16(__uint_as_float(r[8 * j + 6]), __uint_as_float(r[8 * j + 7]));
+              *dst = q;
+            }
+            if (k == 0 && col + 32 < p.N) continue;  // the box's other half follows
+          } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<uint4*>(at(j)) = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            const int x = b16 ? colw : col, hi = u.hi_raw + p.c.hi_offset;
+            if (p.out_mode == 2) tma_reduce_add_4d(&maps.c, stg, x, row0, u.lo, hi);
+            else tma_store_4d(&maps.c, stg, x, row0, u.lo, hi);
+            tma_store_commit();
+          }
+        }
+      }
+      if (++acc == n_acc) { acc = 0; acc_phase ^= 1; }
+    }
+    if (lane == 0) tma_store_wait_all<0>();
   } else {
     const int quarter = warp & 3;
     // two warps per lane quarter, each takes half of the tile's columns (tiles are 64 or 128 wide)
@@ -400,10 +545,11 @@ bgemm_bf16_kernel(const __grid_constant__ BMaps maps, const __grid_constant__ BG
   }
 }
 
+template <bool TMA_OUT>
 int launch_b(const BMaps& maps, const BGemmParams& p, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(bgemm_bf16_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
+    cudaError_t e = cudaFuncSetAttribute(bgemm_bf16_kernel<TMA_OUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
@@ -416,8 +562,13 @@ int launch_b(const BMaps& maps, const BGemmParams& p, cudaStream_t stream) {
   }
   const long long units = (long long)p.n_batch * p.tiles_m * p.tiles_n;
   const int grid = (int)(units < 2 * sms ? units : 2 * sms);
-  bgemm_bf16_kernel<<<grid, BGEMM_THREADS, Smem::TOTAL, stream>>>(maps, p);
+  bgemm_bf16_kernel<TMA_OUT><<<grid, BGEMM_THREADS, Smem::TOTAL, stream>>>(maps, p);
   return fb::launch_ok("bgemm_bf16_kernel");
+}
+
+// A [hi, lo, rows, cols] layout that a tensor map can describe (a stride counts only where there is something to step to).
+bool mappable(const void* ptr, long long ld, long long lo, long long hi, int n_lo, int n_hi, int rows) {
+  return !((uintptr_t)ptr & 15) && (ld > 0 || rows == 1) && (lo > 0 || n_lo == 1) && (hi > 0 || n_hi == 1);
 }
 
 }  // namespace
@@ -484,8 +635,6 @@ int fb_bgemm_bf16(const FbBOperand* ops, int n_pairs, const FbBEpilogue* e, int 
   p.M = M; p.N = N; p.n_pairs = n_pairs; p.sum_lo = sum_lo;
   p.bn = N <= 64 ? 64 : MAX_BN;
   p.a_rows = M <= 64 ? 64 : BM;
-  p.stages = RING_BYTES / ((p.a_rows + p.bn) * BK * 2);
-  if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
   p.tiles_m = (M + BM - 1) / BM;
   p.tiles_n = (N + p.bn - 1) / p.bn;
   p.n_lo = n_lo_batch;
@@ -505,7 +654,32 @@ int fb_bgemm_bf16(const FbBOperand* ops, int n_pairs, const FbBEpilogue* e, int 
   p.status = fb::status_ptr();
   if ((p.C16 != nullptr || p.Cin != nullptr) && p.out_mode == 0) return -3;
   if ((p.C16 != nullptr || p.add16 != nullptr) && ((p.ld16 & 7) || (p.stride_lo16 & 7) || (p.stride_hi16 & 7))) return -2;
+  // results leave by TMA unless there is a state step or an index in the way (see the kernel)
+  const bool out16 = p.out_mode == 0;
+  const int hi_c = p.c.hi_offset + n_hi_batch, hi_add = p.add16i.hi_offset + n_hi_batch;
+  const bool tma_out = p.Cin == nullptr && p.C16 == nullptr && p.c.hi_index == nullptr && p.c.lo_div == 1 && p.c.hi_offset >= 0 &&
+                       mappable(p.C, p.ldc, p.c_stride_lo, p.c_stride_hi, n_lo_batch, hi_c, M) &&
+                       (p.add16 == nullptr ||
+                        (out16 && p.add16i.hi_index == nullptr && p.add16i.hi_offset >= 0 &&
+                         mappable(p.add16, p.ld16, p.stride_lo16, p.stride_hi16, n_lo_batch, hi_add, M)));
+  const int stage_bytes = (p.a_rows + p.bn) * BK * 2;
+  const int stg_warps = !tma_out ? 0 : 2 * (p.a_rows / 32);
+  p.stages = (MAIN_BYTES - stg_warps * STG_BYTES) / stage_bytes;
+  if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
+  p.stg_offset = p.stages * stage_bytes;
+  p.arrivals = !tma_out ? 8 : (p.a_rows / 32) * (p.bn == 64 ? 1 : 2);
   BMaps maps;
+  if (tma_out) {
+    const long long some = 8;  // a stride that is never used
+    int rc = fb::make_tmap_4d(&maps.c, p.C, out16 ? 2 : 4, hi_c, n_lo_batch, M, N, hi_c > 1 ? p.c_stride_hi : some,
+                              n_lo_batch > 1 ? p.c_stride_lo : some, M > 1 ? p.ldc : some, 32, out16 ? 64 : 32, true);
+    if (rc) return rc;
+    if (p.add16 != nullptr) {
+      rc = fb::make_tmap_4d(&maps.add, p.add16, 2, hi_add, n_lo_batch, M, N, hi_add > 1 ? p.stride_hi16 : some,
+                            n_lo_batch > 1 ? p.stride_lo16 : some, M > 1 ? p.ld16 : some, 32, 64, true);
+      if (rc) return rc;
+    }
+  }
   for (int i = 0; i < n_pairs; ++i) {
     const FbBOperand &a = ops[2 * i], &b = ops[2 * i + 1];
     BPair& pr = p.pair[i];
@@ -521,7 +695,7 @@ int fb_bgemm_bf16(const FbBOperand* ops, int n_pairs, const FbBEpilogue* e, int 
               : fb::make_tmap_4d(&maps.b[i], b.ptr, 2, b.n_hi, b.n_lo, N, b.k, b.stride_hi, b.stride_lo, b.ld, p.bn, BK, true);
     if (rc) return rc;
   }
-  return launch_b(maps, p, stream);
+  return tma_out ? launch_b<true>(maps, p, stream) : launch_b<false>(maps, p, stream);
 }
 
 }  // extern "C"

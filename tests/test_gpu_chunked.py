@@ -369,3 +369,49 @@ def test_mamba2_ssd_grouped_heads_match_recurrence():
     out = _run(lambda c: mamba2_ssd(c(x), F.softplus(dtraw.float()) * 0.3, A, c(B) * 0.2, c(C) * 0.2, D, meta), ins, False)
     for a, b in zip(out, ref):
         assert rel_err(a, b) < 3e-2
+
+
+@pytest.mark.parametrize("M", [16, 40, 64, 72, 128, 200])
+@pytest.mark.parametrize("N", [8, 24, 64, 72, 128, 136])
+def test_bgemm_result_boxes(M, N):
+    """Results that leave by TMA, at the edges of the boxes (32 rows, 64 or 32 columns), in padded and token-major storage whose
+    neighbours stay untouched; against fp64.  Sums of K = 72 products of bf16 values in fp32: bf16 rounding of the result (2^-9
+    relative) and of the addend's sum, plus 72 fp32 roundings of the absolute sum."""
+    from flame_b200.ops.bgemm import MASK_STRICT, MASK_TRIL, bgemm
+    torch.manual_seed(M * 1000 + N)
+    dev = torch.device("cuda", 0)
+    hi, lo, K = 5, 3, 72
+    a, b = torch.randn(hi, lo, M, K, device=dev).bfloat16(), torch.randn(hi, lo, N, K, device=dev).bfloat16()
+    scale = torch.rand(hi, lo, M, device=dev) + 0.5
+    full = torch.einsum("hlmk,hlnk->hlmn", a.double(), b.double())
+    size = torch.einsum("hlmk,hlnk->hlmn", a.double().abs(), b.double().abs())
+    pad = (N + 7) // 8 * 8 + 8
+
+    def check(got, want, rounding):
+        assert ((got.double() - want).abs() <= rounding * want.abs() + 2.0 ** -17 * size + 1e-30).all()
+
+    for token_major in (False, True):
+        for dtype in (torch.bfloat16, torch.float32):
+            shape = (hi + 1, M + 1, lo, pad) if token_major else (hi + 1, lo, M + 1, pad)
+            store = torch.full(shape, 7.0, dtype=dtype, device=dev)
+            view = store.permute(0, 2, 1, 3) if token_major else store
+            out = view[1:, :, :M, :N]
+            eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -20
+            bgemm(a, b, out=out, alpha=0.5, rowscale=scale)
+            want = 0.5 * full * scale.double()[..., None]
+            check(out, want, eps)
+            if dtype == torch.float32:
+                bgemm(a, b, out=out, accumulate=True)
+                check(out, want + full, eps)
+            else:
+                add = torch.randn(hi, lo, M, pad, device=dev).bfloat16()[..., :N]
+                bgemm(a, b, out=out, add16=add)
+                check(out, full + add.double(), eps)
+                bgemm(a, b, out=out, add16=out)   # in place
+            if M == N:
+                for mode, want in ((MASK_TRIL, full.tril()), (MASK_STRICT, full.tril(-1))):
+                    bgemm(a, b, out=out, mask=mode)
+                    check(out, want, eps)
+            mask = torch.ones(view.shape, dtype=torch.bool, device=dev)
+            mask[1:, :, :M, :N] = False
+            assert (view[mask] == 7.0).all()
