@@ -244,7 +244,7 @@ template <int LANES>
 __global__ void mamba2_post_bwd_kernel(const __nv_bfloat16* __restrict__ y, const __nv_bfloat16* __restrict__ x, long long ldx,
                                        const __nv_bfloat16* __restrict__ z, long long ldz, const float* __restrict__ D,
                                        const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ dy,
-                                       __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dz,
+                                       __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dz, long long lddz,
                                        float* __restrict__ dD_part, long long T, int H) {
   const int vecs = H * LANES;
   const long long gid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -272,7 +272,7 @@ __global__ void mamba2_post_bwd_kernel(const __nv_bfloat16* __restrict__ y, cons
     }
     *reinterpret_cast<uint4*>(dy + off) = pack8(oy);
     *reinterpret_cast<uint4*>(dx + off) = pack8(ox);
-    *reinterpret_cast<uint4*>(dz + off) = pack8(oz);
+    *reinterpret_cast<uint4*>(dz + t * lddz + v * 8) = pack8(oz);
   }
 #pragma unroll
   for (int o = LANES / 2; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
@@ -327,16 +327,16 @@ int fb_mamba2_post_fwd(const void* y, const void* x, long long ldx, const void* 
   return fb::launch_ok("mamba2_post_fwd_kernel");
 }
 
-// dout: bf16 [T, H * P]; dy, dx, dz: bf16 [T, H * P]; dD_part: fp32 [T, H] (summed over T by the caller)
+// dout: bf16 [T, H * P]; dy, dx: bf16 [T, H * P]; dz the same with row stride lddz; dD_part: fp32 [T, H] (summed over T by the caller)
 int fb_mamba2_post_bwd(const void* y, const void* x, long long ldx, const void* z, long long ldz, const float* D, const void* dout,
-                       void* dy, void* dx, void* dz, float* dD_part, long long T, int H, int P, cudaStream_t stream) {
+                       void* dy, void* dx, void* dz, long long lddz, float* dD_part, long long T, int H, int P, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if ((P != 64 && P != 128 && P != 256) || (ldx % 8) || (ldz % 8) || ((uintptr_t)x & 15) || ((uintptr_t)z & 15)) return -2;
+  if ((P != 64 && P != 128 && P != 256) || (ldx % 8) || (ldz % 8) || (lddz % 8) || ((uintptr_t)dz & 15) || ((uintptr_t)x & 15) || ((uintptr_t)z & 15)) return -2;
   const long long threads = T * H * (P / 8);
   const unsigned blocks = (unsigned)((threads + 255) / 256);
 #define FB_POST_BWD(L) mamba2_post_bwd_kernel<L><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)y, (const __nv_bfloat16*)x, ldx, \
       (const __nv_bfloat16*)z, ldz, D, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dy, (__nv_bfloat16*)dx, (__nv_bfloat16*)dz, \
-      dD_part, T, H)
+      lddz, dD_part, T, H)
   if (P == 64) FB_POST_BWD(8); else if (P == 128) FB_POST_BWD(16); else FB_POST_BWD(32);
 #undef FB_POST_BWD
   return fb::launch_ok("mamba2_post_bwd_kernel");

@@ -15,9 +15,10 @@ import torch.nn.functional as F
 from ..ops import linear_attn as la
 from ..ops.attn_block import qkv_attention
 from ..ops.rope import rope_tables
+from ..ops.slots import reshaped, split_columns
 from ..ops.varlen import VarlenMeta
 from .config import ModelConfig, mamba_dt_rank
-from .modules import Linear, RMSNorm, RMSNormGated, ShortConvolution, fused_projection
+from .modules import Linear, RMSNorm, RMSNormGated, ShortConvolution, fused_projection, side_by_side, split_projections
 
 
 class Attention(nn.Module):
@@ -166,15 +167,18 @@ class GatedLinearAttention(nn.Module):
                 g_out = parts[3]
             gk = self.gk_proj[1](parts[-1].contiguous())
         else:
-            q, k, v = self.q_proj(x), self.k_proj(x), self.v_proj(x)
+            layers = (self.q_proj, self.k_proj, self.v_proj)
+            # (torch's activations are several times slower on column blocks)
+            whole = self.use_short_conv or self.feature_map is None
+            q, k, v = split_projections(x, layers) if whole else (l(x) for l in layers)
             gk = self.gk_proj(x)
         T = q.shape[0]
         if self.use_short_conv:
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
-        q = q.reshape(T, H, self.head_k_dim)
-        k = k.reshape(T, self.num_kv_heads, self.head_k_dim)
+        q = reshaped(q, T, H, self.head_k_dim)
+        k = reshaped(k, T, self.num_kv_heads, self.head_k_dim)
         gk = gk.reshape(T, self.num_kv_heads, self.head_k_dim)
-        v = v.reshape(T, self.num_kv_heads, self.head_v_dim)
+        v = reshaped(v, T, self.num_kv_heads, self.head_v_dim)
         if G > 1:
             k, gk, v = (t.repeat_interleave(G, 1) for t in (k, gk, v))
         gk = F.logsigmoid(gk.float()) / self.gate_logit_normalizer
@@ -238,10 +242,12 @@ class DeltaNet(nn.Module):
     def forward(self, x: torch.Tensor, meta: VarlenMeta) -> torch.Tensor:
         from ..ops.delta_rule import gated_delta_rule
         T, H = x.shape[0], self.num_heads
-        q, k, v = self.q_proj(x), self.k_proj(x), self.v_proj(x)
+        layers = (self.q_proj, self.k_proj, self.v_proj)
         if self.use_short_conv:
+            q, k, v = split_projections(x, layers)
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
         else:
+            q, k, v = (l(x) for l in layers)
             if self.qk_activation == "silu":
                 q, k = F.silu(q), F.silu(k)
             v = F.silu(v)
@@ -314,10 +320,12 @@ class GatedDeltaNet(nn.Module):
         from ..ops.delta_rule import gated_delta_rule
         T = x.shape[0]
         H, HV = self.num_heads, self.num_v_heads
-        q, k, v = self.q_proj(x), self.k_proj(x), self.v_proj(x)
+        layers = (self.q_proj, self.k_proj, self.v_proj)
         if self.use_short_conv:
+            q, k, v = split_projections(x, layers)
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
         else:
+            q, k, v = (l(x) for l in layers)
             q, k, v = F.silu(q), F.silu(k), F.silu(v)
         q, k = q.reshape(T, H, self.head_k_dim), k.reshape(T, H, self.head_k_dim)
         v = v.reshape(T, HV, self.head_v_dim)
@@ -367,16 +375,20 @@ class GatedSlotAttention(nn.Module):
     def forward(self, x: torch.Tensor, meta: VarlenMeta) -> torch.Tensor:
         from ..ops.gla import gsa
         T, H, G = x.shape[0], self.num_heads, self.num_kv_groups
-        q, k, v = self.q_proj(x), self.k_proj(x), self.v_proj(x)
+        layers, sizes = (self.q_proj, self.k_proj, self.v_proj), (self.key_dim, self.key_dim_per_group, self.value_dim_per_group)
         if self.use_short_conv:
+            q, k, v = split_projections(x, layers)
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
-        f = self.f_proj(x)
-        q = q.reshape(T, H, self.head_k_dim)
-        k = k.reshape(T, self.num_kv_heads, self.head_k_dim)
-        v = v.reshape(T, self.num_kv_heads, self.head_v_dim)
-        f = f.reshape(T, self.num_kv_heads, self.num_slots)
-        q, k = _feature_map(self.feature_map, q), _feature_map(self.feature_map, k)
-        v = F.silu(v)
+            q, k, v = _feature_map(self.feature_map, q), _feature_map(self.feature_map, k), F.silu(v)
+        elif self.feature_map in ("swish", "silu") and side_by_side(layers, x):
+            # one activation over the three blocks as they lie: torch's kernels are several times slower on column blocks
+            q, k, v = split_columns(F.silu(fused_projection(x, layers)), sizes)
+        else:
+            q, k, v = _feature_map(self.feature_map, self.q_proj(x)), _feature_map(self.feature_map, self.k_proj(x)), F.silu(self.v_proj(x))
+        q = reshaped(q, T, H, self.head_k_dim)
+        k = reshaped(k, T, self.num_kv_heads, self.head_k_dim)
+        v = reshaped(v, T, self.num_kv_heads, self.head_v_dim)
+        f = self.f_proj(x).reshape(T, self.num_kv_heads, self.num_slots)
         f = F.logsigmoid(f.float()) / self.gate_logit_normalizer
         s = 1 - f.exp()
         if G > 1:

@@ -11,6 +11,7 @@ import torch.nn as nn
 from ..ops import activations, linear as linear_ops, norm as norm_ops
 from ..ops.embedding import embedding
 from ..ops.conv import short_conv
+from ..ops.slots import split_columns
 from ..ops.varlen import VarlenMeta
 
 
@@ -31,6 +32,26 @@ class Linear(nn.Module):
 def fused_projection(x: torch.Tensor, layers: Sequence[Linear]) -> torch.Tensor:
     """One GEMM for several bias-free projections of the same input; returns their outputs side by side."""
     return linear_ops.linear_fused(x, [l.weight for l in layers])
+
+
+def side_by_side(layers: Sequence[Linear], x: torch.Tensor) -> bool:
+    """Whether one product may stand for these layers: plain ones (no bias, no hook, no subclass with a forward of its own),
+    trained or frozen together, their weights next to one another in memory."""
+    for l in layers:
+        if type(l) is not Linear or l.bias is not None or l.weight.requires_grad != layers[0].weight.requires_grad:
+            return False
+        if l._forward_hooks or l._forward_pre_hooks or l._backward_hooks or l._backward_pre_hooks:
+            return False
+    return linear_ops.side_by_side(x, [l.weight for l in layers])
+
+
+def split_projections(x: torch.Tensor, layers: Sequence[Linear]) -> tuple:
+    """The outputs of several projections of the same input.  Where their weights lie side by side (as the engine lays a block
+    out) one GEMM makes them all as column blocks of one matrix, and one GEMM each makes the weights' and the input's
+    gradient: the input is read once and its gradient needs no additions."""
+    if side_by_side(layers, x):
+        return split_columns(fused_projection(x, layers), [l.weight.shape[0] for l in layers])
+    return tuple(l(x) for l in layers)
 
 
 class Embedding(nn.Module):

@@ -5,7 +5,7 @@ from ctypes import c_float, c_int, c_longlong, c_void_p
 
 import torch
 
-from . import _lib
+from . import _lib, slots
 
 _lib.register("fb_delta_inverse", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 6)
 _lib.register("fb_delta_scale", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 3)
@@ -323,6 +323,7 @@ class SelectiveScan(torch.autograd.Function):
     @staticmethod
     def forward(ctx, u, delta, A, B, C, D, z, lay, raw):
         u, delta, B, C = _rows(u), _rows(delta), _rows(B), _rows(C)
+        ctx.z_slot = None if z is None else slots.of(z)
         z = None if z is None else _rows(z)
         A, D = A.contiguous(), D.contiguous()
         A = A if A.data_ptr() % 16 == 0 else A.clone()
@@ -367,7 +368,9 @@ class SelectiveScan(torch.autograd.Function):
                 t[T:].zero_()
             return t
         du, ddl, dB, dC = grad(u), grad(delta), grad(B), grad(C)
-        dz = None if z is None else grad(z)
+        dz = None
+        if z is not None:
+            dz = ctx.z_slot.take(T, Di, z.dtype, dev) if ctx.z_slot is not None and z.shape[0] == T else grad(z)
         nblk = int(L.fb_sscan_channel_blocks(Di))
         adj = torch.empty(lay.NC, 16, DiP, dtype=torch.float32, device=dev)
         dA = torch.empty(lay.NC, 16, DiP, dtype=torch.float32, device=dev)     # per-chunk partials, summed below

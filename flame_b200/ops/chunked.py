@@ -22,18 +22,19 @@ fla/ops/common/chunk_o.py, fla/layers/mamba2.py).
 """
 from __future__ import annotations
 
+import math
 from typing import List, Optional
 
 import torch
 
 from ctypes import c_int, c_longlong, c_void_p
 
-from . import _lib
+from . import _lib, slots
 from .bgemm import MASK_STRICT, MASK_TRIL, _mask, bgemm, bmm
 from .varlen import VarlenMeta
 
 CHUNK = 64
-_lib.register("fb_gather_rows", [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_void_p])
+_lib.register("fb_gather_rows", [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_longlong, c_longlong, c_void_p])
 _lib.register("fb_delta_scan", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_int, c_void_p])
 
@@ -138,9 +139,9 @@ class ChunkLayout:
 
     def pack(self, x: torch.Tensor) -> torch.Tensor:
         """[T, ...] -> [NC, chunk, ...] (zero rows where a document is padded)."""
-        if self.aligned:
+        if self.aligned and (x.is_contiguous() or not _rows_strided(x)):
             return x.reshape(self.NC, self.chunk, *x.shape[1:])
-        return _Pack.apply(x, self).reshape(self.NC, self.chunk, *x.shape[1:])
+        return _Pack.apply(x, self, slots.of(x)).reshape(self.NC, self.chunk, *x.shape[1:])
 
     def unpack(self, y: torch.Tensor) -> torch.Tensor:
         """[NC, chunk, ...] -> [T, ...]."""
@@ -148,16 +149,27 @@ class ChunkLayout:
         return y if self.aligned else _Unpack.apply(y, self)
 
 
-def _gather_rows(x: torch.Tensor, idx: torch.Tensor, n_out: int) -> torch.Tensor:
+def _rows_strided(x: torch.Tensor) -> bool:
+    """Rows that are contiguous and whole 16-byte vectors, at any distance that is one too: what the gather kernel reads."""
+    n = x.numel() // max(x.shape[0], 1)
+    inner = list(x.stride()[1:]) == [math.prod(x.shape[i + 1:]) for i in range(1, x.dim())]
+    return (inner and n * x.element_size() % 16 == 0 and x.stride(0) * x.element_size() % 16 == 0 and x.data_ptr() % 16 == 0
+            and x.stride(0) >= n)
+
+
+def _gather_rows(x: torch.Tensor, idx: torch.Tensor, n_out: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[r] = x[idx[r]]`` (zero where ``idx[r] < 0``) in one pass of the row-gather kernel."""
-    x = x if x.is_contiguous() else x.contiguous()
+    x = x if _rows_strided(x) else x.contiguous()
     row_bytes = (x.numel() // max(x.shape[0], 1)) * x.element_size()
-    if not (_lib.available() and x.is_cuda and row_bytes % 16 == 0 and x.shape[0] > 0):
+    if not (_lib.available() and x.is_cuda and row_bytes % 16 == 0 and x.shape[0] > 0 and x.data_ptr() % 16 == 0):
         safe = idx.clamp_min(0).long()
-        out = x.index_select(0, safe)
-        return out * (idx >= 0).to(x.dtype).view(-1, *([1] * (x.dim() - 1)))
-    out = torch.empty(n_out, *x.shape[1:], dtype=x.dtype, device=x.device)
-    rc = _lib.lib().fb_gather_rows(x.data_ptr(), out.data_ptr(), idx.data_ptr(), n_out, row_bytes, _lib.stream_ptr())
+        r = x.index_select(0, safe)
+        r = r * (idx >= 0).to(x.dtype).view(-1, *([1] * (x.dim() - 1)))
+        return r if out is None else out.copy_(r)
+    if out is None:
+        out = torch.empty(n_out, *x.shape[1:], dtype=x.dtype, device=x.device)
+    rc = _lib.lib().fb_gather_rows(x.data_ptr(), out.data_ptr(), idx.data_ptr(), n_out, row_bytes, x.stride(0) * x.element_size(),
+                                   out.stride(0) * out.element_size(), _lib.stream_ptr())
     _lib.check(rc, "fb_gather_rows")
     _lib.count_launch()
     return out
@@ -165,16 +177,23 @@ def _gather_rows(x: torch.Tensor, idx: torch.Tensor, n_out: int) -> torch.Tensor
 
 class _Pack(torch.autograd.Function):
     """Packed rows into the padded layout (zero rows where a document is padded): a gather through the inverse row map;
-    the map is injective, so the backward is a plain gather too."""
+    the map is injective, so the backward is a plain gather too.  ``slot``: where the gradient of ``x`` belongs (``ops/slots.py``)."""
 
     @staticmethod
-    def forward(ctx, x, lay):
-        ctx.lay = lay
+    def forward(ctx, x, lay, slot):
+        ctx.lay, ctx.slot = lay, slot
         return _gather_rows(x, lay.inv_i32, lay.Tp)
 
     @staticmethod
     def backward(ctx, dy):
-        return _gather_rows(dy, ctx.lay.rows_i32, ctx.lay.T), None
+        lay = ctx.lay
+        out = None
+        if ctx.slot is not None and dy.numel():
+            out = ctx.slot.take(lay.T, dy.numel() // dy.shape[0], dy.dtype, dy.device)
+            out = out.view(lay.T, *dy.shape[1:])
+            if not _rows_strided(out):
+                out = None
+        return _gather_rows(dy, lay.rows_i32, lay.T, out), None, None
 
 
 class _Unpack(torch.autograd.Function):

@@ -11,7 +11,7 @@ from typing import Optional
 
 import torch
 
-from . import _lib, linear_attn as la
+from . import _lib, linear_attn as la, slots
 from .varlen import VarlenMeta
 
 vp, i32, i64 = c_void_p, c_int, c_longlong
@@ -32,6 +32,7 @@ class _ShortConvFn(torch.autograd.Function):
     def forward(ctx, x, weight, bias, meta: VarlenMeta, silu: bool):
         T, D = x.shape
         W = weight.shape[-1]
+        ctx.slot = slots.of(x) if W == 4 else None
         x = x if (x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0) else x.contiguous()
         w2 = _aligned(weight.detach().reshape(D, W))
         b2 = _aligned(bias.detach()) if bias is not None else None
@@ -54,7 +55,9 @@ class _ShortConvFn(torch.autograd.Function):
         dy = _aligned(dy)
         w2 = _aligned(weight.detach().reshape(D, W))
         b2 = _aligned(bias.detach()) if bias is not None else None
-        dx = torch.empty(T, D, dtype=x.dtype, device=x.device)
+        dx = None if ctx.slot is None else ctx.slot.take(T, D, x.dtype, x.device)
+        if dx is None or dx.stride(0) % 8 or dx.data_ptr() % 16:
+            dx = torch.empty(T, D, dtype=x.dtype, device=x.device)
         dpre = torch.empty(T, D, dtype=x.dtype, device=x.device) if W != 4 else None
         strips = int(L.fb_short_conv_strips(T))
         part = torch.empty(strips, D, W + 1, dtype=torch.float32, device=x.device)

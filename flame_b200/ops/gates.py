@@ -13,7 +13,8 @@ from typing import Optional, Tuple
 import torch
 import torch.nn.functional as F
 
-from . import _lib
+from . import _lib, slots
+from .slots import split_columns  # noqa: F401 - the layers take it from here
 
 _lib.register("fb_hgrn2_gate_tiles", [c_longlong])
 _lib.register("fb_hgrn2_gate_fwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p])
@@ -87,34 +88,7 @@ _lib.register("fb_mamba2_pre_bwd", [c_void_p, c_longlong, c_void_p, c_longlong, 
 _lib.register("fb_mamba2_post_fwd", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int,
                                      c_int, c_void_p])
 _lib.register("fb_mamba2_post_bwd", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
-                                     c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p])
-
-
-class SplitColumns(torch.autograd.Function):
-    """Column blocks of a ``[T, N]`` matrix as views; the backward writes the blocks' gradients side by side in ONE pass
-    (autograd's own slice backward zero-fills a full-width matrix per block and adds them up)."""
-
-    @staticmethod
-    def forward(ctx, x, *sizes):
-        ctx.sizes, ctx.dtype = sizes, x.dtype
-        outs, c = [], 0
-        for n in sizes:
-            outs.append(x[:, c:c + n])
-            c += n
-        assert c == x.shape[1], (sizes, x.shape)
-        return tuple(outs)
-
-    @staticmethod
-    def backward(ctx, *grads):
-        T = next(g.shape[0] for g in grads if g is not None)
-        dev = next(g.device for g in grads if g is not None)
-        parts = [g.to(ctx.dtype) if g is not None else torch.zeros(T, n, dtype=ctx.dtype, device=dev)
-                 for g, n in zip(grads, ctx.sizes)]
-        return (torch.cat(parts, dim=1), *([None] * len(ctx.sizes)))
-
-
-def split_columns(x: torch.Tensor, sizes) -> Tuple[torch.Tensor, ...]:
-    return SplitColumns.apply(x, *sizes)
+                                     c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_void_p])
 
 
 def _views_ok(*ts: torch.Tensor) -> bool:
@@ -172,7 +146,7 @@ class _Mamba2Post(torch.autograd.Function):
         _lib.check(rc, "fb_mamba2_post_fwd")
         _lib.count_launch()
         ctx.save_for_backward(y, x, z, d32)
-        ctx.dims, ctx.d_dtype = (H, P), D.dtype
+        ctx.dims, ctx.d_dtype, ctx.z_slot = (H, P), D.dtype, slots.of(z)
         return out
 
     @staticmethod
@@ -183,10 +157,12 @@ class _Mamba2Post(torch.autograd.Function):
         dout = dout.contiguous()
         dy = torch.empty(T, H, P, dtype=x.dtype, device=x.device)
         dx = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
-        dz = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
+        dz = ctx.z_slot.take(T, H * P, x.dtype, x.device) if ctx.z_slot is not None else torch.empty(T, H * P, dtype=x.dtype, device=x.device)
+        if not _views_ok(dz):
+            dz = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
         part = torch.empty(T, H, dtype=torch.float32, device=x.device)
         rc = _lib.lib().fb_mamba2_post_bwd(y.data_ptr(), x.data_ptr(), x.stride(0), z.data_ptr(), z.stride(0), d32.data_ptr(),
-                                           dout.data_ptr(), dy.data_ptr(), dx.data_ptr(), dz.data_ptr(), part.data_ptr(), T, H, P,
+                                           dout.data_ptr(), dy.data_ptr(), dx.data_ptr(), dz.data_ptr(), dz.stride(0), part.data_ptr(), T, H, P,
                                            _lib.stream_ptr())
         _lib.check(rc, "fb_mamba2_post_bwd")
         _lib.count_launch()

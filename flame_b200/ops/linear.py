@@ -198,6 +198,15 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return _with_tape(x, bias, [weight], lambda: F.linear(x, weight, bias))
 
 
+def side_by_side(x: torch.Tensor, weights: Sequence[torch.Tensor]) -> bool:
+    """Whether one GEMM may stand for the products of ``x`` with these weights: adjacent in memory (their ``main_grad``s too, or
+    none has one), bf16 on the GPU, no fp8 scaling per tensor, no tape that counts products (selective checkpointing)."""
+    mgs = [getattr(w, "main_grad", None) for w in weights]
+    return (x.dim() == 2 and all(_kernel_ok(x, w) and not getattr(w, "_fp8", False) for w in weights) and sac.current() is None
+            and _adjacent([w.detach() for w in weights])
+            and (all(m is None for m in mgs) or (all(m is not None for m in mgs) and _adjacent(mgs))))
+
+
 def linear_fused(x: torch.Tensor, weights: Sequence[torch.Tensor]) -> torch.Tensor:
     """``x @ cat(weights, 0).T`` as one ``[..., sum(N_i)]`` tensor."""
     if all(_kernel_ok(x, w) for w in weights):

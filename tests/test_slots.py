@@ -1,0 +1,143 @@
+"""Gradients of column blocks written in place (``ops/slots.py``), and layers whose projections run as one GEMM."""
+import copy
+
+import pytest
+import torch
+
+from flame_b200.ops import slots
+from flame_b200.ops.slots import split_columns
+
+
+class _Scale(torch.autograd.Function):
+    """A consumer that writes its gradient where it belongs."""
+
+    @staticmethod
+    def forward(ctx, x, c):
+        ctx.c, ctx.slot = c, slots.of(x)
+        return x * c
+
+    @staticmethod
+    def backward(ctx, dy):
+        if ctx.slot is None:
+            return dy * ctx.c, None
+        return torch.mul(dy, ctx.c, out=ctx.slot.take(*dy.shape, dy.dtype, dy.device)), None
+
+
+SIZES = (3, 1, 4)
+
+
+def _views(x):
+    return split_columns(x, SIZES), x.split(SIZES, dim=1)
+
+
+@pytest.mark.parametrize("rows", [1, 5])
+def test_same_gradient_as_slices(rows):
+    torch.manual_seed(0)
+    x = torch.randn(rows, sum(SIZES), dtype=torch.float64, requires_grad=True)
+    (a, b, c), (a2, b2, c2) = _views(x)
+    y = _Scale.apply(a, 2.0).square().sum() + _Scale.apply(b, 3.0).sum() + _Scale.apply(b, -1.5).square().sum() + (0.5 * c).cos().sum()
+    w = (2.0 * a2).square().sum() + (3.0 * b2).sum() + (1.5 * b2).square().sum() + (0.5 * c2).cos().sum()
+    want, = torch.autograd.grad(w, x)
+    for _ in range(2):  # a second run of the same graph has a buffer of its own
+        got, = torch.autograd.grad(y, x, retain_graph=True)
+        torch.testing.assert_close(got, want, rtol=1e-12, atol=1e-12)
+
+
+def test_unused_block_and_partial_runs():
+    torch.manual_seed(0)
+    x = torch.randn(4, sum(SIZES), dtype=torch.float64, requires_grad=True)
+    a, b, c = split_columns(x, SIZES)
+    y = _Scale.apply(a, 2.0).square().sum() + _Scale.apply(c, 3.0).square().sum()
+    ga, = torch.autograd.grad(y, a, retain_graph=True)       # stops at the view: keeps its buffer
+    kept = ga.clone()
+    gx, = torch.autograd.grad(2.0 * y, x, retain_graph=True)  # another run: must not write into the first one's
+    torch.testing.assert_close(ga, kept)
+    want = torch.cat([8 * x[:, :3], 0 * x[:, 3:4], 18 * x[:, 4:]], 1).detach()
+    torch.testing.assert_close(gx, 2 * want, rtol=1e-12, atol=1e-12)
+
+
+def _adjacent(layers):
+    """The layers' weights as row blocks of one matrix, their gradients too."""
+    ws = [l.weight for l in layers]
+    n, d = sum(w.shape[0] for w in ws), ws[0].shape[1]
+    flat, grad = torch.empty(n, d, dtype=ws[0].dtype, device=ws[0].device), torch.zeros(n, d, device=ws[0].device)
+    c = 0
+    for w in ws:
+        flat[c:c + w.shape[0]].copy_(w.detach())
+        w.data, w.main_grad = flat[c:c + w.shape[0]], grad[c:c + w.shape[0]]
+        c += w.shape[0]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,kw", [
+    ("GatedLinearAttention", dict(num_heads=2)),
+    ("GatedLinearAttention", dict(num_heads=2, use_short_conv=True)),
+    ("DeltaNet", dict(num_heads=2)),
+    ("DeltaNet", dict(num_heads=2, use_short_conv=False)),
+    ("GatedDeltaNet", dict(num_heads=2, head_dim=64)),
+    ("GatedSlotAttention", dict(num_heads=2)),
+    ("GatedSlotAttention", dict(num_heads=2, use_short_conv=True)),
+    ("GatedSlotAttention", dict(num_heads=2, feature_map="relu")),
+])
+@pytest.mark.parametrize("cu", [(0, 128), (0, 1, 66, 131)])
+def test_layer_with_adjacent_projections(name, kw, cu):
+    """One GEMM for adjacent projections or one each: bf16 rounding of the same sums (the input's gradient is rounded once
+    instead of three times), so both lie within a few bf16 steps (2^-8 of the largest entry) of one another."""
+    from flame_b200.models import layers as layers_mod
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    dev = torch.device("cuda", 0)
+    D, T = 256, cu[-1]
+    one = getattr(layers_mod, name)(D, **kw)
+    for p in one.parameters():
+        torch.nn.init.normal_(p, std=0.05) if p.dim() > 1 else torch.nn.init.uniform_(p, 0.5, 1.0)
+    one = one.to(dev)
+    for n, p in one.named_parameters():
+        if n not in ("A_log", "dt_bias", "D"):
+            p.data = p.data.bfloat16()
+    two = copy.deepcopy(one)
+    trio = lambda m: [m.q_proj, m.k_proj, m.v_proj]  # noqa: E731
+    _adjacent(trio(two))
+    for m in trio(one):
+        m.weight.main_grad = torch.zeros_like(m.weight, dtype=torch.float32)
+    meta = VarlenMeta.from_cu_seqlens(torch.tensor(cu, dtype=torch.int32, device=dev))
+    x = torch.randn(T, D, device=dev).bfloat16()
+    dy = torch.randn(T, D, device=dev).bfloat16()
+    res = []
+    for m in (one, two):
+        xi = x.clone().requires_grad_(True)
+        y = m(xi, meta)
+        y.backward(dy)
+        res.append([y.detach(), xi.grad] + [p.weight.main_grad for p in trio(m)] +
+                   [p.grad for n, p in m.named_parameters() if p.grad is not None])
+    assert len(res[0]) == len(res[1])
+    for a, b in zip(*res):
+        a, b = a.double(), b.double()
+        assert (a - b).abs().max() <= 4 * 2.0 ** -8 * a.abs().max().clamp_min(1e-6), name
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("cols", [(8, 0, 8), (136, 8, 64), (72, 4, 8), (64, 0, 64)])
+def test_pack_of_column_blocks(cols):
+    """Rows gathered out of a wider matrix (and gradients into one): copies, so equal bit for bit, also where the block
+    does not start on 16 bytes."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.varlen import VarlenMeta
+    width, c0, n = cols
+    cu = (0, 3, 70, 199)
+    dev = torch.device("cuda", 0)
+    meta = VarlenMeta.from_cu_seqlens(torch.tensor(cu, dtype=torch.int32, device=dev))
+    lay = ChunkLayout(meta)
+    torch.manual_seed(0)
+    base = torch.randn(cu[-1], width, device=dev).bfloat16()
+    sizes = [s for s in (c0, n, width - c0 - n) if s]
+    k = 1 if c0 else 0
+    got = []
+    for split in (lambda t: split_columns(t, sizes), lambda t: [p.contiguous() for p in t.split(sizes, 1)]):
+        x = base.clone().requires_grad_(True)
+        parts = split(x)
+        y = lay.pack(slots.reshaped(parts[k], cu[-1], 1, n))
+        w = torch.arange(y.numel(), device=dev).reshape(y.shape).remainder(7).to(y.dtype)
+        (y * w).sum().backward()
+        got += [(y.detach(), x.grad)]
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
