@@ -38,6 +38,52 @@ __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf
 // log(sigmoid(x)) without cancellation or underflow
 __device__ __forceinline__ float logsigmoidf_(float x) { return fminf(x, 0.f) - log1pf(__expf(-fabsf(x))); }
 
+// g = logsigmoid(x) / n in fp32 from bf16 x, and with SLOTS s = 1 - exp(g) too (GLA's and GSA's forget gates,
+// fla/layers/gla.py:205-212, fla/layers/gsa.py:173-176).  Bound by memory: torch's chain (widen, logsigmoid, divide, and the same
+// back) moved 24 bytes per element forward and 30 backward where 6 and 8 are needed.
+template <bool SLOTS>
+__global__ void logsigmoid_gate_fwd_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ g, float* __restrict__ s, float n,
+                                           long long vecs) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= vecs) return;
+  float f[8], sv[8];
+  unpack8(reinterpret_cast<const uint4*>(x)[i], f);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    f[c] = __fdiv_rn(logsigmoidf_(f[c]), n);
+    if (SLOTS) sv[c] = -expm1f(f[c]);
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    reinterpret_cast<float4*>(g)[2 * i + h] = make_float4(f[4 * h], f[4 * h + 1], f[4 * h + 2], f[4 * h + 3]);
+    if (SLOTS) reinterpret_cast<float4*>(s)[2 * i + h] = make_float4(sv[4 * h], sv[4 * h + 1], sv[4 * h + 2], sv[4 * h + 3]);
+  }
+}
+
+// dx = (dg - exp(g) ds) sigmoid(-x) / n
+template <bool SLOTS>
+__global__ void logsigmoid_gate_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ dg, const float* __restrict__ ds,
+                                           __nv_bfloat16* __restrict__ dx, float n, long long vecs) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= vecs) return;
+  float f[8], o[8];
+  unpack8(reinterpret_cast<const uint4*>(x)[i], f);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float4 a = reinterpret_cast<const float4*>(dg)[2 * i + h];
+    o[4 * h] = a.x, o[4 * h + 1] = a.y, o[4 * h + 2] = a.z, o[4 * h + 3] = a.w;
+    if (SLOTS) {
+      const float4 b = reinterpret_cast<const float4*>(ds)[2 * i + h];
+      const float bs[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[4 * h + c] -= __expf(__fdiv_rn(logsigmoidf_(f[4 * h + c]), n)) * bs[c];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) o[c] = __fdiv_rn(o[c] * sigmoidf_(-f[c]), n);
+  reinterpret_cast<uint4*>(dx)[i] = pack8(o);
+}
+
 // one thread per (row, 8 channels)
 template <bool HAS_LB>
 __global__ void hgrn2_gate_fwd_kernel(const __nv_bfloat16* __restrict__ qr, const __nv_bfloat16* __restrict__ fr,
@@ -340,6 +386,27 @@ int fb_mamba2_post_bwd(const void* y, const void* x, long long ldx, const void* 
   if (P == 64) FB_POST_BWD(8); else if (P == 128) FB_POST_BWD(16); else FB_POST_BWD(32);
 #undef FB_POST_BWD
   return fb::launch_ok("mamba2_post_bwd_kernel");
+}
+
+// x, dx: bf16 [n]; g, s (optional), dg, ds (with s): fp32 [n]; n a multiple of 8, all 16-byte aligned
+int fb_logsigmoid_gate_fwd(const void* x, float* g, float* s, float normalizer, long long n, cudaStream_t stream) {
+  if (n == 0) return 0;
+  if ((n & 7) || (((uintptr_t)x | (uintptr_t)g | (uintptr_t)s) & 15)) return -2;
+  const long long vecs = n / 8;
+  const unsigned grid = (unsigned)((vecs + 255) / 256);
+  if (s != nullptr) logsigmoid_gate_fwd_kernel<true><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, g, s, normalizer, vecs);
+  else logsigmoid_gate_fwd_kernel<false><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, g, s, normalizer, vecs);
+  return fb::launch_ok("logsigmoid_gate_fwd_kernel");
+}
+
+int fb_logsigmoid_gate_bwd(const void* x, const float* dg, const float* ds, void* dx, float normalizer, long long n, cudaStream_t stream) {
+  if (n == 0) return 0;
+  if ((n & 7) || (((uintptr_t)x | (uintptr_t)dg | (uintptr_t)ds | (uintptr_t)dx) & 15)) return -2;
+  const long long vecs = n / 8;
+  const unsigned grid = (unsigned)((vecs + 255) / 256);
+  if (ds != nullptr) logsigmoid_gate_bwd_kernel<true><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, dg, ds, (__nv_bfloat16*)dx, normalizer, vecs);
+  else logsigmoid_gate_bwd_kernel<false><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, dg, ds, (__nv_bfloat16*)dx, normalizer, vecs);
+  return fb::launch_ok("logsigmoid_gate_bwd_kernel");
 }
 
 int fb_hgrn2_gate_tiles(long long rows) { return (int)((rows + GATE_TILE_ROWS - 1) / GATE_TILE_ROWS); }

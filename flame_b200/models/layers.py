@@ -14,6 +14,7 @@ import torch.nn.functional as F
 
 from ..ops import linear_attn as la
 from ..ops.attn_block import qkv_attention
+from ..ops.gates import logsigmoid_gate
 from ..ops.rope import rope_tables
 from ..ops.slots import reshaped, split_columns
 from ..ops.varlen import VarlenMeta
@@ -181,7 +182,7 @@ class GatedLinearAttention(nn.Module):
         v = reshaped(v, T, self.num_kv_heads, self.head_v_dim)
         if G > 1:
             k, gk, v = (t.repeat_interleave(G, 1) for t in (k, gk, v))
-        gk = F.logsigmoid(gk.float()) / self.gate_logit_normalizer
+        gk = logsigmoid_gate(gk, self.gate_logit_normalizer)
         if self.clamp_min is not None:
             gk = gk.clamp_min(self.clamp_min)
         if self.feature_map is not None:
@@ -389,8 +390,7 @@ class GatedSlotAttention(nn.Module):
         k = reshaped(k, T, self.num_kv_heads, self.head_k_dim)
         v = reshaped(v, T, self.num_kv_heads, self.head_v_dim)
         f = self.f_proj(x).reshape(T, self.num_kv_heads, self.num_slots)
-        f = F.logsigmoid(f.float()) / self.gate_logit_normalizer
-        s = 1 - f.exp()
+        f, s = logsigmoid_gate(f, self.gate_logit_normalizer, with_slots=True)
         if G > 1:
             k, v, f, s = (t.repeat_interleave(G, 1) for t in (k, v, f, s))
         o = gsa(q, k, v, s, f, meta, scale=self.scale)

@@ -4,10 +4,13 @@ framework kernels).
 ``hgrn2_gates(q_raw, f_raw, lower_bound)`` returns ``(q, k, g)`` of fla/layers/hgrn2.py:160-190:
 ``q = silu(q_raw)``, ``g = logsigmoid(f_raw)`` (with a lower bound: ``g = log(lb + (1 - lb) sigmoid(f_raw))``, the closed
 form of the reference's ``logaddexp(log lb, log1p(-lb) + logsigmoid f)``), ``k = 1 - exp(g)``; ``g`` in fp32.
+
+``logsigmoid_gate(x, normalizer, slots)`` returns ``g = logsigmoid(x) / normalizer`` in fp32 and, with ``slots``,
+``1 - exp(g)`` (fla/layers/gla.py:205-212, fla/layers/gsa.py:173-176).
 """
 from __future__ import annotations
 
-from ctypes import c_int, c_longlong, c_void_p
+from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional, Tuple
 
 import torch
@@ -22,6 +25,10 @@ _lib.register("fb_hgrn2_gate_bwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_vo
                                     c_void_p, c_longlong, c_int, c_void_p])
 
 
+_lib.register("fb_logsigmoid_gate_fwd", [c_void_p, c_void_p, c_void_p, c_float, c_longlong, c_void_p])
+_lib.register("fb_logsigmoid_gate_bwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_longlong, c_void_p])
+
+
 def hgrn2_gates_reference(q_raw: torch.Tensor, f_raw: torch.Tensor,
                           lower_bound: Optional[torch.Tensor]) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor]:
     q = F.silu(q_raw)
@@ -31,6 +38,51 @@ def hgrn2_gates_reference(q_raw: torch.Tensor, f_raw: torch.Tensor,
         g = torch.logaddexp(lb.log(), torch.log1p(-lb) + g)
     k = (1 - g.exp()).to(q_raw.dtype)
     return q, k, g
+
+
+def logsigmoid_gate_reference(x: torch.Tensor, normalizer: float, with_slots: bool = False):
+    g = F.logsigmoid(x.float()) / normalizer
+    return (g, 1 - g.exp()) if with_slots else g
+
+
+class _LogSigmoidGate(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, x, normalizer, with_slots):
+        g = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+        s = torch.empty_like(g) if with_slots else None
+        rc = _lib.lib().fb_logsigmoid_gate_fwd(x.data_ptr(), g.data_ptr(), _lib.ptr(s), normalizer, x.numel(), _lib.stream_ptr())
+        _lib.check(rc, "fb_logsigmoid_gate_fwd")
+        _lib.count_launch()
+        ctx.save_for_backward(x)
+        ctx.normalizer, ctx.with_slots = normalizer, with_slots
+        return (g, s) if with_slots else g
+
+    @staticmethod
+    def backward(ctx, dg, ds=None):
+        x, = ctx.saved_tensors
+
+        def full(d):
+            return torch.zeros(x.shape, dtype=torch.float32, device=x.device) if d is None else _aligned(d.float().contiguous())
+
+        dg, ds = full(dg), full(ds) if ctx.with_slots else None
+        dx = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+        rc = _lib.lib().fb_logsigmoid_gate_bwd(x.data_ptr(), dg.data_ptr(), _lib.ptr(ds), dx.data_ptr(), ctx.normalizer, x.numel(),
+                                               _lib.stream_ptr())
+        _lib.check(rc, "fb_logsigmoid_gate_bwd")
+        _lib.count_launch()
+        return dx, None, None
+
+
+def _aligned(x: torch.Tensor) -> torch.Tensor:
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
+def logsigmoid_gate(x: torch.Tensor, normalizer: float, with_slots: bool = False):
+    """``logsigmoid(x) / normalizer`` in fp32, and ``1 - exp`` of it with ``with_slots``.  One pass for contiguous bf16 on the
+    GPU; anything else (other types, odd sizes, column blocks) takes torch's chain."""
+    if _lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() % 8 == 0 and x.data_ptr() % 16 == 0:
+        return _LogSigmoidGate.apply(x, float(normalizer), with_slots)
+    return logsigmoid_gate_reference(x, normalizer, with_slots)
 
 
 class _Hgrn2Gates(torch.autograd.Function):
