@@ -9,8 +9,11 @@
 // fp32 in tensor memory, a bf16 copy in shared memory as the B operand of the next step's MMA.  One step is
 //   T = op(M_c) S16          one tcgen05 product, A tiles streamed by TMA through a two-stage ring
 //   S = alpha_c S - T + add  by the eight epilogue warps (a thread owns half of state rows r and r + 128), written back to tensor
-//                            memory, to shared memory (bf16, the MN-major B layout) and to global memory (bf16: the state
-//                            that the output stage and the backward pass read).
+//                            memory and to shared memory (bf16, the MN-major B layout), from where the TMA unit copies it to
+//                            global memory (the state that the output stage and the backward pass read).  The addend comes
+//                            the same way, a step ahead.  As 16-byte accesses to a row of its own per thread the two cost
+//                            the load/store unit 64 clocks per instruction, 8,000 of the 11,000 clocks of a step.  Per direction at 65,536 tokens, 8
+//                            heads of 128: 0.38 -> 0.205 ms; at 16,384 tokens, 6 heads of 256 x 512: 0.218 -> 0.164 ms.
 // It replaces one batched-GEMM launch per chunk position (about 20 us each, 2 x 63 of them per layer at 4096-token
 // documents) by a walk that costs a few microseconds per step.  Role of the reference's chunk_gated_delta_rule_fwd_h /
 // bwd_dhu kernels (fla/ops/common/chunk_delta_h.py:41-313), in the chunk-transition-matrix form of this library.
@@ -36,7 +39,7 @@ struct ScanParams {
   int reverse, shift;      // shift (reverse only): chunk c of `out` receives the adjoint of the state LEAVING it, L_{c+1} (0 at
                            // a document's last chunk), every chunk is written and L of the first chunk is not computed
   const float* alpha;      // [NC, H]
-  const __nv_bfloat16* add;  // forward: B [NC, H, dk, dv]; reverse: G [NC (+1), H, dk, dv]
+  const __nv_bfloat16* add;  // (initial states; the steps read it through its tensor map)  forward: B [NC, H, dk, dv]; reverse: G [NC (+1), H, dk, dv]
   __nv_bfloat16* out;      // forward: S16 [NC + 1, H, dk, dv] (chunk c + 1 receives the state after chunk c);
                            // reverse: L16 [NC + 1, H, dk, dv] (chunk c receives L_c; L16[last] = G[last] is the caller's)
   int* status;
@@ -48,8 +51,10 @@ struct Smem {
   static constexpr int STAGE_BYTES = DK * 64 * 2;      // one 64-wide k-block of M (either orientation)
   static constexpr int S_OFF = 0;
   static constexpr int RING_OFF = S_BYTES;
-  static constexpr int BAR_OFF = RING_OFF + STAGES * STAGE_BYTES;
-  static constexpr int TOTAL = BAR_OFF + 128 + 1024;
+  static constexpr int ADD_OFF = RING_OFF + STAGES * STAGE_BYTES;  // the step's addend: a box of 32 rows x 64 columns per warp and half
+  static constexpr int BOX_BYTES = 32 * 64 * 2;
+  static constexpr int BAR_OFF = ADD_OFF + 8 * (DK / 128) * BOX_BYTES;
+  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
 __device__ __forceinline__ uint32_t sw128(int row, int col) {  // byte offset inside a [rows][64] bf16 group, 128-byte swizzle
@@ -58,7 +63,8 @@ __device__ __forceinline__ uint32_t sw128(int row, int col) {  // byte offset in
 
 template <int DK>
 __global__ void __launch_bounds__(THREADS, DK == 128 ? 2 : 1)
-delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
+delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant__ CUtensorMap tmAdd, const __grid_constant__ CUtensorMap tmOut,
+                  ScanParams p) {
   using L = Smem<DK>;
   constexpr int HALVES = DK / 128;
   constexpr int KB = DK / 64;
@@ -76,7 +82,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* t_full = empty_bar + STAGES;
   uint64_t* s_ready = t_full + 1;
-  uint32_t* tmem_slot = (uint32_t*)(s_ready + 1);
+  uint64_t* add_bar = s_ready + 1;  // one per update warp
+  uint32_t* tmem_slot = (uint32_t*)(add_bar + 8);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
   const long long mat = (long long)DK * p.dv;                        // elements of one [dk, dv] state
@@ -92,9 +99,12 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
     }
     mbar_init(t_full, 1);
     mbar_init(s_ready, THREADS - 64);
+    for (int w = 0; w < 8; ++w) mbar_init(&add_bar[w], 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmM);
+    tma_prefetch_desc(&tmAdd);
+    tma_prefetch_desc(&tmOut);
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, TCOLS);
@@ -168,6 +178,16 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
     const int c_lo = ((warp - 2) >> 2) * CW, c_hi = c_lo + CW;
     const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
     bool ok = true;
+    uint64_t* my_add = &add_bar[warp - 2];
+    uint8_t* box = smem + L::ADD_OFF + (warp - 2) * HALVES * L::BOX_BYTES;
+    auto fetch_add = [&](int s) {  // lane 0: the addend of step s
+      const int c = p.reverse ? c_last - 1 - s : c_first + s;
+      mbar_expect_tx(my_add, HALVES * L::BOX_BYTES);
+#pragma unroll
+      for (int h = 0; h < HALVES; ++h)
+        tma_load_2d(box + h * L::BOX_BYTES, &tmAdd, my_add, (int)col0 + c_lo, (c * p.H + head) * DK + h * 128 + quarter * 32);
+    };
+    if (lane == 0 && n_steps > 0) fetch_add(0);
     // initial state: forward 0; reverse G[last] (which is also what L16[last] holds)
     {
       const int c_init = c_last;
@@ -219,26 +239,14 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
       const int c = p.reverse ? c_last - 1 - s : c_first + s;
       const int c_out = p.reverse ? c - p.shift : c + 1;
       const float a = __ldg(p.alpha + (long long)c * p.H + head);
-      // the addend rows of this step are fetched BEFORE waiting for the product: their global-memory latency (they are
-      // read once, from L2 or HBM) then overlaps the tensor-core work instead of adding to every 32-column piece
-      // (the second half of a 256-row state fetches its row when its turn comes: 64 more registers would spill)
-      uint4 ad[CW / 8];
-      {
-        const __nv_bfloat16* addrow = state_ptr(p.add, c, r) + c_lo;
-#pragma unroll
-        for (int g = 0; g < CW / 8; ++g) ad[g] = __ldg(reinterpret_cast<const uint4*>(addrow + g * 8));
-      }
+      // the addend came in while the previous step was worked on; the state's last copy to global memory has left the operand
+      if (!mbar_wait_warp(my_add, s & 1, p.status, abort_flag, ERR_WAIT_MISC)) { ok = false; break; }
+      if (lane == 0) tma_store_wait_read<0>();
       if (!mbar_wait_warp(t_full, s & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
 #pragma unroll
       for (int h = 0; h < HALVES; ++h) {
         const int row = h * 128 + r;
-        if (h > 0) {
-          const __nv_bfloat16* addrow = state_ptr(p.add, c, row) + c_lo;
-#pragma unroll
-          for (int g = 0; g < CW / 8; ++g) ad[g] = __ldg(reinterpret_cast<const uint4*>(addrow + g * 8));
-        }
-        __nv_bfloat16* outrow = const_cast<__nv_bfloat16*>(state_ptr(p.out, c_out, row));
 #pragma unroll
         for (int cc = 0; cc < CW; cc += 32) {
           const int c0 = c_lo + cc;
@@ -248,7 +256,8 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
           tmem_ld_wait();
 #pragma unroll
           for (int g = 0; g < 4; ++g) {
-            const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&ad[(cc >> 3) + g]);
+            const uint4 av = *reinterpret_cast<const uint4*>(box + h * L::BOX_BYTES + sw128(lane, cc + g * 8));
+            const __nv_bfloat162* a2 = reinterpret_cast<const __nv_bfloat162*>(&av);
             uint4 q;
             uint32_t* qw = reinterpret_cast<uint32_t*>(&q);
 #pragma unroll
@@ -263,7 +272,6 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
             }
             const int col = c0 + g * 8;
             *reinterpret_cast<uint4*>(sS + (col >> 6) * (DK * 128) + sw128(row, col & 63)) = q;
-            *reinterpret_cast<uint4*>(outrow + col) = q;
           }
           tmem_st_32x32(tmem_base + h * 2 * BN + BN + lane_sel + c0, st);
         }
@@ -272,7 +280,18 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
       tc_fence_before();
       fence_async_smem();
       mbar_arrive(s_ready);
+      __syncwarp();
+      if (lane == 0) {
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h) {
+          const int row = h * 128 + quarter * 32;
+          tma_store_2d(&tmOut, sS + (c_lo >> 6) * (DK * 128) + row * 128, (int)col0 + c_lo, (c_out * p.H + head) * DK + row);
+        }
+        tma_store_commit();
+        if (s + 1 < n_steps) fetch_add(s + 1);
+      }
     }
+    if (lane == 0) tma_store_wait_all<0>();
   }
   tc_fence_before();
   __syncthreads();
@@ -283,7 +302,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, ScanParams p) {
 }
 
 template <int DK>
-int launch_scan(const CUtensorMap& tm, const ScanParams& p, cudaStream_t stream) {
+int launch_scan(const CUtensorMap& tm, const CUtensorMap& tma, const CUtensorMap& tmo, const ScanParams& p, cudaStream_t stream) {
   auto kern = delta_scan_kernel<DK>;
   static bool configured = false;
   if (!configured) {
@@ -292,7 +311,7 @@ int launch_scan(const CUtensorMap& tm, const ScanParams& p, cudaStream_t stream)
     configured = true;
   }
   dim3 grid(p.dv / BN, p.H, p.n_docs);
-  kern<<<grid, THREADS, Smem<DK>::TOTAL, stream>>>(tm, p);
+  kern<<<grid, THREADS, Smem<DK>::TOTAL, stream>>>(tm, tma, tmo, p);
   return fb::launch_ok("delta_scan_kernel");
 }
 
@@ -307,14 +326,19 @@ int fb_delta_scan(const void* M, const void* add, const float* alpha, void* out,
                   int n_docs, int H, int NC, int dk, int dv, int reverse, cudaStream_t stream) {
   if (n_docs <= 0 || NC <= 0) return 0;
   if ((dk != 128 && dk != 256) || (dv % BN) != 0) return -2;
-  CUtensorMap tm;
+  CUtensorMap tm, tma, tmo;
   int rc = fb::make_tmap_2d(&tm, M, 2, (uint64_t)NC * H * dk, (uint64_t)dk, (uint64_t)dk, 64, 64, true);
+  if (rc) return rc;
+  if (((uintptr_t)add | (uintptr_t)out) & 15) return -2;
+  rc = fb::make_tmap_2d(&tma, add, 2, (uint64_t)NC * H * dk, (uint64_t)dv, (uint64_t)dv, 32, 64, true);
+  if (rc) return rc;
+  rc = fb::make_tmap_2d(&tmo, out, 2, (uint64_t)(NC + (reverse == 2 ? 0 : 1)) * H * dk, (uint64_t)dv, (uint64_t)dv, 32, 64, true);
   if (rc) return rc;
   ScanParams p;
   p.first = first; p.last = last; p.n_docs = n_docs; p.H = H; p.NC = NC; p.dk = dk; p.dv = dv; p.reverse = reverse != 0; p.shift = reverse == 2;
   p.alpha = alpha; p.add = (const __nv_bfloat16*)add; p.out = (__nv_bfloat16*)out;
   p.status = fb::status_ptr();
-  return dk == 128 ? launch_scan<128>(tm, p, stream) : launch_scan<256>(tm, p, stream);
+  return dk == 128 ? launch_scan<128>(tm, tma, tmo, p, stream) : launch_scan<256>(tm, tma, tmo, p, stream);
 }
 
 }  // extern "C"
