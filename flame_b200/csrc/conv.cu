@@ -7,7 +7,9 @@
 // Semantics of fla/modules/conv/triton/kernels.py:37-345; the row-strip partial reduction replaces its atomics.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
+#include <stddef.h>
 #include <stdint.h>
+#include <type_traits>
 #include "host_utils.cuh"
 
 namespace {
@@ -225,7 +227,7 @@ __global__ void conv_bwd_kernel(const __nv_bfloat16* __restrict__ dpre, const __
 // four channels (8-byte accesses, a warp covers 128 channels of a row) and a few consecutive rows, and issues all of its
 // loads before it uses any of them; the rows around its own come from L1, where the neighbouring warps of the block bring
 // them.  At 65,536 x 1,024 the walking form of one thread per eight channels took 0.086 ms forward (3.1 TB/s) and
-// 0.33 ms backward in three kernels.
+// 0.33 ms backward in three kernels; this forward takes 0.078 ms.
 constexpr int CW = 4;          // taps
 constexpr int CLANES = 32;     // threads along the channels
 constexpr int CGROUPS = 8;     // row groups of a block
@@ -281,13 +283,17 @@ __global__ void __launch_bounds__(CLANES * CGROUPS) conv4_fwd_kernel(const __nv_
   for (int i = 0; i < FROWS; ++i) p[i] = r0 + i < T ? pos[r0 + i] : 0;
   float wv[CW][4], bias[4];
   load_taps(w, b, d0, wv, bias);
+  bool whole = r0 + FROWS <= T;  // every tap of every row lies in the row's document (the same for the whole warp)
+#pragma unroll
+  for (int i = 0; i < FROWS; ++i) whole = whole && p[i] >= CW - 1;
+  auto rows = [&](auto all) {
 #pragma unroll
   for (int i = 0; i < FROWS; ++i) {
-    if (r0 + i >= T) break;
+    if (!decltype(all)::value && r0 + i >= T) break;
     float acc[4] = {bias[0], bias[1], bias[2], bias[3]};
 #pragma unroll
     for (int j = 0; j < CW; ++j) {
-      if (j <= p[i]) {
+      if (decltype(all)::value || j <= p[i]) {
         float xv[4];
         unpack4(xq[i + CW - 1 - j], xv);
 #pragma unroll
@@ -299,111 +305,199 @@ __global__ void __launch_bounds__(CLANES * CGROUPS) conv4_fwd_kernel(const __nv_
       if (SILU) acc[c] *= sigmoidf_(acc[c]);
     *reinterpret_cast<uint2*>(y + (r0 + i) * ldy + d0) = pack4(acc);
   }
+  };
+  if (whole) rows(std::true_type{});
+  else rows(std::false_type{});
 }
 
-// A block walks the tiles of 64 rows of its strip; dpre of the three rows behind a thread's own is recomputed (11 rows for 8).
+// Two fp32 lanes per instruction (sm_100): the backward forms about 60 products per channel and row.
+using f2 = unsigned long long;
+__device__ __forceinline__ f2 f2_make(float a, float b) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 f2_get(f2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f2 f2_fma(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 f2_mul(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_add(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 f2_unpack2(uint32_t q) { return f2_make(__uint_as_float(q << 16), __uint_as_float(q & 0xffff0000u)); }
+// 8 bytes into shared memory, zeros where `in` is false (nothing is read then)
+__device__ __forceinline__ void cp_async8(void* dst, const void* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(in ? 8 : 0) : "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+constexpr int BCH = 2 * CLANES;  // channels of a block, backward: a thread owns two
+struct alignas(16) ConvTile {  // the stages follow one another: each has to start where 8-byte copies may
+  uint32_t x[BTILE + 2 * (CW - 1)][CLANES];  // rows r0 - 3 .. r0 + 66, two channels a word
+  uint32_t g[BTILE + CW - 1][CLANES];        // rows r0 .. r0 + 66
+  int pos[BTILE + CW + 1];
+};
+constexpr int CSTAGES = 2;
+static_assert(sizeof(ConvTile) % 16 == 0 && offsetof(ConvTile, g) % 8 == 0, "alignment of the copies");
+
+// A block walks the tiles of 64 rows of its strip, the next tile on its way into shared memory (cp.async) while it works on
+// this one; there are as many strips as fill the GPU once (four blocks per SM), so that the partial sums of the taps'
+// gradients are few.  dpre of the three rows behind a thread's own is recomputed (11 rows for 8).  At 65,536 x 1,024 0.155 ms
+// and 0.003 ms to sum the strips' partials; the form that loaded one tile per block into registers before it used any of it took
+// 0.194 ms and 0.035 ms (1,024 strips), four channels per thread with 127 registers 0.16 ms.
 template <bool SILU>
-__global__ void __launch_bounds__(CLANES * CGROUPS, 2) conv4_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+__global__ void __launch_bounds__(CLANES * CGROUPS, 4) conv4_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                                                                         const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ b,
                                                                         const int* __restrict__ pos, __nv_bfloat16* __restrict__ dx,
                                                                         float* __restrict__ part, long long T, int D, long long ldx, long long ldy,
                                                                         long long ldd, int tiles_per_strip) {
-  __shared__ float red[CGROUPS][CLANES * 4 * (CW + 1)];
-  const int d0 = (blockIdx.x * CLANES + threadIdx.x) * 4;
+  extern __shared__ __align__(16) uint8_t conv_smem[];
+  ConvTile* stage = reinterpret_cast<ConvTile*>(conv_smem);
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * CLANES + tx;
+  const int c_block = blockIdx.x * BCH, d0 = c_block + 2 * tx;
   const bool live = d0 < D;
-  float wv[CW][4], bias[4], dw[CW][4], db[4];
-  if (live) load_taps(w, b, d0, wv, bias);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-#pragma unroll
-    for (int j = 0; j < CW; ++j) dw[j][c] = 0.f;
-    db[c] = 0.f;
-  }
   constexpr int H = CW - 1;
-  for (int tile = 0; tile < tiles_per_strip; ++tile) {
-    const long long r0 = (((long long)blockIdx.y * tiles_per_strip + tile) * CGROUPS + threadIdx.y) * BROWS;
-    if (!live || r0 >= T) break;
-    uint2 xq[BROWS + 2 * H], gq[BROWS + H];
-    int p[BROWS + H];
-#pragma unroll
-    for (int i = 0; i < BROWS + 2 * H; ++i) {
-      const long long r = r0 + i - H;
-      xq[i] = r >= 0 && r < T ? *reinterpret_cast<const uint2*>(x + r * ldx + d0) : make_uint2(0u, 0u);
-    }
-#pragma unroll
-    for (int i = 0; i < BROWS + H; ++i) {
-      const bool in = r0 + i < T;
-      gq[i] = in ? *reinterpret_cast<const uint2*>(dy + (r0 + i) * ldy + d0) : make_uint2(0u, 0u);
-      p[i] = in ? pos[r0 + i] : -1;
-    }
-    float g[CW][4];  // dpre of the last four rows, g[0] the newest
-#pragma unroll
-    for (int i = 0; i < BROWS + H; ++i) {
-#pragma unroll
-      for (int j = CW - 1; j >= 1; --j)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) g[j][c] = g[j - 1][c];
-      unpack4(gq[i], g[0]);
-      float xv[CW][4];
-#pragma unroll
-      for (int j = 0; j < CW; ++j) unpack4(xq[i + H - j], xv[j]);
-      if (SILU) {
-        float pre[4] = {bias[0], bias[1], bias[2], bias[3]};
-#pragma unroll
-        for (int j = 0; j < CW; ++j)
-          if (j <= p[i]) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) pre[c] = fmaf(wv[j][c], xv[j][c], pre[c]);
-          }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float sg = sigmoidf_(pre[c]);
-          g[0][c] *= sg * (1.f + pre[c] * (1.f - sg));
+  const long long tile0 = (long long)blockIdx.y * tiles_per_strip;
+  auto fetch = [&](int tile) {
+    const long long r0 = (tile0 + tile) * BTILE;
+    if (tile < tiles_per_strip && r0 < T) {
+      ConvTile& s = stage[tile % CSTAGES];
+      constexpr int PER_ROW = BCH / 4;  // 8-byte pieces
+      const int piece = tid % PER_ROW, c = c_block + piece * 4;
+      if (c < D) {
+        for (int i = tid / PER_ROW; i < BTILE + 2 * H; i += CLANES * CGROUPS / PER_ROW) {
+          const long long r = r0 + i - H;
+          const bool in = r >= 0 && r < T;
+          cp_async8(&s.x[i][piece * 2], in ? x + r * ldx + c : x, in);
+        }
+        for (int i = tid / PER_ROW; i < BTILE + H; i += CLANES * CGROUPS / PER_ROW) {
+          const bool in = r0 + i < T;
+          cp_async8(&s.g[i][piece * 2], in ? dy + (r0 + i) * ldy + c : dy, in);
         }
       }
-      if (i < BROWS) {  // the rows behind belong to other threads' sums
+      if (tid < BTILE + H) s.pos[tid] = r0 + tid < T ? pos[r0 + tid] : -1;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  f2 wv[CW], bias = 0ull, dw[CW], db = 0ull;
+  if (live) {
+    float f[8];
+    unpack8(*reinterpret_cast<const uint4*>(w + (long long)d0 * CW), f);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) db[c] += g[0][c];
+    for (int j = 0; j < CW; ++j) wv[j] = f2_make(f[CW - 1 - j], f[CW + CW - 1 - j]);  // tap at distance j
+    if (b != nullptr) bias = f2_unpack2(*reinterpret_cast<const uint32_t*>(b + d0));
+  }
 #pragma unroll
-        for (int j = 0; j < CW; ++j)
-          if (j <= p[i]) {
+  for (int j = 0; j < CW; ++j) dw[j] = 0ull;
+  fetch(0);
+  for (int tile = 0; tile < tiles_per_strip && (tile0 + tile) * BTILE < T; ++tile) {
+    fetch(tile + 1);
+    cp_async_wait<1>();
+    __syncthreads();
+    const ConvTile& s = stage[tile % CSTAGES];
+    const int first = ty * BROWS;
+    const long long r0 = (tile0 + tile) * BTILE + first;
+    if (live && r0 < T) {
+      bool whole = true;  // every tap of every row lies in the row's document (the same for the whole warp)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) dw[j][c] = fmaf(g[0][c], xv[j][c], dw[j][c]);
+      for (int i = 0; i < BROWS + H; ++i) whole = whole && s.pos[first + i] >= H;
+      __nv_bfloat16* out = dx + r0 * ldd + d0;
+      // straight-line code for whole rows: with a branch per tap the warp waits out each row's sigmoid by itself
+      auto rows = [&](auto all) {
+        f2 g[CW], xv[CW];  // dpre and x of the last four rows, [0] the newest
+        int p[CW];         // their positions
+#pragma unroll
+        for (int j = 1; j < CW; ++j) xv[j - 1] = f2_unpack2(s.x[first + H - j][tx]);
+#pragma unroll
+        for (int i = 0; i < BROWS + H; ++i) {
+#pragma unroll
+          for (int j = CW - 1; j >= 1; --j) g[j] = g[j - 1], xv[j] = xv[j - 1], p[j] = p[j - 1];
+          p[0] = decltype(all)::value ? H : s.pos[first + i];
+          g[0] = f2_unpack2(s.g[first + i][tx]);
+          xv[0] = f2_unpack2(s.x[first + i + H][tx]);
+          if (SILU) {
+            f2 pre = bias;
+#pragma unroll
+            for (int j = 0; j < CW; ++j)
+              if (decltype(all)::value || j <= p[0]) pre = f2_fma(wv[j], xv[j], pre);
+            const float2 z = f2_get(pre);
+            const float s0 = sigmoidf_(z.x), s1 = sigmoidf_(z.y);
+            g[0] = f2_mul(g[0], f2_make(s0 * (1.f + z.x * (1.f - s0)), s1 * (1.f + z.y * (1.f - s1))));
           }
-      }
-      if (i >= H && r0 + i - H < T) {  // dx[s] = sum_j w[tap j] dpre[s + j] while row s + j is at least j tokens into its document
-        float acc[4];
+          if (i < BROWS) {  // the rows behind belong to other threads' sums
+            db = f2_add(db, g[0]);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[c] = wv[0][c] * g[H][c];
-        bool alive = true;
+            for (int j = 0; j < CW; ++j)
+              if (decltype(all)::value || j <= p[0]) dw[j] = f2_fma(g[0], xv[j], dw[j]);
+          }
+          if (i >= H && (decltype(all)::value || r0 + i - H < T)) {
+            // dx[s] = sum_j w[tap j] dpre[s + j] while row s + j is at least j tokens into its document
+            f2 acc = f2_mul(wv[0], g[H]);
+            bool alive = true;
 #pragma unroll
-        for (int j = 1; j < CW; ++j) {
-          alive = alive && p[i - H + j] >= j;
-          if (alive) {
-#pragma unroll
-            for (int c = 0; c < 4; ++c) acc[c] = fmaf(wv[j][c], g[H - j][c], acc[c]);
+            for (int j = 1; j < CW; ++j) {
+              alive = decltype(all)::value || (alive && p[H - j] >= j);
+              if (alive) acc = f2_fma(wv[j], g[H - j], acc);
+            }
+            const float2 a = f2_get(acc);
+            *reinterpret_cast<__nv_bfloat162*>(out + (i - H) * ldd) = __floats2bfloat162_rn(a.x, a.y);
           }
         }
-        *reinterpret_cast<uint2*>(dx + (r0 + i - H) * ldd + d0) = pack4(acc);
-      }
+      };
+      if (whole) rows(std::true_type{});
+      else rows(std::false_type{});
     }
+    __syncthreads();  // the stage is free for the tile after next
   }
-  float* mine = red[threadIdx.y] + threadIdx.x * 4 * (CW + 1);
+  cp_async_wait<0>();
+  float* red = reinterpret_cast<float*>(conv_smem);  // [CGROUPS][BCH * (CW + 1)]: the stages are done with
+  constexpr int NRED = BCH * (CW + 1);
+  float* mine = red + ty * NRED + tx * 2 * (CW + 1);
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-#pragma unroll
-    for (int j = 0; j < CW; ++j) mine[c * (CW + 1) + (CW - 1 - j)] = dw[j][c];
-    mine[c * (CW + 1) + CW] = db[c];
+  for (int j = 0; j < CW; ++j) {
+    const float2 v = f2_get(dw[j]);
+    mine[CW - 1 - j] = v.x;
+    mine[CW + 1 + CW - 1 - j] = v.y;
   }
+  const float2 vb = f2_get(db);
+  mine[CW] = vb.x;
+  mine[CW + 1 + CW] = vb.y;
   __syncthreads();
-  const int n = min(CLANES * 4, D - (int)blockIdx.x * CLANES * 4) * (CW + 1);
-  float* dst = part + ((long long)blockIdx.y * D + (long long)blockIdx.x * CLANES * 4) * (CW + 1);
-  for (int i = threadIdx.y * CLANES + threadIdx.x; i < n; i += CLANES * CGROUPS) {
+  const int n = min(BCH, D - c_block) * (CW + 1);
+  float* dst = part + ((long long)blockIdx.y * D + c_block) * (CW + 1);
+  for (int i = tid; i < n; i += CLANES * CGROUPS) {
     float v = 0.f;
 #pragma unroll
-    for (int k = 0; k < CGROUPS; ++k) v += red[k][i];
+    for (int k = 0; k < CGROUPS; ++k) v += red[k * NRED + i];
     dst[i] = v;
   }
+}
+
+template <bool SILU>
+int launch_conv4_bwd(const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w, const __nv_bfloat16* b, const int* pos,
+                     __nv_bfloat16* dx, float* part, long long T, int D, long long ldx, long long ldy, long long ldd, int per, dim3 grid,
+                     cudaStream_t stream) {
+  constexpr int bytes = CSTAGES * (int)sizeof(ConvTile);
+  static_assert(bytes >= CGROUPS * BCH * (CW + 1) * 4, "the partial sums of a block reuse the stages");
+  static const cudaError_t rc = cudaFuncSetAttribute(conv4_bwd_kernel<SILU>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (rc != cudaSuccess) return (int)rc;
+  conv4_bwd_kernel<SILU><<<grid, dim3(CLANES, CGROUPS), bytes, stream>>>(dy, x, w, b, pos, dx, part, T, D, ldx, ldy, ldd, per);
+  return fb::launch_ok("conv4_bwd_kernel");
 }
 
 // Sums the per-strip partials in a fixed order: a block of 32 outputs x 8 strip groups reads coalesced rows of partials.
@@ -469,12 +563,13 @@ int fb_short_conv_bwd(const void* dy, const void* x, const void* w, const void* 
   const __nv_bfloat16 *gg = (const __nv_bfloat16*)dy, *xx = (const __nv_bfloat16*)x, *ww = (const __nv_bfloat16*)w, *bb = (const __nv_bfloat16*)b;
   if (W == CW) {
     if (((uintptr_t)w & 15) || ((uintptr_t)b & 7) || ((uintptr_t)x & 7) || ((uintptr_t)dy & 7)) return -2;
-    const int tiles = (int)((T + BTILE - 1) / BTILE), per = (tiles + strips - 1) / strips;
+    const int tiles = (int)((T + BTILE - 1) / BTILE), blocks_x = (D + BCH - 1) / BCH;
+    strips = min(strips, max(1, 4 * 148 / blocks_x));  // four blocks on each of 148 SMs
+    const int per = (tiles + strips - 1) / strips;
     strips = (tiles + per - 1) / per;
-    const dim3 grid((D / 4 + CLANES - 1) / CLANES, strips), block(CLANES, CGROUPS);
-    if (silu) conv4_bwd_kernel<true><<<grid, block, 0, stream>>>(gg, xx, ww, bb, pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, ldd, per);
-    else conv4_bwd_kernel<false><<<grid, block, 0, stream>>>(gg, xx, ww, bb, pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, ldd, per);
-    rc = fb::launch_ok("conv4_bwd_kernel");
+    const dim3 grid(blocks_x, strips);
+    rc = silu ? launch_conv4_bwd<true>(gg, xx, ww, bb, pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, ldd, per, grid, stream)
+              : launch_conv4_bwd<false>(gg, xx, ww, bb, pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, ldd, per, grid, stream);
   } else {
     if (ldd != ldx) return -2;
     rc = silu ? launch_conv_point<true, true>(x, w, b, pos, dy, dpre, T, D, W, ldx, ldy, stream)
