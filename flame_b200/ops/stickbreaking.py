@@ -18,6 +18,7 @@ from .varlen import VarlenMeta
 
 vp, i32, i64, f32 = c_void_p, c_int, c_longlong, c_float
 _lib.register("fb_sb_attn_fwd", [vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i64, i32, i32, i64, i64, i64, i64, f32, vp])
+_lib.register("fb_cast_column_blocks", [vp, vp, i64, i32, i64, vp])
 _lib.register("fb_sb_attn_bwd", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i64, i32,
                                  i64, i64, i64, i64, i64, i64, f32, vp])
 
@@ -92,8 +93,9 @@ class _QkvSBFn(torch.autograd.Function):
         do = do if do.is_contiguous() else do.contiguous()
         dqkv = torch.empty_like(qkv).view(T, 3, H, Dh)
         dkv = _backward(q, k, v, o, o_lo, rem, do, None, ctx.meta, ctx.scale, dqkv[:, 0])
-        dqkv[:, 1].copy_(dkv[0])
-        dqkv[:, 2].copy_(dkv[1])
+        rc = _lib.lib().fb_cast_column_blocks(dkv.data_ptr(), dqkv[:, 1].data_ptr(), T, H * Dh, dqkv.stride(0), _lib.stream_ptr())
+        _lib.check(rc, "fb_cast_column_blocks")
+        _lib.count_launch()
         return dqkv.view(T, 3 * H * Dh), None, None, None, None
 
 
