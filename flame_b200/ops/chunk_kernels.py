@@ -226,12 +226,12 @@ _lib.register("fb_gla_prep_fwd", [c_void_p] * 9 + [c_int, c_int, c_int, c_float,
 def gla_prep(qp, kp, gp, scale: float):
     """One pass over a chunk's q, k, g producing the cumulative decay and every scaled operand of the GLA chunk algorithm (see
     ``csrc/chunk.cu: gla_prep_fwd_kernel``).  q, k ``[NC, 64, H, dk]`` bf16, g ``[NC, 64, H, dk]`` fp32, all contiguous.  Returns
-    ``(b, khat, qbar, qt, k3, alpha)``."""
+    ``(b, khat, qbar, qt, k3, alpha)``; qt ``[NC, 48, H, dk]``."""
     NC, C, H, dk = qp.shape
     assert C == 64 and qp.dtype == torch.bfloat16 and gp.dtype == torch.float32
     dev = qp.device
     b = torch.empty_like(gp)
-    khat, qbar, qt = torch.empty_like(kp), torch.empty_like(qp), torch.empty_like(qp)
+    khat, qbar, qt = torch.empty_like(kp), torch.empty_like(qp), torch.empty(NC, 48, H, dk, dtype=torch.bfloat16, device=dev)
     k3 = torch.empty(NC, 3, 48, H, dk, dtype=torch.bfloat16, device=dev)
     alpha = torch.empty(NC, H, dk, dtype=torch.float32, device=dev)
     rc = _lib.lib().fb_gla_prep_fwd(qp.data_ptr(), kp.data_ptr(), gp.data_ptr(), b.data_ptr(), khat.data_ptr(),

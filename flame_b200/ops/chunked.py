@@ -699,7 +699,7 @@ class _Gla(torch.autograd.Function):
         S = _state_scan(lay, alpha, bgemm(_hm(khat), vh, a_mn=True, b_mn=True, out_dtype=torch.float32), q.dtype, reverse=False)
         # off-diagonal sub-blocks: batch (chunk, I) multiplies the 16 query rows of sub-block I, re-based on the sub-block's
         # first row, with the keys before it re-based on the same row; later keys are zero in k3
-        qt3 = qt[:, 16:].reshape(NC * 3, 16, H, dk)
+        qt3 = qt.view(NC * 3, 16, H, dk)
         k3 = k3.view(NC * 3, 48, H, dk)
         A = chunk_kernels.gla_scores(q, k, b, bgemm(_hm(qt3), _hm(k3), alpha=scale), scale)
         o = bgemm(_hm(qbar), S, b_mn=True, more=[(A, vh, False, True, 1)], out=_token_major(NC, H, C, dv, q.dtype, q.device))
@@ -723,11 +723,9 @@ class _Gla(torch.autograd.Function):
         dA = bgemm(doh, vh, mask=MASK_TRIL)
         dqbar, dkhat = bgemm(doh, S, out=tok(dk)), bgemm(vh, Ln, out=tok(dk))
         dblk = dA.view(NC, H, 4, 16, 64)[:, :, 1:, :, :48].permute(0, 2, 1, 3, 4).reshape(NC * 3, H, 16, 48)
-        dqt = torch.empty(NC, 64, H, dk, dtype=dt, device=dev)                            # rows of sub-block 0 are not read
         dqt3 = bgemm(dblk, _hm(k3), b_mn=True, alpha=scale, out=_token_major(NC * 3, H, 16, dk, dt, dev))
-        dqt[:, 16:].copy_(back(dqt3).reshape(NC, 48, H, dk))
         dk3 = bgemm(dblk, _hm(qt3), a_mn=True, b_mn=True, alpha=scale, out=_token_major(NC * 3, H, 48, dk, dt, dev))
-        dq, dkk, dg = chunk_kernels.gla_bwd(q, k, b, dA, back(dkhat), back(dqbar), dqt, back(dk3), _pair_dot(Ln, S, per_row=True), scale)
+        dq, dkk, dg = chunk_kernels.gla_bwd(q, k, b, dA, back(dkhat), back(dqbar), back(dqt3), back(dk3), _pair_dot(Ln, S, per_row=True), scale)
         return dq, dkk, back(dvv), dg, None, None
 
 

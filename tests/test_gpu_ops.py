@@ -547,3 +547,82 @@ def test_mamba2_glue_kernels_match_the_elementwise_chain():
         assert rel_err(a, b) < 1e-2
     for a, b in zip(grads_k, grads_r):
         assert rel_err(a, b) < 2e-2, rel_err(a, b)
+
+
+@pytest.mark.parametrize("with_slots", [False, True])
+@pytest.mark.parametrize("shape", [(1, 8), (3, 5, 8), (77, 4, 64)])
+def test_logsigmoid_gate(shape, with_slots):
+    """One pass against torch in fp64: the results are fp32 (a few ulp of __expf and log1pf; 1 - exp(g) loses none to
+    cancellation), the gradient is rounded to bf16 once (2^-9 relative)."""
+    from flame_b200.ops.gates import logsigmoid_gate
+    torch.manual_seed(0)
+    x = (torch.randn(*shape, device="cuda") * 6).bfloat16()
+    x.view(-1)[:4] = torch.tensor([60.0, -60.0, 0.0, -1e4])
+    x.requires_grad_(True)
+    xr = x.detach().double().requires_grad_(True)
+    got = logsigmoid_gate(x, 16.0, with_slots)
+    want = torch.nn.functional.logsigmoid(xr) / 16.0
+    got = got if with_slots else (got,)
+    wants = (want, 1 - want.exp()) if with_slots else (want,)
+    grads = [torch.randn_like(g) for g in got]
+    for g, w in zip(got, wants):
+        assert g.dtype == torch.float32 and ((g.double() - w).abs() <= 2e-6 * w.abs() + 1e-9).all()
+    dx, = torch.autograd.grad(got, x, grads)
+    dw, = torch.autograd.grad(wants, xr, [g.double() for g in grads])
+    scale = sum(g.double().abs() for g in grads) / 16 * torch.sigmoid(-xr.detach())
+    assert ((dx.double() - dw).abs() <= 2.0 ** -8 * dw.abs() + 1e-5 * scale + 1e-9).all()
+
+
+@pytest.mark.parametrize("with_bias", [False, True])
+@pytest.mark.parametrize("M", [1, 31, 128, 200, 520])
+@pytest.mark.parametrize("N", [8, 40, 64, 72, 256, 264])
+def test_gemm_result_boxes(M, N, with_bias):
+    """bf16 results at the edges of the boxes that leave by TMA (32 rows x 64 columns; tiles of 256 and of 128 rows), in storage
+    whose neighbours stay untouched; fp32 sums of K = 72 products and one bf16 rounding (2^-9 relative)."""
+    from flame_b200.ops.gemm import gemm_nt
+    torch.manual_seed(M * 1000 + N)
+    K = 72
+    a, b = torch.randn(M, K, device=DEV).bfloat16(), torch.randn(N, K, device=DEV).bfloat16()
+    bias = torch.randn(N + 1, device=DEV).bfloat16()
+    want = 0.5 * (a.double() @ b.double().t())
+    size = a.double().abs() @ b.double().abs().t()
+    for offset in (0, 1) if with_bias else (0,):   # an unaligned bias takes scalar loads
+        bb = bias[offset:offset + N] if with_bias else None
+        store = torch.full((M + 2, (N + 7) // 8 * 8 + 8), 7.0, dtype=torch.bfloat16, device=DEV)
+        gemm_nt(a, b, out=store[1:M + 1, :N], alpha=0.5, bias=bb)
+        ref = want + bb.double() if with_bias else want
+        got = store[1:M + 1, :N].double()
+        assert ((got - ref).abs() <= 2.0 ** -8 * ref.abs() + 2.0 ** -17 * size + 1e-30).all()
+        store[1:M + 1, :N] = 7.0
+        assert (store == 7.0).all()
+
+
+@pytest.mark.parametrize("activation", ["silu", None])
+@pytest.mark.parametrize("T,D", [(1, 8), (67, 72), (1333, 2048), (2500, 4096)])
+def test_short_conv_strips(T, D, activation):
+    """Width 4, strips of one and of several 64-row tiles, ragged ends, documents shorter than the taps; against torch in fp32.
+    Outputs and dx are rounded to bf16 once (2^-9); dw and db sum T products in fp32 and are rounded once."""
+    from flame_b200.ops.conv import short_conv
+    torch.manual_seed(T + D)
+    lens, left = [], T
+    for n in [1, 2, 3, 70, 1] + [509] * 9:
+        lens.append(min(n, left))
+        left -= lens[-1]
+        if left == 0:
+            break
+    meta = _meta(lens)
+    x, dy = torch.randn(T, D, device=DEV).bfloat16().requires_grad_(True), torch.randn(T, D, device=DEV).bfloat16()
+    w, b = (torch.randn(D, 1, 4, device=DEV) * 0.4).bfloat16().requires_grad_(True), torch.randn(D, device=DEV).bfloat16().requires_grad_(True)
+    y = short_conv(x, w, b, meta, activation)
+    got = torch.autograd.grad(y, [x, w, b], dy)
+    xr, wr, br = (t.detach().double().requires_grad_(True) for t in (x, w, b))
+    parts, c = [], 0
+    for n in lens:
+        z = torch.nn.functional.conv1d(torch.nn.functional.pad(xr[c:c + n].t()[None], (3, 0)), wr, br, groups=D)[0].t()
+        parts.append(torch.nn.functional.silu(z) if activation else z)
+        c += n
+    want_y = torch.cat(parts)
+    want = torch.autograd.grad(want_y, [xr, wr, br], dy.double())
+    assert rel_err(y, want_y) < 3e-3
+    for g, r in zip(got, want):
+        assert rel_err(g, r) < 5e-3
