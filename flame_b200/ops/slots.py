@@ -9,7 +9,8 @@ copied in.
 A slot serves ONE consumer: two operators reading the same view would overwrite each other's gradient before autograd adds
 them, so a slot is given away once (``of``) and later askers get none.  The buffer belongs to one run of the backward: it
 is allocated by that run's first ``take`` and handed to autograd at the end of it; a run that stopped short of it (gradients
-asked for at the views only) leaves its buffer to whoever got those gradients, and the next run makes its own.
+asked for at the views only) leaves its buffer to whoever got those gradients, and the next run makes its own.  It also belongs
+to the stream it was allocated on: a consumer on another stream gets a matrix of its own, which is copied in.
 """
 from __future__ import annotations
 
@@ -17,10 +18,12 @@ from typing import Optional, Tuple
 
 import torch
 
+from . import _lib
+
 
 class _Holder:
     def __init__(self, width: int) -> None:
-        self.width, self.buffer, self.run = width, None, -1
+        self.width, self.buffer, self.run, self.stream = width, None, -1, 0
 
 
 class Slot:
@@ -33,10 +36,11 @@ class Slot:
         run = torch._C._current_graph_task_id()
         if run == -1:  # not inside a backward run
             return torch.empty(rows, n, dtype=dtype, device=device)
+        stream = _lib.stream_ptr() if device.type == "cuda" else 0
         if h.buffer is None or h.run != run:
-            h.buffer, h.run = torch.empty(rows, h.width, dtype=dtype, device=device), run
+            h.buffer, h.run, h.stream = torch.empty(rows, h.width, dtype=dtype, device=device), run, stream
         b = h.buffer
-        if n != self.n or b.shape[0] != rows or b.dtype != dtype or b.device != device:
+        if n != self.n or h.stream != stream or b.shape[0] != rows or b.dtype != dtype or b.device != device:
             return torch.empty(rows, n, dtype=dtype, device=device)
         return b[:, self.col:self.col + n]
 

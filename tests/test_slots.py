@@ -56,6 +56,18 @@ def test_unused_block_and_partial_runs():
     torch.testing.assert_close(gx, 2 * want, rtol=1e-12, atol=1e-12)
 
 
+def test_another_stream_gets_its_own_matrix(monkeypatch):
+    """The shared buffer is written on the stream that allocated it only; the other block's gradient is copied in."""
+    holder = slots._Holder(5)
+    first, second = slots.Slot(holder, 0, 2), slots.Slot(holder, 2, 3)
+    monkeypatch.setattr(torch._C, "_current_graph_task_id", lambda: 7)
+    a = first.take(4, 2, torch.float32, torch.device("cpu"))
+    holder.stream = 1
+    b = second.take(4, 3, torch.float32, torch.device("cpu"))
+    assert a.untyped_storage().data_ptr() == holder.buffer.untyped_storage().data_ptr()
+    assert b.untyped_storage().data_ptr() != holder.buffer.untyped_storage().data_ptr()
+
+
 def _adjacent(layers):
     """The layers' weights as row blocks of one matrix, their gradients too."""
     ws = [l.weight for l in layers]
