@@ -415,3 +415,28 @@ def test_bgemm_result_boxes(M, N):
             mask = torch.ones(view.shape, dtype=torch.bool, device=dev)
             mask[1:, :, :M, :N] = False
             assert (view[mask] == 7.0).all()
+
+
+@pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("x16", [False, True])
+@pytest.mark.parametrize("rows,cols,per_row", [(3, 12, True), (4, 8, False), (16, 72, True)])
+def test_state_scan_widths(rows, cols, per_row, x16, reverse):
+    """Chunk-state recurrence with 16-byte and with 8-byte accesses, documents of one to nine chunks, against the loop in fp64:
+    fp32 accumulation (a few 2^-24 per step) and one rounding of the state to bf16 (2^-9)."""
+    from flame_b200.ops.chunked import ChunkLayout, _state_scan
+    torch.manual_seed(rows * cols)
+    lens, H = [1, 64, 65, 570], 2
+    lay = ChunkLayout(_meta(lens))
+    X = torch.randn(lay.NC, H, rows, cols, device=DEV).to(torch.bfloat16 if x16 else torch.float32)
+    alpha = torch.rand(lay.NC, H, rows, device=DEV) if per_row else torch.rand(lay.NC, H, device=DEV)
+    got = _state_scan(lay, alpha, X, torch.bfloat16, reverse=reverse)
+    want, c = torch.zeros(lay.NC, H, rows, cols, dtype=torch.float64, device=DEV), 0
+    a = alpha.double()[..., None] if per_row else alpha.double()[..., None, None]
+    for n in lens:
+        k = (n + 63) // 64
+        s = torch.zeros(H, rows, cols, dtype=torch.float64, device=DEV)
+        for i in (range(c + k - 1, c - 1, -1) if reverse else range(c, c + k)):
+            want[i] = s
+            s = a[i] * s + X[i].double()
+        c += k
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
