@@ -654,6 +654,7 @@ int fb_bgemm_bf16(const FbBOperand* ops, int n_pairs, const FbBEpilogue* e, int 
   p.status = fb::status_ptr();
   if ((p.C16 != nullptr || p.Cin != nullptr) && p.out_mode == 0) return -3;
   if ((p.C16 != nullptr || p.add16 != nullptr) && ((p.ld16 & 7) || (p.stride_lo16 & 7) || (p.stride_hi16 & 7))) return -2;
+  if (!fb::aligned(16, e->C16, e->add16, e->Cin)) return -2;
   // results leave by TMA unless there is a state step or an index in the way (see the kernel)
   const bool out16 = p.out_mode == 0;
   const int hi_c = p.c.hi_offset + n_hi_batch, hi_add = p.add16i.hi_offset + n_hi_batch;

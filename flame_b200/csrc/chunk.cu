@@ -266,7 +266,7 @@ extern "C" {
 int fb_delta_inverse(const float* P, const float* beta, const float* b, int NC, int H, int C, void* T, void* Tu, void* Tw, void* A21,
                      float* T32, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if ((C != 64 && C != 128) || (T32 != nullptr && C != 64)) return -2;
+  if ((C != 64 && C != 128) || (T32 != nullptr && C != 64) || !fb::aligned(16, P)) return -2;
   delta_inverse_kernel<<<(unsigned)(NC * H * (C / 64)), 64, 0, stream>>>(P, beta, b, C, H, (__nv_bfloat16*)T, (__nv_bfloat16*)(C == 64 ? Tu : nullptr),
                                                                          (__nv_bfloat16*)Tw, (__nv_bfloat16*)A21, T32);
   return fb::launch_ok("delta_inverse_kernel");
@@ -274,7 +274,7 @@ int fb_delta_inverse(const float* P, const float* beta, const float* b, int NC, 
 
 int fb_delta_scale(const void* T, const float* beta, const float* b, int NC, int H, int C, void* Tu, void* Tw, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if (C != 64 && C != 128) return -2;
+  if ((C != 64 && C != 128) || !fb::aligned(16, T, Tu, Tw)) return -2;
   delta_scale_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)T, beta, b, C, H, (__nv_bfloat16*)Tu, (__nv_bfloat16*)Tw);
   return fb::launch_ok("delta_scale_kernel");
 }
@@ -282,7 +282,7 @@ int fb_delta_scale(const void* T, const float* beta, const float* b, int NC, int
 int fb_delta_bwd_t(const void* T, const void* dTu, const void* dTw, const float* beta, const float* b, int NC, int H, int C, float scale, void* dT,
                    float* dbeta, float* db, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if (C != 64 && C != 128) return -2;
+  if ((C != 64 && C != 128) || !fb::aligned(16, T, dTu, dTw, dT)) return -2;
   delta_bwd_t_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)T, (const __nv_bfloat16*)dTu, (const __nv_bfloat16*)dTw, beta, b,
                                                              C, H, scale, (__nv_bfloat16*)dT, dbeta, db);
   return fb::launch_ok("delta_bwd_t_kernel");
@@ -291,7 +291,7 @@ int fb_delta_bwd_t(const void* T, const void* dTu, const void* dTw, const float*
 int fb_delta_bwd_scores(const float* dA, const float* P, const void* dQ, const void* Q, const float* beta, const float* b, int NC, int H, int C,
                         float scale, void* g, void* gq, float* dbeta, float* db, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if (C != 64 && C != 128) return -2;
+  if ((C != 64 && C != 128) || !fb::aligned(16, dA, P, dQ, Q, g, gq)) return -2;
   delta_bwd_scores_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>(dA, P, (const __nv_bfloat16*)dQ, (const __nv_bfloat16*)Q, beta, b, C, H, scale,
                                                                   (__nv_bfloat16*)g, (__nv_bfloat16*)gq, dbeta, db);
   return fb::launch_ok("delta_bwd_scores_kernel");
@@ -441,14 +441,14 @@ extern "C" {
 int fb_group_prep_fwd(const void* v, const float* g, int NC, int C, int H, int dv, float scale, float* b, float* eb, float* alpha, void* vhat,
                       cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if (!group_shape_ok(C, dv)) return -2;
+  if (!group_shape_ok(C, dv) || !fb::aligned(16, v, vhat)) return -2;
   group_prep_fwd_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)v, g, C, H, dv, scale, b, eb, alpha, (__nv_bfloat16*)vhat);
   return fb::launch_ok("group_prep_fwd_kernel");
 }
 
 int fb_group_bwd1(const void* dout, const void* o1, const float* eb, int NC, int C, int H, int dv, void* dos, float* db, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if (!group_shape_ok(C, dv)) return -2;
+  if (!group_shape_ok(C, dv) || !fb::aligned(16, dout, o1, dos)) return -2;
   group_bwd1_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)dout, (const __nv_bfloat16*)o1, eb, C, H, dv, (__nv_bfloat16*)dos, db);
   return fb::launch_ok("group_bwd1_kernel");
 }
@@ -456,7 +456,7 @@ int fb_group_bwd1(const void* dout, const void* o1, const float* eb, int NC, int
 int fb_group_bwd2(const void* dvhat, const void* vhat, const void* dv1, const float* b, const float* db, const float* alpha, const float* dalpha, int NC,
                   int C, int H, int dv, void* dvo, float* dg, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if (!group_shape_ok(C, dv)) return -2;
+  if (!group_shape_ok(C, dv) || !fb::aligned(16, dvhat, vhat, dv1, dvo)) return -2;
   group_bwd2_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)dvhat, (const __nv_bfloat16*)vhat, (const __nv_bfloat16*)dv1, b, db,
                                                             alpha, dalpha, C, H, dv, (__nv_bfloat16*)dvo, dg);
   return fb::launch_ok("group_bwd2_kernel");
@@ -621,6 +621,7 @@ extern "C" {
 int fb_gla_scores(const void* q, int q32, const void* k, const float* b, const void* blk, void* A, int NC, int H, int dk, float scale,
                   cudaStream_t stream) {
   if (NC <= 0) return 0;
+  if (!fb::aligned(16, blk, A)) return -2;
   constexpr int smem = 3 * 64 * GD_LD * 4;
   static bool configured = false;
   if (!configured) {
@@ -905,7 +906,7 @@ __global__ void __launch_bounds__(256) pair_dot_kernel(const __nv_bfloat16* __re
 
 extern "C" int fb_pair_dot(const void* x, const void* y, float* out, long long B, int R, int C, int per_row, cudaStream_t stream) {
   if (B <= 0) return 0;
-  if (C & 7) return -2;
+  if ((C & 7) || !fb::aligned(16, x, y)) return -2;
   pair_dot_kernel<<<(unsigned)B, 256, 0, stream>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)y, out, R, C, per_row);
   return fb::launch_ok("pair_dot_kernel");
 }
@@ -972,7 +973,7 @@ __global__ void __launch_bounds__(256) state_scan_kernel(const long long* __rest
 extern "C" int fb_state_scan(const long long* first, const long long* last, int n_docs, const float* alpha, int per_row, const void* X,
                              int x16, void* out, int H, int rows, int cols, int reverse, cudaStream_t stream) {
   if (n_docs <= 0) return 0;
-  if (cols & 3) return -2;
+  if ((cols & 3) || !fb::aligned(x16 ? 8 : 16, X) || !fb::aligned(8, out)) return -2;
   const long long per_chunk = (long long)H * rows * cols;
   const bool wide = x16 && (cols & 7) == 0 && !(((uintptr_t)X | (uintptr_t)out) & 15);  // eight bf16 are 16 bytes
   const int v = wide ? 8 : 4;
@@ -1062,7 +1063,7 @@ extern "C" {
 int fb_gla_prep_fwd(const void* q, const void* k, const float* g, float* b, void* khat, void* qbar, void* qt, void* k3,
                     float* alpha, int NC, int H, int dk, float scale, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if (dk & 1) return -2;
+  if ((dk & 1) || !fb::aligned(4, q, k, khat, qbar, qt, k3) || !fb::aligned(8, g, b, alpha)) return -2;
   dim3 grid(NC * H, (dk + 127) / 128);
   gla_prep_fwd_kernel<<<grid, 64, 0, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, g, b, (__nv_bfloat16*)khat,
                                                 (__nv_bfloat16*)qbar, (__nv_bfloat16*)qt, (__nv_bfloat16*)k3, alpha, H, dk, scale);
@@ -1193,7 +1194,7 @@ extern "C" {
 int fb_scalar_prep_fwd(const void* q, const void* k, const float* g, float* b, void* khat, void* qbar, float* alpha, int NC,
                        int C, int H, int dk, float scale, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if (C > 128 || (dk & 7)) return -2;
+  if (C > 128 || (dk & 7) || !fb::aligned(16, q, k, khat, qbar)) return -2;
   scalar_prep_fwd_kernel<<<NC * H, 256, 0, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, g, b, (__nv_bfloat16*)khat,
                                                      (__nv_bfloat16*)qbar, alpha, C, H, dk, scale);
   return fb::launch_ok("scalar_prep_fwd_kernel");
@@ -1204,6 +1205,7 @@ int fb_scalar_prep_bwd(const void* q, const void* k, const float* b, const void*
                        cudaStream_t stream) {
   if (NC <= 0) return 0;
   if (C > 128 || (dk & 7) || ((dk >> 3) & ((dk >> 3) - 1))) return -2;  // dk / 8 must be a power of two
+  if (!fb::aligned(16, q, k, dkhat, dqbar, dq, dk_)) return -2;
   scalar_prep_bwd_kernel<<<NC * H, 256, 0, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)dkhat,
                                                      (const __nv_bfloat16*)dqbar, dalpha, db_in, (__nv_bfloat16*)dq,
                                                      (__nv_bfloat16*)dk_, dg, C, H, dk, scale);

@@ -34,6 +34,12 @@ int make_tmap_3d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t d2
 int make_tmap_4d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t d3, uint64_t d2, uint64_t d1, uint64_t d0,
                  uint64_t stride3, uint64_t stride2, uint64_t stride1, uint32_t b1, uint32_t b0, bool swizzle128);
 
+// Whether every pointer (a null one counts) stands on a boundary of `bytes`: vector loads elsewhere end the context.
+template <typename... P>
+inline bool aligned(unsigned bytes, const P*... p) {
+  return (((uintptr_t)p | ...) & (bytes - 1)) == 0;
+}
+
 inline int launch_ok(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {

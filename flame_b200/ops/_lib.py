@@ -76,6 +76,14 @@ def ptr(t: Optional[torch.Tensor]) -> int:
     return 0 if t is None else t.data_ptr()
 
 
+def dense(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """``t``, contiguous and on a 16-byte boundary: what a kernel that loads vectors may be handed.  ``contiguous()`` alone keeps
+    a whole tensor where it lies, also one with an odd storage offset."""
+    if t is None or (t.is_contiguous() and t.data_ptr() % 16 == 0):
+        return t
+    return t.clone(memory_format=torch.contiguous_format)
+
+
 def check(rc: int, what: str) -> None:
     if rc != 0:
         raise KernelError(f"{what} failed with code {rc}")

@@ -192,7 +192,7 @@ _lib.register("fb_pair_dot", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c
 
 def pair_dot(x: torch.Tensor, y: torch.Tensor, per_row: bool) -> torch.Tensor:
     """fp32 ``sum(x * y)`` over the last two dims (``per_row``: the last dim) of bf16 ``[..., R, C]`` tensors."""
-    x, y = x.contiguous(), y.contiguous()
+    x, y = _lib.dense(x), _lib.dense(y)
     R, C = x.shape[-2:]
     B = x.numel() // (R * C)
     out = torch.empty(*x.shape[:-2], *([R] if per_row else []), dtype=torch.float32, device=x.device)
@@ -209,7 +209,7 @@ _lib.register("fb_state_scan", [c_void_p, c_void_p, c_int, c_void_p, c_int, c_vo
 def state_scan(first: torch.Tensor, last: torch.Tensor, alpha: torch.Tensor, x: torch.Tensor, reverse: bool) -> torch.Tensor:
     """bf16 ``[NC, H, rows, cols]``: the state entering every chunk (reverse: the adjoint of the state leaving it) of the
     recurrence ``s = alpha_c s + x_c`` over the chunks ``first .. last`` (int64) of every document, from zero; ``x`` fp32 or bf16."""
-    x = x.contiguous()
+    x = _lib.dense(x)
     _, H, rows, cols = x.shape
     out = torch.empty(x.shape, dtype=torch.bfloat16, device=x.device)
     per_row = 1 if alpha.dim() == 3 else 0
@@ -283,7 +283,7 @@ class ScalarPrep(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, qp, kp, gp, scale):
-        qp, kp = qp.contiguous(), kp.contiguous()
+        qp, kp = _lib.dense(qp), _lib.dense(kp)
         b, khat, qbar, alpha = scalar_prep(qp, kp, None if gp is None else gp.float().contiguous(), scale)
         ctx.save_for_backward(qp, kp, b)
         ctx.scale = scale
@@ -293,8 +293,8 @@ class ScalarPrep(torch.autograd.Function):
     @staticmethod
     def backward(ctx, db, dkhat, dqbar, dalpha):
         qp, kp, b = ctx.saved_tensors
-        dkhat = None if dkhat is None else dkhat.to(torch.bfloat16).contiguous()
-        dqbar = None if dqbar is None else dqbar.to(torch.bfloat16).contiguous()
+        dkhat = None if dkhat is None else _lib.dense(dkhat.to(torch.bfloat16))
+        dqbar = None if dqbar is None else _lib.dense(dqbar.to(torch.bfloat16))
         db = None if db is None else db.float().contiguous()
         dalpha = None if dalpha is None else dalpha.float().contiguous()
         dq, dk_, dg = scalar_prep_bwd(qp, kp, b, dkhat, dqbar, dalpha, db, ctx.scale)
@@ -325,8 +325,7 @@ class SelectiveScan(torch.autograd.Function):
         u, delta, B, C = _rows(u), _rows(delta), _rows(B), _rows(C)
         ctx.z_slot = None if z is None else slots.of(z)
         z = None if z is None else _rows(z)
-        A, D = A.contiguous(), D.contiguous()
-        A = A if A.data_ptr() % 16 == 0 else A.clone()
+        A, D = _lib.dense(A), D.contiguous()
         T, Di = lay.T, u.shape[1]
         for t in (u, delta, B, C) + (() if z is None else (z,)):
             if t.shape[0] < T:

@@ -285,7 +285,7 @@ class _DecayStates(torch.autograd.Function):
         NC, G, _, dk = khat.shape
         H = u.shape[1]
         # adjoint of the state entering the NEXT chunk; zero where the next chunk belongs to another document
-        Ln = _state_scan(lay, alpha, dS.to(khat.dtype).contiguous(), khat.dtype, reverse=True)
+        Ln = _state_scan(lay, alpha, _lib.dense(dS.to(khat.dtype)), khat.dtype, reverse=True)
         dalpha = dkhat = du = None
         if ctx.needs_input_grad[0]:
             dalpha = _pair_dot(Ln, S, per_row=alpha.dim() == 3)
@@ -400,11 +400,11 @@ class _GatedDelta(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, beta, g, scale, lay):
-        q, k, v, beta = q.contiguous(), k.contiguous(), v.contiguous(), beta.contiguous()
+        q, k, v, beta = (_lib.dense(t) for t in (q, k, v, beta))
         NC, C, H, dk = q.shape
         dv = v.shape[-1]
         if g is not None:
-            b, khat, qbar, alpha = _scalar_prep_raw(q, k, g.contiguous())
+            b, khat, qbar, alpha = _scalar_prep_raw(q, k, _lib.dense(g))
             d = b.permute(0, 2, 1)
         else:
             b = d = None
@@ -436,7 +436,7 @@ class _GatedDelta(torch.autograd.Function):
         dt, dev = q.dtype, q.device
         dv = v.shape[-1]
         gated = b is not None
-        doh = _hm(do.to(dt).contiguous())
+        doh = _hm(_lib.dense(do.to(dt)))
         qh, kh, vh = _hm(q), _hm(k), _hm(v)
         khh, qbh = (_hm(khat), _hm(qbar)) if gated else (kh, qh)
         Tw = Tw if gated else Tu
@@ -482,7 +482,7 @@ class _GroupedScalarGla(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, g, scale, lay):
-        q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+        q, k, v, g = (_lib.dense(t) for t in (q, k, v, g))
         NC, C, H, dv = v.shape
         b, eb, alpha, vhat = _group_prep(v, g, scale)
         d = b.permute(0, 2, 1)
@@ -503,7 +503,7 @@ class _GroupedScalarGla(torch.autograd.Function):
         G, dk = q.shape[2:]
         dt, dev = q.dtype, q.device
         tok = lambda h, n: _token_major(NC, h, C, n, dt, dev)                             # noqa: E731
-        do = do.to(dt).contiguous()
+        do = _lib.dense(do.to(dt))
         dos, db = _group_bwd1(do, o1, eb)
         doh, dosh, qh, kh, vhh = _hm(do), _hm(dos), _hm(q), _hm(k), _hm(vhat)
         gq = _scores_bwd(bgemm(doh, _hm(v), mask=MASK_TRIL), Q, b, db).to(dt)
@@ -691,7 +691,7 @@ class _Gla(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, g, scale, lay):
         from . import chunk_kernels
-        q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+        q, k, v, g = (_lib.dense(t) for t in (q, k, v, g))
         NC, C, H, dk = q.shape
         dv = v.shape[-1]
         b, khat, qbar, qt, k3, alpha = chunk_kernels.gla_prep(q, k, g, scale)
@@ -715,7 +715,7 @@ class _Gla(torch.autograd.Function):
         NC, C, H, dk = q.shape
         dv = v.shape[-1]
         dt, dev = q.dtype, q.device
-        doh, vh = _hm(do.to(dt).contiguous()), _hm(v)
+        doh, vh = _hm(_lib.dense(do.to(dt))), _hm(v)
         tok = lambda n: _token_major(NC, H, C, n, dt, dev)                                # noqa: E731
         back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
         Ln = _state_scan(lay, alpha, bgemm(_hm(qbar), doh, a_mn=True, b_mn=True), dt, reverse=True)
@@ -794,7 +794,7 @@ class _VDecay(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, g, scale, softmax, lay):
         from . import chunk_kernels
-        q, k, v, g = q.contiguous(), k.contiguous(), v.contiguous(), g.contiguous()
+        q, k, v, g = (_lib.dense(t) for t in (q, k, v, g))
         NC, C, H, dk = q.shape
         M = v.shape[-1]
         qh, kh = _hm(q), _hm(k)
@@ -821,7 +821,7 @@ class _VDecay(torch.autograd.Function):
         dt, dev = q.dtype, q.device
         qh, kh = _hm(q), _hm(k)
         back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
-        dqv, d32 = (dout.to(dt).contiguous(), None) if softmax else (None, dout.float().contiguous())
+        dqv, d32 = (_lib.dense(dout.to(dt)), None) if softmax else (None, _lib.dense(dout.float()))
         do, do1, dacc = chunk_kernels.vdecay_bwd1(o, dqv, d32, b, scale)
         do1h, dacch = _hm(do1), _hm(dacc.view(NC * 3, 16, H, M))
         Ln = _state_scan(lay, alpha, bgemm(do1h, qh, a_mn=True, b_mn=True), dt, reverse=True)

@@ -20,13 +20,6 @@ _lib.register("fb_short_conv_fwd", [vp, vp, vp, vp, vp, i64, i32, i32, i64, i64,
 _lib.register("fb_short_conv_bwd", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i64, i64, i64, i32, i32, vp])
 
 
-def _aligned(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
-    """``t``, contiguous and on a 16-byte boundary (the kernels load it in vectors)."""
-    if t is None or (t.is_contiguous() and t.data_ptr() % 16 == 0):
-        return t
-    return t.clone(memory_format=torch.contiguous_format)
-
-
 class _ShortConvFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, meta: VarlenMeta, silu: bool):
@@ -34,8 +27,8 @@ class _ShortConvFn(torch.autograd.Function):
         W = weight.shape[-1]
         ctx.slot = slots.of(x) if W == 4 else None
         x = x if (x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0) else x.contiguous()
-        w2 = _aligned(weight.detach().reshape(D, W))
-        b2 = _aligned(bias.detach()) if bias is not None else None
+        w2 = _lib.dense(weight.detach().reshape(D, W))
+        b2 = _lib.dense(bias.detach()) if bias is not None else None
         y = torch.empty(T, D, dtype=x.dtype, device=x.device)
         pos = meta.position_ids
         rc = _lib.lib().fb_short_conv_fwd(x.data_ptr(), w2.data_ptr(), _lib.ptr(b2), pos.data_ptr(), y.data_ptr(), T, D,
@@ -52,9 +45,9 @@ class _ShortConvFn(torch.autograd.Function):
         T, D = x.shape
         W = weight.shape[-1]
         L = _lib.lib()
-        dy = _aligned(dy)
-        w2 = _aligned(weight.detach().reshape(D, W))
-        b2 = _aligned(bias.detach()) if bias is not None else None
+        dy = _lib.dense(dy)
+        w2 = _lib.dense(weight.detach().reshape(D, W))
+        b2 = _lib.dense(bias.detach()) if bias is not None else None
         dx = None if ctx.slot is None else ctx.slot.take(T, D, x.dtype, x.device)
         if dx is None or dx.stride(0) % 8 or dx.data_ptr() % 16:
             dx = torch.empty(T, D, dtype=x.dtype, device=x.device)

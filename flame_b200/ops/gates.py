@@ -62,7 +62,7 @@ class _LogSigmoidGate(torch.autograd.Function):
         x, = ctx.saved_tensors
 
         def full(d):
-            return torch.zeros(x.shape, dtype=torch.float32, device=x.device) if d is None else _aligned(d.float().contiguous())
+            return torch.zeros(x.shape, dtype=torch.float32, device=x.device) if d is None else _lib.dense(d.float())
 
         dg, ds = full(dg), full(ds) if ctx.with_slots else None
         dx = torch.empty(x.shape, dtype=x.dtype, device=x.device)
@@ -71,10 +71,6 @@ class _LogSigmoidGate(torch.autograd.Function):
         _lib.check(rc, "fb_logsigmoid_gate_bwd")
         _lib.count_launch()
         return dx, None, None
-
-
-def _aligned(x: torch.Tensor) -> torch.Tensor:
-    return x if x.data_ptr() % 16 == 0 else x.clone()
 
 
 def logsigmoid_gate(x: torch.Tensor, normalizer: float, with_slots: bool = False):
@@ -89,7 +85,7 @@ class _Hgrn2Gates(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q_raw, f_raw, lb):
         rows, D = q_raw.shape
-        q_raw, f_raw = q_raw.contiguous(), f_raw.contiguous()
+        q_raw, f_raw = _lib.dense(q_raw), _lib.dense(f_raw)
         lbf = lb.detach().float().contiguous() if lb is not None else None
         q, k = torch.empty_like(q_raw), torch.empty_like(q_raw)
         g = torch.empty(rows, D, dtype=torch.float32, device=q_raw.device)
@@ -106,9 +102,9 @@ class _Hgrn2Gates(torch.autograd.Function):
         q_raw, f_raw, lbf = ctx.saved_tensors
         rows, D = q_raw.shape
         L = _lib.lib()
-        dq = torch.zeros_like(q_raw) if dq is None else dq.contiguous()
-        dk = torch.zeros_like(q_raw) if dk is None else dk.contiguous()
-        dg = torch.zeros(rows, D, dtype=torch.float32, device=q_raw.device) if dg is None else dg.float().contiguous()
+        dq = torch.zeros_like(q_raw) if dq is None else _lib.dense(dq)
+        dk = torch.zeros_like(q_raw) if dk is None else _lib.dense(dk)
+        dg = torch.zeros(rows, D, dtype=torch.float32, device=q_raw.device) if dg is None else _lib.dense(dg.float())
         dq_raw, df_raw = torch.empty_like(q_raw), torch.empty_like(f_raw)
         part = dlb = None
         if lbf is not None:
@@ -171,8 +167,8 @@ class _Mamba2Pre(torch.autograd.Function):
         x, dt_raw, bias32, alog32, dt = ctx.saved_tensors
         H, P = ctx.dims
         T = x.shape[0]
-        dxv = torch.zeros(T, H, P, dtype=x.dtype, device=x.device) if dxv is None else dxv.contiguous()
-        dg = torch.zeros(T, H, dtype=torch.float32, device=x.device) if dg is None else dg.float().contiguous()
+        dxv = torch.zeros(T, H, P, dtype=x.dtype, device=x.device) if dxv is None else _lib.dense(dxv)
+        dg = torch.zeros(T, H, dtype=torch.float32, device=x.device) if dg is None else _lib.dense(dg.float())
         ddt = None if ddt is None else ddt.float().contiguous()
         dx = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
         d_raw = torch.empty(T, H, dtype=torch.float32, device=x.device)
@@ -190,7 +186,7 @@ class _Mamba2Post(torch.autograd.Function):
     @staticmethod
     def forward(ctx, y, x, z, D, H, P):
         T = x.shape[0]
-        y = y.contiguous()
+        y = _lib.dense(y)
         d32 = D.detach().float().contiguous()
         out = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
         rc = _lib.lib().fb_mamba2_post_fwd(y.data_ptr(), x.data_ptr(), x.stride(0), z.data_ptr(), z.stride(0), d32.data_ptr(),
@@ -206,7 +202,7 @@ class _Mamba2Post(torch.autograd.Function):
         y, x, z, d32 = ctx.saved_tensors
         H, P = ctx.dims
         T = x.shape[0]
-        dout = dout.contiguous()
+        dout = _lib.dense(dout)
         dy = torch.empty(T, H, P, dtype=x.dtype, device=x.device)
         dx = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
         dz = ctx.z_slot.take(T, H * P, x.dtype, x.device) if ctx.z_slot is not None else torch.empty(T, H * P, dtype=x.dtype, device=x.device)

@@ -440,3 +440,43 @@ def test_state_scan_widths(rows, cols, per_row, x16, reverse):
             s = a[i] * s + X[i].double()
         c += k
     assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+
+
+def _shifted(t, offset):
+    """The same values in a contiguous tensor that starts ``offset`` elements into its storage."""
+    base = torch.empty(t.numel() + offset, dtype=t.dtype, device=t.device)
+    return base[offset:].view(t.shape).copy_(t)
+
+
+@pytest.mark.parametrize("offset", [1, 2, 4])
+@pytest.mark.parametrize("name", ["gla", "gsa", "vdecay", "grouped", "gated", "plain_delta"])
+def test_contiguous_operands_at_any_storage_offset(name, offset):
+    """Whole chunks are handed on as they lie, so an operand (or the output's gradient) may be contiguous and yet start off a
+    16-byte boundary: it is moved before a kernel loads it in vectors, and the result is the aligned call's bit for bit (the
+    gated delta rule's decay gradient: up to the order of the 64 x 8 partial sums of a chunk that a shared-memory atomic adds)."""
+    from flame_b200.ops import chunked
+    from flame_b200.ops.gla import gsa
+    torch.manual_seed(offset)
+    meta, T, H = _meta([128, 64]), 192, 2
+    u = lambda *s: torch.randn(*s, device=DEV)  # noqa: E731
+    q, k, v = (u(T, 1 if name == "grouped" and i < 2 else H, 64).bfloat16() for i in range(3))
+    per_head, per_key = -torch.rand(T, H, device=DEV) * 0.1, -torch.rand(T, H, 64, device=DEV) * 0.1
+    ins, fn = {
+        "gla": ([q, k, v, per_key], lambda q, k, v, g: chunked.gla_tc(q, k, v, g, meta)),
+        "gsa": ([q, k, v, torch.rand(T, H, 64, device=DEV), per_key], lambda q, k, v, s, g: gsa(q, k, v, s, g, meta)),
+        "vdecay": ([q, k, v, per_key], lambda q, k, v, g: chunked.gla_vdecay_tc(q, k, v, g, meta, 0.5)),
+        "grouped": ([q, k, v, per_head], lambda q, k, v, g: chunked.scalar_gla_tc(q, k, v, g, meta, 0.5)),
+        "gated": ([q * 0.1, k * 0.1, v, torch.rand(T, H, device=DEV), per_head], lambda q, k, v, b, g: chunked.gated_delta_rule_tc(q, k, v, b, g, meta)),
+        "plain_delta": ([q * 0.1, k * 0.1, v, torch.rand(T, H, device=DEV)], lambda q, k, v, b: chunked.gated_delta_rule_tc(q, k, v, b, None, meta)),
+    }[name]
+    dy = u(T, H, 64)
+    res = []
+    for move in (lambda t: t, lambda t: _shifted(t, offset)):
+        args = [move(t).requires_grad_(True) for t in ins]
+        y = fn(*args)
+        res.append([y.detach(), *torch.autograd.grad(y, args, move(dy.to(y.dtype)))])
+    for i, (a, b) in enumerate(zip(*res)):
+        if name == "gated" and i == 5:
+            assert (a - b).abs().max() <= 512 * 2.0 ** -24 * a.abs().max()
+        else:
+            assert torch.equal(a, b), i
