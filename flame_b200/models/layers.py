@@ -63,7 +63,7 @@ class Attention(nn.Module):
         if self.rope_theta is not None:
             max_pos = max(int(self.max_position_embeddings or 0), _max_doc_len(meta))
             rope = rope_tables(Dh, max_pos, float(self.rope_theta), x.device)
-        o = qkv_attention(qkv, meta, H, Hkv, Dh, rope=rope, window=self.window_size or 0)
+        o = qkv_attention(qkv, meta, H, Hkv, Dh, rope=rope, window=self.window_size or 0, own=True)
         if tp is not None:
             from ..parallel.tensor_parallel import linear_reduce_scatter
             return linear_reduce_scatter(o, self.o_proj.weight)

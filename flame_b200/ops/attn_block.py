@@ -1,7 +1,7 @@
 """Fused "RoPE + varlen attention" node working directly on a fused qkv projection output.
 
-Input is the ``[T, (H + 2 Hkv) * Dh]`` output of one qkv GEMM.  RoPE is applied in place on the q and k column
-blocks, attention reads q/k/v as strided views of that same buffer, and the backward produces a single
+Input is the ``[T, (H + 2 Hkv) * Dh]`` output of one qkv GEMM.  RoPE is applied to the q and k column blocks in one pass
+(in place where the caller gives the buffer away), attention reads q/k/v as strided views, and the backward produces a single
 ``[T, (H + 2 Hkv) * Dh]`` gradient buffer (inverse RoPE applied in place) that feeds ONE weight-gradient GEMM.
 The reference does these as separate kernels on separate tensors (fla/layers/attn.py:102-176).
 """
@@ -13,22 +13,25 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib, attention as _attention, sac  # noqa: F401 - attention declares the kernels' signatures
-from .rope import rope_from_fp32_, rope_inplace_, rope_reference
+from .rope import rope_from_fp32_, rope_inplace_, rope_reference, rope_rotated
 from .varlen import VarlenMeta
 
 
 class _QkvAttnFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, qkv, meta: VarlenMeta, H, Hkv, Dh, cos, sin, scale, window):
+    def forward(ctx, qkv, meta: VarlenMeta, H, Hkv, Dh, cos, sin, scale, window, own):
         T = qkv.shape[0]
-        qkv = qkv if qkv.is_contiguous() else qkv.contiguous()
-        q = qkv[:, : H * Dh].view(T, H, Dh)
-        k = qkv[:, H * Dh: (H + Hkv) * Dh].view(T, Hkv, Dh)
-        v = qkv[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
+        whole = _lib.dense(qkv)
+        own, qkv = own or whole is not qkv, whole
+        # q and k are adjacent column blocks of the fused buffer: one launch rotates both
+        qk = qkv[:, : (H + Hkv) * Dh].view(T, H + Hkv, Dh)
         if cos is not None:
-            # q and k are adjacent column blocks of the fused buffer: one launch rotates both
-            qk = qkv[:, : (H + Hkv) * Dh].view(T, H + Hkv, Dh)
-            rope_inplace_(qk, meta.position_ids, cos, sin)
+            if own:
+                rope_inplace_(qk, meta.position_ids, cos, sin)
+            else:
+                qk = rope_rotated(qk, meta.position_ids, cos, sin)
+        q, k = qk[:, :H], qk[:, H:]
+        v = qkv[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
         L = _lib.lib()
         o = torch.empty(T, H, Dh, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(H, T, dtype=torch.float32, device=qkv.device)
@@ -38,18 +41,18 @@ class _QkvAttnFn(torch.autograd.Function):
                            _lib.stream_ptr())
         _lib.check(rc, "fb_attn_fwd")
         _lib.count_launch()
-        ctx.save_for_backward(qkv, o, lse, cos, sin)
+        ctx.save_for_backward(qkv, qk if cos is not None and not own else None, o, lse, cos, sin)
         ctx.meta, ctx.dims, ctx.scale, ctx.window = meta, (H, Hkv, Dh), scale, window
         return o.view(T, H * Dh)
 
     @staticmethod
     def backward(ctx, do):
-        qkv, o, lse, cos, sin = ctx.saved_tensors
+        qkv, qk, o, lse, cos, sin = ctx.saved_tensors
         meta = ctx.meta
         H, Hkv, Dh = ctx.dims
         T = qkv.shape[0]
-        q = qkv[:, : H * Dh].view(T, H, Dh)
-        k = qkv[:, H * Dh: (H + Hkv) * Dh].view(T, Hkv, Dh)
+        qk = qkv[:, : (H + Hkv) * Dh].view(T, H + Hkv, Dh) if qk is None else qk
+        q, k = qk[:, :H], qk[:, H:]
         v = qkv[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
         do = do.reshape(T, H, Dh)
         do = do if do.is_contiguous() else do.contiguous()
@@ -80,13 +83,14 @@ class _QkvAttnFn(torch.autograd.Function):
                 pos = meta.position_ids
                 rope_inplace_(dq, pos, cos, sin, conj=True)
                 rope_inplace_(dk, pos, cos, sin, conj=True)
-        return dqkv, None, None, None, None, None, None, None, None
+        return dqkv, None, None, None, None, None, None, None, None, None
 
 
 def qkv_attention(qkv: torch.Tensor, meta: VarlenMeta, H: int, Hkv: int, Dh: int,
                   rope: Optional[Tuple[torch.Tensor, torch.Tensor]] = None, scale: Optional[float] = None,
-                  window: int = 0) -> torch.Tensor:
-    """Returns the attention output ``[T, H * Dh]`` for a fused qkv buffer ``[T, (H + 2 Hkv) * Dh]``."""
+                  window: int = 0, own: bool = False) -> torch.Tensor:
+    """Returns the attention output ``[T, H * Dh]`` for a fused qkv buffer ``[T, (H + 2 Hkv) * Dh]``.  ``own``: nobody else reads
+    the buffer afterwards (a projection's fresh output), so that q and k may be rotated where they lie."""
     if scale is None:
         scale = 1.0 / math.sqrt(Dh)
     cos, sin = rope if rope is not None else (None, None)
@@ -109,7 +113,7 @@ def qkv_attention(qkv: torch.Tensor, meta: VarlenMeta, H: int, Hkv: int, Dh: int
     # head dim 128 under operator-level selective checkpointing goes through ``attention``, which keeps its output on the tape
     if (_lib.available() and qkv.is_cuda and qkv.dtype == torch.bfloat16
             and (Dh == 64 or (Dh == 128 and (sac.current() is None or not torch.is_grad_enabled())))):
-        return _QkvAttnFn.apply(qkv, meta, H, Hkv, Dh, cos, sin, scale, window or 0)
+        return _QkvAttnFn.apply(qkv, meta, H, Hkv, Dh, cos, sin, scale, window or 0, own)
     q = qkv[:, : H * Dh].reshape(T, H, Dh)
     k = qkv[:, H * Dh: (H + Hkv) * Dh].reshape(T, Hkv, Dh)
     v = qkv[:, (H + Hkv) * Dh:].reshape(T, Hkv, Dh)

@@ -59,6 +59,23 @@ def rope_inplace_(x: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: to
         x.copy_(rope_reference(x, pos, cos, sin, conj))
 
 
+def rope_rotated(x: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor) -> torch.Tensor:
+    """The rotation of a ``[T, H, Dh]`` view (as ``rope_inplace_``) in a tensor of its own, in one pass; no autograd."""
+    T, H, Dh = x.shape
+    rot = 2 * cos.shape[1]
+    if not (_lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and rot == Dh and rot % 16 == 0):
+        y = x.clone(memory_format=torch.contiguous_format)
+        rope_inplace_(y, pos, cos, sin)
+        return y
+    assert x.stride(2) == 1 and x.stride(1) == Dh
+    y = torch.empty(T, H, Dh, dtype=x.dtype, device=x.device)
+    rc = _lib.lib().fb_rope(x.data_ptr(), y.data_ptr(), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, H, Dh, rot,
+                            x.stride(0), y.stride(0), 0, 0, 0, _lib.stream_ptr())
+    _lib.check(rc, "fb_rope")
+    _lib.count_launch()
+    return y
+
+
 def rope_from_fp32_(src: torch.Tensor, dst: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor,
                     conj: bool = False) -> None:
     """``dst (bf16 view) = rotate(src (fp32, contiguous [T, H, Dh]))``: the dtype conversion rides on the rotation."""

@@ -301,7 +301,7 @@ def test_fused_qkv_attention_head_dim_128(H, Hkv, window):
     qkv = torch.randn(T, (H + 2 * Hkv) * Dh, device=DEV, dtype=torch.bfloat16).requires_grad_(True)
     rope = rope_tables(Dh, 512, 10000.0, torch.device(DEV))
     do = torch.randn(T, H * Dh, device=DEV, dtype=torch.bfloat16)
-    o = qkv_attention(qkv * 1.0, meta, H, Hkv, Dh, rope=rope, window=window)   # the node rotates its input in place
+    o = qkv_attention(qkv, meta, H, Hkv, Dh, rope=rope, window=window)
     (got,) = torch.autograd.grad(o, qkv, do)
     f = qkv.detach().float().requires_grad_(True)
     q, k, v = f[:, :H * Dh].view(T, H, Dh), f[:, H * Dh:(H + Hkv) * Dh].view(T, Hkv, Dh), f[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
@@ -309,6 +309,30 @@ def test_fused_qkv_attention_head_dim_128(H, Hkv, window):
     ref = attention_reference(q, k, v, meta, Dh ** -0.5, window).reshape(T, H * Dh)
     (want,) = torch.autograd.grad(ref, f, do.float())
     assert rel_err(o, ref) < 2e-2 and rel_err(got, want) < 2e-2
+
+
+@pytest.mark.parametrize("Dh", [64, 128])
+@pytest.mark.parametrize("offset", [0, 3])
+def test_fused_qkv_attention_leaves_its_input_alone(Dh, offset):
+    """Two calls on one buffer (at any storage offset) give one result and keep the buffer; giving the buffer away changes neither
+    result nor gradient: the same kernels on the same rotated values, so bit for bit (but for dq's fp32 sums: their order)."""
+    from flame_b200.ops.attn_block import qkv_attention
+    from flame_b200.ops.rope import rope_tables
+    torch.manual_seed(18)
+    meta, T, H, Hkv = _meta([200, 1, 77]), 278, 4, 2
+    n = (H + 2 * Hkv) * Dh
+    leaf = torch.empty(T * n + offset, device=DEV, dtype=torch.bfloat16).normal_()[offset:].view(T, n).requires_grad_(True)
+    before = leaf.detach().clone()
+    rope = rope_tables(Dh, 512, 10000.0, torch.device(DEV))
+    do = torch.randn(T, H * Dh, device=DEV, dtype=torch.bfloat16)
+    got = []
+    for buf, own in ((leaf, False), (leaf, False), (leaf * 1.0, True)):
+        o = qkv_attention(buf, meta, H, Hkv, Dh, rope=rope, own=own)
+        got.append((o.detach(), *torch.autograd.grad(o, leaf, do)))
+    assert torch.equal(leaf.detach(), before)
+    for o, g in got[1:]:
+        assert torch.equal(o, got[0][0])
+        assert (g - got[0][1]).abs().max() <= 2.0 ** -8 * got[0][1].abs().max()
 
 
 def test_fused_linear_cross_entropy_and_cross_entropy():
