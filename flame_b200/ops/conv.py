@@ -20,19 +20,25 @@ _lib.register("fb_short_conv_fwd", [vp, vp, vp, vp, vp, i64, i32, i32, i64, i64,
 _lib.register("fb_short_conv_bwd", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i64, i64, i64, i32, i32, vp])
 
 
+def _ld(x: torch.Tensor) -> int:
+    """The distance of the rows of a matrix.  The stride of a single row says nothing: torch takes a ``[1, D]`` block of a wider
+    matrix for contiguous and leaves it the wider stride."""
+    return x.stride(0) if x.shape[0] > 1 else x.shape[1]
+
+
 class _ShortConvFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, weight, bias, meta: VarlenMeta, silu: bool):
         T, D = x.shape
         W = weight.shape[-1]
         ctx.slot = slots.of(x) if W == 4 else None
-        x = x if (x.stride(1) == 1 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0) else x.contiguous()
+        x = x if (x.stride(1) == 1 and _ld(x) % 8 == 0 and x.data_ptr() % 16 == 0) else _lib.dense(x)
         w2 = _lib.dense(weight.detach().reshape(D, W))
         b2 = _lib.dense(bias.detach()) if bias is not None else None
         y = torch.empty(T, D, dtype=x.dtype, device=x.device)
         pos = meta.position_ids
         rc = _lib.lib().fb_short_conv_fwd(x.data_ptr(), w2.data_ptr(), _lib.ptr(b2), pos.data_ptr(), y.data_ptr(), T, D,
-                                          W, x.stride(0), y.stride(0), 1 if silu else 0, _lib.stream_ptr())
+                                          W, _ld(x), _ld(y), 1 if silu else 0, _lib.stream_ptr())
         _lib.check(rc, "fb_short_conv_fwd")
         _lib.count_launch()
         ctx.save_for_backward(x, weight, bias)
@@ -49,7 +55,7 @@ class _ShortConvFn(torch.autograd.Function):
         w2 = _lib.dense(weight.detach().reshape(D, W))
         b2 = _lib.dense(bias.detach()) if bias is not None else None
         dx = None if ctx.slot is None else ctx.slot.take(T, D, x.dtype, x.device)
-        if dx is None or dx.stride(0) % 8 or dx.data_ptr() % 16:
+        if dx is None or _ld(dx) % 8 or dx.data_ptr() % 16:
             dx = torch.empty(T, D, dtype=x.dtype, device=x.device)
         dpre = torch.empty(T, D, dtype=x.dtype, device=x.device) if W != 4 else None
         strips = int(L.fb_short_conv_strips(T))
@@ -65,7 +71,7 @@ class _ShortConvFn(torch.autograd.Function):
         xs = x if W == 4 or x.is_contiguous() else x.contiguous()
         rc = L.fb_short_conv_bwd(dy.data_ptr(), xs.data_ptr(), w2.data_ptr(), _lib.ptr(b2), ctx.meta.position_ids.data_ptr(),
                                  dx.data_ptr(), _lib.ptr(dpre), part.data_ptr(), dw.data_ptr(), _lib.ptr(db), T, D, W,
-                                 xs.stride(0), dy.stride(0), dx.stride(0), 1 if ctx.silu else 0, 1 if use_main else 0,
+                                 _ld(xs), _ld(dy), _ld(dx), 1 if ctx.silu else 0, 1 if use_main else 0,
                                  _lib.stream_ptr())
         _lib.check(rc, "fb_short_conv_bwd")
         _lib.count_launch(2 if W == 4 else 3)

@@ -248,6 +248,26 @@ def test_short_conv_width_four_edges(D, lens, silu):
         assert rel_err(a, r) < 5e-3
 
 
+@pytest.mark.parametrize("W", [1, 2, 3, 4, 5, 8])
+@pytest.mark.parametrize("cols", [(0, 64), (16, 64), (3, 52)])
+def test_short_conv_of_one_row(W, cols):
+    """One token out of a wider matrix: torch calls such a row contiguous whatever its stride.  Against fp64, 5e-3 as above."""
+    from flame_b200.ops import linear_attn as la
+    from flame_b200.ops.conv import short_conv
+    torch.manual_seed(W)
+    (c, width), D, meta = cols, 32, _meta([1])
+    wide = torch.randn(1, width, device=DEV, dtype=torch.bfloat16).requires_grad_(True)
+    w, b = (torch.randn(*n, device=DEV, dtype=torch.bfloat16).requires_grad_(True) for n in ((D, 1, W), (D,)))
+    dy = torch.randn(1, width, device=DEV, dtype=torch.bfloat16)[:, c:c + D]
+    ins = [wide, w, b]
+    y = short_conv(wide[:, c:c + D], w, b, meta, "silu")
+    out = [y] + list(torch.autograd.grad(y, ins, dy))
+    f = [t.detach().double().requires_grad_(True) for t in ins]
+    yr = la.short_conv(f[0][:, c:c + D], f[1], f[2], meta, "silu")
+    for a, r in zip(out, [yr] + list(torch.autograd.grad(yr, f, dy.double()))):
+        assert rel_err(a, r) < 5e-3
+
+
 @pytest.mark.parametrize("V", [8, 1000, 8192, 8200, 16384, 16392, 32000, 32768, 32776])
 def test_cross_entropy_row_lengths(V):
     """Vocabularies around what a CTA holds in registers (and beyond, where it walks the row); ignored rows, a row with -inf
