@@ -63,6 +63,12 @@ def reshaped(x: torch.Tensor, *shape: int) -> torch.Tensor:
     return y
 
 
+def _same_place(a: torch.Tensor, b: torch.Tensor) -> bool:
+    """Whether two ``[T, n]`` matrices are the same memory (a single row's stride says nothing)."""
+    return (a.data_ptr() == b.data_ptr() and a.dtype == b.dtype and a.shape == b.shape
+            and all(n == 1 or s == t for n, s, t in zip(a.shape, a.stride(), b.stride())))
+
+
 class _SplitColumns(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, holder, *sizes):
@@ -88,7 +94,7 @@ class _SplitColumns(torch.autograd.Function):
             dst = buf[:, c:c + n]
             if g is None:
                 dst.zero_()
-            elif not (g.data_ptr() == dst.data_ptr() and g.stride() == dst.stride() and g.dtype == dst.dtype):
+            elif not _same_place(g, dst):
                 dst.copy_(g)
             c += n
         return (buf, None, *([None] * len(ctx.sizes)))

@@ -56,6 +56,31 @@ def test_unused_block_and_partial_runs():
     torch.testing.assert_close(gx, 2 * want, rtol=1e-12, atol=1e-12)
 
 
+class _ScaleHeads(torch.autograd.Function):
+    """A consumer of ``[T, H, d]`` rows (``slots.reshaped``) that writes its gradient where it belongs."""
+
+    @staticmethod
+    def forward(ctx, x):
+        ctx.slot = slots.of(x)
+        return 2.0 * x
+
+    @staticmethod
+    def backward(ctx, dy):
+        T, H, d = dy.shape
+        return ctx.slot.take(T, H * d, dy.dtype, dy.device).view(T, H, d).copy_(2.0 * dy)
+
+
+@pytest.mark.parametrize("rows", [1, 2])
+def test_rows_of_heads(rows):
+    """A gradient that comes back through a reshape is still the block of the buffer it was written to; of one row, the reshape
+    hands back another stride."""
+    x = torch.randn(rows, 12, dtype=torch.float64, requires_grad=True)
+    a, b = split_columns(x, (8, 4))
+    y = _ScaleHeads.apply(slots.reshaped(a, rows, 2, 4)).square().sum() + _ScaleHeads.apply(slots.reshaped(b, rows, 4, 1)).sum()
+    got, = torch.autograd.grad(y, x)
+    torch.testing.assert_close(got, torch.cat([8 * x[:, :8], 0 * x[:, 8:] + 2], 1).detach(), rtol=1e-12, atol=1e-12)
+
+
 def test_another_stream_gets_its_own_matrix(monkeypatch):
     """The shared buffer is written on the stream that allocated it only; the other block's gradient is copied in."""
     holder = slots._Holder(5)
@@ -91,7 +116,7 @@ def _adjacent(layers):
     ("GatedSlotAttention", dict(num_heads=2, use_short_conv=True)),
     ("GatedSlotAttention", dict(num_heads=2, feature_map="relu")),
 ])
-@pytest.mark.parametrize("cu", [(0, 128), (0, 1, 66, 131)])
+@pytest.mark.parametrize("cu", [(0, 1), (0, 128), (0, 1, 66, 131)])
 def test_layer_with_adjacent_projections(name, kw, cu):
     """One GEMM for adjacent projections or one each: bf16 rounding of the same sums (the input's gradient is rounded once
     instead of three times), so both lie within a few bf16 steps (2^-8 of the largest entry) of one another."""
