@@ -149,12 +149,17 @@ class ChunkLayout:
         return y if self.aligned else _Unpack.apply(y, self)
 
 
+def _row_distance(x: torch.Tensor) -> int:
+    """Elements between the rows of ``x``; of one row its length, whatever stride torch keeps for it."""
+    return x.stride(0) if x.shape[0] > 1 else x.numel()
+
+
 def _rows_strided(x: torch.Tensor) -> bool:
     """Rows that are contiguous and whole 16-byte vectors, at any distance that is one too: what the gather kernel reads."""
     n = x.numel() // max(x.shape[0], 1)
     inner = list(x.stride()[1:]) == [math.prod(x.shape[i + 1:]) for i in range(1, x.dim())]
-    return (inner and n * x.element_size() % 16 == 0 and x.stride(0) * x.element_size() % 16 == 0 and x.data_ptr() % 16 == 0
-            and x.stride(0) >= n)
+    ld = _row_distance(x)
+    return inner and n * x.element_size() % 16 == 0 and ld * x.element_size() % 16 == 0 and x.data_ptr() % 16 == 0 and ld >= n
 
 
 def _gather_rows(x: torch.Tensor, idx: torch.Tensor, n_out: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -168,8 +173,8 @@ def _gather_rows(x: torch.Tensor, idx: torch.Tensor, n_out: int, out: Optional[t
         return r if out is None else out.copy_(r)
     if out is None:
         out = torch.empty(n_out, *x.shape[1:], dtype=x.dtype, device=x.device)
-    rc = _lib.lib().fb_gather_rows(x.data_ptr(), out.data_ptr(), idx.data_ptr(), n_out, row_bytes, x.stride(0) * x.element_size(),
-                                   out.stride(0) * out.element_size(), _lib.stream_ptr())
+    rc = _lib.lib().fb_gather_rows(x.data_ptr(), out.data_ptr(), idx.data_ptr(), n_out, row_bytes,
+                                   _row_distance(x) * x.element_size(), _row_distance(out) * out.element_size(), _lib.stream_ptr())
     _lib.check(rc, "fb_gather_rows")
     _lib.count_launch()
     return out

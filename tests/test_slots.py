@@ -154,14 +154,14 @@ def test_layer_with_adjacent_projections(name, kw, cu):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("cols", [(8, 0, 8), (136, 8, 64), (72, 4, 8), (64, 0, 64)])
-def test_pack_of_column_blocks(cols):
+@pytest.mark.parametrize("cols", [(8, 0, 8), (136, 8, 64), (72, 4, 8), (64, 0, 64), (20, 8, 8)])
+@pytest.mark.parametrize("cu", [(0, 3, 70, 199), (0, 1)])
+def test_pack_of_column_blocks(cols, cu):
     """Rows gathered out of a wider matrix (and gradients into one): copies, so equal bit for bit, also where the block
-    does not start on 16 bytes."""
+    does not start on 16 bytes, where the matrix' rows are not whole vectors apart, and of one row."""
     from flame_b200.ops.chunked import ChunkLayout
     from flame_b200.ops.varlen import VarlenMeta
     width, c0, n = cols
-    cu = (0, 3, 70, 199)
     dev = torch.device("cuda", 0)
     meta = VarlenMeta.from_cu_seqlens(torch.tensor(cu, dtype=torch.int32, device=dev))
     lay = ChunkLayout(meta)
