@@ -840,6 +840,23 @@ class _VDecay(torch.autograd.Function):
         return back(dq), back(dkk), dv, dg, None, None, None
 
 
+class _TwoReaders(torch.autograd.Function):
+    """``x`` in ``dtype`` for two readers; their gradients are added in fp32 (autograd would add them in ``dtype``)."""
+
+    @staticmethod
+    def forward(ctx, x, dtype):
+        ctx.dtype = x.dtype
+        y = x.to(dtype)
+        return y, y.detach()
+
+    @staticmethod
+    def backward(ctx, a, b):
+        if a is None or b is None:
+            d = b if a is None else a
+            return None if d is None else d.to(ctx.dtype), None
+        return torch.add(a.float(), b).to(ctx.dtype), None
+
+
 def gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> Optional[torch.Tensor]:
     """Both passes of gated slot attention without leaving the chunk layout between them (the slots' softmax rides on the first
     pass); None where the kernels do not apply."""
@@ -854,10 +871,11 @@ def gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> Optional[torch.
 def _gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> torch.Tensor:
     lay = ChunkLayout.of(meta)
     dt = torch.bfloat16
-    qp, kp, vp, sp = (lay.pack(t).to(dt) for t in (q, k, v, s))
+    qp, kp, vp = (lay.pack(t).to(dt) for t in (q, k, v))
     gp = lay.pack(g.float())
-    qv = _VDecay.apply(qp, kp, sp, gp, scale, True, lay)
-    return lay.unpack(_Gla.apply(qv, sp, vp, gp, 1.0, lay)).to(v.dtype)
+    written, read = _TwoReaders.apply(lay.pack(s), dt)
+    qv = _VDecay.apply(qp, kp, written, gp, scale, True, lay)
+    return lay.unpack(_Gla.apply(qv, read, vp, gp, 1.0, lay)).to(v.dtype)
 
 
 @_recomputable

@@ -353,6 +353,28 @@ def test_gsa_kernels_match_fp32_chunk_reference():
         assert rel_err(a, b) < 4e-2
 
 
+def test_gsa_slot_gradients_are_added_in_fp32():
+    """Both passes read the slots in bf16; for slots in fp32 their gradient is the fp32 sum of the passes' two bf16 gradients, so
+    most of its entries are no bf16 values, and one pass' share of it is."""
+    from flame_b200.ops.chunked import _TwoReaders
+    from flame_b200.ops.gla import gsa
+    torch.manual_seed(7)
+    meta, T = _meta([300, 77]), 377
+    q, k, v = (_bf(T, 2, 64, s=1.0) for _ in range(3))
+    s, g = torch.rand(T, 2, 32, device=DEV).requires_grad_(True), -torch.rand(T, 2, 32, device=DEV) * 0.1
+    o = gsa(q, k, v, s, g, meta)
+    ds, = torch.autograd.grad(o, s, torch.randn_like(o))
+    assert ds.dtype == torch.float32 and (ds == ds.bfloat16().float()).float().mean() < 0.9
+    x = torch.rand(1000, device=DEV).requires_grad_(True)
+    a, b = _TwoReaders.apply(x, torch.bfloat16)
+    assert torch.equal(a, x.bfloat16()) and torch.equal(b, a)
+    da, db = _bf(1000), _bf(1000, s=1e-3)
+    dx, = torch.autograd.grad([a, b], x, [da, db], retain_graph=True)
+    assert torch.equal(dx, da.float() + db.float())
+    dx, = torch.autograd.grad(b, x, db)
+    assert torch.equal(dx, db.float())
+
+
 def test_mamba2_ssd_grouped_heads_match_recurrence():
     from flame_b200.ops import linear_attn as la
     from flame_b200.ops.scan import mamba2_ssd
