@@ -177,14 +177,14 @@ __global__ void __launch_bounds__(256) delta_bwd_t_kernel(const __nv_bfloat16* _
 }
 
 // Backward of the score blocks A = diag(beta) P (strict, P = k k^T decayed) and Q = tril(q k^T decayed):
-//   g_ij  = beta_i dA_ij e^{b_i - b_j} [j < i],   gq_ij = dQ_ij e^{b_i - b_j} [j <= i]     (bf16 operands of the dq, dk products)
+//   g_ij  = beta_i dA_ij e^{b_i - b_j} [j < i],   gq_ij = q_scale dQ_ij e^{b_i - b_j} [j <= i]   (bf16 operands of the dq, dk products)
 //   dbeta_i += scale sum_j dA_ij P_ij,   db_i += scale (row sum_i - column sum_i) of beta dA P + dQ Q
 // dA, P fp32 (null: only the second block, for the scalar-gated attention without a delta rule); dQ, Q bf16 and b only with a
 // decay (without one the products' epilogues already give gq).
 __global__ void __launch_bounds__(256) delta_bwd_scores_kernel(const float* __restrict__ dA, const float* __restrict__ P,
                                                                const __nv_bfloat16* __restrict__ dQ, const __nv_bfloat16* __restrict__ Q,
                                                                const float* __restrict__ beta, const float* __restrict__ b, int C, int H, float scale,
-                                                               __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ gq,
+                                                               float q_scale, __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ gq,
                                                                float* __restrict__ dbeta, float* __restrict__ db) {
   __shared__ float sb[128], srow[128], scol[8][132];
   const long long m = blockIdx.x;
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(256) delta_bwd_scores_kernel(const float* __re
       for (int e = 0; e < 8; ++e) {
         const int j = v * 8 + e;
         const float y = j <= i ? dq[e] * qq[e] : 0.f;
-        gg[e] = j <= i ? dq[e] * __expf(bi - sb[j]) : 0.f;
+        gg[e] = j <= i ? dq[e] * __expf(bi - sb[j]) * q_scale : 0.f;
         rd += y;
         col[e] += y;
       }
@@ -289,11 +289,11 @@ int fb_delta_bwd_t(const void* T, const void* dTu, const void* dTw, const float*
 }
 
 int fb_delta_bwd_scores(const float* dA, const float* P, const void* dQ, const void* Q, const float* beta, const float* b, int NC, int H, int C,
-                        float scale, void* g, void* gq, float* dbeta, float* db, cudaStream_t stream) {
+                        float scale, float q_scale, void* g, void* gq, float* dbeta, float* db, cudaStream_t stream) {
   if (NC <= 0) return 0;
   if ((C != 64 && C != 128) || !fb::aligned(16, dA, P, dQ, Q, g, gq)) return -2;
   delta_bwd_scores_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>(dA, P, (const __nv_bfloat16*)dQ, (const __nv_bfloat16*)Q, beta, b, C, H, scale,
-                                                                  (__nv_bfloat16*)g, (__nv_bfloat16*)gq, dbeta, db);
+                                                                  q_scale, (__nv_bfloat16*)g, (__nv_bfloat16*)gq, dbeta, db);
   return fb::launch_ok("delta_bwd_scores_kernel");
 }
 

@@ -10,7 +10,7 @@ from . import _lib, slots
 _lib.register("fb_delta_inverse", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 6)
 _lib.register("fb_delta_scale", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 3)
 _lib.register("fb_delta_bwd_t", [c_void_p] * 5 + [c_int] * 3 + [c_float] + [c_void_p] * 4)
-_lib.register("fb_delta_bwd_scores", [c_void_p] * 6 + [c_int] * 3 + [c_float] + [c_void_p] * 5)
+_lib.register("fb_delta_bwd_scores", [c_void_p] * 6 + [c_int] * 3 + [c_float] * 2 + [c_void_p] * 5)
 
 
 def tri_inverse(A: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
@@ -66,7 +66,7 @@ def delta_bwd_scores(dA, P, dQ, Q, beta, b, scale: float, dbeta, db):
     g = torch.empty(P.shape, dtype=torch.bfloat16, device=P.device)
     gq = None if b is None else torch.empty_like(g)
     _lib.check(_lib.lib().fb_delta_bwd_scores(dA.data_ptr(), P.data_ptr(), 0 if b is None else dQ.data_ptr(), 0 if b is None else Q.data_ptr(),
-                                              beta.data_ptr(), _lib.ptr(b), NC, H, C, float(scale), g.data_ptr(), _lib.ptr(gq),
+                                              beta.data_ptr(), _lib.ptr(b), NC, H, C, float(scale), 1.0, g.data_ptr(), _lib.ptr(gq),
                                               dbeta.data_ptr(), _lib.ptr(db), _lib.stream_ptr()), "fb_delta_bwd_scores")
     _lib.count_launch()
     return g, gq
@@ -115,12 +115,12 @@ def group_bwd2(dvhat, vhat, dv1, b, db, alpha, dalpha):
     return dvo, dg
 
 
-def scores_bwd(dQ, Q, b, db):
-    """bf16 ``dQ_ij e^{b_i - b_j}`` (j <= i) and, added to ``db [NC, C, H]``, the gradient of ``b`` through ``Q``: the part of
+def scores_bwd(dQ, Q, b, db, scale: float):
+    """bf16 ``scale dQ_ij e^{b_i - b_j}`` (j <= i) and, added to ``db [NC, C, H]``, the gradient of ``b`` through ``Q``: the part of
     ``delta_bwd_scores`` that attention without a delta rule has."""
     NC, H, C, _ = Q.shape
     gq = torch.empty_like(Q)
-    _lib.check(_lib.lib().fb_delta_bwd_scores(0, 0, dQ.data_ptr(), Q.data_ptr(), 0, b.data_ptr(), NC, H, C, 1.0, 0, gq.data_ptr(), 0,
+    _lib.check(_lib.lib().fb_delta_bwd_scores(0, 0, dQ.data_ptr(), Q.data_ptr(), 0, b.data_ptr(), NC, H, C, 1.0, float(scale), 0, gq.data_ptr(), 0,
                                               db.data_ptr(), _lib.stream_ptr()), "fb_delta_bwd_scores")
     _lib.count_launch()
     return gq

@@ -511,9 +511,8 @@ class _GroupedScalarGla(torch.autograd.Function):
         do = _lib.dense(do.to(dt))
         dos, db = _group_bwd1(do, o1, eb)
         doh, dosh, qh, kh, vhh = _hm(do), _hm(dos), _hm(q), _hm(k), _hm(vhat)
-        gq = _scores_bwd(bgemm(doh, _hm(v), mask=MASK_TRIL), Q, b, db).to(dt)
-        if ctx.scale != 1.0:   # Q has the factor (so the gradient of b has it), its operand's gradient not yet
-            gq = gq * ctx.scale
+        # Q has the factor ``scale`` (so the gradient of b has it), its operand's gradient gets it before it is rounded
+        gq = _scores_bwd(bgemm(doh, _hm(v), mask=MASK_TRIL), Q, b, db, ctx.scale).to(dt)
         dv1 = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(H, dv))
         Ln = _state_scan(lay, alpha, bgemm(qh, dosh, a_mn=True, b_mn=True), dt, reverse=True)
         dvhat = bgemm(kh, Ln, b_mn=True, out=tok(H, dv))
@@ -559,16 +558,16 @@ def _group_bwd2(dvhat, vhat, dv1, b, db, alpha, dalpha):
     return dv.to(dv1.dtype), db.flip(1).cumsum(1).flip(1)
 
 
-def _scores_bwd(dQ, Q, b, db):
+def _scores_bwd(dQ, Q, b, db, scale):
     if _lib.available() and Q.is_cuda:
         from . import chunk_kernels
-        return chunk_kernels.scores_bwd(dQ, Q, b, db)
+        return chunk_kernels.scores_bwd(dQ, Q, b, db, scale)
     C = Q.shape[-1]
     d = b.permute(0, 2, 1)
     w = (d[..., :, None] - d[..., None, :]).masked_fill(~_mask(C, C, MASK_TRIL, Q.device), float("-inf")).exp()
     e = dQ.float() * Q.float()
     db += (e.sum(-1) - e.sum(-2)).permute(0, 2, 1)
-    return dQ * w
+    return dQ * w * scale
 
 
 def _scalar_prep_raw(q, k, g):

@@ -204,3 +204,32 @@ def test_column_split_writes_one_gradient_matrix():
     ref[:, :2] = 2
     ref[:, 6:] = 2 * x.detach()[:, 6:]
     assert torch.equal(x.grad, ref)
+
+
+@pytest.mark.parametrize("dev", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_grouped_score_gradient_is_rounded_once(dev, monkeypatch):
+    """The operand of dq and dk is ``scale dQ e^{b_i - b_j}`` rounded to bf16 once: within half a step (2^-8) of its value, plus the
+    exponential's 32-bit error (exponents up to 7: 2^-20 of it)."""
+    from flame_b200.ops import chunked
+    torch.manual_seed(0)
+    cu = torch.tensor([0, 128], dtype=torch.int32)
+    meta, scale = VarlenMeta.from_cu_seqlens(cu, 128, torch.device(dev)), 0.3
+    leaf = lambda *s: torch.randn(*s, device=dev).bfloat16().requires_grad_(True)  # noqa: E731
+    q, k, v, g = leaf(128, 1, 64), leaf(128, 1, 64), leaf(128, 4, 64), -torch.rand(128, 4, device=dev) * 0.1
+    calls = []
+
+    def spy(a, b, **kw):
+        r = bgemm(a, b, **kw)
+        calls.append((kw, r))
+        return r
+    monkeypatch.setattr(chunked, "bgemm", spy)
+    o = scalar_gla_tc(q, k, v, g, meta, scale, chunk=64)
+    calls.clear()
+    torch.autograd.grad(o, [q, k], torch.randn_like(o))
+    dQ = next(r for kw, r in calls if kw.get("mask") == MASK_TRIL).double()
+    used = [kw["more"][0][0].double() for kw, _ in calls if kw.get("sum_lo", 1) > 1]
+    b = g.view(2, 64, 4).double().cumsum(1).permute(0, 2, 1)
+    want = scale * dQ * (b[..., :, None] - b[..., None, :]).exp().tril()
+    assert len(used) == 2 and used[0].dtype == torch.float64
+    for gq in used:
+        assert ((gq - want).abs() <= (2.0 ** -8 + 2.0 ** -19) * want.abs()).all()
