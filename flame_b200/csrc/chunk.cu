@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(256) group_bwd1_kernel(const __nv_bfloat16* __
 }
 
 // dv = dv1 + dvhat e^{b_last - b}; db_i -= sum dvhat vhat, the chunk's last step gets that sum over all steps and
-// alpha dalpha; dg = reverse cumulative sum of db
+// alpha dalpha; dg = reverse cumulative sum of db.  dv1 and dvo null: dv is not wanted; dalpha and dg null: dg is not.
 __global__ void __launch_bounds__(256) group_bwd2_kernel(const __nv_bfloat16* __restrict__ dvhat, const __nv_bfloat16* __restrict__ vhat,
                                                          const __nv_bfloat16* __restrict__ dv1, const float* __restrict__ b,
                                                          const float* __restrict__ db, const float* __restrict__ alpha, const float* __restrict__ dalpha,
@@ -393,20 +393,22 @@ __global__ void __launch_bounds__(256) group_bwd2_kernel(const __nv_bfloat16* __
     float x[8], y[8], z[8], s = 0.f;
     unpack8f(*reinterpret_cast<const uint4*>(dvhat + o), x);
     unpack8f(*reinterpret_cast<const uint4*>(vhat + o), y);
-    unpack8f(*reinterpret_cast<const uint4*>(dv1 + o), z);
-    const float f = __expf(last - b[ob]);
+    if (dvo != nullptr) {
+      unpack8f(*reinterpret_cast<const uint4*>(dv1 + o), z);
+      const float f = __expf(last - b[ob]);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      s = fmaf(x[e], y[e], s);
-      z[e] = fmaf(x[e], f, z[e]);
+      for (int e = 0; e < 8; ++e) z[e] = fmaf(x[e], f, z[e]);
+      *reinterpret_cast<uint4*>(dvo + o) = pack8f(z);
     }
-    *reinterpret_cast<uint4*>(dvo + o) = pack8f(z);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s = fmaf(x[e], y[e], s);
     for (int k = nv >> 1; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
     if (vv == 0) {
       sdb[i] = db[ob] - s;
       sv[i] = s;
     }
   }
+  if (dg == nullptr) return;
   __syncthreads();
   if (threadIdx.x < 32) {  // warp 0: suffix sums, up to four steps per lane
     const int lane = threadIdx.x, per = C >> 5;

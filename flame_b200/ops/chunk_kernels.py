@@ -60,12 +60,13 @@ def delta_bwd_t(T, dTu, dTw, beta, b, scale: float):
 
 
 def delta_bwd_scores(dA, P, dQ, Q, beta, b, scale: float, dbeta, db):
-    """The bf16 operands ``g`` (of k k^T) and, with a decay, ``gq`` (of q k^T) of the dq / dk products; adds to ``dbeta`` and
-    ``db``."""
+    """The bf16 operands ``g`` (of k k^T) and, with a decay and ``dQ``, ``gq`` (of q k^T) of the dq / dk products; adds to ``dbeta``
+    and ``db``."""
     NC, H, C, _ = P.shape
     g = torch.empty(P.shape, dtype=torch.bfloat16, device=P.device)
-    gq = None if b is None else torch.empty_like(g)
-    _lib.check(_lib.lib().fb_delta_bwd_scores(dA.data_ptr(), P.data_ptr(), 0 if b is None else dQ.data_ptr(), 0 if b is None else Q.data_ptr(),
+    both = b is not None and dQ is not None
+    gq = torch.empty_like(g) if both else None
+    _lib.check(_lib.lib().fb_delta_bwd_scores(dA.data_ptr(), P.data_ptr(), dQ.data_ptr() if both else 0, Q.data_ptr() if both else 0,
                                               beta.data_ptr(), _lib.ptr(b), NC, H, C, float(scale), 1.0, g.data_ptr(), _lib.ptr(gq),
                                               dbeta.data_ptr(), _lib.ptr(db), _lib.stream_ptr()), "fb_delta_bwd_scores")
     _lib.count_launch()
@@ -106,11 +107,12 @@ def group_bwd1(do, o1, eb):
 
 
 def group_bwd2(dvhat, vhat, dv1, b, db, alpha, dalpha):
-    """``dv`` and ``dg`` (see ``csrc/chunk.cu: group_bwd2_kernel``)."""
+    """``dv`` and ``dg`` (see ``csrc/chunk.cu: group_bwd2_kernel``), each None without ``dv1`` and ``dalpha``."""
     NC, C, H, dv = vhat.shape
-    dvo, dg = torch.empty_like(vhat), torch.empty_like(b)
-    _lib.check(_lib.lib().fb_group_bwd2(dvhat.data_ptr(), vhat.data_ptr(), dv1.data_ptr(), b.data_ptr(), db.data_ptr(), alpha.data_ptr(),
-                                        dalpha.data_ptr(), NC, C, H, dv, dvo.data_ptr(), dg.data_ptr(), _lib.stream_ptr()), "fb_group_bwd2")
+    dvo = None if dv1 is None else torch.empty_like(vhat)
+    dg = None if dalpha is None else torch.empty_like(b)
+    _lib.check(_lib.lib().fb_group_bwd2(dvhat.data_ptr(), vhat.data_ptr(), _lib.ptr(dv1), b.data_ptr(), db.data_ptr(), alpha.data_ptr(),
+                                        _lib.ptr(dalpha), NC, C, H, dv, _lib.ptr(dvo), _lib.ptr(dg), _lib.stream_ptr()), "fb_group_bwd2")
     _lib.count_launch()
     return dvo, dg
 
@@ -121,7 +123,7 @@ def scores_bwd(dQ, Q, b, db, scale: float):
     NC, H, C, _ = Q.shape
     gq = torch.empty_like(Q)
     _lib.check(_lib.lib().fb_delta_bwd_scores(0, 0, dQ.data_ptr(), Q.data_ptr(), 0, b.data_ptr(), NC, H, C, 1.0, float(scale), 0, gq.data_ptr(), 0,
-                                              db.data_ptr(), _lib.stream_ptr()), "fb_delta_bwd_scores")
+                                              _lib.ptr(db), _lib.stream_ptr()), "fb_delta_bwd_scores")
     _lib.count_launch()
     return gq
 

@@ -391,6 +391,8 @@ def _delta_bwd_scores(dA, P, dQ, Q, beta, b, scale, dbeta, db):
         return dA * br, None
     d = b.permute(0, 2, 1)
     w = (d[..., :, None] - d[..., None, :]).masked_fill(~_mask(C, C, MASK_TRIL, P.device), float("-inf")).exp()
+    if dQ is None:
+        return br * dA * w, None
     e = br * dA * P + dQ * Q
     db += scale * (e.sum(-1) - e.sum(-2)).permute(0, 2, 1)
     return br * dA * w, dQ * w
@@ -441,42 +443,56 @@ class _GatedDelta(torch.autograd.Function):
         dt, dev = q.dtype, q.device
         dv = v.shape[-1]
         gated = b is not None
+        need_q, need_k, need_v, need_beta, need_g = ctx.needs_input_grad[:5]
+        need_g = need_g and gated
+        inner = need_k or need_beta or need_g              # what goes through the inverse and the chunk transitions
         doh = _hm(_lib.dense(do.to(dt)))
         qh, kh, vh = _hm(q), _hm(k), _hm(v)
         khh, qbh = (_hm(khat), _hm(qbar)) if gated else (kh, qh)
         Tw = Tw if gated else Tu
         tok = lambda n: _token_major(NC, H, C, n, dt, dev)                                # noqa: E731
-        dvn = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(dv))
-        gq = bgemm(doh, vn, mask=MASK_TRIL)                                               # dQ (without a decay also its operand)
-        Ln = _delta_adjoint(M, bgemm(qbh, doh, a_mn=True, b_mn=True, more=[(w, dvn, True, True, -1)]), alpha, lay)
-        dM = bgemm(Ln, S, alpha=-1.0)                                                     # [NC, H, dk, dk]
-        du = bgemm(khh, Ln, b_mn=True, add16=dvn, out=tok(dv))
-        dw = bgemm(khh, dM, b_mn=True, more=[(dvn, S, False, False, -1)], out=tok(dk))
-        if gated:
-            dTu, dTw = bgemm(du, vh), bgemm(dw, kh)
-        else:
-            dTu, dTw = bgemm(du, vh, more=[(dw, kh, False, False, 1)]), None
-        dvv = bgemm(Tu, du, a_mn=True, b_mn=True, alpha=scale, out=tok(dv))
-        dT, dbeta, db = _delta_bwd_t(T, dTu, dTw, beta, b, scale)
-        # T = (I + A)^-1: dA = -T^T dT T^T on the strict lower triangle
-        dA = bgemm(bgemm(T, dT, a_mn=True, b_mn=True), T, alpha=-1.0, mask=MASK_STRICT, out_dtype=torch.float32)
-        gk, gq2 = _delta_bwd_scores(dA, P, gq, Q, beta, b, scale, dbeta, db)
-        gk = gk.to(dt)
-        keys = [(gk, kh, False, True, 1), (gk, kh, True, True, 1)]
-        dg = None
-        if gated:
+        back = lambda t: None if t is None else t.permute(0, 2, 1, 3)                     # noqa: E731
+        dq = dkk = dvv = dbeta = db = dg = gk = None
+        # dQ (without a decay also the operand of its products)
+        gq = bgemm(doh, vn, mask=MASK_TRIL) if need_q or need_k or need_g else None
+        if inner or need_v:
+            dvn = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(dv))
+            Ln = _delta_adjoint(M, bgemm(qbh, doh, a_mn=True, b_mn=True, more=[(w, dvn, True, True, -1)]), alpha, lay)
+            du = bgemm(khh, Ln, b_mn=True, add16=dvn, out=tok(dv))
+            if need_v:
+                dvv = bgemm(Tu, du, a_mn=True, b_mn=True, alpha=scale, out=tok(dv))
+        if inner:
+            dM = bgemm(Ln, S, alpha=-1.0)                                                 # [NC, H, dk, dk]
+            dw = bgemm(khh, dM, b_mn=True, more=[(dvn, S, False, False, -1)], out=tok(dk))
+            if gated:
+                dTu, dTw = bgemm(du, vh), bgemm(dw, kh)
+            else:
+                dTu, dTw = bgemm(du, vh, more=[(dw, kh, False, False, 1)]), None
+            dT, dbeta, db = _delta_bwd_t(T, dTu, dTw, beta, b, scale)
+            # T = (I + A)^-1: dA = -T^T dT T^T on the strict lower triangle
+            dA = bgemm(bgemm(T, dT, a_mn=True, b_mn=True), T, alpha=-1.0, mask=MASK_STRICT, out_dtype=torch.float32)
+            gk, gq2 = _delta_bwd_scores(dA, P, gq, Q, beta, b, scale, dbeta, db)
+            gk = gk.to(dt)
+            keys = [(gk, kh, False, True, 1), (gk, kh, True, True, 1)]
+        elif gated and gq is not None:
+            gq2 = _scores_bwd(gq, Q, b, None, 1.0)
+        if gated and gq is not None:
             gq = gq2.to(dt)
-            dqbar, dkhat = bgemm(doh, S, out=tok(dk)), bgemm(u, Ln, alpha=scale, more=[(w, dM, False, False, 1)], out=tok(dk))
-            dalpha = _pair_dot(Ln, S, per_row=False) * scale
-            dq0, dk0, dg = _scalar_prep_raw_bwd(q, k, b, dkhat.permute(0, 2, 1, 3), dqbar.permute(0, 2, 1, 3), dalpha, db, scale)
-            dq = bgemm(gq, kh, b_mn=True, alpha=scale, add16=_hm(dq0), out=tok(dk))
-            dkk = bgemm(Tw, dw, a_mn=True, b_mn=True, alpha=scale, more=keys + [(gq, qh, True, True, 1)], add16=_hm(dk0), out=tok(dk))
-        else:
-            dq = bgemm(doh, S, alpha=scale, more=[(gq, kh, False, True, 1)], out=tok(dk))
-            dkk = bgemm(Tu, dw, a_mn=True, b_mn=True, alpha=scale, out=tok(dk),
-                        more=keys + [(gq, qh, True, True, 1), (u, Ln, False, False, 1), (w, dM, False, False, 1)])
-        back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
-        return back(dq), back(dkk), back(dvv), dbeta, dg, None, None
+            dqbar = bgemm(doh, S, out=tok(dk)) if need_q or need_g else None
+            dkhat = bgemm(u, Ln, alpha=scale, more=[(w, dM, False, False, 1)], out=tok(dk)) if need_k or need_g else None
+            dalpha = _pair_dot(Ln, S, per_row=False) * scale if need_g else None
+            dq0, dk0, dg = _scalar_prep_raw_bwd(q, k, b, back(dkhat), back(dqbar), dalpha, db, scale)
+            if need_q:
+                dq = bgemm(gq, kh, b_mn=True, alpha=scale, add16=_hm(dq0), out=tok(dk))
+            if need_k:
+                dkk = bgemm(Tw, dw, a_mn=True, b_mn=True, alpha=scale, more=keys + [(gq, qh, True, True, 1)], add16=_hm(dk0), out=tok(dk))
+        elif not gated:
+            if need_q:
+                dq = bgemm(doh, S, alpha=scale, more=[(gq, kh, False, True, 1)], out=tok(dk))
+            if need_k:
+                dkk = bgemm(Tu, dw, a_mn=True, b_mn=True, alpha=scale, out=tok(dk),
+                            more=keys + [(gq, qh, True, True, 1), (u, Ln, False, False, 1), (w, dM, False, False, 1)])
+        return back(dq), back(dkk), back(dvv), dbeta if need_beta else None, dg if need_g else None, None, None
 
 
 class _GroupedScalarGla(torch.autograd.Function):
@@ -509,18 +525,28 @@ class _GroupedScalarGla(torch.autograd.Function):
         dt, dev = q.dtype, q.device
         tok = lambda h, n: _token_major(NC, h, C, n, dt, dev)                             # noqa: E731
         do = _lib.dense(do.to(dt))
+        need_q, need_k, need_v, need_g = ctx.needs_input_grad[:4]
         dos, db = _group_bwd1(do, o1, eb)
         doh, dosh, qh, kh, vhh = _hm(do), _hm(dos), _hm(q), _hm(k), _hm(vhat)
-        # Q has the factor ``scale`` (so the gradient of b has it), its operand's gradient gets it before it is rounded
-        gq = _scores_bwd(bgemm(doh, _hm(v), mask=MASK_TRIL), Q, b, db, ctx.scale).to(dt)
-        dv1 = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(H, dv))
-        Ln = _state_scan(lay, alpha, bgemm(qh, dosh, a_mn=True, b_mn=True), dt, reverse=True)
-        dvhat = bgemm(kh, Ln, b_mn=True, out=tok(H, dv))
-        back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
-        dvv, dg = _group_bwd2(back(dvhat), vhat, back(dv1), b, db, alpha, _pair_dot(Ln, S, per_row=False))
+        back = lambda t: None if t is None else t.permute(0, 2, 1, 3)                     # noqa: E731
+        dq = dkk = dvv = dg = dv1 = dalpha = None
         r = H // G
-        dq = bgemm(dosh, S, more=[(gq, kh, False, True, 1)], sum_lo=r, out=tok(G, dk))
-        dkk = bgemm(vhh, Ln, more=[(gq, qh, True, True, 1)], sum_lo=r, out=tok(G, dk))
+        if need_q or need_k or need_g:
+            # Q has the factor ``scale`` (so the gradient of b has it), its operand's gradient gets it before it is rounded
+            gq = _scores_bwd(bgemm(doh, _hm(v), mask=MASK_TRIL), Q, b, db, ctx.scale).to(dt)
+        if need_k or need_v or need_g:
+            Ln = _state_scan(lay, alpha, bgemm(qh, dosh, a_mn=True, b_mn=True), dt, reverse=True)
+        if need_v or need_g:
+            dvhat = bgemm(kh, Ln, b_mn=True, out=tok(H, dv))
+            if need_v:
+                dv1 = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(H, dv))
+            if need_g:
+                dalpha = _pair_dot(Ln, S, per_row=False)
+            dvv, dg = _group_bwd2(back(dvhat), vhat, back(dv1), b, db, alpha, dalpha)
+        if need_q:
+            dq = bgemm(dosh, S, more=[(gq, kh, False, True, 1)], sum_lo=r, out=tok(G, dk))
+        if need_k:
+            dkk = bgemm(vhh, Ln, more=[(gq, qh, True, True, 1)], sum_lo=r, out=tok(G, dk))
         return back(dq), back(dkk), dvv, dg, None, None
 
 
@@ -551,11 +577,15 @@ def _group_bwd2(dvhat, vhat, dv1, b, db, alpha, dalpha):
     if _group_kernels(vhat):
         from . import chunk_kernels
         return chunk_kernels.group_bwd2(dvhat, vhat, dv1, b, db, alpha, dalpha)
-    s = (dvhat.float() * vhat.float()).sum(-1)
-    db = db - s
-    db[:, -1] += s.sum(1) + alpha * dalpha
-    dv = dv1.float() + dvhat.float() * (b[:, -1:] - b).exp()[..., None]
-    return dv.to(dv1.dtype), db.flip(1).cumsum(1).flip(1)
+    dv = dg = None
+    if dv1 is not None:
+        dv = (dv1.float() + dvhat.float() * (b[:, -1:] - b).exp()[..., None]).to(dv1.dtype)
+    if dalpha is not None:
+        s = (dvhat.float() * vhat.float()).sum(-1)
+        db = db - s
+        db[:, -1] += s.sum(1) + alpha * dalpha
+        dg = db.flip(1).cumsum(1).flip(1)
+    return dv, dg
 
 
 def _scores_bwd(dQ, Q, b, db, scale):
@@ -565,8 +595,9 @@ def _scores_bwd(dQ, Q, b, db, scale):
     C = Q.shape[-1]
     d = b.permute(0, 2, 1)
     w = (d[..., :, None] - d[..., None, :]).masked_fill(~_mask(C, C, MASK_TRIL, Q.device), float("-inf")).exp()
-    e = dQ.float() * Q.float()
-    db += (e.sum(-1) - e.sum(-2)).permute(0, 2, 1)
+    if db is not None:
+        e = dQ.float() * Q.float()
+        db += (e.sum(-1) - e.sum(-2)).permute(0, 2, 1)
     return dQ * w * scale
 
 
@@ -581,17 +612,18 @@ def _scalar_prep_raw(q, k, g):
 
 
 def _scalar_prep_raw_bwd(q, k, b, dkhat, dqbar, dalpha, db, scale):
-    """Gradients of ``_scalar_prep_raw``; ``scale`` multiplies ``dqbar`` (the other incoming gradients have it already)."""
+    """Gradients of ``_scalar_prep_raw``; ``scale`` multiplies ``dqbar`` (the other incoming gradients have it already).  An
+    incoming gradient may be None (zero)."""
     if _lib.available() and q.is_cuda:
         from . import chunk_kernels
         if chunk_kernels.scalar_prep_supported(q.shape[1], q.shape[-1]):
             return chunk_kernels.scalar_prep_bwd(q, k, b, dkhat, dqbar, dalpha, db, scale)
     last = b[:, -1:]
-    dq = dqbar.float() * (b.exp() * scale)[..., None]
-    dk = dkhat.float() * (last - b).exp()[..., None]
+    dq = torch.zeros_like(q, dtype=torch.float32) if dqbar is None else dqbar.float() * (b.exp() * scale)[..., None]
+    dk = torch.zeros_like(k, dtype=torch.float32) if dkhat is None else dkhat.float() * (last - b).exp()[..., None]
     kd = (k.float() * dk).sum(-1)
-    db = db + (q.float() * dq).sum(-1) - kd
-    db[:, -1] += kd.sum(1) + dalpha * b[:, -1].exp()
+    db = (0 if db is None else db) + (q.float() * dq).sum(-1) - kd
+    db[:, -1] += kd.sum(1) + (0 if dalpha is None else dalpha * b[:, -1].exp())
     return dq.to(q.dtype), dk.to(k.dtype), db.flip(1).cumsum(1).flip(1)
 
 
@@ -721,9 +753,13 @@ class _Gla(torch.autograd.Function):
         dt, dev = q.dtype, q.device
         doh, vh = _hm(_lib.dense(do.to(dt))), _hm(v)
         tok = lambda n: _token_major(NC, H, C, n, dt, dev)                                # noqa: E731
-        back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
+        back = lambda t: None if t is None else t.permute(0, 2, 1, 3)                     # noqa: E731
+        need_q, need_k, need_v, need_g = ctx.needs_input_grad[:4]
         Ln = _state_scan(lay, alpha, bgemm(_hm(qbar), doh, a_mn=True, b_mn=True), dt, reverse=True)
-        dvv = bgemm(_hm(khat), Ln, b_mn=True, more=[(A, doh, True, True, 1)], out=tok(dv))
+        dvv = bgemm(_hm(khat), Ln, b_mn=True, more=[(A, doh, True, True, 1)], out=tok(dv)) if need_v else None
+        if not (need_q or need_k or need_g):
+            return None, None, back(dvv), None, None, None
+        # one kernel forms the other three gradients, whichever of them are wanted
         dA = bgemm(doh, vh, mask=MASK_TRIL)
         dqbar, dkhat = bgemm(doh, S, out=tok(dk)), bgemm(vh, Ln, out=tok(dk))
         dblk = dA.view(NC, H, 4, 16, 64)[:, :, 1:, :, :48].permute(0, 2, 1, 3, 4).reshape(NC * 3, H, 16, 48)
@@ -823,20 +859,27 @@ class _VDecay(torch.autograd.Function):
         NC, C, H, dk = q.shape
         M = v.shape[-1]
         dt, dev = q.dtype, q.device
+        need_q, need_k, need_v, need_g = ctx.needs_input_grad[:4]
         qh, kh = _hm(q), _hm(k)
-        back = lambda t: t.permute(0, 2, 1, 3)                                            # noqa: E731
+        back = lambda t: None if t is None else t.permute(0, 2, 1, 3)                     # noqa: E731
+        dq = dkk = dvv = dg = None
         dqv, d32 = (_lib.dense(dout.to(dt)), None) if softmax else (None, _lib.dense(dout.float()))
         do, do1, dacc = chunk_kernels.vdecay_bwd1(o, dqv, d32, b, scale)
         do1h, dacch = _hm(do1), _hm(dacc.view(NC * 3, 16, H, M))
-        Ln = _state_scan(lay, alpha, bgemm(do1h, qh, a_mn=True, b_mn=True), dt, reverse=True)
-        dvhat = bgemm(kh, Ln, out=_token_major(NC, H, C, M, dt, dev))
-        dv3 = bgemm(P3, dacch, a_mn=True, b_mn=True, out=_token_major(NC * 3, H, 48, M, dt, dev))
-        # gradient of the scores: off-diagonal sub-blocks by GEMM, the diagonal ones are pairwise sums like GLA's own scores
-        dP = chunk_kernels.gla_scores(do, v, b, bgemm(dacch, _hm(v3)), 1.0)
-        dq = bgemm(do1h, S, b_mn=True, more=[(dP, kh, False, True, 1)], out=_token_major(NC, H, C, dk, dt, dev))
-        dkk = bgemm(_hm(vhat), Ln, b_mn=True, more=[(dP, qh, True, True, 1)], out=_token_major(NC, H, C, dk, dt, dev))
-        dv, dg = chunk_kernels.vdecay_bwd2(P, v, b, do, o, back(dvhat), back(dv3), _pair_dot(Ln, S, per_row=True), scale)
-        return back(dq), back(dkk), dv, dg, None, None, None
+        if need_k or need_v or need_g:
+            Ln = _state_scan(lay, alpha, bgemm(do1h, qh, a_mn=True, b_mn=True), dt, reverse=True)
+        if need_q or need_k:
+            # gradient of the scores: off-diagonal sub-blocks by GEMM, the diagonal ones are pairwise sums like GLA's own scores
+            dP = chunk_kernels.gla_scores(do, v, b, bgemm(dacch, _hm(v3)), 1.0)
+        if need_q:
+            dq = bgemm(do1h, S, b_mn=True, more=[(dP, kh, False, True, 1)], out=_token_major(NC, H, C, dk, dt, dev))
+        if need_k:
+            dkk = bgemm(_hm(vhat), Ln, b_mn=True, more=[(dP, qh, True, True, 1)], out=_token_major(NC, H, C, dk, dt, dev))
+        if need_v or need_g:  # one kernel forms both
+            dvhat = bgemm(kh, Ln, out=_token_major(NC, H, C, M, dt, dev))
+            dv3 = bgemm(P3, dacch, a_mn=True, b_mn=True, out=_token_major(NC * 3, H, 48, M, dt, dev))
+            dvv, dg = chunk_kernels.vdecay_bwd2(P, v, b, do, o, back(dvhat), back(dv3), _pair_dot(Ln, S, per_row=True), scale)
+        return back(dq), back(dkk), dvv, dg, None, None, None
 
 
 class _TwoReaders(torch.autograd.Function):

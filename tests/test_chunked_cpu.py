@@ -233,3 +233,56 @@ def test_grouped_score_gradient_is_rounded_once(dev, monkeypatch):
     assert len(used) == 2 and used[0].dtype == torch.float64
     for gq in used:
         assert ((gq - want).abs() <= (2.0 ** -8 + 2.0 ** -19) * want.abs()).all()
+
+
+_MOST = {"gla": "v", "gsa": "v", "vdecay": "qk"}   # what these can do without (their other gradients come from one kernel)
+
+
+@pytest.mark.parametrize("dev,name", [("cpu", n) for n in ("grouped", "gated", "plain_delta")] + [
+    pytest.param("cuda", n, marks=pytest.mark.gpu) for n in ("grouped", "gated", "plain_delta", "gla", "gsa", "vdecay")])
+def test_only_the_gradients_that_are_asked_for_are_formed(dev, name, monkeypatch):
+    """Every single gradient by itself is the one of the whole backward (the same sums; on the GPU the gated rule's decay up to
+    the order of shared-memory atomics) with fewer products and launches, and the operands that stand still get none."""
+    from flame_b200.ops import _lib, chunked
+    from flame_b200.ops.gla import gsa
+    torch.manual_seed(1)
+    lens = [128, 70, 1]
+    T, H, d = sum(lens), 2, 64
+    cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32)
+    meta = VarlenMeta.from_cu_seqlens(cu, T, torch.device(dev))
+    dt = torch.bfloat16 if dev == "cuda" else torch.float32
+    u = lambda *s: torch.randn(*s, device=dev).to(dt)  # noqa: E731
+    rate = lambda *s: -torch.rand(*s, device=dev) * 0.1  # noqa: E731
+    q, k = (u(T, 1 if name == "grouped" else H, d) * 0.2 for _ in range(2))
+    named, fn = {
+        "grouped": (dict(q=q, k=k, v=u(T, H, d), g=rate(T, H)), lambda q, k, v, g: scalar_gla_tc(q, k, v, g, meta, 0.5)),
+        "gated": (dict(q=q, k=k, v=u(T, H, d), b=torch.rand(T, H, device=dev), g=rate(T, H)),
+                  lambda q, k, v, b, g: gated_delta_rule_tc(q, k, v, b, g, meta)),
+        "plain_delta": (dict(q=q, k=k, v=u(T, H, d), b=torch.rand(T, H, device=dev)), lambda q, k, v, b: gated_delta_rule_tc(q, k, v, b, None, meta)),
+        "gla": (dict(q=q, k=k, v=u(T, H, d), g=rate(T, H, d)), lambda q, k, v, g: gla_tc(q, k, v, g, meta)),
+        "gsa": (dict(q=q, k=k, v=u(T, H, d), s=torch.rand(T, H, d, device=dev), g=rate(T, H, d)), lambda q, k, v, s, g: gsa(q, k, v, s, g, meta)),
+        "vdecay": (dict(q=q, k=k, v=u(T, H, d), g=rate(T, H, d)), lambda q, k, v, g: chunked.gla_vdecay_tc(q, k, v, g, meta, 0.5)),
+    }[name]
+    dy = u(T, H, d)
+    calls = []
+    monkeypatch.setattr(chunked, "bgemm", lambda *a, **kw: calls.append(1) or bgemm(*a, **kw))
+
+    def run(wanted):
+        args = {n: t.clone().requires_grad_(n in wanted) for n, t in named.items()}
+        y = fn(**args)
+        calls.clear()
+        before = _lib.launches()
+        grads = torch.autograd.grad(y, [args[n] for n in wanted], dy.to(y.dtype))
+        return dict(zip(wanted, grads)), (len(calls), _lib.launches() - before)
+    whole, most = run(list(named))
+    for n in named:
+        got, work = run([n])
+        if dev == "cuda" and name == "gated" and n == "g":
+            assert (got[n] - whole[n]).abs().max() <= 512 * 2.0 ** -24 * whole[n].abs().max()
+        else:
+            assert torch.equal(got[n], whole[n]), n
+        if n in _MOST.get(name, n):
+            assert work[0] < most[0] and (dev == "cpu" or work[1] < most[1]), (n, work, most)
+    still = [n for n in named if n not in "qk"]
+    got, work = run(still)
+    assert work[0] < most[0] or name in _MOST
