@@ -48,6 +48,7 @@ struct ScanArgs {
   const int* inv;          // [64 NC]: token of every chunk step, -1 = past the end
   int us, ds, zs, bs, cs;
   int Di, DiP, bc16;       // DiP: Di rounded up to 128, the row length of the state arrays
+  int kept;                // states kept per chunk: NSEG, or 1 where no backward follows
 };
 
 // two fp32 lanes per instruction
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(CT) sscan_local_kernel(ScanArgs a, float* __re
       }
     }
   }
-  float* o = st + (long long)c * NSEG * N * a.DiP + d;
+  float* o = st + (long long)c * a.kept * N * a.DiP + d;
 #pragma unroll
   for (int p = 0; p < N / 2; ++p) {
     float x, y;
@@ -253,7 +254,7 @@ __global__ void sscan_carry_kernel(const long long* __restrict__ first, const lo
 // (3)
 template <bool RAW, bool GATE>
 __global__ void __launch_bounds__(CT, 4) sscan_out_kernel(ScanArgs a, float* __restrict__ st, __nv_bfloat16* __restrict__ y,
-                                                       __nv_bfloat16* __restrict__ out, int keep) {
+                                                       __nv_bfloat16* __restrict__ out) {
   __shared__ alignas(16) float sB[L * N];
   __shared__ alignas(16) float sC[L * N];
   const int c = blockIdx.x, d = blockIdx.y * CT + threadIdx.x;
@@ -265,7 +266,8 @@ __global__ void __launch_bounds__(CT, 4) sscan_out_kernel(ScanArgs a, float* __r
   stage_bc(a, a.C, a.cs, row0, len, sC);
   f2 A2[N / 2], h[N / 2];
   load_A(a, d, live, A2);
-  float* s0 = st + (long long)c * NSEG * N * a.DiP + d;
+  const bool keep = a.kept == NSEG;
+  float* s0 = st + (long long)c * a.kept * N * a.DiP + d;
 #pragma unroll
   for (int p = 0; p < N / 2; ++p) h[p] = pk(s0[(2 * p) * a.DiP], s0[(2 * p + 1) * a.DiP]);
   const float Dd = live ? a.Dv[d] : 0.f;
@@ -683,8 +685,9 @@ __global__ void sscan_bc_reduce_kernel(const float* __restrict__ part, int nblk,
 }
 
 ScanArgs make_args(const void* u, long long us, const void* dl, long long ds, const void* z, long long zs, const void* B, long long bs,
-                   const void* C, long long cs, int bc16, const float* A, const float* Dv, const int* inv, int Di) {
+                   const void* C, long long cs, int bc16, const float* A, const float* Dv, const int* inv, int Di, int keep) {
   ScanArgs a;
+  a.kept = keep ? NSEG : 1;
   a.u = (const __nv_bfloat16*)u, a.dl = dl, a.z = (const __nv_bfloat16*)z, a.B = B, a.C = C, a.A = A, a.Dv = Dv, a.inv = inv;
   a.us = (int)us, a.ds = (int)ds, a.zs = (int)zs, a.bs = (int)bs, a.cs = (int)cs;  // 64 rows of any of them fit 32 bits
   a.Di = Di, a.DiP = (Di + CT - 1) / CT * CT, a.bc16 = bc16;
@@ -700,7 +703,7 @@ int fb_sscan_padded(int Di) { return (Di + CT - 1) / CT * CT; }
 int fb_sscan_channel_blocks(int Di) { return (Di + BC - 1) / BC; }
 
 // Forward.  raw: dl is bf16 and goes through softplus.  z: null, or the gate; then y is the ungated output (null: not wanted)
-// and out = y silu(z).  st: fp32 [NC, 4, 16, DiP]: states entering steps 0, 16, 32, 48 (the last three only with keep);
+// and out = y silu(z).  st: fp32 [NC, 4, 16, DiP], states entering steps 0, 16, 32, 48; without keep (no backward) [NC, 1, 16, DiP];
 // sdl: fp32 [NC, DiP]; y, out: bf16 [T, Di].
 int fb_sscan_fwd(const void* u, long long us, const void* dl, long long ds, int raw, const void* z, long long zs, const void* B, long long bs,
                  const void* C, long long cs, int bc16, const float* A, const float* Dv, const int* inv, const long long* first,
@@ -708,22 +711,22 @@ int fb_sscan_fwd(const void* u, long long us, const void* dl, long long ds, int 
                  cudaStream_t stream) {
   if (NC <= 0) return 0;
   if (n_state != N) return -2;
-  const ScanArgs a = make_args(u, us, dl, ds, z, zs, B, bs, C, cs, bc16, A, Dv, inv, Di);
+  const ScanArgs a = make_args(u, us, dl, ds, z, zs, B, bs, C, cs, bc16, A, Dv, inv, Di, keep);
   const dim3 grid(NC, a.DiP / CT);
   if (raw) sscan_local_kernel<true><<<grid, CT, 0, stream>>>(a, st, sdl);
   else sscan_local_kernel<false><<<grid, CT, 0, stream>>>(a, st, sdl);
   int rc = fb::launch_ok("sscan_local_kernel");
   if (rc) return rc;
-  sscan_carry_kernel<<<dim3(a.DiP * N / 256, n_docs), 256, 0, stream>>>(first, last, A, sdl, st, (long long)NSEG * N * a.DiP, Di, a.DiP, 0);
+  sscan_carry_kernel<<<dim3(a.DiP * N / 256, n_docs), 256, 0, stream>>>(first, last, A, sdl, st, (long long)a.kept * N * a.DiP, Di, a.DiP, 0);
   rc = fb::launch_ok("sscan_carry_kernel");
   if (rc) return rc;
   __nv_bfloat16 *yy = (__nv_bfloat16*)y, *oo = (__nv_bfloat16*)out;
   if (z) {
-    if (raw) sscan_out_kernel<true, true><<<grid, CT, 0, stream>>>(a, st, yy, oo, keep);
-    else sscan_out_kernel<false, true><<<grid, CT, 0, stream>>>(a, st, yy, oo, keep);
+    if (raw) sscan_out_kernel<true, true><<<grid, CT, 0, stream>>>(a, st, yy, oo);
+    else sscan_out_kernel<false, true><<<grid, CT, 0, stream>>>(a, st, yy, oo);
   } else {
-    if (raw) sscan_out_kernel<true, false><<<grid, CT, 0, stream>>>(a, st, yy, oo, keep);
-    else sscan_out_kernel<false, false><<<grid, CT, 0, stream>>>(a, st, yy, oo, keep);
+    if (raw) sscan_out_kernel<true, false><<<grid, CT, 0, stream>>>(a, st, yy, oo);
+    else sscan_out_kernel<false, false><<<grid, CT, 0, stream>>>(a, st, yy, oo);
   }
   return fb::launch_ok("sscan_out_kernel");
 }
@@ -738,7 +741,7 @@ int fb_sscan_bwd(const void* u, long long us, const void* dl, long long ds, int 
                  cudaStream_t stream) {
   if (NC <= 0) return 0;
   if (n_state != N) return -2;
-  const ScanArgs a = make_args(u, us, dl, ds, z, zs, B, bs, C, cs, bc16, A, Dv, inv, Di);
+  const ScanArgs a = make_args(u, us, dl, ds, z, zs, B, bs, C, cs, bc16, A, Dv, inv, Di, 1);
   const dim3 grid(NC, a.DiP / CT);
   const __nv_bfloat16* go = (const __nv_bfloat16*)dout;
   if (z) {

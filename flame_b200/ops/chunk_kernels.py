@@ -320,10 +320,11 @@ class SelectiveScan(torch.autograd.Function):
     """Mamba-1 selective scan on the chunk-parallel kernels of ``csrc/sscan.cu``, on packed tokens: u ``[T, Di]`` bf16, delta
     ``[T, Di]`` (fp32, or with ``raw`` the bf16 argument of a softplus), A ``[Di, 16]`` fp32, B, C ``[T, 16]`` (both bf16 or both
     fp32), D ``[Di]`` fp32; z ``[T, Di]`` bf16 or None.  Rows may have any stride.  Returns bf16 ``[T, Di]``: y, or ``y silu(z)``.
-    ``lay``: the 64-token ``ChunkLayout`` of the documents."""
+    ``lay``: the 64-token ``ChunkLayout`` of the documents; ``keep``: a backward may follow (known to the caller only, as inside
+    of ``forward`` gradients are always off)."""
 
     @staticmethod
-    def forward(ctx, u, delta, A, B, C, D, z, lay, raw):
+    def forward(ctx, u, delta, A, B, C, D, z, lay, raw, keep):
         u, delta, B, C = _rows(u), _rows(delta), _rows(B), _rows(C)
         ctx.z_slot = None if z is None else slots.of(z)
         z = None if z is None else _rows(z)
@@ -335,8 +336,7 @@ class SelectiveScan(torch.autograd.Function):
         dev = u.device
         L = _lib.lib()
         DiP = int(L.fb_sscan_padded(Di))
-        keep = any(ctx.needs_input_grad)
-        st = torch.empty(lay.NC, 4, 16, DiP, dtype=torch.float32, device=dev)
+        st = torch.empty(lay.NC, 4 if keep else 1, 16, DiP, dtype=torch.float32, device=dev)
         sdl = torch.empty(lay.NC, DiP, dtype=torch.float32, device=dev)
         y = torch.empty(T, Di, dtype=torch.bfloat16, device=dev) if keep or z is None else None
         out = torch.empty(T, Di, dtype=torch.bfloat16, device=dev) if z is not None else None
@@ -357,6 +357,7 @@ class SelectiveScan(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dout):
         u, delta, A, B, C, D, z, st, sdl, y = ctx.saved_tensors
+        assert st.shape[1] == 4, "the forward was told that no backward follows"
         lay, raw, DiP = ctx.geometry
         T, Di = lay.T, u.shape[1]
         dev = u.device
@@ -383,7 +384,7 @@ class SelectiveScan(torch.autograd.Function):
                             part.data_ptr(), dD.data_ptr(), dB.data_ptr(), dC.data_ptr(), T, lay.NC, Di, A.shape[1], _lib.stream_ptr())
         _lib.check(rc, "fb_sscan_bwd")
         _lib.count_launch(4)
-        return du, ddl, dA.sum(0)[:, :Di].t(), dB, dC, dD.sum(0)[:Di], dz, None, None
+        return du, ddl, dA.sum(0)[:, :Di].t(), dB, dC, dD.sum(0)[:Di], dz, None, None, None
 
 
 _lib.register("fb_vdecay_prep", [c_void_p] * 6 + [c_int] * 3 + [c_void_p])

@@ -16,11 +16,9 @@ def selective_scan(u, delta, A, B, C, D, meta: VarlenMeta) -> torch.Tensor:
     if sl is not None:
         return _selective_scan_state_passing(u, delta, A, B, C, D, meta, sl)
     if _kernel_ok(u, A):
-        from .chunk_kernels import SelectiveScan
-        from .chunked import ChunkLayout
         if B.dtype != C.dtype or B.dtype not in (torch.bfloat16, torch.float32):
             B, C = B.float(), C.float()
-        return SelectiveScan.apply(u, delta.float(), A.float(), B, C, D.float(), None, ChunkLayout.of(meta, 64), False)
+        return _on_kernels((u, delta.float(), A.float(), B, C, D.float(), None), meta, raw=False)
     return la.selective_scan(u, delta, A, B, C, D, meta)
 
 
@@ -29,14 +27,19 @@ def _kernel_ok(u: torch.Tensor, A: torch.Tensor) -> bool:
     return _lib.available() and u.is_cuda and A.shape[1] == 16 and u.dtype == torch.bfloat16
 
 
+def _on_kernels(operands, meta: VarlenMeta, raw: bool) -> torch.Tensor:
+    from .chunk_kernels import SelectiveScan
+    from .chunked import ChunkLayout
+    keep = torch.is_grad_enabled() and any(t is not None and t.requires_grad for t in operands)
+    return SelectiveScan.apply(*operands, ChunkLayout.of(meta, 64), raw, keep)
+
+
 def mamba_scan_gate(u, dt_raw, A, B, C, D, z, meta: VarlenMeta) -> torch.Tensor:
     """``selective_scan(u, softplus(dt_raw), A, B, C, D) * silu(z)``: with bf16 operands on the GPU the softplus and the gate
     ride on the scan's own sweeps (in fp32), which then read the projections' outputs in place."""
     if (_kernel_ok(u, A) and getattr(meta, "sequence_slice", None) is None
             and all(t.dtype == torch.bfloat16 for t in (dt_raw, B, C, z))):
-        from .chunk_kernels import SelectiveScan
-        from .chunked import ChunkLayout
-        return SelectiveScan.apply(u, dt_raw, A.float(), B, C, D.float(), z, ChunkLayout.of(meta, 64), True)
+        return _on_kernels((u, dt_raw, A.float(), B, C, D.float(), z), meta, raw=True)
     delta = torch.nn.functional.softplus(dt_raw.float())
     return selective_scan(u, delta, A, B, C, D, meta) * torch.nn.functional.silu(z)
 

@@ -338,6 +338,31 @@ def test_selective_scan_edges(Di, lens, gate):
         assert rel_err(a, b) < 1e-2
 
 
+@pytest.mark.parametrize("gate", [False, True])
+def test_selective_scan_without_a_backward_keeps_one_state_a_chunk(gate):
+    """Same output with gradients off, in the memory of the output, one fp32 state and one sum of steps per chunk (and 4 MB),
+    also where a parameter would want a gradient."""
+    from flame_b200.ops.scan import mamba_scan_gate, selective_scan
+    torch.manual_seed(3)
+    lens = [1000, 64, 2999, 33]
+    meta, T, Di = _meta(lens), sum(lens), 1100
+    u, raw, z = (_bf(T, Di) for _ in range(3))
+    B, C = _bf(T, 16), _bf(T, 16)
+    A, D = -torch.rand(Di, 16, device=DEV), torch.randn(Di, device=DEV).requires_grad_(True)
+    delta = F.softplus(raw.float())
+    fn = (lambda: mamba_scan_gate(u, raw, A, B, C, D, z, meta)) if gate else (lambda: selective_scan(u, delta, A, B, C, D, meta))
+    want = fn().detach()
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    with torch.no_grad():
+        got = fn()
+    used = torch.cuda.max_memory_allocated() - before
+    assert torch.equal(got, want)
+    chunks, padded = sum((n + 63) // 64 for n in lens), (Di + 127) // 128 * 128
+    assert used <= 2 * T * Di + 4 * chunks * padded * 17 + (4 << 20)
+
+
 def test_gsa_kernels_match_fp32_chunk_reference():
     from flame_b200.ops import linear_attn as la
     from flame_b200.ops.gla import gsa
