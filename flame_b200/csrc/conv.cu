@@ -529,10 +529,18 @@ __global__ void conv_reduce_kernel(const float* __restrict__ part, int strips, i
 
 extern "C" {
 
-// Strips of at least 64 rows, whose weight-gradient partials the reduction adds up: 65,536 tokens give 1024 strips.
-int fb_short_conv_strips(long long T) {
-  long long s = (T + BTILE - 1) / BTILE;
-  return (int)(s < 1 ? 1 : (s > 2048 ? 2048 : s));
+// Strips of rows whose weight-gradient partials the reduction adds up: of at least 64 rows, at most 2,048 of them, and for width 4
+// no more than fill the GPU once (four blocks on each of 148 SMs): 37 for 65,536 tokens and 1,024 channels.
+int fb_short_conv_strips(long long T, int D, int W) {
+  const long long tiles = (T + BTILE - 1) / BTILE;
+  long long s = tiles < 1 ? 1 : (tiles > 2048 ? 2048 : tiles);
+  if (W == CW) {
+    const int blocks_x = (D + BCH - 1) / BCH;
+    s = min(s, (long long)max(1, 4 * 148 / max(blocks_x, 1)));
+    const long long per = max(1ll, (tiles + s - 1) / s);
+    s = max(1ll, (tiles + per - 1) / per);
+  }
+  return (int)s;
 }
 
 int fb_short_conv_fwd(const void* x, const void* w, const void* b, const int* pos, void* y, long long T, int D, int W,
@@ -553,21 +561,20 @@ int fb_short_conv_fwd(const void* x, const void* w, const void* b, const int* po
 }
 
 // dx: bf16 [T, D], row stride ldd (= ldx unless W is 4); dpre: bf16 [T, D] scratch with dy's row stride, not used when W is 4;
-// part: fp32 [fb_short_conv_strips(T), D, W + 1] scratch; dw: fp32 [D, W]; db: fp32 [D] or null
+// part: fp32 [fb_short_conv_strips(T, D, W), D, W + 1] scratch; dw: fp32 [D, W]; db: fp32 [D] or null
 int fb_short_conv_bwd(const void* dy, const void* x, const void* w, const void* b, const int* pos, void* dx, void* dpre,
                       float* part, float* dw, float* db, long long T, int D, int W, long long ldx, long long ldy, long long ldd, int silu,
                       int accumulate, cudaStream_t stream) {
   if (T == 0) return 0;
   if ((D % 8) || W > MAXW || (ldx % 8) || (ldy % 8) || (ldd % 8)) return -2;
-  int strips = fb_short_conv_strips(T), rc;
+  const int strips = fb_short_conv_strips(T, D, W);
+  int rc;
   const __nv_bfloat16 *gg = (const __nv_bfloat16*)dy, *xx = (const __nv_bfloat16*)x, *ww = (const __nv_bfloat16*)w, *bb = (const __nv_bfloat16*)b;
   if (W == CW) {
     if (((uintptr_t)w & 15) || ((uintptr_t)b & 7) || ((uintptr_t)x & 7) || ((uintptr_t)dy & 7)) return -2;
-    const int tiles = (int)((T + BTILE - 1) / BTILE), blocks_x = (D + BCH - 1) / BCH;
-    strips = min(strips, max(1, 4 * 148 / blocks_x));  // four blocks on each of 148 SMs
-    const int per = (tiles + strips - 1) / strips;
-    strips = (tiles + per - 1) / per;
-    const dim3 grid(blocks_x, strips);
+    const long long tiles = (T + BTILE - 1) / BTILE;
+    const int per = (int)((tiles + strips - 1) / strips);  // the number of strips is such that none is empty
+    const dim3 grid((D + BCH - 1) / BCH, strips);
     rc = silu ? launch_conv4_bwd<true>(gg, xx, ww, bb, pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, ldd, per, grid, stream)
               : launch_conv4_bwd<false>(gg, xx, ww, bb, pos, (__nv_bfloat16*)dx, part, T, D, ldx, ldy, ldd, per, grid, stream);
   } else {

@@ -15,7 +15,7 @@ from . import _lib, linear_attn as la, slots
 from .varlen import VarlenMeta
 
 vp, i32, i64 = c_void_p, c_int, c_longlong
-_lib.register("fb_short_conv_strips", [i64])
+_lib.register("fb_short_conv_strips", [i64, i32, i32])
 _lib.register("fb_short_conv_fwd", [vp, vp, vp, vp, vp, i64, i32, i32, i64, i64, i32, vp])
 _lib.register("fb_short_conv_bwd", [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, i64, i32, i32, i64, i64, i64, i32, i32, vp])
 
@@ -58,7 +58,7 @@ class _ShortConvFn(torch.autograd.Function):
         if dx is None or _ld(dx) % 8 or dx.data_ptr() % 16:
             dx = torch.empty(T, D, dtype=x.dtype, device=x.device)
         dpre = torch.empty(T, D, dtype=x.dtype, device=x.device) if W != 4 else None
-        strips = int(L.fb_short_conv_strips(T))
+        strips = int(L.fb_short_conv_strips(T, D, W))
         part = torch.empty(strips, D, W + 1, dtype=torch.float32, device=x.device)
         mg_w = getattr(weight, "main_grad", None)
         mg_b = getattr(bias, "main_grad", None) if bias is not None else None

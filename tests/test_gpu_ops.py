@@ -670,3 +670,17 @@ def test_short_conv_strips(T, D, activation):
     assert rel_err(y, want_y) < 3e-3
     for g, r in zip(got, want):
         assert rel_err(g, r) < 5e-3
+
+
+def test_short_conv_backward_needs_no_more_partials_than_it_writes():
+    """Width 4, 40,000 tokens x 1,024 channels: beside dx the backward holds 37 strips of partial sums (and 4 MB)."""
+    from flame_b200.ops.conv import short_conv
+    T, D = 40000, 1024
+    x = torch.randn(T, D, device=DEV, dtype=torch.bfloat16).requires_grad_(True)
+    w = torch.randn(D, 1, 4, device=DEV, dtype=torch.bfloat16).requires_grad_(True)
+    y, dy = short_conv(x, w, None, _meta([T]), "silu"), torch.randn(T, D, device=DEV, dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    torch.autograd.grad(y, [x, w], dy)
+    assert torch.cuda.max_memory_allocated() - before <= 2 * T * D + 37 * D * 5 * 4 + (4 << 20)
