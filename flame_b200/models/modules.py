@@ -35,10 +35,14 @@ def fused_projection(x: torch.Tensor, layers: Sequence[Linear]) -> torch.Tensor:
 
 
 def side_by_side(layers: Sequence[Linear], x: torch.Tensor) -> bool:
-    """Whether one product may stand for these layers: plain ones (no bias, no hook, no subclass with a forward of its own),
-    trained or frozen together, their weights next to one another in memory."""
+    """Whether one product may stand for these layers: plain ones (no bias, no hook on them or on all modules, no forward of a
+    subclass' or an instance's own), trained or frozen together, their weights next to one another in memory."""
+    if torch.nn.modules.module._has_any_global_hook():
+        return False
     for l in layers:
         if type(l) is not Linear or l.bias is not None or l.weight.requires_grad != layers[0].weight.requires_grad:
+            return False
+        if "forward" in l.__dict__:
             return False
         if l._forward_hooks or l._forward_pre_hooks or l._backward_hooks or l._backward_pre_hooks:
             return False

@@ -105,6 +105,38 @@ def _adjacent(layers):
         c += w.shape[0]
 
 
+def test_layers_that_somebody_listens_to_run_by_themselves(monkeypatch):
+    """One product stands for three projections only while nobody could tell: hooks on one of them or on all modules, and a
+    forward put on an instance, are honoured."""
+    from torch.nn.modules import module as nn_module
+    from flame_b200.models import modules
+    monkeypatch.setattr(modules.linear_ops, "side_by_side", lambda x, ws: True)   # (as the engine lays them out on a GPU)
+    x = torch.randn(3, 8)
+    layers = [modules.Linear(8, n) for n in SIZES]
+    seen = []
+    note = lambda m, *a: seen.append(m)  # noqa: E731
+    assert modules.side_by_side(layers, x)
+    for register in (layers[1].register_forward_hook, layers[1].register_forward_pre_hook, layers[1].register_full_backward_hook,
+                     nn_module.register_module_forward_hook, nn_module.register_module_forward_pre_hook,
+                     nn_module.register_module_full_backward_hook, nn_module.register_module_full_backward_pre_hook):
+        handle = register(note)
+        try:
+            assert not modules.side_by_side(layers, x), register
+        finally:
+            handle.remove()
+    assert modules.side_by_side(layers, x)
+    handle = nn_module.register_module_forward_hook(note)
+    try:
+        modules.split_projections(x, layers)
+    finally:
+        handle.remove()
+    assert seen == layers
+    plain = layers[2].forward
+    layers[2].forward = lambda t: 2 * plain(t)
+    assert not modules.side_by_side(layers, x)
+    torch.testing.assert_close(modules.split_projections(x, layers)[2], 2 * plain(x))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("name,kw", [
     ("GatedLinearAttention", dict(num_heads=2)),
