@@ -10,10 +10,12 @@ A slot serves ONE consumer: two operators reading the same view would overwrite 
 them, so a slot is given away once (``of``) and later askers get none.  The buffer belongs to one run of the backward: it
 is allocated by that run's first ``take`` and handed to autograd at the end of it; a run that stopped short of it (gradients
 asked for at the views only) leaves its buffer to whoever got those gradients, and the next run makes its own.  It also belongs
-to the stream it was allocated on: a consumer on another stream gets a matrix of its own, which is copied in.
+to the stream it was allocated on: a consumer on another stream gets a matrix of its own, which is copied in.  Runs of one
+retained graph in several threads take turns at the holder, so that a run is never handed another one's buffer.
 """
 from __future__ import annotations
 
+import threading
 from typing import Optional, Tuple
 
 import torch
@@ -23,7 +25,15 @@ from . import _lib
 
 class _Holder:
     def __init__(self, width: int) -> None:
-        self.width, self.buffer, self.run, self.stream = width, None, -1, 0
+        self.width, self.buffer, self.run, self.stream, self.lock = width, None, -1, 0, threading.Lock()
+
+    def give(self, run: int) -> Optional[torch.Tensor]:
+        """The buffer of this run, which the holder lets go of; None if it has none (or another run's)."""
+        with self.lock:
+            if self.run != run:
+                return None
+            b, self.buffer = self.buffer, None
+            return b
 
 
 class Slot:
@@ -37,10 +47,11 @@ class Slot:
         if run == -1:  # not inside a backward run
             return torch.empty(rows, n, dtype=dtype, device=device)
         stream = _lib.stream_ptr() if device.type == "cuda" else 0
-        if h.buffer is None or h.run != run:
-            h.buffer, h.run, h.stream = torch.empty(rows, h.width, dtype=dtype, device=device), run, stream
-        b = h.buffer
-        if n != self.n or h.stream != stream or b.shape[0] != rows or b.dtype != dtype or b.device != device:
+        with h.lock:
+            if h.buffer is None or h.run != run:
+                h.buffer, h.run, h.stream = torch.empty(rows, h.width, dtype=dtype, device=device), run, stream
+            b, owner = h.buffer, h.stream
+        if n != self.n or owner != stream or b.shape[0] != rows or b.dtype != dtype or b.device != device:
             return torch.empty(rows, n, dtype=dtype, device=device)
         return b[:, self.col:self.col + n]
 
@@ -84,8 +95,8 @@ class _SplitColumns(torch.autograd.Function):
     def backward(ctx, *grads):
         T = next(g.shape[0] for g in grads if g is not None)
         dev = next(g.device for g in grads if g is not None)
-        buf, ctx.holder.buffer = ctx.holder.buffer, None
-        if buf is None or ctx.holder.run != torch._C._current_graph_task_id() or buf.shape[0] != T or buf.dtype != ctx.dtype or buf.device != dev:
+        buf = ctx.holder.give(torch._C._current_graph_task_id())
+        if buf is None or buf.shape[0] != T or buf.dtype != ctx.dtype or buf.device != dev:
             parts = [g.to(ctx.dtype) if g is not None else torch.zeros(T, n, dtype=ctx.dtype, device=dev)
                      for g, n in zip(grads, ctx.sizes)]
             return (torch.cat(parts, dim=1), None, *([None] * len(ctx.sizes)))

@@ -1,5 +1,6 @@
 """Gradients of column blocks written in place (``ops/slots.py``), and layers whose projections run as one GEMM."""
 import copy
+import threading
 
 import pytest
 import torch
@@ -91,6 +92,59 @@ def test_another_stream_gets_its_own_matrix(monkeypatch):
     b = second.take(4, 3, torch.float32, torch.device("cpu"))
     assert a.untyped_storage().data_ptr() == holder.buffer.untyped_storage().data_ptr()
     assert b.untyped_storage().data_ptr() != holder.buffer.untyped_storage().data_ptr()
+
+
+def test_runs_in_two_threads_never_share_a_buffer(monkeypatch):
+    """Two backward runs of one graph: the second asks for its columns just when the first has allocated the buffer."""
+    run, between, done = threading.local(), threading.Event(), threading.Event()
+
+    class Holder(slots._Holder):
+        def __setattr__(self, name, value):
+            super().__setattr__(name, value)
+            if name == "stream" and getattr(run, "id", 0) == 1 and not between.is_set():
+                between.set()
+                done.wait(0.5)   # a holder that makes runs take turns lets this time run out
+
+    monkeypatch.setattr(torch._C, "_current_graph_task_id", lambda: run.id)
+    holder, got = Holder(5), {}
+    one, two = slots.Slot(holder, 0, 2), slots.Slot(holder, 2, 3)
+
+    def first():
+        run.id = 1
+        got[1] = one.take(4, 2, torch.float32, torch.device("cpu"))
+
+    def second():
+        run.id = 2
+        between.wait(5)
+        got[2] = two.take(4, 3, torch.float32, torch.device("cpu"))
+        done.set()
+    threads = [threading.Thread(target=f) for f in (first, second)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert got[1].untyped_storage().data_ptr() != got[2].untyped_storage().data_ptr()
+
+
+def test_backward_of_one_graph_in_several_threads():
+    torch.manual_seed(0)
+    x = torch.randn(64, sum(SIZES), dtype=torch.float64, requires_grad=True)
+    a, b, c = split_columns(x, SIZES)
+    y = _Scale.apply(a, 2.0).square().sum() + _Scale.apply(b, 3.0).square().sum() + _Scale.apply(c, -1.0).square().sum()
+    want, = torch.autograd.grad(y, x, retain_graph=True)
+    wrong = []
+
+    def work(i):
+        for _ in range(50):
+            g, = torch.autograd.grad(i * y, x, retain_graph=True)
+            if not torch.equal(g, i * want):
+                wrong.append(i)
+    threads = [threading.Thread(target=work, args=(2.0 ** i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
 
 
 def _adjacent(layers):
