@@ -432,11 +432,12 @@ def vdecay_bwd1(o, dqv, d32, b, scale: float):
 
 
 def vdecay_bwd2(P, v, b, do, o, dvhat, dv3, dalpha, scale: float):
-    """``dv`` (bf16) and ``dg`` (fp32)."""
+    """``dv`` (bf16) and ``dg`` (fp32).  ``o`` and ``do`` both carry ``scale``, so one is taken out (with 0 both are zero)."""
     NC, C, H, M = v.shape
+    inv_scale = 1.0 / scale if scale else 0.0
     dv, dg = torch.empty_like(v), torch.empty_like(b)
     _lib.check(_lib.lib().fb_vdecay_bwd2(P.data_ptr(), v.data_ptr(), b.data_ptr(), do.data_ptr(), o.data_ptr(), dvhat.data_ptr(),
-                                         dv3.data_ptr(), dalpha.data_ptr(), NC, H, M, 1.0 / scale, dv.data_ptr(), dg.data_ptr(),
+                                         dv3.data_ptr(), dalpha.data_ptr(), NC, H, M, inv_scale, dv.data_ptr(), dg.data_ptr(),
                                          _lib.stream_ptr()), "fb_vdecay_bwd2")
     _lib.count_launch()
     return dv, dg

@@ -378,6 +378,23 @@ def test_gsa_kernels_match_fp32_chunk_reference():
         assert rel_err(a, b) < 4e-2
 
 
+def test_value_decay_with_scale_zero():
+    """A scale of 0 (a read-out switched off) is a number like any other: zeros and a uniform softmax, zero gradients behind them."""
+    from flame_b200.ops.chunked import gla_vdecay_tc
+    from flame_b200.ops.gla import gsa
+    torch.manual_seed(11)
+    meta, T = _meta([77, 64]), 141
+    q, k, v = (_bf(T, 2, 64).requires_grad_(True) for _ in range(3))
+    g = (-torch.rand(T, 2, 64, device=DEV)).requires_grad_(True)
+    o = gla_vdecay_tc(q, k, v, g, meta, 0.0)
+    for t in (o.detach(), *torch.autograd.grad(o, [q, k, v, g], torch.randn_like(o))):
+        assert torch.equal(t, torch.zeros_like(t))
+    s = torch.rand(T, 2, 64, device=DEV).requires_grad_(True)
+    o = gsa(q, k, v, s, g, meta, scale=0.0)
+    dq, dk, ds = torch.autograd.grad(o, [q, k, s], torch.randn_like(o))
+    assert torch.equal(dq, torch.zeros_like(dq)) and torch.equal(dk, torch.zeros_like(dk)) and bool(torch.isfinite(ds).all()) and ds.abs().max() > 0
+
+
 def test_gsa_slot_gradients_are_added_in_fp32():
     """Both passes read the slots in bf16; for slots in fp32 their gradient is the fp32 sum of the passes' two bf16 gradients, so
     most of its entries are no bf16 values, and one pass' share of it is."""
