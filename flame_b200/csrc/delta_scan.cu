@@ -3,6 +3,9 @@
 //   forward :  S_{c+1} = alpha_c S_c - M_c   S_c     + B_c      S = 0 at the first chunk of a document
 //   reverse :  L_c     = alpha_c L_{c+1} - M_c^T L_{c+1} + G_c  L = G at the last chunk of a document
 //
+// Forward writes S_c (the state entering a chunk) to chunk c; reverse writes the adjoint of the state LEAVING it, L_{c+1}, which is
+// what every gradient product takes: 0 at a document's last chunk, and L of its first chunk is not formed.
+//
 // with M_c = khat_c^T w_c  [dk, dk] (the chunk transition), B_c = khat_c^T u_c  [dk, dv], G_c = dL/dS_c, all bf16 and
 // produced by batched GEMMs.  The recurrence is sequential along the chunks of one document but independent across
 // (document, head, 128-wide slice of dv), so each CTA owns one such triple and walks its chunks with the state resident:
@@ -36,12 +39,10 @@ struct ScanParams {
   const int* first;        // [n_docs] first chunk of every document
   const int* last;         // [n_docs] last chunk
   int n_docs, H, NC, dk, dv;
-  int reverse, shift;      // shift (reverse only): chunk c of `out` receives the adjoint of the state LEAVING it, L_{c+1} (0 at
-                           // a document's last chunk), every chunk is written and L of the first chunk is not computed
+  int reverse;
   const float* alpha;      // [NC, H]
-  const __nv_bfloat16* add;  // (initial states; the steps read it through its tensor map)  forward: B [NC, H, dk, dv]; reverse: G [NC (+1), H, dk, dv]
-  __nv_bfloat16* out;      // forward: S16 [NC + 1, H, dk, dv] (chunk c + 1 receives the state after chunk c);
-                           // reverse: L16 [NC + 1, H, dk, dv] (chunk c receives L_c; L16[last] = G[last] is the caller's)
+  const __nv_bfloat16* add;  // B or G [NC, H, dk, dv] (for initial states; the steps read it through its tensor map)
+  __nv_bfloat16* out;        // [NC, H, dk, dv]
   int* status;
 };
 
@@ -72,7 +73,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant
   const int vt = blockIdx.x, head = blockIdx.y, doc = blockIdx.z;
   const int c_first = p.first[doc], c_last = p.last[doc];
   const int n_succ = c_last - c_first;    // chunks that have a successor
-  const int n_steps = p.shift ? max(n_succ - 1, 0) : n_succ;
+  const int n_steps = p.reverse ? max(n_succ - 1, 0) : n_succ;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   extern __shared__ uint8_t smem_raw[];
@@ -188,7 +189,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant
         tma_load_2d(box + h * L::BOX_BYTES, &tmAdd, my_add, (int)col0 + c_lo, (c * p.H + head) * DK + h * 128 + quarter * 32);
     };
     if (lane == 0 && n_steps > 0) fetch_add(0);
-    // initial state: forward 0; reverse G[last] (which is also what L16[last] holds)
+    // initial state: forward 0; reverse G[last]
     {
       const int c_init = c_last;
 #pragma unroll
@@ -216,7 +217,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant
         }
       }
       tmem_st_wait();
-      if (p.shift && n_succ > 0) {
+      if (p.reverse && n_succ > 0) {
 #pragma unroll
         for (int h = 0; h < HALVES; ++h) {
           const __nv_bfloat16* src = state_ptr(p.add, c_last, h * 128 + r);
@@ -224,7 +225,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant
           for (int c0 = c_lo; c0 < c_hi; c0 += 8) *reinterpret_cast<uint4*>(dst + c0) = *reinterpret_cast<const uint4*>(src + c0);
         }
       }
-      if (!p.reverse || p.shift) {  // the state entering the first chunk is zero, and so is the adjoint of the one leaving the last
+      {  // the state entering the first chunk is zero, and so is the adjoint of the one leaving the last
         __nv_bfloat16* dst0 = const_cast<__nv_bfloat16*>(state_ptr(p.out, p.reverse ? c_last : c_first, 0));
 #pragma unroll
         for (int h = 0; h < HALVES; ++h)
@@ -237,7 +238,7 @@ delta_scan_kernel(const __grid_constant__ CUtensorMap tmM, const __grid_constant
     }
     for (int s = 0; s < n_steps && ok; ++s) {
       const int c = p.reverse ? c_last - 1 - s : c_first + s;
-      const int c_out = p.reverse ? c - p.shift : c + 1;
+      const int c_out = p.reverse ? c - 1 : c + 1;
       const float a = __ldg(p.alpha + (long long)c * p.H + head);
       // the addend came in while the previous step was worked on; the state's last copy to global memory has left the operand
       if (!mbar_wait_warp(my_add, s & 1, p.status, abort_flag, ERR_WAIT_MISC)) { ok = false; break; }
@@ -319,9 +320,8 @@ int launch_scan(const CUtensorMap& tm, const CUtensorMap& tma, const CUtensorMap
 
 extern "C" {
 
-// M [NC, H, dk, dk], add [>= NC, H, dk, dv], out [NC + 1, H, dk, dv] bf16 contiguous; alpha [NC, H] fp32; first / last
-// [n_docs] chunk indices.  dk in {128, 256}, dv a multiple of 128.  reverse = 0 / 1 as described at the top of the file; 2:
-// reverse with shifted output (out [NC, ...]).
+// M [NC, H, dk, dk], add and out [NC, H, dk, dv] bf16 contiguous; alpha [NC, H] fp32; first / last [n_docs] chunk indices.
+// dk in {128, 256}, dv a multiple of 128.  reverse = 0 / 1 as described at the top of the file.
 int fb_delta_scan(const void* M, const void* add, const float* alpha, void* out, const int* first, const int* last,
                   int n_docs, int H, int NC, int dk, int dv, int reverse, cudaStream_t stream) {
   if (n_docs <= 0 || NC <= 0) return 0;
@@ -332,10 +332,10 @@ int fb_delta_scan(const void* M, const void* add, const float* alpha, void* out,
   if (((uintptr_t)add | (uintptr_t)out) & 15) return -2;
   rc = fb::make_tmap_2d(&tma, add, 2, (uint64_t)NC * H * dk, (uint64_t)dv, (uint64_t)dv, 32, 64, true);
   if (rc) return rc;
-  rc = fb::make_tmap_2d(&tmo, out, 2, (uint64_t)(NC + (reverse == 2 ? 0 : 1)) * H * dk, (uint64_t)dv, (uint64_t)dv, 32, 64, true);
+  rc = fb::make_tmap_2d(&tmo, out, 2, (uint64_t)NC * H * dk, (uint64_t)dv, (uint64_t)dv, 32, 64, true);
   if (rc) return rc;
   ScanParams p;
-  p.first = first; p.last = last; p.n_docs = n_docs; p.H = H; p.NC = NC; p.dk = dk; p.dv = dv; p.reverse = reverse != 0; p.shift = reverse == 2;
+  p.first = first; p.last = last; p.n_docs = n_docs; p.H = H; p.NC = NC; p.dk = dk; p.dv = dv; p.reverse = reverse != 0;
   p.alpha = alpha; p.add = (const __nv_bfloat16*)add; p.out = (__nv_bfloat16*)out;
   p.status = fb::status_ptr();
   return dk == 128 ? launch_scan<128>(tm, tma, tmo, p, stream) : launch_scan<256>(tm, tma, tmo, p, stream);

@@ -323,17 +323,16 @@ def _state_scan(lay: ChunkLayout, alpha, x, dtype, reverse: bool) -> torch.Tenso
 def _delta_states(M, B, alpha, lay: ChunkLayout) -> torch.Tensor:
     """``[NC, H, dk, dv]``: the state entering every chunk of ``S_{c+1} = alpha_c S_c - M_c S_c + B_c``."""
     NC, H, dk, dv = B.shape
-    S = torch.empty(NC + 1, H, dk, dv, dtype=B.dtype, device=B.device)
     if _scan_kernel_ok(M, B, alpha, dk, dv):
-        _delta_scan(M, B, alpha, S, lay, reverse=False)   # one persistent launch walks every document
-    else:
-        # shapes the scan kernel does not cover: one batched GEMM per chunk position; the running state lives in ONE fp32
-        # buffer per document, updated in place by the epilogue
-        S.index_fill_(0, lay.first, 0.0)
-        state = torch.zeros(lay.n_docs, H, dk, dv, dtype=torch.float32, device=B.device)
-        for idx, docs in zip(lay.steps, lay.step_docs):
-            bgemm(M, S, b_mn=True, a_index=idx, b_index=idx, out=state, c_index=docs, cin=state, cin_index=docs, gamma=alpha,
-                  alpha=-1.0, add16=B, add16_index=idx, out16=S, out16_index=idx, out16_offset=1, n_hi=len(idx))
+        return _delta_scan(M, B, alpha, lay, reverse=False)   # one persistent launch walks every document
+    # shapes the scan kernel does not cover: one batched GEMM per chunk position; the running state lives in ONE fp32
+    # buffer per document, updated in place by the epilogue
+    S = torch.empty(NC + 1, H, dk, dv, dtype=B.dtype, device=B.device)
+    S.index_fill_(0, lay.first, 0.0)
+    state = torch.zeros(lay.n_docs, H, dk, dv, dtype=torch.float32, device=B.device)
+    for idx, docs in zip(lay.steps, lay.step_docs):
+        bgemm(M, S, b_mn=True, a_index=idx, b_index=idx, out=state, c_index=docs, cin=state, cin_index=docs, gamma=alpha,
+              alpha=-1.0, add16=B, add16_index=idx, out16=S, out16_index=idx, out16_offset=1, n_hi=len(idx))
     return S[:NC]
 
 
@@ -342,9 +341,7 @@ def _delta_adjoint(M, dS, alpha, lay: ChunkLayout) -> torch.Tensor:
     ``dS`` of the recurrence above."""
     NC, H, dk, dv = dS.shape
     if _scan_kernel_ok(M, dS, alpha, dk, dv):
-        Ln = torch.empty_like(dS)
-        _delta_scan(M, dS, alpha, Ln, lay, reverse=2)
-        return Ln
+        return _delta_scan(M, dS, alpha, lay, reverse=True)
     L = torch.empty(NC + 1, H, dk, dv, dtype=dS.dtype, device=dS.device)
     L[:NC] = dS
     L[NC] = 0
@@ -634,17 +631,16 @@ def _scan_kernel_ok(M: torch.Tensor, add: torch.Tensor, alpha: torch.Tensor, dk:
             and dk in (128, 256) and dv % 128 == 0 and os.environ.get("FLAME_B200_DELTA_SCAN", "1") != "0")
 
 
-def _delta_scan(M: torch.Tensor, add: torch.Tensor, alpha: torch.Tensor, out16: torch.Tensor, lay: "ChunkLayout",
-                reverse: int) -> None:
-    """The chunk-state recurrence of every (document, head) in one persistent kernel (``csrc/delta_scan.cu``); reverse 2:
-    with the output shifted to the chunk that the state leaves."""
+def _delta_scan(M: torch.Tensor, add: torch.Tensor, alpha: torch.Tensor, lay: "ChunkLayout", reverse: bool) -> torch.Tensor:
+    """The chunk-state recurrence of every (document, head) in one persistent kernel (``csrc/delta_scan.cu``)."""
     NC, H, dk, _ = M.shape
     dv = add.shape[-1]
-    first, last = lay.first_i32, lay.last_i32
-    rc = _lib.lib().fb_delta_scan(M.data_ptr(), add.data_ptr(), alpha.data_ptr(), out16.data_ptr(), first.data_ptr(),
-                                  last.data_ptr(), lay.n_docs, H, NC, dk, dv, int(reverse), _lib.stream_ptr())
+    out = torch.empty_like(add)
+    rc = _lib.lib().fb_delta_scan(M.data_ptr(), add.data_ptr(), alpha.data_ptr(), out.data_ptr(), lay.first_i32.data_ptr(),
+                                  lay.last_i32.data_ptr(), lay.n_docs, H, NC, dk, dv, int(reverse), _lib.stream_ptr())
     _lib.check(rc, "fb_delta_scan")
     _lib.count_launch()
+    return out
 
 
 def _pair_dot(x: torch.Tensor, y: torch.Tensor, per_row: bool) -> torch.Tensor:
