@@ -16,17 +16,16 @@ namespace {
 //            which used to be passes of their own over T
 //   C = 128: the two diagonal blocks of T, zeros above them, and A21 = the scaled lower-left block in bf16, from which two
 //            products make T's lower-left block
-// beta, b: element (chunk, head, i) at ((chunk * C + i) * H + head); a null beta means 1.
+// beta, b: element (chunk, head, i) at ((chunk * C + i) * H + head).
 __global__ void __launch_bounds__(64) delta_inverse_kernel(const float* __restrict__ P, const float* __restrict__ beta, const float* __restrict__ b,
                                                            int C, int H, __nv_bfloat16* __restrict__ T, __nv_bfloat16* __restrict__ Tu,
-                                                           __nv_bfloat16* __restrict__ Tw, __nv_bfloat16* __restrict__ A21,
-                                                           float* __restrict__ T32) {
+                                                           __nv_bfloat16* __restrict__ Tw, __nv_bfloat16* __restrict__ A21) {
   __shared__ float sA[64 * 64];
   const int halves = C >> 6;
   const long long m = blockIdx.x / halves;
   const int half = (int)(blockIdx.x - m * halves), ch = (int)(m / H), h = (int)(m - (long long)ch * H);
   const float* a = P + m * C * C + (long long)half * 64 * (C + 1);
-  auto beta_of = [&](int i) { return beta != nullptr ? beta[((long long)ch * C + i) * H + h] : 1.f; };
+  auto beta_of = [&](int i) { return beta[((long long)ch * C + i) * H + h]; };
   for (int i = threadIdx.x; i < 4096 / 4; i += 64) {
     const int r = i >> 4;
     float4 v = *reinterpret_cast<const float4*>(a + (long long)r * C + (i & 15) * 4);
@@ -43,11 +42,6 @@ __global__ void __launch_bounds__(64) delta_inverse_kernel(const float* __restri
 #pragma unroll
     for (int j = 0; j < i; ++j) s = fmaf(-sA[i * 64 + j], x[j], s);
     x[i] = s;
-  }
-  if (T32 != nullptr) {  // C = 64, full precision, nothing else
-#pragma unroll
-    for (int i = 0; i < 64; ++i) T32[m * 4096 + i * 64 + c] = x[i];
-    return;
   }
   __nv_bfloat16* o = T + m * C * C + (long long)half * 64 * (C + 1) + c;
 #pragma unroll
@@ -264,11 +258,11 @@ __global__ void __launch_bounds__(256) delta_bwd_scores_kernel(const float* __re
 extern "C" {
 
 int fb_delta_inverse(const float* P, const float* beta, const float* b, int NC, int H, int C, void* T, void* Tu, void* Tw, void* A21,
-                     float* T32, cudaStream_t stream) {
+                     cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if ((C != 64 && C != 128) || (T32 != nullptr && C != 64) || !fb::aligned(16, P)) return -2;
+  if ((C != 64 && C != 128) || !fb::aligned(16, P)) return -2;
   delta_inverse_kernel<<<(unsigned)(NC * H * (C / 64)), 64, 0, stream>>>(P, beta, b, C, H, (__nv_bfloat16*)T, (__nv_bfloat16*)(C == 64 ? Tu : nullptr),
-                                                                         (__nv_bfloat16*)Tw, (__nv_bfloat16*)A21, T32);
+                                                                         (__nv_bfloat16*)Tw, (__nv_bfloat16*)A21);
   return fb::launch_ok("delta_inverse_kernel");
 }
 

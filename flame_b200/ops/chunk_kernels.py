@@ -7,22 +7,10 @@ import torch
 
 from . import _lib, slots
 
-_lib.register("fb_delta_inverse", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 6)
+_lib.register("fb_delta_inverse", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 5)
 _lib.register("fb_delta_scale", [c_void_p] * 3 + [c_int] * 3 + [c_void_p] * 3)
 _lib.register("fb_delta_bwd_t", [c_void_p] * 5 + [c_int] * 3 + [c_float] + [c_void_p] * 4)
 _lib.register("fb_delta_bwd_scores", [c_void_p] * 6 + [c_int] * 3 + [c_float] * 2 + [c_void_p] * 5)
-
-
-def tri_inverse(A: torch.Tensor, out_dtype: torch.dtype = torch.bfloat16) -> torch.Tensor:
-    """``(I + A)^-1`` for strictly lower-triangular fp32 ``A [..., 64, 64]``."""
-    assert A.shape[-1] == 64 and A.shape[-2] == 64 and A.dtype == torch.float32
-    A = A.contiguous()
-    out = torch.empty(A.shape, dtype=out_dtype, device=A.device)
-    n = A.numel() // 4096
-    o16, o32 = (out.data_ptr(), 0) if out_dtype == torch.bfloat16 else (0, out.data_ptr())
-    _lib.check(_lib.lib().fb_delta_inverse(A.data_ptr(), 0, 0, n, 1, 64, o16, 0, 0, 0, o32, _lib.stream_ptr()), "fb_delta_inverse")
-    _lib.count_launch()
-    return out
 
 
 def delta_inverse(P: torch.Tensor, beta: torch.Tensor, b, bgemm):
@@ -35,7 +23,7 @@ def delta_inverse(P: torch.Tensor, beta: torch.Tensor, b, bgemm):
     A21 = torch.empty(NC, H, 64, 64, dtype=torch.bfloat16, device=P.device) if C == 128 else None
     L = _lib.lib()
     _lib.check(L.fb_delta_inverse(P.data_ptr(), beta.data_ptr(), _lib.ptr(b), NC, H, C, T.data_ptr(), Tu.data_ptr(), _lib.ptr(Tw),
-                                  _lib.ptr(A21), 0, _lib.stream_ptr()), "fb_delta_inverse")
+                                  _lib.ptr(A21), _lib.stream_ptr()), "fb_delta_inverse")
     _lib.count_launch()
     if C == 128:
         X = bgemm(T[..., 64:, 64:], A21, b_mn=True)

@@ -155,13 +155,36 @@ def test_gsa_edges(M, dk, lens):
         assert rel_err(a, b) < 2e-2
 
 
-def test_tri_inverse_and_l2norm():
-    from flame_b200.ops.chunk_kernels import l2norm, tri_inverse
+@pytest.mark.parametrize("C", [64, 128])
+@pytest.mark.parametrize("gated", [False, True])
+@pytest.mark.parametrize("H", [1, 3])
+def test_delta_inverse(C, gated, H):
+    """T = (I + diag(beta) P)^-1 and T scaled by beta and by beta e^b, against the definition in fp64.  Solved in fp32 and rounded to
+    bf16 (2^-8 of an entry); at C = 128 the lower-left block comes from products of the rounded diagonal blocks and the scaled
+    copies from the rounded T: a few more roundings, 2^-7 in the norm."""
+    from flame_b200.ops import chunked
+    torch.manual_seed(C + H)
+    NC = 5
+    P = (torch.randn(NC, H, C, C, device=DEV) * 0.1).tril(-1)
+    beta = torch.rand(NC, C, H, device=DEV)
+    b = (-torch.rand(NC, C, H, device=DEV) * 0.2).cumsum(1).contiguous() if gated else None
+    got = chunked._delta_inverse(P, beta, b)
+    br = beta.double().permute(0, 2, 1)
+    eye = torch.eye(C, dtype=torch.float64, device=DEV)
+    T = torch.linalg.solve_triangular(eye + br[..., None] * P.double(), eye.expand_as(P).contiguous(), upper=False, unitriangular=True)
+    want = [T, T * br[..., None, :], T * (br * b.double().permute(0, 2, 1).exp())[..., None, :] if gated else None]
+    assert (got[2] is None) == (not gated)
+    for g, w in zip(got, want):
+        if w is not None:
+            assert g.dtype == torch.bfloat16 and not g.triu(1).any()
+            if C == 64:
+                assert ((g.double() - w).abs() <= 2.0 ** -8 * w.abs() + 1e-5).all()
+            assert (g.double() - w).norm() <= (2.0 ** -8 if C == 64 else 2.0 ** -7) * w.norm()
+
+
+def test_l2norm():
+    from flame_b200.ops.chunk_kernels import l2norm
     torch.manual_seed(2)
-    A = (torch.randn(7, 3, 64, 64, device=DEV) * 0.2).tril(-1)
-    eye = torch.eye(64, device=DEV)
-    ref = torch.linalg.solve_triangular(eye + A, eye.expand_as(A).contiguous(), upper=False, unitriangular=True)
-    assert rel_err(tri_inverse(A, torch.float32), ref) < 1e-5
     x = torch.randn(1000, 6, 256, device=DEV, dtype=torch.bfloat16, requires_grad=True)
     y = l2norm(x)
     xf = x.detach().float().requires_grad_(True)
