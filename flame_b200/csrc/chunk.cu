@@ -1080,7 +1080,7 @@ __global__ void __launch_bounds__(256) scalar_prep_fwd_kernel(const __nv_bfloat1
                                                               float* __restrict__ alpha, int C, int H, int dk, float scale) {
   __shared__ float sb[128];
   const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
-  for (int i = threadIdx.x; i < C; i += blockDim.x) sb[i] = g != nullptr ? g[((long long)c * C + i) * H + h] : 0.f;
+  for (int i = threadIdx.x; i < C; i += blockDim.x) sb[i] = g[((long long)c * C + i) * H + h];
   __syncthreads();
   if (threadIdx.x == 0) {
     float run = 0.f;

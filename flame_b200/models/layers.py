@@ -478,7 +478,6 @@ class Mamba(nn.Module):
             self.dt_proj.bias.copy_((dt + torch.log(-torch.expm1(-dt))).to(dev))
 
     def forward(self, x: torch.Tensor, meta: VarlenMeta) -> torch.Tensor:
-        from ..ops.gates import split_columns
         from ..ops.scan import mamba_scan_gate
         Di, N, R = self.intermediate_size, self.ssm_state_size, self.time_step_rank
         h, z = split_columns(self.in_proj(x), (Di, Di))
@@ -531,9 +530,9 @@ class Mamba2(nn.Module):
         from ..ops import gates
         zxbcdt = self.in_proj(x)
         # column blocks as views whose gradients are written side by side in one pass
-        z, xBC, dt = gates.split_columns(zxbcdt, (Di, self.conv_dim, zxbcdt.shape[1] - Di - self.conv_dim))
+        z, xBC, dt = split_columns(zxbcdt, (Di, self.conv_dim, zxbcdt.shape[1] - Di - self.conv_dim))
         xBC = self.conv1d(xBC, meta)
-        xs, B, C = gates.split_columns(xBC, (Di, G * N, G * N))
+        xs, B, C = split_columns(xBC, (Di, G * N, G * N))
         if not (self.rmsnorm and self.norm_before_gate):
             # everything elementwise around the SSD core in two kernels: dt = softplus(dt + bias), the log decay and
             # x dt before it; the D skip and the silu(z) gate after it

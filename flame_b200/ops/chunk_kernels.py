@@ -249,7 +249,7 @@ def scalar_prep(qp, kp, gp, scale: float):
     b = torch.empty(NC, C, H, dtype=torch.float32, device=dev)
     khat, qbar = torch.empty_like(kp), torch.empty_like(qp)
     alpha = torch.empty(NC, H, dtype=torch.float32, device=dev)
-    rc = _lib.lib().fb_scalar_prep_fwd(qp.data_ptr(), kp.data_ptr(), _lib.ptr(gp), b.data_ptr(), khat.data_ptr(),
+    rc = _lib.lib().fb_scalar_prep_fwd(qp.data_ptr(), kp.data_ptr(), gp.data_ptr(), b.data_ptr(), khat.data_ptr(),
                                        qbar.data_ptr(), alpha.data_ptr(), NC, C, H, dk, float(scale), _lib.stream_ptr())
     _lib.check(rc, "fb_scalar_prep_fwd")
     _lib.count_launch()
@@ -274,10 +274,9 @@ class ScalarPrep(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qp, kp, gp, scale):
         qp, kp = _lib.dense(qp), _lib.dense(kp)
-        b, khat, qbar, alpha = scalar_prep(qp, kp, None if gp is None else gp.float().contiguous(), scale)
+        b, khat, qbar, alpha = scalar_prep(qp, kp, gp.float().contiguous(), scale)
         ctx.save_for_backward(qp, kp, b)
         ctx.scale = scale
-        ctx.has_g = gp is not None
         return b, khat, qbar, alpha
 
     @staticmethod
@@ -288,7 +287,7 @@ class ScalarPrep(torch.autograd.Function):
         db = None if db is None else db.float().contiguous()
         dalpha = None if dalpha is None else dalpha.float().contiguous()
         dq, dk_, dg = scalar_prep_bwd(qp, kp, b, dkhat, dqbar, dalpha, db, ctx.scale)
-        return dq, dk_, (dg if ctx.has_g else None), None
+        return dq, dk_, dg, None
 
 
 _vp, _i, _ll = c_void_p, c_int, c_longlong

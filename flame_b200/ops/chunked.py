@@ -225,8 +225,8 @@ class _Scores(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, a, b, d, alpha, mask, out_dtype):
-        # a, b: [NC, G, C, dk] views (G heads, G divides H); d: [NC, H, C] fp32: one score block per head from shared q / k
-        out = bgemm(a, b, alpha=alpha, mask=mask, decay=d, out_dtype=out_dtype, n_lo=d.shape[1])
+        # a, b: [NC, H, C, dk] views; d: [NC, H, C] fp32
+        out = bgemm(a, b, alpha=alpha, mask=mask, decay=d, out_dtype=out_dtype)
         ctx.save_for_backward(a, b, d, out)
         ctx.cfg = (alpha, mask)
         return out
@@ -249,10 +249,6 @@ class _Scores(torch.autograd.Function):
             m = _mask(out.shape[-2], out.shape[-1], mask, dc.device)
             w = (d[..., :, None] - d[..., None, :]).masked_fill(~m, float("-inf")).exp()
             g = dcf * w
-        NC, H = g.shape[:2]
-        G = a.shape[1]
-        if G < H:  # shared q / k: the heads of a group add up on the (small) score gradient before the GEMMs
-            g = g.reshape(NC, G, H // G, *g.shape[2:]).float().sum(2)
         g = g.to(a.dtype)
         da = db = None
         if ctx.needs_input_grad[0]:
@@ -276,7 +272,7 @@ class _DecayStates(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, alpha, khat, u, lay: ChunkLayout):
-        # alpha fp32; khat [NC, G, C, dk]; u [NC, H, C, dv] (operand views); keys may be shared by groups of heads
+        # alpha fp32; khat [NC, H, C, dk]; u [NC, H, C, dv] (operand views)
         alpha = alpha.contiguous()
         S = _state_scan(lay, alpha, bgemm(khat, u, a_mn=True, b_mn=True, out_dtype=torch.float32), khat.dtype, reverse=False)
         ctx.save_for_backward(alpha, khat, u, S)
@@ -287,8 +283,7 @@ class _DecayStates(torch.autograd.Function):
     def backward(ctx, dS):
         alpha, khat, u, S = ctx.saved_tensors
         lay = ctx.lay
-        NC, G, _, dk = khat.shape
-        H = u.shape[1]
+        NC, H, _, dk = khat.shape
         # adjoint of the state entering the NEXT chunk; zero where the next chunk belongs to another document
         Ln = _state_scan(lay, alpha, _lib.dense(dS.to(khat.dtype)), khat.dtype, reverse=True)
         dalpha = dkhat = du = None
@@ -298,11 +293,7 @@ class _DecayStates(torch.autograd.Function):
             du = _like(u)
             bgemm(khat, Ln, b_mn=True, out=du)
         if ctx.needs_input_grad[1]:
-            if G < H:  # keys shared by the heads of a group
-                dkh = bgemm(u, Ln, out_dtype=torch.float32, out=_token_major(NC, H, lay.chunk, dk, torch.float32, khat.device))
-                dkhat = dkh.reshape(NC, G, H // G, *dkh.shape[2:]).sum(2).to(khat.dtype)
-            else:
-                dkhat = bgemm(u, Ln, out=_token_major(NC, H, lay.chunk, dk, khat.dtype, khat.device))
+            dkhat = bgemm(u, Ln, out=_token_major(NC, H, lay.chunk, dk, khat.dtype, khat.device))
         return dalpha, dkhat, du, None
 
 
@@ -665,7 +656,7 @@ def _scalar_prep(qp, kp, gp, scale, dt):
         from . import chunk_kernels
         if chunk_kernels.scalar_prep_supported(C, dk):
             return chunk_kernels.ScalarPrep.apply(qp, kp, gp, scale)
-    b = gp.cumsum(1) if gp is not None else torch.zeros(NC, C, H, dtype=torch.float32, device=qp.device)
+    b = gp.cumsum(1)
     b_last = b[:, -1]
     khat = kp * (b_last[:, None] - b).exp().to(dt)[..., None]
     qbar = qp * (b.exp() * scale).to(dt)[..., None]

@@ -17,7 +17,7 @@ import torch
 import torch.nn.functional as F
 
 from . import _lib, slots
-from .slots import split_columns  # noqa: F401 - the layers take it from here
+from .slots import split_columns  # noqa: F401 - part of this module's interface
 
 _lib.register("fb_hgrn2_gate_tiles", [c_longlong])
 _lib.register("fb_hgrn2_gate_fwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_void_p])
