@@ -484,7 +484,9 @@ def test_bgemm_result_boxes(M, N):
                 add = torch.randn(hi, lo, M, pad, device=dev).bfloat16()[..., :N]
                 bgemm(a, b, out=out, add16=add)
                 check(out, full + add.double(), eps)
+                before = out.double()
                 bgemm(a, b, out=out, add16=out)   # in place
+                check(out, full + before, eps)
             if M == N:
                 for mode, want in ((MASK_TRIL, full.tril()), (MASK_STRICT, full.tril(-1))):
                     bgemm(a, b, out=out, mask=mode)
