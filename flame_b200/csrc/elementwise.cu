@@ -738,6 +738,22 @@ __global__ void cast_f32_to_bf16_kernel(const float* __restrict__ x, __nv_bfloat
   }
 }
 
+// out = a + b in fp32 of bf16 operands (gradients of one tensor from two readers).  Bound by memory (8 bytes per element): torch's
+// widening of one and mixed-type sum took 0.025 + 0.029 ms for 8.4 M elements, this takes 0.012.
+__global__ void __launch_bounds__(256) add_bf16_to_f32_kernel(const __nv_bfloat16* __restrict__ a, const __nv_bfloat16* __restrict__ b,
+                                                              float* __restrict__ out, long long n) {
+  const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+  if (i + 8 <= n) {
+    float x[8], y[8];
+    unpack8(*reinterpret_cast<const uint4*>(a + i), x);
+    unpack8(*reinterpret_cast<const uint4*>(b + i), y);
+    reinterpret_cast<float4*>(out + i)[0] = make_float4(x[0] + y[0], x[1] + y[1], x[2] + y[2], x[3] + y[3]);
+    reinterpret_cast<float4*>(out + i)[1] = make_float4(x[4] + y[4], x[5] + y[5], x[6] + y[6], x[7] + y[7]);
+  } else {
+    for (long long k = i; k < n; ++k) out[k] = __bfloat162float(a[k]) + __bfloat162float(b[k]);
+  }
+}
+
 inline unsigned blocks_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
 }  // namespace
@@ -950,6 +966,14 @@ int fb_cast_f32_bf16(const float* x, void* y, long long n, cudaStream_t stream) 
   if (n == 0) return 0;
   cast_f32_to_bf16_kernel<<<blocks_for((n + 3) / 4, 256), 256, 0, stream>>>(x, (__nv_bfloat16*)y, n);
   return fb::launch_ok("cast_f32_to_bf16_kernel");
+}
+
+// a, b: bf16 [n]; out: fp32 [n]; all 16-byte aligned
+int fb_add_bf16_to_f32(const void* a, const void* b, float* out, long long n, cudaStream_t stream) {
+  if (n == 0) return 0;
+  if (!fb::aligned(16, a, b, out)) return -2;
+  add_bf16_to_f32_kernel<<<blocks_for((n + 7) / 8, 256), 256, 0, stream>>>((const __nv_bfloat16*)a, (const __nv_bfloat16*)b, out, n);
+  return fb::launch_ok("add_bf16_to_f32_kernel");
 }
 
 // row_bytes and the distances of rows must be multiples of 16 and both buffers 16-byte aligned; idx: int32 [n_dst], -1 = zero row

@@ -177,6 +177,18 @@ def l2norm(x: torch.Tensor, eps: float = 1e-6) -> torch.Tensor:
     return _L2Norm.apply(x, eps)
 
 
+_lib.register("fb_add_bf16_to_f32", [c_void_p] * 3 + [c_longlong, c_void_p])
+
+
+def add_to_f32(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
+    """``a + b`` in fp32 of two bf16 tensors of one shape."""
+    a, b = _lib.dense(a), _lib.dense(b)
+    out = torch.empty(a.shape, dtype=torch.float32, device=a.device)
+    _lib.check(_lib.lib().fb_add_bf16_to_f32(a.data_ptr(), b.data_ptr(), out.data_ptr(), a.numel(), _lib.stream_ptr()), "fb_add_bf16_to_f32")
+    _lib.count_launch()
+    return out
+
+
 _lib.register("fb_pair_dot", [c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_int, c_void_p])
 
 

@@ -883,6 +883,9 @@ class _TwoReaders(torch.autograd.Function):
         if a is None or b is None:
             d = b if a is None else a
             return None if d is None else d.to(ctx.dtype), None
+        if _lib.available() and a.is_cuda and a.dtype == b.dtype == torch.bfloat16:
+            from . import chunk_kernels
+            return chunk_kernels.add_to_f32(a, b).to(ctx.dtype), None
         return torch.add(a.float(), b).to(ctx.dtype), None
 
 

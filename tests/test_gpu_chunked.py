@@ -420,14 +420,15 @@ def test_gsa_slot_gradients_are_added_in_fp32():
     o = gsa(q, k, v, s, g, meta)
     ds, = torch.autograd.grad(o, s, torch.randn_like(o))
     assert ds.dtype == torch.float32 and (ds == ds.bfloat16().float()).float().mean() < 0.9
-    x = torch.rand(1000, device=DEV).requires_grad_(True)
-    a, b = _TwoReaders.apply(x, torch.bfloat16)
-    assert torch.equal(a, x.bfloat16()) and torch.equal(b, a)
-    da, db = _bf(1000), _bf(1000, s=1e-3)
-    dx, = torch.autograd.grad([a, b], x, [da, db], retain_graph=True)
-    assert torch.equal(dx, da.float() + db.float())
-    dx, = torch.autograd.grad(b, x, db)
-    assert torch.equal(dx, db.float())
+    for n in (1, 7, 8, 9, 1000, 2048, 2051):
+        x = torch.rand(n, device=DEV).requires_grad_(True)
+        a, b = _TwoReaders.apply(x, torch.bfloat16)
+        assert torch.equal(a, x.bfloat16()) and torch.equal(b, a)
+        da, db = _bf(n), _bf(n + 1, s=1e-3)[1:]
+        dx, = torch.autograd.grad([a, b], x, [da, db], retain_graph=True)
+        assert torch.equal(dx, da.float() + db.float())
+        dx, = torch.autograd.grad(b, x, db)
+        assert torch.equal(dx, db.float())
 
 
 def test_mamba2_ssd_grouped_heads_match_recurrence():
