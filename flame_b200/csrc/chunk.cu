@@ -373,6 +373,7 @@ __global__ void __launch_bounds__(256) group_bwd1_kernel(const __nv_bfloat16* __
 
 // dv = dv1 + dvhat e^{b_last - b}; db_i -= sum dvhat vhat, the chunk's last step gets that sum over all steps and
 // alpha dalpha; dg = reverse cumulative sum of db.  dv1 and dvo null: dv is not wanted; dalpha and dg null: dg is not.
+template <bool DV>
 __global__ void __launch_bounds__(256) group_bwd2_kernel(const __nv_bfloat16* __restrict__ dvhat, const __nv_bfloat16* __restrict__ vhat,
                                                          const __nv_bfloat16* __restrict__ dv1, const float* __restrict__ b,
                                                          const float* __restrict__ db, const float* __restrict__ alpha, const float* __restrict__ dalpha,
@@ -387,15 +388,14 @@ __global__ void __launch_bounds__(256) group_bwd2_kernel(const __nv_bfloat16* __
     float x[8], y[8], z[8], s = 0.f;
     unpack8f(*reinterpret_cast<const uint4*>(dvhat + o), x);
     unpack8f(*reinterpret_cast<const uint4*>(vhat + o), y);
-    if (dvo != nullptr) {
-      unpack8f(*reinterpret_cast<const uint4*>(dv1 + o), z);
-      const float f = __expf(last - b[ob]);
+    unpack8f(*reinterpret_cast<const uint4*>((DV ? dv1 : vhat) + o), z);
+    const float f = __expf(last - b[ob]);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) z[e] = fmaf(x[e], f, z[e]);
-      *reinterpret_cast<uint4*>(dvo + o) = pack8f(z);
+    for (int e = 0; e < 8; ++e) {
+      s = fmaf(x[e], y[e], s);
+      z[e] = fmaf(x[e], f, z[e]);
     }
-#pragma unroll
-    for (int e = 0; e < 8; ++e) s = fmaf(x[e], y[e], s);
+    if (DV) *reinterpret_cast<uint4*>(dvo + o) = pack8f(z);
     for (int k = nv >> 1; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
     if (vv == 0) {
       sdb[i] = db[ob] - s;
@@ -453,8 +453,9 @@ int fb_group_bwd2(const void* dvhat, const void* vhat, const void* dv1, const fl
                   int C, int H, int dv, void* dvo, float* dg, cudaStream_t stream) {
   if (NC <= 0) return 0;
   if (!group_shape_ok(C, dv) || !fb::aligned(16, dvhat, vhat, dv1, dvo)) return -2;
-  group_bwd2_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)dvhat, (const __nv_bfloat16*)vhat, (const __nv_bfloat16*)dv1, b, db,
-                                                            alpha, dalpha, C, H, dv, (__nv_bfloat16*)dvo, dg);
+  const auto kernel = dvo != nullptr ? group_bwd2_kernel<true> : group_bwd2_kernel<false>;
+  kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)dvhat, (const __nv_bfloat16*)vhat, (const __nv_bfloat16*)dv1, b, db, alpha, dalpha,
+                                                 C, H, dv, (__nv_bfloat16*)dvo, dg);
   return fb::launch_ok("group_bwd2_kernel");
 }
 
