@@ -90,7 +90,7 @@ def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = 
           more: Sequence[tuple] = (), sum_lo: int = 1) -> torch.Tensor:
     """``out[hi, lo] = alpha * a[hi, lo] @ b[hi, lo]^T`` (no autograd).
 
-    ``more``: up to three further products ``(a, b, a_mn, b_mn, sign)`` of the same result, added (or subtracted) in the
+    ``more``: up to five further products ``(a, b, a_mn, b_mn, sign)`` of the same result, added (or subtracted) in the
     accumulator.  ``rowscale``: fp32 ``[hi, lo, M]`` (any strides), a factor per row.  ``sum_lo``: every product is summed over
     that many consecutive lo coordinates of its operands (the heads of a group, in the accumulator too).
 
