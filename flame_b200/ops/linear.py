@@ -33,8 +33,13 @@ def _adjacent(ts: Sequence[torch.Tensor]) -> bool:
 
 
 def _cat_view(ts: Sequence[torch.Tensor]) -> torch.Tensor:
-    first = ts[0]
+    """Adjacent tensors (``_adjacent``) as one."""
+    first, last = ts[0], ts[-1]
     rows = sum(t.shape[0] for t in ts)
+    # ``set_`` would grow a storage that is too small and hand out what happens to lie there
+    if last.data_ptr() - first.data_ptr() != (rows - last.shape[0]) * first.stride(0) * first.element_size() or \
+            first.untyped_storage().data_ptr() != last.untyped_storage().data_ptr():
+        raise ValueError("not adjacent in memory")
     out = torch.empty(0, dtype=first.dtype, device=first.device)
     out.set_(first.untyped_storage(), first.storage_offset(), (rows, *first.shape[1:]), first.stride())
     return out
@@ -103,7 +108,8 @@ class _LinearFn(torch.autograd.Function):
         dx = None
         if ctx.needs_input_grad[0]:
             if ctx.fused:
-                wcat = weights[0] if len(weights) == 1 else _cat_view(list(weights))
+                # saved-tensor hooks hand back copies, which lie wherever they were put
+                wcat = weights[0] if len(weights) == 1 else _cat_view(weights) if _adjacent(weights) else torch.cat(weights, 0)
                 dx = gemm_nn(dy2, wcat)
             else:
                 dx32 = None

@@ -191,6 +191,49 @@ def test_layers_that_somebody_listens_to_run_by_themselves(monkeypatch):
     torch.testing.assert_close(modules.split_projections(x, layers)[2], 2 * plain(x))
 
 
+def test_one_view_of_tensors_that_are_not_adjacent_is_refused():
+    from flame_b200.ops.linear import _cat_view
+    flat = torch.arange(24.0).view(6, 4)
+    assert torch.equal(_cat_view([flat[:2], flat[2:5]]), flat[:5])
+    with pytest.raises(ValueError):
+        _cat_view([flat[:2].clone(), flat[2:5].clone()])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,kw", [
+    ("Attention", dict(num_heads=4)), ("Attention", dict(num_heads=2, num_kv_heads=1)), ("StickBreakingAttention", dict(num_heads=4)),
+    ("GatedLinearAttention", dict(num_heads=2)), ("DeltaNet", dict(num_heads=2)), ("GatedDeltaNet", dict(num_heads=2, head_dim=64)),
+    ("GatedSlotAttention", dict(num_heads=2)), ("Mamba", dict(intermediate_size=512, time_step_rank=16)), ("Mamba2", dict(num_heads=8)),
+])
+def test_layers_under_saved_tensor_hooks(name, kw):
+    """What is saved for the backward goes to the host and comes back as copies (the projections' weights too, which then lie
+    apart): the same numbers go through the same kernels, so the input's gradient is the same (fp32 sums of attention's dq by
+    atomics: 2^-8 of the largest entry)."""
+    from flame_b200.models import layers as layers_mod
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    dev = torch.device("cuda", 0)
+    D, cu = 256, (0, 1, 66, 131)
+    m = getattr(layers_mod, name)(D, **kw)
+    for p in m.parameters():
+        torch.nn.init.normal_(p, std=0.05) if p.dim() > 1 else torch.nn.init.uniform_(p, 0.5, 1.0)
+    m = m.to(dev)
+    for n, p in m.named_parameters():
+        if n not in ("A_log", "dt_bias", "D"):
+            p.data = p.data.bfloat16()
+    if hasattr(m, "q_proj"):
+        _adjacent([m.q_proj, m.k_proj, m.v_proj])
+        for layer in (m.q_proj, m.k_proj, m.v_proj):
+            del layer.weight.main_grad
+    meta = VarlenMeta.from_cu_seqlens(torch.tensor(cu, dtype=torch.int32, device=dev))
+    x, dy = torch.randn(cu[-1], D, device=dev).bfloat16().requires_grad_(True), torch.randn(cu[-1], D, device=dev).bfloat16()
+    want = torch.autograd.grad(m(x, meta), [x, *m.parameters()], dy)
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t.to(dev)):
+        y = m(x, meta)
+    for a, b in zip(torch.autograd.grad(y, [x, *m.parameters()], dy), want):
+        assert (a.double() - b.double()).abs().max() <= 2.0 ** -8 * b.double().abs().max()
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("name,kw", [
     ("GatedLinearAttention", dict(num_heads=2)),
