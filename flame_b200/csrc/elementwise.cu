@@ -763,13 +763,13 @@ namespace {
 // document come out zero) and its backward in one pass, instead of a fill plus an indexed copy.
 // Four vectors per thread, the indices of all four fetched before the first is used (one vector and a 64-bit division per
 // thread took 0.055 ms for 65,536 rows of 2 KB, this takes 0.041 ms).
-template <typename Index>
-__global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, const int* __restrict__ idx,
+template <typename Vec, typename Index>
+__global__ void __launch_bounds__(256) gather_rows_kernel(const Vec* __restrict__ src, Vec* __restrict__ dst, const int* __restrict__ idx,
                                                           Index total, Index vecs, long long src_ld, long long dst_ld) {
   const Index first = (Index)blockIdx.x * 1024 + threadIdx.x;
   Index row[4];
   int s[4];
-  uint4 q[4];
+  Vec q[4];
 #pragma unroll
   for (int t = 0; t < 4; ++t) {
     row[t] = (first + t * 256) / vecs;
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const uint4* __restric
   }
 #pragma unroll
   for (int t = 0; t < 4; ++t)
-    q[t] = s[t] >= 0 ? src[s[t] * src_ld + (first + t * 256 - row[t] * vecs)] : make_uint4(0, 0, 0, 0);
+    q[t] = s[t] >= 0 ? src[s[t] * src_ld + (first + t * 256 - row[t] * vecs)] : Vec{};
 #pragma unroll
   for (int t = 0; t < 4; ++t)
     if (first + t * 256 < total) dst[(long long)row[t] * dst_ld + (first + t * 256 - row[t] * vecs)] = q[t];
@@ -976,18 +976,26 @@ int fb_add_bf16_to_f32(const void* a, const void* b, float* out, long long n, cu
   return fb::launch_ok("add_bf16_to_f32_kernel");
 }
 
-// row_bytes and the distances of rows must be multiples of 16 and both buffers 16-byte aligned; idx: int32 [n_dst], -1 = zero row
+// row_bytes, the distances of rows and both addresses must be multiples of 16, or else of 4 (six fp32 scalars per token, say, which
+// took four torch kernels); idx: int32 [n_dst], -1 = zero row
 int fb_gather_rows(const void* src, void* dst, const int* idx, long long n_dst, long long row_bytes, long long src_ld, long long dst_ld,
                    cudaStream_t stream) {
   if (n_dst <= 0 || row_bytes <= 0) return 0;
-  if ((row_bytes % 16) || (src_ld % 16) || (dst_ld % 16) || ((uintptr_t)src & 15) || ((uintptr_t)dst & 15)) return -2;
-  const long long vecs = row_bytes / 16, total = n_dst * vecs;
+  const auto whole = [&](int unit) { return !((row_bytes | src_ld | dst_ld | (long long)(uintptr_t)src | (long long)(uintptr_t)dst) & (unit - 1)); };
+  if (!whole(4)) return -2;
+  const int unit = whole(16) ? 16 : 4;
+  const long long vecs = row_bytes / unit, total = n_dst * vecs;
   const unsigned grid = (unsigned)((total + 1023) / 1024);
-  if (total < (1ll << 31))
-    gather_rows_kernel<unsigned><<<grid, 256, 0, stream>>>((const uint4*)src, (uint4*)dst, idx, (unsigned)total, (unsigned)vecs, src_ld / 16,
-                                                           dst_ld / 16);
-  else
-    gather_rows_kernel<unsigned long long><<<grid, 256, 0, stream>>>((const uint4*)src, (uint4*)dst, idx, total, vecs, src_ld / 16, dst_ld / 16);
+  const auto launch = [&](auto vec, auto index) {
+    using Vec = decltype(vec);
+    using Index = decltype(index);
+    gather_rows_kernel<Vec, Index><<<grid, 256, 0, stream>>>((const Vec*)src, (Vec*)dst, idx, (Index)total, (Index)vecs, src_ld / unit, dst_ld / unit);
+  };
+  const bool small = total < (1ll << 31);
+  if (unit == 16 && small) launch(uint4{}, 0u);
+  else if (unit == 16) launch(uint4{}, 0ull);
+  else if (small) launch(0u, 0u);
+  else launch(0u, 0ull);
   return fb::launch_ok("gather_rows_kernel");
 }
 

@@ -19,7 +19,7 @@ from ..ops.rope import rope_tables
 from ..ops.slots import reshaped, split_columns
 from ..ops.varlen import VarlenMeta
 from .config import ModelConfig, mamba_dt_rank
-from .modules import Linear, RMSNorm, RMSNormGated, ShortConvolution, fused_projection, side_by_side, split_projections
+from .modules import Linear, RMSNorm, RMSNormGated, ShortConvolution, fused_projection, plain, side_by_side, split_projections
 
 
 class Attention(nn.Module):
@@ -210,6 +210,14 @@ def _feature_map(name: str, x: torch.Tensor) -> torch.Tensor:
     raise NotImplementedError(f"feature map {name!r}")
 
 
+def _conv_delta_rule(xs, convs, beta, g, meta: VarlenMeta, heads: int) -> Optional[torch.Tensor]:
+    """Short convolutions and (gated) delta rule in one go, or None where something wants the convolutions' own results."""
+    from ..ops.delta_rule import conv_gated_delta_rule
+    if not plain(convs, ShortConvolution):
+        return None
+    return conv_gated_delta_rule(xs, [c.weight for c in convs], [c.bias for c in convs], beta, g, meta, heads)
+
+
 class DeltaNet(nn.Module):
     """DeltaNet (fla/layers/delta_net.py:36-292): short conv + SiLU on q/k/v, L2-normalised q/k, beta = sigmoid."""
 
@@ -244,8 +252,15 @@ class DeltaNet(nn.Module):
         from ..ops.delta_rule import gated_delta_rule
         T, H = x.shape[0], self.num_heads
         layers = (self.q_proj, self.k_proj, self.v_proj)
+        beta = self.b_proj(x).float().sigmoid() if self.use_beta else torch.ones(T, H, device=x.device)
+        if self.allow_neg_eigval:
+            beta = beta * 2.0
         if self.use_short_conv:
             q, k, v = split_projections(x, layers)
+            if self.qk_activation == "silu" and self.qk_norm == "l2":
+                o = _conv_delta_rule((q, k, v), (self.q_conv1d, self.k_conv1d, self.v_conv1d), beta, None, meta, H)
+                if o is not None:
+                    return self._output(x, o)
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
         else:
             q, k, v = (l(x) for l in layers)
@@ -260,10 +275,10 @@ class DeltaNet(nn.Module):
             q, k = F.elu(q) + 1, F.elu(k) + 1
         if self.qk_norm == "sum":
             q, k = q / q.sum(-1, keepdim=True), k / k.sum(-1, keepdim=True)
-        beta = self.b_proj(x).float().sigmoid() if self.use_beta else torch.ones(T, H, device=x.device)
-        if self.allow_neg_eigval:
-            beta = beta * 2.0
-        o = gated_delta_rule(q, k, v, beta, None, meta, l2norm_qk=(self.qk_norm == "l2"))
+        return self._output(x, gated_delta_rule(q, k, v, beta, None, meta, l2norm_qk=(self.qk_norm == "l2")))
+
+    def _output(self, x: torch.Tensor, o: torch.Tensor) -> torch.Tensor:
+        T, H = x.shape[0], self.num_heads
         if self.use_gate:
             o = self.o_norm(o, self.g_proj(x).reshape(T, H, self.head_v_dim))
         else:
@@ -322,8 +337,16 @@ class GatedDeltaNet(nn.Module):
         T = x.shape[0]
         H, HV = self.num_heads, self.num_v_heads
         layers = (self.q_proj, self.k_proj, self.v_proj)
+        beta = self.b_proj(x).float().sigmoid()
+        if self.allow_neg_eigval:
+            beta = beta * 2.0
+        g = la.gdn_gate(self.a_proj(x), self.A_log, self.dt_bias)
         if self.use_short_conv:
             q, k, v = split_projections(x, layers)
+            if HV == H:
+                o = _conv_delta_rule((q, k, v), (self.q_conv1d, self.k_conv1d, self.v_conv1d), beta, g, meta, H)
+                if o is not None:
+                    return self._output(x, o)
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
         else:
             q, k, v = (l(x) for l in layers)
@@ -332,11 +355,10 @@ class GatedDeltaNet(nn.Module):
         v = v.reshape(T, HV, self.head_v_dim)
         if HV > H:
             q, k = q.repeat_interleave(HV // H, 1), k.repeat_interleave(HV // H, 1)
-        beta = self.b_proj(x).float().sigmoid()
-        if self.allow_neg_eigval:
-            beta = beta * 2.0
-        g = la.gdn_gate(self.a_proj(x), self.A_log, self.dt_bias)
-        o = gated_delta_rule(q, k, v, beta, g, meta, l2norm_qk=True)
+        return self._output(x, gated_delta_rule(q, k, v, beta, g, meta, l2norm_qk=True))
+
+    def _output(self, x: torch.Tensor, o: torch.Tensor) -> torch.Tensor:
+        T, HV = x.shape[0], self.num_v_heads
         if self.use_gate:
             o = self.o_norm(o, self.g_proj(x).reshape(T, HV, self.head_v_dim))
         else:

@@ -34,18 +34,22 @@ def fused_projection(x: torch.Tensor, layers: Sequence[Linear]) -> torch.Tensor:
     return linear_ops.linear_fused(x, [l.weight for l in layers])
 
 
-def side_by_side(layers: Sequence[Linear], x: torch.Tensor) -> bool:
-    """Whether one product may stand for these layers: plain ones (no bias, no hook on them or on all modules, no forward of a
-    subclass' or an instance's own), trained or frozen together, their weights next to one another in memory."""
+def plain(layers: Sequence[nn.Module], kind: type) -> bool:
+    """Whether calling these layers does nothing but ``kind.forward``: no hook on them or on all modules, no forward of a subclass'
+    or an instance's own."""
     if torch.nn.modules.module._has_any_global_hook():
         return False
-    for l in layers:
-        if type(l) is not Linear or l.bias is not None or l.weight.requires_grad != layers[0].weight.requires_grad:
-            return False
-        if "forward" in l.__dict__:
-            return False
-        if l._forward_hooks or l._forward_pre_hooks or l._backward_hooks or l._backward_pre_hooks:
-            return False
+    return not any(type(l) is not kind or "forward" in l.__dict__ or l._forward_hooks or l._forward_pre_hooks or l._backward_hooks
+                   or l._backward_pre_hooks for l in layers)
+
+
+def side_by_side(layers: Sequence[Linear], x: torch.Tensor) -> bool:
+    """Whether one product may stand for these layers: plain ones without a bias, trained or frozen together, their weights next
+    to one another in memory."""
+    if not plain(layers, Linear):
+        return False
+    if any(l.bias is not None or l.weight.requires_grad != layers[0].weight.requires_grad for l in layers):
+        return False
     return linear_ops.side_by_side(x, [l.weight for l in layers])
 
 

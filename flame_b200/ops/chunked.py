@@ -34,6 +34,7 @@ from .bgemm import MASK_STRICT, MASK_TRIL, _mask, bgemm, bmm
 from .varlen import VarlenMeta
 
 CHUNK = 64
+NO_ROW = -(1 << 20)  # as in csrc/conv.cu
 _lib.register("fb_gather_rows", [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_longlong, c_longlong, c_void_p])
 _lib.register("fb_delta_scan", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_int, c_void_p])
@@ -94,14 +95,25 @@ class ChunkLayout:
         last = first + nchunks - 1
         inv = np.full(self.Tp, -1, dtype=np.int32)
         inv[rows] = np.arange(self.T, dtype=np.int32)
-        self._first_np, self._nchunks_np = first, nchunks
+        self._first_np, self._nchunks_np, self._rows_np = first, nchunks, rows
+        self._positions = np.arange(self.T, dtype=np.int32) - np.repeat(starts, lens).astype(np.int32)
         self.rows = torch.from_numpy(rows).to(dev)                            # packed token -> padded row
         self.first = torch.from_numpy(first).to(dev)                          # first chunk of every document
         self.last = torch.from_numpy(last).to(dev)                            # last chunk of every document
         self.first_i32, self.last_i32 = self.first.to(torch.int32), self.last.to(torch.int32)
         self.rows_i32 = self.rows.to(torch.int32)
         self.inv_i32 = torch.from_numpy(inv).to(dev)                          # padded row -> packed token, -1 = padding
-        self._steps = None
+        self._steps = self._pos = None
+
+    @property
+    def pos_i32(self) -> torch.Tensor:
+        """int32 ``[Tp]``: offset of every padded row inside its document, ``NO_ROW`` in the padding."""
+        if self._pos is None:
+            import numpy as np
+            pos = np.full(self.Tp, NO_ROW, dtype=np.int32)
+            pos[self._rows_np] = self._positions
+            self._pos = torch.from_numpy(pos).to(self.inv_i32.device)
+        return self._pos
 
     def _build_steps(self) -> None:
         # chunks at in-document position s that have a successor, and the documents they belong to (only the
@@ -155,18 +167,21 @@ def _row_distance(x: torch.Tensor) -> int:
 
 
 def _rows_strided(x: torch.Tensor) -> bool:
-    """Rows that are contiguous and whole 16-byte vectors, at any distance that is one too: what the gather kernel reads."""
+    """Rows that are contiguous and whole 16-byte vectors, at any distance that is one too, or the same with 4-byte words (a
+    few scalars per token): what the gather kernel reads."""
     n = x.numel() // max(x.shape[0], 1)
     inner = list(x.stride()[1:]) == [math.prod(x.shape[i + 1:]) for i in range(1, x.dim())]
     ld = _row_distance(x)
-    return inner and n * x.element_size() % 16 == 0 and ld * x.element_size() % 16 == 0 and x.data_ptr() % 16 == 0 and ld >= n
+    unit = 16 if n * x.element_size() % 16 == 0 else 4
+    return inner and n * x.element_size() % unit == 0 and ld * x.element_size() % unit == 0 and x.data_ptr() % unit == 0 and ld >= n
 
 
 def _gather_rows(x: torch.Tensor, idx: torch.Tensor, n_out: int, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[r] = x[idx[r]]`` (zero where ``idx[r] < 0``) in one pass of the row-gather kernel."""
     x = x if _rows_strided(x) else x.contiguous()
     row_bytes = (x.numel() // max(x.shape[0], 1)) * x.element_size()
-    if not (_lib.available() and x.is_cuda and row_bytes % 16 == 0 and x.shape[0] > 0 and x.data_ptr() % 16 == 0):
+    unit = 16 if row_bytes % 16 == 0 else 4
+    if not (_lib.available() and x.is_cuda and row_bytes % unit == 0 and x.shape[0] > 0 and x.data_ptr() % unit == 0):
         safe = idx.clamp_min(0).long()
         r = x.index_select(0, safe)
         r = r * (idx >= 0).to(x.dtype).view(-1, *([1] * (x.dim() - 1)))
@@ -683,6 +698,14 @@ def gated_delta_rule_tc(q, k, v, beta, g, meta: VarlenMeta, scale: Optional[floa
     qp, kp, vp = lay.pack(q).to(dt), lay.pack(k).to(dt), lay.pack(v).to(dt)   # [NC, C, H, d]
     o = _GatedDelta.apply(qp, kp, vp, lay.pack(beta.float()), None if g is None else lay.pack(g.float()), scale, lay)
     return lay.unpack(o).to(v.dtype)
+
+
+@_recomputable
+def gated_delta_rule_chunks(qp, kp, vp, beta, g, meta: VarlenMeta, lay: "ChunkLayout", scale: float) -> torch.Tensor:
+    """The same with q, k, v already in the rows of ``lay`` (``[Tp, H, d]`` bf16; the padding's q, k and v are zero)."""
+    qp, kp, vp = (t.view(lay.NC, lay.chunk, *t.shape[1:]) for t in (qp, kp, vp))
+    o = _GatedDelta.apply(qp, kp, vp, lay.pack(beta.float()), None if g is None else lay.pack(g.float()), scale, lay)
+    return lay.unpack(o)
 
 
 @_recomputable

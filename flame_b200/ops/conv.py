@@ -181,6 +181,18 @@ def short_conv(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tenso
     return la.short_conv(x, weight, bias, meta, activation)
 
 
+def short_convs_in_chunks(xs, weights, biases, meta: VarlenMeta, activation: Optional[str], chunk: int):
+    """Several width-4 convolutions of the same rows in one launch, their results ``[Tp, D]`` in the padded rows of
+    ``ChunkLayout.of(meta, chunk)`` (zeros in the padding), or None where the kernel does not apply."""
+    if (getattr(meta, "sequence_slice", None) is not None or not 0 < len(xs) <= MAX_TOGETHER or xs[0].shape[0] == 0
+            or not all(_kernel_ok(x, w) and w.shape[-1] == 4 for x, w in zip(xs, weights))):
+        return None
+    from .chunked import ChunkLayout
+    lay = ChunkLayout.of(meta, chunk)
+    if lay.T != xs[0].shape[0]:
+        return None
+    return _ShortConv4.apply(meta, activation in ("silu", "swish"), None if lay.aligned else lay, len(xs), *xs, *weights, *biases)
+
 
 class _PositionsOnly:
     """The part of a ``VarlenMeta`` the convolution reads."""

@@ -684,3 +684,54 @@ def test_short_conv_backward_needs_no_more_partials_than_it_writes():
     before = torch.cuda.memory_allocated()
     torch.autograd.grad(y, [x, w], dy)
     assert torch.cuda.max_memory_allocated() - before <= 2 * T * D + 37 * D * 5 * 4 + (4 << 20)
+
+
+@pytest.mark.parametrize("chunk", [64, 128])
+@pytest.mark.parametrize("lens", [[1], [16, 64, 3], [65, 128, 1, 1, 2], [127, 63, 192], [200, 15, 17, 49], [4097, 5]])
+@pytest.mark.parametrize("main", [False, True])
+def test_short_convs_in_chunk_rows(lens, chunk, main):
+    """Three convolutions of one launch into the padded rows and back, documents that end before, on and behind the tiles of 16 rows and
+    the chunks: bit for bit what one convolution each and a gather give (the same sums in the same order per row), weight gradients
+    (fp32 sums over other strips, at most 4,102 rows: n 2^-24 sqrt(n) of the terms' size) to 1e-4.  The padding's incoming gradient is
+    not looked at."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.conv import short_conv, short_convs_in_chunks
+    torch.manual_seed(len(lens))
+    meta, T = _meta(lens), sum(lens)
+    lay, widths = ChunkLayout.of(meta, chunk), (72, 8, 136)
+    wide = torch.randn(T, sum(widths) + 8, device=DEV).bfloat16()
+    ws = [(torch.randn(n, 1, 4, device=DEV) * 0.4).bfloat16() for n in widths]
+    bs = [None, torch.randn(8, device=DEV).bfloat16(), torch.randn(136, device=DEV).bfloat16()]
+    dys = [torch.randn(lay.Tp, n, device=DEV).bfloat16() for n in widths]
+    results = []
+    for together in (True, False):
+        x = wide.clone().requires_grad_(True)
+        params = [p.clone().requires_grad_(True) for p in ws + [b for b in bs if b is not None]]
+        if main:
+            for p in params:
+                p.main_grad = torch.ones(p.shape, device=DEV)
+        w, b = params[:3], [None, *params[3:]]
+        xs = torch.split(x[:, :sum(widths)], widths, 1)
+        if together:
+            ys = short_convs_in_chunks(xs, w, b, meta, "silu", chunk)
+        else:
+            ys = [lay.pack(short_conv(*a, meta, "silu")).reshape(lay.Tp, -1) for a in zip(xs, w, b)]
+        pad = (lay.inv_i32 < 0)[:, None]
+        torch.autograd.backward(ys, [dy.masked_fill(pad, 7e3 if together else 0) for dy in dys])
+        results.append((list(ys), x.grad, [p.main_grad if main else p.grad for p in params]))
+    (y1, x1, p1), (y2, x2, p2) = results
+    assert all(torch.equal(a, b) for a, b in zip(y1, y2)) and torch.equal(x1, x2)
+    for a, b in zip(p1, p2):
+        assert rel_err(a, b) < (1e-4 if main else 5e-3)   # rounded to bf16 once without main_grad
+
+
+@pytest.mark.parametrize("cols,dtype", [(1, torch.float32), (6, torch.float32), (6, torch.bfloat16), (3, torch.bfloat16), (8, torch.float32)])
+def test_row_gather_of_few_scalars(cols, dtype):
+    """Rows that are whole 16-byte vectors, whole 4-byte words and neither, also out of a wider matrix: exact."""
+    from flame_b200.ops.chunked import ChunkLayout
+    lens = [5, 64, 700, 1]
+    lay = ChunkLayout.of(_meta(lens), 64)
+    for x in (torch.randn(sum(lens), cols, device=DEV).to(dtype), torch.randn(sum(lens), cols + 2, device=DEV).to(dtype)[:, 2:]):
+        got = lay.pack(x).reshape(lay.Tp, cols)
+        want = torch.zeros(lay.Tp, cols, device=DEV, dtype=dtype).index_copy(0, lay.rows, x)
+        assert torch.equal(got, want) and torch.equal(lay.unpack(lay.pack(x)), x)
