@@ -17,6 +17,7 @@
 //
 // Takes the place of flash_attn_varlen_func as called by fla/layers/attn.py:146-174.
 #include "sb_math.cuh"
+#include "attn_tiles.cuh"
 #include "tc05.cuh"
 #include "host_utils.cuh"
 #include <math.h>
@@ -70,16 +71,6 @@ __device__ __forceinline__ float poly_exp2(float x) {
   return __uint_as_float(__float_as_uint(p) + (__float_as_uint(t) << 23));
 }
 
-// largest i in [0, n) with offs[i] <= x
-__device__ __forceinline__ int upper_doc(const int* __restrict__ offs, int n, int x) {
-  int lo = 0, hi = n;
-  while (hi - lo > 1) {
-    int mid = (lo + hi) >> 1;
-    if (offs[mid] <= x) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
 // byte offset of element (row, col) in a [rows][64]-bf16 tile stored with the 128-byte swizzle
 __device__ __forceinline__ uint32_t sw128_offset(int row, int col) {
   const int chunk = (col >> 3) ^ (row & 7);
@@ -107,14 +98,9 @@ __global__ void __launch_bounds__(192, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, AttnParams p) {
   using L = FwdSmem<DH>;
-  const int total_tiles = p.tile_offsets[p.nseq];
-  // heavier tiles (late in their document) are scheduled first
-  const int tile_id = total_tiles - 1 - (int)blockIdx.x;
-  if (tile_id < 0) return;
-  const int head = blockIdx.y;
+  int head, doc, tile_in_doc;
+  if (!attn_tile(p.tile_offsets, p.nseq, p.H, true, head, doc, tile_in_doc)) return;
   const int kv_head = head / (p.H / p.Hkv);
-  const int doc = upper_doc(p.tile_offsets, p.nseq + 1, tile_id);
-  const int tile_in_doc = tile_id - p.tile_offsets[doc];
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
   const int q0 = tile_in_doc * BQ;
@@ -437,13 +423,9 @@ attn_fwd_pt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmV, AttnParams p) {
   using L = FwdPtSmem;
   constexpr int DH = 64;
-  const int total_tiles = p.tile_offsets[p.nseq];
-  const int tile_id = total_tiles - 1 - (int)blockIdx.x;  // heavier tiles first
-  if (tile_id < 0) return;
-  const int head = blockIdx.y;
+  int head, doc, tile_in_doc;
+  if (!attn_tile(p.tile_offsets, p.nseq, p.H, true, head, doc, tile_in_doc)) return;
   const int kv_head = head / (p.H / p.Hkv);
-  const int doc = upper_doc(p.tile_offsets, p.nseq + 1, tile_id);
-  const int tile_in_doc = tile_id - p.tile_offsets[doc];
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
   const int q0 = tile_in_doc * BQ;
@@ -771,13 +753,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const __grid_constant__ CUtensorMap tmdQ, AttnBwdParams p) {
   static_assert(DH == 64, "the backward kernel is laid out for head dim 64");
   using L = BwdSmem<DH>;
-  const int total_tiles = p.tile_offsets[p.nseq];
-  const int tile_id = (int)blockIdx.x;  // early key tiles see the most queries and come first
-  if (tile_id >= total_tiles) return;
-  const int kv_head = blockIdx.y;
+  int kv_head, doc, j;  // early key tiles see the most queries
+  if (!attn_tile(p.tile_offsets, p.nseq, p.Hkv, false, kv_head, doc, j)) return;
   const int group = p.H / p.Hkv;
-  const int doc = upper_doc(p.tile_offsets, p.nseq + 1, tile_id);
-  const int j = tile_id - p.tile_offsets[doc];
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
   const int n_qt = (doc_len + BQ - 1) / BQ;
@@ -1116,13 +1094,9 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmdQ, AttnBwdParams p) {
   using L = Bwd128Smem;
   constexpr int DH = 128, BQ2 = L::BQ2;
-  const int total_tiles = p.tile_offsets[p.nseq];
-  const int tile_id = (int)blockIdx.x;
-  if (tile_id >= total_tiles) return;
-  const int kv_head = blockIdx.y;
+  int kv_head, doc, j;  // early key tiles see the most queries
+  if (!attn_tile(p.tile_offsets, p.nseq, p.Hkv, false, kv_head, doc, j)) return;
   const int group = p.H / p.Hkv;
-  const int doc = upper_doc(p.tile_offsets, p.nseq + 1, tile_id);
-  const int j = tile_id - p.tile_offsets[doc];
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
   const int kv0 = j * BKV;
@@ -1439,16 +1413,68 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
 }
 
-// tile_offsets[i] = sum_{d < i} ceil(len_d / 128); single CTA, sequential over documents in chunks
-__global__ void attn_tile_offsets_kernel(const int* __restrict__ cu, int nseq, int* __restrict__ offs) {
-  if (threadIdx.x == 0) {
-    int acc = 0;
-    offs[0] = 0;
-    for (int d = 0; d < nseq; ++d) {
-      acc += (cu[d + 1] - cu[d] + BQ - 1) / BQ;
-      offs[d + 1] = acc;
+// attn_tiles.cuh's list.  One CTA: documents are counted by their tiles (longer ones than the last bin's in any order), the bins laid
+// out from the longest down, and both prefix sums taken LIST_THREADS documents at a time.
+constexpr int LIST_THREADS = 1024, LIST_BINS = 2048;
+__global__ void __launch_bounds__(LIST_THREADS) attn_tile_list_kernel(const int* __restrict__ cu, int nseq, int* list) {
+  __shared__ int bin[LIST_BINS], scan[LIST_THREADS / 32], total;
+  const int tid = threadIdx.x, lane = tid & 31;
+  int *offs = list, *sorted = list + nseq + 1, *docs = sorted + nseq + 1;
+  auto tiles = [&](int d) { return (cu[d + 1] - cu[d] + BQ - 1) / BQ; };
+  // exclusive prefix sum over the block; every thread gets the block's sum too
+  auto block_scan = [&](int v, int& sum) {
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
+    __syncthreads();
+    if (lane == 31) scan[tid >> 5] = x;
+    __syncthreads();
+    if (tid < 32) {
+      int w = scan[lane];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += y;
+      }
+      scan[lane] = w;
+      if (lane == 31) total = w;
+    }
+    __syncthreads();
+    sum = total;
+    return x - v + (tid >= 32 ? scan[(tid >> 5) - 1] : 0);
+  };
+  for (int i = tid; i < LIST_BINS; i += LIST_THREADS) bin[i] = 0;
+  __syncthreads();
+  int base = 0, sum;
+  for (int d0 = 0; d0 < nseq; d0 += LIST_THREADS) {
+    const int d = d0 + tid, n = d < nseq ? tiles(d) : 0;
+    if (d < nseq) atomicAdd(&bin[LIST_BINS - 1 - min(n, LIST_BINS - 1)], 1);
+    const int at = block_scan(n, sum);
+    if (d < nseq) offs[d] = base + at;
+    base += sum;
   }
+  if (tid == 0) offs[nseq] = base;
+  __syncthreads();
+  base = 0;
+  for (int i0 = 0; i0 < LIST_BINS; i0 += LIST_THREADS) {
+    const int at = block_scan(bin[i0 + tid], sum);
+    bin[i0 + tid] = base + at;
+    base += sum;
+  }
+  __syncthreads();
+  for (int d = tid; d < nseq; d += LIST_THREADS) docs[atomicAdd(&bin[LIST_BINS - 1 - min(tiles(d), LIST_BINS - 1)], 1)] = d;
+  __syncthreads();
+  base = 0;
+  for (int i0 = 0; i0 < nseq; i0 += LIST_THREADS) {
+    const int i = i0 + tid, n = i < nseq ? tiles(docs[i]) : 0;
+    const int at = block_scan(n, sum);
+    if (i < nseq) sorted[i] = base + at;
+    base += sum;
+  }
+  if (tid == 0) sorted[nseq] = base;
 }
 
 template <typename K>
@@ -1473,9 +1499,10 @@ int make_qkv_map(CUtensorMap* m, const void* base, long long T, int H, int DH, l
 extern "C" {
 
 
+// tile_offsets: int32 [3 nseq + 2], see attn_tiles.cuh
 int fb_attn_tile_offsets(const int* cu_seqlens, int nseq, int* tile_offsets, cudaStream_t stream) {
-  attn_tile_offsets_kernel<<<1, 32, 0, stream>>>(cu_seqlens, nseq, tile_offsets);
-  return fb::launch_ok("attn_tile_offsets_kernel");
+  attn_tile_list_kernel<<<1, LIST_THREADS, 0, stream>>>(cu_seqlens, nseq, tile_offsets);
+  return fb::launch_ok("attn_tile_list_kernel");
 }
 
 // max_tiles: an upper bound on the number of 128-row tiles (T / 128 + nseq is always enough).
@@ -1506,7 +1533,7 @@ int fb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse
   p.O_lo = nullptr;
   p.lse = lse;
   p.status = fb::status_ptr();
-  dim3 grid(max_tiles, H);
+  const unsigned grid = (unsigned)max_tiles * H;
   static const bool p_in_tmem = []() {
     const char* e = getenv("FLAME_B200_ATTN_FWD_PT");  // 0: the version of the kernel that stages P in shared memory
     return !(e && e[0] == '0');
@@ -1557,7 +1584,7 @@ int fb_sb_attn_fwd(const void* q, const void* k, const void* v, void* o, void* o
   p.status = fb::status_ptr();
   static bool done = false;
   if (!done) { rc = set_smem(attn_fwd_kernel<64, 1>, FwdSmem<64>::TOTAL); if (rc) return rc; done = true; }
-  dim3 grid(max_tiles, H);
+  const unsigned grid = (unsigned)max_tiles * H;
   attn_fwd_kernel<64, 1><<<grid, 192, FwdSmem<64>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
   return fb::launch_ok("attn_fwd_kernel<sb>");
 }
@@ -1621,7 +1648,7 @@ int fb_attn_bwd(const void* q, const void* k, const void* v, const void* dout, c
   p.dk_stride_t = dk_stride_t;
   p.dv_stride_t = dv_stride_t;
   p.status = fb::status_ptr();
-  dim3 grid(max_tiles, Hkv);
+  const unsigned grid = (unsigned)max_tiles * Hkv;
   if (DH == 128) {
     static bool done128 = false;
     if (!done128) { rc = set_smem(attn_bwd128_kernel, Bwd128Smem::TOTAL); if (rc) return rc; done128 = true; }

@@ -14,6 +14,7 @@
 // the move of one tile (two trips through a staging tile, about as long as the weights' own arithmetic) overlaps the next
 // tile's weights; one group of four did both in turn (12.4 us per tile, 5.7 ms for 8 x 4,096 tokens and 16 heads).  The reference reaches the same sums with spin-locked adds
 // (custom_models/sba/stickbreaking_attention/sb_varlen/sb_varlen_bwd.py:13-52); here nothing spins unbounded.
+#include "attn_tiles.cuh"
 #include "sb_math.cuh"
 #include "tc05.cuh"
 #include "host_utils.cuh"
@@ -38,14 +39,6 @@ struct SbBwdParams {
   int* status;
 };
 
-__device__ __forceinline__ int upper_doc(const int* __restrict__ offs, int n, int x) {
-  int lo = 0, hi = n;
-  while (hi - lo > 1) {
-    int mid = (lo + hi) >> 1;
-    if (offs[mid] <= x) lo = mid; else hi = mid;
-  }
-  return lo;
-}
 __device__ __forceinline__ uint32_t sw128_offset(int row, int col) {
   const int chunk = (col >> 3) ^ (row & 7);
   return (uint32_t)(row * 128 + chunk * 16 + (col & 7) * 2);
@@ -73,12 +66,8 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
                    const __grid_constant__ CUtensorMap tmdK, const __grid_constant__ CUtensorMap tmdV, SbBwdParams p) {
   using L = Smem;
-  const int total_tiles = p.tile_offsets[p.nseq];
-  const int tile_id = total_tiles - 1 - (int)blockIdx.x;  // long walks first
-  if (tile_id < 0) return;
-  const int head = blockIdx.y;
-  const int doc = upper_doc(p.tile_offsets, p.nseq + 1, tile_id);
-  const int ti = tile_id - p.tile_offsets[doc];
+  int head, doc, ti;
+  if (!attn_tile(p.tile_offsets, p.nseq, p.H, true, head, doc, ti)) return;
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
   const int q0 = ti * BQ;
@@ -451,7 +440,7 @@ int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
     if (e != cudaSuccess) return (int)e;
     done = true;
   }
-  dim3 grid(max_tiles, H);
+  const unsigned grid = (unsigned)max_tiles * H;
   sb_attn_bwd_kernel<<<grid, SB_THREADS, Smem::TOTAL, stream>>>(tmQ, tmK, tmV, tmdO, tmdK, tmdV, p);
   return fb::launch_ok("sb_attn_bwd_kernel");
 }

@@ -89,19 +89,20 @@ class VarlenMeta:
 
     @property
     def tile_offsets(self) -> torch.Tensor:
-        """int32 [nseq + 1]: prefix sum of ``ceil(len / 128)`` (attention work list)."""
+        """int32 [nseq + 1]: prefix sum of ``ceil(len / 128)``; on the GPU the kernels find the rest of their work list
+        (``csrc/attn_tiles.cuh``) behind it in memory."""
         if self._tile_offsets is None:
             if self.device.type == "cuda" and _lib.available():
-                t = torch.empty(self.nseq + 1, dtype=torch.int32, device=self.device)
+                t = torch.empty(3 * self.nseq + 2, dtype=torch.int32, device=self.device)
                 rc = _lib.lib().fb_attn_tile_offsets(self.cu_seqlens.data_ptr(), self.nseq, t.data_ptr(),
                                                      _lib.stream_ptr())
                 _lib.check(rc, "fb_attn_tile_offsets")
                 _lib.count_launch()
-            else:
+                self._tile_offsets = t[:self.nseq + 1]
+            else:  # not kept: a kernel would look behind it
                 cu = self.cu_seqlens.long()
                 n = (cu[1:] - cu[:-1] + 127) // 128
-                t = torch.cat([torch.zeros(1, dtype=torch.long, device=self.device), n.cumsum(0)]).to(torch.int32)
-            self._tile_offsets = t
+                return torch.cat([torch.zeros(1, dtype=torch.long, device=self.device), n.cumsum(0)]).to(torch.int32)
         return self._tile_offsets
 
     def lengths_list(self) -> list[int]:

@@ -735,3 +735,22 @@ def test_row_gather_of_few_scalars(cols, dtype):
         got = lay.pack(x).reshape(lay.Tp, cols)
         want = torch.zeros(lay.Tp, cols, device=DEV, dtype=dtype).index_copy(0, lay.rows, x)
         assert torch.equal(got, want) and torch.equal(lay.unpack(lay.pack(x)), x)
+
+
+@pytest.mark.parametrize("lens", [[1], [128], [129, 127, 0, 1], [1] * 1023 + [300, 5], [4096] * 3 + [64] * 1500, [270000, 262016, 130, 262017]])
+def test_attention_work_list(lens):
+    """Prefix sums of the documents' tiles in their order and by falling length (beyond the last bin's 2,047 tiles in any order), over more
+    documents than the block has threads: exact."""
+    import numpy as np
+    from flame_b200.ops.varlen import VarlenMeta
+    n = len(lens)
+    meta = VarlenMeta.from_cu_seqlens(torch.tensor([0] + list(np.cumsum(lens)), dtype=torch.int32), sum(lens), torch.device(DEV))
+    offs = meta.tile_offsets
+    assert offs.shape == (n + 1,)
+    whole = torch.as_strided(offs, (3 * n + 2,), (1,)).tolist()
+    tiles = [-(-x // 128) for x in lens]
+    docs = whole[2 * n + 2:]
+    assert whole[:n + 1] == [0] + list(np.cumsum(tiles))
+    assert sorted(docs) == list(range(n)) and whole[n + 1:2 * n + 2] == [0] + list(np.cumsum([tiles[d] for d in docs]))
+    clipped = [min(tiles[d], 2047) for d in docs]
+    assert clipped == sorted(clipped, reverse=True)
