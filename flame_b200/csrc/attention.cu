@@ -251,21 +251,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
           tc_fence_after();
         }
         float E = m_run;  // m_run doubles as the carried product (starts at 1 for this mode)
-#pragma unroll 1
-        for (int c0 = BKV - 32; c0 >= 0; c0 -= 32) {
-          uint32_t xr[32];
-          tmem_ld_32x32(tmem_S + lane_sel + c0, xr);
+        uint32_t xr[2][16];  // sixteen keys' logits, the next sixteen on their way
+        tmem_ld_32x16(tmem_S + lane_sel + BKV - 16, xr[0]);
+#pragma unroll 2
+        for (int h = 0; h < BKV / 16; ++h) {
+          const int c0 = BKV - 16 - h * 16;
           tmem_ld_wait();
+          if (c0 > 0) tmem_ld_32x16(tmem_S + lane_sel + c0 - 16, xr[(h & 1) ^ 1]);
 #pragma unroll
-          for (int c = 24; c >= 0; c -= 8) {
-            float e[8], sig[8];
-            if (diag) sb_group<true>(xr + c, p.scale_log2, sb_dead_bits(false, true, kv0 + c0 + c, q_idx), E, sig, e);
-            else sb_group<false>(xr + c, p.scale_log2, 0u, E, sig, e);
-            uint4 q;
-            q.x = pack_bf16(e[0], e[1]);
-            q.y = pack_bf16(e[2], e[3]);
-            q.z = pack_bf16(e[4], e[5]);
-            q.w = pack_bf16(e[6], e[7]);
+          for (int c = 8; c >= 0; c -= 8) {
+            sb2 e[4], sig[4];
+            if (diag) sb_group<true>(xr[h & 1] + c, p.scale_log2, sb_dead_bits(false, true, kv0 + c0 + c, q_idx), E, sig, e);
+            else sb_group<false>(xr[h & 1] + c, p.scale_log2, 0u, E, sig, e);
+            const uint4 q = make_uint4(sb_pack(e[0]), sb_pack(e[1]), sb_pack(e[2]), sb_pack(e[3]));
             const int cc = c0 + c;
             *reinterpret_cast<uint4*>(sP + (cc >> 6) * (BQ * 128) + sw128_offset(r, cc & 63)) = q;
           }

@@ -4,15 +4,22 @@
 //   g_ij   = do_i . v_j - drem_i,   dA = att * g,   dl_ij = dA_ij - sigma_ij * sum_{k<=j} dA_ik
 //   dq_i = scale sum_j dl_ij k_j,   dk_j = scale sum_i dl_ij q_i,   dv_j = sum_i att_ij do_i
 //
-// One CTA owns a 128-query tile of one (document, head) and walks the key tiles from the diagonal backwards - the
+// One CTA owns a 128-query tile of one (document, head) and walks the keys, 64 at a time, from the diagonal backwards - the
 // direction in which both running quantities of a row are available: E = prod (1 - sigma) over the keys already
 // seen (so att = sigma * E) and R = sum of dA over the keys already seen; the prefix sum the gradient needs is
 // Tot_i - R with Tot_i = do_i . o_i - drem_i (1 - rem_i), known up front.  Per key tile the tensor core forms S and dP,
-// one thread per query row turns them into P = att and dS = dl (bf16, swizzled smem), and three more MMAs produce the
-// tile's dV, dK (fresh each tile, added to fp32 accumulators in global memory by TMA reduce) and dQ (accumulated in
-// TMEM across the whole walk, no atomics).  Warps: TMA, MMA, four that form P and dS, four that move dV and dK out, so that
-// the move of one tile (two trips through a staging tile, about as long as the weights' own arithmetic) overlaps the next
-// tile's weights; one group of four did both in turn (12.4 us per tile, 5.7 ms for 8 x 4,096 tokens and 16 heads).  The reference reaches the same sums with spin-locked adds
+// one thread per query row turns them into P = att and dS = dl (bf16, swizzled smem), and three more products make the
+// tile's dV and dK (fresh each tile, added to fp32 accumulators in global memory) and dQ (accumulated in
+// TMEM across the whole walk, no atomics).  Warps: TMA, MMA, four that form P and dS, four that move dV and dK out.
+//
+// What bounds it is the chain of a tile: clock stamps give 7,500 cycles per 64 keys, of them 4,100 in the weight warps, which issue
+// a quarter of the time, the rest waits for products and hand-overs.  So two CTAs share an SM: 256
+// tensor-memory columns and 112 KB each.  That is why dV and dK are formed transposed, in ONE accumulator of 128 rows (64
+// of dV, 64 of dK) and 64 columns (keys): [dO | 0]^T P + [0 | Q]^T dS, the zeros a tile in shared memory between the two.  A
+// row of it is one channel of 64 keys, so 32 lanes hold 32 neighbouring floats of a key's gradient and add them
+// to global memory as they are (red.add, 128 bytes per instruction), without a staging tile.  S and dP of the next tile are
+// issued ahead of this tile's other products.  Eight rows of 4,096 tokens, 16 heads: 2.46 -> 2.02 ms (one CTA of
+// 128 x 128 tiles per SM).  The reference reaches the same sums with spin-locked adds
 // (custom_models/sba/stickbreaking_attention/sb_varlen/sb_varlen_bwd.py:13-52); here nothing spins unbounded.
 #include "attn_tiles.cuh"
 #include "sb_math.cuh"
@@ -24,7 +31,7 @@ using namespace tc05;
 
 namespace {
 
-constexpr int BQ = 128, BKV = 128, DH = 64;
+constexpr int BQ = 128, BKV = 64, DH = 64;
 constexpr float kLog2e = 1.4426950408889634f;
 
 struct SbBwdParams {
@@ -34,6 +41,7 @@ struct SbBwdParams {
   float scale, scale_log2;
   const float* tot;    // [H, T]  do.o - drem (1 - rem)
   const float* drem;   // [H, T] or null
+  float *dK, *dV;      // [T, H, DH] fp32, added to
   __nv_bfloat16* dQ;   // [T, H, DH] with token stride dq_stride_t
   long long dq_stride_t;
   int* status;
@@ -45,45 +53,45 @@ __device__ __forceinline__ uint32_t sw128_offset(int row, int col) {
 }
 
 struct Smem {
-  static constexpr int TILE = 128 * DH * 2;          // 16 KB
-  static constexpr int Q_OFF = 0, DO_OFF = TILE;
+  static constexpr int TILE = BQ * DH * 2;           // 16 KB
+  static constexpr int DO_OFF = 0, ZERO_OFF = TILE, Q_OFF = 2 * TILE;  // in this order: the transposed products' A operands
   static constexpr int NSTAGE = 2;
-  static constexpr int RING_OFF = 2 * TILE;          // stage = K tile + V tile
-  static constexpr int STAGE = 2 * TILE;
+  static constexpr int KV = BKV * DH * 2;            // 8 KB
+  static constexpr int RING_OFF = 3 * TILE;          // stage = K tile + V tile
+  static constexpr int STAGE = 2 * KV;
   static constexpr int P_OFF = RING_OFF + NSTAGE * STAGE;
-  static constexpr int PD = BQ * BKV * 2;            // 32 KB
-  static constexpr int DS_OFF = P_OFF + PD;
-  static constexpr int STG_OFF = DS_OFF + PD;        // fp32 staging for the dK / dV reduce: 2 x [128][32]
-  static constexpr int STG = 128 * DH * 4;
-  static constexpr int BAR_OFF = STG_OFF + STG;
-  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static constexpr int DS_OFF = P_OFF + BQ * BKV * 2;
+  static constexpr int BAR_OFF = DS_OFF + BQ * BKV * 2;
+  static constexpr int TOTAL = BAR_OFF + 256;        // 112 KB and the barriers: two CTAs per SM, without room to align the base
 };
 
 constexpr int SB_THREADS = 320;
 
-__global__ void __launch_bounds__(SB_THREADS, 1)
+template <bool DREM>
+__global__ void __launch_bounds__(SB_THREADS, 2)
 sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
-                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
-                   const __grid_constant__ CUtensorMap tmdK, const __grid_constant__ CUtensorMap tmdV, SbBwdParams p) {
+                   const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, SbBwdParams p) {
   using L = Smem;
   int head, doc, ti;
   if (!attn_tile(p.tile_offsets, p.nseq, p.H, true, head, doc, ti)) return;
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
   const int q0 = ti * BQ;
-  const int n_iter = ti + 1;  // key tiles ti, ti-1, ..., 0
+  const int n_iter = min((q0 + BQ) / BKV, (doc_len + BKV - 1) / BKV);  // key tiles n_iter - 1, ..., 0
 
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if (smem_u32(smem) & 1023) {  // the swizzled tiles need it
+    if (threadIdx.x == 0) report(p.status, ERR_BAD_ARG);
+    return;
+  }
   uint64_t* full_bar = (uint64_t*)(smem + L::BAR_OFF);
   uint64_t* empty_bar = full_bar + L::NSTAGE;
   uint64_t* q_full = empty_bar + L::NSTAGE;
   uint64_t* sdp_full = q_full + 1;
   uint64_t* pds_ready = sdp_full + 1;
-  uint64_t* dkv_full = pds_ready + 1;
+  uint64_t* dkv_full = pds_ready + 1;  // also: P and dS may be overwritten
   uint64_t* dkv_free = dkv_full + 1;
-  uint64_t* grp_bar = dkv_free + 1;
-  uint64_t* dq_full = grp_bar + 1;
+  uint64_t* dq_full = dkv_free + 1;
   uint32_t* tmem_slot = (uint32_t*)(dq_full + 1);
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
@@ -98,7 +106,6 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(pds_ready, 128);
     mbar_init(dkv_full, 1);
     mbar_init(dkv_free, 128);
-    mbar_init(grp_bar, 128);
     mbar_init(dq_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -106,93 +113,80 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     tma_prefetch_desc(&tmK);
     tma_prefetch_desc(&tmV);
     tma_prefetch_desc(&tmdO);
-    tma_prefetch_desc(&tmdK);
-    tma_prefetch_desc(&tmdV);
   }
+  for (int i = threadIdx.x; i < L::TILE / 16; i += SB_THREADS) reinterpret_cast<uint4*>(smem + L::ZERO_OFF)[i] = make_uint4(0u, 0u, 0u, 0u);
+  fence_async_smem();
   if (warp == 1) {
-    tmem_alloc(tmem_slot, 512);
+    tmem_alloc(tmem_slot, 256);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + 128, tmem_dV = tmem_base + 256, tmem_dK = tmem_base + 320,
-                 tmem_dQ = tmem_base + 384;
+  const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + 64, tmem_dKV = tmem_base + 128, tmem_dQ = tmem_base + 192;
 
   if (warp == 0) {
     if (lane == 0) {
       mbar_expect_tx(q_full, 2 * L::TILE);
       tma_load_3d(smem + L::Q_OFF, &tmQ, q_full, 0, head, doc_start + q0);
       tma_load_3d(smem + L::DO_OFF, &tmdO, q_full, 0, head, doc_start + q0);
-      bool ok = true;
-      for (int it = 0; it < n_iter && ok; ++it) {
+      for (int it = 0; it < n_iter; ++it) {
         const int stage = it % L::NSTAGE;
-        if (!mbar_wait(&empty_bar[stage], ((it / L::NSTAGE) & 1) ^ 1, p.status, abort_flag, ERR_WAIT_EMPTY)) { ok = false; break; }
-        const int j = ti - it;
+        if (!mbar_wait(&empty_bar[stage], ((it / L::NSTAGE) & 1) ^ 1, p.status, abort_flag, ERR_WAIT_EMPTY)) break;
+        const int row = doc_start + (n_iter - 1 - it) * BKV;
         uint8_t* dst = smem + L::RING_OFF + stage * L::STAGE;
         mbar_expect_tx(&full_bar[stage], L::STAGE);
-        tma_load_3d(dst, &tmK, &full_bar[stage], 0, head, doc_start + j * BKV);
-        tma_load_3d(dst + L::TILE, &tmV, &full_bar[stage], 0, head, doc_start + j * BKV);
+        tma_load_3d(dst, &tmK, &full_bar[stage], 0, head, row);
+        tma_load_3d(dst + L::KV, &tmV, &full_bar[stage], 0, head, row);
       }
     }
   } else if (warp == 1) {
     if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
-      constexpr uint32_t idesc_kv = make_idesc_bf16(BKV, DH, 1, 1);
+      constexpr uint32_t idesc_kv = make_idesc_bf16(2 * DH, BKV, 1, 1);
       constexpr uint32_t idesc_dq = make_idesc_bf16(BQ, DH, 0, 1);
       const uint32_t sQ = smem_u32(smem + L::Q_OFF), sdO = smem_u32(smem + L::DO_OFF);
       const uint32_t sP = smem_u32(smem + L::P_OFF), sDS = smem_u32(smem + L::DS_OFF);
-      bool ok = mbar_wait(q_full, 0, p.status, abort_flag, ERR_WAIT_FULL);
       auto issue_sdp = [&](int it) -> bool {
         const int stage = it % L::NSTAGE;
         if (!mbar_wait(&full_bar[stage], (it / L::NSTAGE) & 1, p.status, abort_flag, ERR_WAIT_FULL)) return false;
         tc_fence_after();
-        const uint32_t sK = smem_u32(smem + L::RING_OFF + stage * L::STAGE), sV = sK + L::TILE;
+        const uint32_t sK = smem_u32(smem + L::RING_OFF + stage * L::STAGE), sV = sK + L::KV;
         const uint64_t aq = make_smem_desc(sQ, 16, 1024), bk = make_smem_desc(sK, 16, 1024);
         const uint64_t ad = make_smem_desc(sdO, 16, 1024), bv = make_smem_desc(sV, 16, 1024);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) mma_ss(tmem_S, desc_advance(aq, k * 32), desc_advance(bk, k * 32), idesc_s, k ? 1u : 0u);
+        for (int k = 0; k < DH / 16; ++k) mma_ss(tmem_S, desc_advance(aq, k * 32), desc_advance(bk, k * 32), idesc_s, k ? 1u : 0u);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) mma_ss(tmem_dP, desc_advance(ad, k * 32), desc_advance(bv, k * 32), idesc_s, k ? 1u : 0u);
+        for (int k = 0; k < DH / 16; ++k) mma_ss(tmem_dP, desc_advance(ad, k * 32), desc_advance(bv, k * 32), idesc_s, k ? 1u : 0u);
         mma_commit(sdp_full);
         return true;
       };
+      bool ok = mbar_wait(q_full, 0, p.status, abort_flag, ERR_WAIT_FULL);
       if (ok) ok = issue_sdp(0);
       for (int it = 0; it < n_iter && ok; ++it) {
         const int stage = it % L::NSTAGE;
         const uint32_t sK = smem_u32(smem + L::RING_OFF + stage * L::STAGE);
-        if (!mbar_wait(pds_ready, it & 1, p.status, abort_flag, ERR_WAIT_MISC)) { ok = false; break; }
+        if (!mbar_wait(pds_ready, it & 1, p.status, abort_flag, ERR_WAIT_MISC)) break;
         tc_fence_after();
+        if (it + 1 < n_iter && !issue_sdp(it + 1)) break;
+        // dO | zeros and zeros | Q: 64-wide groups of the M dimension one tile apart
+        const uint64_t a_do = make_smem_desc(sdO, L::TILE, 1024), a_q = make_smem_desc(smem_u32(smem + L::ZERO_OFF), L::TILE, 1024);
+        const uint64_t bp = make_smem_desc(sP, 16, 1024), bds = make_smem_desc(sDS, 16, 1024);
+        const uint64_t ads = make_smem_desc(sDS, 16, 1024), bk = make_smem_desc(sK, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < BKV / 16; ++k) mma_ss(tmem_dQ, desc_advance(ads, k * 32), desc_advance(bk, k * 2048), idesc_dq, (it > 0 || k > 0) ? 1u : 0u);
         if (it > 0) {  // the previous tile's dK / dV must have left TMEM
-          if (!mbar_wait(dkv_free, (it - 1) & 1, p.status, abort_flag, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
+          if (!mbar_wait(dkv_free, (it - 1) & 1, p.status, abort_flag, ERR_WAIT_TMEM_EMPTY)) break;
           tc_fence_after();
         }
-        {
-          const uint64_t ap = make_smem_desc(sP, BQ * 128, 1024), ads = make_smem_desc(sDS, BQ * 128, 1024);
-          const uint64_t bdo = make_smem_desc(sdO, 16, 1024), bq = make_smem_desc(sQ, 16, 1024);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            mma_ss(tmem_dV, desc_advance(ap, k * 2048), desc_advance(bdo, k * 2048), idesc_kv, k ? 1u : 0u);
+        for (int k = 0; k < BQ / 16; ++k) mma_ss(tmem_dKV, desc_advance(a_do, k * 2048), desc_advance(bp, k * 2048), idesc_kv, k ? 1u : 0u);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)
-            mma_ss(tmem_dK, desc_advance(ads, k * 2048), desc_advance(bq, k * 2048), idesc_kv, k ? 1u : 0u);
-          const uint64_t bk = make_smem_desc(sK, 16, 1024);
-#pragma unroll
-          for (int kb = 0; kb < 2; ++kb) {
-            const uint64_t a2 = make_smem_desc(sDS + kb * (BQ * 128), 16, 1024);
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              mma_ss(tmem_dQ, desc_advance(a2, k * 32), desc_advance(bk, (kb * 4 + k) * 2048), idesc_dq,
-                     (it > 0 || kb > 0 || k > 0) ? 1u : 0u);
-          }
-        }
+        for (int k = 0; k < BQ / 16; ++k) mma_ss(tmem_dKV, desc_advance(a_q, k * 2048), desc_advance(bds, k * 2048), idesc_kv, 1u);
         mma_commit(&empty_bar[stage]);
         mma_commit(dkv_full);
         if (it + 1 == n_iter) mma_commit(dq_full);
-        if (it + 1 < n_iter) {
-          if (!issue_sdp(it + 1)) { ok = false; break; }
-        }
       }
     }
   } else if (warp < 6) {
@@ -207,55 +201,62 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const bool ragged = q0 + BQ > doc_len;
     const long long tok = (long long)doc_start + q_idx;
     const float tot = valid ? p.tot[(long long)head * p.total_tokens + tok] : 0.f;
-    const float drem = (valid && p.drem != nullptr) ? p.drem[(long long)head * p.total_tokens + tok] : 0.f;
+    const float drem = (DREM && valid) ? p.drem[(long long)head * p.total_tokens + tok] : 0.f;
+    const sb2 ndrem = sb_pk(-drem, -drem);
     float E = 1.f;  // product of (1 - sigma) over the keys already seen
     float R = 0.f;  // sum of dA over the keys already seen
     bool ok = true;
     for (int it = 0; it < n_iter && ok; ++it) {
-      const int j = ti - it;
-      const int kv0 = j * BKV;
-      const bool diag = (it == 0);
-      // the commit behind this barrier also covers the previous tile's products: P and dS may be overwritten
+      const int kv0 = (n_iter - 1 - it) * BKV;
+      const bool diag = kv0 + BKV > q0;
       if (!mbar_wait_warp(sdp_full, it & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-#pragma unroll 1
-      for (int c0 = BKV - 32; c0 >= 0; c0 -= 32) {
-        uint32_t xr[32], dr[32];
-        tmem_ld_32x32(tmem_S + lane_sel + c0, xr);
-        tmem_ld_32x32(tmem_dP + lane_sel + c0, dr);
+      uint32_t xr[2][8], dr[2][8];  // a group's logits and dP, the next group's on their way
+      tmem_ld_32x8(tmem_S + lane_sel + BKV - 8, xr[0]);
+      tmem_ld_32x8(tmem_dP + lane_sel + BKV - 8, dr[0]);
+      // the previous tile's products have read P and dS
+      if (it > 0 && !mbar_wait_warp(dkv_full, (it - 1) & 1, p.status, abort_flag, ERR_WAIT_MISC)) { ok = false; break; }
+#pragma unroll 2
+      for (int g = 0; g < BKV / 8; ++g) {
+        const int c = BKV - 8 - g * 8;
         tmem_ld_wait();
-#pragma unroll
-        for (int c = 24; c >= 0; c -= 8) {
-          float sig[8], a[8], d[8];
-          uint32_t dead = 0u;
-          if (diag || ragged) {
-            dead = sb_dead_bits(!valid, diag, kv0 + c0 + c, q_idx);
-            sb_group<true>(xr + c, p.scale_log2, dead, E, sig, a);
-#pragma unroll
-            for (int i = 0; i < 8; ++i)  // what stands in another document's rows does not count, whatever it is
-              if ((dead >> i) & 1u) dr[c + i] = 0u;
-          }
-          else sb_group<false>(xr + c, p.scale_log2, 0u, E, sig, a);
-          uint4 q;
-          q.x = pack_bf16(a[0], a[1]); q.y = pack_bf16(a[2], a[3]); q.z = pack_bf16(a[4], a[5]); q.w = pack_bf16(a[6], a[7]);
-          // The forward formed o from the bf16 rounding of att, and tot = do . o is the total the running sum R has to
-          // meet exactly at the end of the walk: the same rounded weight enters dA here (the remainder term keeps the
-          // fp32 weight, as rem was formed from it).  With fp32 att in this place the mismatch of the two roundings,
-          // multiplied by sigma for every key of the row, was a 20 % error in dq at 4096-token rows.
-          const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-          for (int i = 7; i >= 0; --i) {
-            const float att16 = __uint_as_float((i & 1) ? (qw[i >> 1] & 0xffff0000u) : (qw[i >> 1] << 16));
-            const float dA = att16 * __uint_as_float(dr[c + i]) - a[i] * drem;  // zero for keys that do not count
-            d[i] = dA - sig[i] * (tot - R);
-            R += dA;
-          }
-          const int cc = c0 + c;
-          const uint32_t off = (cc >> 6) * (BQ * 128) + sw128_offset(r, cc & 63);
-          *reinterpret_cast<uint4*>(sP + off) = q;
-          q.x = pack_bf16(d[0], d[1]); q.y = pack_bf16(d[2], d[3]); q.z = pack_bf16(d[4], d[5]); q.w = pack_bf16(d[6], d[7]);
-          *reinterpret_cast<uint4*>(sDS + off) = q;
+        uint32_t(&x)[8] = xr[g & 1];
+        uint32_t(&dp)[8] = dr[g & 1];
+        if (c > 0) {
+          tmem_ld_32x8(tmem_S + lane_sel + c - 8, xr[(g & 1) ^ 1]);
+          tmem_ld_32x8(tmem_dP + lane_sel + c - 8, dr[(g & 1) ^ 1]);
         }
+        sb2 nsig[4], a[4], d[4];
+        if (diag || ragged) {
+          const uint32_t dead = sb_dead_bits(!valid, diag, kv0 + c, q_idx);
+          sb_group<true>(x, p.scale_log2, dead, E, nsig, a);
+#pragma unroll
+          for (int i = 0; i < 8; ++i)  // what stands in another document's rows does not count, whatever it is
+            if ((dead >> i) & 1u) dp[i] = 0u;
+        } else {
+          sb_group<false>(x, p.scale_log2, 0u, E, nsig, a);
+        }
+        const uint4 q = make_uint4(sb_pack(a[0]), sb_pack(a[1]), sb_pack(a[2]), sb_pack(a[3]));
+        // The forward formed o from the bf16 rounding of att, and tot = do . o is the total the running sum of dA has to
+        // meet exactly at the end of the walk: the same rounded weight enters dA here (the remainder term keeps the
+        // fp32 weight, as rem was formed from it).  With fp32 att in this place the mismatch of the two roundings,
+        // multiplied by sigma for every key of the row, was a 20 % error in dq at 4096-token rows.
+        const uint32_t qw[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int i = 3; i >= 0; --i) {  // dA is zero for keys that do not count
+          const sb2 att16 = sb_pk(__uint_as_float(qw[i] << 16), __uint_as_float(qw[i] & 0xffff0000u));
+          sb2 dA = sb_mul2(att16, sb_pk(__uint_as_float(dp[2 * i]), __uint_as_float(dp[2 * i + 1])));
+          if (DREM) dA = sb_fma2(a[i], ndrem, dA);
+          float dA0, dA1;
+          sb_up(dA, dA0, dA1);
+          const float R1 = R;
+          R += dA1;
+          d[i] = sb_fma2(nsig[i], sb_pk(tot - R, tot - R1), dA);
+          R += dA0;
+        }
+        const uint32_t off = sw128_offset(r, c);
+        *reinterpret_cast<uint4*>(sP + off) = q;
+        *reinterpret_cast<uint4*>(sDS + off) = make_uint4(sb_pack(d[0]), sb_pack(d[1]), sb_pack(d[2]), sb_pack(d[3]));
       }
       tc_fence_before();
       fence_async_smem();
@@ -285,61 +286,39 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
     }
   } else {
-    // ------------------------------------------------------------------ dV and dK of every tile
+    // ------------------------------------------------------------------ dV and dK of every tile: a lane is one channel
     const int quarter = warp & 3;
-    const int r = quarter * 32 + lane;
     const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
-    uint8_t* sSTG = smem + L::STG_OFF;
-    const bool issuer = (warp == 6 && lane == 0);
-    bool ok = true;
-    uint32_t grp_phase = 0;
-    auto group_sync = [&]() -> bool {
-      mbar_arrive(grp_bar);
-      const bool done = mbar_wait_warp(grp_bar, grp_phase, p.status, abort_flag, ERR_WAIT_MISC);
-      grp_phase ^= 1;
-      return done;
-    };
-    // adds one [128 keys][64] fp32 tile (TMEM columns at `taddr`, scaled) to the global accumulator behind `tm`
-    auto flush_tile = [&](uint32_t taddr, const CUtensorMap* tm, float mul, int row0) -> bool {
-      if (issuer) tma_store_wait_read<0>();
-      if (!group_sync()) return false;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t v[32];
-        tmem_ld_32x32(taddr + lane_sel + half * 32, v);
-        tmem_ld_wait();
-#pragma unroll
-        for (int g = 0; g < 8; ++g) {
-          float4 q = make_float4(__uint_as_float(v[g * 4 + 0]) * mul, __uint_as_float(v[g * 4 + 1]) * mul,
-                                 __uint_as_float(v[g * 4 + 2]) * mul, __uint_as_float(v[g * 4 + 3]) * mul);
-          *reinterpret_cast<float4*>(sSTG + half * (128 * 128) + r * 128 + ((g ^ (r & 7)) << 4)) = q;
-        }
-      }
-      fence_async_smem();
-      if (!group_sync()) return false;
-      if (issuer) {
-        tma_reduce_add_3d(tm, sSTG, 0, head, row0);
-        tma_reduce_add_3d(tm, sSTG + 128 * 128, 32, head, row0);
-        tma_store_commit();
-      }
-      return true;
-    };
-    for (int it = 0; it < n_iter && ok; ++it) {
-      const int kv0 = (ti - it) * BKV;
-      if (!mbar_wait_warp(dkv_full, it & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+    const long long row = (long long)p.H * DH;
+    float* out = (quarter < 2 ? p.dV : p.dK) + (long long)doc_start * row + head * DH + (quarter & 1) * 32 + lane;
+    const float mul = quarter < 2 ? 1.f : p.scale;
+    for (int it = 0; it < n_iter; ++it) {
+      const int kv0 = (n_iter - 1 - it) * BKV;
+      if (!mbar_wait_warp(dkv_full, it & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) break;
       tc_fence_after();
-      if (!flush_tile(tmem_dV, &tmdV, 1.f, doc_start + kv0)) { ok = false; break; }
-      if (!flush_tile(tmem_dK, &tmdK, p.scale, doc_start + kv0)) { ok = false; break; }
+      uint32_t v[2][32];
+      tmem_ld_32x32(tmem_dKV + lane_sel, v[0]);
+      tmem_ld_32x32(tmem_dKV + lane_sel + 32, v[1]);
+      tmem_ld_wait();
       tc_fence_before();
       mbar_arrive(dkv_free);
+      float* dst = out + kv0 * row;
+      const int n = min(BKV, doc_len - kv0);  // keys of the document
+      if (n == BKV) {
+#pragma unroll
+        for (int c = 0; c < BKV; ++c) atomicAdd(dst + c * row, __uint_as_float(v[c / 32][c % 32]) * mul);
+      } else {
+#pragma unroll
+        for (int c = 0; c < BKV; ++c)
+          if (c < n) atomicAdd(dst + c * row, __uint_as_float(v[c / 32][c % 32]) * mul);
+      }
     }
-    if (issuer) tma_store_wait_all<0>();
   }
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, 256);
   }
 }
 
@@ -391,7 +370,7 @@ __global__ void sb_tot_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bf
 
 extern "C" {
 
-// dk_acc, dv_acc: fp32 [T, H, 64], zero on entry (reduced into with TMA adds); dq: bf16 [T, H, 64] (token stride given).
+// dk_acc, dv_acc: fp32 [T, H, 64], zero on entry (added to); dq: bf16 [T, H, 64] (token stride given).
 // tot: fp32 [H, T] scratch.  rem: fp32 [H, T] from the forward; drem may be null.  o_lo: the forward's second output
 // (bf16 [T, H, 64], contiguous) or null.
 int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* o_lo, const void* dout, const float* rem,
@@ -410,16 +389,14 @@ int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
     int rc = fb::launch_ok("sb_tot_kernel");
     if (rc) return rc;
   }
-  CUtensorMap tmQ, tmK, tmV, tmdO, tmdK, tmdV;
-  auto qkv_map = [&](CUtensorMap* m, const void* base, long long stride) {
-    return fb::make_tmap_3d(m, base, 2, (uint64_t)T, (uint64_t)H, (uint64_t)DH, (uint64_t)stride, (uint64_t)DH, 128, 1, 64, true);
+  CUtensorMap tmQ, tmK, tmV, tmdO;
+  auto map = [&](CUtensorMap* m, const void* base, long long stride, uint32_t rows) {
+    return fb::make_tmap_3d(m, base, 2, (uint64_t)T, (uint64_t)H, (uint64_t)DH, (uint64_t)stride, (uint64_t)DH, rows, 1, 64, true);
   };
-  int rc = qkv_map(&tmQ, q, q_stride_t);
-  if (!rc) rc = qkv_map(&tmK, k, k_stride_t);
-  if (!rc) rc = qkv_map(&tmV, v, v_stride_t);
-  if (!rc) rc = qkv_map(&tmdO, dout, do_stride_t);
-  if (!rc) rc = fb::make_tmap_3d(&tmdK, dk_acc, 4, (uint64_t)T, (uint64_t)H, (uint64_t)DH, (uint64_t)H * DH, (uint64_t)DH, 128, 1, 32, true);
-  if (!rc) rc = fb::make_tmap_3d(&tmdV, dv_acc, 4, (uint64_t)T, (uint64_t)H, (uint64_t)DH, (uint64_t)H * DH, (uint64_t)DH, 128, 1, 32, true);
+  int rc = map(&tmQ, q, q_stride_t, BQ);
+  if (!rc) rc = map(&tmK, k, k_stride_t, BKV);
+  if (!rc) rc = map(&tmV, v, v_stride_t, BKV);
+  if (!rc) rc = map(&tmdO, dout, do_stride_t, BQ);
   if (rc) return rc;
   SbBwdParams p;
   p.cu_seqlens = cu_seqlens;
@@ -431,17 +408,18 @@ int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
   p.scale_log2 = scale * kLog2e;
   p.tot = tot;
   p.drem = drem;
+  p.dK = dk_acc, p.dV = dv_acc;
   p.dQ = (__nv_bfloat16*)dq;
   p.dq_stride_t = dq_stride_t;
   p.status = fb::status_ptr();
-  static bool done = false;
-  if (!done) {
-    cudaError_t e = cudaFuncSetAttribute(sb_attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
+  auto launch = [&](auto kernel) -> int {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem::TOTAL);
     if (e != cudaSuccess) return (int)e;
-    done = true;
-  }
-  const unsigned grid = (unsigned)max_tiles * H;
-  sb_attn_bwd_kernel<<<grid, SB_THREADS, Smem::TOTAL, stream>>>(tmQ, tmK, tmV, tmdO, tmdK, tmdV, p);
+    kernel<<<(unsigned)max_tiles * H, SB_THREADS, Smem::TOTAL, stream>>>(tmQ, tmK, tmV, tmdO, p);
+    return 0;
+  };
+  rc = drem != nullptr ? launch(sb_attn_bwd_kernel<true>) : launch(sb_attn_bwd_kernel<false>);
+  if (rc) return rc;
   return fb::launch_ok("sb_attn_bwd_kernel");
 }
 

@@ -9,29 +9,80 @@
 // multiplication per group (one per key, behind a correctly rounded reciprocal subroutine, held the softmax warps up before).
 // The reciprocal is the hardware approximation and one Newton step: against fp64 the remainder's mean error is that of the
 // correctly rounded one (4.87e-7 both at 512 keys, 4.84e-7 and 4.81e-7 at 4,096).
+//
+// Two keys share an instruction wherever there is a packed one.  It has no negation, so the reciprocal is formed with its sign
+// turned, m = -1 / (1 + t): then 1 + y m is the Newton residual, t m = -sigma, and the sign of the product over k keys, (-1)^k,
+// is put right by the pair (E, -E).
 #pragma once
 #include <stdint.h>
+#include "tc05.cuh"
 
+typedef unsigned long long sb2;  // two fp32 values, the lower key in the lower half
+__device__ __forceinline__ sb2 sb_pk(float a, float b) {
+  sb2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void sb_up(sb2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ sb2 sb_mul2(sb2 a, sb2 b) {
+  sb2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ sb2 sb_add2(sb2 a, sb2 b) {
+  sb2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ sb2 sb_fma2(sb2 a, sb2 b, sb2 c) {
+  sb2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint32_t sb_pack(sb2 v) {  // bf16
+  float a, b;
+  sb_up(v, a, b);
+  return tc05::pack_bf16(a, b);
+}
+
+// nsig: -sigma, att: the weights; [i] holds keys 2 i and 2 i + 1
 template <bool MASK>
-__device__ __forceinline__ void sb_group(const uint32_t* x8, float scale_log2, uint32_t dead, float& E, float (&sig)[8], float (&att)[8]) {
-  float inv[8];
+__device__ __forceinline__ void sb_group(const uint32_t* x8, float scale_log2, uint32_t dead, float& E, sb2 (&nsig)[4], sb2 (&att)[4]) {
+  const sb2 one = sb_pk(1.f, 1.f), scale = sb_pk(scale_log2, scale_log2);
+  float ninv[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const float x = fminf(fmaxf(__uint_as_float(x8[i]) * scale_log2, -100.f), 100.f);
-    float t, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x));
-    const float y = 1.f + t;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
-    r = fmaf(r, fmaf(-y, r, 1.f), r);
-    const bool gone = MASK && ((dead >> i) & 1u);
-    inv[i] = gone ? 1.f : r;
-    sig[i] = gone ? 0.f : t * r;
+  for (int i = 0; i < 4; ++i) {
+    float x0, x1, t0, t1, y0, y1, m0, m1;
+    sb_up(sb_mul2(sb_pk(__uint_as_float(x8[2 * i]), __uint_as_float(x8[2 * i + 1])), scale), x0, x1);
+    x0 = fminf(fmaxf(x0, -100.f), 100.f);
+    x1 = fminf(fmaxf(x1, -100.f), 100.f);
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(x0));
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(x1));
+    const sb2 t = sb_pk(t0, t1), y = sb_add2(t, one);
+    sb_up(y, y0, y1);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(m0) : "f"(-y0));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(m1) : "f"(-y1));
+    sb2 m = sb_pk(m0, m1);
+    m = sb_fma2(m, sb_fma2(y, m, one), m);
+    nsig[i] = sb_mul2(t, m);
+    sb_up(m, ninv[2 * i], ninv[2 * i + 1]);
+    if (MASK) {
+      float s0, s1;
+      sb_up(nsig[i], s0, s1);
+      const bool gone0 = (dead >> (2 * i)) & 1u, gone1 = (dead >> (2 * i + 1)) & 1u;
+      nsig[i] = sb_pk(gone0 ? 0.f : s0, gone1 ? 0.f : s1);
+      ninv[2 * i] = gone0 ? -1.f : ninv[2 * i];
+      ninv[2 * i + 1] = gone1 ? -1.f : ninv[2 * i + 1];
+    }
   }
+  const sb2 e2 = sb_pk(E, -E);
   float p = 1.f;
 #pragma unroll
-  for (int i = 7; i >= 0; --i) {
-    att[i] = (sig[i] * p) * E;
-    p *= inv[i];
+  for (int i = 3; i >= 0; --i) {
+    const float p1 = p;
+    p *= ninv[2 * i + 1];
+    att[i] = sb_mul2(sb_mul2(nsig[i], sb_pk(p, p1)), e2);
+    p *= ninv[2 * i];
   }
   E *= p;
 }
