@@ -200,6 +200,87 @@ __global__ void colsum_rows_kernel(const float* __restrict__ part, int parts, in
 }
 
 // ---------------------------------------------------------------------------------------------------------------
+// The delta rule's gates (fla/layers/delta_net.py:246-252, fla/ops/gated_delta_rule/gate.py:20-44), per token and head:
+//   beta = mul sigmoid(b),   g = -exp(A_log) softplus(a + dt_bias)
+// read from column blocks of the projection and written as fp32 in the padded rows of the chunk layout (zeros in the
+// padding).  A few scalars per token: what they cost is launches, so one kernel stands for ten of torch's forward and one
+// (and the sum of its partials) for fifteen backward.  src: packed token of a padded row (-1: padding), or null: the same.
+template <bool BF16>
+__device__ __forceinline__ float param(const void* p, int h) {
+  return BF16 ? __bfloat162float(((const __nv_bfloat16*)p)[h]) : ((const float*)p)[h];
+}
+// the exponential never overflows, and its logarithm does not round 1 + exp first
+__device__ __forceinline__ float softplus_exact(float x) { return fmaxf(x, 0.f) + log1pf(__expf(-fabsf(x))); }
+
+template <bool BF16>
+__global__ void delta_gates_fwd_kernel(const __nv_bfloat16* __restrict__ b, long long ldb, const __nv_bfloat16* __restrict__ a, long long lda,
+                                       const void* __restrict__ A_log, const void* __restrict__ dt_bias, const int* __restrict__ src,
+                                       long long rows, int H, float mul, float* __restrict__ beta, float* __restrict__ g) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= rows * H) return;
+  const long long r = i / H;
+  const int h = (int)(i - r * H);
+  const long long t = src == nullptr ? r : src[r];
+  float be = 0.f, ge = 0.f;
+  if (t >= 0) {
+    be = mul * sigmoidf_(__bfloat162float(b[t * ldb + h]));
+    if (a != nullptr) ge = -__expf(param<BF16>(A_log, h)) * softplus_exact(__bfloat162float(a[t * lda + h]) + param<BF16>(dt_bias, h));
+  }
+  beta[i] = be;
+  if (a != nullptr) g[i] = ge;
+}
+
+// db, da at their packed rows; part [blocks][2][H]: sums of dg g (for A_log) and of da (for dt_bias)
+constexpr int DG_THREADS = 256, DG_MAXH = 128;
+template <bool BF16>
+__global__ void __launch_bounds__(DG_THREADS) delta_gates_bwd_kernel(
+    const __nv_bfloat16* __restrict__ b, long long ldb, const __nv_bfloat16* __restrict__ a, long long lda, const void* __restrict__ A_log,
+    const void* __restrict__ dt_bias, const int* __restrict__ src, long long rows, int H, float mul, const float* __restrict__ dbeta,
+    const float* __restrict__ dg, __nv_bfloat16* __restrict__ db, long long lddb, __nv_bfloat16* __restrict__ da, long long ldda,
+    float* __restrict__ part) {
+  __shared__ float red[2][DG_THREADS];
+  const int per = DG_THREADS / H;  // rows of the block at a time
+  const int h = threadIdx.x % H, slot = threadIdx.x / H;
+  float sA = 0.f, sdt = 0.f;
+  if (slot < per) {
+    const float nA = a == nullptr ? 0.f : -__expf(param<BF16>(A_log, h)), dt = a == nullptr ? 0.f : param<BF16>(dt_bias, h);
+    for (long long r = (long long)blockIdx.x * per + slot; r < rows; r += (long long)gridDim.x * per) {
+      const long long t = src == nullptr ? r : src[r];
+      if (t < 0) continue;
+      const float s = sigmoidf_(__bfloat162float(b[t * ldb + h]));
+      db[t * lddb + h] = __float2bfloat16(dbeta[r * H + h] * mul * s * (1.f - s));
+      if (a != nullptr) {
+        const float x = __bfloat162float(a[t * lda + h]) + dt, d = dg[r * H + h];
+        const float v = d * nA * sigmoidf_(x);
+        da[t * ldda + h] = __float2bfloat16(v);
+        sA = fmaf(d, nA * softplus_exact(x), sA);
+        sdt += v;
+      }
+    }
+  }
+  if (a == nullptr) return;
+  red[0][threadIdx.x] = sA;
+  red[1][threadIdx.x] = sdt;
+  __syncthreads();
+  if (threadIdx.x < 2 * H) {
+    const int which = threadIdx.x / H, hh = threadIdx.x % H;
+    float v = 0.f;
+    for (int k = 0; k < per; ++k) v += red[which][k * H + hh];
+    part[(long long)blockIdx.x * 2 * H + threadIdx.x] = v;
+  }
+}
+__global__ void delta_gates_sum_kernel(const float* __restrict__ part, int blocks, int H, float* __restrict__ dA, float* __restrict__ ddt, int accumulate) {
+  const int i = blockIdx.x, lane = threadIdx.x;  // one warp per value
+  float v = 0.f;
+  for (int k = lane; k < blocks; k += 32) v += part[(long long)k * 2 * H + i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if (lane != 0) return;
+  float* to = i < H ? dA + i : ddt + (i - H);
+  *to = accumulate ? *to + v : v;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
 // Mamba2 (fla/layers/mamba2.py:241-331): the elementwise work around the SSD core, H heads of P channels.
 //   pre :  dt = softplus(dt_raw + dt_bias),  g = -exp(A_log) dt,  xv = x dt                 (x, dt_raw: strided views)
 //   post:  out = (y + D x) silu(z)                                                           (z: strided view)
@@ -328,6 +409,37 @@ __global__ void mamba2_post_bwd_kernel(const __nv_bfloat16* __restrict__ y, cons
 }  // namespace
 
 extern "C" {
+
+int fb_delta_gates_blocks(long long rows, int H) {
+  const long long per = DG_THREADS / H, n = (rows + per * 8 - 1) / (per * 8);
+  return (int)(n < 1 ? 1 : n > 592 ? 592 : n);
+}
+// a, g null: beta alone.  bf16: A_log and dt_bias are bf16, else fp32.  H up to DG_MAXH.
+int fb_delta_gates_fwd(const void* b, long long ldb, const void* a, long long lda, const void* A_log, const void* dt_bias, int bf16, const int* src,
+                       long long rows, int H, float mul, float* beta, float* g, cudaStream_t stream) {
+  if (rows == 0) return 0;
+  if (H < 1 || H > DG_MAXH) return -2;
+  const unsigned grid = (unsigned)((rows * H + 255) / 256);
+  const auto kernel = bf16 ? delta_gates_fwd_kernel<true> : delta_gates_fwd_kernel<false>;
+  kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)b, ldb, (const __nv_bfloat16*)a, lda, A_log, dt_bias, src, rows, H, mul, beta, g);
+  return fb::launch_ok("delta_gates_fwd_kernel");
+}
+// part: fp32 [fb_delta_gates_blocks(rows, H), 2, H] scratch; dA, ddt: fp32 [H], added to with `accumulate`
+int fb_delta_gates_bwd(const void* b, long long ldb, const void* a, long long lda, const void* A_log, const void* dt_bias, int bf16, const int* src,
+                       long long rows, int H, float mul, const float* dbeta, const float* dg, void* db, long long lddb, void* da, long long ldda,
+                       float* part, float* dA, float* ddt, int accumulate, cudaStream_t stream) {
+  if (rows == 0) return 0;
+  if (H < 1 || H > DG_MAXH) return -2;
+  const int blocks = fb_delta_gates_blocks(rows, H);
+  const auto kernel = bf16 ? delta_gates_bwd_kernel<true> : delta_gates_bwd_kernel<false>;
+  kernel<<<blocks, DG_THREADS, 0, stream>>>((const __nv_bfloat16*)b, ldb, (const __nv_bfloat16*)a, lda, A_log, dt_bias, src, rows, H, mul, dbeta, dg,
+                                            (__nv_bfloat16*)db, lddb, (__nv_bfloat16*)da, ldda, part);
+  int rc = fb::launch_ok("delta_gates_bwd_kernel");
+  if (rc || a == nullptr) return rc;
+  delta_gates_sum_kernel<<<2 * H, 32, 0, stream>>>(part, blocks, H, dA, ddt, accumulate);
+  return fb::launch_ok("delta_gates_sum_kernel");
+}
+
 
 // x: bf16 [T, H * P] view with row stride ldx (elements); dt_raw: bf16 [T, H] view with row stride ld_dt; dt_bias, A_log: fp32 [H]
 // xv: bf16 [T, H, P]; dt, g: fp32 [T, H].  P in {64, 128, 256}; ldx a multiple of 8, x 16-byte aligned.

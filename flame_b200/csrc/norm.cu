@@ -40,18 +40,38 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
 }
 __device__ __forceinline__ float sigmoidf_(float x) { return 1.f / (1.f + __expf(-x)); }
 
+// Where rows lie.  A row is one head of a token.  `map`: the normalised tensor is in the chunk layout of the linear-attention kernels
+// (padded rows), everything else in packed rows: forward map[token] = padded row, backward map[padded row] = token or -1.  The
+// gate may be a column block of a wider matrix: `ldg` elements from token to token (`lddg`: its gradient's).
+struct Rows {
+  const int* map;
+  unsigned heads;
+  long long ldg, lddg;
+};
+__device__ __forceinline__ long long mapped_row(const Rows& rs, long long row) {  // -1: padding
+  if (rs.map == nullptr) return row;
+  const unsigned t = (unsigned)row / rs.heads;
+  const int to = rs.map[t];
+  return to < 0 ? -1 : (long long)to * rs.heads + ((unsigned)row - t * rs.heads);
+}
+__device__ __forceinline__ long long gate_at(unsigned heads, long long ld, long long row, int D) {
+  if (ld == (long long)heads * D) return row * D;
+  const unsigned t = (unsigned)row / heads;
+  return t * ld + (long long)((unsigned)row - t * heads) * D;
+}
+
 // gate_mode: 0 none, 1 swish (g * sigmoid(g)), 2 sigmoid
 template <bool HAS_RES, bool WRITE_RES, int GATE>
 __global__ void __launch_bounds__(WARPS * 32)
 rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in,
                    const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ gate,
                    __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out, float* __restrict__ rstd,
-                   long long rows, int D, float eps) {
+                   long long rows, int D, float eps, const Rows at) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long long row = (long long)blockIdx.x * WARPS + warp;
   if (row >= rows) return;
   const int nvec = D >> 3;
-  const uint4* xr = reinterpret_cast<const uint4*>(x + row * D);
+  const uint4* xr = reinterpret_cast<const uint4*>(x + mapped_row(at, row) * D);
   const uint4* rr = HAS_RES ? reinterpret_cast<const uint4*>(res_in + row * D) : nullptr;
   uint4* ro = WRITE_RES ? reinterpret_cast<uint4*>(res_out + row * D) : nullptr;
   float ss = 0.f;
@@ -77,7 +97,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   if (lane == 0 && rstd != nullptr) rstd[row] = rs;
   const uint4* src = WRITE_RES ? reinterpret_cast<const uint4*>(res_out + row * D) : xr;
   const uint4* wv = reinterpret_cast<const uint4*>(w);
-  const uint4* gv = GATE ? reinterpret_cast<const uint4*>(gate + row * D) : nullptr;
+  const uint4* gv = GATE ? reinterpret_cast<const uint4*>(gate + gate_at(at.heads, at.ldg, row, D)) : nullptr;
   uint4* yo = reinterpret_cast<uint4*>(y + row * D);
   for (int i = lane; i < nvec; i += 32) {
     float a[8], ww[8];
@@ -110,7 +130,7 @@ template <bool HAS_RES, bool WRITE_RES, int GATE, int LPR>
 __global__ void __launch_bounds__(WARPS * 32)
 rmsnorm_fwd_short_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in, const __nv_bfloat16* __restrict__ w,
                          const __nv_bfloat16* __restrict__ gate, __nv_bfloat16* __restrict__ y, __nv_bfloat16* __restrict__ res_out,
-                         float* __restrict__ rstd, long long rows, int D, float eps) {
+                         float* __restrict__ rstd, long long rows, int D, float eps, const Rows at) {
   constexpr int SLOTS = WARPS * 32 / LPR;
   const int l = threadIdx.x % LPR, col = l * 8;
   const bool live = col < D;
@@ -124,9 +144,9 @@ rmsnorm_fwd_short_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
   for (int k = 0; k < FR; ++k) {
     const long long row = r0 + k * SLOTS;
     const bool ok = live && row < rows;
-    xa[k] = ok ? *reinterpret_cast<const uint4*>(x + row * D + col) : make_uint4(0, 0, 0, 0);
+    xa[k] = ok ? *reinterpret_cast<const uint4*>(x + mapped_row(at, row) * D + col) : make_uint4(0, 0, 0, 0);
     if (HAS_RES) ra[k] = ok ? *reinterpret_cast<const uint4*>(res_in + row * D + col) : make_uint4(0, 0, 0, 0);
-    if (GATE) ta[k] = ok ? *reinterpret_cast<const uint4*>(gate + row * D + col) : make_uint4(0, 0, 0, 0);
+    if (GATE) ta[k] = ok ? *reinterpret_cast<const uint4*>(gate + gate_at(at.heads, at.ldg, row, D) + col) : make_uint4(0, 0, 0, 0);
   }
 #pragma unroll
   for (int k = 0; k < FR; ++k) {
@@ -171,12 +191,12 @@ rmsnorm_fwd_short_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 // stay packed in registers, so every operand is read once and enough bytes are in flight to be bound by DRAM; one warp
 // per row, as before, kept one row's loads in flight and re-read D > 1024 and D < 256 through L1 (D = 128, 524,288 rows: 0.28 ms;
 // D = 2048, 32,768 rows: 0.24 ms; both 1.6 TB/s).  dw partials: one row per CTA, which a second kernel sums in order.
-template <bool HAS_DRES, int GATE, int LPR, int BR, int TPB>
+template <bool HAS_DRES, int GATE, int LPR, int BR, int TPB, bool MAP>
 __global__ void __launch_bounds__(TPB, TPB == 256 ? 2 : 1)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ xin, const __nv_bfloat16* __restrict__ w,
                    const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ dres,
                    __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dgate, float* __restrict__ dw_part, long long rows, int D,
-                   int rows_per_cta) {
+                   int rows_per_cta, const Rows at) {
   constexpr int SLOTS = LPR ? WARPS * 32 / (LPR ? LPR : 1) : 1;
   __shared__ float s_c[LPR ? 1 : 2][LPR ? 1 : BR][LPR ? 1 : 32];
   __shared__ float s_dw[LPR ? SLOTS : 1][LPR ? LPR * 8 + 1 : 1];
@@ -194,17 +214,23 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   for (long long rb = row0; rb < row1; rb += SLOTS * BR, flip ^= 1) {
     uint4 xa[BR], ga[BR], ra[HAS_DRES ? BR : 1], ta[GATE ? BR : 1];
     float rs[BR], c[BR];
+    int from[MAP ? BR : 1];  // the packed row, -1 where there is none: its gradient is zero
 #pragma unroll
     for (int k = 0; k < BR; ++k) {
       const long long row = rb + slot + k * SLOTS;
-      const bool ok = live && row < row1;
+      if (MAP) from[k] = row < row1 ? (int)mapped_row(at, row) : -1;
+    }
+#pragma unroll
+    for (int k = 0; k < BR; ++k) {
+      const long long row = rb + slot + k * SLOTS, pr = MAP ? from[k] : row;
+      const bool there = MAP ? pr >= 0 : row < row1, ok = live && there;
       // streaming loads: every operand row is read exactly once
       const uint4 none = make_uint4(0, 0, 0, 0);
       xa[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(xin + row * D + col)) : none;
-      ga[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(dy + row * D + col)) : none;
-      if (HAS_DRES) ra[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(dres + row * D + col)) : none;
-      if (GATE) ta[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(gate + row * D + col)) : none;
-      rs[k] = row < row1 ? rstd[row] : 0.f;
+      ga[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(dy + pr * D + col)) : none;
+      if (HAS_DRES) ra[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(dres + pr * D + col)) : none;
+      if (GATE) ta[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(gate + gate_at(at.heads, at.ldg, pr, D) + col)) : none;
+      rs[k] = there ? rstd[pr] : 0.f;
     }
 #pragma unroll
     for (int k = 0; k < BR; ++k) {
@@ -276,7 +302,8 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
       }
       if (live && row < row1) {
         __stcs(reinterpret_cast<uint4*>(dx + row * D + col), pack8(o));
-        if (GATE) __stcs(reinterpret_cast<uint4*>(dgate + row * D + col), pack8(dgo));
+        if (GATE && (!MAP || from[k] >= 0))
+          __stcs(reinterpret_cast<uint4*>(dgate + gate_at(at.heads, at.lddg, MAP ? from[k] : row, D) + col), pack8(dgo));
       }
     }
   }
@@ -328,10 +355,12 @@ int fb_rmsnorm_bwd_parts(long long rows) {
   return (int)(want < 592 ? (want < 1 ? 1 : want) : 592);  // two resident CTAs on each of 148 SMs: two full waves
 }
 
+// map, heads, ldg (0: the gate's rows are side by side): see Rows
 int fb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, const void* gate, void* y, void* res_out,
-                   float* rstd, long long rows, int D, float eps, int gate_mode, cudaStream_t stream) {
+                   float* rstd, long long rows, int D, float eps, int gate_mode, const int* map, int heads, long long ldg, cudaStream_t stream) {
   if (rows == 0) return 0;
-  if (D % 8) return -2;
+  if (D % 8 || heads < 1 || rows % heads || ldg % 8 || (rows >= (1ll << 31) && (map || ldg))) return -2;
+  const Rows at{map, (unsigned)heads, ldg ? ldg : (long long)heads * D, 0};
   const int lpr = D <= 64 ? 8 : D <= 128 ? 16 : 32;  // lanes of a row, D <= 256
   const int per_block = D <= 256 ? WARPS * 32 / lpr * FR : WARPS;
   const unsigned grid = (unsigned)((rows + per_block - 1) / per_block);
@@ -342,13 +371,13 @@ int fb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, const void*
   auto Y = (__nv_bfloat16*)y;
   auto RO = (__nv_bfloat16*)res_out;
 #define FWD_S(HR, WR, GM, LP) \
-  rmsnorm_fwd_short_kernel<HR, WR, GM, LP><<<grid, WARPS * 32, 0, stream>>>(X, R, W, G, Y, RO, rstd, rows, D, eps)
+  rmsnorm_fwd_short_kernel<HR, WR, GM, LP><<<grid, WARPS * 32, 0, stream>>>(X, R, W, G, Y, RO, rstd, rows, D, eps, at)
 #define FWD(HR, WR, GM)                                                                                            \
   do {                                                                                                             \
     if (D <= 64) FWD_S(HR, WR, GM, 8);                                                                             \
     else if (D <= 128) FWD_S(HR, WR, GM, 16);                                                                      \
     else if (D <= 256) FWD_S(HR, WR, GM, 32);                                                                      \
-    else rmsnorm_fwd_kernel<HR, WR, GM><<<grid, WARPS * 32, 0, stream>>>(X, R, W, G, Y, RO, rstd, rows, D, eps);   \
+    else rmsnorm_fwd_kernel<HR, WR, GM><<<grid, WARPS * 32, 0, stream>>>(X, R, W, G, Y, RO, rstd, rows, D, eps, at);   \
   } while (0)
   if (gate_mode == 0) {
     if (res_in && res_out) FWD(true, true, 0);
@@ -364,20 +393,21 @@ int fb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, const void*
   return fb::launch_ok("rmsnorm_fwd_kernel");
 }
 
-// dw_part: fp32 [fb_rmsnorm_bwd_parts(rows), D] scratch; dw: fp32 [D] (accumulated when accumulate_dw != 0).
-int fb_rmsnorm_bwd(const void* dy, const void* xin, const void* w, const float* rstd, const void* gate,
-                   const void* dres, void* dx, void* dgate, float* dw_part, float* dw, long long rows, int D,
-                   int gate_mode, int accumulate_dw, cudaStream_t stream) {
+// rows: of xin and dx.  dw_part: fp32 [fb_rmsnorm_bwd_parts(rows), D] scratch; dw: fp32 [D] (accumulated when accumulate_dw != 0).
+int fb_rmsnorm_bwd_rows(const void* dy, const void* xin, const void* w, const float* rstd, const void* gate,
+                        const void* dres, void* dx, void* dgate, float* dw_part, float* dw, long long rows, int D,
+                        int gate_mode, int accumulate_dw, const int* map, int heads, long long ldg, long long lddg, cudaStream_t stream) {
   if (rows == 0) return 0;
-  if (D % 8) return -2;
+  if (D % 8 || heads < 1 || rows % heads || ldg % 8 || lddg % 8 || (rows >= (1ll << 31) && (map || ldg || lddg))) return -2;
+  const Rows at{map, (unsigned)heads, ldg ? ldg : (long long)heads * D, lddg ? lddg : (long long)heads * D};
   const int parts = fb_rmsnorm_bwd_parts(rows);
   const int rows_per_cta = (int)((rows + parts - 1) / parts);
   if (D > 7040) return -3;
   const int threads = D <= 256 ? WARPS * 32 : (D / 8 + 31) / 32 * 32;
 #define BWD_N(HD, GM, LP, NR, TPB)                                                                                  \
-  rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB><<<parts, threads, 0, stream>>>(                                           \
+  (map ? rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB, true> : rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB, false>)<<<parts, threads, 0, stream>>>( \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)xin, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)gate, \
-      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dgate, dw_part, rows, D, rows_per_cta)
+      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dgate, dw_part, rows, D, rows_per_cta, at)
   // rows per trip by what 128 registers hold packed; one row where a CTA has more than eight warps to overlap (64 registers)
 #define BWD(HD, GM)                                                                                               \
   do {                                                                                                            \
@@ -403,6 +433,13 @@ int fb_rmsnorm_bwd(const void* dy, const void* xin, const void* w, const float* 
     rc = fb::launch_ok("colsum_partials_kernel");
   }
   return rc;
+}
+
+// The same with every row in its place.
+int fb_rmsnorm_bwd(const void* dy, const void* xin, const void* w, const float* rstd, const void* gate,
+                   const void* dres, void* dx, void* dgate, float* dw_part, float* dw, long long rows, int D,
+                   int gate_mode, int accumulate_dw, cudaStream_t stream) {
+  return fb_rmsnorm_bwd_rows(dy, xin, w, rstd, gate, dres, dx, dgate, dw_part, dw, rows, D, gate_mode, accumulate_dw, nullptr, 1, 0, 0, stream);
 }
 
 }  // extern "C"

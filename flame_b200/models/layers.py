@@ -12,14 +12,13 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from ..ops import linear_attn as la
 from ..ops.attn_block import qkv_attention
-from ..ops.gates import logsigmoid_gate
+from ..ops.gates import delta_gates_torch, logsigmoid_gate
 from ..ops.rope import rope_tables
 from ..ops.slots import reshaped, split_columns
 from ..ops.varlen import VarlenMeta
 from .config import ModelConfig, mamba_dt_rank
-from .modules import Linear, RMSNorm, RMSNormGated, ShortConvolution, fused_projection, plain, side_by_side, split_projections
+from .modules import Linear, RMSNorm, RMSNormGated, ShortConvolution, fused_projection, norm_chunks, plain, side_by_side, split_projections
 
 
 class Attention(nn.Module):
@@ -210,12 +209,20 @@ def _feature_map(name: str, x: torch.Tensor) -> torch.Tensor:
     raise NotImplementedError(f"feature map {name!r}")
 
 
-def _conv_delta_rule(xs, convs, beta, g, meta: VarlenMeta, heads: int) -> Optional[torch.Tensor]:
+def _conv_delta_rule(xs, convs, gates, meta: VarlenMeta, heads: int):
     """Short convolutions and (gated) delta rule in one go, or None where something wants the convolutions' own results."""
     from ..ops.delta_rule import conv_gated_delta_rule
     if not plain(convs, ShortConvolution):
         return None
-    return conv_gated_delta_rule(xs, [c.weight for c in convs], [c.bias for c in convs], beta, g, meta, heads)
+    return conv_gated_delta_rule(xs, [c.weight for c in convs], [c.bias for c in convs], gates, meta, heads)
+
+
+def _projections(x: torch.Tensor, layers, more):
+    """``split_projections`` of all of them if one product can make them all, else of ``layers`` and each of ``more`` by itself."""
+    every = (*layers, *more)
+    if side_by_side(every, x):
+        return split_columns(fused_projection(x, every), [l.weight.shape[0] for l in every])
+    return (*split_projections(x, layers), *(l(x) for l in more))
 
 
 class DeltaNet(nn.Module):
@@ -252,17 +259,17 @@ class DeltaNet(nn.Module):
         from ..ops.delta_rule import gated_delta_rule
         T, H = x.shape[0], self.num_heads
         layers = (self.q_proj, self.k_proj, self.v_proj)
-        beta = self.b_proj(x).float().sigmoid() if self.use_beta else torch.ones(T, H, device=x.device)
-        if self.allow_neg_eigval:
-            beta = beta * 2.0
+        mul, b = 2.0 if self.allow_neg_eigval else 1.0, None
         if self.use_short_conv:
-            q, k, v = split_projections(x, layers)
-            if self.qk_activation == "silu" and self.qk_norm == "l2":
-                o = _conv_delta_rule((q, k, v), (self.q_conv1d, self.k_conv1d, self.v_conv1d), beta, None, meta, H)
+            q, k, v, *b = _projections(x, layers, (self.b_proj,) if self.use_beta else ())
+            b = b[0] if b else None
+            if b is not None and self.qk_activation == "silu" and self.qk_norm == "l2":
+                o = _conv_delta_rule((q, k, v), (self.q_conv1d, self.k_conv1d, self.v_conv1d), (b, None, None, None, mul), meta, H)
                 if o is not None:
-                    return self._output(x, o)
+                    return self._output(x, *o)
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
         else:
+            b = self.b_proj(x) if self.use_beta else None
             q, k, v = (l(x) for l in layers)
             if self.qk_activation == "silu":
                 q, k = F.silu(q), F.silu(k)
@@ -275,14 +282,14 @@ class DeltaNet(nn.Module):
             q, k = F.elu(q) + 1, F.elu(k) + 1
         if self.qk_norm == "sum":
             q, k = q / q.sum(-1, keepdim=True), k / k.sum(-1, keepdim=True)
+        beta = delta_gates_torch(b, None, None, None, mul)[0] if b is not None else torch.full((T, H), mul, device=x.device)
         return self._output(x, gated_delta_rule(q, k, v, beta, None, meta, l2norm_qk=(self.qk_norm == "l2")))
 
-    def _output(self, x: torch.Tensor, o: torch.Tensor) -> torch.Tensor:
+    def _output(self, x: torch.Tensor, o: torch.Tensor, lay=None) -> torch.Tensor:
+        """``lay``: the chunk layout that ``o`` is still in."""
         T, H = x.shape[0], self.num_heads
-        if self.use_gate:
-            o = self.o_norm(o, self.g_proj(x).reshape(T, H, self.head_v_dim))
-        else:
-            o = self.o_norm(o)
+        gate = (self.g_proj(x).reshape(T, H, self.head_v_dim),) if self.use_gate else ()
+        o = self.o_norm(o, *gate) if lay is None else norm_chunks(self.o_norm, o, lay, *gate)
         return self.o_proj(o.reshape(T, self.value_dim))
 
 
@@ -337,32 +344,30 @@ class GatedDeltaNet(nn.Module):
         T = x.shape[0]
         H, HV = self.num_heads, self.num_v_heads
         layers = (self.q_proj, self.k_proj, self.v_proj)
-        beta = self.b_proj(x).float().sigmoid()
-        if self.allow_neg_eigval:
-            beta = beta * 2.0
-        g = la.gdn_gate(self.a_proj(x), self.A_log, self.dt_bias)
+        mul = 2.0 if self.allow_neg_eigval else 1.0
         if self.use_short_conv:
-            q, k, v = split_projections(x, layers)
+            q, k, v, a, b = _projections(x, layers, (self.a_proj, self.b_proj))
             if HV == H:
-                o = _conv_delta_rule((q, k, v), (self.q_conv1d, self.k_conv1d, self.v_conv1d), beta, g, meta, H)
+                o = _conv_delta_rule((q, k, v), (self.q_conv1d, self.k_conv1d, self.v_conv1d), (b, a, self.A_log, self.dt_bias, mul), meta, H)
                 if o is not None:
-                    return self._output(x, o)
+                    return self._output(x, *o)
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
         else:
             q, k, v = (l(x) for l in layers)
             q, k, v = F.silu(q), F.silu(k), F.silu(v)
+            a, b = self.a_proj(x), self.b_proj(x)
         q, k = q.reshape(T, H, self.head_k_dim), k.reshape(T, H, self.head_k_dim)
         v = v.reshape(T, HV, self.head_v_dim)
         if HV > H:
             q, k = q.repeat_interleave(HV // H, 1), k.repeat_interleave(HV // H, 1)
+        beta, g = delta_gates_torch(b, a, self.A_log, self.dt_bias, mul)
         return self._output(x, gated_delta_rule(q, k, v, beta, g, meta, l2norm_qk=True))
 
-    def _output(self, x: torch.Tensor, o: torch.Tensor) -> torch.Tensor:
+    def _output(self, x: torch.Tensor, o: torch.Tensor, lay=None) -> torch.Tensor:
+        """``lay``: the chunk layout that ``o`` is still in."""
         T, HV = x.shape[0], self.num_v_heads
-        if self.use_gate:
-            o = self.o_norm(o, self.g_proj(x).reshape(T, HV, self.head_v_dim))
-        else:
-            o = self.o_norm(o)
+        gate = (self.g_proj(x).reshape(T, HV, self.head_v_dim),) if self.use_gate else ()
+        o = self.o_norm(o, *gate) if lay is None else norm_chunks(self.o_norm, o, lay, *gate)
         return self.o_proj(o.reshape(T, self.value_dim))
 
 

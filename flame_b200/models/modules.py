@@ -87,6 +87,14 @@ class Embedding(nn.Module):
         return _ScatterRowsSum.apply(out)
 
 
+def norm_chunks(norm: nn.Module, o: torch.Tensor, lay, gate: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """``norm(o)`` or ``norm(o, gate)`` of a chunk algorithm's result, still in the rows of ``lay``; as packed rows ``[T, heads, D]``."""
+    if plain((norm,), RMSNorm if gate is None else RMSNormGated):
+        return norm_ops.rms_norm_chunks(o, lay, norm.weight, norm.eps, gate, getattr(norm, "activation", "swish"))
+    o = lay.unpack(o)
+    return norm(o) if gate is None else norm(o, gate)
+
+
 class RMSNorm(nn.Module):
     def __init__(self, hidden_size: int, elementwise_affine: bool = True, eps: float = 1e-6) -> None:
         super().__init__()

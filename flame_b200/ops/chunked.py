@@ -701,11 +701,11 @@ def gated_delta_rule_tc(q, k, v, beta, g, meta: VarlenMeta, scale: Optional[floa
 
 
 @_recomputable
-def gated_delta_rule_chunks(qp, kp, vp, beta, g, meta: VarlenMeta, lay: "ChunkLayout", scale: float) -> torch.Tensor:
-    """The same with q, k, v already in the rows of ``lay`` (``[Tp, H, d]`` bf16; the padding's q, k and v are zero)."""
+def gated_delta_rule_chunks(qp, kp, vp, beta, g, lay: "ChunkLayout", scale: float) -> torch.Tensor:
+    """The same on operands in the rows of ``lay``: q, k, v ``[Tp, H, d]`` bf16 (zero in the padding), beta and g ``[NC, chunk, H]`` fp32; the
+    result stays there, ``[NC, chunk, H, dv]``."""
     qp, kp, vp = (t.view(lay.NC, lay.chunk, *t.shape[1:]) for t in (qp, kp, vp))
-    o = _GatedDelta.apply(qp, kp, vp, lay.pack(beta.float()), None if g is None else lay.pack(g.float()), scale, lay)
-    return lay.unpack(o)
+    return _GatedDelta.apply(qp, kp, vp, beta, g, scale, lay)
 
 
 @_recomputable

@@ -42,19 +42,25 @@ def gated_delta_rule(q, k, v, beta, g, meta: VarlenMeta, scale: Optional[float] 
     return gated_delta_rule_tc(q, k, v, beta, g, meta, scale)
 
 
-def conv_gated_delta_rule(xs, weights, biases, beta, g, meta: VarlenMeta, heads: int) -> Optional[torch.Tensor]:
+def conv_gated_delta_rule(xs, weights, biases, gates, meta: VarlenMeta, heads: int):
     """``gated_delta_rule`` with normalised q, k on the SiLU convolutions of the projections ``xs`` (q, k, v ``[T, heads * d]``), which
-    leave the convolution in the chunk layout; their gradients reach it there.  None where the kernels do not apply."""
+    leave the convolution in the chunk layout; their gradients reach it there.  ``gates``: the projections and parameters
+    of ``gates.delta_gates``.  Returns the result in the rows of the layout and the layout, or None where the kernels do not apply."""
     from .chunk_kernels import l2norm
     from .chunked import ChunkLayout, gated_delta_rule_chunks, scalar_chunk
     from .conv import short_convs_in_chunks
+    from .gates import delta_gates, delta_gates_torch
     dk, dv = xs[0].shape[1] // heads, xs[2].shape[1] // heads
     chunk = scalar_chunk(dk, dv)
     outs = short_convs_in_chunks(xs, weights, biases, meta, "silu", chunk)
     if outs is None:
         return None
+    lay = ChunkLayout.of(meta, chunk)
+    beta_g = delta_gates(*gates, lay)
+    if beta_g is None:
+        beta_g = [t if t is None else lay.pack(t) for t in delta_gates_torch(*gates)]
     q, k, v = (t.view(-1, heads, d) for t, d in zip(outs, (dk, dk, dv)))
-    return gated_delta_rule_chunks(l2norm(q), l2norm(k), v, beta, g, meta, ChunkLayout.of(meta, chunk), dk ** -0.5)
+    return gated_delta_rule_chunks(l2norm(q), l2norm(k), v, *beta_g, lay, dk ** -0.5), lay
 
 
 def _delta_rule_state_passing(q, k, v, beta, g, meta: VarlenMeta, scale, l2norm_qk: bool, sl) -> torch.Tensor:

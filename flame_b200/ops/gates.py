@@ -16,7 +16,7 @@ from typing import Optional, Tuple
 import torch
 import torch.nn.functional as F
 
-from . import _lib, slots
+from . import _lib, linear_attn as la, slots
 from .slots import split_columns  # noqa: F401 - part of this module's interface
 
 _lib.register("fb_hgrn2_gate_tiles", [c_longlong])
@@ -245,3 +245,79 @@ def mamba2_post(y, x, z, D, H: int, P: int):
     if _lib.available() and P in (64, 128, 256) and _views_ok(x, z) and y.is_cuda and y.dtype == torch.bfloat16:
         return _Mamba2Post.apply(y, x, z, D, H, P)
     return mamba2_post_reference(y, x, z, D, H, P)
+
+
+_lib.register("fb_delta_gates_blocks", [c_longlong, c_int])
+_lib.register("fb_delta_gates_fwd", [c_void_p, c_longlong] * 2 + [c_void_p] * 2 + [c_int, c_void_p, c_longlong, c_int, c_float] + [c_void_p] * 3)
+_lib.register("fb_delta_gates_bwd", [c_void_p, c_longlong] * 2 + [c_void_p] * 2 + [c_int, c_void_p, c_longlong, c_int, c_float] + [c_void_p] * 2
+              + [c_void_p, c_longlong] * 2 + [c_void_p] * 3 + [c_int, c_void_p])
+_DELTA_GATES_MAX_HEADS = 128
+
+
+class _DeltaGates(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, b, a, A_log, dt_bias, mul, lay):
+        ctx.slots = slots.of(b), None if a is None else slots.of(a)
+        rows, H = lay.Tp, b.shape[1]
+        src = None if lay.aligned else lay.inv_i32
+        beta = torch.empty(lay.NC, lay.chunk, H, dtype=torch.float32, device=b.device)
+        g = None if a is None else torch.empty_like(beta)
+        rc = _lib.lib().fb_delta_gates_fwd(*_DeltaGates._inputs(b, a, A_log, dt_bias), _lib.ptr(src), rows, H, mul, beta.data_ptr(),
+                                           _lib.ptr(g), _lib.stream_ptr())
+        _lib.check(rc, "fb_delta_gates_fwd")
+        _lib.count_launch()
+        ctx.save_for_backward(b, a, A_log, dt_bias)
+        ctx.params, ctx.cfg = (A_log, dt_bias), (mul, lay, src)
+        return beta, g
+
+    @staticmethod
+    def _inputs(b, a, A_log, dt_bias):
+        return (b.data_ptr(), b.stride(0), _lib.ptr(a), 0 if a is None else a.stride(0), _lib.ptr(A_log), _lib.ptr(dt_bias),
+                int(A_log is not None and A_log.dtype == torch.bfloat16))
+
+    @staticmethod
+    def backward(ctx, dbeta, dg):
+        b, a, A_log, dt_bias = ctx.saved_tensors
+        (mul, lay, src), H, dev = ctx.cfg, b.shape[1], b.device
+        rows = lay.Tp
+
+        def dense(d):
+            return torch.zeros(rows, H, dtype=torch.float32, device=dev) if d is None else _lib.dense(d.float())
+
+        def out(x, slot):
+            y = None if slot is None else slot.take(lay.T, H, x.dtype, dev)
+            return torch.empty(lay.T, H, dtype=x.dtype, device=dev) if y is None else y
+        dbeta, db = dense(dbeta), out(b, ctx.slots[0])
+        dA = ddt = da = part = None
+        main = False
+        L = _lib.lib()
+        if a is not None:
+            dg, da = dense(dg), out(a, ctx.slots[1])
+            main = all(getattr(p, "main_grad", None) is not None for p in ctx.params)
+            dA, ddt = (p.main_grad if main else torch.empty(H, dtype=torch.float32, device=dev) for p in ctx.params)
+            part = torch.empty(L.fb_delta_gates_blocks(rows, H), 2, H, dtype=torch.float32, device=dev)
+        rc = L.fb_delta_gates_bwd(*_DeltaGates._inputs(b, a, A_log, dt_bias), _lib.ptr(src), rows, H, mul, dbeta.data_ptr(), _lib.ptr(dg) if a is not None else 0,
+                                  db.data_ptr(), db.stride(0), _lib.ptr(da), 0 if da is None else da.stride(0), _lib.ptr(part),
+                                  _lib.ptr(dA), _lib.ptr(ddt), int(main), _lib.stream_ptr())
+        _lib.check(rc, "fb_delta_gates_bwd")
+        _lib.count_launch(1 if a is None else 2)
+        gA, gdt = (None, None) if a is None or main else (dA.to(A_log.dtype), ddt.to(dt_bias.dtype))
+        return db, da, gA, gdt, None, None
+
+
+def delta_gates_torch(b: torch.Tensor, a: Optional[torch.Tensor], A_log, dt_bias, mul: float):
+    """The same per token, ``[T, H]``."""
+    beta = b.float().sigmoid()
+    if mul != 1.0:
+        beta = beta * mul
+    return beta, None if a is None else la.gdn_gate(a, A_log, dt_bias)
+
+
+def delta_gates(b: torch.Tensor, a: Optional[torch.Tensor], A_log, dt_bias, mul: float, lay):
+    """``beta = mul sigmoid(b)`` and, with ``a``, the log decay ``-exp(A_log) softplus(a + dt_bias)`` of ``[T, H]`` bf16 projections, in fp32
+    ``[NC, chunk, H]`` in the rows of ``lay`` (``chunked.ChunkLayout``); None where the kernel does not apply."""
+    ok = _lib.available() and b.is_cuda and b.dtype == torch.bfloat16 and b.stride(-1) == 1 and b.shape[0] == lay.T and b.shape[1] <= _DELTA_GATES_MAX_HEADS
+    if a is not None:
+        ok = ok and (a.dtype, a.shape, a.stride(-1)) == (b.dtype, b.shape, 1) and A_log.dtype == dt_bias.dtype and \
+            A_log.dtype in (torch.bfloat16, torch.float32) and A_log.is_contiguous() and dt_bias.is_contiguous()
+    return _DeltaGates.apply(b, a, A_log, dt_bias, float(mul), lay) if ok else None

@@ -15,7 +15,7 @@ from typing import Optional, Sequence
 import torch
 import torch.nn.functional as F
 
-from . import _lib, float8, sac
+from . import _lib, float8, sac, slots
 from .gemm import gemm_nn, gemm_nt, gemm_tn
 
 
@@ -45,9 +45,17 @@ def _cat_view(ts: Sequence[torch.Tensor]) -> torch.Tensor:
     return out
 
 
+def _operands_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
+    return _lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0
+
+
 def _kernel_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
-    return (_lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16
-            and x.shape[-1] % 8 == 0 and w.shape[0] % 8 == 0)
+    return _operands_ok(x, w) and w.shape[0] % 8 == 0
+
+
+def _matrix(rows: int, cols: int, like: torch.Tensor) -> torch.Tensor:
+    """``[rows, cols]`` whose rows are whole 16-byte vectors apart, as the GEMM's operands have to be."""
+    return torch.empty(rows, -(-cols // 8) * 8, dtype=like.dtype, device=like.device)[:, :cols]
 
 
 class _LinearFn(torch.autograd.Function):
@@ -60,6 +68,7 @@ class _LinearFn(torch.autograd.Function):
         shape = x.shape
         K = shape[-1]
         x2 = x.reshape(-1, K)
+        ctx.slot = slots.of(x) if known is None and x.dim() == 2 and x.is_cuda else None
         fused = len(weights) == 1 or _adjacent([w.detach() for w in weights])
         ctx.fp8 = (known is None and fused and bias is None and all(getattr(w, "_fp8", False) for w in weights)
                    and float8.supported(x2) and all(w.shape[0] % 16 == 0 for w in weights))
@@ -81,7 +90,7 @@ class _LinearFn(torch.autograd.Function):
             return y.view(*shape[:-1], y.shape[-1])
         if fused:
             wcat = weights[0].detach() if len(weights) == 1 else _cat_view([w.detach() for w in weights])
-            y = gemm_nt(x2, wcat, bias=bias)
+            y = gemm_nt(x2, wcat, None if wcat.shape[0] % 8 == 0 else _matrix(x2.shape[0], wcat.shape[0], x2), bias=bias)
         else:
             N = sum(w.shape[0] for w in weights)
             y = torch.empty(x2.shape[0], N, dtype=x.dtype, device=x.device)
@@ -103,14 +112,17 @@ class _LinearFn(torch.autograd.Function):
         N = dy.shape[-1]
         dy2 = dy.reshape(-1, N)
         if dy2.stride(-1) != 1 or dy2.stride(0) % 8 != 0:
-            dy2 = dy2.contiguous()
+            dy2 = dy2.contiguous() if N % 8 == 0 or not dy2.is_cuda else _matrix(dy2.shape[0], N, dy2).copy_(dy2)
         K = x2.shape[1]
         dx = None
         if ctx.needs_input_grad[0]:
             if ctx.fused:
                 # saved-tensor hooks hand back copies, which lie wherever they were put
                 wcat = weights[0] if len(weights) == 1 else _cat_view(weights) if _adjacent(weights) else torch.cat(weights, 0)
-                dx = gemm_nn(dy2, wcat)
+                dx = None if ctx.slot is None else ctx.slot.take(x2.shape[0], K, x2.dtype, x2.device)
+                if dx is not None and (dx.stride(0) % 8 or dx.data_ptr() % 16 or wcat.shape[0] != N):
+                    dx = None
+                dx = gemm_nn(dy2, wcat, dx)
             else:
                 dx32 = None
                 c = 0
@@ -122,7 +134,15 @@ class _LinearFn(torch.autograd.Function):
             dx = dx.view(ctx.shape)
         grads = [None] * len(weights)
         mgs = [getattr(w, "main_grad", None) for w in ctx.params]
-        if all(m is not None for m in mgs):
+        if len(weights) > 1 and any(w.shape[0] % 8 for w in weights) and not (all(m is not None for m in mgs) and _adjacent(mgs)):
+            # column blocks that start between vectors cannot be operands of their own
+            whole = gemm_tn(dy2, x2, out_dtype=torch.float32)
+            for i, (part, m) in enumerate(zip(whole.split([w.shape[0] for w in weights]), mgs)):
+                if m is not None:
+                    m += part
+                elif ctx.needs_input_grad[3 + i]:
+                    grads[i] = part.to(weights[i].dtype)
+        elif all(m is not None for m in mgs):
             if ctx.fused and (len(weights) == 1 or _adjacent(mgs)):
                 mg = mgs[0] if len(weights) == 1 else _cat_view(mgs)
                 gemm_tn(dy2, x2, out=mg, accumulate=True)
@@ -208,14 +228,14 @@ def side_by_side(x: torch.Tensor, weights: Sequence[torch.Tensor]) -> bool:
     """Whether one GEMM may stand for the products of ``x`` with these weights: adjacent in memory (their ``main_grad``s too, or
     none has one), bf16 on the GPU, no fp8 scaling per tensor, no tape that counts products (selective checkpointing)."""
     mgs = [getattr(w, "main_grad", None) for w in weights]
-    return (x.dim() == 2 and all(_kernel_ok(x, w) and not getattr(w, "_fp8", False) for w in weights) and sac.current() is None
+    return (x.dim() == 2 and all(_operands_ok(x, w) and not getattr(w, "_fp8", False) for w in weights) and sac.current() is None
             and _adjacent([w.detach() for w in weights])
             and (all(m is None for m in mgs) or (all(m is not None for m in mgs) and _adjacent(mgs))))
 
 
 def linear_fused(x: torch.Tensor, weights: Sequence[torch.Tensor]) -> torch.Tensor:
     """``x @ cat(weights, 0).T`` as one ``[..., sum(N_i)]`` tensor."""
-    if all(_kernel_ok(x, w) for w in weights):
+    if all(_kernel_ok(x, w) for w in weights) or side_by_side(x, weights):
         return _with_tape(x, None, weights, lambda: _LinearFn.apply(x, None, None, *weights))
     if not x.is_cuda and x.dtype == torch.bfloat16 and _cpu_fp8(x, weights):
         return torch.cat([_LinearFn.apply(x, None, None, w) for w in weights], dim=-1)

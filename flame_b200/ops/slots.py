@@ -49,7 +49,9 @@ class Slot:
         stream = _lib.stream_ptr() if device.type == "cuda" else 0
         with h.lock:
             if h.buffer is None or h.run != run:
-                h.buffer, h.run, h.stream = torch.empty(rows, h.width, dtype=dtype, device=device), run, stream
+                # rows whole 16-byte vectors apart (of two-byte values), as the projection's GEMMs read them
+                h.buffer = torch.empty(rows, -(-h.width // 8) * 8, dtype=dtype, device=device)[:, :h.width]
+                h.run, h.stream = run, stream
             b, owner = h.buffer, h.stream
         if n != self.n or owner != stream or b.shape[0] != rows or b.dtype != dtype or b.device != device:
             return torch.empty(rows, n, dtype=dtype, device=device)

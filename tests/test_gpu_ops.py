@@ -754,3 +754,94 @@ def test_attention_work_list(lens):
     assert sorted(docs) == list(range(n)) and whole[n + 1:2 * n + 2] == [0] + list(np.cumsum([tiles[d] for d in docs]))
     clipped = [min(tiles[d], 2047) for d in docs]
     assert clipped == sorted(clipped, reverse=True)
+
+
+@pytest.mark.parametrize("D", [64, 128, 256, 512])
+@pytest.mark.parametrize("gate", [None, "dense", "block"])
+def test_norm_out_of_chunk_rows(D, gate):
+    """A norm that reads the chunk layout, with its gate a column block of a wider matrix: bit for bit what unpacking and a dense gate
+    give, gradients too (zeros in the padding); the weight's gradient sums the same rows over other blocks: 5e-3 after rounding to bf16."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.norm import rms_norm, rms_norm_chunks, rms_norm_gated
+    from flame_b200.ops.slots import reshaped, split_columns
+    torch.manual_seed(D)
+    lens, H = [1, 63, 65, 300, 64, 7], 3
+    T, lay = sum(lens), ChunkLayout.of(_meta(lens), 64)
+    o0 = torch.randn(lay.NC, 64, H, D, device=DEV).bfloat16()
+    wide0, w0, dy = torch.randn(T, 16 + H * D, device=DEV).bfloat16(), torch.randn(D, device=DEV).bfloat16(), torch.randn(T, H, D, device=DEV).bfloat16()
+    out = []
+    for new in (True, False):
+        o, wide, w = (t.clone().requires_grad_(True) for t in (o0, wide0, w0))
+        g = None
+        if gate is not None:
+            g = reshaped(split_columns(wide, (16, H * D))[1], T, H, D) if gate == "block" and new else wide[:, 16:].reshape(T, H, D).contiguous()
+        if new:
+            y = rms_norm_chunks(o, lay, w, 1e-5, g)
+        else:
+            y = rms_norm(lay.unpack(o), w, 1e-5) if g is None else rms_norm_gated(lay.unpack(o), g, w, 1e-5)
+        y.backward(dy)
+        out.append((y.detach(), o.grad, wide.grad, w.grad))
+    for a, b in zip(out[0][:3], out[1][:3]):
+        assert (a is None and b is None) or torch.equal(a, b)
+    assert rel_err(out[0][3], out[1][3]) < 5e-3
+
+
+@pytest.mark.parametrize("H,bf16,decay,mul", [(6, True, True, 1.0), (1, False, True, 2.0), (16, True, False, 1.0), (128, True, True, 2.0)])
+def test_delta_gates(H, bf16, decay, mul):
+    """The delta rule's gates in the chunk layout, from column blocks that start between vectors, against fp64: fp32 results of a few
+    operations (1e-5), gradients of bf16 values rounded once (5e-3), of the parameters summed over the rows in fp32 (1e-3)."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.gates import delta_gates, delta_gates_torch
+    from flame_b200.ops.slots import split_columns
+    torch.manual_seed(H)
+    lens = [1, 63, 65, 2000, 64, 7]
+    T, lay = sum(lens), ChunkLayout.of(_meta(lens), 64)
+    dt = torch.bfloat16 if bf16 else torch.float32
+    x = (torch.randn(T, 3 + 2 * H, device=DEV) * 4).bfloat16().requires_grad_(True)
+    A, d = (torch.randn(H, device=DEV).to(dt).requires_grad_(True) for _ in range(2))
+    _, a, b = split_columns(x, (3, H, H))
+    beta, g = delta_gates(b, a if decay else None, A if decay else None, d if decay else None, mul, lay)
+    dbeta, dg = torch.randn_like(beta), torch.randn_like(beta)
+    ins = [x, A, d] if decay else [x]
+    got = torch.autograd.grad([beta, g] if decay else [beta], ins, [dbeta, dg] if decay else [dbeta])
+    xr, Ar, dr = (t.detach().double().requires_grad_(True) for t in (x, A, d))
+    sp = torch.nn.functional.softplus(xr[:, 3:3 + H] + dr, threshold=100)
+    want_b, want_g = mul * torch.sigmoid(xr[:, 3 + H:]), -Ar.exp() * sp
+    flat = lambda t: t.reshape(lay.Tp, H)  # noqa: E731
+    assert rel_err(flat(beta)[lay.rows], want_b) < 1e-5 and float(flat(beta)[lay.inv_i32 < 0].abs().sum()) == 0
+    want = [(flat(dbeta)[lay.rows].double() * want_b).sum()]
+    if decay:
+        assert rel_err(flat(g)[lay.rows], want_g) < 1e-5 and float(flat(g)[lay.inv_i32 < 0].abs().sum()) == 0
+        want.append((flat(dg)[lay.rows].double() * want_g).sum())
+        plain = delta_gates_torch(b.detach(), a.detach(), A.detach(), d.detach(), mul)
+        assert rel_err(plain[0], want_b) < 1e-5 and rel_err(plain[1], want_g) < 1e-5
+    want = torch.autograd.grad(sum(want), [xr, Ar, dr] if decay else [xr])
+    for i, (p, q) in enumerate(zip(got, want)):
+        assert rel_err(p, q) < (5e-3 if i == 0 or bf16 else 1e-3)
+
+
+@pytest.mark.parametrize("rows", [1, 300])
+@pytest.mark.parametrize("mains", [False, True])
+def test_side_by_side_projections_of_odd_sizes(rows, mains):
+    """One product for projections of which some start between vectors (64 + 6 + 6 rows), their gradients written side by side; against
+    fp64.  bf16 results of 128-term sums (2^-8), weight gradients in fp32 with main_grad."""
+    from flame_b200.ops.linear import linear_fused, side_by_side
+    from flame_b200.ops.slots import split_columns
+    torch.manual_seed(rows)
+    flat, grad = torch.randn(76 * 128, device=DEV).bfloat16() * 0.1, torch.ones(76 * 128, device=DEV)
+    ws, at = [], 0
+    for n in (64, 6, 6):
+        w = torch.nn.Parameter(flat[at:at + n * 128].view(n, 128))
+        if mains:
+            w.main_grad = grad[at:at + n * 128].view(n, 128)
+        ws.append(w)
+        at += n * 128
+    x = torch.randn(rows, 128, device=DEV).bfloat16().requires_grad_(True)
+    assert side_by_side(x, ws)
+    parts = split_columns(linear_fused(x, ws), (64, 6, 6))
+    dys = [torch.randn_like(p) for p in parts]
+    torch.autograd.backward(parts, dys)
+    xr, wr, dy = x.detach().double(), flat.view(76, 128).double(), torch.cat(dys, 1).double()
+    assert rel_err(torch.cat(parts, 1), xr @ wr.T) < 5e-3 and rel_err(x.grad, dy @ wr) < 5e-3
+    got = grad.view(76, 128) - 1 if mains else torch.cat([w.grad for w in ws])
+    assert rel_err(got, dy.T @ xr) < (1e-4 if mains else 5e-3)
