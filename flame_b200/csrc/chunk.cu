@@ -467,67 +467,163 @@ int fb_group_bwd2(const void* dvhat, const void* vhat, const void* dv1, const fl
 // fla/ops/gla/chunk.py:88-170); the sub-blocks left of them come in from a batched GEMM on re-based operands.
 // q, k: [NC, 64, H, dk] bf16; b: [NC, 64, H, dk] fp32 (within-chunk cumulative log decay); blk: [3 NC, H, 16, 48] bf16, entry
 // (3 c + I - 1) holding the 16 rows of sub-block I; A: [NC, H, 64, 64] bf16, written in full.
-// One block per (chunk, head).  The pairs with j <= i of the four sub-blocks are 4 x 136 = 544 = 17 full warps, a thread each;
-// operands of 64 channels at a time in shared memory, rows 4 words apart modulo the banks, read as float4: four loads
-// and an exponential per four channels and pair bound it.  With a thread per (i, j) of a sub-block half of the threads had
-// nothing to do and every operand was a 4-byte load: 0.29 ms at 65,536 tokens, 4 heads of 128.
+// One block per (chunk, head).  Four lanes share a tile of 2 x 2 pairs, a quarter of the channels each: 4 x 36 tiles (of those on
+// the diagonal three pairs count) = 576 threads.  Operands of 64 channels at a time in shared memory, rows 4 words apart modulo
+// the banks; eight 16-byte reads and sixteen exponentials per tile and four
+// channels.  With a thread per pair (four reads for four exponentials, operands brought in two bytes at a time) shared memory
+// bound it: 0.271 ms at 65,536 tokens, 4 heads of 128; this takes 0.193.
 namespace {
+
+// Where the rows of a chunk's q, k and gate lie: packed tokens (src [64 NC]: the token of every chunk row, -1: padding, a chunk's
+// tokens follow one another), ld* elements from row to row, or, src null, in the padded rows themselves.
+struct GlaRows {
+  const int* src;
+  long long ldq, ldk, ldg;
+};
+// log(sigmoid(x)) mul without cancellation or underflow: log(1 + e), e = exp(-|x|) <= 1, is 2 artanh(e / (2 + e)), by the artanh series
+// up to s^13 for s <= 1/3 (relative error below 1e-7)
+__device__ __forceinline__ float log_sigmoid(float x, float mul) {
+  const float e = __expf(-fabsf(x)), s = __fdividef(e, 2.f + e), w = s * s;
+  float p = fmaf(w, 1.f / 13.f, 1.f / 11.f);
+  p = fmaf(p, w, 1.f / 9.f);
+  p = fmaf(p, w, 1.f / 7.f);
+  p = fmaf(p, w, 1.f / 5.f);
+  p = fmaf(p, w, 1.f / 3.f);
+  p = fmaf(p, w, 1.f);
+  return (fminf(x, 0.f) - 2.f * s * p) * mul;
+}
+__device__ __forceinline__ void unpack8_bf16(const uint4& v, float (&f)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[2 * i] = __uint_as_float(w[i] << 16), f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+}
+// first row of chunk c and how many rows it has
+__device__ __forceinline__ void gla_rows(const int* __restrict__ src, int c, long long& row0, int& n) {
+  row0 = 64ll * c, n = 64;
+  if (src == nullptr) return;
+  const int lane = threadIdx.x & 31;
+  const int* s = src + 64ll * c;
+  n = __popc(__ballot_sync(0xffffffffu, s[lane] >= 0)) + __popc(__ballot_sync(0xffffffffu, s[lane + 32] >= 0));
+  row0 = s[0];
+}
 
 constexpr int GD_T = 64;        // channels per trip
 constexpr int GD_LD = GD_T + 4;
-constexpr int GD_THREADS = 544;
+constexpr int GD_THREADS = 576;
 
 template <typename TQ>
 __global__ void __launch_bounds__(GD_THREADS, 2) gla_scores_kernel(const TQ* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                                                                 const float* __restrict__ b, const __nv_bfloat16* __restrict__ blk,
-                                                                __nv_bfloat16* __restrict__ A, int H, int dk, float scale) {
+                                                                __nv_bfloat16* __restrict__ A, const GlaRows at, int H, int dk, float scale, int vec) {
   extern __shared__ __align__(16) float sm[];
   float *sq = sm, *sk = sq + 64 * GD_LD, *sb = sk + 64 * GD_LD;
-  const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
-  const int sub = threadIdx.x / 136, pr = threadIdx.x - sub * 136;
-  int i = (int)((sqrtf(8.f * pr + 1.f) - 1.f) * 0.5f);
-  while ((i + 1) * (i + 2) / 2 <= pr) ++i;
-  while (i * (i + 1) / 2 > pr) --i;
-  const int j = pr - i * (i + 1) / 2;
-  const float4* qi = reinterpret_cast<const float4*>(sq + (sub * 16 + i) * GD_LD);
-  const float4* bi = reinterpret_cast<const float4*>(sb + (sub * 16 + i) * GD_LD);
-  const float4* kj = reinterpret_cast<const float4*>(sk + (sub * 16 + j) * GD_LD);
-  const float4* bj = reinterpret_cast<const float4*>(sb + (sub * 16 + j) * GD_LD);
-  float acc = 0.f;
+  const int ch = blockIdx.x, c = ch / H, h = ch - c * H, tid = threadIdx.x;
+  long long row0;
+  int n;
+  gla_rows(at.src, c, row0, n);
+  const int tile = tid >> 2, part = tid & 3, sub = tile / 36, tt = tile - sub * 36;
+  int ti = (int)((sqrtf(8.f * tt + 1.f) - 1.f) * 0.5f);
+  while ((ti + 1) * (ti + 2) / 2 <= tt) ++ti;
+  while (ti * (ti + 1) / 2 > tt) --ti;
+  const int tj = tt - ti * (ti + 1) / 2;
+  const int ri = (sub * 16 + 2 * ti) * GD_LD + part * 4, rj = (sub * 16 + 2 * tj) * GD_LD + part * 4;
+  constexpr float LOG2E = 1.4426950408889634f;
+  const TQ* qp = q + row0 * at.ldq + (long long)h * dk;
+  const __nv_bfloat16* kp = k + row0 * at.ldk + (long long)h * dk;
+  const float* bp = b + ((long long)c * 64 * H + h) * dk;
+  const long long ldb = (long long)H * dk;
+  // a thread brings eight channels of a row
+  const int lr = tid >> 3, lc = (tid & 7) * 8;
+  uint4 nq[sizeof(TQ) / 2], nk;
+  float4 nb[2];  // a trip's operands between global and shared memory
+  auto fetch = [&](int d0) {
+    const bool in = tid < 512 && d0 + lc < dk, there = in && lr < n;  // dk is a multiple of 8 here
+    const uint4 none = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+    for (int t = 0; t < (int)sizeof(TQ) / 2; ++t) nq[t] = there ? reinterpret_cast<const uint4*>(qp + lr * at.ldq + d0 + lc)[t] : none;
+    nk = there ? *reinterpret_cast<const uint4*>(kp + lr * at.ldk + d0 + lc) : none;
+#pragma unroll
+    for (int t = 0; t < 2; ++t) nb[t] = in ? reinterpret_cast<const float4*>(bp + lr * ldb + d0 + lc)[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  auto put = [&]() {
+    if (tid >= 512) return;
+    float f[8];
+    float4 *oq = reinterpret_cast<float4*>(sq + lr * GD_LD + lc), *ok = reinterpret_cast<float4*>(sk + lr * GD_LD + lc),
+           *ob = reinterpret_cast<float4*>(sb + lr * GD_LD + lc);
+    if constexpr (sizeof(TQ) == 4) {
+      oq[0] = *reinterpret_cast<const float4*>(&nq[0]);
+      oq[1] = *reinterpret_cast<const float4*>(&nq[1]);
+    } else {
+      unpack8_bf16(nq[0], f);
+      oq[0] = make_float4(f[0], f[1], f[2], f[3]), oq[1] = make_float4(f[4], f[5], f[6], f[7]);
+    }
+    unpack8_bf16(nk, f);
+    ok[0] = make_float4(f[0], f[1], f[2], f[3]), ok[1] = make_float4(f[4], f[5], f[6], f[7]);
+#pragma unroll
+    for (int t = 0; t < 2; ++t) ob[t] = make_float4(nb[t].x * LOG2E, nb[t].y * LOG2E, nb[t].z * LOG2E, nb[t].w * LOG2E);
+  };
+  float acc[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
   for (int d0 = 0; d0 < dk; d0 += GD_T) {
-    const int n = min(GD_T, dk - d0);
+    if (vec) fetch(d0);
     __syncthreads();
-    for (int idx = threadIdx.x; idx < 64 * GD_T; idx += GD_THREADS) {
-      const int r = idx / GD_T, d = idx % GD_T;
-      const bool in = d < n;
-      const long long g = (((long long)c * 64 + r) * H + h) * dk + d0 + d;
-      sq[r * GD_LD + d] = in ? (float)q[g] : 0.f;
-      sk[r * GD_LD + d] = in ? __bfloat162float(k[g]) : 0.f;
-      sb[r * GD_LD + d] = in ? b[g] * 1.4426950408889634f : 0.f;
+    if (vec) {
+      put();
+    } else {  // rows that are not whole vectors
+      for (int idx = tid; idx < 64 * GD_T; idx += GD_THREADS) {
+        const int r = idx / GD_T, d = idx % GD_T;
+        const bool in = d0 + d < dk, there = in && r < n;
+        sq[r * GD_LD + d] = there ? (float)qp[r * at.ldq + d0 + d] : 0.f;
+        sk[r * GD_LD + d] = there ? __bfloat162float(kp[r * at.ldk + d0 + d]) : 0.f;
+        sb[r * GD_LD + d] = in ? bp[r * ldb + d0 + d] * LOG2E : 0.f;
+      }
     }
     __syncthreads();
-#pragma unroll 4
-    for (int d = 0; d < GD_T / 4; ++d) {
-      const float4 a4 = qi[d], k4 = kj[d], x = bi[d], y = bj[d];
-      acc = fmaf(a4.x * k4.x, exp2f(x.x - y.x), acc);
-      acc = fmaf(a4.y * k4.y, exp2f(x.y - y.y), acc);
-      acc = fmaf(a4.z * k4.z, exp2f(x.z - y.z), acc);
-      acc = fmaf(a4.w * k4.w, exp2f(x.w - y.w), acc);
+#pragma unroll 2
+    for (int d = 0; d < GD_T; d += 16) {
+      float4 qi[2], bi[2], kj[2], bj[2];
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        qi[t] = *reinterpret_cast<const float4*>(sq + ri + t * GD_LD + d);
+        bi[t] = *reinterpret_cast<const float4*>(sb + ri + t * GD_LD + d);
+        kj[t] = *reinterpret_cast<const float4*>(sk + rj + t * GD_LD + d);
+        bj[t] = *reinterpret_cast<const float4*>(sb + rj + t * GD_LD + d);
+      }
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y) {
+          acc[x][y] = fmaf(qi[x].x * kj[y].x, exp2f(bi[x].x - bj[y].x), acc[x][y]);
+          acc[x][y] = fmaf(qi[x].y * kj[y].y, exp2f(bi[x].y - bj[y].y), acc[x][y]);
+          acc[x][y] = fmaf(qi[x].z * kj[y].z, exp2f(bi[x].z - bj[y].z), acc[x][y]);
+          acc[x][y] = fmaf(qi[x].w * kj[y].w, exp2f(bi[x].w - bj[y].w), acc[x][y]);
+        }
     }
   }
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      acc[x][y] += __shfl_xor_sync(0xffffffffu, acc[x][y], 1);
+      acc[x][y] += __shfl_xor_sync(0xffffffffu, acc[x][y], 2);
+    }
   __nv_bfloat16* o = A + (long long)ch * 4096;
-  o[(sub * 16 + i) * 64 + sub * 16 + j] = __float2bfloat16(acc * scale);
+  {
+    const int x = part >> 1, y = part & 1, i = 2 * ti + x, j = 2 * tj + y;  // the pair of the tile that this lane writes
+    const float v = x ? (y ? acc[1][1] : acc[1][0]) : (y ? acc[0][1] : acc[0][0]);
+    // above the diagonal the exponent is positive and the sum means nothing
+    o[(sub * 16 + i) * 64 + sub * 16 + j] = __float2bfloat16(j <= i ? v * scale : 0.f);
+  }
   // the rest of the matrix: sub-blocks to the left from the GEMM, zeros to the right (16-byte pieces), zeros above the diagonal
-  for (int idx = threadIdx.x; idx < 64 * 8; idx += GD_THREADS) {
+  for (int idx = tid; idx < 64 * 8; idx += GD_THREADS) {
     const int r = idx >> 3, c8 = (idx & 7) * 8, I = r >> 4;
     if ((c8 >> 4) == I) continue;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (c8 < 16 * I) v = *reinterpret_cast<const uint4*>(blk + ((((long long)c * 3 + I - 1) * H + h) * 16 + (r & 15)) * 48 + c8);
     *reinterpret_cast<uint4*>(o + r * 64 + c8) = v;
   }
-  for (int idx = threadIdx.x; idx < 4 * 256; idx += GD_THREADS) {
+  for (int idx = tid; idx < 4 * 256; idx += GD_THREADS) {
     const int I = idx >> 8, r = (idx >> 4) & 15, cc = idx & 15;
-    if (cc > r) o[(I * 16 + r) * 64 + I * 16 + cc] = __float2bfloat16(0.f);
+    if ((cc >> 1) > (r >> 1)) o[(I * 16 + r) * 64 + I * 16 + cc] = __float2bfloat16(0.f);
   }
 }
 
@@ -538,43 +634,48 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gla_scores_kernel(const TQ* __r
 //   dq_id = scale sum_{j<=i} dA_ij k_jd e^{b_id-b_jd} + dqbar_id scale e^{b_id} + dqt_id e^{b_id-r_I}
 //   dk_jd = scale sum_{i>=j} dA_ij q_id e^{b_id-b_jd} + dkhat_jd e^{b_last-b_jd} + sum_I dk3[I]_jd e^{r_I-b_jd}
 //   db    = q dq - k dk (+ what enters through b_last: khat and alpha), dg = reverse cumulative sum of db
-// dA: bf16 [NC, H, 64, 64] (only the diagonal sub-blocks are read).
-__global__ void __launch_bounds__(128, 3) gla_bwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                                                      const float* __restrict__ b, const __nv_bfloat16* __restrict__ dA,
-                                                      const __nv_bfloat16* __restrict__ dkhat, const __nv_bfloat16* __restrict__ dqbar,
-                                                      const __nv_bfloat16* __restrict__ dqt, const __nv_bfloat16* __restrict__ dk3,
-                                                      const float* __restrict__ dalpha, __nv_bfloat16* __restrict__ dq,
-                                                      __nv_bfloat16* __restrict__ dk_, float* __restrict__ dg, int H, int dk, float scale) {
-  __shared__ float sA[4][16][16];
-  __shared__ float sgb[64][128];
-  const int d = blockIdx.y * 128 + threadIdx.x;
-  const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
-  for (int idx = threadIdx.x; idx < 1024; idx += 128) {
-    const int I = idx >> 8, r = (idx >> 4) & 15, cc = idx & 15;
-    sA[I][r][cc] = cc <= r ? __bfloat162float(dA[((long long)ch * 64 + I * 16 + r) * 64 + I * 16 + cc]) * scale : 0.f;
-  }
-  __syncthreads();
-  if (d >= dk) return;
+// dA: bf16 [NC, H, 64, 64] (only the diagonal sub-blocks are read).  q, k, dq, dk and the gate's gradient lie as GlaRows says (`to`: the
+// gradients).  With `raw` the gate is g = logsigmoid(raw) norm, and its gradient is that of raw in bf16.
+// FULL: the chunk has all of its 64 rows; a test per row keeps the loads of the next rows behind it, so only the chunks at the
+// documents' ends make it.  What the second half of a sub-block needs is loaded in front of the pairs, whose 136 exponentials it takes
+// to come: loaded after them it doubled the waits (0.70 ms against 0.66).
+__device__ __forceinline__ unsigned short ld_now(const __nv_bfloat16* p) {  // a read-only load that stays where it is written
+  unsigned short v;
+  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float bf16_of(unsigned short v) { return __uint_as_float((uint32_t)v << 16); }
+template <bool FULL, int TPB>
+__device__ __forceinline__ void gla_bwd_rows(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const float* __restrict__ b,
+                                             const __nv_bfloat16* __restrict__ dkhat, const __nv_bfloat16* __restrict__ dqbar,
+                                             const __nv_bfloat16* __restrict__ dqt, const __nv_bfloat16* __restrict__ dk3,
+                                             __nv_bfloat16* __restrict__ dq, __nv_bfloat16* __restrict__ dk_, void* __restrict__ dg,
+                                             const __nv_bfloat16* __restrict__ raw, float norm, const float (&sA)[4][16][16], float (&sgb)[64][TPB],
+                                             int rs, int ldq, int ldk, int ldg, int lddq, int lddk, int lddg, int n, float dalpha, float scale) {
   constexpr float LOG2E = 1.4426950408889634f;
-  const long long rs = (long long)H * dk;
-  const long long base = ((long long)c * 64 * H + h) * dk + d;
-  dqt -= 16LL * (c + 1) * rs;  // [NC, 48, H, dk], rows of sub-blocks 1..3 only: with this it is read at the others' offsets
-  const long long k3base = (((long long)c * 3) * 48 * H + h) * dk + d;
   float r[4];
 #pragma unroll
-  for (int I = 0; I < 4; ++I) r[I] = b[base + (long long)(16 * I) * rs] * LOG2E;
-  const float b_last = b[base + 63 * rs] * LOG2E;
+  for (int I = 0; I < 4; ++I) r[I] = __ldg(b + 16 * I * rs) * LOG2E;
+  const float b_last = __ldg(b + 63 * rs) * LOG2E;
   float acc_last = 0.f;
 #pragma unroll 1
   for (int I = 0; I < 4; ++I) {
     float qv[16], kv[16], bv[16], gq[16], gk[16];
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const long long off = base + (long long)(I * 16 + i) * rs;
-      qv[i] = __bfloat162float(q[off]);
-      kv[i] = __bfloat162float(k[off]);
-      bv[i] = b[off] * LOG2E;
+      const int row = I * 16 + i;
+      qv[i] = FULL || row < n ? __bfloat162float(__ldg(q + row * ldq)) : 0.f;
+      kv[i] = FULL || row < n ? __bfloat162float(__ldg(k + row * ldk)) : 0.f;
+      bv[i] = __ldg(b + row * rs) * LOG2E;
       gq[i] = gk[i] = 0.f;
+    }
+    unsigned short a_khat[16], a_qbar[16], a_qt[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int off = (I * 16 + i) * rs;
+      a_khat[i] = ld_now(dkhat + off);
+      a_qbar[i] = ld_now(dqbar + off);
+      a_qt[i] = I > 0 ? ld_now(dqt + off) : (unsigned short)0;
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i)
@@ -587,61 +688,109 @@ __global__ void __launch_bounds__(128, 3) gla_bwd_kernel(const __nv_bfloat16* __
     const float rI = r[0] * (I == 0) + r[1] * (I == 1) + r[2] * (I == 2) + r[3] * (I == 3);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
-      const long long off = base + (long long)(I * 16 + i) * rs;
-      const float g_khat = __bfloat162float(dkhat[off]) * exp2f(b_last - bv[i]);
-      gq[i] = fmaf(__bfloat162float(dqbar[off]), exp2f(bv[i]) * scale, gq[i]);
-      if (I > 0) gq[i] = fmaf(__bfloat162float(dqt[off]), exp2f(bv[i] - rI), gq[i]);
+      const int row = I * 16 + i;
+      const float g_khat = bf16_of(a_khat[i]) * exp2f(b_last - bv[i]);
+      gq[i] = fmaf(bf16_of(a_qbar[i]), exp2f(bv[i]) * scale, gq[i]);
+      if (I > 0) gq[i] = fmaf(bf16_of(a_qt[i]), exp2f(bv[i] - rI), gq[i]);
       gk[i] += g_khat;
       acc_last = fmaf(g_khat, kv[i], acc_last);
       if (I < 3) {
 #pragma unroll
         for (int J = 1; J <= 3; ++J)
-          if (J > I) gk[i] = fmaf(__bfloat162float(dk3[k3base + ((long long)(J - 1) * 48 + I * 16 + i) * rs]), exp2f(r[J] - bv[i]), gk[i]);
+          if (J > I) gk[i] = fmaf(__bfloat162float(__ldg(dk3 + ((J - 1) * 48 + row) * rs)), exp2f(r[J] - bv[i]), gk[i]);
       }
-      dq[off] = __float2bfloat16(gq[i]);
-      dk_[off] = __float2bfloat16(gk[i]);
-      sgb[I * 16 + i][threadIdx.x] = qv[i] * gq[i] - kv[i] * gk[i];
+      if (FULL || row < n) {
+        dq[row * lddq] = __float2bfloat16(gq[i]);
+        dk_[row * lddk] = __float2bfloat16(gk[i]);
+      }
+      sgb[row][threadIdx.x] = qv[i] * gq[i] - kv[i] * gk[i];
     }
   }
-  float tail = acc_last + dalpha[(long long)ch * dk + d] * exp2f(b_last);  // gradient of b_last
+  float tail = acc_last + dalpha * exp2f(b_last);  // gradient of b_last
+  if (raw == nullptr) {
 #pragma unroll 8
-  for (int i = 63; i >= 0; --i) {
-    tail += sgb[i][threadIdx.x];
-    dg[base + i * rs] = tail;
+    for (int i = 63; i >= 0; --i) {
+      tail += sgb[i][threadIdx.x];
+      if (FULL || i < n) ((float*)dg)[i * lddg] = tail;
+    }
+  } else {
+#pragma unroll 8
+    for (int i = 63; i >= 0; --i) {
+      tail += sgb[i][threadIdx.x];
+      if (FULL || i < n) ((__nv_bfloat16*)dg)[i * lddg] = __float2bfloat16(tail * norm / (1.f + __expf(__bfloat162float(__ldg(raw + i * ldg)))));
+    }
   }
+}
+
+// TPB: 64 where a head has no more channels, else 128
+template <int TPB>
+__global__ void __launch_bounds__(TPB, 384 / TPB) gla_bwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+                                                      const float* __restrict__ b, const __nv_bfloat16* __restrict__ dA,
+                                                      const __nv_bfloat16* __restrict__ dkhat, const __nv_bfloat16* __restrict__ dqbar,
+                                                      const __nv_bfloat16* __restrict__ dqt, const __nv_bfloat16* __restrict__ dk3,
+                                                      const float* __restrict__ dalpha, __nv_bfloat16* __restrict__ dq,
+                                                      __nv_bfloat16* __restrict__ dk_, void* __restrict__ dg, const __nv_bfloat16* __restrict__ raw,
+                                                      float norm, const GlaRows at, const GlaRows to, int H, int dk, float scale) {
+  __shared__ float sA[4][16][16];
+  __shared__ float sgb[64][TPB];
+  const int d = blockIdx.y * TPB + threadIdx.x;
+  const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
+  long long row0;
+  int n;
+  gla_rows(at.src, c, row0, n);
+  for (int idx = threadIdx.x; idx < 1024; idx += TPB) {
+    const int I = idx >> 8, r = (idx >> 4) & 15, cc = idx & 15;
+    sA[I][r][cc] = cc <= r ? __bfloat162float(dA[((long long)ch * 64 + I * 16 + r) * 64 + I * 16 + cc]) * scale : 0.f;
+  }
+  __syncthreads();
+  if (d >= dk) return;
+  // every row of the chunk lies within 32 bits of its first
+  const int rs = H * dk;
+  const long long base = ((long long)c * 64 * H + h) * dk + d, col = (long long)h * dk + d;
+  const long long g0 = row0 * to.ldg + col;
+  void* dgp = raw == nullptr ? (void*)((float*)dg + g0) : (void*)((__nv_bfloat16*)dg + g0);
+  auto rows = [&](auto full) {
+    gla_bwd_rows<decltype(full)::value, TPB>(q + row0 * at.ldq + col, k + row0 * at.ldk + col, b + base, dkhat + base, dqbar + base,
+                                        dqt + ((long long)c * 48 - 16) * rs + col,  // rows of sub-blocks 1..3 only, read at the others' offsets
+                                        dk3 + (long long)c * 144 * rs + col, dq + row0 * to.ldq + col, dk_ + row0 * to.ldk + col, dgp,
+                                        raw == nullptr ? nullptr : raw + row0 * at.ldg + col, norm, sA, sgb, rs, (int)at.ldq, (int)at.ldk, (int)at.ldg,
+                                        (int)to.ldq, (int)to.ldk, (int)to.ldg, n, dalpha[(long long)ch * dk + d], scale);
+  };
+  if (n == 64) rows(std::true_type{});
+  else rows(std::false_type{});
 }
 
 }  // namespace
 
 extern "C" {
 
-int fb_gla_scores(const void* q, int q32, const void* k, const float* b, const void* blk, void* A, int NC, int H, int dk, float scale,
-                  cudaStream_t stream) {
+// rows: src, ldq, ldk, ldg of GlaRows
+int fb_gla_scores(const void* q, int q32, const void* k, const float* b, const void* blk, void* A, const int* src, long long ldq, long long ldk, int NC,
+                  int H, int dk, float scale, cudaStream_t stream) {
   if (NC <= 0) return 0;
   if (!fb::aligned(16, blk, A)) return -2;
   constexpr int smem = 3 * 64 * GD_LD * 4;
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(gla_scores_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess ||
-        cudaFuncSetAttribute(gla_scores_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
-      return -2;
-    configured = true;
-  }
-  if (q32)
-    gla_scores_kernel<<<NC * H, GD_THREADS, smem, stream>>>((const float*)q, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)blk,
-                                                           (__nv_bfloat16*)A, H, dk, scale);
-  else
-    gla_scores_kernel<<<NC * H, GD_THREADS, smem, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)blk,
-                                                           (__nv_bfloat16*)A, H, dk, scale);
-  return fb::launch_ok("gla_scores_kernel");
+  const GlaRows at{src, ldq, ldk, 0};
+  const int vec = dk % 8 == 0 && ldq % 8 == 0 && ldk % 8 == 0 && fb::aligned(16, q, k, b);
+  auto launch = [&](auto kernel, auto* qq) -> int {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    kernel<<<NC * H, GD_THREADS, smem, stream>>>(qq, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)blk, (__nv_bfloat16*)A, at, H, dk, scale, vec);
+    return fb::launch_ok("gla_scores_kernel");
+  };
+  return q32 ? launch(gla_scores_kernel<float>, (const float*)q) : launch(gla_scores_kernel<__nv_bfloat16>, (const __nv_bfloat16*)q);
 }
 
 int fb_gla_bwd(const void* q, const void* k, const float* b, const void* dA, const void* dkhat, const void* dqbar, const void* dqt,
-               const void* dk3, const float* dalpha, void* dq, void* dk_, float* dg, int NC, int H, int dk, float scale, cudaStream_t stream) {
+               const void* dk3, const float* dalpha, void* dq, void* dk_, void* dg, const void* raw, float norm, const int* src, long long ldq,
+               long long ldk, long long ldg, long long lddq, long long lddk, long long lddg, int NC, int H, int dk, float scale, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  gla_bwd_kernel<<<dim3(NC * H, (dk + 127) / 128), 128, 0, stream>>>(
+  const int tpb = dk <= 64 ? 64 : 128;
+  const auto kernel = dk <= 64 ? gla_bwd_kernel<64> : gla_bwd_kernel<128>;
+  kernel<<<dim3(NC * H, (dk + tpb - 1) / tpb), tpb, 0, stream>>>(
       (const __nv_bfloat16*)q, (const __nv_bfloat16*)k, b, (const __nv_bfloat16*)dA, (const __nv_bfloat16*)dkhat, (const __nv_bfloat16*)dqbar,
-      (const __nv_bfloat16*)dqt, (const __nv_bfloat16*)dk3, dalpha, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk_, dg, H, dk, scale);
+      (const __nv_bfloat16*)dqt, (const __nv_bfloat16*)dk3, dalpha, (__nv_bfloat16*)dq, (__nv_bfloat16*)dk_, dg, (const __nv_bfloat16*)raw, norm,
+      GlaRows{src, ldq, ldk, ldg}, GlaRows{src, lddq, lddk, lddg}, H, dk, scale);
   return fb::launch_ok("gla_bwd_kernel");
 }
 
@@ -995,59 +1144,86 @@ extern "C" int fb_state_scan(const long long* first, const long long* last, int 
 // Every exponent is <= 0.
 namespace {
 
-// Bound by memory (24 bytes per channel and row, 0.12 ms at 65,536 tokens, 4 heads of 128).  A thread owns two channels: with
-// one, its 2-byte accesses took 0.25 ms; this takes 0.205.
-__global__ void __launch_bounds__(64, 10) gla_prep_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
-                                                          const float* __restrict__ g, float* __restrict__ b,
+// Bound by memory (24 bytes per channel and row, 0.12 ms at 65,536 tokens, 4 heads of 128).  A thread owns two channels of one
+// 16-row sub-block and loads all it needs of q, k and g before it uses any; the sub-blocks' sums meet in shared memory.  A
+// thread that walked the 64 rows of a chunk waited for memory sub-block after sub-block and read b back: 0.205 ms; this takes 0.155, with the gate's own arithmetic (0.05 by a kernel before).
+template <bool RAW>
+__global__ void __launch_bounds__(256, 2) gla_prep_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+                                                          const void* __restrict__ g, float norm, const GlaRows at, float* __restrict__ b,
                                                           __nv_bfloat16* __restrict__ khat, __nv_bfloat16* __restrict__ qbar,
                                                           __nv_bfloat16* __restrict__ qt, __nv_bfloat16* __restrict__ k3,
                                                           float* __restrict__ alpha, int H, int dk, float scale) {
-  const int d = blockIdx.y * 128 + 2 * threadIdx.x;
-  if (d >= dk) return;
+  __shared__ float2 total[4][64], first[4][64], last[64];
+  const int x = threadIdx.x & 63, Iq = threadIdx.x >> 6;
+  const int d = blockIdx.y * 128 + 2 * x;
+  const bool live = d < dk;
   const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
-  const long long rs = (long long)H * dk;                       // row stride
-  const long long base = ((long long)c * 64 * H + h) * dk + d;  // element (c, row 0, h, d)
-  auto put = [](__nv_bfloat16* p, long long off, float x, float y) {
-    *reinterpret_cast<__nv_bfloat162*>(p + off) = __floats2bfloat162_rn(x, y);
-  };
-  auto get = [](const __nv_bfloat16* p, long long off) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p + off)); };
-  float2 run = make_float2(0.f, 0.f), r[4];
+  long long row0;
+  int n;
+  gla_rows(at.src, c, row0, n);
+  const long long col = (long long)h * dk + d;
+  const __nv_bfloat16 *qp = q + (row0 + Iq * 16) * at.ldq + col, *kp = k + (row0 + Iq * 16) * at.ldk + col;
+  const int there = live ? n - Iq * 16 : 0;  // rows of this sub-block
+  uint32_t qv[16], kv[16];
+  float2 bv[16];
 #pragma unroll
-  for (int i0 = 0; i0 < 64; i0 += 16) {
-    float2 gv[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) gv[i] = *reinterpret_cast<const float2*>(g + base + (i0 + i) * rs);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      run.x += gv[i].x;
-      run.y += gv[i].y;
-      *reinterpret_cast<float2*>(b + base + (i0 + i) * rs) = run;
-      if (i == 0) r[i0 >> 4] = run;
+  for (int i = 0; i < 16; ++i) {
+    const long long o = (row0 + Iq * 16 + i) * at.ldg + col;
+    if constexpr (RAW) {
+      const uint32_t v = i < there ? *reinterpret_cast<const uint32_t*>((const __nv_bfloat16*)g + o) : 0u;
+      bv[i] = make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+    } else {
+      bv[i] = i < there ? *reinterpret_cast<const float2*>((const float*)g + o) : make_float2(0.f, 0.f);
     }
   }
-  const float2 b_last = run;
-  *reinterpret_cast<float2*>(alpha + (long long)ch * dk + d) = make_float2(__expf(b_last.x), __expf(b_last.y));
-  const long long k3base = (((long long)c * 3) * 48 * H + h) * dk + d;  // element (c, I-1 = 0, row 0, h, d)
-  const long long qtbase = ((long long)c * 48 * H + h) * dk + d;
-#pragma unroll 1  // b comes back from the cache: kept in registers it would leave room for a quarter of the blocks
-  for (int Iq = 0; Iq < 4; ++Iq) {
-    const float2 rq = Iq == 0 ? r[0] : (Iq == 1 ? r[1] : (Iq == 2 ? r[2] : r[3]));
-#pragma unroll 8
-    for (int ii = 0; ii < 16; ++ii) {
-      const int i = Iq * 16 + ii;
-      const long long off = base + i * rs;
-      const float2 bi = *reinterpret_cast<const float2*>(b + off);
-      const float2 qi = get(q, off), ki = get(k, off);
-      put(khat, off, ki.x * __expf(b_last.x - bi.x), ki.y * __expf(b_last.y - bi.y));
-      put(qbar, off, qi.x * __expf(bi.x) * scale, qi.y * __expf(bi.y) * scale);
-      if (Iq > 0) put(qt, qtbase + (i - 16) * rs, qi.x * __expf(bi.x - rq.x), qi.y * __expf(bi.y - rq.y));
-      if (Iq < 3) {
 #pragma unroll
-        for (int I = 1; I <= 3; ++I) {
-          const bool before = Iq < I;
-          put(k3, k3base + ((long long)(I - 1) * 48 + i) * rs, before ? ki.x * __expf(r[I].x - bi.x) : 0.f,
-              before ? ki.y * __expf(r[I].y - bi.y) : 0.f);
-        }
+  for (int i = 0; i < 16; ++i) {
+    qv[i] = i < there ? *reinterpret_cast<const uint32_t*>(qp + i * at.ldq) : 0u;
+    kv[i] = i < there ? *reinterpret_cast<const uint32_t*>(kp + i * at.ldk) : 0u;
+  }
+  float2 run = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    if (RAW) bv[i] = i < there ? make_float2(log_sigmoid(bv[i].x, norm), log_sigmoid(bv[i].y, norm)) : make_float2(0.f, 0.f);
+    run.x += bv[i].x;
+    run.y += bv[i].y;
+    bv[i] = run;
+  }
+  total[Iq][x] = run;
+  __syncthreads();
+  float2 pre = make_float2(0.f, 0.f);
+  for (int I = 0; I < Iq; ++I) pre.x += total[I][x].x, pre.y += total[I][x].y;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) bv[i].x += pre.x, bv[i].y += pre.y;
+  first[Iq][x] = bv[0];
+  if (Iq == 3) last[x] = bv[15];
+  __syncthreads();
+  if (!live) return;
+  const long long rs = (long long)H * dk;                                            // distance of padded rows
+  const long long base = ((long long)c * 64 + Iq * 16) * rs + col;                   // row 0 of the sub-block
+  const long long qtbase = ((long long)c * 48 + Iq * 16 - 16) * rs + col;
+  const long long k3base = ((long long)c * 3 * 48 + Iq * 16) * rs + col;             // (I - 1 = 0, row 0 of the sub-block)
+  const float2 b_last = last[x], rq = bv[0], r1 = first[1][x], r2 = first[2][x], r3 = first[3][x];
+  if (Iq == 0) *reinterpret_cast<float2*>(alpha + (long long)ch * dk + d) = make_float2(__expf(b_last.x), __expf(b_last.y));
+  auto put = [](__nv_bfloat16* p, long long off, float a, float e) {
+    *reinterpret_cast<__nv_bfloat162*>(p + off) = __floats2bfloat162_rn(a, e);
+  };
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const float2 bi = bv[i];
+    const float2 qi = make_float2(__uint_as_float(qv[i] << 16), __uint_as_float(qv[i] & 0xffff0000u));
+    const float2 ki = make_float2(__uint_as_float(kv[i] << 16), __uint_as_float(kv[i] & 0xffff0000u));
+    const long long off = base + i * rs;
+    *reinterpret_cast<float2*>(b + off) = bi;
+    put(khat, off, ki.x * __expf(b_last.x - bi.x), ki.y * __expf(b_last.y - bi.y));
+    put(qbar, off, qi.x * __expf(bi.x) * scale, qi.y * __expf(bi.y) * scale);
+    if (Iq > 0) put(qt, qtbase + i * rs, qi.x * __expf(bi.x - rq.x), qi.y * __expf(bi.y - rq.y));
+    if (Iq < 3) {
+#pragma unroll
+      for (int I = 1; I <= 3; ++I) {
+        const float2 r = I == 1 ? r1 : I == 2 ? r2 : r3;
+        const bool before = Iq < I;
+        put(k3, k3base + ((long long)(I - 1) * 48 + i) * rs, before ? ki.x * __expf(r.x - bi.x) : 0.f, before ? ki.y * __expf(r.y - bi.y) : 0.f);
       }
     }
   }
@@ -1057,13 +1233,17 @@ __global__ void __launch_bounds__(64, 10) gla_prep_fwd_kernel(const __nv_bfloat1
 
 extern "C" {
 
-int fb_gla_prep_fwd(const void* q, const void* k, const float* g, float* b, void* khat, void* qbar, void* qt, void* k3,
-                    float* alpha, int NC, int H, int dk, float scale, cudaStream_t stream) {
+// g: fp32 (raw 0), or bf16 with g = logsigmoid(raw) norm; src, ld*: see GlaRows
+int fb_gla_prep_fwd(const void* q, const void* k, const void* g, int raw, float norm, const int* src, long long ldq, long long ldk, long long ldg,
+                    float* b, void* khat, void* qbar, void* qt, void* k3, float* alpha, int NC, int H, int dk, float scale, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if ((dk & 1) || !fb::aligned(4, q, k, khat, qbar, qt, k3) || !fb::aligned(8, g, b, alpha)) return -2;
-  dim3 grid(NC * H, (dk + 127) / 128);
-  gla_prep_fwd_kernel<<<grid, 64, 0, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, g, b, (__nv_bfloat16*)khat,
-                                                (__nv_bfloat16*)qbar, (__nv_bfloat16*)qt, (__nv_bfloat16*)k3, alpha, H, dk, scale);
+  if ((dk & 1) || (ldq & 1) || (ldk & 1) || (ldg & 1) || !fb::aligned(4, q, k, khat, qbar, qt, k3) || !fb::aligned(8, b, alpha) ||
+      !fb::aligned(raw ? 4 : 8, g))
+    return -2;
+  const dim3 grid(NC * H, (dk + 127) / 128);
+  const auto kernel = raw ? gla_prep_fwd_kernel<true> : gla_prep_fwd_kernel<false>;
+  kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)q, (const __nv_bfloat16*)k, g, norm, GlaRows{src, ldq, ldk, ldg}, b, (__nv_bfloat16*)khat,
+                                   (__nv_bfloat16*)qbar, (__nv_bfloat16*)qt, (__nv_bfloat16*)k3, alpha, H, dk, scale);
   return fb::launch_ok("gla_prep_fwd_kernel");
 }
 

@@ -211,15 +211,22 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   if (w != nullptr && live) unpack8(*reinterpret_cast<const uint4*>(w + col), ww);
   const float inv_d = 1.f / (float)D;
   int flip = 0;
+  int ahead[MAP ? BR : 1];  // the next trip's `from`, on its way while this trip works: without it every trip waits twice
+  auto look = [&](long long rb) {
+#pragma unroll
+    for (int k = 0; k < BR; ++k) {
+      const long long row = rb + slot + k * SLOTS;
+      if (MAP) ahead[k] = row < row1 ? (int)mapped_row(at, row) : -1;
+    }
+  };
+  if (MAP) look(row0);
   for (long long rb = row0; rb < row1; rb += SLOTS * BR, flip ^= 1) {
     uint4 xa[BR], ga[BR], ra[HAS_DRES ? BR : 1], ta[GATE ? BR : 1];
     float rs[BR], c[BR];
     int from[MAP ? BR : 1];  // the packed row, -1 where there is none: its gradient is zero
 #pragma unroll
-    for (int k = 0; k < BR; ++k) {
-      const long long row = rb + slot + k * SLOTS;
-      if (MAP) from[k] = row < row1 ? (int)mapped_row(at, row) : -1;
-    }
+    for (int k = 0; k < (MAP ? BR : 1); ++k)
+      if (MAP) from[k] = ahead[k];
 #pragma unroll
     for (int k = 0; k < BR; ++k) {
       const long long row = rb + slot + k * SLOTS, pr = MAP ? from[k] : row;
@@ -232,6 +239,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
       if (GATE) ta[k] = ok ? __ldcs(reinterpret_cast<const uint4*>(gate + gate_at(at.heads, at.ldg, pr, D) + col)) : none;
       rs[k] = there ? rstd[pr] : 0.f;
     }
+    if (MAP) look(rb + SLOTS * BR);
 #pragma unroll
     for (int k = 0; k < BR; ++k) {
       float a[8], g[8];
@@ -345,9 +353,61 @@ __global__ void __launch_bounds__(32 * CS_GROUPS) colsum_partials_kernel(const f
   out[i] = accumulate ? out[i] + s : s;
 }
 
+// Column sums of a bf16 matrix (a bias' gradient): 256 columns x 8 groups of rows per block, four rows' loads in flight per thread.
+// 65,536 x 512: torch's reduction took 0.057 ms, the bytes take 0.010.
+constexpr int CB_ROWS = 8;
+__global__ void __launch_bounds__(32 * CB_ROWS) colsum_bf16_kernel(const __nv_bfloat16* __restrict__ x, long long ld, long long rows, int cols,
+                                                                   float* __restrict__ part) {
+  __shared__ float red[CB_ROWS][257];
+  const int col = (blockIdx.x * 32 + threadIdx.x) * 8;
+  float s[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) s[j] = 0.f;
+  if (col < cols) {
+    const long long step = (long long)gridDim.y * CB_ROWS;
+    for (long long r = (long long)blockIdx.y * CB_ROWS + threadIdx.y; r < rows; r += 4 * step) {
+      uint4 v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = r + k * step < rows ? *reinterpret_cast<const uint4*>(x + (r + k * step) * ld + col) : make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float f[8];
+        unpack8(v[k], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) s[j] += f[j];
+      }
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) red[threadIdx.y][threadIdx.x * 8 + j] = s[j];
+  __syncthreads();
+  const int t = threadIdx.y * 32 + threadIdx.x, c = blockIdx.x * 256 + t;
+  if (c >= cols) return;
+  float v = 0.f;
+#pragma unroll
+  for (int k = 0; k < CB_ROWS; ++k) v += red[k][t];
+  part[(long long)blockIdx.y * cols + c] = v;
+}
+
 }  // namespace
 
 extern "C" {
+
+int fb_colsum_bf16_parts(long long rows, int cols) {
+  const long long want = (rows + 4 * CB_ROWS - 1) / (4 * CB_ROWS), most = 592 / ((cols + 255) / 256);
+  return (int)(want < 1 ? 1 : want < most ? want : most < 1 ? 1 : most);
+}
+// out[cols] (fp32) = column sums of x [rows, cols] bf16, rows ld elements apart; part: fp32 [fb_colsum_bf16_parts, cols] scratch
+int fb_colsum_bf16(const void* x, long long ld, long long rows, int cols, float* part, float* out, cudaStream_t stream) {
+  if (cols == 0) return 0;
+  if ((cols & 7) || (ld & 7) || !fb::aligned(16, x)) return -2;
+  const int parts = fb_colsum_bf16_parts(rows, cols);
+  colsum_bf16_kernel<<<dim3((cols + 255) / 256, parts), dim3(32, CB_ROWS), 0, stream>>>((const __nv_bfloat16*)x, ld, rows, cols, part);
+  int rc = fb::launch_ok("colsum_bf16_kernel");
+  if (rc) return rc;
+  colsum_partials_kernel<<<(cols + 31) / 32, dim3(32, CS_GROUPS), 0, stream>>>(part, parts, cols, out, 0);
+  return fb::launch_ok("colsum_partials_kernel");
+}
 
 // Number of CTAs (= rows of the dw partial buffer) the backward launches for `rows` rows.
 int fb_rmsnorm_bwd_parts(long long rows) {

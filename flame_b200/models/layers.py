@@ -148,6 +148,7 @@ class GatedLinearAttention(nn.Module):
             self.g_norm = RMSNorm(self.head_v_dim, elementwise_affine, norm_eps)
 
     def forward(self, x: torch.Tensor, meta: VarlenMeta) -> torch.Tensor:
+        from ..ops.chunked import gla_raw_gate
         from ..ops.gla import gla
         H, G = self.num_heads, self.num_kv_groups
         tp = getattr(self, "tp", None)
@@ -170,8 +171,11 @@ class GatedLinearAttention(nn.Module):
             layers = (self.q_proj, self.k_proj, self.v_proj)
             # (torch's activations are several times slower on column blocks)
             whole = self.use_short_conv or self.feature_map is None
-            q, k, v = split_projections(x, layers) if whole else (l(x) for l in layers)
-            gk = self.gk_proj(x)
+            low = plain((self.gk_proj,), nn.Sequential)
+            more = ((self.g_proj,) if self.use_output_gate else ()) + ((self.gk_proj[0],) if low else ())
+            q, k, v, *rest = _projections(x, layers, more) if whole else (l(x) for l in (*layers, *more))
+            gk = self.gk_proj[1](rest[-1]) if low else self.gk_proj(x)
+            g_out = rest[0] if self.use_output_gate else None
         T = q.shape[0]
         if self.use_short_conv:
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
@@ -181,20 +185,24 @@ class GatedLinearAttention(nn.Module):
         v = reshaped(v, T, self.num_kv_heads, self.head_v_dim)
         if G > 1:
             k, gk, v = (t.repeat_interleave(G, 1) for t in (k, gk, v))
-        gk = logsigmoid_gate(gk, self.gate_logit_normalizer)
-        if self.clamp_min is not None:
-            gk = gk.clamp_min(self.clamp_min)
         if self.feature_map is not None:
             q, k = _feature_map(self.feature_map, q), _feature_map(self.feature_map, k)
-        o = gla(q, k, v, gk, meta)
+        o, lay = (gla_raw_gate(q, k, v, gk, self.gate_logit_normalizer, meta) if self.clamp_min is None else None) or (None, None)
+        if o is None:
+            gk = logsigmoid_gate(gk, self.gate_logit_normalizer)
+            if self.clamp_min is not None:
+                gk = gk.clamp_min(self.clamp_min)
+            o = gla(q, k, v, gk, meta)
         if self.use_output_gate:
-            g = g_out if g_out is not None else self.g_proj(x)
             if self.fuse_norm_and_gate:
-                o = self.g_norm_swish_gate(o.contiguous(), g.reshape(T, H, self.head_v_dim).contiguous()).reshape(T, self.value_dim)
+                g = reshaped(g_out, T, H, self.head_v_dim)
+                o = self.g_norm_swish_gate(o, g) if lay is None else norm_chunks(self.g_norm_swish_gate, o, lay, g)
+                o = o.reshape(T, self.value_dim)
             else:
-                o = self.g_norm(o).reshape(T, self.value_dim) * F.silu(g)
+                o = o if lay is None else lay.unpack(o)
+                o = self.g_norm(o).reshape(T, self.value_dim) * F.silu(g_out)
         else:
-            o = self.g_norm(o).reshape(T, self.value_dim)
+            o = (self.g_norm(o) if lay is None else norm_chunks(self.g_norm, o, lay)).reshape(T, self.value_dim)
         if tp is not None:
             from ..parallel.tensor_parallel import linear_reduce_scatter
             return linear_reduce_scatter(o, self.o_proj.weight)

@@ -116,28 +116,59 @@ def scores_bwd(dQ, Q, b, db, scale: float):
     return gq
 
 
-_lib.register("fb_gla_scores", [c_void_p, c_int] + [c_void_p] * 4 + [c_int] * 3 + [c_float, c_void_p])
-_lib.register("fb_gla_bwd", [c_void_p] * 12 + [c_int] * 3 + [c_float, c_void_p])
+_lib.register("fb_gla_scores", [c_void_p, c_int] + [c_void_p] * 5 + [c_longlong] * 2 + [c_int] * 3 + [c_float, c_void_p])
+_lib.register("fb_gla_bwd", [c_void_p] * 13 + [c_float, c_void_p] + [c_longlong] * 6 + [c_int] * 3 + [c_float, c_void_p])
 
 
-def gla_scores(q, k, b, blk, scale: float) -> torch.Tensor:
+def _token_ld(x: torch.Tensor) -> int:
+    """Elements between the tokens of ``[T, H, d]`` (of one token its length, whatever stride torch keeps for it)."""
+    return x.stride(0) if x.shape[0] > 1 else x.shape[1] * x.shape[2]
+
+
+def token_rows(x: torch.Tensor) -> torch.Tensor:
+    """``x [T, H, d]``, or a dense copy: a token's values side by side, tokens whole 16-byte vectors apart, on a 16-byte boundary."""
+    H, d = x.shape[1:]
+    ld, e = _token_ld(x), x.element_size()
+    ok = (d == 1 or x.stride(2) == 1) and (H == 1 or x.stride(1) == d) and ld >= H * d and ld * e % 16 == 0 and x.data_ptr() % 16 == 0
+    return x if ok else _lib.dense(x)
+
+
+def _gla_rows(q, k, lay):
+    """Arguments of ``csrc/chunk.cu: GlaRows`` for q and k: packed tokens of ``lay``, or padded rows ``[NC, 64, H, d]`` (None)."""
+    if lay is None:
+        n = q.shape[2] * q.shape[3]
+        return 0, n, n
+    return lay.inv_i32.data_ptr(), _token_ld(q), _token_ld(k)
+
+
+def gla_scores(q, k, b, blk, scale: float, lay=None) -> torch.Tensor:
     """bf16 ``A [NC, H, 64, 64]``: diagonal 16 x 16 sub-blocks computed here, the ones left of them from ``blk [3 NC, H, 16, 48]``
-    bf16; q (or fp32), k ``[NC, 64, H, dk]`` bf16, b fp32, all contiguous."""
-    NC, _, H, dk = q.shape
+    bf16; q (or fp32), k bf16: contiguous ``[NC, 64, H, dk]``, or with ``lay`` packed ``token_rows``; b fp32 contiguous."""
+    NC, _, H, dk = b.shape
     A = torch.empty(NC, H, 64, 64, dtype=torch.bfloat16, device=q.device)
-    _lib.check(_lib.lib().fb_gla_scores(q.data_ptr(), int(q.dtype == torch.float32), k.data_ptr(), b.data_ptr(), blk.data_ptr(), A.data_ptr(), NC, H, dk, float(scale),
-                                        _lib.stream_ptr()), "fb_gla_scores")
+    src, ldq, ldk = _gla_rows(q, k, lay)
+    _lib.check(_lib.lib().fb_gla_scores(q.data_ptr(), int(q.dtype == torch.float32), k.data_ptr(), b.data_ptr(), blk.data_ptr(), A.data_ptr(),
+                                        src, ldq, ldk, NC, H, dk, float(scale), _lib.stream_ptr()), "fb_gla_scores")
     _lib.count_launch()
     return A
 
 
-def gla_bwd(q, k, b, dA, dkhat, dqbar, dqt, dk3, dalpha, scale: float):
-    """``dq, dk`` (bf16) and ``dg`` (fp32) of a chunk (see ``csrc/chunk.cu: gla_bwd_kernel``); every operand contiguous."""
-    NC, _, H, dk = q.shape
-    dq, dk_, dg = torch.empty_like(q), torch.empty_like(k), torch.empty_like(b)
+def gla_bwd(q, k, b, dA, dkhat, dqbar, dqt, dk3, dalpha, scale: float, lay=None, raw=None, norm: float = 1.0, grads=(None, None)):
+    """``dq, dk`` (bf16) and ``dg`` of a chunk (see ``csrc/chunk.cu: gla_bwd_kernel``): fp32, or with ``raw`` that of the gate's bf16 argument.
+    With ``lay`` q, k, ``raw`` and the gradients are packed tokens; ``grads``: where dq and dk belong ``[T, H, dk]``."""
+    NC, _, H, dk = b.shape
+    if lay is None:
+        dq, dk_, dg = torch.empty_like(q), torch.empty_like(k), torch.empty_like(b)
+        lds = [H * dk] * 6
+    else:
+        new = lambda dt: torch.empty(lay.T, H, dk, dtype=dt, device=q.device)  # noqa: E731
+        dq, dk_ = (new(torch.bfloat16) if t is None else t for t in grads)
+        dg = new(torch.float32 if raw is None else torch.bfloat16)
+        lds = [_token_ld(q), _token_ld(k), H * dk if raw is None else _token_ld(raw), _token_ld(dq), _token_ld(dk_), H * dk]
     _lib.check(_lib.lib().fb_gla_bwd(q.data_ptr(), k.data_ptr(), b.data_ptr(), dA.data_ptr(), dkhat.data_ptr(), dqbar.data_ptr(),
-                                     dqt.data_ptr(), dk3.data_ptr(), dalpha.data_ptr(), dq.data_ptr(), dk_.data_ptr(), dg.data_ptr(), NC,
-                                     H, dk, float(scale), _lib.stream_ptr()), "fb_gla_bwd")
+                                     dqt.data_ptr(), dk3.data_ptr(), dalpha.data_ptr(), dq.data_ptr(), dk_.data_ptr(), dg.data_ptr(), _lib.ptr(raw),
+                                     1.0 / float(norm), 0 if lay is None else lay.inv_i32.data_ptr(), *lds, NC, H, dk, float(scale), _lib.stream_ptr()),
+               "fb_gla_bwd")
     _lib.count_launch()
     return dq, dk_, dg
 
@@ -222,23 +253,23 @@ def state_scan(first: torch.Tensor, last: torch.Tensor, alpha: torch.Tensor, x: 
     return out
 
 
-_lib.register("fb_gla_prep_fwd", [c_void_p] * 9 + [c_int, c_int, c_int, c_float, c_void_p])
+_lib.register("fb_gla_prep_fwd", [c_void_p] * 3 + [c_int, c_float, c_void_p] + [c_longlong] * 3 + [c_void_p] * 6 + [c_int] * 3 + [c_float, c_void_p])
 
 
-def gla_prep(qp, kp, gp, scale: float):
+def gla_prep(q, k, g, scale: float, lay=None, norm=None):
     """One pass over a chunk's q, k, g producing the cumulative decay and every scaled operand of the GLA chunk algorithm (see
-    ``csrc/chunk.cu: gla_prep_fwd_kernel``).  q, k ``[NC, 64, H, dk]`` bf16, g ``[NC, 64, H, dk]`` fp32, all contiguous.  Returns
+    ``csrc/chunk.cu: gla_prep_fwd_kernel``).  q, k ``[NC, 64, H, dk]`` bf16, g fp32, all contiguous; with ``lay`` they are packed
+    ``token_rows [T, H, dk]``, and with ``norm`` too g is the bf16 argument of ``logsigmoid(g) / norm``.  Returns
     ``(b, khat, qbar, qt, k3, alpha)``; qt ``[NC, 48, H, dk]``."""
-    NC, C, H, dk = qp.shape
-    assert C == 64 and qp.dtype == torch.bfloat16 and gp.dtype == torch.float32
-    dev = qp.device
-    b = torch.empty_like(gp)
-    khat, qbar, qt = torch.empty_like(kp), torch.empty_like(qp), torch.empty(NC, 48, H, dk, dtype=torch.bfloat16, device=dev)
-    k3 = torch.empty(NC, 3, 48, H, dk, dtype=torch.bfloat16, device=dev)
-    alpha = torch.empty(NC, H, dk, dtype=torch.float32, device=dev)
-    rc = _lib.lib().fb_gla_prep_fwd(qp.data_ptr(), kp.data_ptr(), gp.data_ptr(), b.data_ptr(), khat.data_ptr(),
-                                    qbar.data_ptr(), qt.data_ptr(), k3.data_ptr(), alpha.data_ptr(), NC, H, dk,
-                                    float(scale), _lib.stream_ptr())
+    NC, (H, dk), dev = q.shape[0] if lay is None else lay.NC, q.shape[-2:], q.device
+    assert q.dtype == k.dtype == torch.bfloat16 and g.dtype == (torch.float32 if norm is None else torch.bfloat16)
+    new = lambda *n, dt=torch.bfloat16: torch.empty(*n, H, dk, dtype=dt, device=dev)  # noqa: E731
+    b, khat, qbar, qt, k3 = new(NC, 64, dt=torch.float32), new(NC, 64), new(NC, 64), new(NC, 48), new(NC, 3, 48)
+    alpha = new(NC, dt=torch.float32)
+    src, ldq, ldk = _gla_rows(q, k, lay)
+    rc = _lib.lib().fb_gla_prep_fwd(q.data_ptr(), k.data_ptr(), g.data_ptr(), int(norm is not None), 1.0 / float(norm or 1.0), src, ldq, ldk,
+                                    H * dk if lay is None else _token_ld(g), b.data_ptr(), khat.data_ptr(), qbar.data_ptr(), qt.data_ptr(),
+                                    k3.data_ptr(), alpha.data_ptr(), NC, H, dk, float(scale), _lib.stream_ptr())
     _lib.check(rc, "fb_gla_prep_fwd")
     _lib.count_launch()
     return b, khat, qbar, qt, k3, alpha

@@ -730,35 +730,44 @@ def scalar_gla_tc(q, k, v, g, meta: VarlenMeta, scale: float = 1.0, chunk: Optio
 
 
 class _Gla(torch.autograd.Function):
-    """The whole chunk pipeline of gated linear attention on packed 64-token chunks, on the kernels: q, k ``[NC, 64, H, dk]``, v
-    ``[NC, 64, H, dv]`` bf16, g ``[NC, 64, H, dk]`` fp32.  One node, so that the two halves of the output and of dv accumulate in
-    one GEMM each, and the channel-wise backward of preparation and diagonal sub-blocks is one kernel."""
+    """The whole chunk pipeline of gated linear attention on 64-token chunks, on the kernels: v ``[NC, 64, H, dv]`` bf16; q, k ``[NC, 64, H, dk]``
+    bf16 and g fp32 there too, or with ``tokens`` packed ``[T, H, dk]`` (``norm``: g is then the bf16 argument of ``logsigmoid(g) / norm``), which
+    the kernels read, and whose gradients they write, where they lie.  One node, so that the two halves of the output and of dv
+    accumulate in one GEMM each, and the channel-wise backward of preparation and diagonal sub-blocks is one kernel."""
 
     @staticmethod
-    def forward(ctx, q, k, v, g, scale, lay):
+    def forward(ctx, q, k, v, g, scale, lay, tokens, norm):
         from . import chunk_kernels
-        q, k, v, g = (_lib.dense(t) for t in (q, k, v, g))
-        NC, C, H, dk = q.shape
-        dv = v.shape[-1]
-        b, khat, qbar, qt, k3, alpha = chunk_kernels.gla_prep(q, k, g, scale)
+        v, rows = _lib.dense(v), lay if tokens else None
+        ctx.slots = None, None
+        if tokens:
+            ctx.slots = slots.of(q), slots.of(k)
+            q, k, g = (chunk_kernels.token_rows(t) for t in (q, k, g))
+        else:
+            q, k, g = (_lib.dense(t) for t in (q, k, g))
+        (NC, C, H, dv), dk = v.shape, q.shape[-1]
+        b, khat, qbar, qt, k3, alpha = chunk_kernels.gla_prep(q, k, g, scale, rows, norm)
         vh = _hm(v)
         S = _state_scan(lay, alpha, bgemm(_hm(khat), vh, a_mn=True, b_mn=True, out_dtype=torch.float32), q.dtype, reverse=False)
         # off-diagonal sub-blocks: batch (chunk, I) multiplies the 16 query rows of sub-block I, re-based on the sub-block's
         # first row, with the keys before it re-based on the same row; later keys are zero in k3
         qt3 = qt.view(NC * 3, 16, H, dk)
         k3 = k3.view(NC * 3, 48, H, dk)
-        A = chunk_kernels.gla_scores(q, k, b, bgemm(_hm(qt3), _hm(k3), alpha=scale), scale)
+        A = chunk_kernels.gla_scores(q, k, b, bgemm(_hm(qt3), _hm(k3), alpha=scale), scale, rows)
         o = bgemm(_hm(qbar), S, b_mn=True, more=[(A, vh, False, True, 1)], out=_token_major(NC, H, C, dv, q.dtype, q.device))
-        ctx.save_for_backward(q, k, v, b, khat, qbar, qt3, k3, alpha, S, A)
-        ctx.cfg = (scale, lay)
+        ctx.save_for_backward(q, k, v, b, khat, qbar, qt3, k3, alpha, S, A, None if norm is None else g)
+        ctx.cfg = (scale, lay, rows, norm)
         return o.permute(0, 2, 1, 3)
 
     @staticmethod
     def backward(ctx, do):
         from . import chunk_kernels
-        q, k, v, b, khat, qbar, qt3, k3, alpha, S, A = ctx.saved_tensors
-        scale, lay = ctx.cfg
-        NC, C, H, dk = q.shape
+        q, k, v, b, khat, qbar, qt3, k3, alpha, S, A, raw = ctx.saved_tensors
+        scale, lay, rows, norm = ctx.cfg
+        if rows is not None:  # saved-tensor hooks hand back copies, which lie wherever they were put
+            q, k = chunk_kernels.token_rows(q), chunk_kernels.token_rows(k)
+            raw = None if raw is None else chunk_kernels.token_rows(raw)
+        NC, C, H, dk = b.shape
         dv = v.shape[-1]
         dt, dev = q.dtype, q.device
         doh, vh = _hm(_lib.dense(do.to(dt))), _hm(v)
@@ -768,15 +777,17 @@ class _Gla(torch.autograd.Function):
         Ln = _state_scan(lay, alpha, bgemm(_hm(qbar), doh, a_mn=True, b_mn=True), dt, reverse=True)
         dvv = bgemm(_hm(khat), Ln, b_mn=True, more=[(A, doh, True, True, 1)], out=tok(dv)) if need_v else None
         if not (need_q or need_k or need_g):
-            return None, None, back(dvv), None, None, None
+            return None, None, back(dvv), None, None, None, None, None
         # one kernel forms the other three gradients, whichever of them are wanted
         dA = bgemm(doh, vh, mask=MASK_TRIL)
         dqbar, dkhat = bgemm(doh, S, out=tok(dk)), bgemm(vh, Ln, out=tok(dk))
         dblk = dA.view(NC, H, 4, 16, 64)[:, :, 1:, :, :48].permute(0, 2, 1, 3, 4).reshape(NC * 3, H, 16, 48)
         dqt3 = bgemm(dblk, _hm(k3), b_mn=True, alpha=scale, out=_token_major(NC * 3, H, 16, dk, dt, dev))
         dk3 = bgemm(dblk, _hm(qt3), a_mn=True, b_mn=True, alpha=scale, out=_token_major(NC * 3, H, 48, dk, dt, dev))
-        dq, dkk, dg = chunk_kernels.gla_bwd(q, k, b, dA, back(dkhat), back(dqbar), back(dqt3), back(dk3), _pair_dot(Ln, S, per_row=True), scale)
-        return dq, dkk, back(dvv), dg, None, None
+        grads = [None if s is None else s.take(lay.T, H * dk, dt, dev).view(lay.T, H, dk) for s in ctx.slots]
+        dq, dkk, dg = chunk_kernels.gla_bwd(q, k, b, dA, back(dkhat), back(dqbar), back(dqt3), back(dk3), _pair_dot(Ln, S, per_row=True), scale,
+                                            rows, raw, norm or 1.0, grads)
+        return dq, dkk, back(dvv), dg, None, None, None, None
 
 
 def _gla_diag(qp, kp, b, scale, sub: int = 16):
@@ -792,6 +803,23 @@ def _gla_diag(qp, kp, b, scale, sub: int = 16):
     return A
 
 
+def gla_raw_gate(q, k, v, raw, norm: float, meta: VarlenMeta, scale: Optional[float] = None):
+    """``gla_tc`` with the gate ``logsigmoid(raw) / norm`` formed inside, from bf16 q, k, raw ``[T, H, dk]``, v ``[T, H, dv]``: the result, still
+    in the rows of the layout, and the layout; None where the kernels do not apply."""
+    if not (_lib.available() and q.is_cuda and all(t.dtype == torch.bfloat16 for t in (q, k, v, raw)) and q.shape == k.shape == raw.shape
+            and q.shape[2] % 2 == 0 and getattr(meta, "sequence_slice", None) is None):
+        return None
+    lay = ChunkLayout.of(meta)
+    if q.shape[0] != lay.T:
+        return None
+    return _gla_raw_gate(q, k, v, raw, q.shape[-1] ** -0.5 if scale is None else scale, lay, float(norm)), lay
+
+
+@_recomputable
+def _gla_raw_gate(q, k, v, raw, scale: float, lay: "ChunkLayout", norm: float) -> torch.Tensor:
+    return _Gla.apply(q, k, lay.pack(v), raw, scale, lay, True, norm)
+
+
 @_recomputable
 def gla_tc(q, k, v, g, meta: VarlenMeta, scale: Optional[float] = None, sub: int = 16) -> torch.Tensor:
     """Chunked gated linear attention with one log decay per key channel: q, k, g ``[T, H, dk]``, v ``[T, H, dv]``.
@@ -802,14 +830,17 @@ def gla_tc(q, k, v, g, meta: VarlenMeta, scale: Optional[float] = None, sub: int
     scale = dk ** -0.5 if scale is None else scale
     lay = ChunkLayout.of(meta)
     dt = torch.bfloat16 if q.is_cuda else q.dtype
-    qp, kp, vp = lay.pack(q).to(dt), lay.pack(k).to(dt), lay.pack(v).to(dt)   # [NC, 64, H, d]
     C = lay.chunk
+    if _lib.available() and q.is_cuda and C == 64 and sub == 16:
+        if q.dtype == k.dtype == dt and q.shape[0] == lay.T:
+            o = _Gla.apply(q, k, lay.pack(v).to(dt), g.float(), scale, lay, True, None)
+        else:
+            o = _Gla.apply(*(lay.pack(t).to(dt) for t in (q, k, v)), lay.pack(g.float()), scale, lay, False, None)
+        return lay.unpack(o).to(v.dtype)
+    qp, kp, vp = lay.pack(q).to(dt), lay.pack(k).to(dt), lay.pack(v).to(dt)   # [NC, 64, H, d]
     nb = C // sub
     NC = qp.shape[0]
     ncol = C - sub
-    if _lib.available() and q.is_cuda and C == 64 and sub == 16:
-        o = _Gla.apply(qp, kp, vp, lay.pack(g.float()), scale, lay)
-        return lay.unpack(o).to(v.dtype)
     b = lay.pack(g.float()).cumsum(1)                                          # [NC, 64, H, dk]
     b_last = b[:, -1]                                                          # [NC, H, dk]
     alpha = b_last.exp()
@@ -930,7 +961,7 @@ def _gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> torch.Tensor:
     gp = lay.pack(g.float())
     written, read = _TwoReaders.apply(lay.pack(s), dt)
     qv = _VDecay.apply(qp, kp, written, gp, scale, True, lay)
-    return lay.unpack(_Gla.apply(qv, read, vp, gp, 1.0, lay)).to(v.dtype)
+    return lay.unpack(_Gla.apply(qv, read, vp, gp, 1.0, lay, False, None)).to(v.dtype)
 
 
 @_recomputable

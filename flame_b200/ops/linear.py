@@ -10,6 +10,7 @@ are kept for checkpoints (fla/layers/attn.py:73-82, fla/modules/mlp.py:58-60 use
 """
 from __future__ import annotations
 
+from ctypes import c_int, c_longlong, c_void_p
 from typing import Optional, Sequence
 
 import torch
@@ -21,13 +22,11 @@ from .gemm import gemm_nn, gemm_nt, gemm_tn
 
 def _adjacent(ts: Sequence[torch.Tensor]) -> bool:
     for a, b in zip(ts[:-1], ts[1:]):
-        if not (a.is_contiguous() and b.is_contiguous()):
+        if a.data_ptr() + a.numel() * a.element_size() != b.data_ptr():
             return False
-        if a.dtype != b.dtype or a.shape[1:] != b.shape[1:]:
+        if not (a.is_contiguous() and b.is_contiguous()) or a.dtype != b.dtype or a.shape[1:] != b.shape[1:]:
             return False
         if a.untyped_storage().data_ptr() != b.untyped_storage().data_ptr():
-            return False
-        if a.storage_offset() + a.numel() != b.storage_offset():
             return False
     return True
 
@@ -36,13 +35,10 @@ def _cat_view(ts: Sequence[torch.Tensor]) -> torch.Tensor:
     """Adjacent tensors (``_adjacent``) as one."""
     first, last = ts[0], ts[-1]
     rows = sum(t.shape[0] for t in ts)
-    # ``set_`` would grow a storage that is too small and hand out what happens to lie there
     if last.data_ptr() - first.data_ptr() != (rows - last.shape[0]) * first.stride(0) * first.element_size() or \
             first.untyped_storage().data_ptr() != last.untyped_storage().data_ptr():
         raise ValueError("not adjacent in memory")
-    out = torch.empty(0, dtype=first.dtype, device=first.device)
-    out.set_(first.untyped_storage(), first.storage_offset(), (rows, *first.shape[1:]), first.stride())
-    return out
+    return first.as_strided((rows, *first.shape[1:]), first.stride())  # stays within the storage, or raises
 
 
 def _operands_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
@@ -56,6 +52,24 @@ def _kernel_ok(x: torch.Tensor, w: torch.Tensor) -> bool:
 def _matrix(rows: int, cols: int, like: torch.Tensor) -> torch.Tensor:
     """``[rows, cols]`` whose rows are whole 16-byte vectors apart, as the GEMM's operands have to be."""
     return torch.empty(rows, -(-cols // 8) * 8, dtype=like.dtype, device=like.device)[:, :cols]
+
+
+_lib.register("fb_colsum_bf16_parts", [c_longlong, c_int])
+_lib.register("fb_colsum_bf16", [c_void_p, c_longlong, c_longlong, c_int, c_void_p, c_void_p, c_void_p])
+
+
+def _column_sums(x: torch.Tensor) -> torch.Tensor:
+    """fp32 sums over the rows of ``x [T, N]``."""
+    T, N = x.shape
+    if not (_lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and N % 8 == 0 and N > 0 and x.stride(1) == 1
+            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0):
+        return x.sum(0, dtype=torch.float32)
+    L = _lib.lib()
+    part = torch.empty(L.fb_colsum_bf16_parts(T, N), N, dtype=torch.float32, device=x.device)
+    out = torch.empty(N, dtype=torch.float32, device=x.device)
+    _lib.check(L.fb_colsum_bf16(x.data_ptr(), x.stride(0), T, N, part.data_ptr(), out.data_ptr(), _lib.stream_ptr()), "fb_colsum_bf16")
+    _lib.count_launch(2)
+    return out
 
 
 class _LinearFn(torch.autograd.Function):
@@ -159,7 +173,7 @@ class _LinearFn(torch.autograd.Function):
                 c += w.shape[0]
         gb = None
         if ctx.has_bias and ctx.needs_input_grad[1]:
-            gb = dy2.sum(0, dtype=torch.float32).to(dy.dtype)
+            gb = _column_sums(dy2).to(dy.dtype)
         return (dx, gb, None, *grads)
 
 
@@ -245,8 +259,6 @@ def linear_fused(x: torch.Tensor, weights: Sequence[torch.Tensor]) -> torch.Tens
 # --------------------------------------------------------------------------------------------------------------
 # gate | up projection with the SwiGLU activation in the GEMM epilogue
 # --------------------------------------------------------------------------------------------------------------
-from ctypes import c_int, c_longlong, c_void_p  # noqa: E402
-
 _lib.register("fb_gemm2_swiglu", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                                   c_longlong, c_longlong, c_int, c_void_p])
 
