@@ -37,9 +37,14 @@ def cuda_present() -> bool:
     return _CUDA_SEEN
 
 
+# ``os.environ.get`` of a variable that is not set raises and catches a KeyError inside; C's getenv sees the same environment
+_getenv = ctypes.PyDLL(None).getenv
+_getenv.argtypes, _getenv.restype = [ctypes.c_char_p], ctypes.c_char_p
+
+
 def available() -> bool:
-    """True when kernels of this library should be used (a CUDA device is present)."""
-    return cuda_present() and os.environ.get("FLAME_B200_FORCE_REFERENCE", "0") != "1"
+    """True when kernels of this library should be used (a CUDA device is present).  Asked several times by every op."""
+    return cuda_present() and _getenv(b"FLAME_B200_FORCE_REFERENCE") != b"1"
 
 
 def lib() -> ctypes.CDLL:
@@ -68,8 +73,9 @@ def reset_launches() -> None:
 
 
 def stream_ptr() -> int:
-    # the raw handle: a Stream object per launch costs more than the launch's own arguments
-    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    # the raw handle: a Stream object per launch costs more than the launch's own arguments (whoever asks has tensors on the
+    # device, so there is nothing left to initialise)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ptr(t: Optional[torch.Tensor]) -> int:

@@ -16,8 +16,8 @@ fla/ops/common/chunk_o.py, fla/ops/gated_delta_rule/wy_fast.py).
 """
 from __future__ import annotations
 
-import ctypes
-from ctypes import POINTER, c_float, c_int, c_longlong, c_void_p
+import struct
+from ctypes import c_char_p, c_int, c_void_p
 from typing import Optional, Sequence
 
 import torch
@@ -25,43 +25,28 @@ import torch
 from . import _lib
 
 
-class _Operand(ctypes.Structure):
-    _fields_ = [("ptr", c_void_p), ("ld", c_longlong), ("stride_lo", c_longlong), ("stride_hi", c_longlong),
-                ("n_lo", c_int), ("n_hi", c_int), ("mn", c_int), ("lo_div", c_int), ("hi_offset", c_int),
-                ("hi_index", c_void_p), ("k", c_int), ("neg", c_int)]
-
-
-class _Epilogue(ctypes.Structure):
-    _fields_ = [("C", c_void_p), ("ldc", c_longlong), ("stride_lo", c_longlong), ("stride_hi", c_longlong),
-                ("c_lo_div", c_int), ("c_hi_offset", c_int), ("c_hi_index", c_void_p),
-                ("Cin", c_void_p), ("cin_hi_offset", c_int), ("cin_hi_index", c_void_p), ("gamma", c_void_p),
-                ("C16", c_void_p), ("c16_hi_offset", c_int), ("c16_hi_index", c_void_p),
-                ("add16", c_void_p), ("add16_hi_offset", c_int), ("add16_hi_index", c_void_p),
-                ("ld16", c_longlong), ("stride_lo16", c_longlong), ("stride_hi16", c_longlong),
-                ("decay", c_void_p), ("d_hi", c_longlong), ("d_lo", c_longlong), ("d_r", c_longlong),
-                ("rowscale", c_void_p), ("r_hi", c_longlong), ("r_lo", c_longlong), ("r_r", c_longlong),
-                ("alpha", c_float), ("out_mode", c_int), ("mask_mode", c_int)]
-
-
-_lib.register("fb_bgemm_bf16", [POINTER(_Operand), c_int, POINTER(_Epilogue), c_int, c_int, c_int, c_int, c_int,
-                                c_void_p])
+# ``FbBOperand`` and ``FbBEpilogue`` of csrc/bgemm.cu, packed in one go: filling ctypes structures field by field took as long as
+# the rest of a call
+_OPERAND = struct.Struct("@PqqqiiiiiPii")
+_EPILOGUE = struct.Struct("@PqqqiiPPiPPPiPPiPqqqPqqqPqqqfii4x")
+_lib.register("fb_bgemm_bf16", [c_char_p, c_int, c_char_p, c_int, c_int, c_int, c_int, c_int, c_void_p])
 
 MASK_NONE, MASK_TRIL, MASK_STRICT = 0, 1, 2
 
 
-def _use_kernel(*ts: torch.Tensor) -> bool:
-    return _lib.available() and all(t.is_cuda for t in ts)
-
-
-def _inner_contig(t: torch.Tensor) -> torch.Tensor:
-    """Kernel operands need inner stride 1, 16-byte aligned rows/batches and no broadcast (stride 0) batch dims."""
-    ok = t.stride(-1) == 1 and t.data_ptr() % 16 == 0 and all(s % 8 == 0 and s > 0 for s in t.stride()[:-1])
-    return t if ok else t.contiguous()
-
-
-def _operand(t: torch.Tensor, mn: bool, lo_div: int, index: Optional[torch.Tensor], offset: int, neg: bool = False) -> _Operand:
-    return _Operand(t.data_ptr(), t.stride(2), t.stride(1), t.stride(0), t.shape[1], t.shape[0], int(mn), lo_div, offset,
-                    _lib.ptr(index), t.shape[2] if mn else t.shape[3], int(neg))
+def _operand(t: torch.Tensor, mn: bool, n_op: int, index: Optional[torch.Tensor], offset: int, neg: bool, hold: list) -> bytes:
+    """Kernel operands need inner stride 1, 16-byte aligned rows/batches and no broadcast (stride 0) batch dims; a copy that has them
+    is put into ``hold``."""
+    hi, lo, rows, inner = t.shape
+    s0, s1, s2, s3 = t.stride()
+    ptr = t.data_ptr()
+    if s3 != 1 or ptr & 15 or (s0 | s1 | s2) & 7 or min(s0, s1, s2) <= 0:
+        t = t.contiguous()
+        hold.append(t)
+        s0, s1, s2, _ = t.stride()
+        ptr = t.data_ptr()
+    assert t.dtype == torch.bfloat16
+    return _OPERAND.pack(ptr, s2, s1, s0, lo, hi, mn, n_op // lo, offset, 0 if index is None else index.data_ptr(), rows if mn else inner, neg)
 
 
 def _mkn(a, b, a_mn, b_mn):
@@ -116,20 +101,12 @@ def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = 
         assert out.dtype == torch.float32
     if n_hi == 0:
         return out
-    if _use_kernel(a, b):
-        a = _inner_contig(a)
-        b = _inner_contig(b)
-        assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
-        ops = (_Operand * (2 + 2 * len(more)))()
-        ops[0] = _operand(a, a_mn, n_op // a.shape[1], a_index, a_offset)
-        ops[1] = _operand(b, b_mn, n_op // b.shape[1], b_index, b_offset)
-        hold = []
-        for i, (ai, bi, ai_mn, bi_mn, sign) in enumerate(more):
-            assert _mkn(ai, bi, ai_mn, bi_mn)[:2] == (M, N) and ai.dtype == bi.dtype == torch.bfloat16
-            ai, bi = _inner_contig(ai), _inner_contig(bi)
-            hold.append((ai, bi))
-            ops[2 + 2 * i] = _operand(ai, ai_mn, n_op // ai.shape[1], None, 0, sign < 0)
-            ops[3 + 2 * i] = _operand(bi, bi_mn, n_op // bi.shape[1], None, 0)
+    if a.is_cuda and b.is_cuda and _lib.available():
+        hold: list = []  # copies live until the launch
+        ops = _operand(a, a_mn, n_op, a_index, a_offset, False, hold) + _operand(b, b_mn, n_op, b_index, b_offset, False, hold)
+        for ai, bi, ai_mn, bi_mn, sign in more:
+            assert _mkn(ai, bi, ai_mn, bi_mn)[:2] == (M, N)
+            ops += _operand(ai, ai_mn, n_op, None, 0, sign < 0, hold) + _operand(bi, bi_mn, n_op, None, 0, False, hold)
         r_hi = r_lo = r_r = 0
         if rowscale is not None:
             assert rowscale.dtype == torch.float32 and rowscale.shape[-1] == M
@@ -151,12 +128,12 @@ def bgemm(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = 
             assert decay.dtype == torch.float32 and decay.shape[-1] == M == N
             d_hi, d_lo, d_r = decay.stride()
         mode = 0 if out.dtype == torch.bfloat16 else (2 if accumulate else 1)
-        ep = _Epilogue(out.data_ptr(), out.stride(2), out.stride(1), out.stride(0), n_lo // out.shape[1], c_offset,
-                       _lib.ptr(c_index), _lib.ptr(cin), cin_offset, _lib.ptr(cin_index), _lib.ptr(gamma),
-                       _lib.ptr(out16), out16_offset, _lib.ptr(out16_index), _lib.ptr(add16), add16_offset,
-                       _lib.ptr(add16_index), ld16, slo16, shi16,
-                       _lib.ptr(decay), d_hi, d_lo, d_r, _lib.ptr(rowscale), r_hi, r_lo, r_r, float(alpha), mode, int(mask))
-        rc = _lib.lib().fb_bgemm_bf16(ops, 1 + len(more), ctypes.byref(ep), n_hi, n_lo, sum_lo, M, N, _lib.stream_ptr())
+        ptr = _lib.ptr
+        c_hi, c_lo, c_r, _ = out.stride()
+        ep = _EPILOGUE.pack(out.data_ptr(), c_r, c_lo, c_hi, n_lo // out.shape[1], c_offset, ptr(c_index), ptr(cin), cin_offset, ptr(cin_index),
+                            ptr(gamma), ptr(out16), out16_offset, ptr(out16_index), ptr(add16), add16_offset, ptr(add16_index), ld16, slo16,
+                            shi16, ptr(decay), d_hi, d_lo, d_r, ptr(rowscale), r_hi, r_lo, r_r, alpha, mode, mask)
+        rc = _lib.lib().fb_bgemm_bf16(ops, 1 + len(more), ep, n_hi, n_lo, sum_lo, M, N, _lib.stream_ptr())
         _lib.check(rc, "fb_bgemm_bf16")
         _lib.count_launch()
         return out
@@ -230,7 +207,7 @@ class _BMM(torch.autograd.Function):
             out = torch.empty(n_hi, M, n_lo, N, dtype=out_dtype, device=a.device).permute(0, 2, 1, 3)
         else:
             out = torch.empty(n_hi, n_lo, M, N, dtype=out_dtype, device=a.device)
-        if addend is not None and _use_kernel(a, b) and out.dtype == torch.bfloat16 and addend.dtype == torch.bfloat16 \
+        if addend is not None and a.is_cuda and b.is_cuda and _lib.available() and out.dtype == torch.bfloat16 and addend.dtype == torch.bfloat16 \
                 and addend.stride() == out.stride():
             bgemm(a, b, a_mn=a_mn, b_mn=b_mn, out=out, alpha=alpha, add16=addend)
         else:

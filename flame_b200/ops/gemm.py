@@ -82,13 +82,14 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
     return ws
 
 
-def _use_kernel(*ts: torch.Tensor) -> bool:
-    return _lib.available() and all(t.is_cuda and t.dtype == torch.bfloat16 for t in ts)
+def _use_kernel(a: torch.Tensor, b: torch.Tensor) -> bool:
+    return a.is_cuda and b.is_cuda and a.dtype is torch.bfloat16 and b.dtype is torch.bfloat16 and _lib.available()
 
 
 def _rows_ok(t: torch.Tensor) -> torch.Tensor:
     # kernel needs: inner stride 1, leading dimension a multiple of 8 elements, base 16-byte aligned
-    if t.stride(-1) != 1 or (t.stride(0) % 8) != 0 or (t.data_ptr() % 16) != 0:
+    ld, inner = t.stride()
+    if inner != 1 or ld & 7 or t.data_ptr() & 15:
         t = t.contiguous()
         if t.stride(0) % 8 != 0:
             raise ValueError("bf16 GEMM operands need a row length that is a multiple of 8 elements")
