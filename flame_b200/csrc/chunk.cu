@@ -638,10 +638,11 @@ __global__ void __launch_bounds__(GD_THREADS, 2) gla_scores_kernel(const TQ* __r
 // gradients).  With `raw` the gate is g = logsigmoid(raw) norm, and its gradient is that of raw in bf16.
 // FULL: the chunk has all of its 64 rows; a test per row keeps the loads of the next rows behind it, so only the chunks at the
 // documents' ends make it.  What the second half of a sub-block needs is loaded in front of the pairs, whose 136 exponentials it takes
-// to come: loaded after them it doubled the waits (0.70 ms against 0.66).
-__device__ __forceinline__ unsigned short ld_now(const __nv_bfloat16* p) {  // a read-only load that stays where it is written
+// to come: loaded after them, and each under a test of its own, they doubled the waits (0.70 ms at 65,536 tokens, 4 heads of 128; this takes
+// 0.418 with the gate's argument, 0.105 instead of 0.166 for 64 channels, 32,767 tokens).  Two blocks of 128 threads per SM (three: 0.451).
+__device__ __forceinline__ unsigned short ld_now(const __nv_bfloat16* p, bool yes) {  // a read-only load that stays where it is written
   unsigned short v;
-  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; mov.b16 %0, 0; @p ld.global.nc.u16 %0, [%1];}" : "=h"(v) : "l"(p), "r"((int)yes));
   return v;
 }
 __device__ __forceinline__ float bf16_of(unsigned short v) { return __uint_as_float((uint32_t)v << 16); }
@@ -673,9 +674,9 @@ __device__ __forceinline__ void gla_bwd_rows(const __nv_bfloat16* __restrict__ q
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int off = (I * 16 + i) * rs;
-      a_khat[i] = ld_now(dkhat + off);
-      a_qbar[i] = ld_now(dqbar + off);
-      a_qt[i] = I > 0 ? ld_now(dqt + off) : (unsigned short)0;
+      a_khat[i] = ld_now(dkhat + off, true);
+      a_qbar[i] = ld_now(dqbar + off, true);
+      a_qt[i] = ld_now(dqt + off, I > 0);
     }
 #pragma unroll
     for (int i = 0; i < 16; ++i)
@@ -687,23 +688,29 @@ __device__ __forceinline__ void gla_bwd_rows(const __nv_bfloat16* __restrict__ q
       }
     const float rI = r[0] * (I == 0) + r[1] * (I == 1) + r[2] * (I == 2) + r[3] * (I == 3);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int row = I * 16 + i;
-      const float g_khat = bf16_of(a_khat[i]) * exp2f(b_last - bv[i]);
-      gq[i] = fmaf(bf16_of(a_qbar[i]), exp2f(bv[i]) * scale, gq[i]);
-      if (I > 0) gq[i] = fmaf(bf16_of(a_qt[i]), exp2f(bv[i] - rI), gq[i]);
-      gk[i] += g_khat;
-      acc_last = fmaf(g_khat, kv[i], acc_last);
-      if (I < 3) {
+    for (int half = 0; half < 16; half += 8) {
+      unsigned short a_k3[3][8];  // all that eight rows need, together: each load under its own test waited for the one before
 #pragma unroll
-        for (int J = 1; J <= 3; ++J)
-          if (J > I) gk[i] = fmaf(__bfloat162float(__ldg(dk3 + ((J - 1) * 48 + row) * rs)), exp2f(r[J] - bv[i]), gk[i]);
+      for (int J = 0; J < 3; ++J)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a_k3[J][i] = ld_now(dk3 + (J * 48 + min(I, 2) * 16 + half + i) * rs, J >= I);
+#pragma unroll
+      for (int ii = 0; ii < 8; ++ii) {
+        const int i = half + ii, row = I * 16 + i;
+        const float g_khat = bf16_of(a_khat[i]) * exp2f(b_last - bv[i]);
+        gq[i] = fmaf(bf16_of(a_qbar[i]), exp2f(bv[i]) * scale, gq[i]);
+        if (I > 0) gq[i] = fmaf(bf16_of(a_qt[i]), exp2f(bv[i] - rI), gq[i]);
+        gk[i] += g_khat;
+        acc_last = fmaf(g_khat, kv[i], acc_last);
+#pragma unroll
+        for (int J = 0; J < 3; ++J)
+          if (J >= I) gk[i] = fmaf(bf16_of(a_k3[J][ii]), exp2f(r[J + 1] - bv[i]), gk[i]);
+        if (FULL || row < n) {
+          dq[row * lddq] = __float2bfloat16(gq[i]);
+          dk_[row * lddk] = __float2bfloat16(gk[i]);
+        }
+        sgb[row][threadIdx.x] = qv[i] * gq[i] - kv[i] * gk[i];
       }
-      if (FULL || row < n) {
-        dq[row * lddq] = __float2bfloat16(gq[i]);
-        dk_[row * lddk] = __float2bfloat16(gk[i]);
-      }
-      sgb[row][threadIdx.x] = qv[i] * gq[i] - kv[i] * gk[i];
     }
   }
   float tail = acc_last + dalpha * exp2f(b_last);  // gradient of b_last
@@ -724,7 +731,7 @@ __device__ __forceinline__ void gla_bwd_rows(const __nv_bfloat16* __restrict__ q
 
 // TPB: 64 where a head has no more channels, else 128
 template <int TPB>
-__global__ void __launch_bounds__(TPB, 384 / TPB) gla_bwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
+__global__ void __launch_bounds__(TPB, 256 / TPB) gla_bwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                                                       const float* __restrict__ b, const __nv_bfloat16* __restrict__ dA,
                                                       const __nv_bfloat16* __restrict__ dkhat, const __nv_bfloat16* __restrict__ dqbar,
                                                       const __nv_bfloat16* __restrict__ dqt, const __nv_bfloat16* __restrict__ dk3,

@@ -40,17 +40,19 @@ __device__ __forceinline__ float logsigmoidf_(float x) { return fminf(x, 0.f) - 
 
 // g = logsigmoid(x) / n in fp32 from bf16 x, and with SLOTS s = 1 - exp(g) too (GLA's and GSA's forget gates,
 // fla/layers/gla.py:205-212, fla/layers/gsa.py:173-176).  Bound by memory: torch's chain (widen, logsigmoid, divide, and the same
-// back) moved 24 bytes per element forward and 30 backward where 6 and 8 are needed.
+// back) moved 24 bytes per element forward and 30 backward where 6 and 8 are needed.  x may be a column block (ldx); with a map g and s are
+// in the padded rows of the chunk layout: forward map[padded row] = row of x or -1 (zeros), backward map[row of x] = padded row.
 template <bool SLOTS>
-__global__ void logsigmoid_gate_fwd_kernel(const __nv_bfloat16* __restrict__ x, float* __restrict__ g, float* __restrict__ s, float n,
-                                           long long vecs) {
+__global__ void logsigmoid_gate_fwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int* __restrict__ map, float* __restrict__ g,
+                                           float* __restrict__ s, float n, long long total, long long vecs) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= vecs) return;
+  if (i >= total) return;
+  const long long row = i / vecs, from = map == nullptr ? row : map[row];
   float f[8], sv[8];
-  unpack8(reinterpret_cast<const uint4*>(x)[i], f);
+  unpack8(from >= 0 ? *reinterpret_cast<const uint4*>(x + from * ldx + (i - row * vecs) * 8) : make_uint4(0, 0, 0, 0), f);
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    f[c] = __fdiv_rn(logsigmoidf_(f[c]), n);
+    f[c] = from >= 0 ? __fdiv_rn(logsigmoidf_(f[c]), n) : 0.f;
     if (SLOTS) sv[c] = -expm1f(f[c]);
   }
 #pragma unroll
@@ -62,18 +64,20 @@ __global__ void logsigmoid_gate_fwd_kernel(const __nv_bfloat16* __restrict__ x, 
 
 // dx = (dg - exp(g) ds) sigmoid(-x) / n
 template <bool SLOTS>
-__global__ void logsigmoid_gate_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ dg, const float* __restrict__ ds,
-                                           __nv_bfloat16* __restrict__ dx, float n, long long vecs) {
+__global__ void logsigmoid_gate_bwd_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, const int* __restrict__ map, const float* __restrict__ dg,
+                                           const float* __restrict__ ds, __nv_bfloat16* __restrict__ dx, long long lddx, float n, long long total,
+                                           long long vecs) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= vecs) return;
+  if (i >= total) return;
+  const long long row = i / vecs, col = i - row * vecs, at = (map == nullptr ? row : map[row]) * vecs + col;
   float f[8], o[8];
-  unpack8(reinterpret_cast<const uint4*>(x)[i], f);
+  unpack8(*reinterpret_cast<const uint4*>(x + row * ldx + col * 8), f);
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
-    const float4 a = reinterpret_cast<const float4*>(dg)[2 * i + h];
+    const float4 a = reinterpret_cast<const float4*>(dg)[2 * at + h];
     o[4 * h] = a.x, o[4 * h + 1] = a.y, o[4 * h + 2] = a.z, o[4 * h + 3] = a.w;
     if (SLOTS) {
-      const float4 b = reinterpret_cast<const float4*>(ds)[2 * i + h];
+      const float4 b = reinterpret_cast<const float4*>(ds)[2 * at + h];
       const float bs[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
       for (int c = 0; c < 4; ++c) o[4 * h + c] -= __expf(__fdiv_rn(logsigmoidf_(f[4 * h + c]), n)) * bs[c];
@@ -81,7 +85,7 @@ __global__ void logsigmoid_gate_bwd_kernel(const __nv_bfloat16* __restrict__ x, 
   }
 #pragma unroll
   for (int c = 0; c < 8; ++c) o[c] = __fdiv_rn(o[c] * sigmoidf_(-f[c]), n);
-  reinterpret_cast<uint4*>(dx)[i] = pack8(o);
+  *reinterpret_cast<uint4*>(dx + row * lddx + col * 8) = pack8(o);
 }
 
 // one thread per (row, 8 channels)
@@ -501,23 +505,24 @@ int fb_mamba2_post_bwd(const void* y, const void* x, long long ldx, const void* 
 }
 
 // x, dx: bf16 [n]; g, s (optional), dg, ds (with s): fp32 [n]; n a multiple of 8, all 16-byte aligned
-int fb_logsigmoid_gate_fwd(const void* x, float* g, float* s, float normalizer, long long n, cudaStream_t stream) {
-  if (n == 0) return 0;
-  if ((n & 7) || (((uintptr_t)x | (uintptr_t)g | (uintptr_t)s) & 15)) return -2;
-  const long long vecs = n / 8;
-  const unsigned grid = (unsigned)((vecs + 255) / 256);
-  if (s != nullptr) logsigmoid_gate_fwd_kernel<true><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, g, s, normalizer, vecs);
-  else logsigmoid_gate_fwd_kernel<false><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, g, s, normalizer, vecs);
+// rows: of g (forward) or of x (backward), cols of each; map: see the kernels
+int fb_logsigmoid_gate_fwd(const void* x, long long ldx, const int* map, float* g, float* s, float normalizer, long long rows, long long cols,
+                           cudaStream_t stream) {
+  if (rows == 0 || cols == 0) return 0;
+  if ((cols & 7) || (ldx & 7) || !fb::aligned(16, x, g, s)) return -2;
+  const long long vecs = cols / 8, total = rows * vecs;
+  const auto kernel = s != nullptr ? logsigmoid_gate_fwd_kernel<true> : logsigmoid_gate_fwd_kernel<false>;
+  kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)x, ldx, map, g, s, normalizer, total, vecs);
   return fb::launch_ok("logsigmoid_gate_fwd_kernel");
 }
 
-int fb_logsigmoid_gate_bwd(const void* x, const float* dg, const float* ds, void* dx, float normalizer, long long n, cudaStream_t stream) {
-  if (n == 0) return 0;
-  if ((n & 7) || (((uintptr_t)x | (uintptr_t)dg | (uintptr_t)ds | (uintptr_t)dx) & 15)) return -2;
-  const long long vecs = n / 8;
-  const unsigned grid = (unsigned)((vecs + 255) / 256);
-  if (ds != nullptr) logsigmoid_gate_bwd_kernel<true><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, dg, ds, (__nv_bfloat16*)dx, normalizer, vecs);
-  else logsigmoid_gate_bwd_kernel<false><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)x, dg, ds, (__nv_bfloat16*)dx, normalizer, vecs);
+int fb_logsigmoid_gate_bwd(const void* x, long long ldx, const int* map, const float* dg, const float* ds, void* dx, long long lddx, float normalizer,
+                           long long rows, long long cols, cudaStream_t stream) {
+  if (rows == 0 || cols == 0) return 0;
+  if ((cols & 7) || (ldx & 7) || (lddx & 7) || !fb::aligned(16, x, dg, ds, dx)) return -2;
+  const long long vecs = cols / 8, total = rows * vecs;
+  const auto kernel = ds != nullptr ? logsigmoid_gate_bwd_kernel<true> : logsigmoid_gate_bwd_kernel<false>;
+  kernel<<<(unsigned)((total + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)x, ldx, map, dg, ds, (__nv_bfloat16*)dx, lddx, normalizer, total, vecs);
   return fb::launch_ok("logsigmoid_gate_bwd_kernel");
 }
 

@@ -409,8 +409,10 @@ class GatedSlotAttention(nn.Module):
         self.o_proj = Linear(self.value_dim, hidden_size)
 
     def forward(self, x: torch.Tensor, meta: VarlenMeta) -> torch.Tensor:
+        from ..ops.activations import silu_out_of_chunks
+        from ..ops.chunked import gsa_in_chunks
         from ..ops.gla import gsa
-        T, H, G = x.shape[0], self.num_heads, self.num_kv_groups
+        T, H, G, f = x.shape[0], self.num_heads, self.num_kv_groups, None
         layers, sizes = (self.q_proj, self.k_proj, self.v_proj), (self.key_dim, self.key_dim_per_group, self.value_dim_per_group)
         if self.use_short_conv:
             q, k, v = split_projections(x, layers)
@@ -418,13 +420,24 @@ class GatedSlotAttention(nn.Module):
             q, k, v = _feature_map(self.feature_map, q), _feature_map(self.feature_map, k), F.silu(v)
         elif self.feature_map in ("swish", "silu") and side_by_side(layers, x):
             # one activation over the three blocks as they lie: torch's kernels are several times slower on column blocks
-            q, k, v = split_columns(F.silu(fused_projection(x, layers)), sizes)
+            if side_by_side((*layers, self.f_proj), x):
+                n = sum(sizes)
+                qkv, f = split_columns(fused_projection(x, (*layers, self.f_proj)), (n, self.f_proj.weight.shape[0]))
+            else:
+                qkv = fused_projection(x, layers)
+            if G == 1:
+                f = reshaped(self.f_proj(x) if f is None else f, T, H, self.num_slots)
+                o = gsa_in_chunks(qkv, sizes, H, f, self.gate_logit_normalizer, meta,
+                                  self.scale if self.scale is not None else self.head_k_dim ** -0.5)
+                if o is not None:
+                    return self.o_proj(self.g_norm(silu_out_of_chunks(*o)))
+            q, k, v = split_columns(F.silu(qkv), sizes)
         else:
             q, k, v = _feature_map(self.feature_map, self.q_proj(x)), _feature_map(self.feature_map, self.k_proj(x)), F.silu(self.v_proj(x))
         q = reshaped(q, T, H, self.head_k_dim)
         k = reshaped(k, T, self.num_kv_heads, self.head_k_dim)
         v = reshaped(v, T, self.num_kv_heads, self.head_v_dim)
-        f = self.f_proj(x).reshape(T, self.num_kv_heads, self.num_slots)
+        f = (self.f_proj(x) if f is None else f).reshape(T, self.num_kv_heads, self.num_slots)
         f, s = logsigmoid_gate(f, self.gate_logit_normalizer, with_slots=True)
         if G > 1:
             k, v, f, s = (t.repeat_interleave(G, 1) for t in (k, v, f, s))

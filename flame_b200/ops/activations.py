@@ -10,7 +10,7 @@ from ctypes import c_int, c_longlong, c_void_p
 import torch
 import torch.nn.functional as F
 
-from . import _lib
+from . import _lib, slots
 
 vp, i32, i64 = c_void_p, c_int, c_longlong
 _lib.register("fb_swiglu_fwd", [vp, vp, vp, i64, i32, i64, i64, i64, vp])
@@ -70,3 +70,64 @@ def swiglu(gu: torch.Tensor) -> torch.Tensor:
     if _lib.available() and gu.is_cuda and gu.dtype == torch.bfloat16 and (gu.shape[-1] // 2) % 8 == 0:
         return _SwiGLUFn.apply(gu)
     return swiglu_reference(gu)
+
+
+_lib.register("fb_silu_rows", [vp, i64, vp, i64, i32, vp, vp, vp, i64, i32, vp])
+
+
+class _SiluRows(torch.autograd.Function):
+    """SiLU of neighbouring column blocks of ``x [rows, *]``, each to a matrix of its own: ``y_p[r] = silu(x[there[r], block p])``, zero rows where
+    ``there`` is negative; ``back`` is the inverse map (both None: the same rows)."""
+
+    @staticmethod
+    def forward(ctx, x, sizes, rows, there, back, slot):
+        ys = [torch.empty(rows, n, dtype=x.dtype, device=x.device) for n in sizes]
+        _SiluRows._launch(x, None, ys, there, rows, 0)
+        ctx.save_for_backward(x)
+        ctx.cfg = sizes, rows, back, slot
+        return tuple(ys)
+
+    @staticmethod
+    def _launch(x, dx, ys, rows_map, rows, backward):
+        p = (vp * len(ys))(*(y.data_ptr() for y in ys))
+        n = (i32 * len(ys))(*(y.shape[1] for y in ys))
+        ld = lambda t: t.stride(0) if t.shape[0] > 1 else -(-t.shape[1] // 8) * 8  # noqa: E731
+        rc = _lib.lib().fb_silu_rows(x.data_ptr(), ld(x), _lib.ptr(dx), 0 if dx is None else ld(dx), len(ys), p, n, _lib.ptr(rows_map), rows,
+                                     backward, _lib.stream_ptr())
+        _lib.check(rc, "fb_silu_rows")
+        _lib.count_launch()
+
+    @staticmethod
+    def backward(ctx, *dys):
+        x, = ctx.saved_tensors
+        sizes, rows, back, slot = ctx.cfg
+        x = x if _rows_ok(x) else x.contiguous()
+        dys = [torch.zeros(rows, n, dtype=x.dtype, device=x.device) if d is None else _lib.dense(d) for d, n in zip(dys, sizes)]
+        dx = None if slot is None else slot.take(x.shape[0], x.shape[1], x.dtype, x.device)
+        if dx is None or not _rows_ok(dx):
+            dx = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+        _SiluRows._launch(x, dx, dys, back, x.shape[0], 1)
+        return dx, None, None, None, None, None
+
+
+def _rows_ok(x: torch.Tensor) -> bool:
+    return x.stride(1) == 1 and (x.shape[0] == 1 or (x.stride(0) % 8 == 0 and x.stride(0) >= x.shape[1])) and x.data_ptr() % 16 == 0
+
+
+def silu_blocks_to_chunks(x: torch.Tensor, sizes, lay):
+    """SiLU of the column blocks of ``x [T, sum(sizes)]`` (up to three) in the padded rows of ``lay`` (``chunked.ChunkLayout``), ``[Tp, n]`` each, zeros
+    in the padding; None where the kernel does not apply."""
+    if not (_lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] == lay.T and len(sizes) <= 3
+            and all(n % 8 == 0 for n in sizes) and _rows_ok(x)):
+        return None
+    maps = (None, None) if lay.aligned else (lay.inv_i32, lay.rows_i32)
+    return _SiluRows.apply(x, tuple(sizes), lay.Tp, *maps, slots.of(x))
+
+
+def silu_out_of_chunks(o: torch.Tensor, lay) -> torch.Tensor:
+    """``silu(lay.unpack(o))`` as ``[T, n]`` for ``o [NC, chunk, ...]`` in the rows of ``lay``."""
+    o = o.reshape(lay.Tp, -1)
+    if not (_lib.available() and o.is_cuda and o.dtype == torch.bfloat16 and o.shape[1] % 8 == 0 and _rows_ok(o)):
+        return F.silu(lay.unpack(o.reshape(lay.NC, lay.chunk, -1)))
+    maps = (None, None) if lay.aligned else (lay.rows_i32, lay.inv_i32)
+    return _SiluRows.apply(o, (o.shape[1],), lay.T, *maps, None)[0]

@@ -956,12 +956,33 @@ def gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> Optional[torch.
 @_recomputable
 def _gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> torch.Tensor:
     lay = ChunkLayout.of(meta)
-    dt = torch.bfloat16
-    qp, kp, vp = (lay.pack(t).to(dt) for t in (q, k, v))
-    gp = lay.pack(g.float())
-    written, read = _TwoReaders.apply(lay.pack(s), dt)
+    qp, kp, vp = (lay.pack(t).to(torch.bfloat16) for t in (q, k, v))
+    return lay.unpack(_gsa_padded.__wrapped__(qp, kp, vp, lay.pack(s), lay.pack(g.float()), lay, scale)).to(v.dtype)
+
+
+def gsa_in_chunks(qkv, sizes, heads: int, f, normalizer: float, meta: VarlenMeta, scale: float):
+    """Both passes on q, k, v = the SiLU of column blocks of ``qkv [T, sum(sizes)]`` and the slots' gates from their bf16 argument ``f [T, heads, M]``;
+    activation and gates go into the chunk layout on the way.  The result, still in the rows of the layout, and the layout; None where
+    the kernels do not apply."""
+    from . import chunk_kernels
+    from .activations import silu_blocks_to_chunks
+    from .gates import logsigmoid_gate
+    M = f.shape[-1]
+    if not (_lib.available() and qkv.is_cuda and M <= chunk_kernels.VDECAY_SOFTMAX_MAX and M % 8 == 0 and getattr(meta, "sequence_slice", None) is None):
+        return None
+    lay = ChunkLayout.of(meta)
+    qkv = silu_blocks_to_chunks(qkv, sizes, lay)
+    if qkv is None:
+        return None
+    g, s = logsigmoid_gate(f, normalizer, True, lay)
+    return _gsa_padded(*(t.view(lay.NC, lay.chunk, heads, -1) for t in qkv), s, g, lay, scale), lay
+
+
+@_recomputable
+def _gsa_padded(qp, kp, vp, sp, gp, lay: "ChunkLayout", scale: float) -> torch.Tensor:
+    written, read = _TwoReaders.apply(sp, torch.bfloat16)
     qv = _VDecay.apply(qp, kp, written, gp, scale, True, lay)
-    return lay.unpack(_Gla.apply(qv, read, vp, gp, 1.0, lay, False, None)).to(v.dtype)
+    return _Gla.apply(qv, read, vp, gp, 1.0, lay, False, None)
 
 
 @_recomputable

@@ -25,8 +25,8 @@ _lib.register("fb_hgrn2_gate_bwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_vo
                                     c_void_p, c_longlong, c_int, c_void_p])
 
 
-_lib.register("fb_logsigmoid_gate_fwd", [c_void_p, c_void_p, c_void_p, c_float, c_longlong, c_void_p])
-_lib.register("fb_logsigmoid_gate_bwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_float, c_longlong, c_void_p])
+_lib.register("fb_logsigmoid_gate_fwd", [c_void_p, c_longlong] + [c_void_p] * 3 + [c_float] + [c_longlong] * 2 + [c_void_p])
+_lib.register("fb_logsigmoid_gate_bwd", [c_void_p, c_longlong] + [c_void_p] * 4 + [c_longlong, c_float] + [c_longlong] * 2 + [c_void_p])
 
 
 def hgrn2_gates_reference(q_raw: torch.Tensor, f_raw: torch.Tensor,
@@ -45,40 +45,74 @@ def logsigmoid_gate_reference(x: torch.Tensor, normalizer: float, with_slots: bo
     return (g, 1 - g.exp()) if with_slots else g
 
 
+def _gate_rows(x: torch.Tensor):
+    """``(rows, columns, distance of rows)`` of a gate's argument as the kernels read it, None if they cannot."""
+    if x.data_ptr() % 16 or x.dim() < 2 or x.numel() == 0:
+        return None
+    T, cols = x.shape[0], x.numel() // x.shape[0]
+    if x.is_contiguous() and cols % 8 == 0:
+        return T, cols, cols
+    try:
+        ld = x.view(T, cols).stride(0) if T > 1 else cols
+    except RuntimeError:
+        return None
+    return (T, cols, ld) if cols % 8 == 0 and ld % 8 == 0 and ld >= cols else None
+
+
 class _LogSigmoidGate(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, normalizer, with_slots):
-        g = torch.empty(x.shape, dtype=torch.float32, device=x.device)
+    def forward(ctx, x, normalizer, with_slots, lay):
+        """``lay`` (``chunked.ChunkLayout``): the results are in its padded rows ``[NC, chunk, ...]``, zeros in the padding."""
+        ctx.slot = slots.of(x)
+        T, cols, ld = _gate_rows(x) or (1, x.numel(), x.numel())
+        shape = x.shape if lay is None else (lay.NC, lay.chunk, *x.shape[1:])
+        src = None if lay is None or lay.aligned else lay.inv_i32
+        g = torch.empty(shape, dtype=torch.float32, device=x.device)
         s = torch.empty_like(g) if with_slots else None
-        rc = _lib.lib().fb_logsigmoid_gate_fwd(x.data_ptr(), g.data_ptr(), _lib.ptr(s), normalizer, x.numel(), _lib.stream_ptr())
+        rc = _lib.lib().fb_logsigmoid_gate_fwd(x.data_ptr(), ld, _lib.ptr(src), g.data_ptr(), _lib.ptr(s), normalizer, T if lay is None else lay.Tp, cols,
+                                               _lib.stream_ptr())
         _lib.check(rc, "fb_logsigmoid_gate_fwd")
         _lib.count_launch()
         ctx.save_for_backward(x)
-        ctx.normalizer, ctx.with_slots = normalizer, with_slots
+        ctx.cfg = normalizer, with_slots, lay, shape
         return (g, s) if with_slots else g
 
     @staticmethod
     def backward(ctx, dg, ds=None):
         x, = ctx.saved_tensors
+        normalizer, with_slots, lay, shape = ctx.cfg
 
         def full(d):
-            return torch.zeros(x.shape, dtype=torch.float32, device=x.device) if d is None else _lib.dense(d.float())
+            return torch.zeros(shape, dtype=torch.float32, device=x.device) if d is None else _lib.dense(d.float())
 
-        dg, ds = full(dg), full(ds) if ctx.with_slots else None
-        dx = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-        rc = _lib.lib().fb_logsigmoid_gate_bwd(x.data_ptr(), dg.data_ptr(), _lib.ptr(ds), dx.data_ptr(), ctx.normalizer, x.numel(),
-                                               _lib.stream_ptr())
+        dg, ds = full(dg), full(ds) if with_slots else None
+        rows = _gate_rows(x)
+        if rows is None:
+            x = x.contiguous()
+            rows = _gate_rows(x) or (1, x.numel(), x.numel())
+        T, cols, ld = rows
+        dx = None if ctx.slot is None or T != x.shape[0] else ctx.slot.take(T, cols, x.dtype, x.device)
+        if dx is None or (T > 1 and dx.stride(0) % 8) or dx.data_ptr() % 16:
+            dx = torch.empty(T, cols, dtype=x.dtype, device=x.device)
+        src = None if lay is None or lay.aligned else lay.rows_i32
+        rc = _lib.lib().fb_logsigmoid_gate_bwd(x.data_ptr(), ld, _lib.ptr(src), dg.data_ptr(), _lib.ptr(ds), dx.data_ptr(),
+                                               dx.stride(0) if T > 1 else cols, normalizer, T, cols, _lib.stream_ptr())
         _lib.check(rc, "fb_logsigmoid_gate_bwd")
         _lib.count_launch()
-        return dx, None, None
+        return dx.view(x.shape), None, None, None
 
 
-def logsigmoid_gate(x: torch.Tensor, normalizer: float, with_slots: bool = False):
-    """``logsigmoid(x) / normalizer`` in fp32, and ``1 - exp`` of it with ``with_slots``.  One pass for contiguous bf16 on the
-    GPU; anything else (other types, odd sizes, column blocks) takes torch's chain."""
-    if _lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and x.is_contiguous() and x.numel() % 8 == 0 and x.data_ptr() % 16 == 0:
-        return _LogSigmoidGate.apply(x, float(normalizer), with_slots)
-    return logsigmoid_gate_reference(x, normalizer, with_slots)
+def logsigmoid_gate(x: torch.Tensor, normalizer: float, with_slots: bool = False, lay=None):
+    """``logsigmoid(x) / normalizer`` in fp32, and ``1 - exp`` of it with ``with_slots``.  One pass for bf16 on the GPU, contiguous or a
+    column block whose rows are whole vectors; anything else (other types, odd sizes) takes torch's chain.  ``lay``: results in the
+    padded rows of a ``chunked.ChunkLayout``."""
+    if _lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and (lay is None or x.shape[0] == lay.T) and \
+            (_gate_rows(x) is not None or (lay is None and x.is_contiguous() and x.numel() % 8 == 0 and x.data_ptr() % 16 == 0)):
+        return _LogSigmoidGate.apply(x, float(normalizer), with_slots, lay)
+    out = logsigmoid_gate_reference(x, normalizer, with_slots)
+    if lay is None:
+        return out
+    return tuple(lay.pack(t) for t in out) if with_slots else lay.pack(out)
 
 
 class _Hgrn2Gates(torch.autograd.Function):

@@ -599,3 +599,53 @@ def test_column_sums(rows, cols, wide):
     from flame_b200.ops.linear import _column_sums
     x = _bf(rows, wide)[:, :cols]
     assert rel_err(_column_sums(x), x.double().sum(0)) < 1e-4
+
+
+@pytest.mark.parametrize("lens", [[1], [64, 128], [15, 17, 63, 65, 1, 200]])
+@pytest.mark.parametrize("sizes", [(8,), (24, 8, 64), (512, 512, 512)])
+def test_silu_into_and_out_of_chunk_rows(lens, sizes):
+    """SiLU of column blocks into the chunk layout, and out of it, against fp64: bf16 results rounded once (2^-8); zeros in the padding
+    both ways, whatever gradient comes from there."""
+    from flame_b200.ops.activations import silu_blocks_to_chunks, silu_out_of_chunks
+    from flame_b200.ops.chunked import ChunkLayout
+    torch.manual_seed(len(lens))
+    T, lay, n = sum(lens), ChunkLayout.of(_meta(lens), 64), sum(sizes)
+    wide = _bf(T, n + 16, s=3.0).requires_grad_(True)
+    ys = silu_blocks_to_chunks(wide[:, 8:8 + n], sizes, lay)
+    dys = [_bf(lay.Tp, m) for m in sizes]
+    pad = lay.inv_i32 < 0
+    torch.autograd.backward(ys, [d.masked_fill(pad[:, None], 5e3) for d in dys])
+    xr = wide.detach()[:, 8:8 + n].double().requires_grad_(True)
+    want = F.silu(xr)
+    want.backward(torch.cat(dys, 1)[lay.rows].double())
+    assert rel_err(torch.cat(ys, 1)[lay.rows], want) < 4e-3 and rel_err(wide.grad[:, 8:8 + n], xr.grad) < 4e-3
+    assert all(float(y[pad].abs().sum()) == 0 for y in ys)
+    o = _bf(lay.Tp, sizes[0], s=3.0).requires_grad_(True)
+    y, dy = silu_out_of_chunks(o.view(lay.NC, 64, -1), lay), _bf(T, sizes[0])
+    y.backward(dy)
+    orr = o.detach()[lay.rows].double().requires_grad_(True)
+    F.silu(orr).backward(dy.double())
+    assert rel_err(y, F.silu(orr)) < 4e-3 and rel_err(o.grad[lay.rows], orr.grad) < 4e-3 and float(o.grad[pad].abs().sum()) == 0
+
+
+@pytest.mark.parametrize("slots", [False, True])
+@pytest.mark.parametrize("lens", [[1], [64, 128], [15, 17, 63, 65, 1, 200]])
+def test_logsigmoid_gate_of_a_block_in_chunk_rows(lens, slots):
+    """The gate of a column block, in the chunk layout: bit for bit what the contiguous form gives, packed; the gradient too."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.gates import logsigmoid_gate
+    T, lay = sum(lens), ChunkLayout.of(_meta(lens), 64)
+    wide, out = _bf(T, 40, s=3.0), []
+    ds = [torch.randn(lay.NC, 64, 2, 8, device=DEV) for _ in range(1 + slots)]
+    for new in (True, False):
+        w = wide.clone().requires_grad_(True)
+        x = w[:, 16:32].view(T, 2, 8)
+        if new:
+            g = logsigmoid_gate(x, 8, slots, lay)
+        else:
+            g = logsigmoid_gate(x.contiguous(), 8, slots)
+            g = tuple(lay.pack(t) for t in g) if slots else lay.pack(g)
+        g = g if slots else (g,)
+        torch.autograd.backward(g, ds)
+        out.append((*g, w.grad))
+    assert all(torch.equal(a, b) for a, b in zip(*out))
