@@ -645,6 +645,11 @@ __device__ __forceinline__ unsigned short ld_now(const __nv_bfloat16* p, bool ye
   asm volatile("{.reg .pred p; setp.ne.s32 p, %2, 0; mov.b16 %0, 0; @p ld.global.nc.u16 %0, [%1];}" : "=h"(v) : "l"(p), "r"((int)yes));
   return v;
 }
+__device__ __forceinline__ float ld_now(const float* p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
 __device__ __forceinline__ float bf16_of(unsigned short v) { return __uint_as_float((uint32_t)v << 16); }
 template <bool FULL, int TPB>
 __device__ __forceinline__ void gla_bwd_rows(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k, const float* __restrict__ b,
@@ -1535,20 +1540,23 @@ __global__ void __launch_bounds__(256) vdecay_bwd1_kernel(const float* __restric
 
 // dv = dvhat e^{b_last - b} + sum_I dv3[I] e^{r_I - b} + diagonal sub-blocks;  db = do o / scale - v dv (+ what enters through
 // b_last: vhat and alpha), dg = reverse cumulative sum.  `o` carries the factor scale and so does `do`, hence the division.
-__global__ void __launch_bounds__(128) vdecay_bwd2_kernel(const float* __restrict__ P, const __nv_bfloat16* __restrict__ v, const float* __restrict__ b,
+// TPB: 64 where a head has no more slots, else 128; loads as in gla_bwd_rows (half of the threads idle and each load of dv3 behind the
+// one before: 0.250 ms at 32,767 tokens, 4 heads of 64 slots; this takes 0.105)
+template <int TPB>
+__global__ void __launch_bounds__(TPB, 256 / TPB) vdecay_bwd2_kernel(const float* __restrict__ P, const __nv_bfloat16* __restrict__ v, const float* __restrict__ b,
                                                           const float* __restrict__ dout, const float* __restrict__ o,
                                                           const __nv_bfloat16* __restrict__ dvhat, const __nv_bfloat16* __restrict__ dv3,
                                                           const float* __restrict__ dalpha, int H, int M, float inv_scale, __nv_bfloat16* __restrict__ dv,
                                                           float* __restrict__ dg) {
   __shared__ float sP[4][16][16];
-  __shared__ float sgb[64][128];
+  __shared__ float sgb[64][TPB];
   const int ch = blockIdx.x, c = ch / H, h = ch - c * H;
-  for (int idx = threadIdx.x; idx < 1024; idx += 128) {
+  for (int idx = threadIdx.x; idx < 1024; idx += TPB) {
     const int I = idx >> 8, r = (idx >> 4) & 15, cc = idx & 15;
     sP[I][r][cc] = P[((long long)ch * 64 + I * 16 + r) * 64 + I * 16 + cc];
   }
   __syncthreads();
-  const int m = blockIdx.y * 128 + threadIdx.x;
+  const int m = blockIdx.y * TPB + threadIdx.x;
   if (m >= M) return;
   const long long rs = (long long)H * M, base = (long long)c * 64 * rs + (long long)h * M + m, base3 = (long long)c * 144 * rs + (long long)h * M + m;
   float r[4];
@@ -1566,24 +1574,39 @@ __global__ void __launch_bounds__(128) vdecay_bwd2_kernel(const float* __restric
       dd[i] = dout[off];
       gv[i] = 0.f;
     }
+    unsigned short a_v[16], a_vhat[16];
+    float a_o[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const long long off = base + (I * 16 + i) * rs;
+      a_v[i] = ld_now(v + off, true);
+      a_vhat[i] = ld_now(dvhat + off, true);
+      a_o[i] = ld_now(o + off);
+    }
 #pragma unroll
     for (int i = 0; i < 16; ++i)
 #pragma unroll
       for (int j = 0; j <= i; ++j) gv[j] = fmaf(sP[I][i][j] * dd[i], i == j ? 1.f : exp2f(bv[i] - bv[j]), gv[j]);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const long long off = base + (I * 16 + i) * rs;
-      const float x = __bfloat162float(v[off]);
-      const float gl = __bfloat162float(dvhat[off]) * exp2f(b_last - bv[i]);
-      gv[i] += gl;
-      acc_last = fmaf(gl, x, acc_last);
-      if (I < 3) {
+    for (int half = 0; half < 16; half += 8) {
+      unsigned short a_v3[3][8];
 #pragma unroll
-        for (int J = 1; J <= 3; ++J)
-          if (J > I) gv[i] = fmaf(__bfloat162float(dv3[base3 + ((J - 1) * 48 + I * 16 + i) * rs]), exp2f(r[J] - bv[i]), gv[i]);
+      for (int J = 0; J < 3; ++J)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a_v3[J][i] = ld_now(dv3 + base3 + (J * 48 + min(I, 2) * 16 + half + i) * rs, J >= I);
+#pragma unroll
+      for (int ii = 0; ii < 8; ++ii) {
+        const int i = half + ii;
+        const float x = bf16_of(a_v[i]);
+        const float gl = bf16_of(a_vhat[i]) * exp2f(b_last - bv[i]);
+        gv[i] += gl;
+        acc_last = fmaf(gl, x, acc_last);
+#pragma unroll
+        for (int J = 0; J < 3; ++J)
+          if (J >= I) gv[i] = fmaf(bf16_of(a_v3[J][ii]), exp2f(r[J + 1] - bv[i]), gv[i]);
+        dv[base + (I * 16 + i) * rs] = __float2bfloat16(gv[i]);
+        sgb[I * 16 + i][threadIdx.x] = dd[i] * a_o[i] * inv_scale - x * gv[i];
       }
-      dv[off] = __float2bfloat16(gv[i]);
-      sgb[I * 16 + i][threadIdx.x] = dd[i] * o[off] * inv_scale - x * gv[i];
     }
   }
   float tail = acc_last + dalpha[(long long)ch * M + m] * exp2f(b_last);
@@ -1627,8 +1650,10 @@ int fb_vdecay_bwd1(const float* o, const void* dqv, const float* d32, const floa
 int fb_vdecay_bwd2(const float* P, const void* v, const float* b, const float* dout, const float* o, const void* dvhat, const void* dv3,
                    const float* dalpha, int NC, int H, int M, float inv_scale, void* dv, float* dg, cudaStream_t stream) {
   if (NC <= 0) return 0;
-  vdecay_bwd2_kernel<<<dim3(NC * H, (M + 127) / 128), 128, 0, stream>>>(P, (const __nv_bfloat16*)v, b, dout, o, (const __nv_bfloat16*)dvhat,
-                                                                        (const __nv_bfloat16*)dv3, dalpha, H, M, inv_scale, (__nv_bfloat16*)dv, dg);
+  const int tpb = M <= 64 ? 64 : 128;
+  const auto kernel = M <= 64 ? vdecay_bwd2_kernel<64> : vdecay_bwd2_kernel<128>;
+  kernel<<<dim3(NC * H, (M + tpb - 1) / tpb), tpb, 0, stream>>>(P, (const __nv_bfloat16*)v, b, dout, o, (const __nv_bfloat16*)dvhat,
+                                                                (const __nv_bfloat16*)dv3, dalpha, H, M, inv_scale, (__nv_bfloat16*)dv, dg);
   return fb::launch_ok("vdecay_bwd2_kernel");
 }
 
