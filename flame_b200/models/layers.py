@@ -579,6 +579,10 @@ class Mamba2(nn.Module):
         zxbcdt = self.in_proj(x)
         # column blocks as views whose gradients are written side by side in one pass
         z, xBC, dt = split_columns(zxbcdt, (Di, self.conv_dim, zxbcdt.shape[1] - Di - self.conv_dim))
+        if G < H and not (self.rmsnorm and self.norm_before_gate):
+            y = self._in_chunks(z, xBC, dt, meta)
+            if y is not None:
+                return self.out_proj((_group_rms(y, self.norm.weight, self.norm_eps, G) if self.rmsnorm else y).to(x.dtype))
         xBC = self.conv1d(xBC, meta)
         xs, B, C = split_columns(xBC, (Di, G * N, G * N))
         if not (self.rmsnorm and self.norm_before_gate):
@@ -596,6 +600,25 @@ class Mamba2(nn.Module):
         y = mamba2_ssd(xs.reshape(T, H, P), dt, A, B.reshape(T, G, N), C.reshape(T, G, N), self.D, meta)
         y = _group_rms(y.reshape(T, Di), self.norm.weight, self.norm_eps, G) * F.silu(z)
         return self.out_proj(y.to(x.dtype))
+
+
+    def _in_chunks(self, z, xBC, dt, meta: VarlenMeta) -> Optional[torch.Tensor]:
+        """Convolution, elementwise work and SSD core without leaving the chunk layout; None where the kernels do not apply."""
+        from ..ops import gates
+        from ..ops.chunked import ChunkLayout, grouped_scalar_gla_chunks, scalar_chunk
+        from ..ops.conv import short_convs_in_chunks
+        Di, H, P, G, N, conv = self.intermediate_size, self.num_heads, self.head_dim, self.n_groups, self.ssm_state_size, self.conv1d
+        if not (plain((conv,), ShortConvolution) and gates.mamba2_kernels(xBC, dt, z, P) and Di % 8 == 0 and G * N % 8 == 0):
+            return None
+        chunk = scalar_chunk(N, P)
+        out = short_convs_in_chunks((xBC,), (conv.weight,), (conv.bias,), meta, conv.activation, chunk)
+        if out is None:
+            return None
+        lay, rows = ChunkLayout.of(meta, chunk), out[0].shape[0]
+        xs, B, C = split_columns(out[0], (Di, G * N, G * N))
+        xv, _, g = gates.mamba2_pre(xs, dt, self.dt_bias, self.A_log, H, P, lay)
+        y = grouped_scalar_gla_chunks(C.reshape(rows, G, N), B.reshape(rows, G, N), xv, g, lay)
+        return gates.mamba2_post(y.reshape(rows, H, P), xs, z, self.D, H, P, lay)
 
 
 def _group_rms(y: torch.Tensor, w: torch.Tensor, eps: float, groups: int) -> torch.Tensor:

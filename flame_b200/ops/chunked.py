@@ -729,6 +729,13 @@ def scalar_gla_tc(q, k, v, g, meta: VarlenMeta, scale: float = 1.0, chunk: Optio
     return lay.unpack(o.permute(0, 2, 1, 3)).to(v.dtype)
 
 
+@_recomputable
+def grouped_scalar_gla_chunks(q, k, v, g, lay: "ChunkLayout") -> torch.Tensor:
+    """``scalar_gla_tc`` for heads in groups on operands in the rows of ``lay``: q, k ``[Tp, G, dk]``, v ``[Tp, H, dv]`` bf16 (zero in the padding), g
+    ``[Tp, H]`` fp32; the result stays there, ``[NC, chunk, H, dv]``."""
+    return _GroupedScalarGla.apply(*(t.reshape(lay.NC, lay.chunk, *t.shape[1:]) for t in (q, k, v, g)), 1.0, lay)
+
+
 class _Gla(torch.autograd.Function):
     """The whole chunk pipeline of gated linear attention on 64-token chunks, on the kernels: v ``[NC, 64, H, dv]`` bf16; q, k ``[NC, 64, H, dk]``
     bf16 and g fp32 there too, or with ``tokens`` packed ``[T, H, dk]`` (``norm``: g is then the bf16 argument of ``logsigmoid(g) / norm``), which

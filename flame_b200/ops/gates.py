@@ -164,13 +164,13 @@ def hgrn2_gates(q_raw: torch.Tensor, f_raw: torch.Tensor,
 # Mamba2: the elementwise work around the SSD core (fla/layers/mamba2.py:241-331)
 # ----------------------------------------------------------------------------------------------------------------------
 _lib.register("fb_mamba2_pre_fwd", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                    c_longlong, c_int, c_int, c_void_p])
+                                    c_void_p, c_longlong, c_int, c_int, c_void_p])
 _lib.register("fb_mamba2_pre_bwd", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                    c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p])
-_lib.register("fb_mamba2_post_fwd", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int,
+                                    c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p])
+_lib.register("fb_mamba2_post_fwd", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_int,
                                      c_int, c_void_p])
 _lib.register("fb_mamba2_post_bwd", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
-                                     c_void_p, c_longlong, c_void_p, c_longlong, c_int, c_int, c_void_p])
+                                     c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p])
 
 
 def _views_ok(*ts: torch.Tensor) -> bool:
@@ -180,14 +180,16 @@ def _views_ok(*ts: torch.Tensor) -> bool:
 
 class _Mamba2Pre(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, dt_raw, dt_bias, A_log, H, P):
+    def forward(ctx, x, dt_raw, dt_bias, A_log, H, P, lay):
+        """``lay`` (``chunked.ChunkLayout``): x and the results are in its padded rows, ``dt_raw`` is per token."""
         T = x.shape[0]
+        ctx.src = None if lay is None or lay.aligned else lay.inv_i32
         bias32, alog32 = dt_bias.detach().float().contiguous(), A_log.detach().float().contiguous()
         xv = torch.empty(T, H, P, dtype=x.dtype, device=x.device)
         dt = torch.empty(T, H, dtype=torch.float32, device=x.device)
         g = torch.empty(T, H, dtype=torch.float32, device=x.device)
         rc = _lib.lib().fb_mamba2_pre_fwd(x.data_ptr(), x.stride(0), dt_raw.data_ptr(), dt_raw.stride(0), bias32.data_ptr(),
-                                          alog32.data_ptr(), xv.data_ptr(), dt.data_ptr(), g.data_ptr(), T, H, P,
+                                          alog32.data_ptr(), xv.data_ptr(), dt.data_ptr(), g.data_ptr(), _lib.ptr(ctx.src), T, H, P,
                                           _lib.stream_ptr())
         _lib.check(rc, "fb_mamba2_pre_fwd")
         _lib.count_launch()
@@ -205,26 +207,28 @@ class _Mamba2Pre(torch.autograd.Function):
         dg = torch.zeros(T, H, dtype=torch.float32, device=x.device) if dg is None else _lib.dense(dg.float())
         ddt = None if ddt is None else ddt.float().contiguous()
         dx = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
-        d_raw = torch.empty(T, H, dtype=torch.float32, device=x.device)
+        d_raw = torch.empty(dt_raw.shape[0], H, dtype=torch.float32, device=x.device)
         rc = _lib.lib().fb_mamba2_pre_bwd(x.data_ptr(), x.stride(0), dt_raw.data_ptr(), dt_raw.stride(0), bias32.data_ptr(),
                                           alog32.data_ptr(), dxv.data_ptr(), dg.data_ptr(), _lib.ptr(ddt), dx.data_ptr(),
-                                          d_raw.data_ptr(), T, H, P, _lib.stream_ptr())
+                                          d_raw.data_ptr(), _lib.ptr(ctx.src), T, H, P, _lib.stream_ptr())
         _lib.check(rc, "fb_mamba2_pre_bwd")
         _lib.count_launch()
         d_bias = d_raw.sum(0)
         d_alog = (dg * dt).sum(0) * (-alog32.exp())     # g = A dt with A = -exp(A_log): dA_log = dA * A
-        return (dx, d_raw.to(ctx.dtypes[2]), d_bias.to(ctx.dtypes[0]), d_alog.to(ctx.dtypes[1]), None, None)
+        return (dx, d_raw.to(ctx.dtypes[2]), d_bias.to(ctx.dtypes[0]), d_alog.to(ctx.dtypes[1]), None, None, None)
 
 
 class _Mamba2Post(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, y, x, z, D, H, P):
+    def forward(ctx, y, x, z, D, H, P, lay):
+        """``lay``: y and x are in its padded rows, z and the result per token."""
         T = x.shape[0]
+        ctx.src = None if lay is None or lay.aligned else lay.inv_i32
         y = _lib.dense(y)
         d32 = D.detach().float().contiguous()
-        out = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
+        out = torch.empty(z.shape[0], H * P, dtype=x.dtype, device=x.device)
         rc = _lib.lib().fb_mamba2_post_fwd(y.data_ptr(), x.data_ptr(), x.stride(0), z.data_ptr(), z.stride(0), d32.data_ptr(),
-                                           out.data_ptr(), T, H, P, _lib.stream_ptr())
+                                           out.data_ptr(), _lib.ptr(ctx.src), T, H, P, _lib.stream_ptr())
         _lib.check(rc, "fb_mamba2_post_fwd")
         _lib.count_launch()
         ctx.save_for_backward(y, x, z, d32)
@@ -239,16 +243,17 @@ class _Mamba2Post(torch.autograd.Function):
         dout = _lib.dense(dout)
         dy = torch.empty(T, H, P, dtype=x.dtype, device=x.device)
         dx = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
-        dz = ctx.z_slot.take(T, H * P, x.dtype, x.device) if ctx.z_slot is not None else torch.empty(T, H * P, dtype=x.dtype, device=x.device)
+        n = z.shape[0]
+        dz = ctx.z_slot.take(n, H * P, x.dtype, x.device) if ctx.z_slot is not None else torch.empty(n, H * P, dtype=x.dtype, device=x.device)
         if not _views_ok(dz):
-            dz = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
+            dz = torch.empty(n, H * P, dtype=x.dtype, device=x.device)
         part = torch.empty(T, H, dtype=torch.float32, device=x.device)
         rc = _lib.lib().fb_mamba2_post_bwd(y.data_ptr(), x.data_ptr(), x.stride(0), z.data_ptr(), z.stride(0), d32.data_ptr(),
-                                           dout.data_ptr(), dy.data_ptr(), dx.data_ptr(), dz.data_ptr(), dz.stride(0), part.data_ptr(), T, H, P,
+                                           dout.data_ptr(), dy.data_ptr(), dx.data_ptr(), dz.data_ptr(), dz.stride(0), part.data_ptr(), _lib.ptr(ctx.src), T, H, P,
                                            _lib.stream_ptr())
         _lib.check(rc, "fb_mamba2_post_bwd")
         _lib.count_launch()
-        return dy, dx, dz, part.sum(0).to(ctx.d_dtype), None, None
+        return dy, dx, dz, part.sum(0).to(ctx.d_dtype), None, None, None
 
 
 def mamba2_pre_reference(x, dt_raw, dt_bias, A_log, H: int, P: int):
@@ -265,19 +270,23 @@ def mamba2_post_reference(y, x, z, D, H: int, P: int):
     return (u.reshape(T, H * P) * F.silu(z.float())).to(x.dtype)
 
 
-def mamba2_pre(x, dt_raw, dt_bias, A_log, H: int, P: int):
+def mamba2_kernels(x, dt_raw, z, P: int) -> bool:
+    """Whether both of the functions below run on their kernels, which also take padded rows (``lay``)."""
+    return _lib.available() and P in (64, 128, 256) and _views_ok(x, z) and dt_raw.is_cuda and dt_raw.dtype == torch.bfloat16 and dt_raw.stride(1) == 1
+
+
+def mamba2_pre(x, dt_raw, dt_bias, A_log, H: int, P: int, lay=None):
     """``x [T, H * P]`` and ``dt_raw [T, H]`` (strided views are fine) -> ``xv = x dt`` ``[T, H, P]``, ``dt = softplus(dt_raw +
     dt_bias)`` and the log decay ``g = -exp(A_log) dt`` (both fp32 ``[T, H]``), in one kernel."""
-    if _lib.available() and P in (64, 128, 256) and _views_ok(x) and dt_raw.is_cuda and dt_raw.dtype == torch.bfloat16 \
-            and dt_raw.stride(1) == 1:
-        return _Mamba2Pre.apply(x, dt_raw, dt_bias, A_log, H, P)
+    if mamba2_kernels(x, dt_raw, x, P):
+        return _Mamba2Pre.apply(x, dt_raw, dt_bias, A_log, H, P, lay)
     return mamba2_pre_reference(x, dt_raw, dt_bias, A_log, H, P)
 
 
-def mamba2_post(y, x, z, D, H: int, P: int):
+def mamba2_post(y, x, z, D, H: int, P: int, lay=None):
     """``(y + D x) silu(z)`` as ``[T, H * P]`` in one kernel; ``x`` and ``z`` may be strided views."""
     if _lib.available() and P in (64, 128, 256) and _views_ok(x, z) and y.is_cuda and y.dtype == torch.bfloat16:
-        return _Mamba2Post.apply(y, x, z, D, H, P)
+        return _Mamba2Post.apply(y, x, z, D, H, P, lay)
     return mamba2_post_reference(y, x, z, D, H, P)
 
 

@@ -649,3 +649,34 @@ def test_logsigmoid_gate_of_a_block_in_chunk_rows(lens, slots):
         torch.autograd.backward(g, ds)
         out.append((*g, w.grad))
     assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("P", [64, 128])
+@pytest.mark.parametrize("lens", [[1], [64, 128], [15, 17, 63, 65, 1, 200]])
+def test_mamba2_elementwise_kernels_in_chunk_rows(lens, P):
+    """What stands around the SSD core, its operands in padded rows (the padding's values are zero, as the convolution leaves them): bit for
+    bit what the same kernels give per token, sums over the tokens in fp32 to 1e-5; the gradient of y is zero in the padding."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.gates import mamba2_post, mamba2_pre
+    torch.manual_seed(P)
+    T, H, lay = sum(lens), 3, ChunkLayout.of(_meta(lens), 64)
+    x0, y0, z0, dt0 = _bf(T, H * P), _bf(T, H, P), _bf(T, H * P, s=2.0), _bf(T, H, s=2.0)
+    par = [torch.randn(H, device=DEV) for _ in range(3)]
+    dxv, dg, dout = _bf(T, H, P), torch.randn(T, H, device=DEV), _bf(T, H * P)
+    pack = lambda t: torch.zeros(lay.Tp, *t.shape[1:], dtype=t.dtype, device=DEV).index_copy(0, lay.rows, t)  # noqa: E731
+    res = []
+    for padded in (True, False):
+        f = pack if padded else (lambda t: t)
+        pick = (lambda t: t[lay.rows]) if padded else (lambda t: t)
+        x, y = f(x0).requires_grad_(True), f(y0).requires_grad_(True)
+        z, dt, A, bias, D = (t.clone().requires_grad_(True) for t in (z0, dt0, *par))
+        xv, dts, g = mamba2_pre(x, dt, bias, A, H, P, lay if padded else None)
+        out = mamba2_post(y, x, z, D, H, P, lay if padded else None)
+        gx = torch.autograd.grad([xv, g], [x, dt, bias, A], [f(dxv), f(dg)])
+        gy = torch.autograd.grad([out], [y, x, z, D], [dout])
+        if padded:
+            pad = lay.inv_i32 < 0
+            assert all(float(t[pad].abs().sum()) == 0 for t in (xv, dts, g, gy[0]))
+        res.append(([pick(xv), pick(dts), pick(g), out, pick(gx[0]), gx[1], pick(gy[0]), pick(gy[1]), gy[2]], [gx[2], gx[3], gy[3]]))
+    assert all(torch.equal(a, b) for a, b in zip(res[0][0], res[1][0]))
+    assert all(rel_err(a, b) < 1e-5 for a, b in zip(res[0][1], res[1][1]))
