@@ -589,7 +589,7 @@ class Mamba2(nn.Module):
             # everything elementwise around the SSD core in two kernels: dt = softplus(dt + bias), the log decay and
             # x dt before it; the D skip and the silu(z) gate after it
             from ..ops.gla import scalar_gla
-            xv, _, g = gates.mamba2_pre(xs, dt, self.dt_bias, self.A_log, H, P)
+            xv, _, g, xs = gates.mamba2_pre_skip(xs, dt, self.dt_bias, self.A_log, H, P)
             y = scalar_gla(C.reshape(T, G, N), B.reshape(T, G, N), xv, g, meta, scale=1.0)
             y = gates.mamba2_post(y, xs, z, self.D, H, P)
             if self.rmsnorm:
@@ -616,7 +616,7 @@ class Mamba2(nn.Module):
             return None
         lay, rows = ChunkLayout.of(meta, chunk), out[0].shape[0]
         xs, B, C = split_columns(out[0], (Di, G * N, G * N))
-        xv, _, g = gates.mamba2_pre(xs, dt, self.dt_bias, self.A_log, H, P, lay)
+        xv, _, g, xs = gates.mamba2_pre_skip(xs, dt, self.dt_bias, self.A_log, H, P, lay)
         y = grouped_scalar_gla_chunks(C.reshape(rows, G, N), B.reshape(rows, G, N), xv, g, lay)
         return gates.mamba2_post(y.reshape(rows, H, P), xs, z, self.D, H, P, lay)
 

@@ -165,8 +165,8 @@ def hgrn2_gates(q_raw: torch.Tensor, f_raw: torch.Tensor,
 # ----------------------------------------------------------------------------------------------------------------------
 _lib.register("fb_mamba2_pre_fwd", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                     c_void_p, c_longlong, c_int, c_int, c_void_p])
-_lib.register("fb_mamba2_pre_bwd", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                                    c_void_p, c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p])
+_lib.register("fb_mamba2_pre_bwd", [c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                    c_void_p, c_longlong, c_void_p, c_void_p, c_longlong, c_int, c_int, c_void_p])
 _lib.register("fb_mamba2_post_fwd", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_longlong, c_int,
                                      c_int, c_void_p])
 _lib.register("fb_mamba2_post_bwd", [c_void_p, c_void_p, c_longlong, c_void_p, c_longlong, c_void_p, c_void_p, c_void_p, c_void_p,
@@ -181,7 +181,9 @@ def _views_ok(*ts: torch.Tensor) -> bool:
 class _Mamba2Pre(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, dt_raw, dt_bias, A_log, H, P, lay):
-        """``lay`` (``chunked.ChunkLayout``): x and the results are in its padded rows, ``dt_raw`` is per token."""
+        """``lay`` (``chunked.ChunkLayout``): x and the results are in its padded rows, ``dt_raw`` is per token.  The last result is x
+        itself for its other reader, whose gradient the backward kernel adds."""
+        ctx.set_materialize_grads(False)
         T = x.shape[0]
         ctx.src = None if lay is None or lay.aligned else lay.inv_i32
         bias32, alog32 = dt_bias.detach().float().contiguous(), A_log.detach().float().contiguous()
@@ -194,23 +196,26 @@ class _Mamba2Pre(torch.autograd.Function):
         _lib.check(rc, "fb_mamba2_pre_fwd")
         _lib.count_launch()
         ctx.save_for_backward(x, dt_raw, bias32, alog32, dt)
-        ctx.dims = (H, P)
+        ctx.dims, ctx.x_slot = (H, P), slots.of(x)
         ctx.dtypes = (dt_bias.dtype, A_log.dtype, dt_raw.dtype)
-        return xv, dt, g
+        return xv, dt, g, x.view_as(x)
 
     @staticmethod
-    def backward(ctx, dxv, ddt, dg):
+    def backward(ctx, dxv, ddt, dg, dskip):
         x, dt_raw, bias32, alog32, dt = ctx.saved_tensors
         H, P = ctx.dims
         T = x.shape[0]
         dxv = torch.zeros(T, H, P, dtype=x.dtype, device=x.device) if dxv is None else _lib.dense(dxv)
         dg = torch.zeros(T, H, dtype=torch.float32, device=x.device) if dg is None else _lib.dense(dg.float())
         ddt = None if ddt is None else ddt.float().contiguous()
-        dx = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
+        dskip = None if dskip is None else _lib.dense(dskip.to(x.dtype))
+        dx = None if ctx.x_slot is None else ctx.x_slot.take(T, H * P, x.dtype, x.device)
+        if dx is None or not _views_ok(dx):
+            dx = torch.empty(T, H * P, dtype=x.dtype, device=x.device)
         d_raw = torch.empty(dt_raw.shape[0], H, dtype=torch.float32, device=x.device)
         rc = _lib.lib().fb_mamba2_pre_bwd(x.data_ptr(), x.stride(0), dt_raw.data_ptr(), dt_raw.stride(0), bias32.data_ptr(),
-                                          alog32.data_ptr(), dxv.data_ptr(), dg.data_ptr(), _lib.ptr(ddt), dx.data_ptr(),
-                                          d_raw.data_ptr(), _lib.ptr(ctx.src), T, H, P, _lib.stream_ptr())
+                                          alog32.data_ptr(), dxv.data_ptr(), dg.data_ptr(), _lib.ptr(ddt), _lib.ptr(dskip),
+                                          dx.data_ptr(), dx.stride(0), d_raw.data_ptr(), _lib.ptr(ctx.src), T, H, P, _lib.stream_ptr())
         _lib.check(rc, "fb_mamba2_pre_bwd")
         _lib.count_launch()
         d_bias = d_raw.sum(0)
@@ -278,9 +283,14 @@ def mamba2_kernels(x, dt_raw, z, P: int) -> bool:
 def mamba2_pre(x, dt_raw, dt_bias, A_log, H: int, P: int, lay=None):
     """``x [T, H * P]`` and ``dt_raw [T, H]`` (strided views are fine) -> ``xv = x dt`` ``[T, H, P]``, ``dt = softplus(dt_raw +
     dt_bias)`` and the log decay ``g = -exp(A_log) dt`` (both fp32 ``[T, H]``), in one kernel."""
+    return mamba2_pre_skip(x, dt_raw, dt_bias, A_log, H, P, lay)[:3]
+
+
+def mamba2_pre_skip(x, dt_raw, dt_bias, A_log, H: int, P: int, lay=None):
+    """``mamba2_pre`` and x once more: the skip connection reads that, and x's two gradients meet in the backward kernel."""
     if mamba2_kernels(x, dt_raw, x, P):
         return _Mamba2Pre.apply(x, dt_raw, dt_bias, A_log, H, P, lay)
-    return mamba2_pre_reference(x, dt_raw, dt_bias, A_log, H, P)
+    return (*mamba2_pre_reference(x, dt_raw, dt_bias, A_log, H, P), x)
 
 
 def mamba2_post(y, x, z, D, H: int, P: int, lay=None):

@@ -680,3 +680,38 @@ def test_mamba2_elementwise_kernels_in_chunk_rows(lens, P):
         res.append(([pick(xv), pick(dts), pick(g), out, pick(gx[0]), gx[1], pick(gy[0]), pick(gy[1]), gy[2]], [gx[2], gx[3], gy[3]]))
     assert all(torch.equal(a, b) for a, b in zip(res[0][0], res[1][0]))
     assert all(rel_err(a, b) < 1e-5 for a, b in zip(res[0][1], res[1][1]))
+
+
+@pytest.mark.parametrize("P", [64, 256])
+@pytest.mark.parametrize("lens", [[1], [128], [15, 17, 63, 65, 1, 200]])
+def test_mamba2_skip_gradient_in_place(lens, P):
+    """x as a column block read by the value and by the skip connection: its gradient, added up in the kernel and written into the block's
+    columns, against the two gradients of separate readers (each rounded to bf16 and so their sum: 3 half ulps); the rest bit for bit."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.gates import mamba2_post, mamba2_pre, mamba2_pre_skip
+    from flame_b200.ops.slots import split_columns
+    torch.manual_seed(P)
+    T, H, lay = sum(lens), 3, ChunkLayout.of(_meta(lens), 64)
+    for rows, lay_ in ((T, None), (lay.Tp, lay)):
+        w0, y0, z0, dt0 = _bf(rows, H * P + 24), _bf(rows, H, P), _bf(T, H * P, s=2.0), _bf(T, H, s=2.0)
+        par = [torch.randn(H, device=DEV) for _ in range(3)]
+        dxv, dg, dout, db = _bf(rows, H, P), torch.randn(rows, H, device=DEV), _bf(T, H * P), _bf(rows, 24)
+        res = []
+        for together in (True, False):
+            w, y, z, dt, A, bias, D = (t.clone().requires_grad_(True) for t in (w0, y0, z0, dt0, *par))
+            if together:
+                x, b = split_columns(w, (H * P, 24))
+                xv, _, g, xs = mamba2_pre_skip(x, dt, bias, A, H, P, lay_)
+            else:
+                x, b = w[:, :H * P], w[:, H * P:]
+                xs = x
+                xv, _, g = mamba2_pre(x, dt, bias, A, H, P, lay_)
+            out = mamba2_post(y, xs, z, D, H, P, lay_)
+            gr = torch.autograd.grad([xv, g, out, b], [w, y, z, dt, bias, A, D], [dxv, dg, dout, db])
+            real = slice(None) if lay_ is None else lay.rows
+            res.append((gr[0][real].float(), [out, *gr[1:]]))
+        assert all(torch.equal(a, b) for a, b in zip(res[0][1], res[1][1]))
+        (a, _), (b, _) = res
+        assert torch.equal(a[:, H * P:], b[:, H * P:])
+        # terms of either sign: each rounding is relative to a term, bounded here by the larger of the terms' sizes
+        assert float((a - b).abs().max()) <= 3 * 2.0 ** -8 * float(max(a.abs().max(), b.abs().max())) and rel_err(a, b) < 3 * 2.0 ** -8
