@@ -4,6 +4,7 @@
 #include <stdint.h>
 #include <type_traits>
 
+#include "fine_math.cuh"
 #include "host_utils.cuh"
 
 namespace {
@@ -480,17 +481,19 @@ struct GlaRows {
   const int* src;
   long long ldq, ldk, ldg;
 };
-// log(sigmoid(x)) mul without cancellation or underflow: log(1 + e), e = exp(-|x|) <= 1, is 2 artanh(e / (2 + e)), by the artanh series
-// up to s^13 for s <= 1/3 (relative error below 1e-7)
-__device__ __forceinline__ float log_sigmoid(float x, float mul) {
-  const float e = __expf(-fabsf(x)), s = __fdividef(e, 2.f + e), w = s * s;
+// log(sigmoid(x)) / norm without cancellation or underflow (inv: 1 / norm): log(1 + e), e = exp(-|x|) <= 1, is 2 artanh(s), s = e / (2 + e), by the
+// artanh series up to s^13 for s <= 1/3 (off by 1.5e-8 relative at most).  Both quotients are corrected by their remainders, so that the
+// exponential (2^-22) is what is left: closer than the chain of kernels before it, whose exponent was rounded to one float.
+__device__ __forceinline__ float log_sigmoid(float x, float norm, float inv) {
+  const float e = exp_neg_fine(-fabsf(x)), y = 2.f + e, r = __fdividef(1.f, y), s0 = e * r, s = fmaf(fmaf(-y, s0, e), r, s0), w = s * s;
   float p = fmaf(w, 1.f / 13.f, 1.f / 11.f);
   p = fmaf(p, w, 1.f / 9.f);
   p = fmaf(p, w, 1.f / 7.f);
   p = fmaf(p, w, 1.f / 5.f);
   p = fmaf(p, w, 1.f / 3.f);
   p = fmaf(p, w, 1.f);
-  return (fminf(x, 0.f) - 2.f * s * p) * mul;
+  const float l = fminf(x, 0.f) - 2.f * s * p, q = l * inv;
+  return l > -3e38f ? fmaf(fmaf(-norm, q, l), inv, q) : q;  // (-inf leaves no remainder)
 }
 __device__ __forceinline__ void unpack8_bf16(const uint4& v, float (&f)[8]) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
@@ -1194,9 +1197,10 @@ __global__ void __launch_bounds__(256, 2) gla_prep_fwd_kernel(const __nv_bfloat1
     kv[i] = i < there ? *reinterpret_cast<const uint32_t*>(kp + i * at.ldk) : 0u;
   }
   float2 run = make_float2(0.f, 0.f);
+  const float inv = RAW ? __frcp_rn(norm) : 0.f;
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
-    if (RAW) bv[i] = i < there ? make_float2(log_sigmoid(bv[i].x, norm), log_sigmoid(bv[i].y, norm)) : make_float2(0.f, 0.f);
+    if (RAW) bv[i] = i < there ? make_float2(log_sigmoid(bv[i].x, norm, inv), log_sigmoid(bv[i].y, norm, inv)) : make_float2(0.f, 0.f);
     run.x += bv[i].x;
     run.y += bv[i].y;
     bv[i] = run;
@@ -1245,7 +1249,7 @@ __global__ void __launch_bounds__(256, 2) gla_prep_fwd_kernel(const __nv_bfloat1
 
 extern "C" {
 
-// g: fp32 (raw 0), or bf16 with g = logsigmoid(raw) norm; src, ld*: see GlaRows
+// g: fp32 (raw 0), or bf16 whose logsigmoid over norm is the gate; src, ld*: see GlaRows
 int fb_gla_prep_fwd(const void* q, const void* k, const void* g, int raw, float norm, const int* src, long long ldq, long long ldk, long long ldg,
                     float* b, void* khat, void* qbar, void* qt, void* k3, float* alpha, int NC, int H, int dk, float scale, cudaStream_t stream) {
   if (NC <= 0) return 0;

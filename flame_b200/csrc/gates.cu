@@ -12,6 +12,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "fine_math.cuh"
 #include "host_utils.cuh"
 
 namespace {
@@ -207,14 +208,19 @@ __global__ void colsum_rows_kernel(const float* __restrict__ part, int parts, in
 // The delta rule's gates (fla/layers/delta_net.py:246-252, fla/ops/gated_delta_rule/gate.py:20-44), per token and head:
 //   beta = mul sigmoid(b),   g = -exp(A_log) softplus(a + dt_bias)
 // read from column blocks of the projection and written as fp32 in the padded rows of the chunk layout (zeros in the
-// padding).  A few scalars per token: what they cost is launches, so one kernel stands for ten of torch's forward and one
+// padding).  A few scalars per token: what they cost is launches, not arithmetic, which is that of torch's fp32 functions or closer
+// to the exact result (fine_math.cuh); one kernel stands for ten of torch's forward and one
 // (and the sum of its partials) for fifteen backward.  src: packed token of a padded row (-1: padding), or null: the same.
 template <bool BF16>
 __device__ __forceinline__ float param(const void* p, int h) {
   return BF16 ? __bfloat162float(((const __nv_bfloat16*)p)[h]) : ((const float*)p)[h];
 }
-// the exponential never overflows, and its logarithm does not round 1 + exp first
-__device__ __forceinline__ float softplus_exact(float x) { return fmaxf(x, 0.f) + log1pf(__expf(-fabsf(x))); }
+// softplus(x), with sigmoid(x) from the same exponential, which never overflows and whose logarithm does not round 1 + exp first
+__device__ __forceinline__ float softplus_fine(float x, float& sigmoid) {
+  const float e = exp_rn(-fabsf(x));
+  sigmoid = __fdiv_rn(x >= 0.f ? 1.f : e, 1.f + e);
+  return fmaxf(x, 0.f) + log1pf(e);
+}
 
 template <bool BF16>
 __global__ void delta_gates_fwd_kernel(const __nv_bfloat16* __restrict__ b, long long ldb, const __nv_bfloat16* __restrict__ a, long long lda,
@@ -227,8 +233,9 @@ __global__ void delta_gates_fwd_kernel(const __nv_bfloat16* __restrict__ b, long
   const long long t = src == nullptr ? r : src[r];
   float be = 0.f, ge = 0.f;
   if (t >= 0) {
-    be = mul * sigmoidf_(__bfloat162float(b[t * ldb + h]));
-    if (a != nullptr) ge = -__expf(param<BF16>(A_log, h)) * softplus_exact(__bfloat162float(a[t * lda + h]) + param<BF16>(dt_bias, h));
+    float s;
+    be = mul * sigmoid_fine(__bfloat162float(b[t * ldb + h]));
+    if (a != nullptr) ge = -exp_rn(param<BF16>(A_log, h)) * softplus_fine(__bfloat162float(a[t * lda + h]) + param<BF16>(dt_bias, h), s);
   }
   beta[i] = be;
   if (a != nullptr) g[i] = ge;
@@ -247,17 +254,18 @@ __global__ void __launch_bounds__(DG_THREADS) delta_gates_bwd_kernel(
   const int h = threadIdx.x % H, slot = threadIdx.x / H;
   float sA = 0.f, sdt = 0.f;
   if (slot < per) {
-    const float nA = a == nullptr ? 0.f : -__expf(param<BF16>(A_log, h)), dt = a == nullptr ? 0.f : param<BF16>(dt_bias, h);
+    const float nA = a == nullptr ? 0.f : -exp_rn(param<BF16>(A_log, h)), dt = a == nullptr ? 0.f : param<BF16>(dt_bias, h);
     for (long long r = (long long)blockIdx.x * per + slot; r < rows; r += (long long)gridDim.x * per) {
       const long long t = src == nullptr ? r : src[r];
       if (t < 0) continue;
-      const float s = sigmoidf_(__bfloat162float(b[t * ldb + h]));
+      const float s = sigmoid_fine(__bfloat162float(b[t * ldb + h]));
       db[t * lddb + h] = __float2bfloat16(dbeta[r * H + h] * mul * s * (1.f - s));
       if (a != nullptr) {
         const float x = __bfloat162float(a[t * lda + h]) + dt, d = dg[r * H + h];
-        const float v = d * nA * sigmoidf_(x);
+        float sx;
+        const float plus = softplus_fine(x, sx), v = d * nA * sx;
         da[t * ldda + h] = __float2bfloat16(v);
-        sA = fmaf(d, nA * softplus_exact(x), sA);
+        sA = fmaf(d, nA * plus, sA);
         sdt += v;
       }
     }

@@ -267,7 +267,7 @@ def gla_prep(q, k, g, scale: float, lay=None, norm=None):
     b, khat, qbar, qt, k3 = new(NC, 64, dt=torch.float32), new(NC, 64), new(NC, 64), new(NC, 48), new(NC, 3, 48)
     alpha = new(NC, dt=torch.float32)
     src, ldq, ldk = _gla_rows(q, k, lay)
-    rc = _lib.lib().fb_gla_prep_fwd(q.data_ptr(), k.data_ptr(), g.data_ptr(), int(norm is not None), 1.0 / float(norm or 1.0), src, ldq, ldk,
+    rc = _lib.lib().fb_gla_prep_fwd(q.data_ptr(), k.data_ptr(), g.data_ptr(), int(norm is not None), float(norm or 1.0), src, ldq, ldk,
                                     H * dk if lay is None else _token_ld(g), b.data_ptr(), khat.data_ptr(), qbar.data_ptr(), qt.data_ptr(),
                                     k3.data_ptr(), alpha.data_ptr(), NC, H, dk, float(scale), _lib.stream_ptr())
     _lib.check(rc, "fb_gla_prep_fwd")

@@ -715,3 +715,37 @@ def test_mamba2_skip_gradient_in_place(lens, P):
         assert torch.equal(a[:, H * P:], b[:, H * P:])
         # terms of either sign: each rounding is relative to a term, bounded here by the larger of the terms' sizes
         assert float((a - b).abs().max()) <= 3 * 2.0 ** -8 * float(max(a.abs().max(), b.abs().max())) and rel_err(a, b) < 3 * 2.0 ** -8
+
+
+def test_gla_gate_formed_in_the_kernel():
+    """log(sigmoid(x)) / 16 of the preparation kernel (the first row of a chunk holds one token's gate) against fp64: the exponential is
+    off by 2^-22, the other operations round to 2^-24 each, 2^-21 together, also where the gate is nearly zero."""
+    from flame_b200.ops import chunk_kernels
+    from flame_b200.ops.chunked import ChunkLayout
+    T, H, dk = 300, 2, 64
+    lay = ChunkLayout.of(_meta([1] * T), 64)
+    x = torch.cat([torch.linspace(-60, 60, T * H * dk - 2, device=DEV), torch.tensor([float("-inf"), 0.0], device=DEV)]).bfloat16().view(T, H, dk)
+    b = chunk_kernels.gla_prep(x, x, x, 1.0, lay, 16.0)[0][:, 0]
+    want = F.logsigmoid(x.double()) / 16
+    assert b[-1, -1, -2] == float("-inf")
+    ok = want.abs() < float("inf")
+    assert ((b.double() - want).abs()[ok] <= 2.0 ** -21 * want.abs()[ok]).all()
+
+
+def test_silu_rows_round_as_often_as_torch():
+    """Every bf16 argument in [-80, 80]: no more results off the correctly rounded one than torch's fp32 chain leaves, both ways."""
+    from flame_b200.ops.activations import silu_out_of_chunks
+    from flame_b200.ops.chunked import ChunkLayout
+    x = torch.arange(1 << 16, device=DEV, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    x = x[(x.abs() <= 80) & (x.abs() >= 2.0 ** -60)]
+    x = x[:len(x) // 64 * 64].view(-1, 64)
+    lay, off = ChunkLayout.of(_meta([x.shape[0]]), 64), []
+    xr = x.double().requires_grad_(True)
+    want = F.silu(xr)
+    want.sum().backward()
+    for new in (True, False):
+        xi = torch.zeros(lay.Tp if new else len(x), 64, device=DEV, dtype=x.dtype).index_copy(0, torch.arange(len(x), device=DEV), x).requires_grad_(True)
+        y = silu_out_of_chunks(xi.view(lay.NC, 64, 64), lay) if new else F.silu(xi)
+        y.sum().backward()
+        off.append([int((a != b.to(a.dtype)).sum()) for a, b in ((y, want), (xi.grad[:len(x)], xr.grad))])
+    assert off[0][0] <= off[1][0] and off[0][1] <= off[1][1], off

@@ -845,3 +845,23 @@ def test_side_by_side_projections_of_odd_sizes(rows, mains):
     assert rel_err(torch.cat(parts, 1), xr @ wr.T) < 5e-3 and rel_err(x.grad, dy @ wr) < 5e-3
     got = grad.view(76, 128) - 1 if mains else torch.cat([w.grad for w in ws])
     assert rel_err(got, dy.T @ xr) < (1e-4 if mains else 5e-3)
+
+
+def test_delta_gates_are_as_exact_as_fp32_allows():
+    """Against fp64, at decay rates of 1 to 16 and arguments whose fp32 sum is exact: an exponential and a logarithm of at most one ulp each
+    (2^-23), a sum and two products or quotients of half of one: 4 x 2^-23 for the decay, 2 x 2^-23 for beta, relative."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.gates import delta_gates
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    T, H = 4096, 16
+    lay = ChunkLayout.of(VarlenMeta.from_cu_seqlens(torch.tensor([0, T], dtype=torch.int32), T, torch.device(DEV)), 64)
+    b = (torch.randn(T, H, device=DEV) * 8).bfloat16()
+    a = (torch.randn(T, H, device=DEV) * 64).round().clamp(-240, 240).div(16).bfloat16()
+    A_log, dt = torch.linspace(0, 2.77, H, device=DEV), torch.randint(-32, 32, (H,), device=DEV) / 16.0
+    beta, g = delta_gates(b, a, A_log, dt, 2.0, lay)
+    wb = 2 * b.double().sigmoid()
+    x = a.double() + dt.double()
+    wg = -A_log.double().exp() * (x.clamp_min(0) + torch.log1p((-x.abs()).exp()))
+    assert ((beta.view(T, H).double() - wb) / wb).abs().max() <= 2 * 2.0 ** -23
+    assert ((g.view(T, H).double() - wg) / wg).abs().max() <= 4 * 2.0 ** -23
