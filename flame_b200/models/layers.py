@@ -220,7 +220,7 @@ def _feature_map(name: str, x: torch.Tensor) -> torch.Tensor:
 def _conv_delta_rule(xs, convs, gates, meta: VarlenMeta, heads: int):
     """Short convolutions and (gated) delta rule in one go, or None where something wants the convolutions' own results."""
     from ..ops.delta_rule import conv_gated_delta_rule
-    if not plain(convs, ShortConvolution):
+    if not plain(convs, ShortConvolution) or any(c.activation not in ("silu", "swish") for c in convs):
         return None
     return conv_gated_delta_rule(xs, [c.weight for c in convs], [c.bias for c in convs], gates, meta, heads)
 

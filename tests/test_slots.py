@@ -307,3 +307,31 @@ def test_pack_of_column_blocks(cols, cu):
         (y * w).sum().backward()
         got += [(y.detach(), x.grad)]
     assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,kw", [("DeltaNet", dict(num_heads=2)), ("GatedDeltaNet", dict(num_heads=2, head_dim=64))])
+@pytest.mark.parametrize("which", ["q_conv1d", "v_conv1d"])
+def test_a_convolution_without_activation_stays_without(name, kw, which):
+    """Convolutions and delta rule run in one go only as SiLU convolutions.  The other side's convolutions are called as modules (a hook that
+    does nothing): the same operations on packed rows, bf16 results up to a few roundings (2^-8 of the largest entry)."""
+    from flame_b200.models import layers as layers_mod
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    dev, D = torch.device("cuda", 0), 256
+    m = getattr(layers_mod, name)(D, **kw)
+    for p in m.parameters():
+        torch.nn.init.normal_(p, std=0.3) if p.dim() > 1 else torch.nn.init.uniform_(p, 0.5, 1.0)
+    m = m.to(dev).bfloat16()
+    meta = VarlenMeta.from_cu_seqlens(torch.tensor((0, 1, 66, 131), dtype=torch.int32, device=dev))
+    x, out = torch.randn(131, D, device=dev).bfloat16(), []
+    getattr(m, which).activation = None
+    with torch.no_grad():
+        out.append(m(x, meta).double())
+        handle = m.k_conv1d.register_forward_hook(lambda *a: None)
+        out.append(m(x, meta).double())
+        handle.remove()
+        getattr(m, which).activation = "silu"
+        with_silu = m(x, meta).double()
+    scale = out[1].abs().max()
+    assert (out[0] - out[1]).abs().max() <= 4 * 2.0 ** -8 * scale < (with_silu - out[1]).abs().max()
