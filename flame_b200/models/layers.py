@@ -171,7 +171,7 @@ class GatedLinearAttention(nn.Module):
             layers = (self.q_proj, self.k_proj, self.v_proj)
             # (torch's activations are several times slower on column blocks)
             whole = self.use_short_conv or self.feature_map is None
-            low = plain((self.gk_proj,), nn.Sequential)
+            low = plain((self.gk_proj,), nn.Sequential) and len(self.gk_proj) == 2
             more = ((self.g_proj,) if self.use_output_gate else ()) + ((self.gk_proj[0],) if low else ())
             q, k, v, *rest = _projections(x, layers, more) if whole else (l(x) for l in (*layers, *more))
             gk = self.gk_proj[1](rest[-1]) if low else self.gk_proj(x)

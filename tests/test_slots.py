@@ -335,3 +335,31 @@ def test_a_convolution_without_activation_stays_without(name, kw, which):
         with_silu = m(x, meta).double()
     scale = out[1].abs().max()
     assert (out[0] - out[1]).abs().max() <= 4 * 2.0 ** -8 * scale < (with_silu - out[1]).abs().max()
+
+
+def test_a_longer_low_rank_gate_runs_whole():
+    """GLA takes its low-rank gate projection apart only when it is the two layers that it makes itself: one with a third entry, or with one
+    alone, gives what the same modules give as a module of another kind."""
+    from flame_b200.models.layers import GatedLinearAttention
+    from flame_b200.models.modules import Linear
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    m = GatedLinearAttention(32, num_heads=2)
+    for extra in (lambda s: torch.nn.Sequential(*s, torch.nn.Tanh()), lambda s: torch.nn.Sequential(Linear(32, 16))):
+        m.gk_proj = extra(m.gk_proj)
+        for p in m.parameters():
+            torch.nn.init.normal_(p, std=0.5)
+
+        class Whole(torch.nn.Module):
+            def __init__(self, seq):
+                super().__init__()
+                self.seq = seq
+
+            def forward(self, x):
+                return self.seq(x)
+
+        x, meta = torch.randn(7, 32), VarlenMeta.dense(1, 7, torch.device("cpu"))
+        got = m(x, meta)
+        m.gk_proj = Whole(m.gk_proj)
+        torch.testing.assert_close(got, m(x, meta))
+        m.gk_proj = m.gk_proj.seq
