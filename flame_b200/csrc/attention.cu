@@ -34,7 +34,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 struct AttnParams {
   const int* cu_seqlens;    // [nseq + 1]
-  const int* tile_offsets;  // [nseq + 1] prefix sum of ceil(len / 128)
+  const int* tile_list;  // see attn_tiles.cuh
   int nseq;
   int H, Hkv;
   int total_tokens;
@@ -99,7 +99,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                 const __grid_constant__ CUtensorMap tmV, AttnParams p) {
   using L = FwdSmem<DH>;
   int head, doc, tile_in_doc;
-  if (!attn_tile(p.tile_offsets, p.nseq, p.H, true, head, doc, tile_in_doc)) return;
+  if (!attn_tile(p.tile_list, p.nseq, p.H, true, head, doc, tile_in_doc)) return;
   const int kv_head = head / (p.H / p.Hkv);
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
@@ -422,7 +422,7 @@ attn_fwd_pt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   using L = FwdPtSmem;
   constexpr int DH = 64;
   int head, doc, tile_in_doc;
-  if (!attn_tile(p.tile_offsets, p.nseq, p.H, true, head, doc, tile_in_doc)) return;
+  if (!attn_tile(p.tile_list, p.nseq, p.H, true, head, doc, tile_in_doc)) return;
   const int kv_head = head / (p.H / p.Hkv);
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
@@ -678,7 +678,7 @@ attn_fwd_pt_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // ------------------------------------------------------------------------------------------------
 struct AttnBwdParams {
   const int* cu_seqlens;
-  const int* tile_offsets;
+  const int* tile_list;
   int nseq;
   int H, Hkv;
   int total_tokens;
@@ -752,7 +752,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   static_assert(DH == 64, "the backward kernel is laid out for head dim 64");
   using L = BwdSmem<DH>;
   int kv_head, doc, j;  // early key tiles see the most queries
-  if (!attn_tile(p.tile_offsets, p.nseq, p.Hkv, false, kv_head, doc, j)) return;
+  if (!attn_tile(p.tile_list, p.nseq, p.Hkv, false, kv_head, doc, j)) return;
   const int group = p.H / p.Hkv;
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
@@ -1093,7 +1093,7 @@ attn_bwd128_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   using L = Bwd128Smem;
   constexpr int DH = 128, BQ2 = L::BQ2;
   int kv_head, doc, j;  // early key tiles see the most queries
-  if (!attn_tile(p.tile_offsets, p.nseq, p.Hkv, false, kv_head, doc, j)) return;
+  if (!attn_tile(p.tile_list, p.nseq, p.Hkv, false, kv_head, doc, j)) return;
   const int group = p.H / p.Hkv;
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
@@ -1497,15 +1497,15 @@ int make_qkv_map(CUtensorMap* m, const void* base, long long T, int H, int DH, l
 extern "C" {
 
 
-// tile_offsets: int32 [3 nseq + 2], see attn_tiles.cuh
-int fb_attn_tile_offsets(const int* cu_seqlens, int nseq, int* tile_offsets, cudaStream_t stream) {
-  attn_tile_list_kernel<<<1, LIST_THREADS, 0, stream>>>(cu_seqlens, nseq, tile_offsets);
+// tile_list: int32 [3 nseq + 2], see attn_tiles.cuh
+int fb_attn_tile_list(const int* cu_seqlens, int nseq, int* tile_list, cudaStream_t stream) {
+  attn_tile_list_kernel<<<1, LIST_THREADS, 0, stream>>>(cu_seqlens, nseq, tile_list);
   return fb::launch_ok("attn_tile_list_kernel");
 }
 
 // max_tiles: an upper bound on the number of 128-row tiles (T / 128 + nseq is always enough).
 int fb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse, const int* cu_seqlens,
-                const int* tile_offsets, int nseq, int max_tiles, long long T, int H, int Hkv, int DH,
+                const int* tile_list, int nseq, int max_tiles, long long T, int H, int Hkv, int DH,
                 long long q_stride_t, long long k_stride_t, long long v_stride_t, long long o_stride_t, float scale,
                 int window, cudaStream_t stream) {
   if (T == 0) return 0;
@@ -1518,7 +1518,7 @@ int fb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse
   if (rc) return rc;
   AttnParams p;
   p.cu_seqlens = cu_seqlens;
-  p.tile_offsets = tile_offsets;
+  p.tile_list = tile_list;
   p.nseq = nseq;
   p.H = H;
   p.Hkv = Hkv;
@@ -1555,7 +1555,7 @@ int fb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse
 // Stick-breaking attention forward (head dim 64): o = sum_j att_ij v_j without normalisation, rem[h, t] = 1 - sum_j att_ij.
 // o_lo: optional bf16 [T, H, 64] that receives the part of the fp32 result the bf16 output lost (null: not written).
 int fb_sb_attn_fwd(const void* q, const void* k, const void* v, void* o, void* o_lo, float* rem, const int* cu_seqlens,
-                   const int* tile_offsets, int nseq, int max_tiles, long long T, int H, int DH, long long q_stride_t,
+                   const int* tile_list, int nseq, int max_tiles, long long T, int H, int DH, long long q_stride_t,
                    long long k_stride_t, long long v_stride_t, long long o_stride_t, float scale, cudaStream_t stream) {
   if (T == 0) return 0;
   if (DH != 64) return -2;
@@ -1567,7 +1567,7 @@ int fb_sb_attn_fwd(const void* q, const void* k, const void* v, void* o, void* o
   if (rc) return rc;
   AttnParams p;
   p.cu_seqlens = cu_seqlens;
-  p.tile_offsets = tile_offsets;
+  p.tile_list = tile_list;
   p.nseq = nseq;
   p.H = H;
   p.Hkv = H;
@@ -1604,7 +1604,7 @@ int fb_attn_delta(const void* o, const void* dout, float* delta, long long T, in
 
 // dq_accum: fp32 [T, H, DH], must be zero on entry.  Head dims 64 and 128 (two kernels, see above).
 int fb_attn_bwd(const void* q, const void* k, const void* v, const void* dout, const float* lse, const float* delta,
-                float* dq_accum, void* dk, void* dv, const int* cu_seqlens, const int* tile_offsets, int nseq,
+                float* dq_accum, void* dk, void* dv, const int* cu_seqlens, const int* tile_list, int nseq,
                 int max_tiles, long long T, int H, int Hkv, int DH, long long q_stride_t, long long k_stride_t,
                 long long v_stride_t, long long do_stride_t, long long dk_stride_t, long long dv_stride_t, float scale,
                 int window, cudaStream_t stream) {
@@ -1630,7 +1630,7 @@ int fb_attn_bwd(const void* q, const void* k, const void* v, const void* dout, c
   if (rc) return rc;
   AttnBwdParams p;
   p.cu_seqlens = cu_seqlens;
-  p.tile_offsets = tile_offsets;
+  p.tile_list = tile_list;
   p.nseq = nseq;
   p.H = H;
   p.Hkv = Hkv;

@@ -1,6 +1,7 @@
-// The work list of the attention kernels: 128-row tiles of packed documents, built once per batch (fb_attn_tile_offsets).
+// The work list of the attention kernels: 128-row tiles of packed documents, built once per batch (fb_attn_tile_list): one
+// int32 array of 3 nseq + 2,
 //
-//   int32 [nseq + 1]  prefix sum of the tiles of the documents, in their order
+//   int32 [nseq + 1]  prefix sum of the tiles of the documents, in their order (VarlenMeta.tile_offsets; no kernel reads it)
 //   int32 [nseq + 1]  the same over the documents by falling length
 //   int32 [nseq]      those documents
 //

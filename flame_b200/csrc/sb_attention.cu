@@ -36,7 +36,7 @@ constexpr float kLog2e = 1.4426950408889634f;
 
 struct SbBwdParams {
   const int* cu_seqlens;
-  const int* tile_offsets;
+  const int* tile_list;
   int nseq, H, total_tokens;
   float scale, scale_log2;
   const float* tot;    // [H, T]  do.o - drem (1 - rem)
@@ -73,7 +73,7 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO, SbBwdParams p) {
   using L = Smem;
   int head, doc, ti;
-  if (!attn_tile(p.tile_offsets, p.nseq, p.H, true, head, doc, ti)) return;
+  if (!attn_tile(p.tile_list, p.nseq, p.H, true, head, doc, ti)) return;
   const int doc_start = p.cu_seqlens[doc];
   const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
   const int q0 = ti * BQ;
@@ -375,7 +375,7 @@ extern "C" {
 // (bf16 [T, H, 64], contiguous) or null.
 int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, const void* o_lo, const void* dout, const float* rem,
                    const float* drem, float* tot, void* dq, float* dk_acc, float* dv_acc, const int* cu_seqlens,
-                   const int* tile_offsets, int nseq, int max_tiles, long long T, int H, long long q_stride_t,
+                   const int* tile_list, int nseq, int max_tiles, long long T, int H, long long q_stride_t,
                    long long k_stride_t, long long v_stride_t, long long o_stride_t, long long do_stride_t,
                    long long dq_stride_t, float scale, cudaStream_t stream) {
   if (T == 0) return 0;
@@ -400,7 +400,7 @@ int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
   if (rc) return rc;
   SbBwdParams p;
   p.cu_seqlens = cu_seqlens;
-  p.tile_offsets = tile_offsets;
+  p.tile_list = tile_list;
   p.nseq = nseq;
   p.H = H;
   p.total_tokens = (int)T;

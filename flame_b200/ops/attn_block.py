@@ -36,7 +36,7 @@ class _QkvAttnFn(torch.autograd.Function):
         o = torch.empty(T, H, Dh, dtype=qkv.dtype, device=qkv.device)
         lse = torch.empty(H, T, dtype=torch.float32, device=qkv.device)
         rc = L.fb_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), lse.data_ptr(),
-                           meta.cu_seqlens.data_ptr(), meta.tile_offsets.data_ptr(), meta.nseq, meta.max_tiles128, T, H,
+                           meta.cu_seqlens.data_ptr(), meta.tile_list.data_ptr(), meta.nseq, meta.max_tiles128, T, H,
                            Hkv, Dh, q.stride(0), k.stride(0), v.stride(0), o.stride(0), float(scale), int(window),
                            _lib.stream_ptr())
         _lib.check(rc, "fb_attn_fwd")
@@ -68,7 +68,7 @@ class _QkvAttnFn(torch.autograd.Function):
         dv = dqkv[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
         rc = L.fb_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), do.data_ptr(), lse.data_ptr(), delta.data_ptr(),
                            dq_acc.data_ptr(), dk.data_ptr(), dv.data_ptr(), meta.cu_seqlens.data_ptr(),
-                           meta.tile_offsets.data_ptr(), meta.nseq, meta.max_tiles128, T, H, Hkv, Dh, q.stride(0),
+                           meta.tile_list.data_ptr(), meta.nseq, meta.max_tiles128, T, H, Hkv, Dh, q.stride(0),
                            k.stride(0), v.stride(0), do.stride(0), dk.stride(0), dv.stride(0), float(ctx.scale),
                            int(ctx.window), _lib.stream_ptr())
         _lib.check(rc, "fb_attn_bwd")

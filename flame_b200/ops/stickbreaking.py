@@ -30,7 +30,7 @@ def _forward(q, k, v, meta: VarlenMeta, scale: float, keep_lo: bool):
     o_lo = torch.empty(T, H, Dh, dtype=q.dtype, device=q.device) if keep_lo else None
     rem = torch.ones(H, T, dtype=torch.float32, device=q.device)
     rc = _lib.lib().fb_sb_attn_fwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), _lib.ptr(o_lo), rem.data_ptr(),
-                                   meta.cu_seqlens.data_ptr(), meta.tile_offsets.data_ptr(), meta.nseq,
+                                   meta.cu_seqlens.data_ptr(), meta.tile_list.data_ptr(), meta.nseq,
                                    meta.max_tiles128, T, H, Dh, q.stride(0), k.stride(0), v.stride(0), o.stride(0),
                                    float(scale), _lib.stream_ptr())
     _lib.check(rc, "fb_sb_attn_fwd")
@@ -45,7 +45,7 @@ def _backward(q, k, v, o, o_lo, rem, do, dr, meta: VarlenMeta, scale: float, dq)
     dkv = torch.zeros(2, T, H, Dh, dtype=torch.float32, device=q.device)
     rc = _lib.lib().fb_sb_attn_bwd(q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), _lib.ptr(o_lo), do.data_ptr(),
                                    rem.data_ptr(), _lib.ptr(dr), tot.data_ptr(), dq.data_ptr(), dkv[0].data_ptr(),
-                                   dkv[1].data_ptr(), meta.cu_seqlens.data_ptr(), meta.tile_offsets.data_ptr(),
+                                   dkv[1].data_ptr(), meta.cu_seqlens.data_ptr(), meta.tile_list.data_ptr(),
                                    meta.nseq, meta.max_tiles128, T, H, q.stride(0), k.stride(0), v.stride(0),
                                    o.stride(0), do.stride(0), dq.stride(0), float(scale), _lib.stream_ptr())
     _lib.check(rc, "fb_sb_attn_bwd")

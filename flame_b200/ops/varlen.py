@@ -15,7 +15,7 @@ import torch
 from . import _lib
 
 _lib.register("fb_position_ids", [c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p])
-_lib.register("fb_attn_tile_offsets", [c_void_p, c_int, c_void_p, c_void_p])
+_lib.register("fb_attn_tile_list", [c_void_p, c_int, c_void_p, c_void_p])
 
 
 @dataclass
@@ -26,7 +26,7 @@ class VarlenMeta:
     max_tiles128: int  # upper bound on the number of 128-token tiles over all documents
     _pos: Optional[torch.Tensor] = None
     _seq_id: Optional[torch.Tensor] = None
-    _tile_offsets: Optional[torch.Tensor] = None
+    _tile_list: Optional[torch.Tensor] = None
     _cu_cpu: Optional[torch.Tensor] = None
     cache: dict = field(default_factory=dict)
 
@@ -88,22 +88,24 @@ class VarlenMeta:
         return self._seq_id
 
     @property
+    def tile_list(self) -> torch.Tensor:
+        """int32 [3 nseq + 2] on the GPU: the attention kernels' work list (``csrc/attn_tiles.cuh``)."""
+        if self._tile_list is None:
+            t = torch.empty(3 * self.nseq + 2, dtype=torch.int32, device=self.device)
+            rc = _lib.lib().fb_attn_tile_list(self.cu_seqlens.data_ptr(), self.nseq, t.data_ptr(), _lib.stream_ptr())
+            _lib.check(rc, "fb_attn_tile_list")
+            _lib.count_launch()
+            self._tile_list = t
+        return self._tile_list
+
+    @property
     def tile_offsets(self) -> torch.Tensor:
-        """int32 [nseq + 1]: prefix sum of ``ceil(len / 128)``; on the GPU the kernels find the rest of their work list
-        (``csrc/attn_tiles.cuh``) behind it in memory."""
-        if self._tile_offsets is None:
-            if self.device.type == "cuda" and _lib.available():
-                t = torch.empty(3 * self.nseq + 2, dtype=torch.int32, device=self.device)
-                rc = _lib.lib().fb_attn_tile_offsets(self.cu_seqlens.data_ptr(), self.nseq, t.data_ptr(),
-                                                     _lib.stream_ptr())
-                _lib.check(rc, "fb_attn_tile_offsets")
-                _lib.count_launch()
-                self._tile_offsets = t[:self.nseq + 1]
-            else:  # not kept: a kernel would look behind it
-                cu = self.cu_seqlens.long()
-                n = (cu[1:] - cu[:-1] + 127) // 128
-                return torch.cat([torch.zeros(1, dtype=torch.long, device=self.device), n.cumsum(0)]).to(torch.int32)
-        return self._tile_offsets
+        """int32 [nseq + 1]: prefix sum of ``ceil(len / 128)``, on the GPU the head of ``tile_list``."""
+        if self.device.type == "cuda" and _lib.available():
+            return self.tile_list[:self.nseq + 1]
+        cu = self.cu_seqlens.long()
+        n = (cu[1:] - cu[:-1] + 127) // 128
+        return torch.cat([torch.zeros(1, dtype=torch.long, device=self.device), n.cumsum(0)]).to(torch.int32)
 
     def lengths_list(self) -> list[int]:
         cu = self.cu_cpu().tolist()

@@ -865,3 +865,25 @@ def test_delta_gates_are_as_exact_as_fp32_allows():
     wg = -A_log.double().exp() * (x.clamp_min(0) + torch.log1p((-x.abs()).exp()))
     assert ((beta.view(T, H).double() - wb) / wb).abs().max() <= 2 * 2.0 ** -23
     assert ((g.view(T, H).double() - wg) / wg).abs().max() <= 4 * 2.0 ** -23
+
+
+@pytest.mark.parametrize("kind", ["softmax", "stickbreaking"])
+def test_attention_reads_the_work_list_by_its_own_name(kind, monkeypatch):
+    """The kernels' work list is a tensor of its whole length: a copy of it serves as well, and nobody asks for the prefix sums that are
+    its head (a copy of those would end where the kernels begin to read).  Same list, so the forward is the same bit for bit."""
+    from flame_b200.ops.attention import attention
+    from flame_b200.ops.stickbreaking import sb_attention
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    lens = [129, 1, 300]
+    meta, T = _meta(lens), sum(lens)
+    assert meta.tile_list.shape == (3 * len(lens) + 2,) and torch.equal(meta.tile_offsets, meta.tile_list[:len(lens) + 1])
+    q, k, v = (torch.randn(T, 2, 64, device=DEV).bfloat16().requires_grad_(True) for _ in range(3))
+    call = (lambda m: attention(q, k, v, m)) if kind == "softmax" else (lambda m: sb_attention(q, k, v, m)[0])
+    want = call(meta)
+    other = _meta(lens)
+    other._tile_list = meta.tile_list.clone()
+    monkeypatch.setattr(VarlenMeta, "tile_offsets", property(lambda self: pytest.fail("prefix sums asked for")))
+    got = call(other)
+    got.sum().backward()
+    assert torch.equal(got, want) and all(torch.isfinite(t.grad).all() for t in (q, k, v))
