@@ -298,7 +298,7 @@ __global__ void delta_gates_sum_kernel(const float* __restrict__ part, int block
 //   post:  out = (y + D x) silu(z)                                                           (z: strided view)
 // A thread owns 8 channels of one token; the P / 8 threads of a head reduce over the head with shuffles.  x, y, xv, dt, g and their
 // gradients may be in the padded rows of the chunk layout: src[row] is the token of a padded row (-1: padding), null the row itself;
-// dt_raw, z, out and theirs are always per token.  The padding's dt, g and dy are zero, its dx is not written.  All four are bound by
+// dt_raw, z, out and theirs are always per token.  The padding's dt, g, dy and dx are zero.  All four are bound by
 // memory; what the mapping saves is the passes that moved x, B, C and y between the two orders around them (layer at 32,761 tokens,
 // 32 heads of 64, forward and backward: 3.90 -> 3.76 ms).
 __device__ __forceinline__ float softplusf_(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
@@ -343,10 +343,12 @@ __global__ void mamba2_pre_bwd_kernel(const __nv_bfloat16* __restrict__ x, long 
   const long long t = gid / vecs;
   const long long tok = t >= T ? -1 : src == nullptr ? t : src[t];
   const bool live = tok >= 0;
-  const int v = live ? (int)(gid - t * vecs) : 0;
+  const int v = t < T ? (int)(gid - t * vecs) : 0;
   const int h = v / LANES;
   float part = 0.f, pre = 0.f;
-  if (live) {
+  if (t < T && !live) {
+    *reinterpret_cast<uint4*>(dx + t * lddx + v * 8) = make_uint4(0, 0, 0, 0);
+  } else if (live) {
     pre = __bfloat162float(dt_raw[tok * ld_dt + h]) + dt_bias[h];
     const float dt = softplusf_(pre);
     float a[8], g[8], o[8];
@@ -408,6 +410,7 @@ __global__ void mamba2_post_bwd_kernel(const __nv_bfloat16* __restrict__ y, cons
   float part = 0.f;
   if (live && tok < 0) {
     *reinterpret_cast<uint4*>(dy + (t * vecs + v) * 8) = make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(dx + (t * vecs + v) * 8) = make_uint4(0, 0, 0, 0);
   } else if (live) {
     const float d = D[h];
     float a[8], b[8], g[8], go[8], oy[8], ox[8], oz[8];

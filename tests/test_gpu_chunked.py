@@ -749,3 +749,29 @@ def test_silu_rows_round_as_often_as_torch():
         y.sum().backward()
         off.append([int((a != b.to(a.dtype)).sum()) for a, b in ((y, want), (xi.grad[:len(x)], xr.grad))])
     assert off[0][0] <= off[1][0] and off[0][1] <= off[1][1], off
+
+
+@pytest.mark.parametrize("add", [False, True])
+@pytest.mark.parametrize("lens", [[1], [15, 17, 63, 65, 1, 200]])
+def test_mamba2_gradients_of_the_padding_are_zero(lens, add):
+    """What the backward hands on for padded rows is seen by tensor hooks and gradient statistics: zeros, not what stood in the memory (free
+    blocks of its size are filled with NaN first)."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.gates import mamba2_post, mamba2_pre_skip
+    T, H, P, lay = sum(lens), 3, 64, ChunkLayout.of(_meta(lens), 64)
+    pad = lay.inv_i32 < 0
+    x = _bf(lay.Tp, H * P).masked_fill(pad[:, None], 0).requires_grad_(True)
+    y, z, dt = _bf(lay.Tp, H, P).requires_grad_(True), _bf(T, H * P), _bf(T, H)
+    par = [torch.randn(H, device=DEV) for _ in range(3)]
+    xv, _, g, xs = mamba2_pre_skip(x, dt, par[0], par[1], H, P, lay)
+    out = mamba2_post(y, xs.detach().requires_grad_(True) if not add else xs, z, par[2], H, P, lay)
+    dirty = [torch.full((lay.Tp, H * P), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(8)]
+    del dirty
+    gx, gy = torch.autograd.grad([xv, g, out], [x, y], [torch.ones_like(xv), torch.ones_like(g), torch.ones_like(out)])
+    for t in (gx, gy):
+        assert torch.isfinite(t).all() and float(t[pad].abs().sum()) == 0
+    xl = xs.detach().requires_grad_(True)
+    dirty = [torch.full((lay.Tp, H * P), float("nan"), device=DEV, dtype=torch.bfloat16) for _ in range(8)]
+    del dirty
+    mamba2_post(y, xl, z, par[2], H, P, lay).backward(torch.ones_like(out))
+    assert torch.isfinite(xl.grad).all() and float(xl.grad[pad].abs().sum()) == 0
