@@ -117,7 +117,7 @@ def _rows_ok(x: torch.Tensor) -> bool:
 def silu_blocks_to_chunks(x: torch.Tensor, sizes, lay):
     """SiLU of the column blocks of ``x [T, sum(sizes)]`` (up to three) in the padded rows of ``lay`` (``chunked.ChunkLayout``), ``[Tp, n]`` each, zeros
     in the padding; None where the kernel does not apply."""
-    if not (_lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.shape[0] == lay.T and len(sizes) <= 3
+    if not (_lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and x.dim() == 2 and x.shape == (lay.T, sum(sizes)) and len(sizes) <= 3
             and all(n % 8 == 0 for n in sizes) and _rows_ok(x)):
         return None
     maps = (None, None) if lay.aligned else (lay.inv_i32, lay.rows_i32)

@@ -290,13 +290,18 @@ def mamba2_pre_skip(x, dt_raw, dt_bias, A_log, H: int, P: int, lay=None):
     """``mamba2_pre`` and x once more: the skip connection reads that, and x's two gradients meet in the backward kernel."""
     if mamba2_kernels(x, dt_raw, x, P):
         return _Mamba2Pre.apply(x, dt_raw, dt_bias, A_log, H, P, lay)
-    return (*mamba2_pre_reference(x, dt_raw, dt_bias, A_log, H, P), x)
+    if lay is None:
+        return (*mamba2_pre_reference(x, dt_raw, dt_bias, A_log, H, P), x)
+    out = mamba2_pre_reference(x.index_select(0, lay.rows), dt_raw, dt_bias, A_log, H, P)
+    return (*(lay.pack(t).flatten(0, 1) for t in out), x)
 
 
 def mamba2_post(y, x, z, D, H: int, P: int, lay=None):
     """``(y + D x) silu(z)`` as ``[T, H * P]`` in one kernel; ``x`` and ``z`` may be strided views."""
     if _lib.available() and P in (64, 128, 256) and _views_ok(x, z) and y.is_cuda and y.dtype == torch.bfloat16:
         return _Mamba2Post.apply(y, x, z, D, H, P, lay)
+    if lay is not None:
+        y, x = y.index_select(0, lay.rows), x.index_select(0, lay.rows)
     return mamba2_post_reference(y, x, z, D, H, P)
 
 

@@ -286,3 +286,28 @@ def test_only_the_gradients_that_are_asked_for_are_formed(dev, name, monkeypatch
     still = [n for n in named if n not in "qk"]
     got, work = run(still)
     assert work[0] < most[0] or name in _MOST
+
+
+@pytest.mark.parametrize("lens", [[64, 128], LENS])
+def test_mamba2_elementwise_reference_in_chunk_rows(lens):
+    """Where the kernels do not apply, operands in the padded rows of a layout give the same numbers as packed ones, zeros in the padding;
+    x's gradient too.  The same fp32 operations on the same rows: equal (the parameters' gradients are sums over the tokens: 1e-5)."""
+    from flame_b200.ops.gates import mamba2_post, mamba2_pre_skip
+    torch.manual_seed(0)
+    T, H, P, lay = sum(lens), 2, 4, ChunkLayout.of(_meta(lens), 64)
+    x0, y0, z0, dt0 = torch.randn(T, H * P), torch.randn(T, H, P), torch.randn(T, H * P), torch.randn(T, H)
+    par, res = [torch.randn(H) for _ in range(3)], []
+    for padded in (True, False):
+        f = (lambda t: lay.pack(t).flatten(0, 1).clone()) if padded else torch.clone
+        pick = (lambda t: t[lay.rows]) if padded else (lambda t: t)
+        x, y = f(x0).requires_grad_(True), f(y0).requires_grad_(True)
+        z, dt, bias, A, D = (t.clone().requires_grad_(True) for t in (z0, dt0, *par))
+        xv, dts, g, xs = mamba2_pre_skip(x, dt, bias, A, H, P, lay if padded else None)
+        out = mamba2_post(y, xs, z, D, H, P, lay if padded else None)
+        if padded:
+            assert xv.shape[0] == dts.shape[0] == g.shape[0] == lay.Tp
+            assert all(float(t[lay.inv_i32 < 0].abs().sum()) == 0 for t in (xv, dts, g))
+        total = (pick(xv) * x0.view(T, H, P)).sum() + (pick(g) * dt0).sum() + (out * z0).sum()
+        res.append([pick(xv), pick(dts), pick(g), out] + [pick(t) if i < 2 else t for i, t in enumerate(torch.autograd.grad(total, [x, y, z, dt, bias, A, D]))])
+    for a, b in zip(*res):
+        assert rel_err(a, b) < 1e-5

@@ -775,3 +775,11 @@ def test_mamba2_gradients_of_the_padding_are_zero(lens, add):
     del dirty
     mamba2_post(y, xl, z, par[2], H, P, lay).backward(torch.ones_like(out))
     assert torch.isfinite(xl.grad).all() and float(xl.grad[pad].abs().sum()) == 0
+
+
+@pytest.mark.parametrize("sizes,fits", [((8, 16), True), ((8,), False), ((16, 16), False)])
+def test_silu_blocks_are_all_of_the_columns(sizes, fits):
+    """Blocks that leave columns over (whose gradient nobody would write) or reach past them are not taken."""
+    from flame_b200.ops.activations import silu_blocks_to_chunks
+    from flame_b200.ops.chunked import ChunkLayout
+    assert (silu_blocks_to_chunks(_bf(70, 24), sizes, ChunkLayout.of(_meta([70]), 64)) is not None) == fits
