@@ -15,8 +15,9 @@
 // What bounds it is the chain of a tile: clock stamps give 7,500 cycles per 64 keys, of them 4,100 in the weight warps, which issue
 // a quarter of the time, the rest waits for products and hand-overs.  So two CTAs share an SM: 256
 // tensor-memory columns and 112 KB each.  That is why dV and dK are formed transposed, in ONE accumulator of 128 rows (64
-// of dV, 64 of dK) and 64 columns (keys): [dO | 0]^T P + [0 | Q]^T dS, the zeros a tile in shared memory between the two.  A
-// row of it is one channel of 64 keys, so 32 lanes hold 32 neighbouring floats of a key's gradient and add them
+// of dV, 64 of dK) and 64 columns (keys): [dO | 0]^T P + [0 | Q]^T dS, the zeros a tile in shared memory between the two.  (A
+// dS that is not finite would reach dV as 0 x dS; it is taken out of its tile, and dQ of its query and dK of its key become NaN.)  A
+// row of the accumulator is one channel of 64 keys, so 32 lanes hold 32 neighbouring floats of a key's gradient and add them
 // to global memory as they are (red.add, 128 bytes per instruction), without a staging tile.  S and dP of the next tile are
 // issued ahead of this tile's other products.  Eight rows of 4,096 tokens, 16 heads: 2.46 -> 2.02 ms (one CTA of
 // 128 x 128 tiles per SM).  The reference reaches the same sums with spin-locked adds
@@ -66,6 +67,23 @@ struct Smem {
 };
 
 constexpr int SB_THREADS = 320;
+
+// Takes the values that are not finite out of row r of a tile of dS: the accumulator shared by dV and dK forms 0 x dS in dV's rows, which
+// P and dO alone decide.  Their keys' dK (n of them belong to the document; `dst`: the first one's) becomes NaN here instead.  Whether
+// there was any.
+__device__ __noinline__ bool take_out_not_finite(uint8_t* sDS, int r, int n, float* dst, long long row) {
+  bool any = false;
+  for (int c = 0; c < BKV; ++c) {
+    uint16_t* v = reinterpret_cast<uint16_t*>(sDS + sw128_offset(r, c));
+    if ((*v & 0x7f80) != 0x7f80) continue;
+    *v = 0;
+    any = true;
+    float* k = dst + c * row;
+    if (c >= n || isnan(*reinterpret_cast<volatile float*>(k))) continue;  // (NaN stays NaN whatever is added)
+    for (int i = 0; i < DH; ++i) k[i] = __uint_as_float(0x7fc00000u);
+  }
+  return any;
+}
 
 template <bool DREM>
 __global__ void __launch_bounds__(SB_THREADS, 2)
@@ -205,7 +223,10 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const sb2 ndrem = sb_pk(-drem, -drem);
     float E = 1.f;  // product of (1 - sigma) over the keys already seen
     float R = 0.f;  // sum of dA over the keys already seen
-    bool ok = true;
+    // dS is made of tot, R and their differences, and a dA that is not finite stays in R: as long as this sum over every eighth R is far
+    // from overflow all of dS is finite (checked value by value it took 0.05 ms of 2.0)
+    float size = fabsf(tot);
+    bool ok = true, lost = false;  // lost: some dS of this row was not finite
     for (int it = 0; it < n_iter && ok; ++it) {
       const int kv0 = (n_iter - 1 - it) * BKV;
       const bool diag = kv0 + BKV > q0;
@@ -257,7 +278,10 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t off = sw128_offset(r, c);
         *reinterpret_cast<uint4*>(sP + off) = q;
         *reinterpret_cast<uint4*>(sDS + off) = make_uint4(sb_pack(d[0]), sb_pack(d[1]), sb_pack(d[2]), sb_pack(d[3]));
+        size += fabsf(R);
       }
+      if (!(size < 1e38f))
+        lost |= take_out_not_finite(sDS, r, doc_len - kv0, p.dK + (long long)(doc_start + kv0) * p.H * DH + head * DH, (long long)p.H * DH);
       tc_fence_before();
       fence_async_smem();
       mbar_arrive(pds_ready);
@@ -272,6 +296,10 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         uint32_t v[32];
         tmem_ld_32x32(tmem_dQ + lane_sel + half * 32, v);
         tmem_ld_wait();
+        if (lost) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] = 0x7fc00000u;
+        }
         if (valid) {
 #pragma unroll
           for (int g = 0; g < 4; ++g) {

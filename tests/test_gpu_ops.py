@@ -887,3 +887,27 @@ def test_attention_reads_the_work_list_by_its_own_name(kind, monkeypatch):
     got = call(other)
     got.sum().backward()
     assert torch.equal(got, want) and all(torch.isfinite(t.grad).all() for t in (q, k, v))
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan")])
+def test_stickbreaking_value_gradient_does_not_see_what_is_not_finite_elsewhere(bad):
+    """A value that is not finite spoils the gradients of queries and keys, but the values' gradient is the weights times dO alone:
+    as without it, up to the order in which fp32 partial sums are added, which turns the bf16 rounding (2^-8) of less than one entry in
+    ten: 1e-3, in that document and in the others."""
+    from flame_b200.ops.stickbreaking import sb_attention
+    torch.manual_seed(0)
+    lens, H = [300, 70, 129], 2
+    meta, T = _meta(lens), sum(lens)
+    q, k, v, do = (torch.randn(T, H, 64, device=DEV).bfloat16() for _ in range(4))
+    grads = []
+    for x in (None, bad):
+        args = [t.clone() for t in (q, k, v)]
+        if x is not None:
+            args[2][150, 0, 3] = x
+        args = [t.requires_grad_(True) for t in args]
+        grads.append(torch.autograd.grad(sb_attention(*args, meta)[0], args, do))
+    assert torch.isfinite(grads[1][2]).all() and rel_err(grads[1][2], grads[0][2]) < 1e-3
+    for clean, spoilt in zip(grads[0][:2], grads[1][:2]):
+        assert rel_err(spoilt[300:], clean[300:]) < 1e-3 and rel_err(spoilt[:, 1], clean[:, 1]) < 1e-3
+        assert torch.isfinite(spoilt[:128, 0]).all() if clean is grads[0][0] else True
+        assert not torch.isfinite(spoilt[:300, 0]).all()
