@@ -254,7 +254,7 @@ struct ConvArgs {
   ConvPart part[MAXPART];
   int parts, rows, per, D;  // rows to walk (padded ones included), tiles of a strip, all channels
   const int* src;           // [rows] packed row of a padded row (-1: padding); null: the rows themselves
-  const int* pos;           // [rows] offset in the document (NO_ROW: padding)
+  const int* pos;           // [T] offset of a packed row in its document
   float* partial;           // [blocks along y][D][W + 1]
   long long T;              // rows of x
   int* status;
@@ -334,9 +334,14 @@ struct ConvWalk {
     if (k - batch0 >= 32) load_batch(k);
     return __shfl_sync(0xffffffffu, batch, k - batch0);
   }
-  __device__ __forceinline__ int pos_of(int k) const {  // lane i: position of row i of the tile
-    const long long t = (long long)k * ROWS + lane;
-    return lane < ROWS && t < a.rows ? a.pos[t] : NO_ROW;
+  // lane i: position of the i-th packed row from s on.  A padded tile whose first row is s holds those that follow it in its document, which
+  // `in_tile` tells by the positions alone (and only when they are needed: it waits for them).
+  __device__ __forceinline__ int pos_of(int s) const {
+    const long long r = (long long)s + lane;
+    return s >= 0 && lane < ROWS && r < a.T ? a.pos[r] : NO_ROW;
+  }
+  __device__ __forceinline__ int in_tile(int p) const {
+    return a.src == nullptr || p == __shfl_sync(0xffffffffu, p, 0) + lane ? p : NO_ROW;
   }
   __device__ __forceinline__ void fetch(int k, int s) {  // row s of x (and the tile of g) into the ring
     if (k < k1 && s >= 0 && lane == 0) {
@@ -390,7 +395,7 @@ __global__ void __launch_bounds__(32 * WARPS, FOCC) conv4_fwd_kernel(const __gri
   }
   f2 wv[CW], bias, xv[CW];  // x of the last rows, [0] the newest
   load_taps2(p, d0, live, wv, bias);
-  int pos_l = w.pos_of(w.k0);
+  int pos_l = w.in_tile(w.pos_of(row[0]));
 #pragma unroll
   for (int j = 0; j < H3; ++j) {
     const bool in = live && row[0] - 1 - j >= 0;
@@ -399,7 +404,7 @@ __global__ void __launch_bounds__(32 * WARPS, FOCC) conv4_fwd_kernel(const __gri
   xv[H3] = 0ull;
   int stage = 0, phase = 0;
   for (int k = w.k0; k < w.k1; ++k) {
-    const int pos_next = w.pos_of(k + 1);
+    const int pos_next = w.pos_of(row[1]);
     const uint32_t* xs = &w.ring.data[stage][0][0][lane];
     __nv_bfloat16* out = p.out + (long long)k * FROWS * p.ldo + d0;
     const int src = row[0];
@@ -444,7 +449,7 @@ __global__ void __launch_bounds__(32 * WARPS, FOCC) conv4_fwd_kernel(const __gri
     for (int s = 0; s + 1 < FSTAGES; ++s) row[s] = row[s + 1];
     row[FSTAGES - 1] = w.row_of(k + FSTAGES);
     w.fetch(k + FSTAGES, row[FSTAGES - 1]);
-    pos_l = pos_next;
+    pos_l = w.in_tile(pos_next);
     stage = stage + 1 == FSTAGES ? 0 : stage + 1;
   }
 }
@@ -485,7 +490,7 @@ __global__ void __launch_bounds__(32 * WARPS, BOCC) conv4_bwd_kernel(const __gri
     load_taps2(p, d0, live, wv, bias);
 #pragma unroll
     for (int j = 0; j < CW; ++j) g[j] = 0ull, q[j] = NO_ROW;
-    int pos_l = w.pos_of(w.k0);
+    int pos_l = w.in_tile(w.pos_of(row[0]));
 #pragma unroll
     for (int j = 0; j < H3; ++j) {
       const bool in = live && row[0] - 1 - j >= 0;
@@ -533,7 +538,7 @@ __global__ void __launch_bounds__(32 * WARPS, BOCC) conv4_bwd_kernel(const __gri
     };
     int k = w.k0;
     for (; k < w.k1; ++k) {
-      const int pos_next = w.pos_of(k + 1);
+      const int pos_next = w.pos_of(row[1]);
       const uint32_t *xs = &w.ring.data[stage][0][0][lane], *gs = &w.ring.data[stage][1][0][lane];
       const int src = row[0];
       if (src >= 0 && !tc05::mbar_wait_warp(&w.full[stage], (phase >> stage) & 1, a.status, w.abort_flag, tc05::ERR_WAIT_FULL)) break;
@@ -578,7 +583,7 @@ __global__ void __launch_bounds__(32 * WARPS, BOCC) conv4_bwd_kernel(const __gri
       for (int s = 0; s + 1 < BSTAGES; ++s) row[s] = row[s + 1];
       row[BSTAGES - 1] = w.row_of(k + BSTAGES);
       w.fetch(k + BSTAGES, row[BSTAGES - 1]);
-      pos_l = pos_next;
+      pos_l = w.in_tile(pos_next);
       stage = stage + 1 == BSTAGES ? 0 : stage + 1;
     }
     if (k == w.k1) {  // the three rows behind the strip, for the gradients of its last three

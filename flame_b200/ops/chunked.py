@@ -34,7 +34,6 @@ from .bgemm import MASK_STRICT, MASK_TRIL, _mask, bgemm, bmm
 from .varlen import VarlenMeta
 
 CHUNK = 64
-NO_ROW = -(1 << 20)  # as in csrc/conv.cu
 _lib.register("fb_gather_rows", [c_void_p, c_void_p, c_void_p, c_longlong, c_longlong, c_longlong, c_longlong, c_void_p])
 _lib.register("fb_delta_scan", [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_int, c_void_p])
@@ -95,25 +94,14 @@ class ChunkLayout:
         last = first + nchunks - 1
         inv = np.full(self.Tp, -1, dtype=np.int32)
         inv[rows] = np.arange(self.T, dtype=np.int32)
-        self._first_np, self._nchunks_np, self._rows_np = first, nchunks, rows
-        self._positions = np.arange(self.T, dtype=np.int32) - np.repeat(starts, lens).astype(np.int32)
+        self._first_np, self._nchunks_np = first, nchunks
         self.rows = torch.from_numpy(rows).to(dev)                            # packed token -> padded row
         self.first = torch.from_numpy(first).to(dev)                          # first chunk of every document
         self.last = torch.from_numpy(last).to(dev)                            # last chunk of every document
         self.first_i32, self.last_i32 = self.first.to(torch.int32), self.last.to(torch.int32)
         self.rows_i32 = self.rows.to(torch.int32)
         self.inv_i32 = torch.from_numpy(inv).to(dev)                          # padded row -> packed token, -1 = padding
-        self._steps = self._pos = None
-
-    @property
-    def pos_i32(self) -> torch.Tensor:
-        """int32 ``[Tp]``: offset of every padded row inside its document, ``NO_ROW`` in the padding."""
-        if self._pos is None:
-            import numpy as np
-            pos = np.full(self.Tp, NO_ROW, dtype=np.int32)
-            pos[self._rows_np] = self._positions
-            self._pos = torch.from_numpy(pos).to(self.inv_i32.device)
-        return self._pos
+        self._steps = None
 
     def _build_steps(self) -> None:
         # chunks at in-document position s that have a successor, and the documents they belong to (only the

@@ -52,7 +52,7 @@ class _ShortConv4(torch.autograd.Function):
         ctx.slots = [slots.of(x) for x in xs]
         T = xs[0].shape[0]
         xs = [_rows16(x) for x in xs]
-        rows, src, pos = (T, None, meta.position_ids) if lay is None else (lay.Tp, lay.inv_i32, lay.pos_i32)
+        (rows, src), pos = (T, None) if lay is None else (lay.Tp, lay.inv_i32), meta.position_ids
         ys = [torch.empty(rows, x.shape[1], dtype=x.dtype, device=x.device) for x in xs]
         ws = [_lib.dense(w.detach()) for w in weights]
         bs = [_lib.dense(b.detach()) if b is not None else None for b in biases]

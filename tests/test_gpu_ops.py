@@ -911,3 +911,20 @@ def test_stickbreaking_value_gradient_does_not_see_what_is_not_finite_elsewhere(
         assert rel_err(spoilt[300:], clean[300:]) < 1e-3 and rel_err(spoilt[:, 1], clean[:, 1]) < 1e-3
         assert torch.isfinite(spoilt[:128, 0]).all() if clean is grads[0][0] else True
         assert not torch.isfinite(spoilt[:300, 0]).all()
+
+
+def test_short_convs_in_chunk_rows_copy_nothing_for_a_new_batch():
+    """The layout's maps are all that the host makes for a new batch: the positions of the padded rows come from those of the packed ones,
+    on the device, so with the layout there the convolutions wait for no copy."""
+    from flame_b200.ops.chunked import ChunkLayout
+    from flame_b200.ops.conv import short_convs_in_chunks
+    lens = [65, 1, 200]
+    x, w = torch.randn(sum(lens), 64, device=DEV).bfloat16(), torch.randn(64, 1, 4, device=DEV).bfloat16()
+    meta = _meta(lens)
+    ChunkLayout.of(meta, 64)
+    torch.cuda.synchronize()
+    torch.cuda.set_sync_debug_mode("error")
+    try:
+        assert short_convs_in_chunks((x,), (w,), (None,), meta, "silu", 64) is not None
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
