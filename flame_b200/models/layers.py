@@ -410,7 +410,7 @@ class GatedSlotAttention(nn.Module):
 
     def forward(self, x: torch.Tensor, meta: VarlenMeta) -> torch.Tensor:
         from ..ops.activations import silu_out_of_chunks
-        from ..ops.chunked import gsa_in_chunks
+        from ..ops.chunked import gsa_in_chunks, gsa_in_chunks_ok
         from ..ops.gla import gsa
         T, H, G, f = x.shape[0], self.num_heads, self.num_kv_groups, None
         layers, sizes = (self.q_proj, self.k_proj, self.v_proj), (self.key_dim, self.key_dim_per_group, self.value_dim_per_group)
@@ -419,13 +419,15 @@ class GatedSlotAttention(nn.Module):
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)
             q, k, v = _feature_map(self.feature_map, q), _feature_map(self.feature_map, k), F.silu(v)
         elif self.feature_map in ("swish", "silu") and side_by_side(layers, x):
-            # one activation over the three blocks as they lie: torch's kernels are several times slower on column blocks
-            if side_by_side((*layers, self.f_proj), x):
+            # one activation over the three blocks as they lie: torch's kernels are several times slower on column blocks (also on the three
+            # beside the slots' gates, so those join them only where the kernels read the blocks)
+            in_chunks = G == 1 and gsa_in_chunks_ok(self.num_slots, meta)
+            if in_chunks and side_by_side((*layers, self.f_proj), x):
                 n = sum(sizes)
                 qkv, f = split_columns(fused_projection(x, (*layers, self.f_proj)), (n, self.f_proj.weight.shape[0]))
             else:
                 qkv = fused_projection(x, layers)
-            if G == 1:
+            if in_chunks:
                 f = reshaped(self.f_proj(x) if f is None else f, T, H, self.num_slots)
                 o = gsa_in_chunks(qkv, sizes, H, f, self.gate_logit_normalizer, meta,
                                   self.scale if self.scale is not None else self.head_k_dim ** -0.5)

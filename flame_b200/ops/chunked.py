@@ -955,15 +955,19 @@ def _gsa_chunks(q, k, v, s, g, meta: VarlenMeta, scale: float) -> torch.Tensor:
     return lay.unpack(_gsa_padded.__wrapped__(qp, kp, vp, lay.pack(s), lay.pack(g.float()), lay, scale)).to(v.dtype)
 
 
+def gsa_in_chunks_ok(slots: int, meta: VarlenMeta) -> bool:
+    """Whether ``gsa_in_chunks`` takes bf16 operands with this many slots; asked before the projections are made."""
+    from . import chunk_kernels
+    return _lib.available() and slots <= chunk_kernels.VDECAY_SOFTMAX_MAX and slots % 8 == 0 and getattr(meta, "sequence_slice", None) is None
+
+
 def gsa_in_chunks(qkv, sizes, heads: int, f, normalizer: float, meta: VarlenMeta, scale: float):
     """Both passes on q, k, v = the SiLU of column blocks of ``qkv [T, sum(sizes)]`` and the slots' gates from their bf16 argument ``f [T, heads, M]``;
     activation and gates go into the chunk layout on the way.  The result, still in the rows of the layout, and the layout; None where
     the kernels do not apply."""
-    from . import chunk_kernels
     from .activations import silu_blocks_to_chunks
     from .gates import logsigmoid_gate
-    M = f.shape[-1]
-    if not (_lib.available() and qkv.is_cuda and M <= chunk_kernels.VDECAY_SOFTMAX_MAX and M % 8 == 0 and getattr(meta, "sequence_slice", None) is None):
+    if not (gsa_in_chunks_ok(f.shape[-1], meta) and qkv.is_cuda):
         return None
     lay = ChunkLayout.of(meta)
     qkv = silu_blocks_to_chunks(qkv, sizes, lay)

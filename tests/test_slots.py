@@ -363,3 +363,23 @@ def test_a_longer_low_rank_gate_runs_whole():
         m.gk_proj = Whole(m.gk_proj)
         torch.testing.assert_close(got, m(x, meta))
         m.gk_proj = m.gk_proj.seq
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kw", [dict(num_kv_heads=2), dict(num_slots=520)])
+def test_gsa_activations_see_whole_rows(kw, monkeypatch):
+    """Where the chunk kernels do not take GSA's projections (fewer key heads, more than 512 slots), torch's activation runs over a matrix of
+    its own, not over column blocks beside the slots' gates, on which it is several times slower."""
+    from flame_b200.models import layers as layers_mod
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    dev = torch.device("cuda", 0)
+    m = layers_mod.GatedSlotAttention(256, num_heads=4, **kw).to(dev).bfloat16()
+    for p in m.parameters():
+        torch.nn.init.normal_(p, std=0.05)
+    _adjacent([m.q_proj, m.k_proj, m.v_proj, m.f_proj])
+    seen, silu = [], torch.nn.functional.silu
+    monkeypatch.setattr(torch.nn.functional, "silu", lambda t, *a: (seen.append(t.is_contiguous()), silu(t, *a))[1])
+    x = torch.randn(131, 256, device=dev).bfloat16()
+    m(x, VarlenMeta.from_cu_seqlens(torch.tensor((0, 1, 66, 131), dtype=torch.int32, device=dev)))
+    assert seen and all(seen)
