@@ -172,10 +172,11 @@ class GatedLinearAttention(nn.Module):
             # (torch's activations are several times slower on column blocks)
             whole = self.use_short_conv or self.feature_map is None
             low = plain((self.gk_proj,), nn.Sequential) and len(self.gk_proj) == 2
-            more = ((self.g_proj,) if self.use_output_gate else ()) + ((self.gk_proj[0],) if low else ())
+            more = ((self.g_proj,) if self.fuse_norm_and_gate else ()) + ((self.gk_proj[0],) if low else ())
             q, k, v, *rest = _projections(x, layers, more) if whole else (l(x) for l in (*layers, *more))
             gk = self.gk_proj[1](rest[-1]) if low else self.gk_proj(x)
-            g_out = rest[0] if self.use_output_gate else None
+            if self.use_output_gate:
+                g_out = rest[0] if self.fuse_norm_and_gate else self.g_proj(x)
         T = q.shape[0]
         if self.use_short_conv:
             q, k, v = self.q_conv1d(q, meta), self.k_conv1d(k, meta), self.v_conv1d(v, meta)

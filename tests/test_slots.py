@@ -383,3 +383,21 @@ def test_gsa_activations_see_whole_rows(kw, monkeypatch):
     x = torch.randn(131, 256, device=dev).bfloat16()
     m(x, VarlenMeta.from_cu_seqlens(torch.tensor((0, 1, 66, 131), dtype=torch.int32, device=dev)))
     assert seen and all(seen)
+
+
+@pytest.mark.gpu
+def test_gla_output_gate_is_whole_where_torch_activates_it(monkeypatch):
+    """Without the fused norm, torch's activation runs over the output gate: over a matrix of its own, not a column block."""
+    from flame_b200.models import layers as layers_mod
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    dev = torch.device("cuda", 0)
+    m = layers_mod.GatedLinearAttention(256, num_heads=2, fuse_norm=False).to(dev).bfloat16()
+    for p in m.parameters():
+        torch.nn.init.normal_(p, std=0.05)
+    _adjacent([m.q_proj, m.k_proj, m.v_proj, m.g_proj, m.gk_proj[0]])
+    seen, silu = [], torch.nn.functional.silu
+    monkeypatch.setattr(torch.nn.functional, "silu", lambda t, *a: (seen.append(t.is_contiguous()), silu(t, *a))[1])
+    x = torch.randn(131, 256, device=dev).bfloat16()
+    m(x, VarlenMeta.from_cu_seqlens(torch.tensor((0, 1, 66, 131), dtype=torch.int32, device=dev)))
+    assert seen and all(seen)
