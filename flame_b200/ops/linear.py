@@ -125,8 +125,9 @@ class _LinearFn(torch.autograd.Function):
         x2, *weights = ctx.saved_tensors
         N = dy.shape[-1]
         dy2 = dy.reshape(-1, N)
-        if dy2.stride(-1) != 1 or dy2.stride(0) % 8 != 0:
-            dy2 = dy2.contiguous() if N % 8 == 0 or not dy2.is_cuda else _matrix(dy2.shape[0], N, dy2).copy_(dy2)
+        odd = N % 8 != 0 and dy2.is_cuda  # no contiguous matrix of this width is an operand
+        if dy2.stride(-1) != 1 or dy2.stride(0) % 8 != 0 or (odd and (dy2.stride(0) < N or dy2.data_ptr() % 16 != 0)):
+            dy2 = _matrix(dy2.shape[0], N, dy2).copy_(dy2) if odd else dy2.contiguous()
         K = x2.shape[1]
         dx = None
         if ctx.needs_input_grad[0]:

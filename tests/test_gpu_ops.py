@@ -928,3 +928,18 @@ def test_short_convs_in_chunk_rows_copy_nothing_for_a_new_batch():
         assert short_convs_in_chunks((x,), (w,), (None,), meta, "silu", 64) is not None
     finally:
         torch.cuda.set_sync_debug_mode("default")
+
+
+@pytest.mark.parametrize("form", ["block", "broadcast"])
+def test_side_by_side_projections_of_odd_sizes_take_any_gradient(form):
+    """The gradient of one product for projections of 64 + 6 + 6 rows as a block that starts between vectors of wider rows, and as one row for
+    all tokens: the same numbers as dense."""
+    from flame_b200.ops.linear import linear_fused, side_by_side
+    torch.manual_seed(0)
+    flat = torch.randn(76 * 128, device=DEV).bfloat16() * 0.1
+    ws = [torch.nn.Parameter(flat[a * 128:b * 128].view(b - a, 128)) for a, b in ((0, 64), (64, 70), (70, 76))]
+    x = torch.randn(300, 128, device=DEV).bfloat16().requires_grad_(True)
+    assert side_by_side(x, ws)
+    dy = torch.randn(300, 88, device=DEV).bfloat16()[:, 3:79] if form == "block" else torch.randn(76, device=DEV).bfloat16().expand(300, 76)
+    got, want = (torch.autograd.grad(linear_fused(x, ws), [x, *ws], d) for d in (dy, dy.contiguous()))
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
