@@ -283,12 +283,14 @@ __global__ void __launch_bounds__(DG_THREADS) delta_gates_bwd_kernel(
 }
 __global__ void delta_gates_sum_kernel(const float* __restrict__ part, int blocks, int H, float* __restrict__ dA, float* __restrict__ ddt, int accumulate) {
   const int i = blockIdx.x, lane = threadIdx.x;  // one warp per value
+  float* to = i < H ? dA : ddt;
+  if (to == nullptr) return;  // frozen
   float v = 0.f;
   for (int k = lane; k < blocks; k += 32) v += part[(long long)k * 2 * H + i];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if (lane != 0) return;
-  float* to = i < H ? dA + i : ddt + (i - H);
+  to += i < H ? i : i - H;
   *to = accumulate ? *to + v : v;
 }
 
@@ -455,7 +457,7 @@ int fb_delta_gates_fwd(const void* b, long long ldb, const void* a, long long ld
   kernel<<<grid, 256, 0, stream>>>((const __nv_bfloat16*)b, ldb, (const __nv_bfloat16*)a, lda, A_log, dt_bias, src, rows, H, mul, beta, g);
   return fb::launch_ok("delta_gates_fwd_kernel");
 }
-// part: fp32 [fb_delta_gates_blocks(rows, H), 2, H] scratch; dA, ddt: fp32 [H], added to with `accumulate`
+// part: fp32 [fb_delta_gates_blocks(rows, H), 2, H] scratch; dA, ddt: fp32 [H] (either may be null), added to with `accumulate`
 int fb_delta_gates_bwd(const void* b, long long ldb, const void* a, long long lda, const void* A_log, const void* dt_bias, int bf16, const int* src,
                        long long rows, int H, float mul, const float* dbeta, const float* dg, void* db, long long lddb, void* da, long long ldda,
                        float* part, float* dA, float* ddt, int accumulate, cudaStream_t stream) {

@@ -351,15 +351,16 @@ class _DeltaGates(torch.autograd.Function):
         L = _lib.lib()
         if a is not None:
             dg, da = dense(dg), out(a, ctx.slots[1])
-            main = all(getattr(p, "main_grad", None) is not None for p in ctx.params)
-            dA, ddt = (p.main_grad if main else torch.empty(H, dtype=torch.float32, device=dev) for p in ctx.params)
+            need = ctx.needs_input_grad[2:4]
+            main = all(getattr(p, "main_grad", None) is not None for p, n in zip(ctx.params, need) if n)
+            dA, ddt = (None if not n else p.main_grad if main else torch.empty(H, dtype=torch.float32, device=dev) for p, n in zip(ctx.params, need))
             part = torch.empty(L.fb_delta_gates_blocks(rows, H), 2, H, dtype=torch.float32, device=dev)
         rc = L.fb_delta_gates_bwd(*_DeltaGates._inputs(b, a, A_log, dt_bias), _lib.ptr(src), rows, H, mul, dbeta.data_ptr(), _lib.ptr(dg) if a is not None else 0,
                                   db.data_ptr(), db.stride(0), _lib.ptr(da), 0 if da is None else da.stride(0), _lib.ptr(part),
                                   _lib.ptr(dA), _lib.ptr(ddt), int(main), _lib.stream_ptr())
         _lib.check(rc, "fb_delta_gates_bwd")
         _lib.count_launch(1 if a is None else 2)
-        gA, gdt = (None, None) if a is None or main else (dA.to(A_log.dtype), ddt.to(dt_bias.dtype))
+        gA, gdt = (None if main or d is None else d.to(p.dtype) for d, p in ((dA, A_log), (ddt, dt_bias)))
         return db, da, gA, gdt, None, None
 
 

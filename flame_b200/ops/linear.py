@@ -149,7 +149,10 @@ class _LinearFn(torch.autograd.Function):
             dx = dx.view(ctx.shape)
         grads = [None] * len(weights)
         mgs = [getattr(w, "main_grad", None) for w in ctx.params]
-        if len(weights) > 1 and any(w.shape[0] % 8 for w in weights) and not (all(m is not None for m in mgs) and _adjacent(mgs)):
+        odd = len(weights) > 1 and any(w.shape[0] % 8 for w in weights)
+        if odd and not any(ctx.needs_input_grad[3:]):
+            pass  # frozen, as torch's own products of such sizes would leave them
+        elif odd and not (all(m is not None for m in mgs) and _adjacent(mgs)):
             # column blocks that start between vectors cannot be operands of their own
             whole = gemm_tn(dy2, x2, out_dtype=torch.float32)
             for i, (part, m) in enumerate(zip(whole.split([w.shape[0] for w in weights]), mgs)):

@@ -401,3 +401,36 @@ def test_gla_output_gate_is_whole_where_torch_activates_it(monkeypatch):
     x = torch.randn(131, 256, device=dev).bfloat16()
     m(x, VarlenMeta.from_cu_seqlens(torch.tensor((0, 1, 66, 131), dtype=torch.int32, device=dev)))
     assert seen and all(seen)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("frozen", [("A_log",), ("dt_bias",), ("A_log", "dt_bias"), ("q_proj", "k_proj", "v_proj", "a_proj", "b_proj")])
+def test_frozen_parameters_of_the_delta_rule_gates_collect_nothing(frozen):
+    """What is frozen keeps its gradient buffer as it is, although the kernels write the others' in place; those get what they get otherwise."""
+    from flame_b200.models import layers as layers_mod
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    dev, D, T = torch.device("cuda", 0), 256, 131
+    m = layers_mod.GatedDeltaNet(D, num_heads=2, head_dim=64).to(dev)
+    for n, p in m.named_parameters():
+        torch.nn.init.normal_(p, std=0.05) if p.dim() > 1 else torch.nn.init.uniform_(p, 0.5, 1.0)
+        if n not in ("A_log", "dt_bias"):
+            p.data = p.data.bfloat16()
+    _adjacent([m.q_proj, m.k_proj, m.v_proj, m.a_proj, m.b_proj])
+    for p in m.parameters():
+        p.main_grad = getattr(p, "main_grad", torch.zeros(p.shape, device=dev))
+    meta = VarlenMeta.from_cu_seqlens(torch.tensor((0, 1, 66, 131), dtype=torch.int32, device=dev))
+    x, dy = torch.randn(T, D, device=dev).bfloat16(), torch.randn(T, D, device=dev).bfloat16()
+    res = []
+    for freeze in (False, True):
+        for n, p in m.named_parameters():
+            p.main_grad.fill_(1.0)
+            p.grad = None
+            p.requires_grad_(not (freeze and n.split(".")[0] in frozen))
+        m(x.clone().requires_grad_(True), meta).backward(dy)
+        res.append({n: p.main_grad.clone() if p.grad is None else p.main_grad + p.grad for n, p in m.named_parameters()})
+    for n, p in m.named_parameters():
+        if p.requires_grad:
+            assert (res[0][n] - res[1][n]).abs().max() <= 1e-5 * res[0][n].abs().max(), n
+        else:
+            assert (res[1][n] == 1).all() and p.grad is None, n
