@@ -419,7 +419,8 @@ int fb_rmsnorm_bwd_parts(long long rows) {
 int fb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, const void* gate, void* y, void* res_out,
                    float* rstd, long long rows, int D, float eps, int gate_mode, const int* map, int heads, long long ldg, cudaStream_t stream) {
   if (rows == 0) return 0;
-  if (D % 8 || heads < 1 || rows % heads || ldg % 8 || (rows >= (1ll << 31) && (map || ldg))) return -2;
+  if (D % 8 || heads < 1 || rows % heads || ldg % 8 || (rows >= (1ll << 31) && (map || ldg)) || !fb::aligned(16, x, res_in, w, gate, y, res_out))
+    return -2;
   const Rows at{map, (unsigned)heads, ldg ? ldg : (long long)heads * D, 0};
   const int lpr = D <= 64 ? 8 : D <= 128 ? 16 : 32;  // lanes of a row, D <= 256
   const int per_block = D <= 256 ? WARPS * 32 / lpr * FR : WARPS;
@@ -458,7 +459,9 @@ int fb_rmsnorm_bwd_rows(const void* dy, const void* xin, const void* w, const fl
                         const void* dres, void* dx, void* dgate, float* dw_part, float* dw, long long rows, int D,
                         int gate_mode, int accumulate_dw, const int* map, int heads, long long ldg, long long lddg, cudaStream_t stream) {
   if (rows == 0) return 0;
-  if (D % 8 || heads < 1 || rows % heads || ldg % 8 || lddg % 8 || (rows >= (1ll << 31) && (map || ldg || lddg))) return -2;
+  if (D % 8 || heads < 1 || rows % heads || ldg % 8 || lddg % 8 || (rows >= (1ll << 31) && (map || ldg || lddg)) ||
+      !fb::aligned(16, dy, xin, w, gate, dres, dx, dgate))
+    return -2;
   const Rows at{map, (unsigned)heads, ldg ? ldg : (long long)heads * D, lddg ? lddg : (long long)heads * D};
   const int parts = fb_rmsnorm_bwd_parts(rows);
   const int rows_per_cta = (int)((rows + parts - 1) / parts);

@@ -47,7 +47,7 @@ def _gate_rows(gate: torch.Tensor, T: int, heads: int, D: int):
     ld = g.stride(0) if T > 1 else heads * D
     if ld >= heads * D and ld % 8 == 0 and g.data_ptr() % 16 == 0 and g.stride(2) == 1 and (heads == 1 or g.stride(1) == D):
         return g, ld
-    return g.contiguous(), heads * D
+    return _lib.dense(g), heads * D
 
 
 class _RMSNormFn(torch.autograd.Function):
@@ -57,15 +57,13 @@ class _RMSNormFn(torch.autograd.Function):
         comes back padded, with zeros."""
         shape = x.shape
         D = shape[-1]
-        x2 = x.reshape(-1, D)
-        x2 = x2 if x2.is_contiguous() else x2.contiguous()
+        x2 = _lib.dense(x.reshape(-1, D))
         heads = 1 if lay is None and gate is None or x.dim() < 3 else shape[-2]
         rows = x2.shape[0] if lay is None else lay.T * heads
         out_shape = shape if lay is None else (lay.T, *shape[1:])
         res2 = None
         if residual is not None:
-            res2 = residual.reshape(-1, D)
-            res2 = res2 if res2.is_contiguous() else res2.contiguous()
+            res2 = _lib.dense(residual.reshape(-1, D))
         g2, ldg, ctx.slot = None, 0, None
         if gate is not None:
             ctx.slot = slots.of(gate)
@@ -92,12 +90,10 @@ class _RMSNormFn(torch.autograd.Function):
         xin, weight, rstd, g2 = ctx.saved_tensors
         D, lay, heads = ctx.shape[-1], ctx.lay, ctx.heads
         rows = xin.shape[0]
-        dy2 = dy.reshape(-1, D)
-        dy2 = dy2 if dy2.is_contiguous() else dy2.contiguous()
+        dy2 = _lib.dense(dy.reshape(-1, D))
         dres2 = None
         if ctx.prenorm and dres_out is not None:
-            dres2 = dres_out.reshape(-1, D)
-            dres2 = dres2 if dres2.is_contiguous() else dres2.contiguous()
+            dres2 = _lib.dense(dres_out.reshape(-1, D))
         L = _lib.lib()
         dx = torch.empty_like(xin)
         dgate, ldg, lddg = None, 0, 0

@@ -943,3 +943,25 @@ def test_side_by_side_projections_of_odd_sizes_take_any_gradient(form):
     dy = torch.randn(300, 88, device=DEV).bfloat16()[:, 3:79] if form == "block" else torch.randn(76, device=DEV).bfloat16().expand(300, 76)
     got, want = (torch.autograd.grad(linear_fused(x, ws), [x, *ws], d) for d in (dy, dy.contiguous()))
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("offset", [1, 4])
+@pytest.mark.parametrize("form", ["plain", "residual", "gate"])
+def test_norm_operands_start_anywhere(form, offset):
+    """Contiguous operands (and the gradients that come back) that start between vectors are moved before a kernel loads them: bit for bit
+    the aligned call's results."""
+    from flame_b200.ops.norm import rms_norm, rms_norm_gated
+
+    def shifted(t):
+        return torch.empty(t.numel() + offset, dtype=t.dtype, device=DEV)[offset:].view(t.shape).copy_(t)
+    torch.manual_seed(offset)
+    x, other, dy, dr = (torch.randn(37, 3, 128, device=DEV).bfloat16() for _ in range(4))
+    w, res = torch.rand(128, device=DEV).bfloat16(), []
+    for move in (lambda t: t.clone(), shifted):
+        args = [move(t).requires_grad_(True) for t in ((x,) if form == "plain" else (x, other))]
+        if form == "gate":
+            ys = (rms_norm_gated(args[0], args[1], w),)
+        else:
+            ys = rms_norm(args[0], w, 1e-6, args[1], True) if form == "residual" else (rms_norm(args[0], w),)
+        res.append([*ys, *torch.autograd.grad(ys, args, [move(dy), move(dr)][:len(ys)])])
+    assert all(torch.equal(a, b) for a, b in zip(*res))
