@@ -153,18 +153,17 @@ def gla_scores(q, k, b, blk, scale: float, lay=None) -> torch.Tensor:
     return A
 
 
-def gla_bwd(q, k, b, dA, dkhat, dqbar, dqt, dk3, dalpha, scale: float, lay=None, raw=None, norm: float = 1.0, grads=(None, None)):
+def gla_bwd(q, k, b, dA, dkhat, dqbar, dqt, dk3, dalpha, scale: float, lay=None, raw=None, norm: float = 1.0, grads=(None, None, None)):
     """``dq, dk`` (bf16) and ``dg`` of a chunk (see ``csrc/chunk.cu: gla_bwd_kernel``): fp32, or with ``raw`` that of the gate's bf16 argument.
-    With ``lay`` q, k, ``raw`` and the gradients are packed tokens; ``grads``: where dq and dk belong ``[T, H, dk]``."""
+    With ``lay`` q, k, ``raw`` and the gradients are packed tokens; ``grads``: where dq, dk and dg belong ``[T, H, dk]``."""
     NC, _, H, dk = b.shape
     if lay is None:
         dq, dk_, dg = torch.empty_like(q), torch.empty_like(k), torch.empty_like(b)
         lds = [H * dk] * 6
     else:
         new = lambda dt: torch.empty(lay.T, H, dk, dtype=dt, device=q.device)  # noqa: E731
-        dq, dk_ = (new(torch.bfloat16) if t is None else t for t in grads)
-        dg = new(torch.float32 if raw is None else torch.bfloat16)
-        lds = [_token_ld(q), _token_ld(k), H * dk if raw is None else _token_ld(raw), _token_ld(dq), _token_ld(dk_), H * dk]
+        dq, dk_, dg = (new(torch.float32 if i == 2 and raw is None else torch.bfloat16) if t is None else t for i, t in enumerate(grads))
+        lds = [_token_ld(q), _token_ld(k), H * dk if raw is None else _token_ld(raw), *(_token_ld(t) for t in (dq, dk_, dg))]
     _lib.check(_lib.lib().fb_gla_bwd(q.data_ptr(), k.data_ptr(), b.data_ptr(), dA.data_ptr(), dkhat.data_ptr(), dqbar.data_ptr(),
                                      dqt.data_ptr(), dk3.data_ptr(), dalpha.data_ptr(), dq.data_ptr(), dk_.data_ptr(), dg.data_ptr(), _lib.ptr(raw),
                                      1.0 / float(norm), 0 if lay is None else lay.inv_i32.data_ptr(), *lds, NC, H, dk, float(scale), _lib.stream_ptr()),

@@ -779,7 +779,7 @@ class _Gla(torch.autograd.Function):
         dblk = dA.view(NC, H, 4, 16, 64)[:, :, 1:, :, :48].permute(0, 2, 1, 3, 4).reshape(NC * 3, H, 16, 48)
         dqt3 = bgemm(dblk, _hm(k3), b_mn=True, alpha=scale, out=_token_major(NC * 3, H, 16, dk, dt, dev))
         dk3 = bgemm(dblk, _hm(qt3), a_mn=True, b_mn=True, alpha=scale, out=_token_major(NC * 3, H, 48, dk, dt, dev))
-        grads = [None if s is None else s.take(lay.T, H * dk, dt, dev).view(lay.T, H, dk) for s in ctx.slots]
+        grads = [None if s is None else s.take(lay.T, H * dk, dt, dev).view(lay.T, H, dk) for s in (*ctx.slots, None)]
         dq, dkk, dg = chunk_kernels.gla_bwd(q, k, b, dA, back(dkhat), back(dqbar), back(dqt3), back(dk3), _pair_dot(Ln, S, per_row=True), scale,
                                             rows, raw, norm or 1.0, grads)
         return dq, dkk, back(dvv), dg, None, None, None, None

@@ -567,7 +567,7 @@ def test_contiguous_operands_at_any_storage_offset(name, offset):
 def test_gla_reads_and_writes_packed_tokens(dk, dv, H, lens):
     """q, k and the gate's argument read as column blocks of one matrix, their gradients written there, against the form with separate
     operands and the gate formed outside.  Both form the same fp32 gates and products; what may differ is a bf16 rounding of a
-    re-ordered sum: 5e-3.  The padding is never written: a canary behind the last token stays."""
+    re-ordered sum: 5e-3."""
     from flame_b200.ops.chunked import gla_raw_gate, gla_tc
     from flame_b200.ops.gates import logsigmoid_gate
     from flame_b200.ops.slots import reshaped, split_columns
@@ -783,3 +783,27 @@ def test_silu_blocks_are_all_of_the_columns(sizes, fits):
     from flame_b200.ops.activations import silu_blocks_to_chunks
     from flame_b200.ops.chunked import ChunkLayout
     assert (silu_blocks_to_chunks(_bf(70, 24), sizes, ChunkLayout.of(_meta([70]), 64)) is not None) == fits
+
+
+@pytest.mark.parametrize("raw", [False, True])
+@pytest.mark.parametrize("lens", [[1], [64, 128], [15, 17, 63, 65, 1, 200], [300, 16, 33]])
+def test_gla_backward_writes_its_tokens_alone(lens, raw):
+    """The three gradients as column blocks of wider matrices with a chunk's worth of rows behind the last token: the blocks hold what
+    matrices of their own do, and everything around them is what it was."""
+    from flame_b200.ops import chunk_kernels
+    from flame_b200.ops.chunked import ChunkLayout
+    torch.manual_seed(len(lens))
+    T, H, dk, lay = sum(lens), 2, 72, ChunkLayout.of(_meta(lens), 64)
+    NC, n = lay.NC, H * dk
+    q, k, g = _bf(T, H, dk), _bf(T, H, dk), _bf(T, H, dk, s=3.0)
+    b = chunk_kernels.gla_prep(q, k, g, 0.1, lay, 16.0)[0]
+    ins = (q, k, b, _bf(NC, H, 64, 64), _bf(NC, 64, H, dk), _bf(NC, 64, H, dk), _bf(NC * 3, 16, H, dk), _bf(NC * 3, 48, H, dk),
+           torch.randn(NC, H, dk, device=DEV))
+    want = chunk_kernels.gla_bwd(*ins, 0.1, lay, g if raw else None, 16.0)
+    store = [torch.full((T + 64, n + 16), 7.0, dtype=t.dtype, device=DEV) for t in want]
+    blocks = [s[:T, 8:8 + n].view(T, H, dk) for s in store]
+    chunk_kernels.gla_bwd(*ins, 0.1, lay, g if raw else None, 16.0, blocks)
+    for s, block, w in zip(store, blocks, want):
+        assert torch.equal(block, w)
+        block.fill_(7.0)
+        assert (s == 7.0).all()

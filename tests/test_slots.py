@@ -434,3 +434,80 @@ def test_frozen_parameters_of_the_delta_rule_gates_collect_nothing(frozen):
             assert (res[0][n] - res[1][n]).abs().max() <= 1e-5 * res[0][n].abs().max(), n
         else:
             assert (res[1][n] == 1).all() and p.grad is None, n
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name,kw,every,where", [
+    ("GatedLinearAttention", dict(num_heads=2), ("q_proj", "k_proj", "v_proj", "g_proj", "gk_proj.0"), "chunked.gla_raw_gate"),
+    ("GatedLinearAttention", dict(num_heads=3, use_output_gate=False), ("q_proj", "k_proj", "v_proj", "gk_proj.0"), "chunked.gla_raw_gate"),
+    ("GatedSlotAttention", dict(num_heads=3, num_slots=40), ("q_proj", "k_proj", "v_proj", "f_proj"), "chunked.gsa_in_chunks"),
+    ("DeltaNet", dict(num_heads=3), ("q_proj", "k_proj", "v_proj", "b_proj"), "delta_rule.conv_gated_delta_rule"),
+    ("DeltaNet", dict(num_heads=3, use_gate=True, allow_neg_eigval=True), ("q_proj", "k_proj", "v_proj", "b_proj"), "delta_rule.conv_gated_delta_rule"),
+    ("GatedDeltaNet", dict(num_heads=3, head_dim=64), ("q_proj", "k_proj", "v_proj", "a_proj", "b_proj"), "delta_rule.conv_gated_delta_rule"),
+    ("Mamba2", dict(num_heads=8, n_groups=2), ("in_proj",), "conv.short_convs_in_chunks"),
+])
+@pytest.mark.parametrize("cu", [(0, 128), (0, 1, 66, 131), (0, 200, 263, 264, 300)])
+def test_layer_forms_that_training_takes(name, kw, every, where, cu, monkeypatch):
+    """One product for ALL projections of a layer, its gradients in one buffer, and the convolutions, gates and norms in the chunk layout, as
+    the engine's flat parameters make a layer run, against each projection and convolution by itself on packed rows (weights apart, a hook
+    that does nothing on the convolutions and norms): bf16 roundings of the same sums, a few steps (2^-8) of the largest entry.  And once
+    more with everything saved for the backward going to the host and back: the same kernels on the same numbers (2^-8)."""
+    import importlib
+    from flame_b200.models import layers as layers_mod, modules
+    from flame_b200.ops.varlen import VarlenMeta
+    torch.manual_seed(0)
+    dev, D, T = torch.device("cuda", 0), 256 if name == "Mamba2" else 384, cu[-1]
+    one = getattr(layers_mod, name)(D, **kw)
+    for p in one.parameters():
+        torch.nn.init.normal_(p, std=0.05) if p.dim() > 1 else torch.nn.init.uniform_(p, 0.5, 1.0)
+    one = one.to(dev)
+    for n, p in one.named_parameters():
+        if n not in ("A_log", "dt_bias", "D"):
+            p.data = p.data.bfloat16()
+    two = copy.deepcopy(one)
+    for n, sub in one.named_modules():
+        if isinstance(sub, (modules.ShortConvolution, modules.RMSNorm, modules.RMSNormGated)):
+            sub.register_forward_hook(lambda *a: None)
+    for m, apart in ((one, True), (two, False)):
+        projections = [m.get_submodule(n) for n in every]
+        _adjacent(projections)
+        x = torch.randn(T, D, device=dev).bfloat16()
+        if apart:  # (the same values, each at a place of its own)
+            for l in projections:
+                l.weight.data, l.weight.main_grad = l.weight.data.clone(), l.weight.main_grad.clone()
+        assert modules.side_by_side(projections, x) == (not apart or len(every) == 1)
+        for p in m.parameters():
+            if not hasattr(p, "main_grad"):
+                p.main_grad = torch.zeros(p.shape, device=dev)
+    meta = VarlenMeta.from_cu_seqlens(torch.tensor(cu, dtype=torch.int32, device=dev))
+    dy = torch.randn(T, D, device=dev).bfloat16()
+    module, function = where.split(".")
+    module = importlib.import_module("flame_b200.ops." + module)
+    took, real = [], getattr(module, function)
+    monkeypatch.setattr(module, function, lambda *a, **k: (took.append(real(*a, **k)), took[-1])[1])
+
+    def run(m, save=None):
+        for p in m.parameters():
+            p.main_grad.zero_()
+            p.grad = None
+        xi = x.clone().requires_grad_(True)
+        if save is None:
+            y = m(xi, meta)
+        else:
+            with torch.autograd.graph.saved_tensors_hooks(*save):
+                y = m(xi, meta)
+        y.backward(dy)
+        return [y.detach(), xi.grad] + [p.main_grad.clone() if p.grad is None else p.main_grad + p.grad for p in m.parameters()]
+
+    want = run(one)
+    fused = name.startswith("Gated") and "Delta" not in name  # (GLA and GSA have no convolution to listen to: both sides may take the form)
+    assert fused or not any(t is not None for t in took)
+    took.clear()
+    got = run(two)
+    assert took and took[0] is not None
+    hooked = run(two, (lambda t: t.cpu(), lambda t: t.to(dev)))
+    names = ["y", "dx"] + [n for n, _ in two.named_parameters()]
+    for n, a, b, c in zip(names, got, want, hooked):
+        a, b, c = a.double(), b.double(), c.double()
+        assert (a - b).abs().max() <= 4 * 2.0 ** -8 * b.abs().max().clamp_min(1e-6), n
+        assert (a - c).abs().max() <= 2.0 ** -8 * a.abs().max().clamp_min(1e-6), n
