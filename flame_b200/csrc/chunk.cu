@@ -479,7 +479,7 @@ namespace {
 // tokens follow one another), ld* elements from row to row, or, src null, in the padded rows themselves.
 struct GlaRows {
   const int* src;
-  long long ldq, ldk, ldg;
+  long long ldq, ldk, ldg;  // (the scores read no gate)
 };
 // log(sigmoid(x)) / norm without cancellation or underflow (inv: 1 / norm): log(1 + e), e = exp(-|x|) <= 1, is 2 artanh(s), s = e / (2 + e), by the
 // artanh series up to s^13 for s <= 1/3 (off by 1.5e-8 relative at most).  Both quotients are corrected by their remainders, so that the
@@ -1159,9 +1159,11 @@ extern "C" int fb_state_scan(const long long* first, const long long* last, int 
 // Every exponent is <= 0.
 namespace {
 
-// Bound by memory (24 bytes per channel and row, 0.12 ms at 65,536 tokens, 4 heads of 128).  A thread owns two channels of one
+// Bound by memory: 20 bytes per channel and row with the gate's bf16 argument (6 in, 14 out: b 4, khat and qbar 2 each, qt 1.5, k3 4.5), 22
+// with the gate in fp32; 0.104 ms at 65,536 tokens, 4 heads of 128.  A thread owns two channels of one
 // 16-row sub-block and loads all it needs of q, k and g before it uses any; the sub-blocks' sums meet in shared memory.  A
-// thread that walked the 64 rows of a chunk waited for memory sub-block after sub-block and read b back: 0.205 ms; this takes 0.155, with the gate's own arithmetic (0.05 by a kernel before).
+// thread that walked the 64 rows of a chunk waited for memory sub-block after sub-block and read b back: 0.205 ms.  This takes 0.155, with the
+// gate's own arithmetic (0.05 by a kernel before; 0.146 with an exponent rounded to one float).
 template <bool RAW>
 __global__ void __launch_bounds__(256, 2) gla_prep_fwd_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ k,
                                                           const void* __restrict__ g, float norm, const GlaRows at, float* __restrict__ b,

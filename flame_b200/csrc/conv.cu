@@ -224,8 +224,9 @@ __global__ void conv_bwd_kernel(const __nv_bfloat16* __restrict__ dpre, const __
 
 // Width 4.  Both directions move each row once, so what should bound them is memory; what did was instructions (21 and 55 per
 // element, 0.078 and 0.158 ms at 65,536 x 1,024, 38 % and 29 % of the memory's rate).  So: a warp owns 64 channels of a strip
-// of rows, two channels per lane as packed fp32 pairs, and walks it with the last three rows in registers - nothing is computed
-// or read twice, also not dpre, which the gradient of a row needs from the three rows behind it (dx lags three rows).  The rows come
+// of rows, two channels per lane as packed fp32 pairs, and walks it with the last three rows in registers.  dpre, which the gradient of
+// a row needs from the three rows behind it, is formed once too: dx lags three rows.  Only the three rows in front of a strip are
+// read twice, and in the backward those behind it, with their dpre.  The rows come
 // by TMA (no address arithmetic), each warp through a ring of its own: there is no barrier in the walk.
 //
 // Rows may be taken in a padded order (`src`): the chunk layout of the linear-attention kernels, where every document starts on

@@ -788,7 +788,7 @@ __global__ void __launch_bounds__(256) gather_rows_kernel(const Vec* __restrict_
 // kernels on the way.  The backward is a row of x at a time: dx[r, block p] = dy_p[map[r]] silu'(x[r, block p]), zero where there is none.  Bound by
 // memory; torch's activation, and a gather per block and direction behind it, took 0.093 + 0.060 ms forward and 0.118 + 0.060 ms
 // backward at 32,767 x 3,072, this takes 0.083 and 0.106 (0.022 and 0.029 more for 1,024 columns out of
-// the layout).
+// the layout).  The exponential is the hardware's: no more bf16 results are off the nearest one than with torch's (expm1f instead: 0.159 and 0.230).
 struct SiluRows {
   const __nv_bfloat16* x;
   long long ldx, ldd;

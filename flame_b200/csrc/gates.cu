@@ -534,8 +534,8 @@ int fb_mamba2_post_bwd(const void* y, const void* x, long long ldx, const void* 
   return fb::launch_ok("mamba2_post_bwd_kernel");
 }
 
-// x, dx: bf16 [n]; g, s (optional), dg, ds (with s): fp32 [n]; n a multiple of 8, all 16-byte aligned
-// rows: of g (forward) or of x (backward), cols of each; map: see the kernels
+// x, dx: bf16, rows ldx / lddx elements apart; g, s (optional), dg, ds (with s): fp32, rows side by side; rows: of g (forward) or of x
+// (backward), cols of each; map: see the kernels.  cols, ldx and lddx multiples of 8, all 16-byte aligned.
 int fb_logsigmoid_gate_fwd(const void* x, long long ldx, const int* map, float* g, float* s, float normalizer, long long rows, long long cols,
                            cudaStream_t stream) {
   if (rows == 0 || cols == 0) return 0;
