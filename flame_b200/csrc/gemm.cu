@@ -539,6 +539,7 @@ extern "C" int fb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N
                              long long ldc, int a_mn, int b_mn, int out_mode, float alpha, int splits, void* workspace,
                              int sm_count, cudaStream_t stream);
 
+extern "C" long long fb_gemm2_cut_bytes(int M, int N, int K, int sm_count);
 extern "C" int fb_gemm2_allgather_a(const unsigned long long* shard_ptrs, int world, int rank, int rows_per_rank, long long ld,
                                     void* a_full, int* chunk_flags, const int* ready, int epoch, const void* B, void* C, int N,
                                     int K, long long ldb, long long ldc, int b_mn, int sm_count, cudaStream_t stream);
@@ -560,7 +561,11 @@ long long fb_gemm_workspace_bytes(int M, int N, int splits) {
   return splits > 1 ? (long long)splits * M * N * 4 : 0;
 }
 
-// Chooses a split-K factor with a small cost model: waves of work units times K blocks per unit, plus the
+// Bytes of workspace for splits == 0 of fb_gemm_bf16 without bias: 0 where none is needed, -1 where that form does not apply (single-CTA
+// kernel) and fb_gemm_pick_splits chooses.
+long long fb_gemm_cut_bytes(int M, int N, int K) { return g_variant == 2 ? fb_gemm2_cut_bytes(M, N, K, sm_count_cached()) : -1; }
+
+// For the single-CTA kernel: chooses a split-K factor with a small cost model: waves of work units times K blocks per unit, plus the
 // traffic of writing and re-reading the fp32 partials.  Few-tile, long-K GEMMs (weight gradients) gain most.
 int fb_gemm_pick_splits(int M, int N, int K) {
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + 255) / 256);
@@ -588,7 +593,8 @@ int fb_gemm_pick_splits(int M, int N, int K) {
 //  a_mn: 0 -> A stored [M, lda] (K contiguous); 1 -> A stored [K, lda] (M contiguous)
 //  b_mn: 0 -> B stored [N, ldb] (K contiguous); 1 -> B stored [K, ldb] (N contiguous)
 //  out_mode: 0 bf16 store, 1 fp32 store, 2 fp32 accumulate
-//  splits > 1 needs `workspace` of fb_gemm_workspace_bytes(); the partial sums are reduced in a fixed order.
+//  splits > 1 needs `workspace` of fb_gemm_workspace_bytes(); the partial sums are reduced in a fixed order.  splits == 0: the CTA
+//  pairs may cut the tiles of their last round along K, with `workspace` of fb_gemm_cut_bytes().
 // Returns 0 on success.
 int fb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
                  long long ldc, int a_mn, int b_mn, int out_mode, float alpha, const void* bias, int splits,
@@ -605,6 +611,8 @@ int fb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lon
   p.tiles_m = (M + BM - 1) / BM;
   p.tiles_n = (N + BN - 1) / BN;
   p.num_kb = (K + BK - 1) / BK;
+  if (splits == 0 && g_variant == 2 && bias == nullptr)
+    return fb_gemm2_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, out_mode, alpha, 0, workspace, sm_count_cached(), stream);
   if (splits < 1) splits = 1;
   if (splits > p.num_kb) splits = p.num_kb;
   p.kb_per_split = (p.num_kb + splits - 1) / splits;

@@ -66,8 +66,12 @@ struct Gemm2Params {
   int s_world;          // > 0: scatter mode, rows are stored into the owner rank's receive slot
   int s_rank, s_rows_per_rank;
   void* s_dst[16];
-  int tma_c = 0;        // bf16 results leave through shared memory and TMA (see the epilogue)
+  int tma_c = 0;        // results leave through shared memory and TMA (see the epilogue)
+  // the last cut_tiles tiles are cut along K into cut_pieces pieces of kb_per_piece K blocks (see Work)
+  int cut_tiles = 0, cut_pieces = 1, kb_per_piece = 0;
 };
+
+constexpr long long TILE_FLOATS = (long long)BM2 * BN;
 
 struct Smem2 {
   static constexpr int A_BYTES = BMH * BK * 2;
@@ -149,6 +153,37 @@ __device__ __forceinline__ void unit_to_tile(const Gemm2Params& p, int unit, int
     tm += p.m_rot;
     if (tm >= p.tiles_m) tm -= p.tiles_m;
   }
+}
+
+// The work of a pair, in order: whole tiles, then pieces of the tiles that are cut along K.
+// Whole tiles alone take ceil(tiles / pairs) rounds, and a last round that few of the pairs have work in costs as much as a
+// full one.  So its tiles are cut, all at the same K, and their pieces dealt out.  A piece goes to the workspace in fp32; a
+// kernel of all SMs adds a tile's pieces in the order of K.  Pieces of the same K run side by side, so that an operand row is
+// fetched once for all tiles.  What else was measured: ranges of K that start anywhere, dealt out evenly, have every pair at
+// another K and all of its operands from DRAM (3,072 x 1,024 x 65,536: 0.48 ms, 0.32 uncut); the sum by whoever brings the last
+// piece costs one SM 20 us and more.
+struct Work {
+  int tm, tn, kb0, kb1, split;
+  int tile, piece;            // of the cut tiles: number and piece; piece == -1: a whole tile
+};
+
+__device__ __forceinline__ bool get_work(const Gemm2Params& p, int unit, Work& w) {
+  const int whole = (p.tiles_m * p.tiles_n - p.cut_tiles) * p.splits;
+  if (unit < whole) {
+    w.piece = -1;
+    unit_to_tile(p, unit, w.tm, w.tn, w.split);
+    w.kb0 = w.split * p.kb_per_split;
+    w.kb1 = min(p.num_kb, w.kb0 + p.kb_per_split);
+    return true;
+  }
+  unit -= whole;
+  if (unit >= p.cut_tiles * p.cut_pieces) return false;
+  w.piece = unit / p.cut_tiles;
+  w.tile = unit - w.piece * p.cut_tiles;
+  unit_to_tile(p, whole + w.tile, w.tm, w.tn, w.split);
+  w.kb0 = w.piece * p.kb_per_piece;
+  w.kb1 = min(p.num_kb, w.kb0 + p.kb_per_piece);
+  return true;
 }
 
 __device__ __forceinline__ int ld_acquire_gpu2(const int* addr) {
@@ -345,7 +380,7 @@ __device__ void gather_flat_role2(const Gemm2Params& p, uint8_t* smem, uint64_t*
 template <bool A_MN, bool B_MN, bool FP8>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
-                  const __grid_constant__ Gemm2Params p) {
+                  const __grid_constant__ CUtensorMap tmP, const __grid_constant__ Gemm2Params p) {
   using L = Smem2;
   static_assert(!FP8 || (!A_MN && !B_MN), "fp8 operands are K-major");
   constexpr int BKE = FP8 ? 2 * BK : BK;  // elements of K per stage
@@ -367,8 +402,6 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const uint32_t rank = cluster_ctarank();
   const bool leader = rank == 0;
   const int pair = ((int)blockIdx.x - p.g_ncopy) >> 1, npairs = ((int)gridDim.x - p.g_ncopy) >> 1;
-  const int total_units = p.tiles_m * p.tiles_n * p.splits;
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&full_bar[s], 2);
@@ -383,6 +416,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
     if (p.tma_c) tma_prefetch_desc(&tmC);
+    if (p.cut_tiles) tma_prefetch_desc(&tmP);
   }
   if (warp == 1) {
     tmem_alloc2(tmem_slot, 512);
@@ -400,11 +434,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       uint32_t phase = 0;
       bool ok = true;
       int b_waited_tn = -1;  // flat gather mode: the tile column whose B chunks were already awaited
-      for (int unit = pair; unit < total_units && ok; unit += npairs) {
-        int tm, tn, split;
-        unit_to_tile(p, unit, tm, tn, split);
-        const int kb0 = split * p.kb_per_split;
-        const int kb1 = min(p.num_kb, kb0 + p.kb_per_split);
+      Work w;
+      for (int unit = pair; ok && get_work(p, unit, w); unit += npairs) {
+        const int tm = w.tm, tn = w.tn, kb0 = w.kb0, kb1 = w.kb1;
         if (p.g_ncopy > 0 && p.g_mode == 1) {
           // this CTA's half of the B tile comes out of the gathered flat buffer: K-major B = 128 consecutive rows of the
           // weight (one byte range); MN-major B touches every row, so the whole weight must have landed
@@ -465,11 +497,9 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      for (int unit = pair; unit < total_units && ok; unit += npairs, ++it) {
-        int tm, tn, split;
-        unit_to_tile(p, unit, tm, tn, split);
-        const int kb0 = split * p.kb_per_split;
-        const int kb1 = min(p.num_kb, kb0 + p.kb_per_split);
+      Work w;
+      for (int unit = pair; ok && get_work(p, unit, w); unit += npairs, ++it) {
+        const int kb0 = w.kb0, kb1 = w.kb1;
         const int acc = it & 1;
         if (!mbar_wait(&tempty_bar[acc], ((it >> 1) & 1) ^ 1, p.status, abort_flag, ERR_WAIT_TMEM_EMPTY)) { ok = false; break; }
         tc_fence_after();
@@ -506,20 +536,26 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (p.alpha_a) alpha *= __ldg(p.alpha_a);
       if (p.alpha_b) alpha *= __ldg(p.alpha_b);
     }
-    for (int unit = pair; unit < total_units && ok; unit += npairs, ++it) {
-      int tm, tn, split;
-      unit_to_tile(p, unit, tm, tn, split);
+    Work w;
+    for (int unit = pair; ok && get_work(p, unit, w); unit += npairs, ++it) {
+      const int tm = w.tm, tn = w.tn, split = w.split;
       const int acc = it & 1;
       if (!mbar_wait_warp(&tfull_bar[acc], (it >> 1) & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
       const int row = tm * BM2 + (int)rank * BMH + quarter * 32 + lane;
       const bool row_ok = row < p.M;
       const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
+      const bool piece = w.piece >= 0;
       if (p.tma_c) {
-        // A box of 32 rows x 64 columns per TMA store.  As 16-byte stores to a row per thread a tile took the load/store
-        // unit 8,000 clocks (64 per instruction: 32 rows), as long as its products at K = 1024.  Two projections of
+        // A box of 32 rows x 64 bf16 (or 32 fp32) columns per TMA store.  As 16-byte stores to a row per thread a tile took the
+        // load/store unit 8,000 clocks (64 per instruction: 32 rows), as long as its products at K = 1024.  Two projections of
         // 65,536 x 1,024, forward: 0.405 -> 0.373 ms; gate, up and down: 0.907 -> 0.848; vocabulary: 0.618 -> 0.552.
-        const int row0 = tm * BM2 + (int)rank * BMH + quarter * 32;
+        // Accumulating fp32 results are added in L2 (one addition per element, so in no order).
+        const int row_in = (int)rank * BMH + quarter * 32, row0 = tm * BM2 + row_in;
+        const int epi = piece ? 1 : p.epi;
+        const CUtensorMap* map = piece ? &tmP : &tmC;
+        // pieces lie below one another, 256 columns wide
+        const int out_row = piece ? (w.piece * p.cut_tiles + w.tile) * BM2 + row_in : row0, out_col = piece ? 0 : tn * BN;
 #pragma unroll 1
         for (int c = 0; c < BN; c += 64) {
           const int col0 = tn * BN + c;
@@ -534,24 +570,49 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             if (lane == 0) remote_arrive(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
           }
           if (row0 < p.M) {
-            uint8_t* box = boxes + (n_box & 1) * L::BOX_BYTES;
-            ++n_box;
-            if (lane == 0) tma_store_wait_read<1>();  // the store before last has left this box
-            __syncwarp();
+            if (epi == 0) {
+              uint8_t* box = boxes + (n_box & 1) * L::BOX_BYTES;
+              ++n_box;
+              if (lane == 0) tma_store_wait_read<1>();  // the store before last has left this box
+              __syncwarp();
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              uint4 q;
-              uint32_t* w = reinterpret_cast<uint32_t*>(&q);
+              for (int j = 0; j < 8; ++j) {
+                uint4 q;
+                uint32_t* o = reinterpret_cast<uint32_t*>(&q);
 #pragma unroll
-              for (int e = 0; e < 4; ++e)
-                w[e] = pack_bf16(__uint_as_float(r[8 * j + 2 * e]) * alpha, __uint_as_float(r[8 * j + 2 * e + 1]) * alpha);
-              *reinterpret_cast<uint4*>(box + lane * 128 + ((j ^ (lane & 7)) << 4)) = q;
-            }
-            fence_async_smem();
-            __syncwarp();
-            if (lane == 0) {
-              tma_store_2d(&tmC, box, col0, row0);
-              tma_store_commit();
+                for (int e = 0; e < 4; ++e)
+                  o[e] = pack_bf16(__uint_as_float(r[8 * j + 2 * e]) * alpha, __uint_as_float(r[8 * j + 2 * e + 1]) * alpha);
+                *reinterpret_cast<uint4*>(box + lane * 128 + ((j ^ (lane & 7)) << 4)) = q;
+              }
+              fence_async_smem();
+              __syncwarp();
+              if (lane == 0) {
+                tma_store_2d(&tmC, box, col0, row0);
+                tma_store_commit();
+              }
+            } else {
+#pragma unroll
+              for (int h = 0; h < 2; ++h) {
+                if (col0 + h * 32 >= p.N) break;
+                uint8_t* box = boxes + (n_box & 1) * L::BOX_BYTES;
+                ++n_box;
+                if (lane == 0) tma_store_wait_read<1>();
+                __syncwarp();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  const uint32_t* o = &r[h * 32 + 4 * j];
+                  *reinterpret_cast<float4*>(box + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                      make_float4(__uint_as_float(o[0]) * alpha, __uint_as_float(o[1]) * alpha, __uint_as_float(o[2]) * alpha,
+                                  __uint_as_float(o[3]) * alpha);
+                }
+                fence_async_smem();
+                __syncwarp();
+                if (lane == 0) {
+                  if (epi == 2) tma_reduce_add_2d(map, box, out_col + c + h * 32, out_row);
+                  else tma_store_2d(map, box, out_col + c + h * 32, out_row);
+                  tma_store_commit();
+                }
+              }
             }
           }
           if (last) break;
@@ -663,13 +724,111 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   }
 }
 
+// CTA pairs that can be resident at once (a GPC with an odd number of free SMs strands one); the same for every form of the
+// kernel, as each takes a whole SM
+int max_pairs(int sm_count) {
+  static int pairs = 0;
+  if (pairs == 0) {
+    auto kern = gemm2_bf16_kernel<false, false, false>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((sm_count / 2) * 2);
+    cfg.blockDim = dim3(192);
+    cfg.dynamicSmemBytes = Smem2::TOTAL;
+    int n = 0;
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem2::TOTAL);
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = sm_count / 2;
+    }
+    pairs = n < sm_count / 2 ? n : sm_count / 2;
+  }
+  return pairs;
+}
+
+// Tiles of the last round to be cut along K, and into how many pieces; 0 tiles where that does not pay.  In microseconds: a
+// round costs 0.3 per K block (256 x 256 x 64) with a few pairs at work, 0.4 with all; a piece 0.12 for writing and reading its
+// 256 KB, the second kernel 5.  One round of pieces is not always the best: 48 tiles on 74 pairs cut in three take two rounds of
+// a third.  At most three pieces per pair bound the workspace.
+int cut_last_round(long long tiles, int num_kb, int pairs, int* pieces) {
+  const int rest = (int)(tiles % pairs);
+  *pieces = 1;
+  if (rest == 0) return 0;
+  double best = num_kb * (0.3 + 0.1 * rest / pairs);
+  for (int s = 2; s <= 16 && s * rest <= 3 * pairs && s * 4 <= num_kb; ++s) {
+    const int kb = (num_kb + s - 1) / s, units = s * rest, rounds = (units + pairs - 1) / pairs;
+    if ((s - 1) * kb >= num_kb) continue;  // the last piece would be empty
+    const double cost = rounds * kb * (0.3 + 0.1 * (rounds > 1 ? 1.0 : (double)units / pairs)) + 5.0 + 0.12 * units;
+    if (cost < best * 0.97) {
+      best = cost;
+      *pieces = s;
+    }
+  }
+  return *pieces > 1 ? rest : 0;
+}
+
+// Rows of tiles that share a sweep over N.  Weight matrices that do not fit L2 beside the rest want many rows per sweep, as each
+// sweep fetches them again, as long as the rows themselves fit (12,289 x 32,000 x 1,024: 8 rows 602 us, 16 586, 32 576).  Where a
+// sweep is short and its rows are long, few rows: a round of tiles then ends near the end of a sweep, and the next does not
+// fetch long rows again (16,384 x 2,048 x 7,000: 8 rows 340 us, 4 333, 2 328; 65,536 x 1,024 x 3,072 the other way, 285 and 289).
+int sweep_rows(int tiles_n, int N, int K) {
+  if (tiles_n <= 8) return K >= 4096 ? 2 : 8;
+  if ((long long)N * K * 2 <= 24ll << 20) return 8;
+  const long long fit = (24ll << 20) / ((long long)BM2 * K * 2);
+  return fit < 8 ? 8 : fit > 32 ? 32 : (int)fit;
+}
+
+// Adds the pieces of the cut tiles in the order of K: a thread four columns of a row, a block four rows.
+__global__ void __launch_bounds__(256) gemm2_add_pieces_kernel(const float* __restrict__ part, Gemm2Params p) {
+  const int tile = blockIdx.x >> 6, row = (blockIdx.x & 63) * 4 + (threadIdx.x >> 6), col = (threadIdx.x & 63) * 4;
+  int tm, tn, split;
+  unit_to_tile(p, p.tiles_m * p.tiles_n - p.cut_tiles + tile, tm, tn, split);
+  const int r = tm * BM2 + row, c = tn * BN + col;
+  if (r >= p.M || c >= p.N) return;
+  const float4* q = reinterpret_cast<const float4*>(part + tile * TILE_FLOATS + row * BN + col);
+  const long long step = p.cut_tiles * (TILE_FLOATS / 4);
+  float4 v = __ldcs(q);
+#pragma unroll 4
+  for (int i = 1; i < p.cut_pieces; ++i) {
+    const float4 o = __ldcs(q + i * step);
+    v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
+  }
+  const float e[4] = {v.x, v.y, v.z, v.w};
+  const bool whole = c + 4 <= p.N;
+  if (p.epi == 0) {
+    __nv_bfloat16* d = (__nv_bfloat16*)p.C + r * p.ldc + c;
+    if (whole && ((uintptr_t)d & 7) == 0) {
+      *reinterpret_cast<uint2*>(d) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+    } else {
+      for (int i = 0; i < 4 && c + i < p.N; ++i) d[i] = __float2bfloat16(e[i]);
+    }
+  } else {
+    float* d = (float*)p.C + r * p.ldc + c;
+    const bool add = p.epi == 2;
+    if (whole && ((uintptr_t)d & 15) == 0) {
+      if (add) {
+        const float4 o = *reinterpret_cast<const float4*>(d);
+        v.x += o.x, v.y += o.y, v.z += o.z, v.w += o.w;
+      }
+      *reinterpret_cast<float4*>(d) = v;
+    } else {
+      for (int i = 0; i < 4 && c + i < p.N; ++i) d[i] = add ? d[i] + e[i] : e[i];
+    }
+  }
+}
+
 template <bool A_MN, bool B_MN, bool FP8 = false>
-int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, int sm_count, cudaStream_t stream) {
-  CUtensorMap tmC = tmA;
-  if (p.epi == 0 && p.s_world == 0 && p.swiglu_I == 0 && (p.ldc & 7) == 0 && p.ldc >= p.N && !((uintptr_t)p.C & 15)) {
-    const int rc = fb::make_tmap_2d(&tmC, p.C, 2, p.M, p.N, p.ldc, 32, 64, true);
+int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, int sm_count, cudaStream_t stream, float* part = nullptr) {
+  CUtensorMap tmC = tmA, tmP = tmA;
+  const int c_bytes = p.epi == 0 ? 2 : 4;
+  if (p.s_world == 0 && p.swiglu_I == 0 && p.splits == 1 && (p.ldc * c_bytes & 15) == 0 && p.ldc >= p.N && !((uintptr_t)p.C & 15)) {
+    const int rc = fb::make_tmap_2d(&tmC, p.C, c_bytes, p.M, p.N, p.ldc, 32, 128 / c_bytes, true);
     if (rc) return rc;
     p.tma_c = 1;
+  }
+  if (!p.tma_c) p.cut_tiles = 0;
+  if (p.cut_tiles) {
+    const int rc = fb::make_tmap_2d(&tmP, part, 4, (uint64_t)p.cut_tiles * p.cut_pieces * BM2, BN, BN, 32, 32, true);
+    if (rc) return rc;
   }
   auto kern = gemm2_bf16_kernel<A_MN, B_MN, FP8>;
   static bool configured = false;
@@ -678,33 +837,31 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, int 
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  // CTA pairs that can be resident at once (a GPC with an odd number of free SMs strands one)
-  static int max_pairs = 0;
-  if (max_pairs == 0) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((sm_count / 2) * 2);
-    cfg.blockDim = dim3(192);
-    cfg.dynamicSmemBytes = Smem2::TOTAL;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = sm_count / 2;
-    }
-    max_pairs = n < sm_count / 2 ? n : sm_count / 2;
-  }
-  int units = p.tiles_m * p.tiles_n * p.splits;
-  int avail = max_pairs - p.g_ncopy / 2;  // the copy pairs of the gather mode occupy SMs of their own
+  const int units = p.tiles_m * p.tiles_n * p.splits;
+  int avail = max_pairs(sm_count) - p.g_ncopy / 2;  // the copy pairs of the gather mode occupy SMs of their own
   if (avail < 1) avail = 1;
-  int pairs = units < avail ? units : avail;
-  kern<<<pairs * 2 + p.g_ncopy, 192, Smem2::TOTAL, stream>>>(tmA, tmB, tmC, p);
-  return fb::launch_ok(FP8 ? "gemm2_fp8_kernel" : "gemm2_bf16_kernel");
+  const int pairs = units < avail && p.cut_tiles == 0 ? units : avail;
+  kern<<<pairs * 2 + p.g_ncopy, 192, Smem2::TOTAL, stream>>>(tmA, tmB, tmC, tmP, p);
+  const int rc = fb::launch_ok(FP8 ? "gemm2_fp8_kernel" : "gemm2_bf16_kernel");
+  if (rc || !p.cut_tiles) return rc;
+  gemm2_add_pieces_kernel<<<p.cut_tiles * 64, 256, 0, stream>>>(part, p);
+  return fb::launch_ok("gemm2_add_pieces_kernel");
 }
 
 }  // namespace
 
 extern "C" {
 
-// Same contract as fb_gemm_bf16 without bias; splits > 1 writes fp32 partials [splits, M, N] into `workspace`
+// Bytes of workspace with which fb_gemm2_bf16 cuts the tiles of its last round along K; 0 where it would not.
+long long fb_gemm2_cut_bytes(int M, int N, int K, int sm_count) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  int pieces;
+  const long long cut = cut_last_round((long long)((M + BM2 - 1) / BM2) * ((N + BN - 1) / BN), (K + BK - 1) / BK, max_pairs(sm_count), &pieces);
+  return cut * pieces * TILE_FLOATS * 4;
+}
+
+// Same contract as fb_gemm_bf16 without bias; splits == 0: the last round may be cut, `workspace` (or null) as
+// fb_gemm2_cut_bytes says; splits > 1 writes fp32 partials [splits, M, N] into `workspace`
 // (the caller reduces them with the split-K reduction of gemm.cu).  Returns 0 on success.
 int fb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb, long long ldc,
                   int a_mn, int b_mn, int out_mode, float alpha, int splits, void* workspace, int sm_count,
@@ -716,13 +873,17 @@ int fb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
   p.tiles_m = (M + BM2 - 1) / BM2;
   p.tiles_n = (N + BN - 1) / BN;
   p.num_kb = (K + BK - 1) / BK;
+  if (splits == 0 && workspace != nullptr) {
+    p.cut_tiles = cut_last_round((long long)p.tiles_m * p.tiles_n, p.num_kb, max_pairs(sm_count), &p.cut_pieces);
+    p.kb_per_piece = (p.num_kb + p.cut_pieces - 1) / p.cut_pieces;
+  }
   if (splits < 1) splits = 1;
   if (splits > p.num_kb) splits = p.num_kb;
   p.kb_per_split = (p.num_kb + splits - 1) / splits;
   p.splits = (p.num_kb + p.kb_per_split - 1) / p.kb_per_split;
   p.alpha = alpha;
   p.alpha_a = nullptr; p.alpha_b = nullptr; p.fp8_formats = 0;
-  p.group_m = 8;
+  p.group_m = sweep_rows(p.tiles_n, N, K);
   p.status = fb::status_ptr();
   p.m_rot = 0; p.g_ncopy = 0; p.g_mode = 0; p.s_world = 0; p.swiglu_I = 0;
   if (p.splits > 1) {
@@ -739,10 +900,11 @@ int fb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
   if (!b_mn) rc = fb::make_tmap_2d(&tmB, B, 2, N, K, ldb, BNH, BK, true);
   else       rc = fb::make_tmap_2d(&tmB, B, 2, K, N, ldb, BK, 64, true);
   if (rc) return rc;
-  if (!a_mn && !b_mn) return launch2<false, false>(tmA, tmB, p, sm_count, stream);
-  if (!a_mn && b_mn)  return launch2<false, true>(tmA, tmB, p, sm_count, stream);
-  if (a_mn && !b_mn)  return launch2<true, false>(tmA, tmB, p, sm_count, stream);
-  return launch2<true, true>(tmA, tmB, p, sm_count, stream);
+  float* part = (float*)workspace;
+  if (!a_mn && !b_mn) return launch2<false, false>(tmA, tmB, p, sm_count, stream, part);
+  if (!a_mn && b_mn)  return launch2<false, true>(tmA, tmB, p, sm_count, stream, part);
+  if (a_mn && !b_mn)  return launch2<true, false>(tmA, tmB, p, sm_count, stream, part);
+  return launch2<true, true>(tmA, tmB, p, sm_count, stream, part);
 }
 
 

@@ -158,6 +158,8 @@ def _declare(L: ctypes.CDLL) -> None:
         fn.restype = c_int
     L.fb_gemm_workspace_bytes.argtypes = [i, i, i]
     L.fb_gemm_workspace_bytes.restype = c_longlong
+    L.fb_gemm_cut_bytes.argtypes = [i, i, i]
+    L.fb_gemm_cut_bytes.restype = c_longlong
     for name, args, res in _EXTRA_SIGS:
         fn = getattr(L, name, None)
         if fn is not None:

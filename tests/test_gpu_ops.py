@@ -54,6 +54,37 @@ def test_gemm_split_k_and_accumulate():
     assert torch.equal(o1, o2)
 
 
+@pytest.mark.parametrize("M,N,K", [(136, 72, 5000), (1000, 520, 9000), (256, 256, 2048), (2040, 2312, 8200), (5640, 1024, 4096)])
+def test_gemm_tiles_cut_along_k(M, N, K):
+    """Tiles of the last round in pieces of K: few tiles and many, ragged in every dimension, all output forms, also where the result's rows
+    or start rule out tensor copies (then nothing is cut).  fp32 results: the accumulator takes 16 products a step and cuts off below its last place, on average half
+    of it, always in the same direction: K / 16 steps of 2^-24.  bf16 results: 2^-8."""
+    from flame_b200.ops import _lib, gemm
+    if (M, N) != (5640, 1024):
+        assert _lib.lib().fb_gemm_cut_bytes(M, N, K) > 0
+    tol = K / 16 * 2 ** -24
+    torch.manual_seed(2)
+    at = torch.randn(K, M, device=DEV, dtype=torch.bfloat16)
+    bt = torch.randn(K, N, device=DEV, dtype=torch.bfloat16)
+    a, b = at.t().contiguous(), bt.t().contiguous()
+    ref = a.float() @ b.float().t()
+    for fn, x, y in ((gemm.gemm_nt, a, b), (gemm.gemm_nn, a, bt), (gemm.gemm_tn, at, bt)):
+        assert rel_err(fn(x, y), ref) < 2 ** -8
+        out = fn(x, y, out_dtype=torch.float32)
+        assert rel_err(out, ref) < tol
+        assert torch.equal(out, fn(x, y, out_dtype=torch.float32))
+        assert rel_err(fn(x, y, out_dtype=torch.float32, alpha=0.5), 0.5 * ref) < tol
+        wide = torch.ones(M, N + 9, device=DEV)
+        for lo, hi in ((4, 4 + N), (1, 1 + N)):     # rows of 4 (N + 9) bytes: no tensor copies
+            fn(x, y, out=wide[:, lo:hi], accumulate=True)
+        assert rel_err(wide[:, 5:N], (ref[:, 1:N - 4] + 1) + ref[:, 4:N - 1]) < tol
+        assert torch.equal(wide[:, [0, N + 5]], torch.ones(M, 2, device=DEV))
+        wide = torch.ones(M, N + 8, device=DEV)     # a column block
+        fn(x, y, out=wide[:, 4:4 + N], accumulate=True)
+        assert rel_err(wide[:, 4:4 + N], ref + 1) < tol
+        assert torch.equal(wide[:, [0, 3, N + 4, N + 7]], torch.ones(M, 4, device=DEV))
+
+
 @pytest.mark.parametrize("lens,H,Hkv,Dh,window", [([128], 1, 1, 64, 0), ([300, 77, 129], 2, 1, 64, 0),
                                                    ([1000, 24, 512], 4, 4, 64, 0), ([640], 2, 2, 64, 200),
                                                    ([300, 200], 2, 1, 128, 0), ([300, 200], 2, 2, 128, 100),
