@@ -61,8 +61,6 @@ struct Gemm2Params {
   // 128 up rows, so the 256 accumulator columns of a row are gate_j | up_j for the same 128 hidden indices j, and the
   // epilogue writes gate and up (kept for the backward pass) and z = silu(gate) * up in one go
   int swiglu_I;
-  __nv_bfloat16* Z;
-  long long ldz;
   int s_world;          // > 0: scatter mode, rows are stored into the owner rank's receive slot
   int s_rank, s_rows_per_rank;
   void* s_dst[16];
@@ -73,15 +71,19 @@ struct Gemm2Params {
 
 constexpr long long TILE_FLOATS = (long long)BM2 * BN;
 
+template <int NSTAGES, int NBOXES>
 struct Smem2 {
   static constexpr int A_BYTES = BMH * BK * 2;
   static constexpr int B_BYTES = BNH * BK * 2;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;  // 32 KB
-  static constexpr int STG_OFFSET = STAGES * STAGE_BYTES;
-  static constexpr int BOX_BYTES = 32 * 128;             // 32 rows x 64 bf16, two per epilogue warp
-  static constexpr int BAR_OFFSET = STG_OFFSET + 4 * 2 * BOX_BYTES;
+  static constexpr int STG_OFFSET = NSTAGES * STAGE_BYTES;
+  static constexpr int BOX_BYTES = 32 * 128;             // 32 rows x 64 bf16 or 32 fp32, NBOXES per epilogue warp
+  static constexpr int BAR_OFFSET = STG_OFFSET + 4 * NBOXES * BOX_BYTES;
   static constexpr int TOTAL = BAR_OFFSET + 256 + 1024;
+  static_assert(TOTAL <= 227 * 1024, "shared memory of a block");
 };
+typedef Smem2<STAGES, 2> SmemPlain;
+typedef Smem2<STAGES - 1, 4> SmemSwigluBwd;  // eight epilogue warps with two boxes each
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
   uint32_t r;
@@ -240,7 +242,7 @@ __device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uin
 
 __device__ void gather_copy_role2(const Gemm2Params& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag) {
   constexpr int NSLOT = STAGES;
-  constexpr uint32_t SLOT = Smem2::STAGE_BYTES;  // 32 KB
+  constexpr uint32_t SLOT = SmemPlain::STAGE_BYTES;  // 32 KB
   if (threadIdx.x != 0) return;
   for (int s = 0; s < NSLOT; ++s) mbar_init(&bars[s], 1);
   *abort_flag = 0;
@@ -324,7 +326,7 @@ __device__ void gather_copy_role2(const Gemm2Params& p, uint8_t* smem, uint64_t*
 // here waits for another GPU: the launch is ordered after a bounded wait for the peers' "parameters written" flags.
 __device__ void gather_flat_role2(const Gemm2Params& p, uint8_t* smem, uint64_t* bars, volatile int* abort_flag) {
   constexpr int NSLOT = STAGES;
-  constexpr long long SLOT = Smem2::STAGE_BYTES;  // 32 KB
+  constexpr long long SLOT = SmemPlain::STAGE_BYTES;  // 32 KB
   if (threadIdx.x != 0) return;
   for (int s = 0; s < NSLOT; ++s) mbar_init(&bars[s], 1);
   *abort_flag = 0;
@@ -377,23 +379,28 @@ __device__ void gather_flat_role2(const Gemm2Params& p, uint8_t* smem, uint64_t*
 }
 
 // FP8: both operands are K-major 8-bit floats; a stage still holds 128-byte rows, i.e. 128 elements of K instead of 64.
-template <bool A_MN, bool B_MN, bool FP8>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(192, 1)
+// SWB: the accumulator is the gradient dz of z = silu(gate) * up, and what leaves are the gradients of gate and up (tmC: both,
+// side by side; tmP: gate and up themselves).
+template <bool A_MN, bool B_MN, bool FP8, bool SWB>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SWB ? 320 : 192, 1)
 gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmC,
                   const __grid_constant__ CUtensorMap tmP, const __grid_constant__ Gemm2Params p) {
-  using L = Smem2;
+  constexpr int NST = SWB ? STAGES - 1 : STAGES;
+  constexpr int EPI_WARPS = SWB ? 8 : 4;
+  using L = Smem2<NST, SWB ? 4 : 2>;
   static_assert(!FP8 || (!A_MN && !B_MN), "fp8 operands are K-major");
   constexpr int BKE = FP8 ? 2 * BK : BK;  // elements of K per stage
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full_bar = (uint64_t*)(smem + L::BAR_OFFSET);
-  uint64_t* empty_bar = full_bar + STAGES;
-  uint64_t* tfull_bar = empty_bar + STAGES;
+  uint64_t* empty_bar = full_bar + NST;
+  uint64_t* tfull_bar = empty_bar + NST;
   uint64_t* tempty_bar = tfull_bar + 2;
-  uint32_t* tmem_slot = (uint32_t*)(tempty_bar + 2);
+  uint64_t* box_bar = tempty_bar + 2;  // SWB: one per epilogue warp
+  uint32_t* tmem_slot = (uint32_t*)(box_bar + (SWB ? EPI_WARPS : 0));
   volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
 
-  if (p.g_ncopy > 0 && (int)blockIdx.x < p.g_ncopy) {  // whole CTA pairs take this branch: nobody waits for them
+  if (!SWB && p.g_ncopy > 0 && (int)blockIdx.x < p.g_ncopy) {  // whole CTA pairs take this branch: nobody waits for them
     if (p.g_mode == 1) gather_flat_role2(p, smem, full_bar, abort_flag);
     else gather_copy_role2(p, smem, full_bar, abort_flag);
     return;
@@ -403,20 +410,23 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   const bool leader = rank == 0;
   const int pair = ((int)blockIdx.x - p.g_ncopy) >> 1, npairs = ((int)gridDim.x - p.g_ncopy) >> 1;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < NST; ++s) {
       mbar_init(&full_bar[s], 2);
       mbar_init(&empty_bar[s], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&tfull_bar[a], 1);
-      mbar_init(&tempty_bar[a], 8);
+      mbar_init(&tempty_bar[a], 2 * EPI_WARPS);
+    }
+    if (SWB) {
+      for (int b = 0; b < EPI_WARPS; ++b) mbar_init(&box_bar[b], 1);
     }
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmA);
     tma_prefetch_desc(&tmB);
     if (p.tma_c) tma_prefetch_desc(&tmC);
-    if (p.cut_tiles) tma_prefetch_desc(&tmP);
+    if (p.cut_tiles || p.swiglu_I || SWB) tma_prefetch_desc(&tmP);
   }
   if (warp == 1) {
     tmem_alloc2(tmem_slot, 512);
@@ -437,7 +447,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       Work w;
       for (int unit = pair; ok && get_work(p, unit, w); unit += npairs) {
         const int tm = w.tm, tn = w.tn, kb0 = w.kb0, kb1 = w.kb1;
-        if (p.g_ncopy > 0 && p.g_mode == 1) {
+        if (!SWB && p.g_ncopy > 0 && p.g_mode == 1) {
           // this CTA's half of the B tile comes out of the gathered flat buffer: K-major B = 128 consecutive rows of the
           // weight (one byte range); MN-major B touches every row, so the whole weight must have landed
           if (B_MN ? (b_waited_tn < 0) : (b_waited_tn != tn)) {
@@ -456,7 +466,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             asm volatile("fence.proxy.async.global;" ::: "memory");
             b_waited_tn = tn;
           }
-        } else if (p.g_ncopy > 0) {
+        } else if (!SWB && p.g_ncopy > 0) {
           // this CTA's 128 rows of A come from one gathered chunk: wait until the copy CTAs published it, then order
           // their generic-proxy writes before the TMA reads of the async proxy
           if (!wait_flag2<false>(p.g_flags + (tm * BM2 + (int)rank * BMH) / p.g_chunk_rows, p.g_epoch, p.status, p.g_wait_ns + kWaitLimitNs)) *abort_flag = 1;
@@ -482,7 +492,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 #pragma unroll
             for (int g = 0; g < BNH / 64; ++g) tma_load_2d_pair(sB + g * (64 * BK * 2), &tmB, lead_full, n0 + g * 64, kb * BK);
           }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (++stage == NST) { stage = 0; phase ^= 1; }
         }
       }
     }
@@ -521,7 +531,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
                       (kb > kb0 || k > 0) ? 1u : 0u);
           }
           mma2_commit_both(&empty_bar[stage]);
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+          if (++stage == NST) { stage = 0; phase ^= 1; }
         }
         if (ok) mma2_commit_both(&tfull_bar[acc]);
       }
@@ -529,15 +539,110 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   } else {
     const int quarter = warp & 3;
     int it = 0, n_box = 0;
-    uint8_t* boxes = smem + L::STG_OFFSET + quarter * 2 * L::BOX_BYTES;
+    uint8_t* boxes = smem + L::STG_OFFSET + (SWB ? warp - 2 : quarter) * 2 * L::BOX_BYTES;
     bool ok = true;
     float alpha = p.alpha;
     if (FP8) {
       if (p.alpha_a) alpha *= __ldg(p.alpha_a);
       if (p.alpha_b) alpha *= __ldg(p.alpha_b);
     }
+    if constexpr (SWB) {
+      // Eight warps, two for each 32 rows, 64 hidden columns a step: gate and up come as two boxes by TMA, as soon as the gradients
+      // of the step before have left these boxes; while one warp of a scheduler waits for its boxes the other one works.  What
+      // bounds it is the memory traffic (1.5 GB at 65,536 x 2,816 x 1,024) that competes with the operands' loads: without its loads
+      // and stores the kernel takes 289 us instead of 395, without its arithmetic 400.  Product and a pass of its own: 507.  Four
+      // warps with one pair of boxes and a stage more 452, with two pairs 414, with three and a stage less 403; at 16,384 x 5,632 x
+      // 2,048, where the operands count for more, 315, 321 and 335 against 344 here and 366 unfused.
+      const int I = p.N, half = (warp - 2) >> 2;
+      constexpr int BW = BN / (EPI_WARPS / 4);  // columns of a tile that are a warp's
+      uint8_t *gbox = boxes, *ubox = boxes + L::BOX_BYTES;
+      uint64_t* bar = &box_bar[warp - 2];
+      Work w, nw;
+      int nunit = pair, nc = half * BW, step = 0, fetched = 0;
+      bool more = get_work(p, nunit, nw);
+      auto skip = [&]() {  // to this warp's next step inside the matrix
+        while (more && (nc >= (half + 1) * BW || nw.tn * BN + nc >= I)) {
+          nc = half * BW;
+          nunit += npairs;
+          more = get_work(p, nunit, nw);
+        }
+      };
+      auto fetch = [&]() {
+        if (!more) return;
+        ++fetched;
+        if (lane == 0) {
+          const int row0 = nw.tm * BM2 + (int)rank * BMH + quarter * 32, col0 = nw.tn * BN + nc;
+          tma_store_wait_read<0>();
+          mbar_expect_tx(bar, 2 * L::BOX_BYTES);
+          tma_load_2d(gbox, &tmP, bar, col0, row0);
+          tma_load_2d(ubox, &tmP, bar, I + col0, row0);
+        }
+        nc += 64;
+        skip();
+      };
+      skip();
+      fetch();
+      for (int unit = pair; ok && get_work(p, unit, w); unit += npairs, ++it) {
+        const int acc = it & 1;
+        if (!mbar_wait_warp(&tfull_bar[acc], (it >> 1) & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+        tc_fence_after();
+        const int row0 = w.tm * BM2 + (int)rank * BMH + quarter * 32;
+        const uint32_t t_row = tmem_base + acc * BN + ((uint32_t)(quarter * 32) << 16);
+        const int c1 = min((half + 1) * BW, I - w.tn * BN);
+        if (c1 <= half * BW) {  // the matrix ends before this half of the tile
+          __syncwarp();
+          if (lane == 0) remote_arrive(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+        }
+#pragma unroll 1
+        for (int c = half * BW; c < c1; c += 64, ++step) {
+          const int col0 = w.tn * BN + c;
+          uint32_t r[64];
+          tmem_ld_32x32(t_row + c, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+          tmem_ld_32x32(t_row + c + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+          tmem_ld_wait();
+          if (c + 64 >= c1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) remote_arrive(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+          }
+          if (!mbar_wait_warp(bar, step & 1, p.status, abort_flag, ERR_WAIT_FULL)) { ok = false; break; }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int at = lane * 128 + ((j ^ (lane & 7)) << 4);
+            uint4 gq = *reinterpret_cast<const uint4*>(gbox + at), uq = *reinterpret_cast<const uint4*>(ubox + at);
+            uint32_t *wg = reinterpret_cast<uint32_t*>(&gq), *wu = reinterpret_cast<uint32_t*>(&uq);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wg[e]));
+              const float2 u = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wu[e]));
+              // rounded as the product alone would store it, so that both forms give the same gradients
+              const uint32_t dq = pack_bf16(__uint_as_float(r[8 * j + 2 * e]), __uint_as_float(r[8 * j + 2 * e + 1]));
+              const float2 d = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&dq));
+              const float s0 = 1.f / (1.f + __expf(-g.x)), s1 = 1.f / (1.f + __expf(-g.y));
+              wg[e] = pack_bf16(d.x * u.x * s0 * (1.f + g.x * (1.f - s0)), d.y * u.y * s1 * (1.f + g.y * (1.f - s1)));
+              wu[e] = pack_bf16(d.x * g.x * s0, d.y * g.y * s1);
+            }
+            *reinterpret_cast<uint4*>(gbox + at) = gq;
+            *reinterpret_cast<uint4*>(ubox + at) = uq;
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) {
+            if (row0 < p.M) {
+              tma_store_2d(&tmC, gbox, col0, row0);
+              tma_store_2d(&tmC, ubox, I + col0, row0);
+            }
+            tma_store_commit();
+          }
+          fetch();
+        }
+      }
+      // after a failed wait: nothing may land in this shared memory once it belongs to another block
+      for (; !ok && lane == 0 && step < fetched; ++step)
+        for (int tries = 0; tries < 50000 && !mbar_try_wait(bar, step & 1); ++tries) {}
+    }
     Work w;
-    for (int unit = pair; ok && get_work(p, unit, w); unit += npairs, ++it) {
+    for (int unit = pair; !SWB && ok && get_work(p, unit, w); unit += npairs, ++it) {
       const int tm = w.tm, tn = w.tn, split = w.split;
       const int acc = it & 1;
       if (!mbar_wait_warp(&tfull_bar[acc], (it >> 1) & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
@@ -620,40 +725,54 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         continue;
       }
       if (p.swiglu_I > 0) {
-        __nv_bfloat16* grow = (__nv_bfloat16*)p.C + (long long)row * p.ldc + tn * BNH;
-        __nv_bfloat16* urow = grow + p.swiglu_I;
-        __nv_bfloat16* zrow = p.Z + (long long)row * p.ldz + tn * BNH;
+        // three boxes per 64 hidden columns: gate, up (tmC) and z (tmP)
+        const int row0 = tm * BM2 + (int)rank * BMH + quarter * 32;
 #pragma unroll 1
-        for (int c = 0; c < BNH; c += 32) {
-          uint32_t g[32], u[32];
-          tmem_ld_32x32(t_row + c, g);
-          tmem_ld_32x32(t_row + BNH + c, u);
+        for (int c = 0; c < BNH; c += 64) {
+          const int col0 = tn * BNH + c;
+          uint32_t r[128];
+#pragma unroll
+          for (int h = 0; h < 4; ++h) tmem_ld_32x32(t_row + (h >> 1) * BNH + c + (h & 1) * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[h * 32]));
           tmem_ld_wait();
-          if (!row_ok) continue;
+          if (c + 64 >= BNH) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) remote_arrive(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
+          }
+          if (row0 >= p.M) continue;
+          // the activation is taken on the bf16 values that are stored, so a backward pass that re-reads gate and up sees
+          // exactly the operands of z
 #pragma unroll
-          for (int j = 0; j < 32; j += 8) {
-            uint4 qg, qu, qz;
-            uint32_t* wg = reinterpret_cast<uint32_t*>(&qg);
-            uint32_t* wu = reinterpret_cast<uint32_t*>(&qu);
-            uint32_t* wz = reinterpret_cast<uint32_t*>(&qz);
+          for (int j = 0; j < 32; ++j) {
+            r[j] = pack_bf16(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+            r[64 + j] = pack_bf16(__uint_as_float(r[64 + 2 * j]), __uint_as_float(r[64 + 2 * j + 1]));
+          }
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              // the activation is taken on the bf16 values that are stored, so a backward pass that re-reads gate and up
-              // sees exactly the operands of z
-              wg[e] = pack_bf16(__uint_as_float(g[j + 2 * e]), __uint_as_float(g[j + 2 * e + 1]));
-              wu[e] = pack_bf16(__uint_as_float(u[j + 2 * e]), __uint_as_float(u[j + 2 * e + 1]));
-              const float2 gf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wg[e]));
-              const float2 uf = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wu[e]));
-              wz[e] = pack_bf16(gf.x / (1.f + __expf(-gf.x)) * uf.x, gf.y / (1.f + __expf(-gf.y)) * uf.y);
+          for (int b = 0; b < 3; ++b) {
+            uint8_t* box = boxes + (n_box & 1) * L::BOX_BYTES;
+            ++n_box;
+            if (b == 2) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                const float2 g = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r[j]));
+                const float2 u = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&r[64 + j]));
+                r[j] = pack_bf16(g.x / (1.f + __expf(-g.x)) * u.x, g.y / (1.f + __expf(-g.y)) * u.y);
+              }
             }
-            *reinterpret_cast<uint4*>(grow + c + j) = qg;
-            *reinterpret_cast<uint4*>(urow + c + j) = qu;
-            *reinterpret_cast<uint4*>(zrow + c + j) = qz;
+            if (lane == 0) tma_store_wait_read<1>();
+            __syncwarp();
+            const uint32_t* o = b == 1 ? r + 64 : r;
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              *reinterpret_cast<uint4*>(box + lane * 128 + ((j ^ (lane & 7)) << 4)) = make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+            fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              tma_store_2d(b == 2 ? &tmP : &tmC, box, b == 1 ? p.swiglu_I + col0 : col0, row0);
+              tma_store_commit();
+            }
           }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) remote_arrive(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
         continue;
       }
 #pragma unroll 1
@@ -712,7 +831,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       __syncwarp();
       if (lane == 0) remote_arrive(map_to_cta(smem_u32(&tempty_bar[acc]), 0));
     }
-    if (p.tma_c && lane == 0) tma_store_wait_all<0>();
+    if ((p.tma_c || p.swiglu_I || SWB) && lane == 0) tma_store_wait_all<0>();
   }
 
   tc_fence_before();
@@ -729,13 +848,13 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 int max_pairs(int sm_count) {
   static int pairs = 0;
   if (pairs == 0) {
-    auto kern = gemm2_bf16_kernel<false, false, false>;
+    auto kern = gemm2_bf16_kernel<false, false, false, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((sm_count / 2) * 2);
     cfg.blockDim = dim3(192);
-    cfg.dynamicSmemBytes = Smem2::TOTAL;
+    cfg.dynamicSmemBytes = SmemPlain::TOTAL;
     int n = 0;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem2::TOTAL);
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SmemPlain::TOTAL);
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
       cudaGetLastError();
       n = sm_count / 2;
@@ -816,6 +935,25 @@ __global__ void __launch_bounds__(256) gemm2_add_pieces_kernel(const float* __re
   }
 }
 
+template <bool A_MN, bool B_MN, bool FP8, bool SWB>
+int start2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tmC, const CUtensorMap& tmP, const Gemm2Params& p, int sm_count,
+           cudaStream_t stream) {
+  constexpr int SMEM = SWB ? SmemSwigluBwd::TOTAL : SmemPlain::TOTAL;
+  auto kern = gemm2_bf16_kernel<A_MN, B_MN, FP8, SWB>;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured = true;
+  }
+  const int units = p.tiles_m * p.tiles_n * p.splits;
+  int avail = max_pairs(sm_count) - p.g_ncopy / 2;  // the copy pairs of the gather mode occupy SMs of their own
+  if (avail < 1) avail = 1;
+  const int pairs = units < avail && p.cut_tiles == 0 ? units : avail;
+  kern<<<pairs * 2 + p.g_ncopy, SWB ? 320 : 192, SMEM, stream>>>(tmA, tmB, tmC, tmP, p);
+  return fb::launch_ok(FP8 ? "gemm2_fp8_kernel" : "gemm2_bf16_kernel");
+}
+
 template <bool A_MN, bool B_MN, bool FP8 = false>
 int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, int sm_count, cudaStream_t stream, float* part = nullptr) {
   CUtensorMap tmC = tmA, tmP = tmA;
@@ -830,19 +968,7 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, int 
     const int rc = fb::make_tmap_2d(&tmP, part, 4, (uint64_t)p.cut_tiles * p.cut_pieces * BM2, BN, BN, 32, 32, true);
     if (rc) return rc;
   }
-  auto kern = gemm2_bf16_kernel<A_MN, B_MN, FP8>;
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem2::TOTAL);
-    if (e != cudaSuccess) return (int)e;
-    configured = true;
-  }
-  const int units = p.tiles_m * p.tiles_n * p.splits;
-  int avail = max_pairs(sm_count) - p.g_ncopy / 2;  // the copy pairs of the gather mode occupy SMs of their own
-  if (avail < 1) avail = 1;
-  const int pairs = units < avail && p.cut_tiles == 0 ? units : avail;
-  kern<<<pairs * 2 + p.g_ncopy, 192, Smem2::TOTAL, stream>>>(tmA, tmB, tmC, tmP, p);
-  const int rc = fb::launch_ok(FP8 ? "gemm2_fp8_kernel" : "gemm2_bf16_kernel");
+  const int rc = start2<A_MN, B_MN, FP8, false>(tmA, tmB, tmC, tmP, p, sm_count, stream);
   if (rc || !p.cut_tiles) return rc;
   gemm2_add_pieces_kernel<<<p.cut_tiles * 64, 256, 0, stream>>>(part, p);
   return fb::launch_ok("gemm2_add_pieces_kernel");
@@ -945,7 +1071,7 @@ int fb_gemm2_allgather_a(const unsigned long long* shard_ptrs, int world, int ra
                          long long ldb, long long ldc, int b_mn, int sm_count, cudaStream_t stream) {
   const int M = world * rows_per_rank;
   if (world > 16 || (rows_per_rank % BMH) || (M % BM2) || (ld & 7) || (ldb & 7) || (K & 7)) return -2;
-  if (ld != K && (long long)K * 2 > Smem2::STAGE_BYTES) return -2;  // a strided row must fit one 32 KB copy slot
+  if (ld != K && (long long)K * 2 > SmemPlain::STAGE_BYTES) return -2;  // a strided row must fit one 32 KB copy slot
   int chunk_rows = 1024;
   while (rows_per_rank % chunk_rows) chunk_rows >>= 1;
   Gemm2Params p;
@@ -999,14 +1125,50 @@ int fb_gemm2_swiglu(const void* A, const void* W, void* GU, void* Z, int M, int 
   p.group_m = 8;
   p.status = fb::status_ptr();
   p.m_rot = 0; p.g_ncopy = 0; p.g_mode = 0; p.s_world = 0;
-  p.swiglu_I = I; p.Z = (__nv_bfloat16*)Z; p.ldz = ldz;
+  p.swiglu_I = I;
   p.C = GU; p.ldc = ldgu; p.split_stride = 0; p.epi = 0;
   CUtensorMap tmA, tmB;
   int rc = fb::make_tmap_2d(&tmA, A, 2, M, K, lda, BMH, BK, true);
   if (rc) return rc;
   rc = fb::make_tmap_2d(&tmB, W, 2, 2 * I, K, ldw, BNH, BK, true);
   if (rc) return rc;
-  return launch2<false, false>(tmA, tmB, p, sm_count, stream);
+  CUtensorMap tmGU, tmZ;
+  rc = fb::make_tmap_2d(&tmGU, GU, 2, M, 2 * I, ldgu, 32, 64, true);
+  if (rc) return rc;
+  rc = fb::make_tmap_2d(&tmZ, Z, 2, M, I, ldz, 32, 64, true);
+  if (rc) return rc;
+  return start2<false, false, false, false>(tmA, tmB, tmGU, tmZ, p, sm_count, stream);
+}
+
+// Backward of the above through the down projection: dz[M, I] = DY[M, K] * W[K, I] stays in the accumulators, and from it and
+// GU[M, 2 I] (gate columns first, then up) come DGU[M, 2 I], the gradients of gate and up; I must be a multiple of 128.
+int fb_gemm2_swiglu_bwd(const void* DY, const void* W, const void* GU, void* DGU, int M, int I, int K, long long lddy, long long ldw,
+                        long long ldgu, long long lddgu, int sm_count, cudaStream_t stream) {
+  if (M <= 0 || I <= 0 || K <= 0) return 0;
+  if ((I % BNH) || (lddy & 7) || (ldw & 7) || (ldgu & 7) || (lddgu & 7) || ((uintptr_t)DY & 15) || ((uintptr_t)W & 15) ||
+      ((uintptr_t)GU & 15) || ((uintptr_t)DGU & 15))
+    return -2;
+  Gemm2Params p;
+  p.M = M; p.N = I; p.K = K;
+  p.tiles_m = (M + BM2 - 1) / BM2;
+  p.tiles_n = (I + BN - 1) / BN;
+  p.num_kb = (K + BK - 1) / BK;
+  p.splits = 1; p.kb_per_split = p.num_kb;
+  p.alpha = 1.f; p.alpha_a = nullptr; p.alpha_b = nullptr; p.fp8_formats = 0;
+  p.group_m = sweep_rows(p.tiles_n, I, K);
+  p.status = fb::status_ptr();
+  p.m_rot = 0; p.g_ncopy = 0; p.g_mode = 0; p.s_world = 0; p.swiglu_I = 0;
+  p.C = DGU; p.ldc = lddgu; p.split_stride = 0; p.epi = 0;
+  CUtensorMap tmA, tmB, tmGU, tmDGU;
+  int rc = fb::make_tmap_2d(&tmA, DY, 2, M, K, lddy, BMH, BK, true);
+  if (rc) return rc;
+  rc = fb::make_tmap_2d(&tmB, W, 2, K, I, ldw, BK, 64, true);
+  if (rc) return rc;
+  rc = fb::make_tmap_2d(&tmGU, GU, 2, M, 2 * I, ldgu, 32, 64, true);
+  if (rc) return rc;
+  rc = fb::make_tmap_2d(&tmDGU, DGU, 2, M, 2 * I, lddgu, 32, 64, true);
+  if (rc) return rc;
+  return start2<false, true, false, true>(tmA, tmB, tmDGU, tmGU, p, sm_count, stream);
 }
 
 // Sharded-parameter all-gather fused into the first GEMM that consumes one of the gathered weights.

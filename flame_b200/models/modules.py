@@ -133,11 +133,11 @@ class GatedMLP(nn.Module):
             from ..parallel.tensor_parallel import allgather_linear, linear_reduce_scatter
             gu = allgather_linear(x, (self.gate_proj.weight, self.up_proj.weight))
             return linear_reduce_scatter(activations.swiglu(gu), self.down_proj.weight)
-        from ..ops.linear import gate_up_swiglu
-        z = gate_up_swiglu(x, self.gate_proj.weight, self.up_proj.weight)   # activation in the GEMM epilogue (opt-in)
-        if z is None:
-            z = activations.swiglu(fused_projection(x, (self.gate_proj, self.up_proj)))
-        return self.down_proj(z)
+        if plain((self.down_proj,), Linear) and self.down_proj.bias is None:
+            y = linear_ops.gated_mlp(x, self.gate_proj.weight, self.up_proj.weight, self.down_proj.weight)
+            if y is not None:
+                return y
+        return self.down_proj(activations.swiglu(fused_projection(x, (self.gate_proj, self.up_proj))))
 
 
 class ShortConvolution(nn.Module):

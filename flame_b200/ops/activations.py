@@ -30,11 +30,7 @@ class _SwiGLUFn(torch.autograd.Function):
         gu2 = gu.reshape(-1, 2 * I)
         gu2 = gu2 if gu2.is_contiguous() else gu2.contiguous()
         T = gu2.shape[0]
-        a = torch.empty(T, I, dtype=gu.dtype, device=gu.device)
-        rc = _lib.lib().fb_swiglu_fwd(gu2.data_ptr(), gu2.data_ptr() + 2 * I, a.data_ptr(), T, I, 2 * I, 2 * I, I,
-                                      _lib.stream_ptr())
-        _lib.check(rc, "fb_swiglu_fwd")
-        _lib.count_launch()
+        a = swiglu_forward(gu2, torch.empty(T, I, dtype=gu.dtype, device=gu.device))
         ctx.save_for_backward(gu2)
         ctx.shape = shape
         return a.view(*shape[:-1], I)
@@ -42,16 +38,18 @@ class _SwiGLUFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, da):
         (gu2,) = ctx.saved_tensors
-        T, I2 = gu2.shape
-        I = I2 // 2
-        da2 = da.reshape(-1, I)
+        da2 = da.reshape(-1, gu2.shape[1] // 2)
         da2 = da2 if da2.is_contiguous() else da2.contiguous()
-        dgu = torch.empty_like(gu2)
-        rc = _lib.lib().fb_swiglu_bwd(da2.data_ptr(), gu2.data_ptr(), gu2.data_ptr() + 2 * I, dgu.data_ptr(),
-                                      dgu.data_ptr() + 2 * I, 0, T, I, I, I2, I2, I2, I2, I, _lib.stream_ptr())
-        _lib.check(rc, "fb_swiglu_bwd")
-        _lib.count_launch()
-        return dgu.view(ctx.shape)
+        return swiglu_backward(da2, gu2).view(ctx.shape)
+
+
+def swiglu_forward(gu2: torch.Tensor, a: torch.Tensor) -> torch.Tensor:
+    """``a [T, I] = silu(gate) * up`` of ``[gate | up] [T, 2 I]``, both contiguous."""
+    T, I = a.shape
+    rc = _lib.lib().fb_swiglu_fwd(gu2.data_ptr(), gu2.data_ptr() + 2 * I, a.data_ptr(), T, I, 2 * I, 2 * I, I, _lib.stream_ptr())
+    _lib.check(rc, "fb_swiglu_fwd")
+    _lib.count_launch()
+    return a
 
 
 def swiglu_backward(da2: torch.Tensor, gu2: torch.Tensor) -> torch.Tensor:

@@ -261,76 +261,154 @@ def linear_fused(x: torch.Tensor, weights: Sequence[torch.Tensor]) -> torch.Tens
 
 
 # --------------------------------------------------------------------------------------------------------------
-# gate | up projection with the SwiGLU activation in the GEMM epilogue
+# SwiGLU in the epilogues of the products around it
 # --------------------------------------------------------------------------------------------------------------
 _lib.register("fb_gemm2_swiglu", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
                                   c_longlong, c_longlong, c_int, c_void_p])
+_lib.register("fb_gemm2_swiglu_bwd", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_longlong, c_longlong,
+                                      c_longlong, c_longlong, c_int, c_void_p])
+
+
+def _rows(x: torch.Tensor) -> torch.Tensor:
+    """``x [..., N]`` as a matrix the GEMM kernels read: rows of whole 16-byte vectors."""
+    x = x.reshape(-1, x.shape[-1])
+    if x.stride(1) != 1 or x.stride(0) % 8 or x.data_ptr() % 16 or (x.shape[0] > 1 and x.stride(0) < x.shape[1]):
+        x = x.clone(memory_format=torch.contiguous_format)
+    return x
+
+
+def _gate_up(x2: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor):
+    """``gate | up [T, 2 I]`` and ``z = silu(gate) * up`` from ONE kernel: the GEMM's epilogue holds gate_j and up_j of the same hidden
+    index side by side (the two CTAs of a pair load the gate rows and the up rows of the fused weight) and writes both, which the
+    backward needs, and the activation."""
+    from . import gemm as gemm_ops
+    T, K = x2.shape
+    I = wg.shape[0]
+    wcat = _cat_view([wg.detach(), wu.detach()])
+    gu = torch.empty(T, 2 * I, dtype=x2.dtype, device=x2.device)
+    z = torch.empty(T, I, dtype=x2.dtype, device=x2.device)
+    pend = gemm_ops.pending_gather()
+    if pend is not None and not pend.done and pend.touches(wcat):  # a plain product may fetch the weights on its way
+        from .activations import swiglu_forward
+        return gemm_nt(x2, wcat, gu), swiglu_forward(gu, z)
+    rc = _lib.lib().fb_gemm2_swiglu(x2.data_ptr(), wcat.data_ptr(), gu.data_ptr(), z.data_ptr(), T, I, K, x2.stride(0),
+                                    wcat.stride(0), gu.stride(0), z.stride(0), gemm_ops._sm_count(x2.device),
+                                    _lib.stream_ptr())
+    _lib.check(rc, "fb_gemm2_swiglu")
+    _lib.count_launch()
+    return gu, z
+
+
+def _gate_up_grads(dgu, x2, wg, wu, params, need, dx=None):
+    """Gradients of the input and, unless they went to ``main_grad``, of the two weights; ``need`` as ``needs_input_grad`` of
+    (x, gate, up); ``dx``: where the input's gradient is wanted, or None."""
+    I = wg.shape[0]
+    if need[0]:
+        dx = gemm_nn(dgu, _cat_view([wg, wu]) if _adjacent([wg, wu]) else torch.cat([wg, wu], 0), dx)
+    mgs = [getattr(w, "main_grad", None) for w in params]
+    if all(m is not None for m in mgs) and _adjacent(mgs):
+        gemm_tn(dgu, x2, out=_cat_view(mgs), accumulate=True)
+        return dx, None, None
+    grads = []
+    for w, m, d, n in zip(params, mgs, (dgu[:, :I], dgu[:, I:]), need[1:]):
+        if m is not None:
+            gemm_tn(d, x2, out=m, accumulate=True)
+        grads.append(gemm_tn(d, x2, out_dtype=torch.float32).to(w.dtype) if m is None and n else None)
+    return (dx, *grads)
 
 
 class _GateUpSwiGLU(torch.autograd.Function):
-    """``z = silu(x @ Wg.T) * (x @ Wu.T)`` from ONE kernel: the GEMM's epilogue holds gate_j and up_j of the same hidden
-    index side by side (the two CTAs of a pair load the gate rows and the up rows of the fused weight), writes both (the
-    backward pass needs them) and the activation.  Saves the pass that re-read ``[T, 2 I]`` to write ``[T, I]``."""
+    """``z = silu(x @ Wg.T) * (x @ Wu.T)``, see ``_gate_up``."""
 
     @staticmethod
     def forward(ctx, x, wg, wu):
-        from . import gemm as gemm_ops
         shape = x.shape
-        K = shape[-1]
-        x2 = x.reshape(-1, K)
-        x2 = x2 if x2.is_contiguous() else x2.contiguous()
-        T, I = x2.shape[0], wg.shape[0]
-        wcat = _cat_view([wg.detach(), wu.detach()])
-        pend = gemm_ops.pending_gather()
-        if pend is not None and not pend.done and pend.touches(wcat):
-            pend.flush()
-        gu = torch.empty(T, 2 * I, dtype=x.dtype, device=x.device)
-        z = torch.empty(T, I, dtype=x.dtype, device=x.device)
-        rc = _lib.lib().fb_gemm2_swiglu(x2.data_ptr(), wcat.data_ptr(), gu.data_ptr(), z.data_ptr(), T, I, K, x2.stride(0),
-                                        wcat.stride(0), gu.stride(0), z.stride(0), gemm_ops._sm_count(x.device),
-                                        _lib.stream_ptr())
-        _lib.check(rc, "fb_gemm2_swiglu")
-        _lib.count_launch()
+        x2 = _rows(x)
+        gu, z = _gate_up(x2, wg, wu)
         ctx.save_for_backward(x2, gu, wg, wu)
         ctx.params = (wg, wu)
         ctx.shape = shape
-        return z.view(*shape[:-1], I)
+        return z.view(*shape[:-1], z.shape[1])
 
     @staticmethod
     def backward(ctx, dz):
         from .activations import swiglu_backward
         x2, gu, wg, wu = ctx.saved_tensors
-        I = wg.shape[0]
-        dz2 = dz.reshape(-1, I)
+        dz2 = dz.reshape(-1, wg.shape[0])
         dgu = swiglu_backward(dz2 if dz2.is_contiguous() else dz2.contiguous(), gu)
+        dx, gg, gu_ = _gate_up_grads(dgu, x2, wg, wu, ctx.params, ctx.needs_input_grad)
+        return None if dx is None else dx.view(ctx.shape), gg, gu_
+
+
+class _GatedMLP(torch.autograd.Function):
+    """``(silu(x @ Wg.T) * (x @ Wu.T)) @ Wd.T`` as one node: the activation is formed in the epilogue of the first product, and its backward
+    in the epilogue of the down projection's data gradient, which never goes to memory."""
+
+    @staticmethod
+    def forward(ctx, x, wg, wu, wd):
+        shape = x.shape
+        ctx.slot = slots.of(x) if x.dim() == 2 else None
+        x2 = _rows(x)
+        gu, z = _gate_up(x2, wg, wu)
+        y = gemm_nt(z, wd.detach())
+        ctx.save_for_backward(x2, gu, z, wg, wu, wd)
+        ctx.params = (wg, wu, wd)
+        ctx.shape = shape
+        return y.view(*shape[:-1], y.shape[1])
+
+    @staticmethod
+    def backward(ctx, dy):
+        from . import gemm as gemm_ops
+        from .activations import swiglu_backward
+        x2, gu, z, wg, wu, wd = ctx.saved_tensors
+        T, I, D = z.shape[0], z.shape[1], wd.shape[0]
+        need_x, need_g, need_u, need_d = ctx.needs_input_grad
+        dy2 = _rows(dy)
+        dgu = None
+        if need_x or need_g or need_u:
+            wd2, gu = _rows(wd), _rows(gu)  # saved-tensor hooks hand back copies, which lie wherever they were put
+            pend = gemm_ops.pending_gather()
+            if pend is not None and not pend.done and pend.touches(wd2):  # a plain product may fetch the weights on its way
+                dgu = swiglu_backward(gemm_nn(dy2, wd2), gu)
+            else:
+                dgu = torch.empty(T, 2 * I, dtype=gu.dtype, device=gu.device)
+                rc = _lib.lib().fb_gemm2_swiglu_bwd(dy2.data_ptr(), wd2.data_ptr(), gu.data_ptr(), dgu.data_ptr(), T, I, D, dy2.stride(0),
+                                                    wd2.stride(0), gu.stride(0), dgu.stride(0), gemm_ops._sm_count(gu.device),
+                                                    _lib.stream_ptr())
+                _lib.check(rc, "fb_gemm2_swiglu_bwd")
+                _lib.count_launch()
+        gd = None
+        mg = getattr(ctx.params[2], "main_grad", None)
+        if mg is not None:
+            gemm_tn(dy2, z, out=mg, accumulate=True)
+        elif need_d:
+            gd = gemm_tn(dy2, z, out_dtype=torch.float32).to(wd.dtype)
+        if dgu is None:
+            return None, None, None, gd
         dx = None
-        if ctx.needs_input_grad[0]:
-            dx = gemm_nn(dgu, _cat_view([wg, wu]) if _adjacent([wg, wu]) else torch.cat([wg, wu], 0)).view(ctx.shape)
-        mgs = [getattr(w, "main_grad", None) for w in ctx.params]
-        gg = gu_ = None
-        if all(m is not None for m in mgs) and _adjacent(mgs):
-            gemm_tn(dgu, x2, out=_cat_view(mgs), accumulate=True)
-        elif all(m is not None for m in mgs):
-            gemm_tn(dgu[:, :I], x2, out=mgs[0], accumulate=True)
-            gemm_tn(dgu[:, I:], x2, out=mgs[1], accumulate=True)
-        else:
-            gg = gemm_tn(dgu[:, :I], x2, out_dtype=torch.float32).to(wg.dtype)
-            gu_ = gemm_tn(dgu[:, I:], x2, out_dtype=torch.float32).to(wu.dtype)
-        return dx, gg, gu_
+        if need_x:
+            dx = None if ctx.slot is None else ctx.slot.take(T, x2.shape[1], x2.dtype, x2.device)
+            if dx is not None and (dx.stride(0) % 8 or dx.data_ptr() % 16):
+                dx = None
+        dx, gg, gu_ = _gate_up_grads(dgu, x2, wg, wu, ctx.params[:2], (need_x, need_g, need_u), dx)
+        return None if dx is None else dx.view(ctx.shape), gg, gu_, gd
+
+
+def _swiglu_epilogue_ok(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor) -> bool:
+    return (_kernel_ok(x, wg) and _kernel_ok(x, wu) and wg.shape == wu.shape and wg.shape[0] % 128 == 0 and x.numel() > 0
+            and not getattr(wg, "_fp8", False) and not getattr(wu, "_fp8", False) and sac.current() is None
+            and _adjacent([wg.detach(), wu.detach()]) and wg.data_ptr() % 16 == 0)
 
 
 def gate_up_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor) -> Optional[torch.Tensor]:
-    """The fused projection + activation when ``FLAME_B200_FUSED_SWIGLU=1`` and its conditions hold (bf16 on the GPU,
-    adjacent weights, I a multiple of 128, no fp8 weights, no selective-checkpointing tape); ``None`` tells the caller to
-    take the two-step path.  Opt-in because it measured slower: at 65,536 x 5632 x 1024 the GEMM with the activation in
-    its epilogue takes 0.84 ms against 0.73 ms for the plain GEMM plus the SwiGLU kernel (the epilogue writes three
-    tiles - gate, up and the product, which the backward needs - per accumulator instead of two, and that costs the
-    pipeline more than the saved 0.7 GB read is worth)."""
-    import os
-    if not (_kernel_ok(x, wg) and _kernel_ok(x, wu) and wg.shape == wu.shape and wg.shape[0] % 128 == 0):
+    """``silu(x @ Wg.T) * (x @ Wu.T)`` from one product (bf16 on the GPU, adjacent weights, I a multiple of 128, no fp8 weights, no
+    selective-checkpointing tape, which counts products); ``None`` tells the caller to take the two-step path."""
+    return _GateUpSwiGLU.apply(x, wg, wu) if _swiglu_epilogue_ok(x, wg, wu) else None
+
+
+def gated_mlp(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor, wd: torch.Tensor) -> Optional[torch.Tensor]:
+    """The whole bias-free SwiGLU MLP under the conditions of ``gate_up_swiglu``; ``None`` where they do not hold."""
+    if not (_swiglu_epilogue_ok(x, wg, wu) and wd.dtype is torch.bfloat16 and wd.is_cuda and wd.shape[1] == wg.shape[0] and wd.shape[0] % 8 == 0
+            and wd.is_contiguous() and wd.data_ptr() % 16 == 0 and not getattr(wd, "_fp8", False)):
         return None
-    if getattr(wg, "_fp8", False) or getattr(wu, "_fp8", False) or sac.current() is not None:
-        return None
-    if not _adjacent([wg.detach(), wu.detach()]) or os.environ.get("FLAME_B200_FUSED_SWIGLU", "0") != "1":
-        return None
-    return _GateUpSwiGLU.apply(x, wg, wu)
+    return _GatedMLP.apply(x, wg, wu, wd)

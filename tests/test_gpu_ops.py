@@ -555,6 +555,41 @@ def test_gate_up_projection_with_swiglu_epilogue(monkeypatch):
     assert rel_err(x.grad, xf.grad) < 2e-2 and rel_err(wg.grad, gf.grad) < 2e-2 and rel_err(wu.grad, uf.grad) < 2e-2
 
 
+@pytest.mark.parametrize("T,K,I,grads", [(1, 64, 128, "autograd"), (255, 64, 384, "adjacent"), (257, 72, 128, "apart"), (1000, 512, 1408, "adjacent"),
+                                         (20000, 128, 256, "autograd"), (300, 64, 384, "hooks"), (300, 64, 384, "frozen")])
+def test_gated_mlp_in_one_node(T, K, I, grads):
+    """Both activations in the products' epilogues against 64 bits, over partial tiles in rows and columns, several rounds of tiles, and
+    every way the weights' gradients go.  Operands and results of bf16, sums of up to 1,408 terms: each output within a few 2^-8 of
+    itself."""
+    from flame_b200.ops import linear as ops
+    torch.manual_seed(13)
+    flat = (torch.randn(3 * I * K, device=DEV) * K ** -0.5).to(torch.bfloat16)
+    ws = [torch.nn.Parameter(flat[i * I * K:(i + 1) * I * K].view(*((I, K) if i < 2 else (K, I)))) for i in range(3)]
+    if grads in ("adjacent", "apart"):
+        acc = torch.ones(3, 2 * I * K, device=DEV)
+        for i, w in enumerate(ws):
+            w.main_grad = (acc.view(-1)[i * I * K:(i + 1) * I * K] if grads == "adjacent" else acc[i, :I * K]).view(w.shape)
+    if grads == "frozen":
+        ws[0].requires_grad_(False), ws[2].requires_grad_(False)
+    x = torch.randn(T, 2 * K, device=DEV, dtype=torch.bfloat16)[:, K:].requires_grad_(True)   # rows apart
+    dy = torch.randn(T, K + 3, device=DEV, dtype=torch.bfloat16)[:, 3:]                       # rows that start between vectors
+    pack = (lambda t: t.clone()) if grads == "hooks" else (lambda t: t)
+    with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t):
+        y = ops.gated_mlp(x, *ws)
+    y.backward(dy)
+    xr, *wr = (t.detach().double().requires_grad_(True) for t in (x, *ws))
+    yr = (torch.nn.functional.silu(xr @ wr[0].t()) * (xr @ wr[1].t())) @ wr[2].t()
+    yr.backward(dy.double())
+    assert rel_err(y, yr) < 1e-2 and rel_err(x.grad, xr.grad) < 1.5e-2
+    for i, (w, r) in enumerate(zip(ws, wr)):
+        if not w.requires_grad:
+            assert w.grad is None
+            continue
+        assert rel_err(w.main_grad - 1 if hasattr(w, "main_grad") else w.grad, r.grad) < 1.5e-2
+    if grads == "apart":
+        assert torch.equal(acc[:, I * K:], torch.ones(3, I * K, device=DEV))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("with_lb", [False, True])
 def test_hgrn2_gate_kernels_match_the_elementwise_chain(with_lb):
