@@ -418,17 +418,18 @@ class _GatedDelta(torch.autograd.Function):
         w = bgemm(Tw, kh, b_mn=True, out=_token_major(NC, H, C, dk, q.dtype, q.device))
         M = bgemm(khh, w, a_mn=True, b_mn=True)                                           # [NC, H, dk, dk] chunk transition
         S = _delta_states(M, bgemm(khh, u, a_mn=True, b_mn=True), alpha, lay)             # [NC, H, dk, dv]
-        vn = bgemm(w, S, b_mn=True, alpha=-1.0, add16=u, out=_token_major(NC, H, C, dv, q.dtype, q.device))      # u - w S
+        # u - w S; u again as a product in the same accumulator: added from its bf16 copy it would be rounded twice
+        vn = bgemm(Tu, vh, b_mn=True, more=[(w, S, False, True, -1)], out=_token_major(NC, H, C, dv, q.dtype, q.device))
         o = bgemm(qbh, S, b_mn=True, alpha=scale, more=[(Q, vn, False, True, 1)],
                   out=_token_major(NC, H, C, dv, q.dtype, q.device))
         ctx.save_for_backward(q, k, v, beta, b, khat if b is not None else None, qbar if b is not None else None, alpha, P, Q, T, Tu,
-                              Tw if b is not None else None, u, w, M, S, vn)
+                              Tw if b is not None else None, w, M, S, vn)
         ctx.cfg = (scale, lay)
         return o.permute(0, 2, 1, 3)
 
     @staticmethod
     def backward(ctx, do):
-        q, k, v, beta, b, khat, qbar, alpha, P, Q, T, Tu, Tw, u, w, M, S, vn = ctx.saved_tensors
+        q, k, v, beta, b, khat, qbar, alpha, P, Q, T, Tu, Tw, w, M, S, vn = ctx.saved_tensors
         scale, lay = ctx.cfg
         NC, C, H, dk = q.shape
         dt, dev = q.dtype, q.device
@@ -449,12 +450,13 @@ class _GatedDelta(torch.autograd.Function):
         if inner or need_v:
             dvn = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(dv))
             Ln = _delta_adjoint(M, bgemm(qbh, doh, a_mn=True, b_mn=True, more=[(w, dvn, True, True, -1)]), alpha, lay)
-            du = bgemm(khh, Ln, b_mn=True, add16=dvn, out=tok(dv))
+            # dvn again as a product in the same accumulator: added from its bf16 copy it would be rounded twice
+            du = bgemm(khh, Ln, b_mn=True, more=[(Q, doh, True, True, 1)], out=tok(dv))
             if need_v:
                 dvv = bgemm(Tu, du, a_mn=True, b_mn=True, alpha=scale, out=tok(dv))
         if inner:
-            dM = bgemm(Ln, S, alpha=-1.0)                                                 # [NC, H, dk, dk]
-            dw = bgemm(khh, dM, b_mn=True, more=[(dvn, S, False, False, -1)], out=tok(dk))
+            # S leaves a chunk as alpha S + khat^T vn, vn = u - w S: what reaches vn reaches u and, times -S^T, w
+            dw = bgemm(du, S, alpha=-1.0, out=tok(dk))
             if gated:
                 dTu, dTw = bgemm(du, vh), bgemm(dw, kh)
             else:
@@ -470,7 +472,7 @@ class _GatedDelta(torch.autograd.Function):
         if gated and gq is not None:
             gq = gq2.to(dt)
             dqbar = bgemm(doh, S, out=tok(dk)) if need_q or need_g else None
-            dkhat = bgemm(u, Ln, alpha=scale, more=[(w, dM, False, False, 1)], out=tok(dk)) if need_k or need_g else None
+            dkhat = bgemm(vn, Ln, alpha=scale, out=tok(dk)) if need_k or need_g else None
             dalpha = _pair_dot(Ln, S, per_row=False) * scale if need_g else None
             dq0, dk0, dg = _scalar_prep_raw_bwd(q, k, b, back(dkhat), back(dqbar), dalpha, db, scale)
             if need_q:
@@ -482,7 +484,7 @@ class _GatedDelta(torch.autograd.Function):
                 dq = bgemm(doh, S, alpha=scale, more=[(gq, kh, False, True, 1)], out=tok(dk))
             if need_k:
                 dkk = bgemm(Tu, dw, a_mn=True, b_mn=True, alpha=scale, out=tok(dk),
-                            more=keys + [(gq, qh, True, True, 1), (u, Ln, False, False, 1), (w, dM, False, False, 1)])
+                            more=keys + [(gq, qh, True, True, 1), (vn, Ln, False, False, 1)])
         return back(dq), back(dkk), back(dvv), dbeta if need_beta else None, dg if need_g else None, None, None
 
 
