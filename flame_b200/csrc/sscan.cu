@@ -16,16 +16,17 @@
 // What bounds it: one exponential per state element and sweep, 16 MUFU results per clock and SM: 0.24 ms per sweep at 32,768
 // tokens x 2,048 channels; the forward needs two sweeps, the backward three.  Everything else has to stay below that in
 // issue slots: sweeps (1), (3), (4) give a thread a whole channel (16 states, B / C read as float4 broadcasts, no
-// shuffles), sweep (6) gives it 2 channels x 4 states, so that the sums over states and over channels are mostly
-// additions in registers, finished through shared memory; pairs of states use the packed fp32x2 instructions.  Every
-// sweep fetches its operands a group of four steps ahead: waiting for memory at each group, not the MUFU, set the pace before.
-// At that size with gate and softplus, before and after: (1) 0.44 -> 0.31 ms, (3) 0.84 -> 0.47, (4) 0.59 -> 0.36,
-// (6) 2.17 -> 1.63.
+// shuffles), sweep (6) gives it 4 channels x 4 states (see there); pairs of states, or of channels, use the packed fp32x2
+// instructions.  Every sweep fetches its operands ahead: waiting for memory at each group of steps, not the MUFU, set the pace
+// before.  At that size with gate and softplus, before and after: (1) 0.44 -> 0.31 ms, (3) 0.84 -> 0.47, (4) 0.59 -> 0.36,
+// (6) 2.17 -> 1.63 -> 1.26.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <type_traits>
 
 #include "host_utils.cuh"
+#include "tc05.cuh"
 
 namespace {
 
@@ -100,6 +101,33 @@ __device__ __forceinline__ float softplus(float x) {
   p = fmaf(p, w, 1.f);
   return fmaf(2.f * s, p, fmaxf(x, 0.f));
 }
+
+// two channels at a time
+__device__ __forceinline__ f2 dup(float v) { return pk(v, v); }
+__device__ __forceinline__ f2 rcp2(f2 v) {
+  float a, b;
+  up(v, a, b);
+  return pk(__fdividef(1.f, a), __fdividef(1.f, b));
+}
+__device__ __forceinline__ f2 sigm2(f2 x) { return rcp2(add2(ex2v(mul2(x, dup(-LOG2E))), dup(1.f))); }
+// softplus and its derivative from one exponential
+__device__ __forceinline__ void softplus2(f2 x, f2& sp, f2& sg) {
+  float x0, x1;
+  up(x, x0, x1);
+  const f2 e = ex2v(mul2(pk(-fabsf(x0), -fabsf(x1)), dup(LOG2E))), s = mul2(e, rcp2(add2(e, dup(2.f)))), w = mul2(s, s);
+  f2 p = fma2(w, dup(1.f / 13.f), dup(1.f / 11.f));
+  p = fma2(p, w, dup(1.f / 9.f));
+  p = fma2(p, w, dup(1.f / 7.f));
+  p = fma2(p, w, dup(1.f / 5.f));
+  p = fma2(p, w, dup(1.f / 3.f));
+  p = fma2(p, w, dup(1.f));
+  sp = fma2(add2(s, s), p, pk(fmaxf(x0, 0.f), fmaxf(x1, 0.f)));
+  float r0, r1, e0, e1;
+  up(rcp2(add2(e, dup(1.f))), r0, r1);
+  up(e, e0, e1);
+  sg = pk(x0 >= 0.f ? r0 : e0 * r0, x1 >= 0.f ? r1 : e1 * r1);
+}
+__device__ __forceinline__ f2 bf2(uint32_t v) { return pk(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
 
 __device__ __forceinline__ float load_bc(const ScanArgs& a, const void* p, int stride, long long row, int n) {
   return a.bc16 ? __bfloat162float(((const __nv_bfloat16*)p)[row * stride + n]) : ((const float*)p)[row * stride + n];
@@ -395,23 +423,35 @@ __global__ void __launch_bounds__(CT) sscan_local_bwd_kernel(ScanArgs a, const _
   }
 }
 
-// (6): all gradients of one chunk and 64 channels, 16 steps at a time from the back.  Lane = (channel pair cg, state quad q).
-// Per 16 steps: recompute the states from the kept one, leaving one every four steps in shared memory; then per four steps
-// recompute decay and decayed state into registers and walk back.  Four steps' partial sums go to shared memory, from
-// where the warp adds them: over the four quads (ddelta, du) and over the eight channel pairs (dB, dC).
+// (6): all gradients of one chunk and 128 channels, 16 steps at a time from the back.  A warp has 32 channels: lane = (channel
+// quad cg, state quad q), a thread 4 channels x 4 states in eight channel pairs.  Per 16 steps: recompute the states from the
+// kept one, leaving one every four steps in shared memory; then per four steps recompute decays and states, leaving them in
+// tensor memory (32 columns a step, the thread's own lane: the 128 registers they would take cost a third of the warps), and
+// walk back.  What bounds it: issue slots (355 instructions per warp and step, two per clock with 12 warps an SM), of which eight
+// packed multiply-adds per pair on the way back and three forward are the work.  The sums over states (ddelta, du) and over
+// channels (dB, dC) are halved from lane to lane by shuffles: a thread's registers are numbered so that what a lane keeps lies
+// in the same registers on every lane (register k holds state k ^ (cg & 3) of the quad, register j channel pair j ^ (q >> 1)),
+// which leaves six selects per step instead of 26.  Measured at 32,768 tokens x 2,048 channels: 2 channels x 4 states and sums
+// through shared memory (73 % of its bandwidth) 1.62 ms; this split with all four steps in registers (8 warps) 1.85, in tensor
+// memory 1.48, a step's sums under the next one's loads and results through shared memory 1.39, two channels staged at a
+// time 1.26.
 constexpr int BT = 128;                    // threads
-constexpr int BC = 64;                     // channels per block
-constexpr int RROW = 36;                   // float4 per row of the reduction buffer (32 lanes + 4: rows start on other banks)
+constexpr int BC = 128;                    // channels per block
+constexpr int G = 4;                       // steps recomputed into registers together
 struct BwdSmem {
-  float4 dl[SEG][BC / 2];                  // (delta, delta) of two channels
-  float4 x[SEG][BC / 2];                   // (delta u, delta u)
-  float4 dy[SEG][BC / 2];
-  float B[SEG][N];
-  float C[SEG][N];
-  float4 ck[3][2][BT];                     // states entering steps 0, 4, 8 of the segment
-  float4 red[BT / 32][4 * 3 * RROW];
+  float dl[SEG][BC];
+  float sg[SEG][BC];                       // derivative of delta by its argument
+  float u[SEG][BC];
+  float dy[SEG][BC];
+  float2 B[SEG][N];                        // (value, value)
+  float2 C[SEG][N];
+  f2 ck[SEG / G - 1][8][BT];               // states entering steps 0, 4, 8 of the segment
   float bc[BT / 32][SEG][2 * N];           // per-warp dB | dC
+  uint32_t tmem;
 };
+
+__device__ __forceinline__ f2 lds2(const void* p) { return *reinterpret_cast<const f2*>(p); }
+__device__ __forceinline__ float shx(float v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
 
 template <bool RAW, bool GATE>
 __global__ void __launch_bounds__(BT, 3) sscan_bwd_kernel(ScanArgs a, const __nv_bfloat16* __restrict__ dout, const __nv_bfloat16* __restrict__ y,
@@ -426,213 +466,309 @@ __global__ void __launch_bounds__(BT, 3) sscan_bwd_kernel(ScanArgs a, const __nv
   long long row0;
   int len;
   chunk_rows(a, c, row0, len);
-  const int cp = warp * 8 + cg;            // channel pair of this lane within the block
-  const int dc = d0 + 2 * cp;
-  f2 A2[2][2], carry[2][2], dAa[2][2], h[2][2];
-  const float* ad = adj + (long long)c * N * a.DiP + dc;
-#pragma unroll
-  for (int k = 0; k < 2; ++k) {
-    const float4 v = dc + k < a.Di ? *reinterpret_cast<const float4*>(a.A + (long long)(dc + k) * N + q * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
-    A2[k][0] = pk(v.x * LOG2E, v.y * LOG2E);
-    A2[k][1] = pk(v.z * LOG2E, v.w * LOG2E);
-    dAa[k][0] = dAa[k][1] = 0ull;
+  if (warp == 0) {
+    tc05::tmem_alloc(&s.tmem, 32 * G);
+    tc05::tmem_relinquish();
   }
+  tc05::tc_fence_before();
+  __syncthreads();
+  tc05::tc_fence_after();
+  const uint32_t taddr = s.tmem + ((uint32_t)(warp * 32) << 16);
+  int ch[2], nn[4];                        // channel pairs within the block and states of this thread's registers
 #pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    const int n = q * 4 + 2 * p;
-    const float2 lo = *reinterpret_cast<const float2*>(ad + n * a.DiP), hi = *reinterpret_cast<const float2*>(ad + (n + 1) * a.DiP);
-    carry[0][p] = pk(lo.x, hi.x);
-    carry[1][p] = pk(lo.y, hi.y);
-  }
-  // the lane that finishes sums over states handles step t = lane / 8 (of four) and channel pair lane % 8 of its warp
-  const int fcp = warp * 8 + (lane & 7), fd = d0 + 2 * fcp;
-  const float D0 = fd < a.Di ? a.Dv[fd] : 0.f, D1 = fd + 1 < a.Di ? a.Dv[fd + 1] : 0.f;
-  float dD0 = 0.f, dD1 = 0.f;
-  const int st_ch = tid % BC, st_t = tid / BC, st_d = d0 + st_ch;
-  const bool st_live = st_d < a.Di;
-  const DeltaCol<RAW> delta(a, row0, st_d), fdelta(a, row0, fd);
-  const Col16 ucol(a.u, row0, a.us, st_d), ocol(dout, row0, a.Di, st_d), zcol(GATE ? a.z : dout, row0, GATE ? a.zs : a.Di, st_d),
-      ycol(GATE ? y : dout, row0, a.Di, st_d), fu(a.u, row0, a.us, fd);
-  __nv_bfloat16* pdz = GATE ? dz + row0 * dzs + st_d : nullptr;
+  for (int j = 0; j < 2; ++j) ch[j] = warp * 32 + cg * 4 + 2 * (j ^ (q >> 1));
+#pragma unroll
+  for (int k = 0; k < 4; ++k) nn[k] = q * 4 + (k ^ (cg & 3));
+  f2 A2[2][4], carry[2][4], dAa[2][4], h[2][4];
+  const float* ad = adj + (long long)c * N * a.DiP + d0;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int d = d0 + ch[j];
+      const float lo = d < a.Di ? a.A[(long long)d * N + nn[k]] : 0.f, hi = d + 1 < a.Di ? a.A[(long long)(d + 1) * N + nn[k]] : 0.f;
+      A2[j][k] = pk(lo * LOG2E, hi * LOG2E);
+      carry[j][k] = lds2(ad + nn[k] * a.DiP + ch[j]);
+      dAa[j][k] = 0ull;
+    }
+  // after the sums over states a lane holds one channel pair: ddelta where q is even, du where it is odd
+  const bool is_du = q & 1;
+  const int fch = ch[0], fd = d0 + fch;
+  const f2 Df = is_du ? pk(fd < a.Di ? a.Dv[fd] : 0.f, fd + 1 < a.Di ? a.Dv[fd + 1] : 0.f) : 0ull;
+  const float* ffac = is_du ? &s.dl[0][fch] : &s.sg[0][fch];
+  const bool hi = cg & 4;
+  const bool even = (a.Di & 1) == 0;
+  const f2 ln2 = pk(LN2, LN2);
 
+  // a thread stages two neighbouring channels of eight steps
+  const int sc = 2 * (tid & 63), st0 = (tid >> 6) * 8, sd = d0 + sc;
+  const bool live0 = sd < a.Di, live1 = sd + 1 < a.Di;
+  const uintptr_t bases = (uintptr_t)a.u | (RAW ? (uintptr_t)a.dl : (uintptr_t)a.dl >> 1) | (uintptr_t)dout | (GATE ? (uintptr_t)a.z | (uintptr_t)y | (uintptr_t)dz : 0);
+  const bool vec = live1 && even && (bases & 3) == 0 && ((a.us | a.ds | (GATE ? a.zs | dzs : 0)) & 1) == 0;
+  f2 dDa = 0ull;
+  const u16* pu = reinterpret_cast<const u16*>(a.u) + row0 * a.us + sd;
+  const u16* po = reinterpret_cast<const u16*>(dout) + row0 * a.Di + sd;
+  const u16* pz = GATE ? reinterpret_cast<const u16*>(a.z) + row0 * a.zs + sd : nullptr;
+  const u16* py = GATE ? reinterpret_cast<const u16*>(y) + row0 * a.Di + sd : nullptr;
+  const u16* pr = RAW ? reinterpret_cast<const u16*>(a.dl) + row0 * a.ds + sd : nullptr;
+  const float* pf = RAW ? nullptr : reinterpret_cast<const float*>(a.dl) + row0 * a.ds + sd;
+  u16* pdz = GATE ? reinterpret_cast<u16*>(dz) + row0 * dzs + sd : nullptr;
+  u16* pdu = reinterpret_cast<u16*>(du) + row0 * a.Di + sd;
+  u16* pdd = reinterpret_cast<u16*>(ddl) + row0 * a.Di + sd;
+  // a row's two values; FULL: both channels and all rows exist and lie on four bytes
+  auto two = [&](auto full, const u16* p, bool row) -> uint32_t {
+    if constexpr (decltype(full)::value) return __ldg(reinterpret_cast<const uint32_t*>(p));
+    const uint32_t lo = row && live0 ? __ldg(p) : (u16)0, hi = row && live1 ? __ldg(p + 1) : (u16)0;
+    return lo | hi << 16;
+  };
+  auto stage = [&](auto full, int tb) {
+    constexpr bool FULL = decltype(full)::value;
+    uint32_t rd[8], ru[8], ro[8], rz[8], ry[8];
+    f2 rf[8];
+    const int r0 = tb + st0;
+    const u16 *qu = pu + r0 * a.us, *qo = po + r0 * a.Di, *qz = GATE ? pz + r0 * a.zs : nullptr, *qy = GATE ? py + r0 * a.Di : nullptr,
+              *qr = RAW ? pr + r0 * a.ds : nullptr;
+    u16* qdz = GATE ? pdz + r0 * dzs : nullptr;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const bool row = FULL || r0 + i < len;
+      ru[i] = two(full, qu + i * a.us, row);
+      ro[i] = two(full, qo + i * a.Di, row);
+      if (RAW) {
+        rd[i] = two(full, qr + i * a.ds, row);
+      } else {
+        const float* q = pf + (r0 + i) * a.ds;
+        rf[i] = pk(row && live0 ? __ldg(q) : 0.f, row && live1 ? __ldg(q + 1) : 0.f);
+      }
+      if (GATE) {
+        rz[i] = two(full, qz + i * a.zs, row);
+        ry[i] = two(full, qy + i * a.Di, row);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = st0 + i;
+      const bool row = FULL || r0 + i < len;
+      const f2 uv = bf2(ru[i]);
+      f2 dyv = bf2(ro[i]);
+      if (GATE) {
+        const f2 z = bf2(rz[i]), g = sigm2(z), l = mul2(z, g), om = fma2(g, dup(-1.f), dup(1.f));
+        float q0, q1;
+        up(mul2(mul2(dyv, bf2(ry[i])), fma2(l, om, g)), q0, q1);
+        const uint32_t q = tc05::pack_bf16(q0, q1);
+        if (FULL) {
+          *reinterpret_cast<uint32_t*>(qdz + i * dzs) = q;
+        } else {
+          if (row && live0) qdz[i * dzs] = (u16)q;
+          if (row && live1) qdz[i * dzs + 1] = (u16)(q >> 16);
+        }
+        dyv = mul2(dyv, l);
+      }
+      f2 dl, sg = dup(1.f);
+      if (RAW) {
+        softplus2(bf2(rd[i]), dl, sg);
+        if (!FULL) {
+          float d0_, d1_;
+          up(dl, d0_, d1_);
+          dl = pk(row && live0 ? d0_ : 0.f, row && live1 ? d1_ : 0.f);
+        }
+      } else {
+        dl = rf[i];
+      }
+      *reinterpret_cast<f2*>(&s.dl[t][sc]) = dl;
+      *reinterpret_cast<f2*>(&s.sg[t][sc]) = sg;
+      *reinterpret_cast<f2*>(&s.u[t][sc]) = uv;
+      *reinterpret_cast<f2*>(&s.dy[t][sc]) = dyv;
+      dDa = fma2(dyv, uv, dDa);
+    }
+  };
+
+#pragma unroll 1
   for (int seg = (len - 1) / SEG; seg >= 0; --seg) {
     const int tb = seg * SEG;
     __syncthreads();
-    // a thread stages one channel of eight steps; all of its loads go out first, the kept states' with them
-    const float* hs = st + ((long long)c * NSEG + seg) * N * a.DiP + dc;
-    float2 hv[4];
+    const float* hs = st + ((long long)c * NSEG + seg) * N * a.DiP + d0;
 #pragma unroll
-    for (int p = 0; p < 4; ++p) hv[p] = __ldg(reinterpret_cast<const float2*>(hs + (q * 4 + p) * a.DiP));
-    {
-      constexpr int NT = SEG * BC / BT;
-      typename DeltaCol<RAW>::T rd[NT];
-      u16 ru[NT], ro[NT], rz[NT], ry[NT];
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        const int r = tb + i * (BT / BC) + st_t;
-        const bool ok = r < len && st_live;
-        rd[i] = delta(r, ok);
-        ru[i] = ucol(r, ok);
-        ro[i] = ocol(r, ok);
-        if (GATE) {
-          rz[i] = zcol(r, ok);
-          ry[i] = ycol(r, ok);
-        }
-      }
-#pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        const int t = i * (BT / BC) + st_t, r = tb + t;
-        const bool ok = r < len && st_live;
-        const float dlv = DeltaCol<RAW>::value(rd[i], ok), uv = bf(ru[i]);
-        float dyv = bf(ro[i]);
-        if (GATE) {
-          const float z = bf(rz[i]), sg = sigm(z), sl = z * sg;
-          if (ok) pdz[r * dzs] = __float2bfloat16(dyv * bf(ry[i]) * (sg + sl * (1.f - sg)));
-          dyv *= sl;
-        }
-        reinterpret_cast<float2*>(&s.dl[t][0])[st_ch] = make_float2(dlv, dlv);
-        reinterpret_cast<float2*>(&s.x[t][0])[st_ch] = make_float2(dlv * uv, dlv * uv);
-        reinterpret_cast<float2*>(&s.dy[t][0])[st_ch] = make_float2(dyv, dyv);
-      }
-    }
+      for (int k = 0; k < 4; ++k) h[j][k] = __ldg(reinterpret_cast<const f2*>(hs + nn[k] * a.DiP + ch[j]));
+    if (vec && tb + SEG <= len) stage(std::true_type(), tb);
+    else stage(std::false_type(), tb);
     for (int i = tid; i < SEG * N; i += BT) {
       const int t = i / N, n = i % N;
       const bool ok = tb + t < len;
-      s.B[t][n] = ok ? load_bc(a, a.B, a.bs, row0 + tb + t, n) : 0.f;
-      s.C[t][n] = ok ? load_bc(a, a.C, a.cs, row0 + tb + t, n) : 0.f;
-    }
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      h[0][p] = pk(hv[2 * p].x, hv[2 * p + 1].x);
-      h[1][p] = pk(hv[2 * p].y, hv[2 * p + 1].y);
+      const float b = ok ? load_bc(a, a.B, a.bs, row0 + tb + t, n) : 0.f, cc = ok ? load_bc(a, a.C, a.cs, row0 + tb + t, n) : 0.f;
+      s.B[t][n] = make_float2(b, b);
+      s.C[t][n] = make_float2(cc, cc);
     }
     __syncthreads();
     // states entering steps 4, 8, 12
+#pragma unroll 1
+    for (int sb = 0; sb < SEG / G - 1; ++sb) {
 #pragma unroll
-    for (int sb = 0; sb < 3; ++sb) {
-      *reinterpret_cast<F4*>(&s.ck[sb][0][tid]) = F4{h[0][0], h[0][1]};
-      *reinterpret_cast<F4*>(&s.ck[sb][1][tid]) = F4{h[1][0], h[1][1]};
+      for (int e = 0; e < 8; ++e) s.ck[sb][e][tid] = h[e >> 2][e & 3];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = sb * 4 + i;
-        const F4 b = *reinterpret_cast<const F4*>(&s.B[t][q * 4]);
-        const F4 dl = *reinterpret_cast<const F4*>(&s.dl[t][cp]), x = *reinterpret_cast<const F4*>(&s.x[t][cp]);
-        h[0][0] = fma2(ex2v(mul2(dl.a, A2[0][0])), h[0][0], mul2(x.a, b.a));
-        h[0][1] = fma2(ex2v(mul2(dl.a, A2[0][1])), h[0][1], mul2(x.a, b.b));
-        h[1][0] = fma2(ex2v(mul2(dl.b, A2[1][0])), h[1][0], mul2(x.b, b.a));
-        h[1][1] = fma2(ex2v(mul2(dl.b, A2[1][1])), h[1][1], mul2(x.b, b.b));
+      for (int i = 0; i < G; ++i) {
+        const int t = sb * G + i;
+        f2 bb[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) bb[k] = lds2(&s.B[t][nn[k]]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const f2 dl = lds2(&s.dl[t][ch[j]]), x = mul2(dl, lds2(&s.u[t][ch[j]]));
+#pragma unroll
+          for (int k = 0; k < 4; ++k) h[j][k] = fma2(ex2v(mul2(dl, A2[j][k])), h[j][k], mul2(x, bb[k]));
+        }
       }
     }
 #pragma unroll 1
-    for (int sb = 3; sb >= 0; --sb) {
-      if (sb < 3) {
-        const F4 k0 = *reinterpret_cast<const F4*>(&s.ck[sb][0][tid]), k1 = *reinterpret_cast<const F4*>(&s.ck[sb][1][tid]);
-        h[0][0] = k0.a, h[0][1] = k0.b, h[1][0] = k1.a, h[1][1] = k1.b;
+    for (int sb = SEG / G - 1; sb >= 0; --sb) {
+      if (sb < SEG / G - 1) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) h[e >> 2][e & 3] = s.ck[sb][e][tid];
       }
-      // what the finishing lanes need of u and raw, on its way while the states are recomputed
-      const int ft = tb + sb * 4 + (lane >> 3);
-      const bool f0 = ft < len && fd < a.Di, f1 = ft < len && fd + 1 < a.Di;
-      const u16 fu0 = fu(ft, f0), fu1 = f1 ? __ldg(fu.p + ft * fu.stride + 1) : (u16)0;
-      u16 fr0 = 0, fr1 = 0;
-      if constexpr (RAW) {
-        fr0 = fdelta(ft, f0);
-        fr1 = f1 ? __ldg(fdelta.c.p + ft * fdelta.c.stride + 1) : (u16)0;
-      }
-      f2 dec[4][2][2], w[4][2][2];
+      // decay of a step and the state before it: 32 columns of tensor memory a step, a lane a thread
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int t = sb * 4 + i;
-        const F4 b = *reinterpret_cast<const F4*>(&s.B[t][q * 4]);
-        const F4 dl = *reinterpret_cast<const F4*>(&s.dl[t][cp]), x = *reinterpret_cast<const F4*>(&s.x[t][cp]);
+      for (int i = 0; i < G; ++i) {
+        const int t = sb * G + i;
+        union { f2 p[2][2][4]; uint32_t r[32]; } hist;
+        f2 bb[4], xb[2][4];
 #pragma unroll
-        for (int k = 0; k < 2; ++k)
+        for (int k = 0; k < 4; ++k) bb[k] = lds2(&s.B[t][nn[k]]);
 #pragma unroll
-          for (int p = 0; p < 2; ++p) {
-            dec[i][k][p] = ex2v(mul2(k ? dl.b : dl.a, A2[k][p]));
-            w[i][k][p] = mul2(dec[i][k][p], h[k][p]);
-            h[k][p] = fma2(k ? x.b : x.a, p ? b.b : b.a, w[i][k][p]);
+        for (int j = 0; j < 2; ++j) {
+          const f2 dl = lds2(&s.dl[t][ch[j]]), x = mul2(dl, lds2(&s.u[t][ch[j]]));
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            hist.p[1][j][k] = h[j][k];
+            hist.p[0][j][k] = ex2v(mul2(dl, A2[j][k]));
+            xb[j][k] = mul2(x, bb[k]);
           }
-      }
-      __syncwarp();  // the previous four steps' sums have been read
-#pragma unroll
-      for (int i = 3; i >= 0; --i) {
-        const int t = sb * 4 + i;
-        const F4 b = *reinterpret_cast<const F4*>(&s.B[t][q * 4]), cc = *reinterpret_cast<const F4*>(&s.C[t][q * 4]);
-        const F4 dl = *reinterpret_cast<const F4*>(&s.dl[t][cp]), x = *reinterpret_cast<const F4*>(&s.x[t][cp]);
-        const F4 dy = *reinterpret_cast<const F4*>(&s.dy[t][cp]);
-        f2 s1[2], s2[2], vb[2], vc[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k)
-#pragma unroll
-          for (int p = 0; p < 2; ++p) {
-            const f2 bb = p ? b.b : b.a, xx = k ? x.b : x.a, dd = k ? dl.b : dl.a, yy = k ? dy.b : dy.a;
-            const f2 g = fma2(p ? cc.b : cc.a, yy, carry[k][p]);
-            const f2 ht = fma2(xx, bb, w[i][k][p]);
-            const f2 gw = mul2(g, w[i][k][p]);
-            vb[p] = k ? fma2(g, xx, vb[p]) : mul2(g, xx);
-            vc[p] = k ? fma2(ht, yy, vc[p]) : mul2(ht, yy);
-            s1[k] = p ? fma2(gw, A2[k][p], s1[k]) : mul2(gw, A2[k][p]);
-            s2[k] = p ? fma2(g, bb, s2[k]) : mul2(g, bb);
-            dAa[k][p] = fma2(gw, dd, dAa[k][p]);
-            carry[k][p] = mul2(dec[i][k][p], g);
-          }
-        float4* r = s.red[warp] + i * 3 * RROW + lane;
-        r[0] = make_float4(sum2(s1[0]), sum2(s2[0]), sum2(s1[1]), sum2(s2[1]));
-        *reinterpret_cast<F4*>(r + RROW) = F4{vb[0], vb[1]};
-        *reinterpret_cast<F4*>(r + 2 * RROW) = F4{vc[0], vc[1]};
-      }
-      __syncwarp();
-      {
-        // over the four state quads; the order of the quads is rotated per lane so that eight lanes read eight banks groups
-        const int i = lane >> 3, g8 = lane & 7, t = sb * 4 + i;
-        const F4* r = reinterpret_cast<const F4*>(s.red[warp] + i * 3 * RROW + g8 * 4);
-        F4 v = r[(g8 >> 1) & 3];
-#pragma unroll
-        for (int k = 1; k < 4; ++k) {
-          const F4 o = r[(k + (g8 >> 1)) & 3];
-          v.a = add2(v.a, o.a);
-          v.b = add2(v.b, o.b);
         }
-        if (tb + t < len) {
-          const long long row = row0 + tb + t;
-          const F4 dl = *reinterpret_cast<const F4*>(&s.dl[t][fcp]), dy = *reinterpret_cast<const F4*>(&s.dy[t][fcp]);
-          float dlv[2], dyv[2], tmp, m1[2], m2[2];
-          up(dl.a, dlv[0], tmp), up(dl.b, dlv[1], tmp);
-          up(dy.a, dyv[0], tmp), up(dy.b, dyv[1], tmp);
-          up(v.a, m1[0], m2[0]), up(v.b, m1[1], m2[1]);
+        tc05::tmem_st_32x32(taddr + i * 32, hist.r);
 #pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const int d = fd + k;
-            if (d < a.Di) {
-              const float uv = bf(k ? fu1 : fu0);
-              float dd = fmaf(uv, m2[k], m1[k] * LN2);
-              du[row * a.Di + d] = __float2bfloat16(fmaf(k ? D1 : D0, dyv[k], dlv[k] * m2[k]));
-              if (RAW) {
-                dd *= sigm(bf(k ? fr1 : fr0));
-                ((__nv_bfloat16*)ddl)[row * a.Di + d] = __float2bfloat16(dd);
-              } else {
-                ((float*)ddl)[row * a.Di + d] = dd;
-              }
-              if (k) dD1 = fmaf(dyv[k], uv, dD1);
-              else dD0 = fmaf(dyv[k], uv, dD0);
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) h[j][k] = fma2(hist.p[0][j][k], h[j][k], xb[j][k]);
+      }
+      tc05::tmem_st_wait();
+      // back through the four steps.  A step's sums over lanes are formed while the next step's operands are on their way; dC of a
+      // step is formed a step late, when the state after it (the next one's state before) has been fetched.
+      union { f2 p[2][2][4]; uint32_t r[32]; } hist;
+      f2 bb[4], cc[4], dl[2], uu[2], dy[2];
+      float vc3[4];                          // the group's last step's
+      f2 val[G];
+      auto fetch = [&](int i) {
+        const int t = sb * G + i;
+        tc05::tmem_ld_32x32(taddr + i * 32, hist.r);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          bb[k] = lds2(&s.B[t][nn[k]]);
+          cc[k] = lds2(&s.C[t][nn[k]]);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          dl[j] = lds2(&s.dl[t][ch[j]]);
+          uu[j] = lds2(&s.u[t][ch[j]]);
+        }
+      };
+#pragma unroll
+      for (int j = 0; j < 2; ++j) dy[j] = lds2(&s.dy[sb * G + G - 1][ch[j]]);
+      fetch(G - 1);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) vc3[k] = sum2(fma2(h[1][k], dy[1], mul2(h[0][k], dy[0])));
+#pragma unroll
+      for (int i = G - 1; i >= 0; --i) {
+        const int t = sb * G + i;
+        f2 vb[4], s1[2], s2[2], dyb[2];
+        float vc[4];
+        if (i > 0) {
+#pragma unroll
+          for (int j = 0; j < 2; ++j) dyb[j] = lds2(&s.dy[t - 1][ch[j]]);
+        }
+        const f2 fac = lds2(ffac + t * BC), dyf = lds2(&s.dy[t][fch]);
+        tc05::tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const f2 x = mul2(dl[j], uu[j]);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const f2 g = fma2(cc[k], dy[j], carry[j][k]);
+            vb[k] = j ? fma2(g, x, vb[k]) : mul2(g, x);
+            s2[j] = k ? fma2(g, bb[k], s2[j]) : mul2(g, bb[k]);
+            carry[j][k] = mul2(hist.p[0][j][k], g);
+            const f2 gw = mul2(carry[j][k], hist.p[1][j][k]);
+            s1[j] = k ? fma2(gw, A2[j][k], s1[j]) : mul2(gw, A2[j][k]);
+            dAa[j][k] = fma2(gw, dl[j], dAa[j][k]);
+          }
+          s1[j] = fma2(uu[j], s2[j], mul2(s1[j], ln2));
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) vc[k] = i > 0 ? sum2(fma2(hist.p[1][1][k], dyb[1], mul2(hist.p[1][0][k], dyb[0]))) : vc3[k];
+        if (i > 0) {
+          dy[0] = dyb[0], dy[1] = dyb[1];
+          fetch(i - 1);
+        }
+        // over the channels: states by bits 1 and 0 of cg, dB or dC by bit 2
+        float b0 = sum2(vb[0]) + shx(sum2(vb[2]), 8), b1 = sum2(vb[1]) + shx(sum2(vb[3]), 8);
+        float c0 = vc[0] + shx(vc[2], 8), c1 = vc[1] + shx(vc[3], 8);
+        b0 += shx(b1, 4);
+        c0 += shx(c1, 4);
+        // over the states: channel pair by bit 1 of q, ddelta or du by bit 0
+        float e0, e1, f0, f1, x0, x1;
+        up(s1[1], x0, x1);
+        up(add2(s1[0], pk(shx(x0, 2), shx(x1, 2))), e0, e1);
+        up(s2[1], x0, x1);
+        up(add2(s2[0], pk(shx(x0, 2), shx(x1, 2))), f0, f1);
+        s.bc[warp][hi ? (i > 0 ? t - 1 : sb * G + G - 1) : t][(hi ? N : 0) + nn[0]] = (hi ? c0 : b0) + shx(hi ? b0 : c0, 16);
+        const f2 got = pk(shx(is_du ? e0 : f0, 1), shx(is_du ? e1 : f1, 1));
+        val[i] = fma2(add2(pk(is_du ? f0 : e0, is_du ? f1 : e1), got), fac, mul2(Df, dyf));
+      }
+      if (RAW) {  // the place of the pair's factor, which this group has read, takes both results
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+          float v0, v1;
+          up(val[i], v0, v1);
+          reinterpret_cast<uint32_t*>(&s.sg[sb * G + i][fch])[is_du] = tc05::pack_bf16(v0, v1);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+          const int t = sb * G + i;
+          const long long o = (row0 + tb + t) * a.Di + fd;
+          float v0, v1;
+          up(val[i], v0, v1);
+          if (tb + t < len) {
+            if (is_du) {
+              if (fd < a.Di) du[o] = __float2bfloat16(v0);
+              if (fd + 1 < a.Di) du[o + 1] = __float2bfloat16(v1);
+            } else {
+              if (fd < a.Di) ((float*)ddl)[o] = v0;
+              if (fd + 1 < a.Di) ((float*)ddl)[o + 1] = v1;
             }
           }
         }
       }
-      {
-        // over the eight channel pairs
-        const int i = lane >> 3, k = (lane >> 2) & 1, q8 = lane & 3;
-        const F4* r = reinterpret_cast<const F4*>(s.red[warp] + (i * 3 + 1 + k) * RROW + q8);
-        F4 v = r[0];
-#pragma unroll
-        for (int g = 1; g < 8; ++g) {
-          v.a = add2(v.a, r[g * 4].a);
-          v.b = add2(v.b, r[g * 4].b);
-        }
-        *reinterpret_cast<F4*>(&s.bc[warp][sb * 4 + i][k * N + q8 * 4]) = v;
-      }
     }
     __syncthreads();
+    if (RAW) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int t = st0 + i, r = tb + t;
+        const uint2 v = *reinterpret_cast<const uint2*>(&s.sg[t][sc]);  // ddelta, du
+        u16 *p0 = pdd + r * a.Di, *p1 = pdu + r * a.Di;
+        if (r < len && live0) {
+          if (even) {
+            *reinterpret_cast<uint32_t*>(p0) = v.x;
+            *reinterpret_cast<uint32_t*>(p1) = v.y;
+          } else {
+            p0[0] = (u16)v.x, p1[0] = (u16)v.y;
+            if (live1) p0[1] = (u16)(v.x >> 16), p1[1] = (u16)(v.y >> 16);
+          }
+        }
+      }
+    }
     for (int i = tid; i < SEG * 2 * N; i += BT) {
       const int t = i / (2 * N);
       if (tb + t < len) {
@@ -645,20 +781,20 @@ __global__ void __launch_bounds__(BT, 3) sscan_bwd_kernel(ScanArgs a, const __nv
   }
   // dA per chunk, dD per chunk: the caller adds the chunks up
 #pragma unroll
-  for (int p = 0; p < 2; ++p) {
-    float lo0, hi0, lo1, hi1;
-    up(dAa[0][p], lo0, hi0);
-    up(dAa[1][p], lo1, hi1);
-    float* o = dA + ((long long)c * N + q * 4 + 2 * p) * a.DiP + dc;
-    *reinterpret_cast<float2*>(o) = make_float2(lo0, lo1);
-    *reinterpret_cast<float2*>(o + a.DiP) = make_float2(hi0, hi1);
-  }
+  for (int j = 0; j < 2; ++j)
 #pragma unroll
-  for (int o = 8; o < 32; o <<= 1) {
-    dD0 += __shfl_xor_sync(0xffffffffu, dD0, o);
-    dD1 += __shfl_xor_sync(0xffffffffu, dD1, o);
+    for (int k = 0; k < 4; ++k) *reinterpret_cast<f2*>(dA + ((long long)c * N + nn[k]) * a.DiP + d0 + ch[j]) = dAa[j][k];
+  __syncthreads();
+  if (st0) *reinterpret_cast<f2*>(&s.dl[0][sc]) = dDa;
+  tc05::tc_fence_before();
+  __syncthreads();
+  if (!st0) {
+    *reinterpret_cast<f2*>(dD + (long long)c * a.DiP + sd) = add2(dDa, lds2(&s.dl[0][sc]));
   }
-  if (lane < 8) *reinterpret_cast<float2*>(dD + (long long)c * a.DiP + fd) = make_float2(dD0, dD1);
+  if (warp == 0) {
+    tc05::tc_fence_after();
+    tc05::tmem_dealloc(s.tmem, 32 * G);
+  }
 }
 
 // dB, dC: sum of the channel blocks' partials, written in the operands' type

@@ -351,6 +351,32 @@ def test_selective_scan_edges(Di, lens, gate):
         assert rel_err(a, b) < 1e-2
 
 
+def test_selective_scan_gate_and_softplus_far_out():
+    """Arguments where the sigmoids and the softplus saturate, underflow or vanish: finite results that match fp64 to 2^-7 of the largest value of
+    their kind (bf16 results of single steps)."""
+    from flame_b200.ops.scan import mamba_scan_gate
+    torch.manual_seed(8)
+    T, Di = 40, 130
+    meta = _meta([T])
+    far = torch.tensor([-300., -100., -88., -40., -10., -1e-3, 0., 1e-3, 10., 40., 88., 100., 300.], device=DEV)
+    pick = lambda: far[torch.randint(len(far), (T, Di), device=DEV)].to(torch.bfloat16).requires_grad_(True)  # noqa: E731
+    raw, z = pick(), pick()
+    u, B, C = (torch.randn(T, n, device=DEV, dtype=torch.bfloat16).requires_grad_(True) for n in (Di, 16, 16))
+    A, D = (-torch.rand(Di, 16, device=DEV)).requires_grad_(True), torch.randn(Di, device=DEV).requires_grad_(True)
+    ins, dy = [u, raw, B, C, z, A, D], torch.randn(T, Di, device=DEV, dtype=torch.bfloat16)
+    y = mamba_scan_gate(u, raw, A, B, C, D, z, meta)
+    got = [y.detach()] + list(torch.autograd.grad(y, ins, dy))
+    ud, rd, Bd, Cd, zd, Ad, Dd = ref_in = [t.detach().double().requires_grad_(True) for t in ins]
+    h, rows, dl = torch.zeros(Di, 16, device=DEV, dtype=torch.float64), [], F.softplus(rd)
+    for t in range(T):
+        h = h * (dl[t][:, None] * Ad).exp() + (dl[t] * ud[t])[:, None] * Bd[t][None]
+        rows.append((h * Cd[t][None]).sum(-1) + Dd * ud[t])
+    yr = torch.stack(rows) * F.silu(zd)
+    for a, b in zip(got, [yr.detach()] + list(torch.autograd.grad(yr, ref_in, dy.double()))):
+        assert torch.isfinite(a).all()
+        assert float((a.double() - b).abs().max()) < 2 ** -7 * float(b.abs().max())
+
+
 @pytest.mark.parametrize("gate", [False, True])
 def test_selective_scan_without_a_backward_keeps_one_state_a_chunk(gate):
     """Same output with gradients off, in the memory of the output, one fp32 state and one sum of steps per chunk (and 4 MB),
