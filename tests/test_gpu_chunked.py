@@ -524,6 +524,43 @@ def test_bgemm_result_boxes(M, N):
 
 
 @pytest.mark.parametrize("reverse", [False, True])
+@pytest.mark.parametrize("rows,cols,Ha,Hb,per_row", [(64, 64, 2, 2, True), (128, 64, 1, 6, False), (128, 192, 3, 3, True), (64, 320, 2, 1, False),
+                                                     (32, 64, 2, 2, True)])
+def test_decay_states_in_one_kernel(rows, cols, Ha, Hb, per_row, reverse):
+    """Increments and states of documents of one to nine chunks against the loop in fp64, heads shared on either side, operands as strided
+    blocks, one that lies between vectors, and a size that goes through product and scan.  fp32 sums of 64 products a chunk, a decay each
+    chunk, one rounding of the state (2^-9); the increments of (32, 64) going backwards are rounded too."""
+    from flame_b200.ops.chunked import ChunkLayout, _decay_states
+    torch.manual_seed(rows + cols)
+    lens, H = [1, 64, 65, 570], max(Ha, Hb)
+    lay = ChunkLayout(_meta(lens))
+    alpha = torch.rand(lay.NC, H, rows, device=DEV) if per_row else torch.rand(lay.NC, H, device=DEV)
+    wide = torch.randn(lay.NC, 64, Ha, rows + 8, device=DEV, dtype=torch.bfloat16)
+    a = wide[..., 8:].permute(0, 2, 1, 3)
+    odd = torch.randn(lay.NC * 64 * Hb * cols + 1, device=DEV, dtype=torch.bfloat16)
+    for b in (odd[:-1].view(lay.NC, 64, Hb, cols).permute(0, 2, 1, 3), odd[1:].view(lay.NC, Hb, 64, cols))[:1 if rows == 32 else 2]:
+        got = _decay_states(lay, alpha, a, b, reverse)
+        x = torch.einsum("nhtr,nhtc->nhrc", a.double().repeat_interleave(H // Ha, 1), b.double().repeat_interleave(H // Hb, 1))
+        want, c = torch.zeros(lay.NC, H, rows, cols, dtype=torch.float64, device=DEV), 0
+        al = alpha.double()[..., None] if per_row else alpha.double()[..., None, None]
+        for n in lens:
+            k = (n + 63) // 64
+            s = torch.zeros(H, rows, cols, dtype=torch.float64, device=DEV)
+            for i in (range(c + k - 1, c - 1, -1) if reverse else range(c, c + k)):
+                want[i] = s
+                s = al[i] * s + x[i]
+            c += k
+        assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + (0.2 if reverse and rows == 32 else 1e-4)).all()
+        if reverse:  # the decay's gradient on the way: fp32 sums of products of two bf16 states
+            S = torch.randn(lay.NC, H, rows, cols, device=DEV, dtype=torch.bfloat16)
+            again, dot = _decay_states(lay, alpha, a, b, reverse, S)
+            terms = got.double() * S.double()
+            dims = (-1,) if per_row else (-1, -2)
+            assert torch.equal(again, got) and dot.shape == alpha.shape
+            assert ((dot.double() - terms.sum(dims)).abs() <= 2.0 ** -18 * terms.abs().sum(dims)).all()
+
+
+@pytest.mark.parametrize("reverse", [False, True])
 @pytest.mark.parametrize("x16", [False, True])
 @pytest.mark.parametrize("rows,cols,per_row", [(3, 12, True), (4, 8, False), (16, 72, True)])
 def test_state_scan_widths(rows, cols, per_row, x16, reverse):
