@@ -16,7 +16,6 @@
 // works on the transposed score tile (see attn_bwd128_kernel).
 //
 // Takes the place of flash_attn_varlen_func as called by fla/layers/attn.py:146-174.
-#include "sb_math.cuh"
 #include "attn_tiles.cuh"
 #include "tc05.cuh"
 #include "host_utils.cuh"
@@ -43,9 +42,6 @@ struct AttnParams {
   float scale_log2;  // scale * log2(e)
   __nv_bfloat16* O;
   long long o_stride_t;
-  // Optional second output [T, H, Dh] (contiguous): the bf16 rounding of (O_fp32 - O), i.e. the low half of a two-term
-  // bf16 split of the fp32 result.  The stick-breaking backward needs do . o to fp32 accuracy (see sb_attention.cu).
-  __nv_bfloat16* O_lo;
   float* lse;  // [H, T] in log2 domain of the scaled logits
   int* status;
 };
@@ -90,10 +86,7 @@ struct FwdSmem {
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
-// MODE 0: softmax attention.  MODE 1: stick-breaking attention (strictly causal; key tiles are walked from the diagonal
-// backwards so that each row can carry the running sum of log(1 - sigmoid) over the keys already seen; weights never
-// exceed one, so there is no running maximum and O is never rescaled; `lse` receives the remainder 1 - sum_j att_ij).
-template <int DH, int MODE>
+template <int DH>
 __global__ void __launch_bounds__(192, 2)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                 const __grid_constant__ CUtensorMap tmV, AttnParams p) {
@@ -163,7 +156,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         const int slot = n % L::NSLOT;
         const uint32_t par = ((n / L::NSLOT) & 1) ^ 1;
         if (!mbar_wait(&empty_bar[slot], par, p.status, abort_flag, ERR_WAIT_EMPTY)) { ok = false; break; }
-        const int j = MODE == 0 ? j_start + (n >> 1) : j_end - (n >> 1);
+        const int j = j_start + (n >> 1);
         uint8_t* dst = smem + L::RING_OFF + slot * L::TILE_BYTES;
         mbar_expect_tx(&full_bar[slot], L::TILE_BYTES);
         const CUtensorMap* tm = (n & 1) ? &tmV : &tmK;
@@ -231,47 +224,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int q_idx = q0 + r;           // position inside the document
     const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
     uint8_t* sP = smem + L::P_OFF;
-    float m_run = MODE == 0 ? -INFINITY : 1.f;  // stale running max (log2 domain, scaled) / carried remainder product
+    float m_run = -INFINITY;  // stale running max (log2 domain, scaled)
     float l_run = 0.f;
     bool ok = true;
     for (int jj = 0; jj < nblk && ok; ++jj) {
-      const int kv0 = (MODE == 0 ? j_start + jj : j_end - jj) * BKV;
+      const int kv0 = (j_start + jj) * BKV;
       const bool mask_causal = (kv0 + BKV - 1 > q0);
       const bool mask_window = (p.window > 0) && (kv0 <= q0 + BQ - 1 - p.window);
       const bool need_mask = mask_causal || mask_window;
       if (!mbar_wait_warp(s_full, jj & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
-      if (MODE == 1) {
-        // stick-breaking: sigma = t / (1 + t) with t = 2^x, x the logit in log2 units; att_j = sigma_j * E_j with
-        // E_j = prod (1 - sigma) over the later keys of this row, carried from tile to tile (two MUFU ops per element,
-        // no logarithm).  The row is consumed in four 32-column pieces from the right.
-        const bool diag = (jj == 0);
-        if (jj > 0) {
-          if (!mbar_wait_warp(pv_done, (jj - 1) & 1, p.status, abort_flag, ERR_WAIT_MISC)) { ok = false; break; }
-          tc_fence_after();
-        }
-        float E = m_run;  // m_run doubles as the carried product (starts at 1 for this mode)
-        uint32_t xr[2][16];  // sixteen keys' logits, the next sixteen on their way
-        tmem_ld_32x16(tmem_S + lane_sel + BKV - 16, xr[0]);
-#pragma unroll 2
-        for (int h = 0; h < BKV / 16; ++h) {
-          const int c0 = BKV - 16 - h * 16;
-          tmem_ld_wait();
-          if (c0 > 0) tmem_ld_32x16(tmem_S + lane_sel + c0 - 16, xr[(h & 1) ^ 1]);
-#pragma unroll
-          for (int c = 8; c >= 0; c -= 8) {
-            sb2 e[4], sig[4];
-            if (diag) sb_group<true>(xr[h & 1] + c, p.scale_log2, sb_dead_bits(false, true, kv0 + c0 + c, q_idx), E, sig, e);
-            else sb_group<false>(xr[h & 1] + c, p.scale_log2, 0u, E, sig, e);
-            const uint4 q = make_uint4(sb_pack(e[0]), sb_pack(e[1]), sb_pack(e[2]), sb_pack(e[3]));
-            const int cc = c0 + c;
-            *reinterpret_cast<uint4*>(sP + (cc >> 6) * (BQ * 128) + sw128_offset(r, cc & 63)) = q;
-          }
-        }
-        m_run = E;
-        tc_fence_before();
-        mbar_arrive(s_free);
-      } else {
       // the whole score row moves to registers in one go, which frees S for the next tile right away
       uint32_t sr[BKV];
       tmem_ld_32x32(tmem_S + lane_sel + 0, *reinterpret_cast<uint32_t(*)[32]>(&sr[0]));
@@ -341,7 +303,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         *reinterpret_cast<uint4*>(sP + (c >> 6) * (BQ * 128) + sw128_offset(r, c & 63)) = q;
       }
       l_run += (l0 + l1) + (l2 + l3);
-      }
       tc_fence_before();
       fence_async_smem();
       mbar_arrive(p_ready);
@@ -350,7 +311,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     if (ok) {
       tc_fence_after();
       const bool valid = q_idx < doc_len;
-      const float inv_l = MODE == 0 ? (l_run > 0.f ? 1.f / l_run : 0.f) : 1.f;
+      const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
       const long long tok = (long long)doc_start + q_idx;
       __nv_bfloat16* orow = p.O + tok * p.o_stride_t + (long long)head * DH;
 #pragma unroll 1
@@ -367,21 +328,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
             q.z = pack_bf16(__uint_as_float(v[g * 8 + 4]) * inv_l, __uint_as_float(v[g * 8 + 5]) * inv_l);
             q.w = pack_bf16(__uint_as_float(v[g * 8 + 6]) * inv_l, __uint_as_float(v[g * 8 + 7]) * inv_l);
             *reinterpret_cast<uint4*>(orow + c + g * 8) = q;
-            if (MODE == 1 && p.O_lo != nullptr) {
-              const __nv_bfloat162* hi = reinterpret_cast<const __nv_bfloat162*>(&q);
-              uint4 lo;
-              uint32_t* lw = reinterpret_cast<uint32_t*>(&lo);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float2 h = __bfloat1622float2(hi[e]);
-                lw[e] = pack_bf16(__uint_as_float(v[g * 8 + 2 * e]) * inv_l - h.x, __uint_as_float(v[g * 8 + 2 * e + 1]) * inv_l - h.y);
-              }
-              *reinterpret_cast<uint4*>(p.O_lo + (tok * p.H + head) * DH + c + g * 8) = lo;
-            }
           }
         }
       }
-      if (valid) p.lse[(long long)head * p.total_tokens + tok] = MODE == 0 ? m_run + log2f(l_run) : m_run;
+      if (valid) p.lse[(long long)head * p.total_tokens + tok] = m_run + log2f(l_run);
     }
   }
   tc_fence_before();
@@ -395,7 +345,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 // ------------------------------------------------------------------------------------------------
 // forward, head dim 64, softmax mode, P in tensor memory
 // ------------------------------------------------------------------------------------------------
-// Same tiling and roles as attn_fwd_kernel<64, 0>, with two changes that take the probability tile off shared memory:
+// Same tiling and roles as attn_fwd_kernel<64>, with two changes that take the probability tile off shared memory:
 // (1) P is written as bf16 pairs into 64 TMEM columns and read from there as the A operand of O += P V, so a tile no
 //     longer costs 32 KB of shared-memory stores, a proxy fence and 32 KB of operand reads by the tensor core;
 // (2) P is handed over in two halves of 64 keys with a barrier pair each, so the PV product of the first half runs while
@@ -1528,7 +1478,6 @@ int fb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse
   p.scale_log2 = scale * kLog2e;
   p.O = (__nv_bfloat16*)o;
   p.o_stride_t = o_stride_t;
-  p.O_lo = nullptr;
   p.lse = lse;
   p.status = fb::status_ptr();
   const unsigned grid = (unsigned)max_tiles * H;
@@ -1542,49 +1491,14 @@ int fb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse
     attn_fwd_pt_kernel<<<grid, 192, FwdPtSmem::TOTAL, stream>>>(tmQ, tmK, tmV, p);
   } else if (DH == 64) {
     static bool done = false;
-    if (!done) { rc = set_smem(attn_fwd_kernel<64, 0>, FwdSmem<64>::TOTAL); if (rc) return rc; done = true; }
-    attn_fwd_kernel<64, 0><<<grid, 192, FwdSmem<64>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
+    if (!done) { rc = set_smem(attn_fwd_kernel<64>, FwdSmem<64>::TOTAL); if (rc) return rc; done = true; }
+    attn_fwd_kernel<64><<<grid, 192, FwdSmem<64>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
   } else {
     static bool done = false;
-    if (!done) { rc = set_smem(attn_fwd_kernel<128, 0>, FwdSmem<128>::TOTAL); if (rc) return rc; done = true; }
-    attn_fwd_kernel<128, 0><<<grid, 192, FwdSmem<128>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
+    if (!done) { rc = set_smem(attn_fwd_kernel<128>, FwdSmem<128>::TOTAL); if (rc) return rc; done = true; }
+    attn_fwd_kernel<128><<<grid, 192, FwdSmem<128>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
   }
   return fb::launch_ok("attn_fwd_kernel");
-}
-
-// Stick-breaking attention forward (head dim 64): o = sum_j att_ij v_j without normalisation, rem[h, t] = 1 - sum_j att_ij.
-// o_lo: optional bf16 [T, H, 64] that receives the part of the fp32 result the bf16 output lost (null: not written).
-int fb_sb_attn_fwd(const void* q, const void* k, const void* v, void* o, void* o_lo, float* rem, const int* cu_seqlens,
-                   const int* tile_list, int nseq, int max_tiles, long long T, int H, int DH, long long q_stride_t,
-                   long long k_stride_t, long long v_stride_t, long long o_stride_t, float scale, cudaStream_t stream) {
-  if (T == 0) return 0;
-  if (DH != 64) return -2;
-  if ((q_stride_t % 8) || (k_stride_t % 8) || (v_stride_t % 8) || (o_stride_t % 8)) return -3;
-  CUtensorMap tmQ, tmK, tmV;
-  int rc = make_qkv_map(&tmQ, q, T, H, DH, q_stride_t);
-  if (!rc) rc = make_qkv_map(&tmK, k, T, H, DH, k_stride_t);
-  if (!rc) rc = make_qkv_map(&tmV, v, T, H, DH, v_stride_t);
-  if (rc) return rc;
-  AttnParams p;
-  p.cu_seqlens = cu_seqlens;
-  p.tile_list = tile_list;
-  p.nseq = nseq;
-  p.H = H;
-  p.Hkv = H;
-  p.total_tokens = (int)T;
-  p.window = 0;
-  p.scale = scale;
-  p.scale_log2 = scale * kLog2e;
-  p.O = (__nv_bfloat16*)o;
-  p.o_stride_t = o_stride_t;
-  p.O_lo = (__nv_bfloat16*)o_lo;
-  p.lse = rem;
-  p.status = fb::status_ptr();
-  static bool done = false;
-  if (!done) { rc = set_smem(attn_fwd_kernel<64, 1>, FwdSmem<64>::TOTAL); if (rc) return rc; done = true; }
-  const unsigned grid = (unsigned)max_tiles * H;
-  attn_fwd_kernel<64, 1><<<grid, 192, FwdSmem<64>::TOTAL, stream>>>(tmQ, tmK, tmV, p);
-  return fb::launch_ok("attn_fwd_kernel<sb>");
 }
 
 int fb_attn_delta(const void* o, const void* dout, float* delta, long long T, int H, int DH, long long o_stride_t,

@@ -1,4 +1,4 @@
-// Stick-breaking attention backward for sm_100a (head dim 64), packed variable-length documents.
+// Stick-breaking attention for sm_100a (head dim 64), packed variable-length documents: backward, then forward.
 //
 //   att_ij = sigma_ij * prod_{j<m<i} (1 - sigma_im)   (j < i),   o_i = sum_j att_ij v_j,   rem_i = 1 - sum_j att_ij
 //   g_ij   = do_i . v_j - drem_i,   dA = att * g,   dl_ij = dA_ij - sigma_ij * sum_{k<=j} dA_ik
@@ -19,14 +19,17 @@
 // dS that is not finite would reach dV as 0 x dS; it is taken out of its tile, and dQ of its query and dK of its key become NaN.)  A
 // row of the accumulator is one channel of 64 keys, so 32 lanes hold 32 neighbouring floats of a key's gradient and add them
 // to global memory as they are (red.add, 128 bytes per instruction), without a staging tile.  S and dP of the next tile are
-// issued ahead of this tile's other products.  Eight rows of 4,096 tokens, 16 heads: 2.46 -> 2.02 ms (one CTA of
-// 128 x 128 tiles per SM).  The reference reaches the same sums with spin-locked adds
+// issued ahead of this tile's other products, and the weights of eight keys finished while the next eight's exponentials and
+// reciprocals run (one loop for masked tiles and one for the others: with both in one the compiler kept the parts apart, 2.18 ms).
+// Eight rows of 4,096 tokens, 16 heads: 2.46 ms with one CTA of 128 x 128 tiles per SM, 2.03 with two, 1.94 with the eights
+// interleaved, 1.90 with one reciprocal for two keys.  The reference reaches the same sums with spin-locked adds
 // (custom_models/sba/stickbreaking_attention/sb_varlen/sb_varlen_bwd.py:13-52); here nothing spins unbounded.
 #include "attn_tiles.cuh"
 #include "sb_math.cuh"
 #include "tc05.cuh"
 #include "host_utils.cuh"
 #include <math.h>
+#include <type_traits>
 
 using namespace tc05;
 
@@ -232,30 +235,44 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const bool diag = kv0 + BKV > q0;
       if (!mbar_wait_warp(sdp_full, it & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
       tc_fence_after();
+      auto walk = [&](auto mask) -> bool {
+      constexpr bool MASK = decltype(mask)::value;
       uint32_t xr[2][8], dr[2][8];  // a group's logits and dP, the next group's on their way
+      sb2 nsig_n[4];
+      float ninv_n[8];
+      auto sigma = [&](int g, const uint32_t* x) {
+        const int c = BKV - 8 - g * 8;
+        sb_sigma<MASK>(x, p.scale_log2, MASK ? sb_dead_bits(!valid, diag, kv0 + c, q_idx) : 0u, nsig_n, ninv_n);
+      };
       tmem_ld_32x8(tmem_S + lane_sel + BKV - 8, xr[0]);
+      tmem_ld_wait();
+      tmem_ld_32x8(tmem_S + lane_sel + BKV - 16, xr[1]);
       tmem_ld_32x8(tmem_dP + lane_sel + BKV - 8, dr[0]);
+      sigma(0, xr[0]);
       // the previous tile's products have read P and dS
-      if (it > 0 && !mbar_wait_warp(dkv_full, (it - 1) & 1, p.status, abort_flag, ERR_WAIT_MISC)) { ok = false; break; }
+      if (it > 0 && !mbar_wait_warp(dkv_full, (it - 1) & 1, p.status, abort_flag, ERR_WAIT_MISC)) return false;
 #pragma unroll 2
       for (int g = 0; g < BKV / 8; ++g) {
         const int c = BKV - 8 - g * 8;
         tmem_ld_wait();
-        uint32_t(&x)[8] = xr[g & 1];
         uint32_t(&dp)[8] = dr[g & 1];
-        if (c > 0) {
-          tmem_ld_32x8(tmem_S + lane_sel + c - 8, xr[(g & 1) ^ 1]);
-          tmem_ld_32x8(tmem_dP + lane_sel + c - 8, dr[(g & 1) ^ 1]);
-        }
         sb2 nsig[4], a[4], d[4];
-        if (diag || ragged) {
+        float ninv[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) nsig[i] = nsig_n[i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ninv[i] = ninv_n[i];
+        if (c > 8) tmem_ld_32x8(tmem_S + lane_sel + c - 16, xr[g & 1]);
+        if (c > 0) {
+          tmem_ld_32x8(tmem_dP + lane_sel + c - 8, dr[(g & 1) ^ 1]);
+          sigma(g + 1, xr[(g & 1) ^ 1]);
+        }
+        sb_weights(E, nsig, ninv, a);
+        if (MASK) {
           const uint32_t dead = sb_dead_bits(!valid, diag, kv0 + c, q_idx);
-          sb_group<true>(x, p.scale_log2, dead, E, nsig, a);
 #pragma unroll
           for (int i = 0; i < 8; ++i)  // what stands in another document's rows does not count, whatever it is
             if ((dead >> i) & 1u) dp[i] = 0u;
-        } else {
-          sb_group<false>(x, p.scale_log2, 0u, E, nsig, a);
         }
         const uint4 q = make_uint4(sb_pack(a[0]), sb_pack(a[1]), sb_pack(a[2]), sb_pack(a[3]));
         // The forward formed o from the bf16 rounding of att, and tot = do . o is the total the running sum of dA has to
@@ -280,6 +297,10 @@ sb_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         *reinterpret_cast<uint4*>(sDS + off) = make_uint4(sb_pack(d[0]), sb_pack(d[1]), sb_pack(d[2]), sb_pack(d[3]));
         size += fabsf(R);
       }
+      return true;
+      };
+      ok = diag || ragged ? walk(std::true_type()) : walk(std::false_type());
+      if (!ok) break;
       if (!(size < 1e38f))
         lost |= take_out_not_finite(sDS, r, doc_len - kv0, p.dK + (long long)(doc_start + kv0) * p.H * DH + head * DH, (long long)p.H * DH);
       tc_fence_before();
@@ -394,9 +415,274 @@ __global__ void sb_tot_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bf
   }
 }
 
+// ------------------------------------------------------------------------------------------------
+// forward
+// ------------------------------------------------------------------------------------------------
+//   o_i = sum_j att_ij v_j (att of the head of this file),   rem_i = 1 - sum_j att_ij = prod_j (1 - sigma_ij)
+//
+// One CTA per 128-query tile, two per SM, the keys from the diagonal backwards, 64 at a time, a thread per query row.  Weights
+// never exceed one, so there is no running maximum and the output is never rescaled.  What bounds it is the weight warps' chain
+// (special functions 61 % of their peak): the scores of the next tile and a second tile of weights are there, so that they
+// wait for no product, and the weights of eight keys are finished while the next eight's exponentials and reciprocals run.
+// Eight rows of 4,096 tokens, 16 heads: 128 keys at a time with one tile of scores and weights 1.00 ms, eights finished under the
+// next 0.94, two tiles of 64 keys 0.85 (and one reciprocal for two keys 0.80).
+struct FwdParams {
+  const int* cu_seqlens;
+  const int* tile_list;
+  int nseq, H, total_tokens;
+  float scale_log2;
+  __nv_bfloat16* O;
+  long long o_stride_t;
+  // Optional second output [T, H, DH] (contiguous): the bf16 rounding of (O_fp32 - O), i.e. the low half of a two-term
+  // bf16 split of the fp32 result.  The backward needs do . o to fp32 accuracy.
+  __nv_bfloat16* O_lo;
+  float* rem;  // [H, T]
+  int* status;
+};
+
+struct FwdSmem {
+  static constexpr int TILE = BQ * DH * 2;   // 16 KB
+  static constexpr int KV = BKV * DH * 2;    // 8 KB
+  static constexpr int NSLOT = 6;            // K and V tiles in turn
+  static constexpr int Q_OFF = 0, RING_OFF = TILE, P_OFF = RING_OFF + NSLOT * KV;
+  static constexpr int BAR_OFF = P_OFF + 2 * BQ * BKV * 2;
+  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+};
+
+__global__ void __launch_bounds__(192, 2)
+sb_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                   FwdParams p) {
+  using L = FwdSmem;
+  int head, doc, ti;
+  if (!attn_tile(p.tile_list, p.nseq, p.H, true, head, doc, ti)) return;
+  const int doc_start = p.cu_seqlens[doc];
+  const int doc_len = p.cu_seqlens[doc + 1] - doc_start;
+  const int q0 = ti * BQ;
+  const int n_iter = min((q0 + BQ) / BKV, (doc_len + BKV - 1) / BKV);  // key tiles n_iter - 1, ..., 0
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* full_bar = (uint64_t*)(smem + L::BAR_OFF);
+  uint64_t* empty_bar = full_bar + L::NSLOT;
+  uint64_t* q_full = empty_bar + L::NSLOT;
+  uint64_t* s_full = q_full + 1;    // [2] scores of a tile
+  uint64_t* p_ready = s_full + 2;   // [2] its weights, and its scores have been read
+  uint64_t* pv_done = p_ready + 2;  // [2] its product, which has read the weights
+  uint32_t* tmem_slot = (uint32_t*)(pv_done + 2);
+  volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < L::NSLOT; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    mbar_init(q_full, 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&s_full[b], 1);
+      mbar_init(&p_ready[b], 128);
+      mbar_init(&pv_done[b], 1);
+    }
+    *abort_flag = 0;
+    mbar_fence_init();
+    tma_prefetch_desc(&tmQ);
+    tma_prefetch_desc(&tmK);
+    tma_prefetch_desc(&tmV);
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 256);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_S = tmem_base, tmem_O = tmem_base + 2 * BKV;  // two tiles of scores
+
+  if (warp == 0) {
+    if (lane == 0) {
+      mbar_expect_tx(q_full, L::TILE);
+      tma_load_3d(smem + L::Q_OFF, &tmQ, q_full, 0, head, doc_start + q0);
+      // in the order in which the products take them: K 0, K 1, V 0, K 2, V 1, ..., the last V
+      for (int n = 0, k = 0, v = 0; n < 2 * n_iter; ++n) {
+        const bool is_k = k < n_iter && k <= v + 1;
+        const int row = doc_start + (n_iter - 1 - (is_k ? k++ : v++)) * BKV, slot = n % L::NSLOT;
+        if (!mbar_wait(&empty_bar[slot], ((n / L::NSLOT) & 1) ^ 1, p.status, abort_flag, ERR_WAIT_EMPTY)) break;
+        mbar_expect_tx(&full_bar[slot], L::KV);
+        tma_load_3d(smem + L::RING_OFF + slot * L::KV, is_k ? &tmK : &tmV, &full_bar[slot], 0, head, row);
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = make_idesc_bf16(BQ, BKV, 0, 0);
+      constexpr uint32_t idesc_o = make_idesc_bf16(BQ, DH, 0, 1);
+      const uint32_t sQ = smem_u32(smem + L::Q_OFF);
+      int n = 0;  // tiles taken from the ring
+      auto tile = [&](uint32_t& addr) -> uint64_t* {
+        const int slot = n % L::NSLOT;
+        if (!mbar_wait(&full_bar[slot], (n / L::NSLOT) & 1, p.status, abort_flag, ERR_WAIT_FULL)) return nullptr;
+        tc_fence_after();
+        ++n;
+        addr = smem_u32(smem + L::RING_OFF + slot * L::KV);
+        return &empty_bar[slot];
+      };
+      auto scores = [&](int it) -> bool {
+        uint32_t sK;
+        uint64_t* done = tile(sK);
+        if (!done) return false;
+        const uint64_t a = make_smem_desc(sQ, 16, 1024), b = make_smem_desc(sK, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < DH / 16; ++k)
+          mma_ss(tmem_S + (it & 1) * BKV, desc_advance(a, k * 32), desc_advance(b, k * 32), idesc_s, k ? 1u : 0u);
+        mma_commit(done);
+        mma_commit(&s_full[it & 1]);
+        return true;
+      };
+      bool ok = mbar_wait(q_full, 0, p.status, abort_flag, ERR_WAIT_FULL) && scores(0);
+      if (ok && n_iter > 1) ok = scores(1);
+      for (int it = 0; it < n_iter && ok; ++it) {
+        if (!mbar_wait(&p_ready[it & 1], (it >> 1) & 1, p.status, abort_flag, ERR_WAIT_MISC)) break;
+        tc_fence_after();
+        uint32_t sV;
+        uint64_t* done = tile(sV);
+        if (!done) break;
+        const uint64_t a = make_smem_desc(smem_u32(smem + L::P_OFF) + (it & 1) * (BQ * BKV * 2), 16, 1024), b = make_smem_desc(sV, 16, 1024);
+#pragma unroll
+        for (int k = 0; k < BKV / 16; ++k)
+          mma_ss(tmem_O, desc_advance(a, k * 32), desc_advance(b, k * 2048), idesc_o, (it > 0 || k > 0) ? 1u : 0u);
+        mma_commit(done);
+        mma_commit(&pv_done[it & 1]);
+        if (it + 2 < n_iter) ok = scores(it + 2);
+      }
+    }
+  } else {
+    const int quarter = warp & 3;
+    const int r = quarter * 32 + lane;
+    const int q_idx = q0 + r;
+    const uint32_t lane_sel = (uint32_t)(quarter * 32) << 16;
+    float E = 1.f;  // product of (1 - sigma) over the keys already seen
+    bool ok = true;
+    for (int it = 0; it < n_iter && ok; ++it) {
+      const int kv0 = (n_iter - 1 - it) * BKV;
+      const uint32_t t_s = tmem_S + (it & 1) * BKV + lane_sel;
+      uint8_t* sP = smem + L::P_OFF + (it & 1) * (BQ * BKV * 2);
+      if (!mbar_wait_warp(&s_full[it & 1], (it >> 1) & 1, p.status, abort_flag, ERR_WAIT_TMEM_FULL)) { ok = false; break; }
+      if (it > 1 && !mbar_wait_warp(&pv_done[it & 1], ((it >> 1) - 1) & 1, p.status, abort_flag, ERR_WAIT_MISC)) { ok = false; break; }
+      tc_fence_after();
+      auto walk = [&](auto mask) {
+        constexpr bool MASK = decltype(mask)::value;
+        uint32_t x[BKV];  // the row's scores, sixteen at a time from the right
+        sb2 nsig[4], att[4];
+        float ninv[8];
+        auto sigma = [&](int c) {
+          sb_sigma<MASK>(x + c, p.scale_log2, MASK ? sb_dead_bits(false, true, kv0 + c, q_idx) : 0u, nsig, ninv);
+        };
+        auto load = [&](int c) { tmem_ld_32x16(t_s + c, *reinterpret_cast<uint32_t(*)[16]>(&x[c])); };
+        load(BKV - 16);
+        tmem_ld_wait();
+        load(BKV - 32);
+        sigma(BKV - 8);
+#pragma unroll
+        for (int c = BKV - 8; c >= 0; c -= 8) {  // the weights of the eight keys at c
+          sb2 ns[4];
+          float ni[8];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) ns[i] = nsig[i];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) ni[i] = ninv[i];
+          if (c > 0) {
+            if (c % 16 == 0) {
+              tmem_ld_wait();
+              if (c > 16) load(c - 32);
+            }
+            sigma(c - 8);
+          }
+          sb_weights(E, ns, ni, att);
+          *reinterpret_cast<uint4*>(sP + sw128_offset(r, c)) = make_uint4(sb_pack(att[0]), sb_pack(att[1]), sb_pack(att[2]), sb_pack(att[3]));
+        }
+      };
+      if (kv0 + BKV > q0) walk(std::true_type());
+      else walk(std::false_type());
+      tc_fence_before();
+      fence_async_smem();
+      mbar_arrive(&p_ready[it & 1]);
+    }
+    if (ok) ok = mbar_wait_warp(&pv_done[(n_iter - 1) & 1], ((n_iter - 1) >> 1) & 1, p.status, abort_flag, ERR_WAIT_MISC);
+    if (ok) {
+      tc_fence_after();
+      const bool valid = q_idx < doc_len;
+      const long long tok = (long long)doc_start + q_idx;
+      __nv_bfloat16* orow = p.O + tok * p.o_stride_t + (long long)head * DH;
+#pragma unroll 1
+      for (int c = 0; c < DH; c += 32) {
+        uint32_t v[32];
+        tmem_ld_32x32(tmem_O + lane_sel + c, v);
+        tmem_ld_wait();
+        if (!valid) continue;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+          uint4 q, lo;
+          uint32_t *qw = reinterpret_cast<uint32_t*>(&q), *lw = reinterpret_cast<uint32_t*>(&lo);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float v0 = __uint_as_float(v[g * 8 + 2 * e]), v1 = __uint_as_float(v[g * 8 + 2 * e + 1]);
+            qw[e] = pack_bf16(v0, v1);
+            lw[e] = pack_bf16(v0 - __uint_as_float(qw[e] << 16), v1 - __uint_as_float(qw[e] & 0xffff0000u));
+          }
+          *reinterpret_cast<uint4*>(orow + c + g * 8) = q;
+          if (p.O_lo != nullptr) *reinterpret_cast<uint4*>(p.O_lo + (tok * p.H + head) * DH + c + g * 8) = lo;
+        }
+      }
+      if (valid) p.rem[(long long)head * p.total_tokens + tok] = E;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 256);
+  }
+}
+
+// dims (inner to outer): [DH, H, T]; box [64, 1, rows]
+int make_map(CUtensorMap* m, const void* base, long long T, int H, long long stride, uint32_t rows) {
+  return fb::make_tmap_3d(m, base, 2, (uint64_t)T, (uint64_t)H, (uint64_t)DH, (uint64_t)stride, (uint64_t)DH, rows, 1, 64, true);
+}
+
 }  // namespace
 
 extern "C" {
+
+// o = sum_j att_ij v_j without normalisation (head dim 64), rem[h, t] = 1 - sum_j att_ij.
+// o_lo: optional bf16 [T, H, 64] that receives the part of the fp32 result the bf16 output lost (null: not written).
+int fb_sb_attn_fwd(const void* q, const void* k, const void* v, void* o, void* o_lo, float* rem, const int* cu_seqlens,
+                   const int* tile_list, int nseq, int max_tiles, long long T, int H, int dh, long long q_stride_t,
+                   long long k_stride_t, long long v_stride_t, long long o_stride_t, float scale, cudaStream_t stream) {
+  if (T == 0) return 0;
+  if (dh != DH) return -2;
+  if ((q_stride_t % 8) || (k_stride_t % 8) || (v_stride_t % 8) || (o_stride_t % 8)) return -3;
+  CUtensorMap tmQ, tmK, tmV;
+  int rc = make_map(&tmQ, q, T, H, q_stride_t, BQ);
+  if (!rc) rc = make_map(&tmK, k, T, H, k_stride_t, BKV);
+  if (!rc) rc = make_map(&tmV, v, T, H, v_stride_t, BKV);
+  if (rc) return rc;
+  FwdParams p;
+  p.cu_seqlens = cu_seqlens;
+  p.tile_list = tile_list;
+  p.nseq = nseq;
+  p.H = H;
+  p.total_tokens = (int)T;
+  p.scale_log2 = scale * kLog2e;
+  p.O = (__nv_bfloat16*)o;
+  p.o_stride_t = o_stride_t;
+  p.O_lo = (__nv_bfloat16*)o_lo;
+  p.rem = rem;
+  p.status = fb::status_ptr();
+  const cudaError_t e = cudaFuncSetAttribute(sb_attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FwdSmem::TOTAL);
+  if (e != cudaSuccess) return (int)e;
+  sb_attn_fwd_kernel<<<(unsigned)max_tiles * H, 192, FwdSmem::TOTAL, stream>>>(tmQ, tmK, tmV, p);
+  return fb::launch_ok("sb_attn_fwd_kernel");
+}
 
 // dk_acc, dv_acc: fp32 [T, H, 64], zero on entry (added to); dq: bf16 [T, H, 64] (token stride given).
 // tot: fp32 [H, T] scratch.  rem: fp32 [H, T] from the forward; drem may be null.  o_lo: the forward's second output
@@ -418,13 +704,10 @@ int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
     if (rc) return rc;
   }
   CUtensorMap tmQ, tmK, tmV, tmdO;
-  auto map = [&](CUtensorMap* m, const void* base, long long stride, uint32_t rows) {
-    return fb::make_tmap_3d(m, base, 2, (uint64_t)T, (uint64_t)H, (uint64_t)DH, (uint64_t)stride, (uint64_t)DH, rows, 1, 64, true);
-  };
-  int rc = map(&tmQ, q, q_stride_t, BQ);
-  if (!rc) rc = map(&tmK, k, k_stride_t, BKV);
-  if (!rc) rc = map(&tmV, v, v_stride_t, BKV);
-  if (!rc) rc = map(&tmdO, dout, do_stride_t, BQ);
+  int rc = make_map(&tmQ, q, T, H, q_stride_t, BQ);
+  if (!rc) rc = make_map(&tmK, k, T, H, k_stride_t, BKV);
+  if (!rc) rc = make_map(&tmV, v, T, H, v_stride_t, BKV);
+  if (!rc) rc = make_map(&tmdO, dout, T, H, do_stride_t, BQ);
   if (rc) return rc;
   SbBwdParams p;
   p.cu_seqlens = cu_seqlens;

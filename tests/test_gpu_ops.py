@@ -201,6 +201,29 @@ def test_stickbreaking_attention_forward_backward(lens, H):
     assert rel_err(v.grad, vf.grad) < 3e-2
 
 
+@pytest.mark.parametrize("size", [1.0, 6.0])
+def test_stickbreaking_attention_at_tile_edges_and_far_out(size):
+    """Documents around the 64-key and 128-query tiles against fp64, with logits of some units and of some forty (neighbours beyond 2^60 : 1,
+    where the weights are 0 or 1 and the kernels cut off): outputs and value gradients of bf16 weights and operands, 1e-2; gradients
+    through the logits, small differences of their sums, 3e-2 where the weights are not saturated, and finite."""
+    from flame_b200.ops.linear_attn import stickbreaking_reference
+    from flame_b200.ops.stickbreaking import sb_attention
+    torch.manual_seed(11)
+    lens, H = [1, 2, 63, 64, 65, 127, 128, 129, 191, 192, 193, 320], 2
+    meta, T = _meta(lens), sum(lens)
+    q, k, v = ((torch.randn(T, H, 64, device=DEV) * (size if i < 2 else 1)).bfloat16().requires_grad_(True) for i in range(3))
+    do, drem = torch.randn(T, H, 64, device=DEV).bfloat16(), None
+    o, rem = sb_attention(q, k, v, meta)
+    qd, kd, vd = (t.detach().double().requires_grad_(True) for t in (q, k, v))
+    od, remd = stickbreaking_reference(qd, kd, vd, meta)
+    drem = torch.randn_like(rem) * 0.3
+    torch.autograd.backward([o, rem], [do, drem])
+    torch.autograd.backward([od, remd], [do.double(), drem.double()])
+    assert rel_err(o, od) < 1e-2 and rel_err(v.grad, vd.grad) < 1e-2 and (rem - remd).abs().max().item() < 1e-5
+    for a, b in ((q, qd), (k, kd)):
+        assert torch.isfinite(a.grad).all() and (size > 1 or rel_err(a.grad, b.grad) < 3e-2)
+
+
 def test_short_conv_forward_backward():
     from flame_b200.ops import linear_attn as la
     from flame_b200.ops.conv import short_conv
