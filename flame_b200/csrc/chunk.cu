@@ -9,10 +9,30 @@
 
 namespace {
 
+__device__ __forceinline__ void unpack8f(const uint4& q, float (&f)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 t = __bfloat1622float2(h[i]);
+    f[2 * i] = t.x, f[2 * i + 1] = t.y;
+  }
+}
+__device__ __forceinline__ uint4 pack8f(const float (&f)[8]) {
+  uint4 q;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) reinterpret_cast<__nv_bfloat162*>(&q)[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
+  return q;
+}
+
 // T = (I + diag(beta) P)^-1 of the strictly lower-triangular score blocks P (the WY "solve" of the delta rule; the reference
 // does it by blockwise forward substitution in fla/ops/utils/solve_tril.py).  One 64-thread block per 64 x 64 diagonal block:
-// thread c solves (I + A) x = e_c by forward substitution with x in registers; every A element is a shared-memory
-// broadcast.  P: [n, C, C] fp32, C = 64 or 128; T: [n, C, C] bf16.
+// thread c solves (I + A) x = e_c by forward substitution, 16 rows at a time: what the rows before contribute is sixteen sums
+// side by side, A in 16-byte broadcasts from shared memory, then the 16 x 16 corner in registers.  Warp 1 skips the zeros that
+// its columns have above row 32, and T is written in 16-byte vectors over the rows of A that are done with (more shared memory
+// than the 16 KB of A costs resident blocks: with T beside it the gated form took 72 us instead of 32).  Written out over all 64
+// rows it was one chain of 2,016 multiply-adds and as many reads: 150 us at 65,536 tokens, 8 heads of 128, where the bytes take
+// 41; this takes 89, in the same order of operations.
+// P: [n, C, C] fp32, C = 64 or 128; T: [n, C, C] bf16.
 //   C = 64:  also Tu = T diag(beta) and (b given) Tw = T diag(beta e^b), the matrices the values and keys are multiplied with,
 //            which used to be passes of their own over T
 //   C = 128: the two diagonal blocks of T, zeros above them, and A21 = the scaled lower-left block in bf16, from which two
@@ -21,51 +41,100 @@ namespace {
 __global__ void __launch_bounds__(64) delta_inverse_kernel(const float* __restrict__ P, const float* __restrict__ beta, const float* __restrict__ b,
                                                            int C, int H, __nv_bfloat16* __restrict__ T, __nv_bfloat16* __restrict__ Tu,
                                                            __nv_bfloat16* __restrict__ Tw, __nv_bfloat16* __restrict__ A21) {
-  __shared__ float sA[64 * 64];
+  __shared__ alignas(16) float sA[64 * 64];  // from the top down, the rows of A that are done with make room for those of T
+  __shared__ float sbeta[64], sw[64];
   const int halves = C >> 6;
   const long long m = blockIdx.x / halves;
   const int half = (int)(blockIdx.x - m * halves), ch = (int)(m / H), h = (int)(m - (long long)ch * H);
   const float* a = P + m * C * C + (long long)half * 64 * (C + 1);
-  auto beta_of = [&](int i) { return beta[((long long)ch * C + i) * H + h]; };
-  for (int i = threadIdx.x; i < 4096 / 4; i += 64) {
+  const int c = threadIdx.x;
+  const long long at = ((long long)ch * C + half * 64 + c) * H + h;
+  sbeta[c] = beta[at];
+  if (Tw != nullptr) sw[c] = sbeta[c] * __expf(b[at]);
+  __syncthreads();
+#pragma unroll 4
+  for (int i = c; i < 4096 / 4; i += 64) {
     const int r = i >> 4;
-    float4 v = *reinterpret_cast<const float4*>(a + (long long)r * C + (i & 15) * 4);
-    const float f = beta_of(half * 64 + r);
+    float4 v = __ldcs(reinterpret_cast<const float4*>(a + (long long)r * C + (i & 15) * 4));
+    const float f = sbeta[r];
     v.x *= f, v.y *= f, v.z *= f, v.w *= f;
     reinterpret_cast<float4*>(sA)[i] = v;
   }
   __syncthreads();
-  const int c = threadIdx.x;
-  float x[64];
+  const int first = c & 32;  // T is lower triangular: the second warp's columns are zero above row 32
+#pragma unroll 1
+  for (int I = 0; I < 64; I += 16) {
+    float s[16];
 #pragma unroll
-  for (int i = 0; i < 64; ++i) {
-    float s = (i == c) ? 1.f : 0.f;
+    for (int i = 0; i < 16; ++i) s[i] = I + i == c ? 1.f : 0.f;
+    const float4* row = reinterpret_cast<const float4*>(sA + I * 64);
+    if (I >= first) {
+#pragma unroll 1
+      for (int j = first; j < I; j += 4) {
+        float x[4];
 #pragma unroll
-    for (int j = 0; j < i; ++j) s = fmaf(-sA[i * 64 + j], x[j], s);
-    x[i] = s;
+        for (int k = 0; k < 4; ++k) x[k] = sA[(j + k) * 64 + c];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float4 v = row[i * 16 + j / 4];
+          s[i] = fmaf(-v.x, x[0], s[i]);
+          s[i] = fmaf(-v.y, x[1], s[i]);
+          s[i] = fmaf(-v.z, x[2], s[i]);
+          s[i] = fmaf(-v.w, x[3], s[i]);
+        }
+      }
+#pragma unroll
+      for (int i = 1; i < 16; ++i)
+#pragma unroll
+        for (int j = 0; j < i; j += 4) {
+          const float4 v = row[i * 16 + (I + j) / 4];
+          s[i] = fmaf(-v.x, s[j], s[i]);
+          if (j + 1 < i) s[i] = fmaf(-v.y, s[j + 1], s[i]);
+          if (j + 2 < i) s[i] = fmaf(-v.z, s[j + 2], s[i]);
+          if (j + 3 < i) s[i] = fmaf(-v.w, s[j + 3], s[i]);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) sA[(I + i) * 64 + c] = s[i];
   }
-  __nv_bfloat16* o = T + m * C * C + (long long)half * 64 * (C + 1) + c;
+  __syncthreads();
+  // out in vectors of eight columns
+  __nv_bfloat16* o = T + m * C * C + (long long)half * 64 * (C + 1);
+  const int v8 = (c & 7) * 8;
+#pragma unroll 2
+  for (int r = c >> 3; r < 64; r += 8) {
+    float x[8], y[8];
 #pragma unroll
-  for (int i = 0; i < 64; ++i) o[(long long)i * C] = __float2bfloat16(x[i]);
-  if (Tu != nullptr) {
-    const float f = beta_of(c);
-    __nv_bfloat16* u = Tu + m * 4096 + c;
+    for (int k = 0; k < 8; k += 4) *reinterpret_cast<float4*>(x + k) = *reinterpret_cast<const float4*>(sA + r * 64 + v8 + k);
+    *reinterpret_cast<uint4*>(o + (long long)r * C + v8) = pack8f(x);
+    if (Tu != nullptr) {
 #pragma unroll
-    for (int i = 0; i < 64; ++i) u[i * 64] = __float2bfloat16(x[i] * f);
-    if (Tw != nullptr) {
-      const float fw = f * __expf(b[((long long)ch * C + c) * H + h]);
-      __nv_bfloat16* w = Tw + m * 4096 + c;
+      for (int k = 0; k < 8; ++k) y[k] = x[k] * sbeta[v8 + k];
+      *reinterpret_cast<uint4*>(Tu + m * 4096 + r * 64 + v8) = pack8f(y);
+      if (Tw != nullptr) {
 #pragma unroll
-      for (int i = 0; i < 64; ++i) w[i * 64] = __float2bfloat16(x[i] * fw);
+        for (int k = 0; k < 8; ++k) y[k] = x[k] * sw[v8 + k];
+        *reinterpret_cast<uint4*>(Tw + m * 4096 + r * 64 + v8) = pack8f(y);
+      }
     }
   }
   if (C == 128) {
     if (half == 0) {
-      __nv_bfloat16* z = T + m * C * C + 64 + c;
-      for (int i = 0; i < 64; ++i) z[(long long)i * C] = __float2bfloat16(0.f);
+      __nv_bfloat16* z = T + m * C * C + 64 + v8;
+#pragma unroll
+      for (int r = c >> 3; r < 64; r += 8) *reinterpret_cast<uint4*>(z + (long long)r * C) = make_uint4(0, 0, 0, 0);
     } else {
-      const float* a21 = P + m * C * C + 64ll * C + c;
-      for (int i = 0; i < 64; ++i) A21[m * 4096 + i * 64 + c] = __float2bfloat16(a21[(long long)i * C] * beta_of(64 + i));
+      const float* a21 = P + m * C * C + 64ll * C + v8;
+#pragma unroll 4
+      for (int r = c >> 3; r < 64; r += 8) {
+        float x[8];
+#pragma unroll
+        for (int k = 0; k < 8; k += 4) *reinterpret_cast<float4*>(x + k) = __ldcs(reinterpret_cast<const float4*>(a21 + (long long)r * C + k));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) x[k] *= sbeta[r];
+        *reinterpret_cast<uint4*>(A21 + m * 4096 + r * 64 + v8) = pack8f(x);
+      }
     }
   }
 }
@@ -98,62 +167,67 @@ __global__ void __launch_bounds__(256) delta_scale_kernel(const __nv_bfloat16* _
   }
 }
 
-__device__ __forceinline__ void unpack8f(const uint4& q, float (&f)[8]) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 t = __bfloat1622float2(h[i]);
-    f[2 * i] = t.x, f[2 * i + 1] = t.y;
-  }
-}
-__device__ __forceinline__ uint4 pack8f(const float (&f)[8]) {
-  uint4 q;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) reinterpret_cast<__nv_bfloat162*>(&q)[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-  return q;
-}
-
 // Backward of Tu and Tw: dT = dTu diag(beta) + dTw diag(beta e^b) (bf16), and over the rows
 //   dbeta_j = scale sum_i T_ij (dTu_ij + e^{b_j} dTw_ij),   db_j = scale sum_i beta_j e^{b_j} T_ij dTw_ij      (written, not added).
 // dTw and b null: one matrix served both products.  One block of 256 threads per (chunk, head); a thread keeps eight
-// columns' sums over its rows in registers, so a row costs no atomics.
+// columns' sums over its rows in registers, so a row costs no atomics.  A thread has two (C = 64) or eight rows: their loads go
+// out two rows at a time, the first before the factors are fetched, and T above its diagonal is not read.  One row after the
+// other it waited for memory four times per block: 70 us at 65,536 tokens, 8 heads of 128 (the bytes take 26); this takes 40.
+template <int C, bool W>
 __global__ void __launch_bounds__(256) delta_bwd_t_kernel(const __nv_bfloat16* __restrict__ T, const __nv_bfloat16* __restrict__ dTu,
                                                           const __nv_bfloat16* __restrict__ dTw, const float* __restrict__ beta,
-                                                          const float* __restrict__ b, int C, int H, float scale, __nv_bfloat16* __restrict__ dT,
+                                                          const float* __restrict__ b, int H, float scale, __nv_bfloat16* __restrict__ dT,
                                                           float* __restrict__ dbeta, float* __restrict__ db) {
-  __shared__ float su[16][132], sw[16][132];
+  constexpr int nv = C / 8, groups = 256 / nv;  // 32 or 16 groups of rows
+  __shared__ float su[8][C + 4], sw[8][C + 4];
   const long long m = blockIdx.x;
   const int ch = (int)(m / H), h = (int)(m - (long long)ch * H);
-  const int nv = C >> 3, v = threadIdx.x % nv, r0 = threadIdx.x / nv, groups = 256 / nv;  // 32 or 16 groups of rows
+  const int v = threadIdx.x % nv, r0 = threadIdx.x / nv;
+  uint4 rt[2], ru[2], rw[2];
+  auto load = [&](int i0) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = i0 + u * groups;
+      const long long o = (m * C * C + (long long)i * C) / 8 + v;
+      rt[u] = v * 8 <= i ? __ldcs(reinterpret_cast<const uint4*>(T) + o) : make_uint4(0, 0, 0, 0);  // T is lower triangular
+      ru[u] = __ldcs(reinterpret_cast<const uint4*>(dTu) + o);
+      if constexpr (W) rw[u] = __ldcs(reinterpret_cast<const uint4*>(dTw) + o);
+    }
+  };
+  load(r0);
   float fu[8], fe[8], au[8], aw[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     const long long o = ((long long)ch * C + v * 8 + e) * H + h;
     fu[e] = beta[o];
-    fe[e] = b != nullptr ? __expf(b[o]) : 0.f;
+    if constexpr (W) fe[e] = __expf(b[o]);
     au[e] = aw[e] = 0.f;
   }
-  for (int i = r0; i < C; i += groups) {
-    const long long o = (m * C * C + (long long)i * C) / 8 + v;
-    float t[8], gu[8], gw[8];
-    unpack8f(reinterpret_cast<const uint4*>(T)[o], t);
-    unpack8f(reinterpret_cast<const uint4*>(dTu)[o], gu);
-    if (dTw != nullptr) unpack8f(reinterpret_cast<const uint4*>(dTw)[o], gw);
+#pragma unroll 1
+  for (int i0 = r0; i0 < C; i0 += 2 * groups) {
+    if (i0 != r0) load(i0);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      const float w = dTw != nullptr ? gw[e] * fe[e] : 0.f;
-      au[e] = fmaf(t[e], gu[e] + w, au[e]);
-      aw[e] = fmaf(t[e], w, aw[e]);
-      gu[e] = fu[e] * (gu[e] + w);
+    for (int u = 0; u < 2; ++u) {
+      float t[8], gu[8], gw[8];
+      unpack8f(rt[u], t);
+      unpack8f(ru[u], gu);
+      if constexpr (W) unpack8f(rw[u], gw);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float w = W ? gw[e] * fe[e] : 0.f;
+        au[e] = fmaf(t[e], gu[e] + w, au[e]);
+        if constexpr (W) aw[e] = fmaf(t[e], w, aw[e]);
+        gu[e] = fu[e] * (gu[e] + w);
+      }
+      reinterpret_cast<uint4*>(dT)[(m * C * C + (long long)(i0 + u * groups) * C) / 8 + v] = pack8f(gu);
     }
-    reinterpret_cast<uint4*>(dT)[o] = pack8f(gu);
   }
   // lanes of a warp hold the same columns for 32 / nv groups: add those by shuffle, the warps through shared memory
 #pragma unroll
   for (int e = 0; e < 8; ++e)
     for (int o = nv; o < 32; o <<= 1) {
       au[e] += __shfl_xor_sync(0xffffffffu, au[e], o);
-      aw[e] += __shfl_xor_sync(0xffffffffu, aw[e], o);
+      if constexpr (W) aw[e] += __shfl_xor_sync(0xffffffffu, aw[e], o);
     }
   const int warp = threadIdx.x >> 5;
   if ((threadIdx.x & 31) < nv) {
@@ -175,65 +249,105 @@ __global__ void __launch_bounds__(256) delta_bwd_t_kernel(const __nv_bfloat16* _
 //   g_ij  = beta_i dA_ij e^{b_i - b_j} [j < i],   gq_ij = q_scale dQ_ij e^{b_i - b_j} [j <= i]   (bf16 operands of the dq, dk products)
 //   dbeta_i += scale sum_j dA_ij P_ij,   db_i += scale (row sum_i - column sum_i) of beta dA P + dQ Q
 // dA, P fp32 (null: only the second block, for the scalar-gated attention without a delta rule); dQ, Q bf16 and b only with a
-// decay (without one the products' epilogues already give gq).
+// decay (without one the products' epilogues already give gq).  A, B: which of the two there are; one kernel for all three cases
+// held the registers of both (80 instead of 48), and with that two thirds of the warps.  Loads as in delta_bwd_t_kernel, and
+// nothing above the diagonal is read.  Before and after: 185 and 76 us (Q alone, 512 chunks of 64, 32 heads; the bytes take 45),
+// 85 and 54 us (A alone, 1,024 chunks of 64, 8 heads; 33), 69 and 46 us (both, 128 chunks of 128, 6 heads).
+template <int C, bool A, bool B>
 __global__ void __launch_bounds__(256) delta_bwd_scores_kernel(const float* __restrict__ dA, const float* __restrict__ P,
                                                                const __nv_bfloat16* __restrict__ dQ, const __nv_bfloat16* __restrict__ Q,
-                                                               const float* __restrict__ beta, const float* __restrict__ b, int C, int H, float scale,
+                                                               const float* __restrict__ beta, const float* __restrict__ b, int H, float scale,
                                                                float q_scale, __nv_bfloat16* __restrict__ g, __nv_bfloat16* __restrict__ gq,
                                                                float* __restrict__ dbeta, float* __restrict__ db) {
-  __shared__ float sb[128], srow[128], scol[8][132];
+  constexpr int nv = C / 8, groups = 256 / nv;
+  __shared__ float sb[C], sbeta[C], srow[C], scol[8][C + 4];
   const long long m = blockIdx.x;
   const int ch = (int)(m / H), h = (int)(m - (long long)ch * H);
-  for (int i = threadIdx.x; i < C; i += 256) sb[i] = b != nullptr ? b[((long long)ch * C + i) * H + h] : 0.f;
+  const int v = threadIdx.x % nv, r0 = threadIdx.x / nv;
+  float4 da[2][2], pp[2][2];
+  uint4 dq[2], qq[2];
+  auto load = [&](int i0) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      const int i = i0 + u * groups;
+      const long long row = m * C * C + (long long)i * C + v * 8;
+      if (v * 8 > i) continue;
+      if constexpr (A) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          da[u][k] = __ldcs(reinterpret_cast<const float4*>(dA + row + 4 * k));
+          pp[u][k] = __ldcs(reinterpret_cast<const float4*>(P + row + 4 * k));
+        }
+      }
+      if constexpr (B) {
+        dq[u] = __ldcs(reinterpret_cast<const uint4*>(dQ + row));
+        qq[u] = __ldcs(reinterpret_cast<const uint4*>(Q + row));
+      }
+    }
+  };
+  load(r0);
+  float db_old = 0.f;  // read ahead: each is this block's own to add to
+  if (threadIdx.x < C) {
+    const long long at = ((long long)ch * C + threadIdx.x) * H + h;
+    sb[threadIdx.x] = b != nullptr ? b[at] : 0.f;
+    if constexpr (A) sbeta[threadIdx.x] = beta != nullptr ? beta[at] : 0.f;
+    if (db != nullptr) db_old = db[at];
+  }
   __syncthreads();
-  const int nv = C >> 3, v = threadIdx.x % nv, r0 = threadIdx.x / nv, groups = 256 / nv;
   float col[8];
 #pragma unroll
   for (int e = 0; e < 8; ++e) col[e] = 0.f;
-  for (int i = r0; i < C; i += groups) {
-    const long long row = m * C * C + (long long)i * C + v * 8;
-    const long long ob = ((long long)ch * C + i) * H + h;
-    const float bi = sb[i], be = beta != nullptr ? beta[ob] : 0.f;
-    float gg[8], rs = 0.f, rd = 0.f;
-    if (dA != nullptr) {
-      float da[8], pp[8];
+#pragma unroll 1
+  for (int i0 = r0; i0 < C; i0 += 2 * groups) {
+    if (i0 != r0) load(i0);
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        *reinterpret_cast<float4*>(da + 4 * k) = *reinterpret_cast<const float4*>(dA + row + 4 * k);
-        *reinterpret_cast<float4*>(pp + 4 * k) = *reinterpret_cast<const float4*>(P + row + 4 * k);
+    for (int u = 0; u < 2; ++u) {
+      const int i = i0 + u * groups;
+      const long long row = m * C * C + (long long)i * C + v * 8;
+      float rs = 0.f, rd = 0.f;
+      if (v * 8 > i) {  // nothing above the diagonal
+        if constexpr (A) *reinterpret_cast<uint4*>(g + row) = make_uint4(0, 0, 0, 0);
+        if constexpr (B) *reinterpret_cast<uint4*>(gq + row) = make_uint4(0, 0, 0, 0);
+      } else {
+        const float bi = sb[i], be = A ? sbeta[i] : 0.f;
+        float gg[8];
+        if constexpr (A) {
+          const float *a = reinterpret_cast<const float*>(da[u]), *p = reinterpret_cast<const float*>(pp[u]);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int j = v * 8 + e;
+            const float x = j < i ? a[e] : 0.f, y = j < i ? x * p[e] : 0.f;
+            gg[e] = j < i ? x * be * (b != nullptr ? __expf(bi - sb[j]) : 1.f) : 0.f;
+            rs += y;
+            rd += be * y;
+            col[e] += be * y;
+          }
+          *reinterpret_cast<uint4*>(g + row) = pack8f(gg);
+        }
+        if constexpr (B) {
+          float x[8], q[8];
+          unpack8f(dq[u], x);
+          unpack8f(qq[u], q);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int j = v * 8 + e;
+            const float y = j <= i ? x[e] * q[e] : 0.f;
+            gg[e] = j <= i ? x[e] * __expf(bi - sb[j]) * q_scale : 0.f;
+            rd += y;
+            col[e] += y;
+          }
+          *reinterpret_cast<uint4*>(gq + row) = pack8f(gg);
+        }
       }
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int j = v * 8 + e;
-        const float x = j < i ? da[e] : 0.f, y = j < i ? x * pp[e] : 0.f;  // both operands are zero or unread above the diagonal
-        gg[e] = j < i ? x * be * (b != nullptr ? __expf(bi - sb[j]) : 1.f) : 0.f;
-        rs += y;
-        rd += be * y;
-        col[e] += be * y;
+      for (int o = nv >> 1; o > 0; o >>= 1) {
+        if constexpr (A) rs += __shfl_xor_sync(0xffffffffu, rs, o);
+        rd += __shfl_xor_sync(0xffffffffu, rd, o);
       }
-      *reinterpret_cast<uint4*>(g + row) = pack8f(gg);
-    }
-    if (dQ != nullptr) {
-      float dq[8], qq[8];
-      unpack8f(*reinterpret_cast<const uint4*>(dQ + row), dq);
-      unpack8f(*reinterpret_cast<const uint4*>(Q + row), qq);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int j = v * 8 + e;
-        const float y = j <= i ? dq[e] * qq[e] : 0.f;
-        gg[e] = j <= i ? dq[e] * __expf(bi - sb[j]) * q_scale : 0.f;
-        rd += y;
-        col[e] += y;
+      if (v == 0) {
+        if (A && dbeta != nullptr) dbeta[((long long)ch * C + i) * H + h] += scale * rs;
+        srow[i] = rd;
       }
-      *reinterpret_cast<uint4*>(gq + row) = pack8f(gg);
-    }
-    for (int o = nv >> 1; o > 0; o >>= 1) {
-      rs += __shfl_xor_sync(0xffffffffu, rs, o);
-      rd += __shfl_xor_sync(0xffffffffu, rd, o);
-    }
-    if (v == 0) {
-      if (dbeta != nullptr) dbeta[ob] += scale * rs;
-      srow[i] = rd;
     }
   }
   if (db == nullptr) return;
@@ -246,11 +360,12 @@ __global__ void __launch_bounds__(256) delta_bwd_scores_kernel(const float* __re
     for (int e = 0; e < 8; ++e) scol[warp][v * 8 + e] = col[e];
   }
   __syncthreads();
-  for (int j = threadIdx.x; j < C; j += 256) {
+  if (threadIdx.x < C) {
+    const int j = threadIdx.x;
     float x = srow[j];
 #pragma unroll
     for (int w = 0; w < 8; ++w) x -= scol[w][j];
-    db[((long long)ch * C + j) * H + h] += scale * x;
+    db[((long long)ch * C + j) * H + h] = db_old + scale * x;
   }
 }
 
@@ -261,7 +376,7 @@ extern "C" {
 int fb_delta_inverse(const float* P, const float* beta, const float* b, int NC, int H, int C, void* T, void* Tu, void* Tw, void* A21,
                      cudaStream_t stream) {
   if (NC <= 0) return 0;
-  if ((C != 64 && C != 128) || !fb::aligned(16, P)) return -2;
+  if ((C != 64 && C != 128) || !fb::aligned(16, P, T, Tu, Tw, A21)) return -2;
   delta_inverse_kernel<<<(unsigned)(NC * H * (C / 64)), 64, 0, stream>>>(P, beta, b, C, H, (__nv_bfloat16*)T, (__nv_bfloat16*)(C == 64 ? Tu : nullptr),
                                                                          (__nv_bfloat16*)Tw, (__nv_bfloat16*)A21);
   return fb::launch_ok("delta_inverse_kernel");
@@ -278,8 +393,11 @@ int fb_delta_bwd_t(const void* T, const void* dTu, const void* dTw, const float*
                    float* dbeta, float* db, cudaStream_t stream) {
   if (NC <= 0) return 0;
   if ((C != 64 && C != 128) || !fb::aligned(16, T, dTu, dTw, dT)) return -2;
-  delta_bwd_t_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)T, (const __nv_bfloat16*)dTu, (const __nv_bfloat16*)dTw, beta, b,
-                                                             C, H, scale, (__nv_bfloat16*)dT, dbeta, db);
+  if ((dTw == nullptr) != (b == nullptr)) return -2;
+  const auto kernel = C == 64 ? (b != nullptr ? delta_bwd_t_kernel<64, true> : delta_bwd_t_kernel<64, false>)
+                              : (b != nullptr ? delta_bwd_t_kernel<128, true> : delta_bwd_t_kernel<128, false>);
+  kernel<<<(unsigned)(NC * H), 256, 0, stream>>>((const __nv_bfloat16*)T, (const __nv_bfloat16*)dTu, (const __nv_bfloat16*)dTw, beta, b, H, scale,
+                                                 (__nv_bfloat16*)dT, dbeta, db);
   return fb::launch_ok("delta_bwd_t_kernel");
 }
 
@@ -287,8 +405,16 @@ int fb_delta_bwd_scores(const float* dA, const float* P, const void* dQ, const v
                         float scale, float q_scale, void* g, void* gq, float* dbeta, float* db, cudaStream_t stream) {
   if (NC <= 0) return 0;
   if ((C != 64 && C != 128) || !fb::aligned(16, dA, P, dQ, Q, g, gq)) return -2;
-  delta_bwd_scores_kernel<<<(unsigned)(NC * H), 256, 0, stream>>>(dA, P, (const __nv_bfloat16*)dQ, (const __nv_bfloat16*)Q, beta, b, C, H, scale,
-                                                                  q_scale, (__nv_bfloat16*)g, (__nv_bfloat16*)gq, dbeta, db);
+  auto go = [&](auto kernel) {
+    kernel<<<(unsigned)(NC * H), 256, 0, stream>>>(dA, P, (const __nv_bfloat16*)dQ, (const __nv_bfloat16*)Q, beta, b, H, scale, q_scale,
+                                                   (__nv_bfloat16*)g, (__nv_bfloat16*)gq, dbeta, db);
+  };
+  if (dA == nullptr)
+    go(C == 64 ? delta_bwd_scores_kernel<64, false, true> : delta_bwd_scores_kernel<128, false, true>);
+  else if (dQ == nullptr)
+    go(C == 64 ? delta_bwd_scores_kernel<64, true, false> : delta_bwd_scores_kernel<128, true, false>);
+  else
+    go(C == 64 ? delta_bwd_scores_kernel<64, true, true> : delta_bwd_scores_kernel<128, true, true>);
   return fb::launch_ok("delta_bwd_scores_kernel");
 }
 
@@ -306,13 +432,22 @@ __device__ __forceinline__ void group_rows(int C, int H, int dv, int& ch, int& h
   v = threadIdx.x % nv, r0 = threadIdx.x / nv, groups = blockDim.x / nv;
 }
 
-// b = cumsum(g), eb = scale e^b (fp32, the factor of an output row), alpha = e^{b_last}, vhat = v e^{b_last - b}
+// b = cumsum(g), eb = scale e^b (fp32, the factor of an output row), alpha = e^{b_last}, vhat = v e^{b_last - b}.  The rows of v
+// are fetched before the sum of the gates, which is a chain: 67 -> 58 us at 32,768 tokens, 32 heads of 64 (the bytes take 41).
+// (Two rows at a time made group_bwd2_kernel slower, 101 -> 117 us: three operands of two rows cost it warps.)
 __global__ void __launch_bounds__(256) group_prep_fwd_kernel(const __nv_bfloat16* __restrict__ v, const float* __restrict__ g, int C, int H, int dv,
                                                              float scale, float* __restrict__ b, float* __restrict__ eb, float* __restrict__ alpha,
                                                              __nv_bfloat16* __restrict__ vhat) {
   __shared__ float sb[128];
   int ch, h, vv, r0, groups;
   group_rows(C, H, dv, ch, h, vv, r0, groups);
+  uint4 raw[2];
+  auto load = [&](int i0) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+      if (i0 + u * groups < C) raw[u] = __ldcs(reinterpret_cast<const uint4*>(v + (((long long)ch * C + i0 + u * groups) * H + h) * dv + vv * 8));
+  };
+  load(r0);  // on their way while the gates are summed up
   if (threadIdx.x < 32) {  // warp 0: inclusive sum of up to 128 steps, four per lane
     const int lane = threadIdx.x, per = C >> 5;
     float loc[4], s = 0.f;
@@ -337,14 +472,19 @@ __global__ void __launch_bounds__(256) group_prep_fwd_kernel(const __nv_bfloat16
     eb[o] = scale * __expf(sb[i]);
   }
   if (threadIdx.x == 0) alpha[(long long)ch * H + h] = __expf(last);
-  for (int i = r0; i < C; i += groups) {
-    const long long o = (((long long)ch * C + i) * H + h) * dv + vv * 8;
-    float x[8];
-    unpack8f(*reinterpret_cast<const uint4*>(v + o), x);
-    const float f = __expf(last - sb[i]);
+  for (int i0 = r0; i0 < C; i0 += 2 * groups) {
+    if (i0 != r0) load(i0);
 #pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] *= f;
-    *reinterpret_cast<uint4*>(vhat + o) = pack8f(x);
+    for (int u = 0; u < 2; ++u) {
+      const int i = i0 + u * groups;
+      if (i >= C) break;
+      float x[8];
+      unpack8f(raw[u], x);
+      const float f = __expf(last - sb[i]);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[e] *= f;
+      *reinterpret_cast<uint4*>(vhat + (((long long)ch * C + i) * H + h) * dv + vv * 8) = pack8f(x);
+    }
   }
 }
 

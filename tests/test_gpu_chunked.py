@@ -156,6 +156,63 @@ def test_gsa_edges(M, dk, lens):
 
 
 @pytest.mark.parametrize("C", [64, 128])
+@pytest.mark.parametrize("H", [1, 3])
+@pytest.mark.parametrize("form", ["plain", "gated", "shared"])
+def test_chunk_stages_read_nothing_above_the_diagonal(C, H, form):
+    """The inverse, the gradient through the scaled inverses and that through the scores, against 64 bits, with NaN above the diagonal
+    of the scores and their gradients.  bf16 results: rounded once (2^-8 of the result) after fp32 arithmetic with an exponential
+    that is good to 2^-20; sums of C fp32 terms: 2^-16 of the sum of their absolutes covers C 2^-24 and the exponential."""
+    from flame_b200.ops import chunk_kernels as ck
+    from flame_b200.ops.bgemm import bgemm
+    torch.manual_seed(C + H)
+    NC = 3
+    upper = torch.ones(C, C, dtype=torch.bool, device=DEV).triu(1)
+    nan = lambda x, m=upper: x.masked_fill(m, float("nan"))  # noqa: E731
+    beta = torch.rand(NC, C, H, device=DEV)
+    b = None if form == "plain" else (-torch.rand(NC, C, H, device=DEV) * 0.2).cumsum(1).contiguous()
+    rows = lambda x: x.double().permute(0, 2, 1)  # noqa: E731
+    br, e = rows(beta), torch.ones(NC, H, C, device=DEV).double() if b is None else rows(b).exp()
+    P = (torch.randn(NC, H, C, C, device=DEV) * 0.1).tril(-1)
+    dA, dQ, Q = torch.randn(NC, H, C, C, device=DEV), _bf(NC, H, C, C), _bf(NC, H, C, C)
+    d = (e.log()[..., :, None] - e.log()[..., None, :]).tril().exp().tril()
+    dq, q = dQ.double().tril(), Q.double().tril()
+
+    def near(got, want, size, tol):
+        assert ((got.double() - want).abs() <= tol * size + 2.0 ** -8 * want.abs() * (got.dtype == torch.bfloat16)).all()
+
+    if form == "shared":  # attention with a decay, no delta rule
+        db = torch.ones(NC, C, H, device=DEV)
+        near(ck.scores_bwd(nan(dQ), nan(Q), b, db, 0.5), 0.5 * dq * d, dq.abs(), 2.0 ** -20)
+        y = dq * q
+        near(rows(db), 1 + y.sum(-1) - y.sum(-2), 1 + y.abs().sum(-1) + y.abs().sum(-2), 2.0 ** -16)
+        return
+    T, Tu, Tw = ck.delta_inverse(nan(P, upper | torch.eye(C, dtype=torch.bool, device=DEV)) if C == 64 else P, beta, b, bgemm)
+    eye = torch.eye(C, dtype=torch.float64, device=DEV)
+    want = torch.linalg.solve_triangular(eye + br[..., None] * P.double(), eye.expand_as(P).contiguous(), upper=False, unitriangular=True)
+    assert not T.triu(1).any() and (T.double() - want).norm() <= (2.0 ** -8 if C == 64 else 2.0 ** -7) * want.norm()
+    dTu, dTw = _bf(NC, H, C, C), None if b is None else _bf(NC, H, C, C)
+    w = 0 if b is None else dTw.double() * e[..., None, :]
+    dT, dbeta, db = ck.delta_bwd_t(T, dTu, dTw, beta, b, 0.5)
+    t, both = T.double(), dTu.double() + w
+    size = dTu.double().abs() + (0 if b is None else w.abs())
+    near(dT, br[..., None, :] * both, size, 2.0 ** -20)
+    near(rows(dbeta), 0.5 * (t * both).sum(-2), (t.abs() * size).sum(-2), 2.0 ** -16)
+    if b is not None:
+        near(rows(db), 0.5 * br * (t * w).sum(-2), (t * w).abs().sum(-2), 2.0 ** -16)
+    strict = dA.double().tril(-1)
+    y, y2 = strict * P.double(), dq * q if b is not None else torch.zeros_like(q)
+    old, oldb = rows(dbeta), None if b is None else rows(db)
+    diag = upper | torch.eye(C, dtype=torch.bool, device=DEV)
+    g, gq = ck.delta_bwd_scores(nan(dA, diag), nan(P, diag), nan(dQ), nan(Q), beta, b, 0.5, dbeta, db)
+    near(g, br[..., None] * strict * d, strict.abs(), 2.0 ** -20)
+    near(rows(dbeta), old + 0.5 * y.sum(-1), old.abs() + y.abs().sum(-1), 2.0 ** -16)
+    if b is not None:
+        near(gq, dq * d, dq.abs(), 2.0 ** -20)
+        z = br[..., None] * y + y2
+        near(rows(db), oldb + 0.5 * (z.sum(-1) - z.sum(-2)), oldb.abs() + z.abs().sum(-1) + z.abs().sum(-2), 2.0 ** -16)
+
+
+@pytest.mark.parametrize("C", [64, 128])
 @pytest.mark.parametrize("gated", [False, True])
 @pytest.mark.parametrize("H", [1, 3])
 def test_delta_inverse(C, gated, H):
