@@ -25,6 +25,7 @@ vp, i32, i64, f32 = c_void_p, c_int, c_longlong, c_float
 _lib.register("fb_count_valid", [vp, i64, i32, vp, vp])
 _lib.register("fb_cross_entropy", [vp, vp, vp, vp, vp, f32, i64, i32, i64, i32, i32, vp])
 _lib.register("fb_cross_entropy_opt", [vp, vp, vp, vp, vp, f32, i64, i32, i64, i32, i32, f32, f32, f32, f32, vp])
+_lib.register("fb_scale_by", [vp, vp, vp, i64, vp])
 _lib.register("fb_mean_loss", [vp, i64, vp, vp, i32, vp])
 
 
@@ -68,6 +69,22 @@ def cross_entropy_reference(logits: torch.Tensor, labels: torch.Tensor, ignore_i
 
 def _kernel_ok(x: torch.Tensor) -> bool:
     return _lib.available() and x.is_cuda and x.dtype == torch.bfloat16
+
+
+def _times(g: torch.Tensor, dloss: torch.Tensor) -> torch.Tensor:
+    """``g * dloss`` for the bf16 gradient ``g`` that the forward formed and the scalar gradient of the loss."""
+    plain = dloss.dtype == torch.float32 and dloss.device == g.device and g.is_contiguous()
+    plain = plain and not torch.is_grad_enabled()  # (enabled: this product becomes part of a graph)
+    try:
+        at = dloss.data_ptr() if plain else 0
+    except RuntimeError:  # a batch of gradients at once has no storage of its own
+        at = 0
+    if not at or g.data_ptr() % 16:
+        return g * dloss.to(g.dtype)
+    out = torch.empty_like(g)
+    _lib.check(_lib.lib().fb_scale_by(g.data_ptr(), at, out.data_ptr(), g.numel(), _lib.stream_ptr()), "fb_scale_by")
+    _lib.count_launch()
+    return out
 
 
 class _FLCEFn(torch.autograd.Function):
@@ -118,7 +135,7 @@ class _FLCEFn(torch.autograd.Function):
         dx, dw = ctx.saved_tensors
         # Gradients were formed in the forward with d(loss) = grad_scale.  With a main_grad weight the incoming
         # dloss must be 1 (the trainer passes its 1/accumulation factor as grad_scale instead).
-        gx = dx * dloss.to(dx.dtype) if dx is not None else None
+        gx = _times(dx, dloss) if dx is not None else None
         gw = None
         if dw is not None:
             gw = (dw * dloss).to(torch.bfloat16)
@@ -171,7 +188,7 @@ class _CEFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dloss):
         (g,) = ctx.saved_tensors
-        return g * dloss.to(g.dtype), None, None, None
+        return _times(g, dloss), None, None, None
 
 
 def cross_entropy(logits: torch.Tensor, labels: torch.Tensor, ignore_index: int = -100, label_smoothing: float = 0.0,

@@ -345,6 +345,54 @@ def test_cross_entropy_row_lengths(V):
     assert rel_err(got, want) < 4e-3
 
 
+@pytest.mark.parametrize("V", [1024, 1032, 2048, 2056, 4096, 4104, 12296])
+def test_cross_entropy_by_threads_of_a_row(V):
+    """Rows around the lengths at which a row's CTA changes its threads or vectors, against 64 bits entry by entry: three roundings of
+    fp32 and two exponentials (2^-18), and bf16 twice, in the gradient and in its product with the loss's gradient (2^-7).  A row with
+    its target in the first and one in the last vector, an ignored row with a target inside, a row of NaN, one with +inf."""
+    from flame_b200.ops.cross_entropy import cross_entropy
+    torch.manual_seed(V)
+    rows = 303
+    base = (torch.randn(rows, V, device=DEV) * 4).to(torch.bfloat16)
+    lab = torch.randint(0, V, (rows,), device=DEV)
+    lab[0], lab[1], lab[2] = 0, V - 1, 5
+    lab[lab == 5] = 6
+    lab[2] = 5
+    base[3, 7] = float("-inf")
+    ref_in = base.double().requires_grad_(True)
+    (want,) = torch.autograd.grad(torch.nn.functional.cross_entropy(ref_in, lab, ignore_index=5), ref_in)
+    leaf = base.clone().requires_grad_(True)
+    loss = cross_entropy(leaf * 1.0, lab, ignore_index=5)
+    (got,) = torch.autograd.grad(loss, leaf, torch.tensor(0.75, device=DEV))
+    size = want.abs() + (lab[:, None] == torch.arange(V, device=DEV)) / rows  # (p - 1: the difference keeps the error of p and 1)
+    assert ((got.double() - 0.75 * want).abs() <= 2.0 ** -7 * 0.75 * want.abs() + 2.0 ** -18 * size).all()
+    base[4, 9], base[5, V - 1] = float("nan"), float("inf")
+    leaf = base.clone().requires_grad_(True)
+    loss = cross_entropy(leaf * 1.0, lab, ignore_index=5)
+    (bad,) = torch.autograd.grad(loss, leaf)
+    assert loss.isnan() and bad[4].isnan().all() and bad[5, V - 1].isnan()
+    rest = torch.arange(rows, device=DEV) > 5
+    assert torch.equal((bad[rest].float() * 0.75).to(torch.bfloat16), got[rest])
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 4096, 100003])
+def test_gradient_of_the_loss_as_a_factor(n):
+    """The product with the scalar in device memory equals that of two bf16 tensors bit for bit; other forms take the tensors'."""
+    from flame_b200.ops.cross_entropy import _times
+    torch.manual_seed(n)
+    g, s = torch.randn(n, device=DEV).to(torch.bfloat16), torch.tensor(0.3, device=DEV)
+    want = g * s.to(torch.bfloat16)
+    with torch.no_grad():
+        assert torch.equal(_times(g, s), want)
+        odd = torch.empty(n + 1, dtype=torch.bfloat16, device=DEV)[1:].copy_(g)
+        assert torch.equal(_times(odd, s), want)
+        both = torch.vmap(lambda f: _times(g, f))(torch.stack([s, -s]))
+        assert torch.equal(both[0], want) and torch.equal(both[1], -want)
+    f = s.clone().requires_grad_(True)
+    (d,) = torch.autograd.grad(_times(g, f).float().sum(), f)
+    assert d is not None
+
+
 def test_embedding_backward_runs_of_ids():
     """Runs of one id longer than a warp, ids outside the table (another rank's vocabulary slice), against index_add in fp64."""
     from flame_b200.ops.embedding import embedding
