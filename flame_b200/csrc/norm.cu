@@ -185,9 +185,11 @@ rmsnorm_fwd_short_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 }
 
 // Backward.  `xin` is the tensor that was normalised (the stored residual sum when a residual was fused).  A thread owns
-// eight columns and keeps their dw in registers over all rows of its CTA; a row belongs to LPR lanes of a warp (D <= 256,
-// LPR = D / 8 rounded up to a power of two, several rows side by side) or to the whole CTA (LPR = 0, D / 8 threads rounded
-// up to warps, sums through shared memory).  BR rows per trip: their 2 BR to 3 BR 16-byte loads are issued together and
+// eight columns and keeps their dw in registers over all rows of its CTA; a row belongs to LPR lanes (D <= 512, LPR = D / 8
+// rounded up to a power of two, several rows side by side; 64 lanes are two warps, whose sums meet in shared memory) or to the
+// whole CTA (LPR = 0, D / 8 threads rounded up to warps, sums through shared memory).  Rows of 257 to 512 as CTAs of 64 threads
+// left an SM with eight warps: 98,304 rows of 512 with a gate 157 us, 65,536 of 320 107; four rows side by side take 118 and 77.
+// For 1,024 two rows side by side and one CTA each are equal (105 : 111 us with a residual, 91 : 87 without): one CTA each stays.  BR rows per trip: their 2 BR to 3 BR 16-byte loads are issued together and
 // stay packed in registers, so every operand is read once and enough bytes are in flight to be bound by DRAM; one warp
 // per row, as before, kept one row's loads in flight and re-read D > 1024 and D < 256 through L1 (D = 128, 524,288 rows: 0.28 ms;
 // D = 2048, 32,768 rows: 0.24 ms; both 1.6 TB/s).  dw partials: one row per CTA, which a second kernel sums in order.
@@ -198,13 +200,14 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dgate, float* __restrict__ dw_part, long long rows, int D,
                    int rows_per_cta, const Rows at) {
   constexpr int SLOTS = LPR ? WARPS * 32 / (LPR ? LPR : 1) : 1;
-  __shared__ float s_c[LPR ? 1 : 2][LPR ? 1 : BR][LPR ? 1 : 32];
+  constexpr bool WIDE = LPR == 0 || LPR > 32;  // a row belongs to several warps
+  __shared__ float s_c[WIDE ? 2 : 1][WIDE ? BR : 1][WIDE ? 32 : 1];
   __shared__ float s_dw[LPR ? SLOTS : 1][LPR ? LPR * 8 + 1 : 1];
   const int l = LPR ? threadIdx.x % (LPR ? LPR : 1) : threadIdx.x, slot = LPR ? threadIdx.x / (LPR ? LPR : 1) : 0;
   const int col = l * 8;
   const bool live = col < D;
   const long long row0 = (long long)blockIdx.x * rows_per_cta, row1 = min(rows, row0 + rows_per_cta);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = (LPR ? LPR : blockDim.x) >> 5;
   float ww[8], dw[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) ww[j] = 1.f, dw[j] = 0.f;
@@ -258,10 +261,10 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 #pragma unroll
       for (int j = 0; j < 8; ++j) s += g[j] * ww[j] * a[j] * rs[k];
 #pragma unroll
-      for (int o = (LPR ? LPR : 32) / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      for (int o = (WIDE ? 32 : LPR) / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       c[k] = s * inv_d;
     }
-    if constexpr (LPR == 0) {
+    if constexpr (WIDE) {
       if (lane == 0) {
 #pragma unroll
         for (int k = 0; k < BR; ++k) s_c[flip][k][warp] = c[k];
@@ -270,7 +273,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 #pragma unroll
       for (int k = 0; k < BR; ++k) {
         float s = 0.f;
-        for (int i = 0; i < nwarps; ++i) s += s_c[flip][k][i];
+        for (int i = 0; i < nwarps; ++i) s += s_c[flip][k][slot * nwarps + i];
         c[k] = s;
       }
     }
@@ -466,7 +469,7 @@ int fb_rmsnorm_bwd_rows(const void* dy, const void* xin, const void* w, const fl
   const int parts = fb_rmsnorm_bwd_parts(rows);
   const int rows_per_cta = (int)((rows + parts - 1) / parts);
   if (D > 7040) return -3;
-  const int threads = D <= 256 ? WARPS * 32 : (D / 8 + 31) / 32 * 32;
+  const int threads = D <= 512 ? WARPS * 32 : (D / 8 + 31) / 32 * 32;
 #define BWD_N(HD, GM, LP, NR, TPB)                                                                                  \
   (map ? rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB, true> : rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB, false>)<<<parts, threads, 0, stream>>>( \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)xin, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)gate, \
@@ -477,6 +480,7 @@ int fb_rmsnorm_bwd_rows(const void* dy, const void* xin, const void* w, const fl
     if (D <= 64) BWD_N(HD, GM, 8, (GM ? 2 : 4), 256);                                                             \
     else if (D <= 128) BWD_N(HD, GM, 16, (GM ? 2 : 4), 256);                                                      \
     else if (D <= 256) BWD_N(HD, GM, 32, (GM ? 2 : 4), 256);                                                      \
+    else if (D <= 512) BWD_N(HD, GM, 64, (GM ? 2 : 4), 256);                                                      \
     else if (D <= 2048) BWD_N(HD, GM, 0, (GM ? 2 : 4), 256);                                                      \
     else BWD_N(HD, GM, 0, 1, 1024);                                                                               \
   } while (0)

@@ -142,6 +142,28 @@ def test_rmsnorm_residual_and_gated():
     assert rel_err(o.grad, of.grad) < 2e-2 and rel_err(g.grad, gf.grad) < 2e-2 and rel_err(w2.grad, w2f.grad) < 2e-2
 
 
+@pytest.mark.parametrize("D", [256, 264, 320, 512, 520])
+@pytest.mark.parametrize("rows,gate", [(1, None), (5, "swish"), (777, "sigmoid"), (4803, "swish")])
+def test_rmsnorm_backward_of_rows_side_by_side(D, rows, gate):
+    """Widths around those at which a row's lanes change, and numbers of rows that end inside a trip, against 64 bits.  dx and dgate:
+    three fp32 roundings and a row sum of D terms (2^-20 of the row's largest), rounded to bf16 (2^-8); dw: a sum over the rows."""
+    from flame_b200.ops.norm import rms_norm, rms_norm_gated
+    torch.manual_seed(D + rows)
+    mk = lambda *s: torch.randn(*s, device=DEV).to(torch.bfloat16).requires_grad_(True)  # noqa: E731
+    x, g, w = mk(rows, D), mk(rows, D), mk(D)
+    dy = torch.randn(rows, D, device=DEV).to(torch.bfloat16)
+    ins = (x, w) if gate is None else (x, w, g)
+    y = rms_norm(x, w, 1e-5) if gate is None else rms_norm_gated(x, g, w, 1e-5, gate)
+    got = torch.autograd.grad(y, ins, dy)
+    xd, gd, wd = (t.detach().double().requires_grad_(True) for t in (x, g, w))
+    rstd = torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5)
+    act = {None: 1.0, "swish": gd * gd.sigmoid(), "sigmoid": gd.sigmoid()}[gate]
+    want = torch.autograd.grad(xd * rstd * wd * act, (xd, wd) if gate is None else (xd, wd, gd), dy.double())
+    for a, r, i in zip(got, want, ins):
+        big = r.abs().amax(-1, keepdim=True) if r.dim() == 2 else (dy.double() * xd * rstd * act).abs().sum(0).detach()
+        assert ((a.double() - r).abs() <= 2.0 ** -8 * r.abs() + 2.0 ** -18 * big).all(), i.shape
+
+
 def test_swiglu_rope_embedding():
     from flame_b200.ops.activations import swiglu, swiglu_reference
     from flame_b200.ops.embedding import embedding
