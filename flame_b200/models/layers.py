@@ -620,7 +620,7 @@ class Mamba2(nn.Module):
         lay, rows = ChunkLayout.of(meta, chunk), out[0].shape[0]
         xs, B, C = split_columns(out[0], (Di, G * N, G * N))
         xv, _, g, xs = gates.mamba2_pre_skip(xs, dt, self.dt_bias, self.A_log, H, P, lay)
-        y = grouped_scalar_gla_chunks(C.reshape(rows, G, N), B.reshape(rows, G, N), xv, g, lay)
+        y = grouped_scalar_gla_chunks(reshaped(C, rows, G, N), reshaped(B, rows, G, N), xv, g, lay)
         return gates.mamba2_post(y.reshape(rows, H, P), xs, z, self.D, H, P, lay)
 
 

@@ -324,6 +324,14 @@ _lib.register("fb_decay_scan", ([c_void_p] + [c_longlong] * 3 + [c_int]) * 2 + [
 WALK_US = 0.55, 0.95
 
 
+def _rows_of_vectors(t: torch.Tensor) -> torch.Tensor:
+    """``t`` (four dimensions, bf16), as it lies if the kernels' tile copies can read it there: rows of consecutive elements on 16-byte
+    boundaries."""
+    s = t.stride()
+    ok = s[3] == 1 and min(s) > 0 and not (s[0] | s[1] | s[2]) & 7 and not t.data_ptr() & 15
+    return t if ok else _lib.dense(t)
+
+
 def _decay_states(lay: ChunkLayout, alpha, a, b, reverse: bool, with_state=None):
     """``_state_scan`` over the increments ``x_c = a_c^T b_c`` of operands ``[NC, heads, chunk, rows]`` and ``[NC, heads, chunk, cols]`` (heads of
     either may serve several of alpha's), in the operands' type.  ``with_state`` (contiguous, as the result): returns the pair of the result
@@ -334,8 +342,7 @@ def _decay_states(lay: ChunkLayout, alpha, a, b, reverse: bool, with_state=None)
     if (lay.chunk == 64 and rows in (64, 128) and cols % 64 == 0 and cols > 0 and a.is_cuda and a.dtype == b.dtype == torch.bfloat16 and _lib.available()
             and alpha.dtype == torch.float32 and alpha.is_contiguous() and lay.n_docs <= 65535 and lay.NC * H * rows < 1 << 31
             and lay.longest * WALK_US[with_state is not None] < 20 + lay.NC * H * rows * cols * 1.8e-6):
-        a, b = (t if t.stride(3) == 1 and not t.data_ptr() & 15 and not (t.stride(0) | t.stride(1) | t.stride(2)) & 7 and min(t.stride()) > 0
-                else _lib.dense(t) for t in (a, b))
+        a, b = _rows_of_vectors(a), _rows_of_vectors(b)
         out = torch.empty(lay.NC, H, rows, cols, dtype=a.dtype, device=a.device)
         part = None
         if with_state is not None:
@@ -538,7 +545,9 @@ class _GroupedScalarGla(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, g, scale, lay):
-        q, k, v, g = (_lib.dense(t) for t in (q, k, v, g))
+        ctx.slots = slots.of(q), slots.of(k)
+        q, k = (_rows_of_vectors(t) if t.dtype == torch.bfloat16 else _lib.dense(t) for t in (q, k))  # (column blocks, as a rule)
+        v, g = _lib.dense(v), _lib.dense(g)
         NC, C, H, dv = v.shape
         b, eb, alpha, vhat = _group_prep(v, g, scale)
         d = b.permute(0, 2, 1)
@@ -559,6 +568,15 @@ class _GroupedScalarGla(torch.autograd.Function):
         G, dk = q.shape[2:]
         dt, dev = q.dtype, q.device
         tok = lambda h, n: _token_major(NC, h, C, n, dt, dev)                             # noqa: E731
+
+        def block(i):  # where the gradient of q or k belongs
+            if ctx.slots[i] is None:
+                return tok(G, dk)
+            m = ctx.slots[i].take(NC * C, G * dk, dt, dev)
+            if (m.data_ptr() // m.element_size() | m.stride(0) | dk) & 7:  # the product writes vectors of eight
+                return tok(G, dk)
+            return m.view(NC, C, G, dk).permute(0, 2, 1, 3)
+
         do = _lib.dense(do.to(dt))
         need_q, need_k, need_v, need_g = ctx.needs_input_grad[:4]
         dos, db = _group_bwd1(do, o1, eb)
@@ -577,9 +595,9 @@ class _GroupedScalarGla(torch.autograd.Function):
                 dv1 = bgemm(Q, doh, a_mn=True, b_mn=True, out=tok(H, dv))
             dvv, dg = _group_bwd2(back(dvhat), vhat, back(dv1), b, db, alpha, dalpha)
         if need_q:
-            dq = bgemm(dosh, S, more=[(gq, kh, False, True, 1)], sum_lo=r, out=tok(G, dk))
+            dq = bgemm(dosh, S, more=[(gq, kh, False, True, 1)], sum_lo=r, out=block(0))
         if need_k:
-            dkk = bgemm(vhh, Ln, more=[(gq, qh, True, True, 1)], sum_lo=r, out=tok(G, dk))
+            dkk = bgemm(vhh, Ln, more=[(gq, qh, True, True, 1)], sum_lo=r, out=block(1))
         return back(dq), back(dkk), dvv, dg, None, None
 
 
@@ -763,7 +781,7 @@ def scalar_gla_tc(q, k, v, g, meta: VarlenMeta, scale: float = 1.0, chunk: Optio
 def grouped_scalar_gla_chunks(q, k, v, g, lay: "ChunkLayout") -> torch.Tensor:
     """``scalar_gla_tc`` for heads in groups on operands in the rows of ``lay``: q, k ``[Tp, G, dk]``, v ``[Tp, H, dv]`` bf16 (zero in the padding), g
     ``[Tp, H]`` fp32; the result stays there, ``[NC, chunk, H, dv]``."""
-    return _GroupedScalarGla.apply(*(t.reshape(lay.NC, lay.chunk, *t.shape[1:]) for t in (q, k, v, g)), 1.0, lay)
+    return _GroupedScalarGla.apply(*(slots.reshaped(t, lay.NC, lay.chunk, *t.shape[1:]) for t in (q, k, v, g)), 1.0, lay)
 
 
 class _Gla(torch.autograd.Function):

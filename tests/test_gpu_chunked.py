@@ -927,3 +927,28 @@ def test_gla_backward_writes_its_tokens_alone(lens, raw):
         assert torch.equal(block, w)
         block.fill_(7.0)
         assert (s == 7.0).all()
+
+
+@pytest.mark.parametrize("G,N,lead", [(1, 128, 512), (2, 64, 512), (1, 64, 516), (2, 40, 512)])
+def test_shared_queries_and_keys_as_column_blocks(G, N, lead):
+    """q and k read as blocks of one matrix, and their gradients written into one, equal whole tensors bit for bit: also blocks that do
+    not start on 16 bytes (copied), a state size of the general path, a second run of a retained graph, and through saved-tensor hooks."""
+    from flame_b200.ops.chunked import ChunkLayout, grouped_scalar_gla_chunks
+    from flame_b200.ops.slots import reshaped, split_columns
+    torch.manual_seed(G + N)
+    lay = ChunkLayout.of(_meta([130, 1, 64]), 64)
+    H, P, rows = 4, 64, lay.Tp
+    x = _bf(rows, lead + 2 * G * N, s=0.3).requires_grad_(True)
+    v, g = _bf(rows, H, P), -torch.rand(rows, H, device=DEV) * 0.1
+    do = _bf(lay.NC, 64, H, P)
+
+    def grads(blocks, hooks=False):
+        first, k, q = split_columns(x, (lead, G * N, G * N)) if blocks else (t.contiguous() for t in x.split((lead, G * N, G * N), 1))
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.cpu(), lambda t: t.to(DEV)) if hooks else torch.enable_grad():
+            o = grouped_scalar_gla_chunks(reshaped(q, rows, G, N), reshaped(k, rows, G, N), v, g, lay)
+        out = [torch.autograd.grad((o, first), x, (do, torch.ones_like(first)), retain_graph=True)[0] for _ in range(2)]
+        return [o.detach(), *out]
+
+    want = grads(False)
+    for got in (grads(True), grads(True, hooks=True)):
+        assert all(torch.equal(a, b) for a, b in zip(got, want))
