@@ -345,6 +345,17 @@ def _rows(x: torch.Tensor) -> torch.Tensor:
     return x if x.stride(1) == 1 or x.shape[1] == 1 else x.contiguous()
 
 
+_lib.register("fb_colsum_parts", [c_void_p, c_int, c_int, c_void_p, c_void_p])
+
+
+def _sum_parts(x: torch.Tensor) -> torch.Tensor:
+    """``x.sum(0)`` of contiguous fp32 partials ``[parts, ...]``, in a fixed order."""
+    out = torch.empty(x.shape[1:], dtype=torch.float32, device=x.device)
+    _lib.check(_lib.lib().fb_colsum_parts(x.data_ptr(), x.shape[0], out.numel(), out.data_ptr(), _lib.stream_ptr()), "fb_colsum_parts")
+    _lib.count_launch()
+    return out
+
+
 class SelectiveScan(torch.autograd.Function):
     """Mamba-1 selective scan on the chunk-parallel kernels of ``csrc/sscan.cu``, on packed tokens: u ``[T, Di]`` bf16, delta
     ``[T, Di]`` (fp32, or with ``raw`` the bf16 argument of a softplus), A ``[Di, 16]`` fp32, B, C ``[T, 16]`` (both bf16 or both
@@ -413,7 +424,8 @@ class SelectiveScan(torch.autograd.Function):
                             part.data_ptr(), dD.data_ptr(), dB.data_ptr(), dC.data_ptr(), T, lay.NC, Di, A.shape[1], _lib.stream_ptr())
         _lib.check(rc, "fb_sscan_bwd")
         _lib.count_launch(4)
-        return du, ddl, dA.sum(0)[:, :Di].t(), dB, dC, dD.sum(0)[:Di], dz, None, None, None
+        dA, dD = _sum_parts(dA), _sum_parts(dD)
+        return du, ddl, dA[:, :Di].t(), dB, dC, dD[:Di], dz, None, None, None
 
 
 _lib.register("fb_vdecay_prep", [c_void_p] * 6 + [c_int] * 3 + [c_void_p])

@@ -952,3 +952,13 @@ def test_shared_queries_and_keys_as_column_blocks(G, N, lead):
     want = grads(False)
     for got in (grads(True), grads(True, hooks=True)):
         assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+@pytest.mark.parametrize("shape", [(1, 5), (15, 16, 40), (17, 33), (518, 16, 96), (0, 64)])
+def test_sums_of_partials(shape):
+    """fp32 partials added up in a fixed order, against 64 bits: as many roundings as terms of a thread and groups (2^-24 each)."""
+    from flame_b200.ops.chunk_kernels import _sum_parts
+    torch.manual_seed(3)
+    x = torch.randn(shape, device=DEV)
+    bound = (shape[0] / 16 + 17) * 2.0 ** -24 * x.double().abs().sum(0)
+    assert ((_sum_parts(x).double() - x.double().sum(0)).abs() <= bound).all()
