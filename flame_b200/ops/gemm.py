@@ -21,8 +21,6 @@ import torch
 
 from . import _lib
 
-_WORKSPACES: dict = {}
-
 
 class PendingGather:
     """A unit of sharded parameters whose bytes ``[lo, hi)`` have not been fetched into the staging buffer yet.  The first
@@ -72,14 +70,10 @@ def _sm_count(device: torch.device) -> int:
 
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    """Per-device split-K scratch, grown on demand and reused (stream-ordered reuse is safe because
-    every consumer runs on the launching stream)."""
-    key = (device.index, torch.cuda.current_stream().cuda_stream)
-    ws = _WORKSPACES.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _WORKSPACES[key] = ws
-    return ws
+    """Scratch of one product.  Not kept: the pieces are written by one launch and added up by the next, and another thread's product may
+    come between the two on the same stream; a captured graph goes on using what it was captured with.  The allocator hands the
+    bytes on in the order of the stream."""
+    return torch.empty(nbytes, dtype=torch.uint8, device=device)
 
 
 def _use_kernel(a: torch.Tensor, b: torch.Tensor) -> bool:

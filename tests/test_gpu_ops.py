@@ -85,6 +85,42 @@ def test_gemm_tiles_cut_along_k(M, N, K):
         assert torch.equal(wide[:, [0, 3, N + 4, N + 7]], torch.ones(M, 4, device=DEV))
 
 
+def test_gemm_scratch_belongs_to_one_product():
+    """Products in pieces share no scratch: threads on one stream, each between whose two launches another's may come, and a captured
+    product that is replayed after a larger one on its stream, with the memory in between handed to others.  All bits as alone."""
+    import threading
+    from flame_b200.ops import _lib, gemm
+    M, N, K = 136, 72, 5000
+    assert _lib.lib().fb_gemm_cut_bytes(M, N, K) > 0 and _lib.lib().fb_gemm_cut_bytes(2040, 2312, 8200) > _lib.lib().fb_gemm_cut_bytes(M, N, K)
+    torch.manual_seed(4)
+    mk = lambda *s: torch.randn(*s, device=DEV, dtype=torch.bfloat16)  # noqa: E731
+    pairs = [(mk(M, K), mk(N, K)) for _ in range(4)]
+    want = [gemm.gemm_nt(a, b, out_dtype=torch.float32) for a, b in pairs]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        for _ in range(50):
+            if not torch.equal(gemm.gemm_nt(*pairs[i], out_dtype=torch.float32), want[i]):
+                bad.append(i)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        gemm.gemm_nt(*pairs[0], out_dtype=torch.float32)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            out = gemm.gemm_nt(*pairs[0], out_dtype=torch.float32)
+        gemm.gemm_nt(mk(2040, 8200), mk(2312, 8200))
+        others = [torch.full((1 << 18,), 7.0, device=DEV) for _ in range(64)]
+        graph.replay()
+    s.synchronize()
+    assert torch.equal(out, want[0]) and all(bool((o == 7).all()) for o in others)
+
+
 @pytest.mark.parametrize("lens,H,Hkv,Dh,window", [([128], 1, 1, 64, 0), ([300, 77, 129], 2, 1, 64, 0),
                                                    ([1000, 24, 512], 4, 4, 64, 0), ([640], 2, 2, 64, 200),
                                                    ([300, 200], 2, 1, 128, 0), ([300, 200], 2, 2, 128, 100),
