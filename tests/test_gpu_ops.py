@@ -200,6 +200,40 @@ def test_rmsnorm_backward_of_rows_side_by_side(D, rows, gate):
         assert ((a.double() - r).abs() <= 2.0 ** -8 * r.abs() + 2.0 ** -18 * big).all(), i.shape
 
 
+@pytest.mark.parametrize("H", [1, 3, 4, 5, 9])
+@pytest.mark.parametrize("Dh,rot", [(64, 64), (128, 128), (64, 32), (48, 16)])
+@pytest.mark.parametrize("many", [False, True])
+def test_rope_heads_of_one_thread(H, Dh, rot, many):
+    """Numbers of heads around what a thread takes, partial rotation, both directions, in place in a wider matrix, beside it and from fp32,
+    against 64 bits: two products and a sum (2^-22 of the larger operand), rounded to bf16 (2^-8)."""
+    from flame_b200.ops.rope import rope_from_fp32_, rope_inplace_, rope_rotated
+    torch.manual_seed(H + Dh + rot)
+    T = 333 + many * (600000 * 16 // (H * rot))   # beyond this a thread takes several heads
+    pos = torch.randint(0, 500, (T,), device=DEV, dtype=torch.int32)
+    ang = torch.rand(500, rot // 2, device=DEV) * 6
+    cos, sin = ang.cos(), ang.sin()
+    wide = torch.randn(T, (H + 2) * Dh, device=DEV).to(torch.bfloat16)
+    x = wide[:, Dh:(H + 1) * Dh].view(T, H, Dh)
+    src, before = x.clone(), wide.clone()
+
+    def check(y, src, sign):
+        a, b = src[..., :rot // 2].double(), src[..., rot // 2:rot].double()
+        c, s = cos[pos.long(), None].double(), sign * sin[pos.long(), None].double()
+        want, size = torch.cat([a * c - b * s, a * s + b * c], -1), torch.maximum(a.abs(), b.abs()).repeat(1, 1, 2)
+        assert ((y[..., :rot].double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -22 * size).all()
+
+    check(rope_rotated(x, pos, cos, sin), src, 1)
+    assert torch.equal(wide, before)
+    rope_inplace_(x, pos, cos, sin, conj=True)
+    check(x, src, -1)
+    assert torch.equal(x[..., rot:], src[..., rot:])
+    assert torch.equal(wide[:, :Dh], before[:, :Dh]) and torch.equal(wide[:, (H + 1) * Dh:], before[:, (H + 1) * Dh:])
+    if rot == Dh:
+        f = torch.randn(T, H, Dh, device=DEV)
+        rope_from_fp32_(f, x, pos, cos, sin, conj=True)
+        check(x, f, -1)
+
+
 def test_swiglu_rope_embedding():
     from flame_b200.ops.activations import swiglu, swiglu_reference
     from flame_b200.ops.embedding import embedding
