@@ -189,17 +189,21 @@ rmsnorm_fwd_short_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 // rounded up to a power of two, several rows side by side; 64 lanes are two warps, whose sums meet in shared memory) or to the
 // whole CTA (LPR = 0, D / 8 threads rounded up to warps, sums through shared memory).  Rows of 257 to 512 as CTAs of 64 threads
 // left an SM with eight warps: 98,304 rows of 512 with a gate 157 us, 65,536 of 320 107; four rows side by side take 118 and 77.
-// For 1,024 two rows side by side and one CTA each are equal (105 : 111 us with a residual, 91 : 87 without): one CTA each stays.  BR rows per trip: their 2 BR to 3 BR 16-byte loads are issued together and
-// stay packed in registers, so every operand is read once and enough bytes are in flight to be bound by DRAM; one warp
-// per row, as before, kept one row's loads in flight and re-read D > 1024 and D < 256 through L1 (D = 128, 524,288 rows: 0.28 ms;
-// D = 2048, 32,768 rows: 0.24 ms; both 1.6 TB/s).  dw partials: one row per CTA, which a second kernel sums in order.
+// For 1,024 two rows side by side and one CTA each are equal (105 : 111 us with a residual, 91 : 87 without): one CTA each stays.
+// BR rows per trip: their 2 BR to 3 BR 16-byte loads are issued together and stay packed in registers, so every operand is read
+// once.  The next trip's go out before this trip's sums (AHEAD), so memory is busy while the CTA computes; what 128 registers hold
+// of two trips sets BR, and 80 where a gate leaves more to compute and three CTAs pay: 98,304 rows of 512 with a gate 118 -> 101 us,
+// 262,144 of 256 142 -> 130 (of the chunk layout 156 -> 148), 65,536 of 320 77 -> 66, of 1,024 with a residual 111 -> 101, 32,768 of 2,048
+// 95 -> 89.  Gated rows of a whole CTA are slower with it (150 -> 158) and keep two rows and no lead.
+// dw partials: one row per CTA, which a second kernel sums in order.
 template <bool HAS_DRES, int GATE, int LPR, int BR, int TPB, bool MAP>
-__global__ void __launch_bounds__(TPB, TPB == 256 ? 2 : 1)
+__global__ void __launch_bounds__(TPB, TPB != 256 ? 1 : GATE && LPR ? 3 : 2)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ xin, const __nv_bfloat16* __restrict__ w,
                    const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ gate, const __nv_bfloat16* __restrict__ dres,
                    __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dgate, float* __restrict__ dw_part, long long rows, int D,
                    int rows_per_cta, const Rows at) {
   constexpr int SLOTS = LPR ? WARPS * 32 / (LPR ? LPR : 1) : 1;
+  constexpr bool AHEAD = TPB == 256 && !(GATE && LPR == 0);  // the next trip's loads go out before this trip's sums
   constexpr bool WIDE = LPR == 0 || LPR > 32;  // a row belongs to several warps
   __shared__ float s_c[WIDE ? 2 : 1][WIDE ? BR : 1][WIDE ? 32 : 1];
   __shared__ float s_dw[LPR ? SLOTS : 1][LPR ? LPR * 8 + 1 : 1];
@@ -223,10 +227,11 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
     }
   };
   if (MAP) look(row0);
-  for (long long rb = row0; rb < row1; rb += SLOTS * BR, flip ^= 1) {
-    uint4 xa[BR], ga[BR], ra[HAS_DRES ? BR : 1], ta[GATE ? BR : 1];
-    float rs[BR], c[BR];
-    int from[MAP ? BR : 1];  // the packed row, -1 where there is none: its gradient is zero
+  uint4 xa[BR], ga[BR], ra[HAS_DRES ? BR : 1], ta[GATE ? BR : 1];
+  float rs[BR], c[BR];
+  int from[MAP ? BR : 1];  // the packed row, -1 where there is none: its gradient is zero
+  auto load = [&](long long rb, uint4 (&xa)[BR], uint4 (&ga)[BR], uint4 (&ra)[HAS_DRES ? BR : 1], uint4 (&ta)[GATE ? BR : 1], float (&rs)[BR],
+                  int (&from)[MAP ? BR : 1]) {
 #pragma unroll
     for (int k = 0; k < (MAP ? BR : 1); ++k)
       if (MAP) from[k] = ahead[k];
@@ -243,6 +248,24 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
       rs[k] = there ? rstd[pr] : 0.f;
     }
     if (MAP) look(rb + SLOTS * BR);
+  };
+  uint4 xn[BR], gn[BR], rn[HAS_DRES ? BR : 1], tn[GATE ? BR : 1];  // AHEAD: the next trip's
+  float sn[BR];
+  int fn[MAP ? BR : 1];
+  if constexpr (AHEAD) load(row0, xn, gn, rn, tn, sn, fn);
+  for (long long rb = row0; rb < row1; rb += SLOTS * BR, flip ^= 1) {
+    if constexpr (AHEAD) {
+#pragma unroll
+      for (int k = 0; k < BR; ++k) {
+        xa[k] = xn[k], ga[k] = gn[k], rs[k] = sn[k];
+        if (HAS_DRES) ra[k] = rn[k];
+        if (GATE) ta[k] = tn[k];
+        if (MAP) from[k] = fn[k];
+      }
+      load(rb + SLOTS * BR, xn, gn, rn, tn, sn, fn);
+    } else {
+      load(rb, xa, ga, ra, ta, rs, from);
+    }
 #pragma unroll
     for (int k = 0; k < BR; ++k) {
       float a[8], g[8];
@@ -474,7 +497,8 @@ int fb_rmsnorm_bwd_rows(const void* dy, const void* xin, const void* w, const fl
       !fb::aligned(16, dy, xin, w, gate, dres, dx, dgate))
     return -2;
   const Rows at{map, (unsigned)heads, ldg ? ldg : (long long)heads * D, lddg ? lddg : (long long)heads * D};
-  const int parts = fb_rmsnorm_bwd_parts(rows);
+  // resident CTAs: two on each of 148 SMs, two waves of them; three with a gate and rows side by side, one wave
+  const int most = fb_rmsnorm_bwd_parts(rows), parts = gate_mode && D <= 512 && most > 444 ? 444 : most;
   const int rows_per_cta = (int)((rows + parts - 1) / parts);
   if (D > 7040) return -3;
   const int threads = D <= 512 ? WARPS * 32 : (D / 8 + 31) / 32 * 32;
@@ -482,14 +506,14 @@ int fb_rmsnorm_bwd_rows(const void* dy, const void* xin, const void* w, const fl
   (map ? rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB, true> : rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB, false>)<<<parts, threads, 0, stream>>>( \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)xin, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)gate, \
       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dgate, dw_part, rows, D, rows_per_cta, at)
-  // rows per trip by what 128 registers hold packed; one row where a CTA has more than eight warps to overlap (64 registers)
+  // rows per trip by what the registers hold packed; one row and no lead where a CTA has more than eight warps to overlap (64 registers)
 #define BWD(HD, GM)                                                                                               \
   do {                                                                                                            \
-    if (D <= 64) BWD_N(HD, GM, 8, (GM ? 2 : 4), 256);                                                             \
-    else if (D <= 128) BWD_N(HD, GM, 16, (GM ? 2 : 4), 256);                                                      \
-    else if (D <= 256) BWD_N(HD, GM, 32, (GM ? 2 : 4), 256);                                                      \
-    else if (D <= 512) BWD_N(HD, GM, 64, (GM ? 2 : 4), 256);                                                      \
-    else if (D <= 2048) BWD_N(HD, GM, 0, (GM ? 2 : 4), 256);                                                      \
+    if (D <= 64) BWD_N(HD, GM, 8, (GM ? 1 : HD ? 2 : 4), 256);                                                             \
+    else if (D <= 128) BWD_N(HD, GM, 16, (GM ? 1 : HD ? 2 : 4), 256);                                                      \
+    else if (D <= 256) BWD_N(HD, GM, 32, (GM ? 1 : HD ? 2 : 4), 256);                                                      \
+    else if (D <= 512) BWD_N(HD, GM, 64, (GM ? 1 : 2), 256);                                                      \
+    else if (D <= 2048) BWD_N(HD, GM, 0, 2, 256);                                                                 \
     else BWD_N(HD, GM, 0, 1, 1024);                                                                               \
   } while (0)
   if (gate_mode == 0) {

@@ -200,6 +200,37 @@ def test_rmsnorm_backward_of_rows_side_by_side(D, rows, gate):
         assert ((a.double() - r).abs() <= 2.0 ** -8 * r.abs() + 2.0 ** -18 * big).all(), i.shape
 
 
+@pytest.mark.parametrize("D", [64, 128, 256, 320, 768, 1024, 2048, 2056])
+@pytest.mark.parametrize("rows,form", [(1, "residual"), (9, "residual"), (4803, "residual"), (4803, "plain"), (4803, "swish")])
+def test_rmsnorm_backward_with_the_next_rows_on_their_way(D, rows, form):
+    """Every width class, with the gradient of a residual and without, with a gate, and numbers of rows that end inside a trip; bounds as in
+    the test above."""
+    from flame_b200.ops.norm import rms_norm, rms_norm_gated
+    torch.manual_seed(D + rows)
+    mk = lambda *s: torch.randn(*s, device=DEV).to(torch.bfloat16).requires_grad_(True)  # noqa: E731
+    x, r, g, w = mk(rows, D), mk(rows, D), mk(rows, D), mk(D)
+    dy, dz = (torch.randn(rows, D, device=DEV).to(torch.bfloat16) for _ in range(2))
+    xd, gd, wd = (t.detach().double().requires_grad_(True) for t in (x, g, w))
+    act = gd * gd.sigmoid() if form == "swish" else 1.0
+    if form == "residual":
+        y, z = rms_norm(x, w, 1e-5, r, True)
+        got = torch.autograd.grad((y, z), (x, w), (dy, dz))
+        xd = z.detach().double().requires_grad_(True)     # the sum as it was rounded
+    elif form == "plain":
+        got = torch.autograd.grad(rms_norm(x, w, 1e-5), (x, w), dy)
+    else:
+        got = torch.autograd.grad(rms_norm_gated(x, g, w, 1e-5, form), (x, w, g), dy)
+    rstd = torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5)
+    want = list(torch.autograd.grad(xd * rstd * wd * act, (xd, wd, gd) if form == "swish" else (xd, wd), dy.double()))
+    size = [v.abs().amax(-1, keepdim=True) for v in want]
+    size[1] = (dy.double() * xd * rstd * act).abs().sum(0).detach()
+    if form == "residual":
+        want[0] = want[0] + dz.double()
+        size[0] = size[0] + dz.double().abs()
+    for a, b, big in zip(got, want, size):
+        assert ((a.double() - b).abs() <= 2.0 ** -8 * b.abs() + 2.0 ** -18 * big).all(), b.shape
+
+
 @pytest.mark.parametrize("H", [1, 3, 4, 5, 9])
 @pytest.mark.parametrize("Dh,rot", [(64, 64), (128, 128), (64, 32), (48, 16)])
 @pytest.mark.parametrize("many", [False, True])
