@@ -231,6 +231,34 @@ def test_rmsnorm_backward_with_the_next_rows_on_their_way(D, rows, form):
         assert ((a.double() - b).abs() <= 2.0 ** -8 * b.abs() + 2.0 ** -18 * big).all(), b.shape
 
 
+@pytest.mark.parametrize("D", [264, 512, 520, 1024, 1032, 2048, 2056])
+@pytest.mark.parametrize("rows,form", [(1, "plain"), (9, "sum"), (777, "prenorm"), (777, "swish"), (777, "sigmoid"), (777, "bare")])
+def test_rmsnorm_forward_of_rows_in_registers(D, rows, form):
+    """Widths around what a lane holds, with a residual (the sum kept, or not), a gate and without a weight, against 64 bits: a sum of D
+    squares and four roundings in fp32 (2^-18), rounded to bf16 (2^-8); the kept sum is the rounded one."""
+    from flame_b200.ops.norm import rms_norm, rms_norm_gated
+    torch.manual_seed(D + rows)
+    x, r, w = (torch.randn(*s, device=DEV).to(torch.bfloat16) for s in ((rows, D), (rows, D), (D,)))
+    v = x.double()
+    if form == "prenorm":
+        y, z = rms_norm(x, w, 1e-5, r, True)
+        assert torch.equal(z, x + r)
+        v = z.double()
+    elif form == "sum":
+        y, v = rms_norm(x, w, 1e-5, r), None
+        both = [x.double() + r.double(), (x + r).double()]   # whether the sum is rounded is the operator's choice
+    elif form in ("swish", "sigmoid"):
+        y = rms_norm_gated(x, r, w, 1e-5, form)
+    else:
+        y = rms_norm(x, None if form == "bare" else w, 1e-5)
+    act = {"swish": r.double() * r.double().sigmoid(), "sigmoid": r.double().sigmoid()}.get(form, 1.0)
+    near = []
+    for v in both if form == "sum" else [v]:
+        want = v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-5) * (1.0 if form == "bare" else w.double()) * act
+        near.append(bool(((y.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * want.abs().amax(-1, keepdim=True)).all()))
+    assert any(near)
+
+
 @pytest.mark.parametrize("H", [1, 3, 4, 5, 9])
 @pytest.mark.parametrize("Dh,rot", [(64, 64), (128, 128), (64, 32), (48, 16)])
 @pytest.mark.parametrize("many", [False, True])
