@@ -411,7 +411,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             const long long lrow = (long long)p.s_rank * p.s_rows_per_rank + (row - owner * p.s_rows_per_rank);
             dst = (__nv_bfloat16*)p.s_dst[owner] + lrow * p.ldc + col0;
           }
-          if (full && ((p.ldc & 7) == 0)) {
+          if (full && (p.ldc & 7) == 0 && ((uintptr_t)dst & 15) == 0) {  // (a block of a matrix may start anywhere)
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               uint4 q;
@@ -428,7 +428,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         } else {
           float* dst = (float*)p.C + (long long)split * p.split_stride + (long long)row * p.ldc + col0;
           const bool accumulate = (p.epi == EPI_F32_ACC);
-          if (full && ((p.ldc & 3) == 0)) {
+          if (full && (p.ldc & 3) == 0 && ((uintptr_t)dst & 15) == 0) {
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
               float4 q = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
@@ -471,17 +471,26 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ part, int splits,
     s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
   }
   if (out_fp32) {
-    float4* o = reinterpret_cast<float4*>((float*)out + i);
-    if (accumulate) {
-      float4 t = *o;
-      s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+    float* o = (float*)out + i;
+    if (((uintptr_t)o & 15) == 0) {
+      float4* o4 = reinterpret_cast<float4*>(o);
+      if (accumulate) {
+        float4 t = *o4;
+        s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+      }
+      *o4 = s;
+    } else {
+      const float e[4] = {s.x, s.y, s.z, s.w};
+      for (int k = 0; k < 4; ++k) o[k] = accumulate ? o[k] + e[k] : e[k];
     }
-    *o = s;
   } else {
-    uint2 q;
-    q.x = pack_bf16(s.x, s.y);
-    q.y = pack_bf16(s.z, s.w);
-    *reinterpret_cast<uint2*>((__nv_bfloat16*)out + i) = q;
+    __nv_bfloat16* o = (__nv_bfloat16*)out + i;
+    if (((uintptr_t)o & 7) == 0) {
+      *reinterpret_cast<uint2*>(o) = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
+    } else {
+      const float e[4] = {s.x, s.y, s.z, s.w};
+      for (int k = 0; k < 4; ++k) o[k] = __float2bfloat16(e[k]);
+    }
   }
 }
 

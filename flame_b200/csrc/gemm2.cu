@@ -794,7 +794,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
             const long long lrow = (long long)p.s_rank * p.s_rows_per_rank + (row - owner * p.s_rows_per_rank);
             dst = (__nv_bfloat16*)p.s_dst[owner] + lrow * p.ldc + col0;
           }
-          if (full && ((p.ldc & 7) == 0)) {
+          if (full && (p.ldc & 7) == 0 && ((uintptr_t)dst & 15) == 0) {  // (a block of a matrix may start anywhere)
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               uint4 q;
@@ -811,7 +811,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         } else {
           float* dst = (float*)p.C + (long long)split * p.split_stride + (long long)row * p.ldc + col0;
           const bool accumulate = (p.epi == 2);
-          if (full && ((p.ldc & 3) == 0)) {
+          if (full && (p.ldc & 3) == 0 && ((uintptr_t)dst & 15) == 0) {
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
               float4 q = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);

@@ -85,6 +85,39 @@ def test_gemm_tiles_cut_along_k(M, N, K):
         assert torch.equal(wide[:, [0, 3, N + 4, N + 7]], torch.ones(M, 4, device=DEV))
 
 
+@pytest.mark.parametrize("variant", [1, 2])
+@pytest.mark.parametrize("splits", [1, 4])
+def test_gemm_results_that_start_between_vectors(variant, splits):
+    """Results whose rows are whole vectors apart (or lie back to back) but start between vectors: every output form, with a bias too, in
+    both kernels and after a split along K, equals the result on a boundary bit for bit and leaves its neighbours alone."""
+    from flame_b200.ops import _lib, gemm
+    torch.manual_seed(6)
+    M, N, K = 136, 296, 1024
+    at, bt = (torch.randn(K, n, device=DEV, dtype=torch.bfloat16) for n in (M, N))
+    bias = torch.randn(N, device=DEV).to(torch.bfloat16)
+    a, b = at.t().contiguous(), bt.t().contiguous()
+    old = _lib.lib().fb_gemm_set_variant(variant)
+    try:
+        forms = [(torch.float32, dict(accumulate=True)), (torch.float32, {}), (torch.bfloat16, {}), (torch.bfloat16, dict(bias=bias))]
+        for dtype, more in forms[:4 if splits == 1 else 3]:
+            want = torch.ones(M, N, device=DEV, dtype=dtype)
+            gemm.gemm_nt(a, b, out=want, splits=splits, **more)
+            for start in (1, 2, 3, 4, 5):
+                for pitch in (N, N + 8) if splits == 1 else (N,):
+                    store = torch.ones(M * pitch + 16, device=DEV, dtype=dtype)
+                    out = store[start:start + M * pitch].view(M, pitch)[:, :N]
+                    gemm.gemm_nt(a, b, out=out, splits=splits, **more)
+                    assert torch.equal(out, want)
+                    out.fill_(1)
+                    assert (store == 1).all()
+                    if not more.get("bias") is None:
+                        continue
+                    gemm.gemm_tn(at, bt, out=out, **more)   # the library's own choice of a split
+                    assert rel_err(out, want) < 2 ** -8
+    finally:
+        _lib.lib().fb_gemm_set_variant(old)
+
+
 def test_gemm_scratch_belongs_to_one_product():
     """Products in pieces share no scratch: threads on one stream, each between whose two launches another's may come, and a captured
     product that is replayed after a larger one on its stream, with the memory in between handed to others.  All bits as alone."""
