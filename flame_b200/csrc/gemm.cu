@@ -549,6 +549,7 @@ extern "C" int fb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N
                              int sm_count, cudaStream_t stream);
 
 extern "C" long long fb_gemm2_cut_bytes(int M, int N, int K, int sm_count);
+extern "C" long long fb_gemm2_cut_bytes_into(const void* C, long long ldc, int out_mode, int M, int N, int K, int sm_count);
 extern "C" int fb_gemm2_allgather_a(const unsigned long long* shard_ptrs, int world, int rank, int rows_per_rank, long long ld,
                                     void* a_full, int* chunk_flags, const int* ready, int epoch, const void* B, void* C, int N,
                                     int K, long long ldb, long long ldc, int b_mn, int sm_count, cudaStream_t stream);
@@ -574,7 +575,12 @@ long long fb_gemm_workspace_bytes(int M, int N, int splits) {
 // kernel) and fb_gemm_pick_splits chooses.
 long long fb_gemm_cut_bytes(int M, int N, int K) { return g_variant == 2 ? fb_gemm2_cut_bytes(M, N, K, sm_count_cached()) : -1; }
 
-// For the single-CTA kernel: chooses a split-K factor with a small cost model: waves of work units times K blocks per unit, plus the
+// The same for the result that fb_gemm_bf16 is to be given: -1 also where its rows or its start rule out tensor copies.
+long long fb_gemm_cut_bytes_into(const void* C, long long ldc, int out_mode, int M, int N, int K) {
+  return g_variant == 2 ? fb_gemm2_cut_bytes_into(C, ldc, out_mode, M, N, K, sm_count_cached()) : -1;
+}
+
+// Where nothing is cut (the single-CTA kernel, results that no tensor copy can write): chooses a split-K factor with a small cost model: waves of work units times K blocks per unit, plus the
 // traffic of writing and re-reading the fp32 partials.  Few-tile, long-K GEMMs (weight gradients) gain most.
 int fb_gemm_pick_splits(int M, int N, int K) {
   const long long tiles = (long long)((M + BM - 1) / BM) * ((N + 255) / 256);

@@ -954,11 +954,14 @@ int start2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
   return fb::launch_ok(FP8 ? "gemm2_fp8_kernel" : "gemm2_bf16_kernel");
 }
 
+// Whether a result of N columns of `bytes` each can leave by TMA: rows and start on 16 bytes.
+bool tma_result(const void* C, long long ldc, int N, int bytes) { return (ldc * bytes & 15) == 0 && ldc >= N && !((uintptr_t)C & 15); }
+
 template <bool A_MN, bool B_MN, bool FP8 = false>
 int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, int sm_count, cudaStream_t stream, float* part = nullptr) {
   CUtensorMap tmC = tmA, tmP = tmA;
   const int c_bytes = p.epi == 0 ? 2 : 4;
-  if (p.s_world == 0 && p.swiglu_I == 0 && p.splits == 1 && (p.ldc * c_bytes & 15) == 0 && p.ldc >= p.N && !((uintptr_t)p.C & 15)) {
+  if (p.s_world == 0 && p.swiglu_I == 0 && p.splits == 1 && tma_result(p.C, p.ldc, p.N, c_bytes)) {
     const int rc = fb::make_tmap_2d(&tmC, p.C, c_bytes, p.M, p.N, p.ldc, 32, 128 / c_bytes, true);
     if (rc) return rc;
     p.tma_c = 1;
@@ -984,6 +987,11 @@ long long fb_gemm2_cut_bytes(int M, int N, int K, int sm_count) {
   int pieces;
   const long long cut = cut_last_round((long long)((M + BM2 - 1) / BM2) * ((N + BN - 1) / BN), (K + BK - 1) / BK, max_pairs(sm_count), &pieces);
   return cut * pieces * TILE_FLOATS * 4;
+}
+
+// The same for a given result; -1 where it cannot leave by TMA, which the pieces' tiles have to.
+long long fb_gemm2_cut_bytes_into(const void* C, long long ldc, int out_mode, int M, int N, int K, int sm_count) {
+  return tma_result(C, ldc, N, out_mode == 0 ? 2 : 4) ? fb_gemm2_cut_bytes(M, N, K, sm_count) : -1;
 }
 
 // Same contract as fb_gemm_bf16 without bias; splits == 0: the last round may be cut, `workspace` (or null) as

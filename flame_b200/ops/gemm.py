@@ -122,7 +122,7 @@ def _launch(a, b, M, N, K, a_mn, b_mn, out, accumulate, alpha, bias, splits):
             pend.flush()  # this product reads the unit but cannot carry the gather: fetch with the stand-alone kernel
     ws, launches = None, 1
     if splits is None:
-        need = L.fb_gemm_cut_bytes(M, N, K) if bias is None else -1
+        need = L.fb_gemm_cut_bytes_into(out.data_ptr(), out.stride(0), mode, M, N, K) if bias is None else -1
         if need >= 0:   # the CTA pairs cut the tiles of their last round along K where that pays
             splits = 0
             if need:

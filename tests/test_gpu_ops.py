@@ -118,6 +118,29 @@ def test_gemm_results_that_start_between_vectors(variant, splits):
         _lib.lib().fb_gemm_set_variant(old)
 
 
+@pytest.mark.parametrize("N,dtype,start,pitch", [(70, torch.float32, 0, 70), (68, torch.bfloat16, 0, 68), (72, torch.float32, 2, 72),
+                                                 (72, torch.float32, 0, 77), (72, torch.bfloat16, 3, 80)])
+def test_gemm_results_without_tensor_copies_are_split_or_whole(N, dtype, start, pitch):
+    """Few tiles and a long K into results that no tensor copy can write: where the rows lie back to back the sum is split over the whole K
+    as the library's model says (equal to that split asked for, bit for bit), else it is whole: one launch, no scratch."""
+    from flame_b200.ops import _lib, gemm
+    M, K = 136, 5000
+    torch.manual_seed(9)
+    a, b = torch.randn(K, M, device=DEV, dtype=torch.bfloat16), torch.randn(K, 80, device=DEV, dtype=torch.bfloat16)[:, :N]
+    assert _lib.lib().fb_gemm_cut_bytes(M, N, K) > 0
+    split = int(_lib.lib().fb_gemm_pick_splits(M, N, K)) if pitch == N else 1
+    assert (split > 1) == (pitch == N)
+    got, want = (torch.zeros(M * pitch + 8, device=DEV, dtype=dtype)[start:start + M * pitch].view(M, pitch)[:, :N] for _ in range(2))
+    gemm.gemm_tn(a, b, out=want, splits=split)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before, held = _lib.launches(), torch.cuda.memory_allocated()
+    gemm.gemm_tn(a, b, out=got)
+    assert _lib.launches() - before == (2 if split > 1 else 1)
+    assert split > 1 or torch.cuda.max_memory_allocated() == held
+    assert torch.equal(got, want)
+
+
 def test_gemm_scratch_belongs_to_one_product():
     """Products in pieces share no scratch: threads on one stream, each between whose two launches another's may come, and a captured
     product that is replayed after a larger one on its stream, with the memory in between handed to others.  All bits as alone."""
