@@ -425,7 +425,7 @@ __global__ void sb_tot_kernel(const __nv_bfloat16* __restrict__ O, const __nv_bf
 // (special functions 61 % of their peak): the scores of the next tile and a second tile of weights are there, so that they
 // wait for no product, and the weights of eight keys are finished while the next eight's exponentials and reciprocals run.
 // Eight rows of 4,096 tokens, 16 heads: 128 keys at a time with one tile of scores and weights 1.00 ms, eights finished under the
-// next 0.94, two tiles of 64 keys 0.85 (and one reciprocal for two keys 0.80).
+// next 0.94, two tiles of 64 keys 0.85 (and one reciprocal for two keys 0.82).
 struct FwdParams {
   const int* cu_seqlens;
   const int* tile_list;

@@ -1,7 +1,8 @@
 """Stick-breaking attention: ``sb_attention(q, k, v, meta) -> (out, remainder)``.
 
 ``att_ij = sigmoid(l_ij) * prod_{j<m<i} (1 - sigmoid(l_im))`` for ``j < i`` inside one document, ``out = att @ v``,
-``remainder = 1 - sum_j att_ij``.  On CUDA (bf16, head dim 64) the tcgen05 kernels of ``csrc/sb_attention.cu`` run; packed documents are supported, which the reference layer does not offer
+``remainder = 1 - sum_j att_ij``.  On CUDA (bf16, head dim 64) the tcgen05 kernels of ``csrc/sb_attention.cu`` run, in which a logit
+counts as at most 2^100 : 1 (69.3); packed documents are supported, which the reference layer does not offer
 (custom_models/sba/sba_layer.py:84-87 asserts ``cu_seqlens is None``).  Elsewhere the definition is evaluated directly.
 """
 from __future__ import annotations

@@ -431,6 +431,25 @@ def test_stickbreaking_attention_at_tile_edges_and_far_out(size):
         assert torch.isfinite(a.grad).all() and (size > 1 or rel_err(a.grad, b.grad) < 3e-2)
 
 
+@pytest.mark.parametrize("nats", [1.0, 30.0, 41.0, 43.0, 55.0, 69.0])
+def test_stickbreaking_remainder_beside_dominating_keys(nats):
+    """What one or two keys of large logits leave of a row, relative to itself: the exponent's argument is rounded twice (100 2^-24), the
+    rest are a handful of fp32 roundings, 2^-17 together.  The two are neighbours that share a reciprocal, or are not; a logit counts up to 2^100 : 1."""
+    from flame_b200.ops.stickbreaking import sb_attention
+    n, H = 12, 2
+    q, k = torch.zeros(n, H, 64, device=DEV), torch.zeros(n, H, 64, device=DEV)
+    q[:, :, 0], k[3, 0, 0], k[2 if nats < 40 else 5, 1, 0] = 16.0, nats / 2, -nats / 2   # logits +-nats, the others 0
+    k[6, :, 0] = nats / 2 if nats < 40 else 0.0
+    q, k, v = q.bfloat16(), k.bfloat16(), torch.randn(n, H, 64, device=DEV).bfloat16()
+    o, rem = sb_attention(q, k, v, _meta([n]))
+    logits = torch.einsum("ihd,jhd->hij", q.double(), k.double()) / 8
+    stay = torch.nn.functional.logsigmoid(-logits).masked_fill(torch.ones(n, n, device=DEV, dtype=torch.bool).triu(), 0.0)
+    want = stay.sum(-1).exp()
+    rem = rem if rem.shape == want.shape else rem.t()
+    assert want.min() > 1e-36
+    assert ((rem.double() - want).abs() <= 2.0 ** -17 * want).all()
+
+
 def test_short_conv_forward_backward():
     from flame_b200.ops import linear_attn as la
     from flame_b200.ops.conv import short_conv
