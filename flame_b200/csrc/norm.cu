@@ -271,6 +271,9 @@ rmsnorm_fwd_short_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat1
 // of two trips sets BR, and 80 where a gate leaves more to compute and three CTAs pay: 98,304 rows of 512 with a gate 118 -> 101 us,
 // 262,144 of 256 142 -> 130 (of the chunk layout 156 -> 148), 65,536 of 320 77 -> 66, of 1,024 with a residual 111 -> 101, 32,768 of 2,048
 // 95 -> 89.  Gated rows of a whole CTA are slower with it (150 -> 158) and keep two rows and no lead.
+// Rows of up to 256 without gate and residual: two per trip while the operands stay in L2 (below 2^24 elements), 65,536 of 64 12.9 us and
+// 8,192 9.7 where four per trip take 13.3 and 11.4; four beyond, 1,048,576 of 64 73 us where two take 83.  A lead and four rows of 129 to 256
+// are more than the registers hold (spilled): 262,144 of 256 75 us without the lead, 90 with it.
 // dw partials: one row per CTA, which a second kernel sums in order.
 template <bool HAS_DRES, int GATE, int LPR, int BR, int TPB, bool MAP>
 __global__ void __launch_bounds__(TPB, TPB != 256 ? 1 : GATE && LPR ? 3 : 2)
@@ -279,7 +282,8 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    __nv_bfloat16* __restrict__ dx, __nv_bfloat16* __restrict__ dgate, float* __restrict__ dw_part, long long rows, int D,
                    int rows_per_cta, const Rows at) {
   constexpr int SLOTS = LPR ? WARPS * 32 / (LPR ? LPR : 1) : 1;
-  constexpr bool AHEAD = TPB == 256 && !(GATE && LPR == 0);  // the next trip's loads go out before this trip's sums
+  // the next trip's loads go out before this trip's sums
+  constexpr bool AHEAD = TPB == 256 && !(GATE && LPR == 0) && !(BR == 4 && LPR == 32);
   constexpr bool WIDE = LPR == 0 || LPR > 32;  // a row belongs to several warps
   __shared__ float s_c[WIDE ? 2 : 1][WIDE ? BR : 1][WIDE ? 32 : 1];
   __shared__ float s_dw[LPR ? SLOTS : 1][LPR ? LPR * 8 + 1 : 1];
@@ -588,12 +592,18 @@ int fb_rmsnorm_bwd_rows(const void* dy, const void* xin, const void* w, const fl
   (map ? rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB, true> : rmsnorm_bwd_kernel<HD, GM, LP, NR, TPB, false>)<<<parts, threads, 0, stream>>>( \
       (const __nv_bfloat16*)dy, (const __nv_bfloat16*)xin, (const __nv_bfloat16*)w, rstd, (const __nv_bfloat16*)gate, \
       (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dgate, dw_part, rows, D, rows_per_cta, at)
+  const bool four = rows * D >= (1ll << 24);
+#define BWD_S(HD, GM, LP)                                                                                         \
+  do {                                                                                                            \
+    if (!GM && !HD && four) BWD_N(HD, GM, LP, (GM || HD ? 2 : 4), 256);                                           \
+    else BWD_N(HD, GM, LP, (GM ? 1 : 2), 256);                                                                    \
+  } while (0)
   // rows per trip by what the registers hold packed; one row and no lead where a CTA has more than eight warps to overlap (64 registers)
 #define BWD(HD, GM)                                                                                               \
   do {                                                                                                            \
-    if (D <= 64) BWD_N(HD, GM, 8, (GM ? 1 : HD ? 2 : 4), 256);                                                             \
-    else if (D <= 128) BWD_N(HD, GM, 16, (GM ? 1 : HD ? 2 : 4), 256);                                                      \
-    else if (D <= 256) BWD_N(HD, GM, 32, (GM ? 1 : HD ? 2 : 4), 256);                                                      \
+    if (D <= 64) BWD_S(HD, GM, 8);                                                                                \
+    else if (D <= 128) BWD_S(HD, GM, 16);                                                                         \
+    else if (D <= 256) BWD_S(HD, GM, 32);                                                                         \
     else if (D <= 512) BWD_N(HD, GM, 64, (GM ? 1 : 2), 256);                                                      \
     else if (D <= 2048) BWD_N(HD, GM, 0, 2, 256);                                                                 \
     else BWD_N(HD, GM, 0, 1, 1024);                                                                               \
@@ -606,6 +616,7 @@ int fb_rmsnorm_bwd_rows(const void* dy, const void* xin, const void* w, const fl
     BWD(false, 2);
   }
 #undef BWD
+#undef BWD_S
 #undef BWD_N
   int rc = fb::launch_ok("rmsnorm_bwd_kernel");
   if (rc) return rc;

@@ -287,6 +287,26 @@ def test_rmsnorm_backward_with_the_next_rows_on_their_way(D, rows, form):
         assert ((a.double() - b).abs() <= 2.0 ** -8 * b.abs() + 2.0 ** -18 * big).all(), b.shape
 
 
+@pytest.mark.parametrize("D", [56, 64, 128, 136, 256])
+@pytest.mark.parametrize("extra", [-1, 0, 5])
+def test_rmsnorm_backward_of_plain_rows_around_four_per_trip(D, extra):
+    """Short rows without gate and residual around the 2^24 elements from which a trip takes four of them; dx as in the tests above, dw: a sum of
+    all rows in fp32, at most 500 terms one after the other in a thread and as many partial sums (2^-24 of the sum of absolutes each)."""
+    from flame_b200.ops.norm import rms_norm
+    torch.manual_seed(D)
+    rows = -(-(1 << 24) // D) + extra
+    x, w = (torch.randn(*s, device=DEV).to(torch.bfloat16).requires_grad_(True) for s in ((rows, D), (D,)))
+    dy = torch.randn(rows, D, device=DEV).to(torch.bfloat16)
+    dx, dw = torch.autograd.grad(rms_norm(x, w, 1e-5), (x, w), dy)
+    v, g = x.detach().double(), dy.double()
+    rstd = torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-5)
+    gw = g * w.detach().double()
+    want = rstd * (gw - v * rstd * (gw * v * rstd).mean(-1, keepdim=True))
+    assert ((dx.double() - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -18 * want.abs().amax(-1, keepdim=True)).all()
+    terms = g * v * rstd
+    assert ((dw.double() - terms.sum(0)).abs() <= 2.0 ** -8 * terms.sum(0).abs() + 1000 * 2.0 ** -24 * terms.abs().sum(0)).all()
+
+
 @pytest.mark.parametrize("D", [264, 512, 520, 1024, 1032, 2048, 2056])
 @pytest.mark.parametrize("rows,form", [(1, "plain"), (9, "sum"), (777, "prenorm"), (777, "swish"), (777, "sigmoid"), (777, "bare")])
 def test_rmsnorm_forward_of_rows_in_registers(D, rows, form):
