@@ -349,8 +349,8 @@ cross_entropy_kernel(__nv_bfloat16* __restrict__ logits, const long long* __rest
 // The plain loss (no smoothing, scaling, capping or z-loss) of rows that fit the registers of their CTA: NV 16-byte vectors per
 // thread are loaded at once and stay packed, so a row is read from memory once, with the whole row in flight, and the maximum
 // needs no exponentials.  An SM holds two rows of 32,000 and loads one while it computes the other, so every instruction counts:
-// exponentials of pairs of floats, the maximum on packed bf16, and the target's entry put right by the thread that has it instead
-// of a comparison per element (17 -> 8 instructions per entry).  At an in-place copy's rate 12,289 rows of 32,000 take 236 us; they
+// sums and products of pairs of floats, the maximum on packed bf16, and the target's entry put right by the thread that has it instead
+// of a comparison per element (17 -> 9 instructions per entry).  At an in-place copy's rate 12,289 rows of 32,000 take 236 us; they
 // took 309, this takes 287.  Tried: CTAs that walk over rows with the next row on its way into shared memory (cp.async; 324: its
 // wait and the reads back cost more than the loads they hide), 1,024 threads with four vectors (385).  A CTA has as many threads as
 // the row can feed: 16,384 rows of 4,096 took 121 us with 512 threads, 77 with one vector each, 49 with 128 threads and four.
@@ -374,14 +374,10 @@ __device__ __forceinline__ uint64_t ce_mul(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-// e^(x - m) of two packed bf16, as __expf forms it
+// e^(x - m) of two packed bf16
 __device__ __forceinline__ uint64_t ce_exp(uint32_t w, uint64_t neg_m) {
-  constexpr float kLog2e = 1.4426950408889634f;
-  const uint64_t x = ce_pair(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-  float2 t = ce_split(ce_mul(ce_add(x, neg_m), ce_pair(kLog2e, kLog2e)));
-  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(t.x));
-  asm("ex2.approx.ftz.f32 %0, %0;" : "+f"(t.y));
-  return ce_pair(t.x, t.y);
+  const float2 t = ce_split(ce_add(ce_pair(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)), neg_m));
+  return ce_pair(__expf(t.x), __expf(t.y));
 }
 template <int NV, int TH>
 __global__ void __launch_bounds__(TH, (NV == 8 ? 1024 : NV == 4 ? 1536 : 2048) / TH)

@@ -621,6 +621,37 @@ def test_cross_entropy_by_threads_of_a_row(V):
     assert torch.equal((bad[rest].float() * 0.75).to(torch.bfloat16), got[rest])
 
 
+@pytest.mark.parametrize("V", [1000, 4096, 32000])
+@pytest.mark.parametrize("spread", [1.0, 20.0, 100.0])
+def test_cross_entropy_exponentials_far_below_the_maximum(V, spread):
+    """Logits down to 100 below the row's largest, loss and gradient against 64 bits.  __expf(y) is documented to be good to 2 + 1.173 |y| units
+    in the last place (2^-23); a gradient is that of its entry and that of the sum (of entries near the maximum, and V roundings),
+    two products, and bf16 twice (2^-7)."""
+    from flame_b200.ops.cross_entropy import cross_entropy
+    torch.manual_seed(V)
+    rows = 67
+    base = (-torch.rand(rows, V, device=DEV) * spread).to(torch.bfloat16)
+    base[:, 3] = 0.0
+    base[1] = -100.0
+    base[1, 8] = 0.0
+    lab = torch.randint(0, V, (rows,), device=DEV)
+    lab[2] = 3
+    ref = base.double().requires_grad_(True)
+    want_loss = torch.nn.functional.cross_entropy(ref, lab, reduction="none")
+    leaf = base.clone().requires_grad_(True)
+    loss = cross_entropy(leaf * 1.0, lab)
+    (got,) = torch.autograd.grad(loss, leaf)
+    (want,) = torch.autograd.grad(want_loss.mean(), ref)
+    loss, want_loss = loss.item(), want_loss.mean().item()
+    y = ref.detach() - ref.detach().amax(1, keepdim=True)
+    p = y.exp() / y.exp().sum(1, keepdim=True)
+    of_exp = (2 + 1.173 * y.abs()) * 2.0 ** -23
+    of_sum = (p * of_exp).sum(1, keepdim=True) + 2.0 ** -18   # at most 64 entries one after the other in a thread, then shuffles
+    bound = 2.0 ** -7 * want.abs() + (p * (of_exp + of_sum + 2.0 ** -22) + 2.0 ** -23 * (lab[:, None] == torch.arange(V, device=DEV))) / rows
+    assert ((got.double() - want).abs() <= bound + 1.2e-38).all()
+    assert abs(loss - want_loss) <= of_sum.max().item() + 2.0 ** -21 * want_loss
+
+
 @pytest.mark.parametrize("n", [1, 7, 8, 4096, 100003])
 def test_gradient_of_the_loss_as_a_factor(n):
     """The product with the scalar in device memory equals that of two bf16 tensors bit for bit; other forms take the tensors'."""
