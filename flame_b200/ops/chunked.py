@@ -318,10 +318,16 @@ def _state_scan(lay: ChunkLayout, alpha, x, dtype, reverse: bool) -> torch.Tenso
 _lib.register("fb_decay_scan", ([c_void_p] + [c_longlong] * 3 + [c_int]) * 2 + [c_void_p, c_int] + [c_void_p] * 5 + [c_int] * 6 + [c_void_p])
 
 
-# Microseconds a chunk takes where one document alone is walked, without and with the decay's gradient.  Product and scan have all chunks'
-# products side by side and take 20 us and ten bytes per state element at 5.5 TB/s.  GLA (4 heads of 128 x 256) at 65,536 tokens in 8
-# documents: forward 277 us against 101 here, backward 271 against 142; in 2 documents 300 against 287 and 327 against 482.
-WALK_US = 0.55, 0.95
+# Where the one kernel pays, without and with the decay's gradient, in microseconds: it takes a time per chunk of the longest document, however
+# many documents and heads there are beside it (until memory bounds it, far below the other form); product and scan have all chunks'
+# products side by side and take a time per state element, and some microseconds more of launches.  Measured at 161 combinations of 1,024 to
+# 65,536 tokens in 1 to 32 documents and 2 x 64 x 64 (heads x rows x columns), 4 x 64 x 256, 4 x 64 x 512, 4 x 128 x 256, 16 x 128 x 512,
+# 32 x 128 x 64 and 64 x 128 x 64 states: the rule's choice is the faster one or within 1 % of it forward, and the faster one or within 7 us
+# with the gradient (the worst: 24 for 18 at 1,024 tokens of 32 x 128 x 64).  4 x 128 x 256 at 65,536
+# tokens, one kernel and the other form: 8 documents 103 and 276 us, with the gradient 142 and 263; 2 documents 295 and 302, 489 and 322.
+# 2 x 64 x 64 at 16,384 tokens: 16 documents 13 and 14, 22 and 21; 4 documents 36 and 22, 63 and 28.
+# The two differ by roundings: going backwards the other form rounds the increments to bf16, this one keeps them in fp32.
+WALK_US = (0.55, 8.0, 2.1e-6), (1.05, 14.0, 1.9e-6)   # per chunk; launches, per state element
 
 
 def _rows_of_vectors(t: torch.Tensor) -> torch.Tensor:
@@ -332,6 +338,11 @@ def _rows_of_vectors(t: torch.Tensor) -> torch.Tensor:
     return t if ok else _lib.dense(t)
 
 
+def _walk_pays(lay: ChunkLayout, elements: int, gradient: bool) -> bool:
+    chunk, launches, element = WALK_US[gradient]
+    return lay.longest * chunk < launches + lay.NC * elements * element
+
+
 def _decay_states(lay: ChunkLayout, alpha, a, b, reverse: bool, with_state=None):
     """``_state_scan`` over the increments ``x_c = a_c^T b_c`` of operands ``[NC, heads, chunk, rows]`` and ``[NC, heads, chunk, cols]`` (heads of
     either may serve several of alpha's), in the operands' type.  ``with_state`` (contiguous, as the result): returns the pair of the result
@@ -340,8 +351,8 @@ def _decay_states(lay: ChunkLayout, alpha, a, b, reverse: bool, with_state=None)
     rows, cols, H = a.shape[3], b.shape[3], alpha.shape[1]
     per_row = alpha.dim() == 3
     if (lay.chunk == 64 and rows in (64, 128) and cols % 64 == 0 and cols > 0 and a.is_cuda and a.dtype == b.dtype == torch.bfloat16 and _lib.available()
-            and alpha.dtype == torch.float32 and alpha.is_contiguous() and lay.n_docs <= 65535 and lay.NC * H * rows < 1 << 31
-            and lay.longest * WALK_US[with_state is not None] < 20 + lay.NC * H * rows * cols * 1.8e-6):
+            and alpha.dtype == torch.float32 and alpha.is_contiguous() and max(lay.n_docs, H) <= 65535 and lay.NC * H * rows < 1 << 31
+            and _walk_pays(lay, H * rows * cols, with_state is not None)):
         a, b = _rows_of_vectors(a), _rows_of_vectors(b)
         out = torch.empty(lay.NC, H, rows, cols, dtype=a.dtype, device=a.device)
         part = None

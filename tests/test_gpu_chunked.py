@@ -617,6 +617,39 @@ def test_decay_states_in_one_kernel(rows, cols, Ha, Hb, per_row, reverse):
             assert ((dot.double() - terms.sum(dims)).abs() <= 2.0 ** -18 * terms.abs().sum(dims)).all()
 
 
+@pytest.mark.parametrize("lens", [[3900], [70, 3900, 1], [65] * 60])
+def test_decay_states_both_ways_of_forming_them(lens, monkeypatch):
+    """A long document, which the rule leaves to product and scan, and many short ones, which it gives to the one kernel, each formed in both
+    ways against the loop in fp64: states rounded once (2^-8) after fp32 sums of at most 3,900 terms (1e-3), where the increments are
+    rounded too (product and scan backwards) by as much again, each at its own size; the decay's gradient: sums of products of two bf16 states."""
+    from flame_b200.ops import chunked
+    torch.manual_seed(5)
+    H, R, W = 2, 64, 128
+    lay = chunked.ChunkLayout(_meta(lens))
+    alpha = torch.rand(lay.NC, H, R, device=DEV)
+    a, b = _bf(lay.NC, H, 64, R), _bf(lay.NC, H, 64, W)
+    S = _bf(lay.NC, H, R, W)
+    assert [chunked._walk_pays(lay, H * R * W, g) for g in (False, True)] == [len(lens) == 60] * 2
+    x = a.double().transpose(-1, -2) @ b.double()
+    one_kernel, other = ((0.0, 1.0, 1.0),) * 2, ((1.0, 0.0, 0.0),) * 2
+    for reverse in (False, True):
+        want, size, c = torch.zeros_like(x), torch.zeros_like(x), 0
+        for n in lens:
+            k, s, z = (n + 63) // 64, torch.zeros_like(x[0]), torch.zeros_like(x[0])
+            for i in (range(c + k - 1, c - 1, -1) if reverse else range(c, c + k)):
+                want[i], size[i] = s, z
+                s, z = alpha[i].double()[..., None] * s + x[i], alpha[i].double()[..., None] * z + x[i].abs()
+            c += k
+        for rule in (one_kernel, other):
+            monkeypatch.setattr(chunked, "WALK_US", rule)
+            got = chunked._decay_states(lay, alpha, a, b, reverse)
+            rounded = 2.0 ** -8 * size if rule is other and reverse else 0
+            assert ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + rounded + 1e-3).all()
+            again, dot = chunked._decay_states(lay, alpha, a, b, reverse, S)
+            terms = got.double() * S.double()
+            assert torch.equal(again, got) and ((dot.double() - terms.sum(-1)).abs() <= 2.0 ** -18 * terms.abs().sum(-1)).all()
+
+
 @pytest.mark.parametrize("reverse", [False, True])
 @pytest.mark.parametrize("x16", [False, True])
 @pytest.mark.parametrize("rows,cols,per_row", [(3, 12, True), (4, 8, False), (16, 72, True)])
