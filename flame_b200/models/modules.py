@@ -137,7 +137,10 @@ class GatedMLP(nn.Module):
             y = linear_ops.gated_mlp(x, self.gate_proj.weight, self.up_proj.weight, self.down_proj.weight)
             if y is not None:
                 return y
-        return self.down_proj(activations.swiglu(fused_projection(x, (self.gate_proj, self.up_proj))))
+        z = linear_ops.gate_up_swiglu(x, self.gate_proj.weight, self.up_proj.weight)
+        if z is None:
+            z = activations.swiglu(fused_projection(x, (self.gate_proj, self.up_proj)))
+        return self.down_proj(z)
 
 
 class ShortConvolution(nn.Module):

@@ -318,7 +318,7 @@ def _gate_up_grads(dgu, x2, wg, wu, params, need, dx=None):
 
 
 class _GateUpSwiGLU(torch.autograd.Function):
-    """``z = silu(x @ Wg.T) * (x @ Wu.T)``, see ``_gate_up``."""
+    """``z = silu(x @ Wg.T) * (x @ Wu.T)``, see ``_gate_up``; what is left of ``_GatedMLP`` where the down projection is a call of its own."""
 
     @staticmethod
     def forward(ctx, x, wg, wu):
@@ -402,7 +402,8 @@ def _swiglu_epilogue_ok(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor) -> 
 
 def gate_up_swiglu(x: torch.Tensor, wg: torch.Tensor, wu: torch.Tensor) -> Optional[torch.Tensor]:
     """``silu(x @ Wg.T) * (x @ Wu.T)`` from one product (bf16 on the GPU, adjacent weights, I a multiple of 128, no fp8 weights, no
-    selective-checkpointing tape, which counts products); ``None`` tells the caller to take the two-step path."""
+    selective-checkpointing tape, which counts products), for a down projection that does more than a product: a bias, a hook, a
+    forward of its own; ``None`` tells the caller to take the two-step path."""
     return _GateUpSwiGLU.apply(x, wg, wu) if _swiglu_epilogue_ok(x, wg, wu) else None
 
 

@@ -218,32 +218,33 @@ def bench_elementwise(args) -> None:
 
 
 def bench_swiglu(args) -> None:
-    """gate | up projection + SwiGLU: the GEMM with the activation in its epilogue against GEMM + elementwise kernel."""
+    """SwiGLU MLP: the node with both activations in the GEMMs' epilogues against GEMMs + elementwise kernels."""
     from flame_b200.ops import activations, linear as linear_ops
     _, peak, tag = peaks()
     T, D, I = args.tokens, 1024, 2816
     x = torch.randn(T, D, device="cuda", dtype=torch.bfloat16).requires_grad_(True)
     w = (torch.randn(2 * I, D, device="cuda", dtype=torch.bfloat16) * 0.02)
+    wd = (torch.randn(D, I, device="cuda", dtype=torch.bfloat16) * 0.02).requires_grad_(True)
     wg, wu = w[:I].detach().requires_grad_(True), w[I:].detach().requires_grad_(True)
     wg.data, wu.data = w[:I], w[I:]   # adjacent in memory, like the parameters of a unit
-    dz = torch.randn(T, I, device="cuda", dtype=torch.bfloat16)
-    fl = 2.0 * T * 2 * I * D
+    dy = torch.randn(T, D, device="cuda", dtype=torch.bfloat16)
+    fl = 2.0 * T * 3 * I * D
 
     def fused():
-        return linear_ops.gate_up_swiglu(x, wg, wu)
+        return linear_ops.gated_mlp(x, wg, wu, wd)
 
     def unfused():
-        return activations.swiglu(linear_ops.linear_fused(x, [wg, wu]))
+        return linear_ops.linear(activations.swiglu(linear_ops.linear_fused(x, [wg, wu])), wd)
 
-    for name, fn in (("GEMM with SwiGLU epilogue", fused), ("GEMM + swiglu kernel", unfused)):
+    for name, fn in (("GEMMs with SwiGLU epilogues", fused), ("GEMMs + swiglu kernels", unfused)):
         def nograd():
             with torch.no_grad():
                 return fn()
         f = timeit(nograd, iters=args.iters)
 
         def fb():
-            x.grad = wg.grad = wu.grad = None
-            fn().backward(dz)
+            x.grad = wg.grad = wu.grad = wd.grad = None
+            fn().backward(dy)
         b = timeit(fb, iters=args.iters)
         print(f"  {name:28s} fwd {f:.3f} ms ({fl / f / 1e9:5.0f} TF, {fl / f / 1e-3 / peak:.2f} {tag})   fwd+bwd {b:.3f} ms")
 

@@ -880,9 +880,8 @@ def test_cross_entropy_options_match_the_written_out_loss(opts):
     assert rel_err(lg2.grad, lf.grad) < 3e-2
 
 
-def test_gate_up_projection_with_swiglu_epilogue(monkeypatch):
+def test_gate_up_projection_with_swiglu_epilogue():
     """The fused gate | up GEMM with the activation in its epilogue against the GEMM followed by the SwiGLU kernel."""
-    monkeypatch.setenv("FLAME_B200_FUSED_SWIGLU", "1")   # the fused form is opt-in: it measured slower than the two kernels
     from flame_b200.ops.activations import swiglu
     from flame_b200.ops.linear import gate_up_swiglu, linear_fused
     torch.manual_seed(12)
@@ -936,6 +935,34 @@ def test_gated_mlp_in_one_node(T, K, I, grads):
         assert rel_err(w.main_grad - 1 if hasattr(w, "main_grad") else w.grad, r.grad) < 1.5e-2
     if grads == "apart":
         assert torch.equal(acc[:, I * K:], torch.ones(3, I * K, device=DEV))
+
+
+@pytest.mark.parametrize("how", ["hook", "bias"])
+def test_mlp_whose_down_projection_is_a_call_of_its_own(how):
+    """A hook on the down projection is called, a bias of its own is added, and all else equals the MLP in one node bit for bit."""
+    from flame_b200.models.modules import GatedMLP
+    from flame_b200.ops import linear as ops
+    torch.manual_seed(3)
+    D, I, T = 64, 256, 300
+    flat = (torch.randn(3 * I * D, device=DEV) * 0.1).to(torch.bfloat16)
+    mlp = GatedMLP(D, I)
+    for i, m in enumerate((mlp.gate_proj, mlp.up_proj, mlp.down_proj)):
+        m.weight = torch.nn.Parameter(flat[i * I * D:(i + 1) * I * D].view(m.weight.shape))
+    x, dy = (torch.randn(T, D, device=DEV).to(torch.bfloat16).requires_grad_(i == 0) for i in range(2))
+    ins = [x, mlp.gate_proj.weight, mlp.up_proj.weight, mlp.down_proj.weight]
+    assert ops.gated_mlp(*ins) is not None
+    want = mlp(x)
+    grads = torch.autograd.grad(want, ins, dy)
+    seen = []
+    if how == "hook":
+        mlp.down_proj.register_forward_hook(lambda m, i, o: seen.append(i[0].shape))
+    else:
+        mlp.down_proj.bias = torch.nn.Parameter(torch.ones(D, device=DEV, dtype=torch.bfloat16))
+    got = mlp(x)
+    again = torch.autograd.grad(got, ins, dy)
+    assert seen == [(T, I)] * (how == "hook")
+    assert torch.equal(got, want) if how == "hook" else rel_err(got, want.float() + 1) < 2 ** -8
+    assert all(torch.equal(a, b) for a, b in zip(again, grads))
 
 
 @pytest.mark.gpu
