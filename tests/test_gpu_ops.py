@@ -965,6 +965,78 @@ def test_mlp_whose_down_projection_is_a_call_of_its_own(how):
     assert all(torch.equal(a, b) for a, b in zip(again, grads))
 
 
+@pytest.mark.parametrize("grads", ["autograd", "main_grad"])
+@pytest.mark.parametrize("reentrant", [False, True])
+def test_mlp_in_one_node_under_activation_checkpointing(grads, reentrant):
+    """Recomputed in the backward pass, where the saved weights are other tensors than the parameters: output and gradients, which go to
+    main_grad or to autograd, equal those without, bit for bit."""
+    from torch.utils.checkpoint import checkpoint
+    from flame_b200.ops import linear as ops
+    torch.manual_seed(4)
+    D, I, T = 64, 256, 300
+    flat = (torch.randn(3 * I * D, device=DEV) * 0.1).to(torch.bfloat16)
+    x, dy = (torch.randn(T, D, device=DEV).to(torch.bfloat16) for _ in range(2))
+
+    def run(fn):
+        ws = [torch.nn.Parameter(flat[i * I * D:(i + 1) * I * D].view((I, D) if i < 2 else (D, I))) for i in range(3)]
+        acc = torch.zeros(3 * I * D, device=DEV)
+        if grads == "main_grad":
+            for i, w in enumerate(ws):
+                w.main_grad = acc[i * I * D:(i + 1) * I * D].view(w.shape)
+        leaf = x.clone().requires_grad_(True)
+        y = fn(lambda t: ops.gated_mlp(t, *ws), leaf)
+        y.backward(dy)
+        assert all((w.grad is None) == (grads == "main_grad") for w in ws)
+        return [y.detach(), leaf.grad, acc] + [w.grad for w in ws if w.grad is not None]
+
+    want = run(lambda f, t: f(t))
+    assert want[2].any() == (grads == "main_grad")
+    assert all(torch.equal(a, b) for a, b in zip(run(lambda f, t: checkpoint(f, t, use_reentrant=reentrant)), want))
+
+
+@pytest.mark.parametrize("covered", [True, False])
+def test_mlp_in_one_node_whose_weights_are_still_to_be_gathered(covered):
+    """The unit's weights lie in a shard (of a world of one) and their place holds NaN: the first product of the forward pass that reads them
+    fetches them on its way, and so does the backward's; a gather that does not cover the weight is flushed before.  All bits as with
+    the weights in place, and no gather is left behind."""
+    import numpy as np
+    from flame_b200.ops import gemm, linear as ops
+    torch.manual_seed(5)
+    D, I, T, shift = 256, 384, 700, 14
+    n = 3 * I * D
+    shard = (torch.randn(n, device=DEV) * 0.1).to(torch.bfloat16)
+    assert n * 2 % (1 << shift) == 0
+    flat = shard.clone()
+    ws = [torch.nn.Parameter(flat[i * I * D:(i + 1) * I * D].view((I, D) if i < 2 else (D, I))) for i in range(3)]
+    x, dy = (torch.randn(T, D, device=DEV).to(torch.bfloat16).requires_grad_(i == 0) for i in range(2))
+    want = ops.gated_mlp(x, *ws)
+    grads = torch.autograd.grad(want, [x, *ws], dy)
+    flags, flushed = torch.zeros((n * 2 >> shift) + 1, dtype=torch.int32, device=DEV), []
+
+    def pend(epoch, lo, hi):
+        flat.data.fill_(float("nan"))
+
+        def flush():
+            flat.data.copy_(shard)
+            p.done = True
+            gemm.set_pending_gather(None)
+            flushed.append(epoch)
+        p = gemm.PendingGather(None, flat.data_ptr(), lo, hi, np.array([shard.data_ptr()], dtype=np.uint64), 1, 0, n * 2, shift, flags, epoch, flush)
+        gemm.set_pending_gather(p)
+        return p
+
+    try:
+        first = pend(1, 0, n * 2 if covered else I * D * 2)                       # not covered: ends before the up projection
+        got = ops.gated_mlp(x, *ws)
+        assert first.done and torch.equal(got, want) and flushed == ([] if covered else [1])
+        second = pend(2, 0 if covered else n * 2 - 16, n * 2)                     # not covered: begins inside the down projection
+        again = torch.autograd.grad(got, [x, *ws], dy)
+        assert second.done and all(torch.equal(a, b) for a, b in zip(again, grads)) and flushed == ([] if covered else [1, 2])
+        assert torch.equal(flat, shard)
+    finally:
+        gemm.set_pending_gather(None)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("with_lb", [False, True])
 def test_hgrn2_gate_kernels_match_the_elementwise_chain(with_lb):
