@@ -1504,7 +1504,7 @@ int fb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* lse
 int fb_attn_delta(const void* o, const void* dout, float* delta, long long T, int H, int DH, long long o_stride_t,
                   long long do_stride_t, cudaStream_t stream) {
   if (T == 0) return 0;
-  if (DH != 64 && DH != 128) return -2;
+  if ((DH != 64 && DH != 128) || !fb::aligned(16, o, dout)) return -2;
   const long long threads = T * H * (DH / 8);
   const unsigned blocks = (unsigned)((threads + 255) / 256);
   if (DH == 64)

@@ -930,7 +930,7 @@ int fb_rope(const void* x, void* y, const int* pos, const float* cos_t, const fl
             int rot, long long x_stride_t, long long y_stride_t, int seq_len_mod, int conj, int x_fp32,
             cudaStream_t stream) {
   if (T == 0) return 0;
-  if ((rot % 16) || (Dh % 8) || (x_stride_t % 8) || (y_stride_t % 8)) return -2;
+  if ((rot % 16) || (Dh % 8) || (x_stride_t % 8) || (y_stride_t % 8) || !fb::aligned(16, x, y, cos_t, sin_t)) return -2;
   // Below some 600,000 threads (four to a lane of the chip) a head each keeps more of them busy: 1,000 tokens of 24 heads 2.5 : 3.0 us.
   const long long each = T * H * (rot / 16);
   const int hpt = x_fp32 ? 2 : each < 600000 ? 1 : 4, G = (H + hpt - 1) / hpt;
@@ -952,7 +952,7 @@ int fb_rope(const void* x, void* y, const int* pos, const float* cos_t, const fl
 int fb_swiglu_fwd(const void* g, const void* u, void* a, long long T, int I, long long ld_g, long long ld_u,
                   long long ld_a, cudaStream_t stream) {
   if (T == 0) return 0;
-  if ((I % 8) || (ld_g % 8) || (ld_u % 8) || (ld_a % 8)) return -2;
+  if ((I % 8) || (ld_g % 8) || (ld_u % 8) || (ld_a % 8) || !fb::aligned(16, g, u, a)) return -2;
   const long long vec = I / 8, total = T * vec;
   const unsigned grid = (unsigned)((total + 511) / 512);
   if (total < (1ll << 31))
@@ -967,7 +967,8 @@ int fb_swiglu_bwd(const void* da, const void* g, const void* u, void* dg, void* 
                   long long ld_da, long long ld_g, long long ld_u, long long ld_dg, long long ld_du, long long ld_a,
                   cudaStream_t stream) {
   if (T == 0) return 0;
-  if ((I % 8) || (ld_da % 8) || (ld_g % 8) || (ld_u % 8) || (ld_dg % 8) || (ld_du % 8) || (ld_a % 8)) return -2;
+  if ((I % 8) || (ld_da % 8) || (ld_g % 8) || (ld_u % 8) || (ld_dg % 8) || (ld_du % 8) || (ld_a % 8) || !fb::aligned(16, da, g, u, dg, du, a_out))
+    return -2;
   const long long vec = I / 8, total = T * vec;
   const unsigned grid = (unsigned)((total + 511) / 512);
   if (total < (1ll << 31))
@@ -1052,7 +1053,7 @@ int fb_mean_loss(const float* rows, long long n, const int* n_valid, float* out,
 int fb_embedding_fwd(const long long* ids, const void* table, void* out, long long T, int D, long long V,
                      cudaStream_t stream) {
   if (T == 0) return 0;
-  if (D % 8) return -2;
+  if (D % 8 || !fb::aligned(16, table, out)) return -2;
   embedding_fwd_kernel<<<blocks_for(T * (D / 8), 256), 256, 0, stream>>>(ids, (const __nv_bfloat16*)table,
                                                                         (__nv_bfloat16*)out, T, D, V);
   return fb::launch_ok("embedding_fwd_kernel");
@@ -1060,7 +1061,7 @@ int fb_embedding_fwd(const long long* ids, const void* table, void* out, long lo
 int fb_embedding_bwd_sorted(const long long* sorted_ids, const long long* perm, long long T, const void* dout, float* dtable, int D,
                             long long V, cudaStream_t stream) {
   if (T == 0) return 0;
-  if (D % 8) return -2;
+  if (D % 8 || !fb::aligned(16, dout, dtable)) return -2;
   embedding_bwd_sorted_kernel<<<(unsigned)((T * 32 + 255) / 256), 256, 0, stream>>>(sorted_ids, perm, T, (const __nv_bfloat16*)dout, dtable, D, V);
   return fb::launch_ok("embedding_bwd_sorted_kernel");
 }

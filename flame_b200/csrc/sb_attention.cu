@@ -695,6 +695,7 @@ int fb_sb_attn_bwd(const void* q, const void* k, const void* v, const void* o, c
   if (T == 0) return 0;
   if ((q_stride_t % 8) || (k_stride_t % 8) || (v_stride_t % 8) || (o_stride_t % 8) || (do_stride_t % 8) || (dq_stride_t % 8))
     return -3;
+  if (!fb::aligned(16, o, o_lo, dout, dq)) return -2;
   {
     const long long threads = T * H * (DH / 8);
     sb_tot_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, stream>>>((const __nv_bfloat16*)o, (const __nv_bfloat16*)o_lo,

@@ -27,8 +27,7 @@ class _SwiGLUFn(torch.autograd.Function):
     def forward(ctx, gu):
         shape = gu.shape
         I = shape[-1] // 2
-        gu2 = gu.reshape(-1, 2 * I)
-        gu2 = gu2 if gu2.is_contiguous() else gu2.contiguous()
+        gu2 = _lib.dense(gu.reshape(-1, 2 * I))
         T = gu2.shape[0]
         a = swiglu_forward(gu2, torch.empty(T, I, dtype=gu.dtype, device=gu.device))
         ctx.save_for_backward(gu2)
@@ -38,9 +37,7 @@ class _SwiGLUFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, da):
         (gu2,) = ctx.saved_tensors
-        da2 = da.reshape(-1, gu2.shape[1] // 2)
-        da2 = da2 if da2.is_contiguous() else da2.contiguous()
-        return swiglu_backward(da2, gu2).view(ctx.shape)
+        return swiglu_backward(_lib.dense(da.reshape(-1, gu2.shape[1] // 2)), _lib.dense(gu2)).view(ctx.shape)
 
 
 def swiglu_forward(gu2: torch.Tensor, a: torch.Tensor) -> torch.Tensor:

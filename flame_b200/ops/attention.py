@@ -87,7 +87,7 @@ class _AttnFn(torch.autograd.Function):
         meta = ctx.meta
         T, H, Dh = q.shape
         Hkv = k.shape[1]
-        do = do.contiguous()
+        do = _lib.dense(do)
         L = _lib.lib()
         delta = torch.empty(H, T, dtype=torch.float32, device=q.device)
         rc = L.fb_attn_delta(o.data_ptr(), do.data_ptr(), delta.data_ptr(), T, H, Dh, o.stride(0), do.stride(0),

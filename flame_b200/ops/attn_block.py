@@ -55,7 +55,7 @@ class _QkvAttnFn(torch.autograd.Function):
         q, k = qk[:, :H], qk[:, H:]
         v = qkv[:, (H + Hkv) * Dh:].view(T, Hkv, Dh)
         do = do.reshape(T, H, Dh)
-        do = do if do.is_contiguous() else do.contiguous()
+        do = _lib.dense(do)
         L = _lib.lib()
         delta = torch.empty(H, T, dtype=torch.float32, device=qkv.device)
         rc = L.fb_attn_delta(o.data_ptr(), do.data_ptr(), delta.data_ptr(), T, H, Dh, o.stride(0), do.stride(0),

@@ -38,7 +38,7 @@ class _EmbeddingFn(torch.autograd.Function):
         V, D = weight.shape
         T = flat.numel()
         d2 = dout.reshape(T, D)
-        d2 = d2 if d2.is_contiguous() else d2.contiguous()
+        d2 = _lib.dense(d2)
         sorted_ids, perm = torch.sort(flat, stable=True)
         mg = getattr(weight, "main_grad", None)
         dtable = mg if mg is not None else torch.zeros(V, D, dtype=torch.float32, device=weight.device)

@@ -334,8 +334,7 @@ class _GateUpSwiGLU(torch.autograd.Function):
     def backward(ctx, dz):
         from .activations import swiglu_backward
         x2, gu, wg, wu = ctx.saved_tensors
-        dz2 = dz.reshape(-1, wg.shape[0])
-        dgu = swiglu_backward(dz2 if dz2.is_contiguous() else dz2.contiguous(), gu)
+        dgu = swiglu_backward(_lib.dense(dz.reshape(-1, wg.shape[0])), _lib.dense(gu))
         dx, gg, gu_ = _gate_up_grads(dgu, x2, wg, wu, ctx.params, ctx.needs_input_grad)
         return None if dx is None else dx.view(ctx.shape), gg, gu_
 

@@ -49,7 +49,7 @@ def rope_inplace_(x: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: to
     """In-place rotation of a ``[T, H, Dh]`` view (token stride arbitrary, head stride Dh)."""
     T, H, Dh = x.shape
     rot = 2 * cos.shape[1]
-    if _lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and rot % 16 == 0:
+    if _lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and rot % 16 == 0 and x.data_ptr() % 16 == 0:
         assert x.stride(2) == 1 and x.stride(1) == Dh
         rc = _lib.lib().fb_rope(x.data_ptr(), x.data_ptr(), pos.data_ptr(), cos.data_ptr(), sin.data_ptr(), T, H, Dh, rot,
                                 x.stride(0), x.stride(0), 0, 1 if conj else 0, 0, _lib.stream_ptr())
@@ -63,7 +63,7 @@ def rope_rotated(x: torch.Tensor, pos: torch.Tensor, cos: torch.Tensor, sin: tor
     """The rotation of a ``[T, H, Dh]`` view (as ``rope_inplace_``) in a tensor of its own, in one pass; no autograd."""
     T, H, Dh = x.shape
     rot = 2 * cos.shape[1]
-    if not (_lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and rot == Dh and rot % 16 == 0):
+    if not (_lib.available() and x.is_cuda and x.dtype == torch.bfloat16 and rot == Dh and rot % 16 == 0 and x.data_ptr() % 16 == 0):
         y = x.clone(memory_format=torch.contiguous_format)
         rope_inplace_(y, pos, cos, sin)
         return y

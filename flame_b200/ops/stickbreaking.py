@@ -64,7 +64,7 @@ class _SBFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, do, drem):
         q, k, v, o, rem, o_lo = ctx.saved_tensors
-        do = do if do.is_contiguous() else do.contiguous()
+        do = _lib.dense(do)
         dr = None
         if drem is not None and ctx.needs_input_grad[0]:
             dr = drem.t().contiguous().float()
@@ -90,7 +90,7 @@ class _QkvSBFn(torch.autograd.Function):
         qkv, o, rem, o_lo = ctx.saved_tensors
         T, (H, Dh) = qkv.shape[0], ctx.dims
         q, k, v = qkv.view(T, 3, H, Dh).unbind(1)
-        do = do if do.is_contiguous() else do.contiguous()
+        do = _lib.dense(do)
         dqkv = torch.empty_like(qkv).view(T, 3, H, Dh)
         dkv = _backward(q, k, v, o, o_lo, rem, do, None, ctx.meta, ctx.scale, dqkv[:, 0])
         rc = _lib.lib().fb_cast_column_blocks(dkv.data_ptr(), dqkv[:, 1].data_ptr(), T, H * Dh, dqkv.stride(0), _lib.stream_ptr())

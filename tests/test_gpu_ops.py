@@ -369,6 +369,54 @@ def test_rope_heads_of_one_thread(H, Dh, rot, many):
         check(x, f, -1)
 
 
+@pytest.mark.parametrize("op", ["swiglu", "gate_up", "embedding", "attention64", "attention128", "qkv_attention", "stickbreaking", "qkv_stickbreaking"])
+def test_gradients_that_start_between_vectors(op):
+    """A whole gradient that begins off a 16-byte boundary gives what one on a boundary gives (attention adds dq up in no fixed order)."""
+    from flame_b200.ops.activations import swiglu
+    from flame_b200.ops.attention import attention
+    from flame_b200.ops.attn_block import qkv_attention
+    from flame_b200.ops.embedding import embedding
+    from flame_b200.ops.linear import gate_up_swiglu
+    from flame_b200.ops.stickbreaking import sb_attention, sb_qkv_attention
+    torch.manual_seed(2)
+    T, H, meta = 200, 2, _meta([77, 123])
+    leaf = lambda *s: torch.randn(*s, device=DEV).to(torch.bfloat16).requires_grad_(True)  # noqa: E731
+    D = 128 if op == "attention128" else 64
+    w = leaf(2 * 128, 64)
+    ins, run = {
+        "swiglu": ([leaf(T, 256)], swiglu),
+        "gate_up": ([leaf(T, 64)], lambda x: gate_up_swiglu(x, w.detach()[:128], w.detach()[128:])),
+        "embedding": ([leaf(50, 64)], lambda t: embedding(torch.arange(T, device=DEV) % 50, t)),
+        "qkv_attention": ([leaf(T, 3 * H * 64)], lambda x: qkv_attention(x, meta, H, H, 64)),
+        "stickbreaking": ([leaf(T, H, 64) for _ in range(3)], lambda q, k, v: sb_attention(q, k, v, meta)[0]),
+        "qkv_stickbreaking": ([leaf(T, 3 * H * 64)], lambda x: sb_qkv_attention(x, meta, H, 64)),
+    }.get(op, ([leaf(T, H, D) for _ in range(3)], lambda q, k, v: attention(q, k, v, meta)))
+    y = run(*ins)
+    y = y[0] if isinstance(y, tuple) else y
+    dy = torch.randn(y.shape, device=DEV).to(torch.bfloat16)
+    odd = torch.empty(y.numel() + 3, device=DEV, dtype=torch.bfloat16)[3:].view(y.shape).copy_(dy)
+    assert odd.data_ptr() % 16
+    want = torch.autograd.grad(y, ins, dy, retain_graph=True)
+    for a, b in zip(torch.autograd.grad(y, ins, odd), want):
+        assert rel_err(a, b) < (2 ** -9 if "att" in op or "stick" in op else 1e-9)
+
+
+def test_activations_and_rotations_between_vectors():
+    """Whole operands that begin off a 16-byte boundary."""
+    from flame_b200.ops.activations import swiglu
+    from flame_b200.ops.rope import rope_inplace_, rope_rotated
+    torch.manual_seed(2)
+    x = torch.randn(200, 256, device=DEV).to(torch.bfloat16)
+    odd = torch.empty(x.numel() + 3, device=DEV, dtype=torch.bfloat16)[3:].view(x.shape).copy_(x)
+    assert torch.equal(swiglu(odd), swiglu(x))
+    pos = torch.arange(200, device=DEV, dtype=torch.int32)
+    ang = torch.rand(200, 32, device=DEV)
+    want = rope_rotated(x.view(200, 4, 64), pos, ang.cos(), ang.sin())
+    assert rel_err(rope_rotated(odd.view(200, 4, 64), pos, ang.cos(), ang.sin()), want) < 2 ** -8
+    rope_inplace_(odd.view(200, 4, 64), pos, ang.cos(), ang.sin())
+    assert rel_err(odd.view(200, 4, 64), want) < 2 ** -8
+
+
 def test_swiglu_rope_embedding():
     from flame_b200.ops.activations import swiglu, swiglu_reference
     from flame_b200.ops.embedding import embedding
