@@ -121,18 +121,19 @@ def _launch(a, b, M, N, K, a_mn, b_mn, out, accumulate, alpha, bias, splits):
         if pend.touches(a) or pend.touches(b):
             pend.flush()  # this product reads the unit but cannot carry the gather: fetch with the stand-alone kernel
     ws, launches = None, 1
+    dst, ldc = out.data_ptr(), out.stride(0)
     if splits is None:
-        need = L.fb_gemm_cut_bytes_into(out.data_ptr(), out.stride(0), mode, M, N, K) if bias is None else -1
+        need = L.fb_gemm_cut_bytes_into(dst, ldc, mode, M, N, K) if bias is None else -1
         if need >= 0:   # the CTA pairs cut the tiles of their last round along K where that pays
             splits = 0
             if need:
                 ws, launches = _workspace(out.device, need), 2
         else:
-            splits = int(L.fb_gemm_pick_splits(M, N, K)) if out.stride(0) == N and (M * N) % 4 == 0 else 1
+            splits = int(L.fb_gemm_pick_splits(M, N, K)) if ldc == N and (M * N) % 4 == 0 else 1
     if splits > 1:
         launches = 2
         ws = _workspace(out.device, int(L.fb_gemm_workspace_bytes(M, N, splits)))
-    rc = L.fb_gemm_bf16(a.data_ptr(), b.data_ptr(), out.data_ptr(), M, N, K, a.stride(0), b.stride(0), out.stride(0),
+    rc = L.fb_gemm_bf16(a.data_ptr(), b.data_ptr(), dst, M, N, K, a.stride(0), b.stride(0), ldc,
                         int(a_mn), int(b_mn), mode, float(alpha), _lib.ptr(bias), int(splits), _lib.ptr(ws),
                         _lib.stream_ptr())
     _lib.check(rc, "fb_gemm_bf16")
