@@ -19,7 +19,8 @@
 // shuffles), sweep (6) gives it 4 channels x 4 states (see there); pairs of states, or of channels, use the packed fp32x2
 // instructions.  Every sweep fetches its operands ahead: waiting for memory at each group of steps, not the MUFU, set the pace
 // before.  At that size with gate and softplus, before and after: (1) 0.44 -> 0.31 ms, (3) 0.84 -> 0.47, (4) 0.59 -> 0.36,
-// (6) 2.17 -> 1.63 -> 1.26.
+// (6) 2.17 -> 1.63 -> 1.26.  (1) and (4) keep the MUFU 80 and 78 % busy.  (3) keeps it and the issue slots at 59 % (126 registers leave 15
+// warps an SM, whose stalls are fixed latencies); an eighth of its decays as polynomials on the multiply-add pipe made it 40 us slower.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -479,7 +479,7 @@ def test_stickbreaking_attention_forward_backward(lens, H):
 @pytest.mark.parametrize("size", [1.0, 6.0])
 def test_stickbreaking_attention_at_tile_edges_and_far_out(size):
     """Documents around the 64-key and 128-query tiles against fp64, with logits of some units and of some forty (neighbours beyond 2^60 : 1,
-    where the weights are 0 or 1 and the kernels cut off): outputs and value gradients of bf16 weights and operands, 1e-2; gradients
+    where the weights are 0 or 1): outputs and value gradients of bf16 weights and operands, 1e-2; gradients
     through the logits, small differences of their sums, 3e-2 where the weights are not saturated, and finite."""
     from flame_b200.ops.linear_attn import stickbreaking_reference
     from flame_b200.ops.stickbreaking import sb_attention
