@@ -124,8 +124,9 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 
 // The same for rows that a warp's registers hold (D <= 2048): NV vectors per lane of every operand, loaded at once and kept packed,
 // so nothing is read twice and the second sweep waits for nothing: 32,768 rows of 2,048 65 -> 49 us, 65,536 of 1,024 64 -> 47 (with a
-// residual 94 -> 86), 98,304 of 512 55 -> 37, with a gate 65 -> 59.  A gate of 2,048 leaves too few warps (84 -> 88): that and wider rows
-// take the form above.
+// residual 94 -> 86), 98,304 of 512 55 -> 37, with a gate 65 -> 59.  Vectors that a row does not fill cost warps: with a gate, three per lane
+// for rows of up to 768 (131,072 of 520: 102 us with four, 84 with three, 92 by the form above), with a residual five for up to 1,280 (65,536
+// of 1,152: 113 with eight, 91, 104).  A gate of 2,048 leaves too few warps (84 -> 88): that and wider rows take the form above.
 template <bool HAS_RES, bool WRITE_RES, int GATE, int NV>
 __global__ void __launch_bounds__(WARPS * 32)
 rmsnorm_fwd_row_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res_in, const __nv_bfloat16* __restrict__ w,
@@ -555,7 +556,9 @@ int fb_rmsnorm_fwd(const void* x, const void* res_in, const void* w, const void*
     else if (D <= 128) FWD_S(HR, WR, GM, 16);                                                                      \
     else if (D <= 256) FWD_S(HR, WR, GM, 32);                                                                      \
     else if (D <= 512) FWD_R(HR, WR, GM, 2);                                                                       \
+    else if (D <= 768) FWD_R(HR, WR, GM, (GM ? 3 : 4));                                                            \
     else if (D <= 1024) FWD_R(HR, WR, GM, 4);                                                                      \
+    else if (D <= 1280 && !GM) FWD_R(HR, WR, GM, (GM ? 4 : HR ? 5 : 8));                                           \
     else if (D <= 2048 && !GM) FWD_R(HR, WR, GM, (GM ? 4 : 8));                                                    \
     else rmsnorm_fwd_kernel<HR, WR, GM><<<grid, WARPS * 32, 0, stream>>>(X, R, W, G, Y, RO, rstd, rows, D, eps, at);   \
   } while (0)

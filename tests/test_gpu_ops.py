@@ -335,6 +335,13 @@ def test_rmsnorm_forward_of_rows_in_registers(D, rows, form):
     assert any(near)
 
 
+@pytest.mark.parametrize("D", [640, 768, 776, 1272, 1280, 1288])
+@pytest.mark.parametrize("form", ["plain", "sum", "prenorm", "swish", "sigmoid"])
+def test_rmsnorm_forward_of_rows_that_fill_their_vectors(D, form):
+    """Widths around those at which a lane takes three or five vectors instead of four or eight; bounds as in the test above."""
+    test_rmsnorm_forward_of_rows_in_registers(D, 777, form)
+
+
 @pytest.mark.parametrize("H", [1, 3, 4, 5, 9])
 @pytest.mark.parametrize("Dh,rot", [(64, 64), (128, 128), (64, 32), (48, 16)])
 @pytest.mark.parametrize("many", [False, True])
