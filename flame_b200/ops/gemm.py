@@ -122,6 +122,8 @@ def _launch(a, b, M, N, K, a_mn, b_mn, out, accumulate, alpha, bias, splits):
             pend.flush()  # this product reads the unit but cannot carry the gather: fetch with the stand-alone kernel
     ws, launches = None, 1
     dst, ldc = out.data_ptr(), out.stride(0)
+    if splits is None and K <= 448:   # fewer than eight blocks of K: neither form of the library cuts or splits them, no need to ask
+        splits = 0
     if splits is None:
         need = L.fb_gemm_cut_bytes_into(dst, ldc, mode, M, N, K) if bias is None else -1
         if need >= 0:   # the CTA pairs cut the tiles of their last round along K where that pays
