@@ -866,10 +866,10 @@ int max_pairs(int sm_count) {
 
 // Tiles of the last round to be cut along K, and into how many pieces; 0 tiles where that does not pay.  In microseconds: a
 // round costs 0.28 per K block (256 x 256 x 64) with a few pairs at work, 0.38 with all; a piece 0.03 for writing and reading its
-// 256 KB, the second kernel 3; 2 more have to be saved, as the scratch and the second launch cost the host some 5.  One round of
+// 256 KB, the second kernel 3; 1 more has to be saved, as the scratch and the second launch cost the host some 5.  One round of
 // pieces is not always the best: 48 tiles on 74 pairs cut in three take two rounds of a third.  At most three pieces per pair bound the
-// workspace.  Measured with 1 to 16 pieces at 358 products of 1 to 4,000 tiles and 8 to 1,024 K blocks: 1.2 % above the best number of
-// pieces in the mean, 3 us at most in small products (with 0.12 for a piece 3.9 % and 7 us, where a few tiles of 24 to 128 K blocks stayed
+// workspace.  Measured with 1 to 16 pieces at 358 products of 1 to 4,000 tiles and 8 to 1,024 K blocks: 0.8 % above the best number of
+// pieces in the mean, 2 us at most in small products (with 0.12 for a piece 3.9 % and 7 us, where a few tiles of 24 to 128 K blocks stayed
 // whole: 4 tiles of 32 blocks 15.4 us whole, 11.8 in 8 pieces).
 int cut_last_round(long long tiles, int num_kb, int pairs, int* pieces) {
   const int rest = (int)(tiles % pairs);
@@ -879,7 +879,7 @@ int cut_last_round(long long tiles, int num_kb, int pairs, int* pieces) {
   for (int s = 2; s <= 16 && s * rest <= 3 * pairs && s * 4 <= num_kb; ++s) {
     const int kb = (num_kb + s - 1) / s, units = s * rest, rounds = (units + pairs - 1) / pairs;
     if ((s - 1) * kb >= num_kb) continue;  // the last piece would be empty
-    const double cost = rounds * kb * (0.28 + 0.1 * (rounds > 1 ? 1.0 : (double)units / pairs)) + 5.0 + 0.03 * units;
+    const double cost = rounds * kb * (0.28 + 0.1 * (rounds > 1 ? 1.0 : (double)units / pairs)) + 4.0 + 0.03 * units;
     if (cost < best * 0.99) {
       best = cost;
       *pieces = s;
