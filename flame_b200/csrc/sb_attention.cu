@@ -22,7 +22,7 @@
 // issued ahead of this tile's other products, and the weights of eight keys finished while the next eight's exponentials and
 // reciprocals run (one loop for masked tiles and one for the others: with both in one the compiler kept the parts apart, 2.18 ms).
 // Eight rows of 4,096 tokens, 16 heads: 2.46 ms with one CTA of 128 x 128 tiles per SM, 2.03 with two, 1.94 with the eights
-// interleaved, 1.90 with one reciprocal for two keys.  The reference reaches the same sums with spin-locked adds
+// interleaved, 1.87 with one reciprocal for two keys.  The reference reaches the same sums with spin-locked adds
 // (custom_models/sba/stickbreaking_attention/sb_varlen/sb_varlen_bwd.py:13-52); here nothing spins unbounded.
 #include "attn_tiles.cuh"
 #include "sb_math.cuh"

@@ -8,11 +8,12 @@
 // so the eight exponentials, reciprocals and local products of a group overlap with its neighbours'; only E is a chain, one
 // multiplication per group (one per key, behind a correctly rounded reciprocal subroutine, held the softmax warps up before).
 // Two keys share one hardware reciprocal, of the product of their denominators (three special functions for two keys instead of
-// four: forward 854 -> 824 us, backward 1,934 -> 1,900 at eight rows of 4,096 tokens, 16 heads), and each gets a Newton step, which
+// four: forward 854 -> 819 us, backward 1,934 -> 1,872 at eight rows of 4,096 tokens, 16 heads), and each gets a Newton step, which
 // takes out the roundings of the products as well (the remainder against fp64: mean error 3.18e-7, as with one each).  A logit
-// counts as at most 2^100 : 1, so the product of two denominators lies in [1, 2^200]; formed with one of them times 2^-76 it stays,
-// like its reciprocal, a normal number (2^-76 to 2^124), and no bit depends on that factor.  (It costs the forward 27 us and the
-// backward nothing; as t 2^-76 + 2^-76 beside the sum 45, as two scalar products 41.)
+// counts as at most 2^100 : 1.  The product of two denominators has to stay below 2^126, so that its reciprocal is a normal number:
+// the left one of two keys that together exceed 2^124 : 1 counts as what is left of that.  Its weight's sigma is 1 in fp32 all
+// the same (the rest is 2^24 : 1 or more), and what both leave of the row, less than 2^-124, is at the end of the range of fp32.
+// (One clamp at 2^60 : 1 was 22 us less forward and 31 more backward; one denominator times 2^-76 instead 5 and 30 more.)
 //
 // Two keys share an instruction wherever there is a packed one.  It has no negation, so the reciprocal is formed with its sign
 // turned, m = -1 / (1 + t): then 1 + y m is the Newton residual, t m = -sigma, and the sign of the product over k keys, (-1)^k,
@@ -52,21 +53,21 @@ __device__ __forceinline__ uint32_t sb_pack(sb2 v) {  // bf16
 // What does not depend on the keys to the right.  nsig: -sigma, ninv: sigma - 1; nsig[i] holds keys 2 i and 2 i + 1
 template <bool MASK>
 __device__ __forceinline__ void sb_sigma(const uint32_t* x8, float scale_log2, uint32_t dead, sb2 (&nsig)[4], float (&ninv)[8]) {
-  const sb2 one = sb_pk(1.f, 1.f), scale = sb_pk(scale_log2, scale_log2), low = sb_pk(0x1p-76f, 0x1p-76f);
+  const sb2 one = sb_pk(1.f, 1.f), scale = sb_pk(scale_log2, scale_log2);
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    float x0, x1, t0, t1, y0, y1, z0, z1;
+    float x0, x1, t0, t1, y0, y1;
     sb_up(sb_mul2(sb_pk(__uint_as_float(x8[2 * i]), __uint_as_float(x8[2 * i + 1])), scale), x0, x1);
-    x0 = fminf(fmaxf(x0, -100.f), 100.f);
+    if (MASK && ((dead >> (2 * i + 1)) & 1u)) x1 = -100.f;  // a key that does not count takes nothing from its neighbour
     x1 = fminf(fmaxf(x1, -100.f), 100.f);
+    x0 = fminf(fminf(fmaxf(x0, -100.f), 100.f), 124.f - x1);
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(x0));
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(x1));
     const sb2 t = sb_pk(t0, t1), y = sb_add2(t, one);
     sb_up(y, y0, y1);
-    sb_up(sb_mul2(y, low), z0, z1);
     float both;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(both) : "f"(-y0 * z1));
-    sb2 m = sb_pk(both * z1, both * z0);
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(both) : "f"(-y0 * y1));
+    sb2 m = sb_pk(both * y1, both * y0);
     m = sb_fma2(m, sb_fma2(y, m, one), m);
     nsig[i] = sb_mul2(t, m);
     sb_up(m, ninv[2 * i], ninv[2 * i + 1]);

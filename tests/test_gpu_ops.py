@@ -525,6 +525,31 @@ def test_stickbreaking_remainder_beside_dominating_keys(nats):
     assert ((rem.double() - want).abs() <= 2.0 ** -17 * want).all()
 
 
+@pytest.mark.parametrize("left,right", [(42.0, 42.0), (16.0, 69.0), (69.0, 16.0), (60.0, 25.5), (69.0, 69.0), (80.0, 80.0), (5.0, 69.0)])
+@pytest.mark.parametrize("at", [4, 5])
+def test_stickbreaking_remainder_beside_two_dominating_neighbours(left, right, at):
+    """Two large logits next to one another, at either place in a pair of keys: what they leave of a row, relative to itself down to 2^-124 (bound of
+    the test above, twice), below 2^-123 where it is less; the weights of the keys around them likewise."""
+    from flame_b200.ops.stickbreaking import sb_attention
+    n = 10
+    q, k, v = (torch.zeros(n, 1, 64, device=DEV) for _ in range(3))
+    q[:, 0, 0], k[at, 0, 0], k[at + 1, 0, 0] = 16.0, left / 2, right / 2
+    v[:, 0, :n] = torch.eye(n, device=DEV)     # outputs are the weights
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    o, rem = sb_attention(q, k, v, _meta([n]))
+    rem = rem.reshape(n)
+    logits = q[:, 0].double() @ k[:, 0].double().t() / 8
+    logits = logits.clamp(max=100 * 0.6931471805599453)
+    mask = torch.ones(n, n, device=DEV, dtype=torch.bool).triu()
+    stay = torch.nn.functional.logsigmoid(-logits).masked_fill(mask, 0.0)
+    want = stay.sum(-1).exp()
+    att = ((torch.nn.functional.logsigmoid(logits) + stay.flip(-1).cumsum(-1).flip(-1) - stay).exp()).masked_fill(mask, 0.0)
+    small = want < 2.0 ** -124
+    assert ((rem.double() - want).abs() <= 2.0 ** -16 * want)[~small].all() and (rem[small] < 2.0 ** -123).all()
+    got = o[:, 0, :n].double()
+    assert ((got - att).abs() <= 2.0 ** -8 * att + 2.0 ** -123).all()
+
+
 def test_short_conv_forward_backward():
     from flame_b200.ops import linear_attn as la
     from flame_b200.ops.conv import short_conv
