@@ -549,7 +549,6 @@ extern "C" int fb_gemm2_bf16(const void* A, const void* B, void* C, int M, int N
                              int sm_count, cudaStream_t stream);
 
 extern "C" long long fb_gemm2_cut_bytes(int M, int N, int K, int sm_count);
-extern "C" long long fb_gemm2_cut_bytes_into(const void* C, long long ldc, int out_mode, int M, int N, int K, int sm_count);
 extern "C" int fb_gemm2_allgather_a(const unsigned long long* shard_ptrs, int world, int rank, int rows_per_rank, long long ld,
                                     void* a_full, int* chunk_flags, const int* ready, int epoch, const void* B, void* C, int N,
                                     int K, long long ldb, long long ldc, int b_mn, int sm_count, cudaStream_t stream);
@@ -571,14 +570,9 @@ long long fb_gemm_workspace_bytes(int M, int N, int splits) {
   return splits > 1 ? (long long)splits * M * N * 4 : 0;
 }
 
-// Bytes of workspace for splits == 0 of fb_gemm_bf16 without bias: 0 where none is needed, -1 where that form does not apply (single-CTA
-// kernel) and fb_gemm_pick_splits chooses.
+// Bytes of workspace for splits == 0 of fb_gemm_bf16 without bias and with a result that starts and has its rows on 16 bytes: 0 where none is
+// needed, -1 where that form does not apply (single-CTA kernel) and, as for other results, fb_gemm_pick_splits chooses.
 long long fb_gemm_cut_bytes(int M, int N, int K) { return g_variant == 2 ? fb_gemm2_cut_bytes(M, N, K, sm_count_cached()) : -1; }
-
-// The same for the result that fb_gemm_bf16 is to be given: -1 also where its rows or its start rule out tensor copies.
-long long fb_gemm_cut_bytes_into(const void* C, long long ldc, int out_mode, int M, int N, int K) {
-  return g_variant == 2 ? fb_gemm2_cut_bytes_into(C, ldc, out_mode, M, N, K, sm_count_cached()) : -1;
-}
 
 // Where nothing is cut (the single-CTA kernel, results that no tensor copy can write): chooses a split-K factor with a small cost model: waves of work units times K blocks per unit, plus the
 // traffic of writing and re-reading the fp32 partials.  Few-tile, long-K GEMMs (weight gradients) gain most.

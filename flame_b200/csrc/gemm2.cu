@@ -866,21 +866,24 @@ int max_pairs(int sm_count) {
 
 // Tiles of the last round to be cut along K, and into how many pieces; 0 tiles where that does not pay.  In microseconds: a
 // round costs 0.28 per K block (256 x 256 x 64) with a few pairs at work, 0.38 with all; a piece 0.03 for writing and reading its
-// 256 KB, the second kernel 3; 1 more has to be saved, as the scratch and the second launch cost the host some 5.  One round of
-// pieces is not always the best: 48 tiles on 74 pairs cut in three take two rounds of a third.  At most three pieces per pair bound the
-// workspace.  Measured with 1 to 16 pieces at 358 products of 1 to 4,000 tiles and 8 to 1,024 K blocks: 0.8 % above the best number of
-// pieces in the mean, 2 us at most in small products (with 0.12 for a piece 3.9 % and 7 us, where a few tiles of 24 to 128 K blocks stayed
-// whole: 4 tiles of 32 blocks 15.4 us whole, 11.8 in 8 pieces).
+// 256 KB, the second kernel 3 (and 1 to be saved).  Measured with 1 to 16 pieces at 358 products of 1 to 4,000 tiles and 8 to 1,024 K
+// blocks: 0.8 % above the best number of pieces in the mean.  Products of less than 40 us stand in passes that the host bounds, whom
+// scratch and a second launch cost 8 and, with what they displace, up to 17 (an MLP pass over 2,048 tokens, 340M width: 352 us, with three
+// products cut that take 3 to 7 us less so, 433): there a piece counts as 0.12, the second kernel as 5 and a K block as 0.02 more, which
+// leaves few tiles of up to some 40 blocks whole (4 tiles of 32 blocks: 15.4 us, 11.8 in 8 pieces).  One round of pieces is not always
+// the best: 48 tiles on 74 pairs cut in three take two rounds of a third.  At most three pieces per pair bound the workspace.
 int cut_last_round(long long tiles, int num_kb, int pairs, int* pieces) {
   const int rest = (int)(tiles % pairs);
   *pieces = 1;
   if (rest == 0) return 0;
-  double best = num_kb * (0.28 + 0.1 * rest / pairs);
+  const bool brief = num_kb * (0.28 + 0.1 * rest / pairs + 0.38 * (double)(tiles / pairs)) < 40.0;
+  const double block = brief ? 0.3 : 0.28, second = brief ? 5.0 : 4.0, each = brief ? 0.12 : 0.03;
+  double best = num_kb * (block + 0.1 * rest / pairs);
   for (int s = 2; s <= 16 && s * rest <= 3 * pairs && s * 4 <= num_kb; ++s) {
     const int kb = (num_kb + s - 1) / s, units = s * rest, rounds = (units + pairs - 1) / pairs;
     if ((s - 1) * kb >= num_kb) continue;  // the last piece would be empty
-    const double cost = rounds * kb * (0.28 + 0.1 * (rounds > 1 ? 1.0 : (double)units / pairs)) + 4.0 + 0.03 * units;
-    if (cost < best * 0.99) {
+    const double cost = rounds * kb * (block + 0.1 * (rounds > 1 ? 1.0 : (double)units / pairs)) + second + each * units;
+    if (cost < best * 0.97) {
       best = cost;
       *pieces = s;
     }
@@ -957,7 +960,8 @@ int start2(const CUtensorMap& tmA, const CUtensorMap& tmB, const CUtensorMap& tm
   return fb::launch_ok(FP8 ? "gemm2_fp8_kernel" : "gemm2_bf16_kernel");
 }
 
-// Whether a result of N columns of `bytes` each can leave by TMA: rows and start on 16 bytes.
+// Whether a result of N columns of `bytes` each can leave by TMA: rows and start on 16 bytes.  (ops/gemm.py asks the same before it provides
+// scratch: others are not cut.)
 bool tma_result(const void* C, long long ldc, int N, int bytes) { return (ldc * bytes & 15) == 0 && ldc >= N && !((uintptr_t)C & 15); }
 
 template <bool A_MN, bool B_MN, bool FP8 = false>
@@ -984,17 +988,12 @@ int launch2(const CUtensorMap& tmA, const CUtensorMap& tmB, Gemm2Params& p, int 
 
 extern "C" {
 
-// Bytes of workspace with which fb_gemm2_bf16 cuts the tiles of its last round along K; 0 where it would not.
+// Bytes of workspace with which fb_gemm2_bf16 cuts the tiles of its last round along K if the result can leave by TMA; 0 where it would not.
 long long fb_gemm2_cut_bytes(int M, int N, int K, int sm_count) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   int pieces;
   const long long cut = cut_last_round((long long)((M + BM2 - 1) / BM2) * ((N + BN - 1) / BN), (K + BK - 1) / BK, max_pairs(sm_count), &pieces);
   return cut * pieces * TILE_FLOATS * 4;
-}
-
-// The same for a given result; -1 where it cannot leave by TMA, which the pieces' tiles have to.
-long long fb_gemm2_cut_bytes_into(const void* C, long long ldc, int out_mode, int M, int N, int K, int sm_count) {
-  return tma_result(C, ldc, N, out_mode == 0 ? 2 : 4) ? fb_gemm2_cut_bytes(M, N, K, sm_count) : -1;
 }
 
 // Same contract as fb_gemm_bf16 without bias; splits == 0: the last round may be cut, `workspace` (or null) as

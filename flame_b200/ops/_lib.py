@@ -160,8 +160,6 @@ def _declare(L: ctypes.CDLL) -> None:
     L.fb_gemm_workspace_bytes.restype = c_longlong
     L.fb_gemm_cut_bytes.argtypes = [i, i, i]
     L.fb_gemm_cut_bytes.restype = c_longlong
-    L.fb_gemm_cut_bytes_into.argtypes = [vp, ll, i, i, i, i]
-    L.fb_gemm_cut_bytes_into.restype = c_longlong
     for name, args, res in _EXTRA_SIGS:
         fn = getattr(L, name, None)
         if fn is not None:

@@ -125,8 +125,10 @@ def _launch(a, b, M, N, K, a_mn, b_mn, out, accumulate, alpha, bias, splits):
     if splits is None and K <= 448:   # fewer than eight blocks of K: neither form of the library cuts or splits them, no need to ask
         splits = 0
     if splits is None:
-        need = L.fb_gemm_cut_bytes_into(dst, ldc, mode, M, N, K) if bias is None else -1
-        if need >= 0:   # the CTA pairs cut the tiles of their last round along K where that pays
+        # the CTA pairs cut the tiles of their last round along K where that pays, if tensor copies can write the result
+        copies = bias is None and not dst & 15 and not ldc & (3 if mode else 7) and ldc >= N
+        need = L.fb_gemm_cut_bytes(M, N, K) if copies else -1
+        if need >= 0:
             splits = 0
             if need:
                 ws, launches = _workspace(out.device, need), 2
